@@ -8,6 +8,7 @@
 // model/mlp.py:12-26, model/embedding.py:9-29, training/loss.py:19-102,
 // training/optimizer.py:28-39 (torch.optim.AdamW update rule).
 #include "common.cuh"
+#include "skinny_common.cuh"
 
 namespace kf {
 
@@ -82,6 +83,8 @@ kf_rmsnorm_fwd(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
   __shared__ float red[40];
   const int nvec = D >> 3;
   constexpr int CACHED = NORM_CACHE * NORM_THREADS;  // vectors kept in registers per row
+  grid_dep_wait();
+  grid_dep_launch();
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const __nv_bfloat16* xr = x + size_t(row) * D;
     F8 cache[NORM_CACHE];
@@ -614,13 +617,28 @@ static inline int grid_for(long long work, int threads, int cap = 148 * 16) {
 
 extern "C" {
 
-int kf_rmsnorm_fwd_bf16(const void* x, const void* w, void* y, void* rstd, int rows, int D, float eps,
-                        void* stream) {
+// pdl: programmatic launch (the kernel reads nothing before its griddepcontrol.wait, so any predecessor is fine).
+int kf_rmsnorm_fwd_pdl_bf16(const void* x, const void* w, void* y, void* rstd, int rows, int D, float eps, int pdl,
+                            void* stream) {
   using namespace kf;
   if (D % 8) return 1;
-  kf_rmsnorm_fwd<<<rows < 148 * 8 ? rows : 148 * 8, NORM_THREADS, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, (float*)rstd, rows, D, eps);
-  KF_LAUNCH_CHECK();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(rows < 148 * 8 ? rows : 148 * 8);
+  cfg.blockDim = dim3(NORM_THREADS);
+  cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kf_rmsnorm_fwd, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
+                                     (__nv_bfloat16*)y, (float*)rstd, rows, D, eps);
+  return e == cudaSuccess ? 0 : 400 + (int)e;
+}
+
+int kf_rmsnorm_fwd_bf16(const void* x, const void* w, void* y, void* rstd, int rows, int D, float eps,
+                        void* stream) {
+  return kf_rmsnorm_fwd_pdl_bf16(x, w, y, rstd, rows, D, eps, 0, stream);
 }
 
 // Number of fp32 partial rows rmsnorm_bwd writes (the workspace must hold nblocks * D floats).

@@ -251,14 +251,19 @@ int launch_gemm_2cta(const void* A, const void* B, void* C, const void* R, int M
 }
 
 namespace kf2 {
-int launch_gemm_swiglu_2cta(const void* A, const void* W, void* H, void* GU, int M, int F, int K, int lda, int ldw, int ldh,
-                            int ldgu, int num_sms, cudaStream_t stream, int* status);
+int launch_gemm_swiglu_2cta(const void* A, const void* Wg, const void* Wu, void* H, void* GU, int M, int F, int K, int lda,
+                            int ldw, int ldh, int ldgu, int num_sms, cudaStream_t stream, int* status);
 }
 
 namespace kf2 {
-int launch_gemm_rope_2cta(const void* A, const void* W, void* C, int M, int N, int K, int lda, int ldw, int ldc,
-                          const float* cosT, const float* sinT, int S, int rope_cols, int hd, int num_sms,
+int launch_gemm_rope_2cta(const void* A, const void* const* W, const int* rows, void* C, int M, int N, int K, int lda,
+                          int ldw, int ldc, const float* cosT, const float* sinT, int S, int rope_cols, int hd, int num_sms,
                           cudaStream_t stream, int* status);
+}
+
+namespace kf2 {
+int launch_gemm_stacked_k_2cta(const void* A, const void* const* W, const int* rows, void* C, int M, int N, int K, int lda,
+                               int ldw, int ldc, int num_sms, cudaStream_t stream, int* status);
 }
 
 namespace kf2 {
@@ -288,6 +293,17 @@ int kf_gemm_swiglu_bwd_bf16(const void* dy, const void* w, const void* gu, void*
   if ((lda & 7) || (ldw & 7) || (ldgu & 7) || (F & 7) || (K % 64)) return 5;
   return kf2::launch_gemm_swiglu_bwd_2cta(dy, w, gu, dgu, M, F, K, lda, ldw, ldgu, num_sms, (cudaStream_t)stream,
                                           kf::status_ptr());
+}
+
+// Input gradient of a projection whose weight is up to three matrices [n_i][K] stacked along the output (n1 = n2 = 0: one):
+// out[M, K] = dy[M, n0 + n1 + n2] * [w0 ; w1 ; w2].  All but the last n_i a multiple of 64; pitches multiples of 8.
+int kf_gemm_dgrad_stacked_bf16(const void* dy, const void* w0, const void* w1, const void* w2, void* out, int M, int K,
+                               int n0, int n1, int n2, int lda, int ldw, int ldc, int num_sms, void* stream) {
+  if ((lda & 7) || (ldw & 7) || (ldc & 7) || M <= 0 || K <= 0) return 5;
+  const void* w[3] = {w0, w1, w2};
+  const int rows[3] = {n0, n1, n2};
+  return kf2::launch_gemm_stacked_k_2cta(dy, w, rows, out, M, K, n0 + n1 + n2, lda, ldw, ldc, num_sms, (cudaStream_t)stream,
+                                         kf::status_ptr());
 }
 
 // Symmetric product with a polynomial epilogue (the Gram matrix and the quintic of Muon's Newton-Schulz iteration):
@@ -320,21 +336,25 @@ int kf_gemm_gather_bf16(int epi, const void* x, void* out, const void* R, int M,
 
 // Fused Q | K | V projection with the rotary embedding in the epilogue: out[M, N] = x W^T, then every head of `hd`
 // columns inside the first `rope_cols` columns is rotated by the angle of position (row % S); cos / sin are fp32
-// [S][hd / 2].  N and rope_cols multiples of hd (64, 128 or 256); pitches in elements, multiples of 8.
-int kf_gemm_rope_bf16(const void* x, const void* w, void* out, int M, int N, int K, int lda, int ldw, int ldc,
-                      const void* cosT, const void* sinT, int S, int rope_cols, int hd, int num_sms, void* stream) {
+// [S][hd / 2].  W = up to three matrices [n_i][K] stacked along N (n1 = n2 = 0: one), all but the last with n_i % 128 == 0.
+// N and rope_cols multiples of hd (64, 128 or 256); pitches in elements, multiples of 8.
+int kf_gemm_rope_bf16(const void* x, const void* w0, const void* w1, const void* w2, void* out, int M, int n0, int n1,
+                      int n2, int K, int lda, int ldw, int ldc, const void* cosT, const void* sinT, int S, int rope_cols,
+                      int hd, int num_sms, void* stream) {
   if ((lda & 7) || (ldw & 7) || (ldc & 7)) return 5;
-  return kf2::launch_gemm_rope_2cta(x, w, out, M, N, K, lda, ldw, ldc, (const float*)cosT, (const float*)sinT, S,
+  const void* w[3] = {w0, w1, w2};
+  const int rows[3] = {n0, n1, n2};
+  return kf2::launch_gemm_rope_2cta(x, w, rows, out, M, n0 + n1 + n2, K, lda, ldw, ldc, (const float*)cosT, (const float*)sinT, S,
                                     rope_cols, hd, num_sms, (cudaStream_t)stream, kf::status_ptr());
 }
 
-// SwiGLU up-projection in one kernel: h[M, F] = silu(x Wg^T) * (x Wu^T), W = [Wg ; Wu] stacked as [2F][K] (K contiguous).
+// SwiGLU up-projection in one kernel: h[M, F] = silu(x Wg^T) * (x Wu^T), Wg and Wu [F][K] (K contiguous) of one pitch.
 // gu (optional, [M, 2F]) receives the bf16 pre-activations (gate | up) for the backward pass.  F must be a multiple of
 // 128; pitches in elements, multiples of 8.
-int kf_gemm_swiglu_bf16(const void* x, const void* w, void* h, void* gu, int M, int F, int K, int lda, int ldw, int ldh,
-                        int ldgu, int num_sms, void* stream) {
+int kf_gemm_swiglu_bf16(const void* x, const void* wg, const void* wu, void* h, void* gu, int M, int F, int K, int lda,
+                        int ldw, int ldh, int ldgu, int num_sms, void* stream) {
   if ((F % 128) || (lda & 7) || (ldw & 7) || (ldh & 7) || (gu && (ldgu & 7))) return 5;
-  return kf2::launch_gemm_swiglu_2cta(x, w, h, gu, M, F, K, lda, ldw, ldh, ldgu, num_sms, (cudaStream_t)stream,
+  return kf2::launch_gemm_swiglu_2cta(x, wg, wu, h, gu, M, F, K, lda, ldw, ldh, ldgu, num_sms, (cudaStream_t)stream,
                                       kf::status_ptr());
 }
 

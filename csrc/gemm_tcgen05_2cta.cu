@@ -99,9 +99,19 @@ struct RopeArgs {
   float alpha, beta, diag;  // SWIGLU == 4 only
 };
 
+// Weight operand made of up to three matrices stacked along N (q | k | v; SwiGLU == 1: gate and up): one tensor map each,
+// so separate Linear weights are read in place.  start[i] = first stacked row of matrix i, a multiple of HALF_N, so the
+// 128 rows one CTA loads never straddle two matrices.  With B_MN (the same stack read for an input gradient, the stacked
+// rows being the reduction index) the segments lie along K and the starts are multiples of BK.  An operand in one piece
+// has start[1] = start[2] = INT_MAX.
+struct WeightSegs {
+  CUtensorMap map[3];
+  int start[3];
+};
+
 template <bool A_MN, bool B_MN, typename OutT, int SWIGLU = 0, bool GATHER = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GATHER ? THREADS_GATHER : THREADS, 1)
-kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ WeightSegs ws,
                           OutT* __restrict__ C, const OutT* __restrict__ R, int M, int N, int K, int ldc, int ldr,
                           int accumulate, int* status, RopeArgs rope, const __grid_constant__ GatherArgs ga) {
   extern __shared__ uint8_t smem_raw[];
@@ -160,7 +170,7 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
     mbar_init(drain_bar, 1);
     mbar_fence_init();
     tma_prefetch_desc(&map_a);
-    tma_prefetch_desc(&map_b);
+    tma_prefetch_desc(&ws.map[0]);
   }
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, TMEM_COLS);
@@ -180,12 +190,16 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
         const TileCoord tc = tile_at(t);
         const int m0 = tc.m * TILE_M + int(rank) * CTA_M;
-        const int n0 = SWIGLU == 1 ? tc.n * HALF_N + int(rank) * N  // leader: gate rows, peer: the matching up rows
-                                   : tc.n * TILE_N + int(rank) * HALF_N;
+        const int n_op = SWIGLU == 1 ? tc.n * HALF_N + int(rank) * N  // leader: gate rows, peer: the matching up rows
+                                     : tc.n * TILE_N + int(rank) * HALF_N;
+        // matrix that holds these operand rows, and the first of them inside it
+        const int sg = B_MN ? 0 : int(n_op >= ws.start[1]) + int(n_op >= ws.start[2]);
+        const CUtensorMap* map_b = &ws.map[sg];
+        const int n0 = n_op - ws.start[sg];
         if constexpr (GATHER) {
           // the 128 weight rows this CTA loads must have landed in the staging copy
-          if (n0 < N * (SWIGLU == 1 ? 2 : 1)) {
-            if (!flag_wait_ge(ga.flags + n0 / HALF_N, ga.chunks_per_rb, status)) { ok = false; break; }
+          if (n_op < N * (SWIGLU == 1 ? 2 : 1)) {
+            if (!flag_wait_ge(ga.flags + n_op / HALF_N, ga.chunks_per_rb, status)) { ok = false; break; }
             asm volatile("fence.proxy.async;" ::: "memory");  // generic-proxy stores -> this thread's TMA reads
           }
         }
@@ -206,11 +220,12 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
               tma_load_2d_pair(a_dst + c * (64 * BK * 2), &map_a, lead_full, m0 + 64 * c, k0);
           }
           if (!B_MN) {
-            tma_load_2d_pair(b_dst, &map_b, lead_full, k0, n0);
+            tma_load_2d_pair(b_dst, map_b, lead_full, k0, n0);
           } else {
+            const int ks = int(k0 >= ws.start[1]) + int(k0 >= ws.start[2]);
 #pragma unroll
             for (int c = 0; c < HALF_N / 64; ++c)
-              tma_load_2d_pair(b_dst + c * (64 * BK * 2), &map_b, lead_full, n0 + 64 * c, k0);
+              tma_load_2d_pair(b_dst + c * (64 * BK * 2), &ws.map[ks], lead_full, n0 + 64 * c, k0 - ws.start[ks]);
           }
         }
       }
@@ -488,6 +503,10 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
   }
 }
 
+static WeightSegs one_piece(const CUtensorMap& m) {
+  return WeightSegs{{m, m, m}, {0, 0x7fffffff, 0x7fffffff}};
+}
+
 template <bool A_MN, bool B_MN, typename OutT>
 static int launch(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb, int ldc,
                   int ldr, int accumulate, int num_sms, cudaStream_t stream, int* status) {
@@ -506,21 +525,27 @@ static int launch(const void* A, const void* B, void* C, const void* R, int M, i
   const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N);
   int pairs = num_sms / 2;
   if (tiles < pairs) pairs = tiles;
-  kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, mb, reinterpret_cast<OutT*>(C),
+  kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, one_piece(mb), reinterpret_cast<OutT*>(C),
                                                    reinterpret_cast<const OutT*>(R), M, N, K, ldc, ldr, accumulate,
                                                    status, RopeArgs{nullptr, nullptr, 1, 0, 64}, GatherArgs{});
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
-// h[M, F] = silu(x Wg^T) * (x Wu^T) with W = [Wg ; Wu] stacked ([2F][K]); gu (optional) receives [M, 2F] pre-activations
-int launch_gemm_swiglu_2cta(const void* A, const void* W, void* H, void* GU, int M, int F, int K, int lda, int ldw, int ldh,
-                            int ldgu, int num_sms, cudaStream_t stream, int* status) {
-  CUtensorMap ma, mb;
+// h[M, F] = silu(x Wg^T) * (x Wu^T), Wg and Wu [F][K] each; gu (optional) receives [M, 2F] pre-activations.  F % 128 == 0.
+int launch_gemm_swiglu_2cta(const void* A, const void* Wg, const void* Wu, void* H, void* GU, int M, int F, int K, int lda,
+                            int ldw, int ldh, int ldgu, int num_sms, cudaStream_t stream, int* status) {
+  CUtensorMap ma;
+  WeightSegs ws;
   int rc = make_map_2d_bf16(&ma, A, M, K, lda, BK, CTA_M);
   if (rc) return 100 + rc;
-  rc = make_map_2d_bf16(&mb, W, 2 * (uint64_t)F, K, ldw, BK, HALF_N);
+  rc = make_map_2d_bf16(&ws.map[0], Wg, F, K, ldw, BK, HALF_N);
+  if (!rc) rc = make_map_2d_bf16(&ws.map[1], Wu, F, K, ldw, BK, HALF_N);
   if (rc) return 200 + rc;
+  ws.map[2] = ws.map[1];
+  ws.start[0] = 0;
+  ws.start[1] = F;
+  ws.start[2] = 0x7fffffff;
   auto kern = kf_gemm_bf16_tcgen05_2cta<false, false, __nv_bfloat16, 1>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -531,7 +556,7 @@ int launch_gemm_swiglu_2cta(const void* A, const void* W, void* H, void* GU, int
   const int tiles = ((M + TILE_M - 1) / TILE_M) * ((F + HALF_N - 1) / HALF_N);
   int pairs = num_sms / 2;
   if (tiles < pairs) pairs = tiles;
-  kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, mb, reinterpret_cast<__nv_bfloat16*>(H),
+  kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, ws, reinterpret_cast<__nv_bfloat16*>(H),
                                                    reinterpret_cast<const __nv_bfloat16*>(GU), M, F, K, ldh, ldgu, 0, status,
                                                    RopeArgs{nullptr, nullptr, 1, 0, 64}, GatherArgs{});
   cudaError_t e = cudaGetLastError();
@@ -540,15 +565,28 @@ int launch_gemm_swiglu_2cta(const void* A, const void* W, void* H, void* GU, int
 
 // qkv[M, N] = x W^T with the rotary embedding applied to the first `rope_cols` output columns (heads of `hd` columns,
 // position = row % S).  N and rope_cols must be multiples of hd; hd in {64, 128, 256}; tables fp32 [S][hd / 2].
-int launch_gemm_rope_2cta(const void* A, const void* W, void* C, int M, int N, int K, int lda, int ldw, int ldc,
-                          const float* cosT, const float* sinT, int S, int rope_cols, int hd, int num_sms,
+// The weight is up to three matrices of rows[i] x K (rows[0] + rows[1] + rows[2] == N, all but the last a multiple of 128).
+int launch_gemm_rope_2cta(const void* A, const void* const* W, const int* rows, void* C, int M, int N, int K, int lda,
+                          int ldw, int ldc, const float* cosT, const float* sinT, int S, int rope_cols, int hd, int num_sms,
                           cudaStream_t stream, int* status) {
   if ((hd != 64 && hd != 128 && hd != 256) || N % hd || rope_cols % hd || rope_cols > N || S <= 0) return 6;
-  CUtensorMap ma, mb;
+  CUtensorMap ma;
+  WeightSegs ws;
   int rc = make_map_2d_bf16(&ma, A, M, K, lda, BK, CTA_M);
   if (rc) return 100 + rc;
-  rc = make_map_2d_bf16(&mb, W, N, K, ldw, BK, HALF_N);
-  if (rc) return 200 + rc;
+  int at = 0, n = 0;
+  for (; n < 3 && rows[n] > 0; ++n) {
+    if (at % HALF_N) return 6;
+    rc = make_map_2d_bf16(&ws.map[n], W[n], rows[n], K, ldw, BK, HALF_N);
+    if (rc) return 200 + rc;
+    ws.start[n] = at;
+    at += rows[n];
+  }
+  if (n == 0 || at != N) return 6;
+  for (; n < 3; ++n) {
+    ws.map[n] = ws.map[0];
+    ws.start[n] = 0x7fffffff;
+  }
   auto kern = kf_gemm_bf16_tcgen05_2cta<false, false, __nv_bfloat16, 2>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -559,7 +597,7 @@ int launch_gemm_rope_2cta(const void* A, const void* W, void* C, int M, int N, i
   const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N);
   int pairs = num_sms / 2;
   if (tiles < pairs) pairs = tiles;
-  kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, mb, reinterpret_cast<__nv_bfloat16*>(C), nullptr, M, N, K, ldc, 0, 0,
+  kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, ws, reinterpret_cast<__nv_bfloat16*>(C), nullptr, M, N, K, ldc, 0, 0,
                                                    status, RopeArgs{cosT, sinT, S, rope_cols, hd}, GatherArgs{});
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
@@ -590,7 +628,7 @@ int launch_gemm_symm_2cta(int x_mn, const void* X, void* C, const void* R, int n
       if (e != cudaSuccess) return 300 + (int)e;                                                                     \
       attr_set = true;                                                                                               \
     }                                                                                                                \
-    kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, mb, reinterpret_cast<__nv_bfloat16*>(C),                    \
+    kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, one_piece(mb), reinterpret_cast<__nv_bfloat16*>(C),                    \
                                                      reinterpret_cast<const __nv_bfloat16*>(R), n, n, K, ldc, ldr, 0, \
                                                      status, ra, GatherArgs{});                                      \
   }
@@ -653,7 +691,7 @@ int launch_gemm_gather_2cta(int epi, const void* A, void* C, const void* R, int 
       if (e != cudaSuccess) return 300 + (int)e;                                                                     \
       attr_set = true;                                                                                               \
     }                                                                                                                \
-    kern<<<pairs * 2, THREADS_GATHER, SMEM_BYTES, stream>>>(ma, mb, reinterpret_cast<__nv_bfloat16*>(C),             \
+    kern<<<pairs * 2, THREADS_GATHER, SMEM_BYTES, stream>>>(ma, one_piece(mb), reinterpret_cast<__nv_bfloat16*>(C),  \
                                                             reinterpret_cast<const __nv_bfloat16*>(R), M, N, K, ldc, ldr, \
                                                             0, status, ra, ga);                                      \
   }
@@ -682,9 +720,46 @@ int launch_gemm_swiglu_bwd_2cta(const void* DY, const void* W, const void* GU, v
   const int tiles = ((M + TILE_M - 1) / TILE_M) * ((F + TILE_N - 1) / TILE_N);
   int pairs = num_sms / 2;
   if (tiles < pairs) pairs = tiles;
-  kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, mb, reinterpret_cast<__nv_bfloat16*>(DGU),
+  kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, one_piece(mb), reinterpret_cast<__nv_bfloat16*>(DGU),
                                                    reinterpret_cast<const __nv_bfloat16*>(GU), M, F, K, ldgu, ldgu, 0, status,
                                                    RopeArgs{nullptr, nullptr, 1, 0, 64}, GatherArgs{});
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 400 + (int)e;
+}
+
+// C[M, N] = A[M, K] * W with W = up to three matrices [rows[i]][N] stacked along K (rows summing to K, all but the last a
+// multiple of 64): the input gradient of a projection with several weights.
+int launch_gemm_stacked_k_2cta(const void* A, const void* const* W, const int* rows, void* C, int M, int N, int K, int lda,
+                               int ldw, int ldc, int num_sms, cudaStream_t stream, int* status) {
+  CUtensorMap ma;
+  WeightSegs ws;
+  int rc = make_map_2d_bf16(&ma, A, M, K, lda, BK, CTA_M);
+  if (rc) return 100 + rc;
+  int at = 0, n = 0;
+  for (; n < 3 && rows[n] > 0; ++n) {
+    if (at % BK) return 6;
+    rc = make_map_2d_bf16(&ws.map[n], W[n], rows[n], N, ldw, 64, BK);
+    if (rc) return 200 + rc;
+    ws.start[n] = at;
+    at += rows[n];
+  }
+  if (n == 0 || at != K) return 6;
+  for (; n < 3; ++n) {
+    ws.map[n] = ws.map[0];
+    ws.start[n] = 0x7fffffff;
+  }
+  auto kern = kf_gemm_bf16_tcgen05_2cta<false, true, __nv_bfloat16>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    if (e != cudaSuccess) return 300 + (int)e;
+    attr_set = true;
+  }
+  const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N);
+  int pairs = num_sms / 2;
+  if (tiles < pairs) pairs = tiles;
+  kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, ws, reinterpret_cast<__nv_bfloat16*>(C), nullptr, M, N, K, ldc, 0, 0,
+                                                   status, RopeArgs{nullptr, nullptr, 1, 0, 64}, GatherArgs{});
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }

@@ -98,6 +98,13 @@ class TransformerBlock(nn.Module):
         return x + self.mlp(self.mlp_norm(x))
 
     def forward(self, x, rope_cos, rope_sin, *, kv_cache: KVCache | None = None, doc_ids=None, key_padding_mask=None):
+        if (x.is_cuda and doc_ids is None and key_padding_mask is None and not _FUSED_BLOCK_OFF
+                and not torch.is_grad_enabled() and F.use_native(x)):
+            from kempnerforge_b200.ops import fused_infer
+
+            y = fused_infer.run(self, x, rope_cos, rope_sin, kv_cache)
+            if y is not None:
+                return y
         if (x.is_cuda and self.ac_mode in ("none", "full") and not _FUSED_BLOCK_OFF
                 and not getattr(self, "_kf_fp8_block", False)):
             from kempnerforge_b200.ops import fused_block

@@ -11,6 +11,7 @@ from __future__ import annotations
 import ctypes
 import math
 import os
+from array import array
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
 import torch
@@ -50,8 +51,15 @@ def _declare(L: ctypes.CDLL) -> None:
     vp, i, ll, f = c_void_p, c_int, c_longlong, c_float
     sigs = {
         "kf_gemm_bf16": [vp, vp, vp, vp, i, i, i, i, i, i, i, i, i, i, i, i, i, vp],
-        "kf_gemm_swiglu_bf16": [vp, vp, vp, vp, i, i, i, i, i, i, i, i, vp],
-        "kf_gemm_rope_bf16": [vp, vp, vp, i, i, i, i, i, i, vp, vp, i, i, i, i, vp],
+        "kf_gemm_swiglu_bf16": [vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, vp],
+        "kf_gemm_rope_bf16": [vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, vp, vp, i, i, i, i, vp],
+        "kf_gemm_dgrad_stacked_bf16": [vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, i, vp],
+        "kf_gemm_skinny_bf16": [vp] * 6 + [i] * 14 + [vp],
+        "kf_gemm_skinny_swiglu_bf16": [vp] * 4 + [i] * 9 + [vp],
+        "kf_gemm_skinny_qkv_bf16": [vp] * 7 + [i] * 11 + [ll, vp, vp, i, i, vp],
+        "kf_rmsnorm_fwd_pdl_bf16": [vp, vp, vp, vp, i, i, f, i, vp],
+        "kf_attn_decode_bf16": [vp] * 4 + [i] * 5 + [ll] * 5 + [f, i, i, i, vp],
+        "kf_block_decode_bf16": [vp, vp, vp],
         "kf_gemm_swiglu_bwd_bf16": [vp, vp, vp, vp, i, i, i, i, i, i, i, vp],
         "kf_gemm_symm_bf16": [i, vp, vp, vp, i, i, i, i, i, f, f, f, i, vp],
         "kf_rmsnorm_fwd_bf16": [vp, vp, vp, vp, i, i, f, vp],
@@ -120,9 +128,9 @@ def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
-def _check(code: int, what: str) -> None:
+def _check(code: int, what: str, launches: int = 1) -> None:
     global LAUNCH_COUNT
-    LAUNCH_COUNT += 1
+    LAUNCH_COUNT += launches
     if code != 0:
         raise NativeKernelError(f"{what} failed with code {code}")
 
@@ -221,14 +229,11 @@ def gemm(
             f"gemm operands must have 16-byte aligned bases and row pitches (lda={lda}, ldb={ldb}, ldc={ldc})"
         )
     if rope is not None:
-        cos, sin, seq_len, rope_cols, hd = rope
-        assert a_kmajor and b_kmajor and not out_f32 and not accumulate and residual is None
-        assert cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
-        assert cos.shape[-1] == hd // 2 and cos.numel() >= seq_len * (hd // 2) and M % seq_len == 0
-        code = lib().kf_gemm_rope_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, lda, ldb, ldc, cos.data_ptr(),
-                                       sin.data_ptr(), int(seq_len), int(rope_cols), int(hd), sm_count(), _stream())
-        _check(code, "kf_gemm_rope_bf16")
-        return out
+        assert a_kmajor and b_kmajor and not accumulate and residual is None
+        return _gemm_rope(a, [b], out, rope)
+    if (mode in (None, 0) and GEMM_MODE == 0 and _few_rows(M, N) and a_kmajor and b_kmajor and not out_f32
+            and not accumulate and N % 8 == 0 and K % 8 == 0):
+        return gemm_rows(a, [b], residual, out)
     ldr = 0
     if residual is not None:
         assert residual.shape == (M, N) and residual.dtype == out.dtype and residual.stride(1) == 1
@@ -242,6 +247,132 @@ def gemm(
     )
     _check(code, "kf_gemm_bf16")
     return out
+
+
+# --------------------------------------------------------------------------- few rows / separate weights
+# Up to this many rows of x the weight-streaming kernel (csrc/gemm_skinny_tcgen05.cu) is considered at all.
+SKINNY_MAX_ROWS = 256
+
+
+def _few_rows(m: int, n: int) -> bool:
+    """Whether the weight-streaming kernel beats the 128 x 256 tiles for (m, n): always up to 64 rows (equal at worst, where
+    the tiles fill the machine by themselves), above while the tiles leave half of the SMs idle.  Measured, L2 flushed, us
+    (streaming / tiles): 1 x 4096, K 4096: 18 / 33; 64 x 28672, K 4096: 58 / 58; 128 x 28672: 71 / 59 (112 tiles);
+    256 x 6144: 32 / 39 (48 tiles); 256 x 4096, K 14336: 51 / 98 (32 tiles); 128 x 32000, K 768: 29 / 23 (125 tiles)."""
+    return m <= 64 or (m <= SKINNY_MAX_ROWS and 2 * (-(-n // 256)) * (-(-m // 128)) <= sm_count())
+
+
+def _ptr(t: torch.Tensor | None):
+    return t.data_ptr() if t is not None else None
+
+
+def _weights3(weights):
+    """(pointers, rows, row pitches) of up to three stacked matrices, padded with empty ones."""
+    n = 3 - len(weights)
+    return ([w.data_ptr() for w in weights] + [None] * n, [w.shape[0] for w in weights] + [0] * n,
+            [w.stride(0) for w in weights] + [0] * n)
+
+
+def gemm_rows(x2: torch.Tensor, weights, residual: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
+    """x2 (M, K) times up to three (n_i, K) weights stacked along the output (+ ``residual``) -> bf16 (M, sum n_i).  With few
+    rows the weights are read where they are; otherwise they are stacked for the tile kernels."""
+    m, k = x2.shape
+    if not _few_rows(m, sum(w.shape[0] for w in weights)) or any(w.shape[0] % 8 or w.stride(0) % 8 or w.data_ptr() % 16 for w in weights) or k % 8:
+        return gemm(x2, stack_rows(weights), residual=residual, out=out)
+    ptrs, rows, pitch = _weights3(weights)
+    n = sum(rows)
+    if out is None:
+        out = torch.empty((m, n), dtype=torch.bfloat16, device=x2.device)
+    ldr = 0
+    if residual is not None:
+        assert residual.shape == (m, n) and residual.dtype == torch.bfloat16 and residual.stride(1) == 1
+        ldr = residual.stride(0)
+        if ldr % 8 or residual.data_ptr() % 16:
+            raise NativeKernelError("gemm residual must be 16-byte aligned")
+    if x2.stride(0) % 8 or x2.data_ptr() % 16 or out.stride(0) % 8 or out.data_ptr() % 16:
+        raise NativeKernelError("gemm operands must have 16-byte aligned bases and row pitches")
+    _check(lib().kf_gemm_skinny_bf16(x2.data_ptr(), *ptrs, out.data_ptr(), residual.data_ptr() if residual is not None else None,
+                                     m, k, *rows, x2.stride(0), *pitch, out.stride(0), ldr, 0, 0, sm_count(), _stream()),
+           "kf_gemm_skinny_bf16")
+    return out
+
+
+def swiglu_rows(x2: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor) -> torch.Tensor:
+    """silu(x2 Wgᵀ) * (x2 Wuᵀ) without keeping the pre-activations."""
+    m, k = x2.shape
+    f = wg.shape[0]
+    if m <= SKINNY_MAX_ROWS and f % 8 == 0 and k % 8 == 0:
+        h = torch.empty((m, f), dtype=torch.bfloat16, device=x2.device)
+        _check(lib().kf_gemm_skinny_swiglu_bf16(x2.data_ptr(), wg.data_ptr(), wu.data_ptr(), h.data_ptr(), m, f, k,
+                                                x2.stride(0), wg.stride(0), wu.stride(0), f, 0, sm_count(), _stream()),
+               "kf_gemm_skinny_swiglu_bf16")
+        return h
+    if gemm_swiglu_pair_supported(x2, wg, f) and wg.stride() == wu.stride():
+        return gemm_swiglu_pair(x2, wg, wu, want_gu=False)[0]
+    return swiglu_fwd(gemm_rows(x2, [wg, wu]))
+
+
+def _gemm_rope(x2: torch.Tensor, weights, out: torch.Tensor, rope: tuple) -> torch.Tensor:
+    cos, sin, seq_len, rope_cols, hd = rope
+    m, k = x2.shape
+    assert out.dtype == torch.bfloat16
+    assert cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
+    assert cos.shape[-1] == hd // 2 and cos.numel() >= seq_len * (hd // 2) and m % seq_len == 0
+    ptrs, rows, pitch = _weights3(weights)
+    _check(lib().kf_gemm_rope_bf16(x2.data_ptr(), *ptrs, out.data_ptr(), m, *rows, k, x2.stride(0), pitch[0], out.stride(0),
+                                   cos.data_ptr(), sin.data_ptr(), int(seq_len), int(rope_cols), int(hd), sm_count(), _stream()),
+           "kf_gemm_rope_bf16")
+    return out
+
+
+def qkv_rope(x2: torch.Tensor, weights, cos, sin, s: int, hd: int) -> torch.Tensor:
+    """Fused q | k | v projection (M, (H + 2 Hkv) hd) of M = B * s rows with q and k rotated by position ``row % s``."""
+    wq, wk, wv = weights
+    m = x2.shape[0]
+    n = wq.shape[0] + wk.shape[0] + wv.shape[0]
+    rope_cols = wq.shape[0] + wk.shape[0]
+    if (m > SKINNY_MAX_ROWS and gemm_rope_supported(x2, wq, hd) and wk.shape[0] % hd == 0 and n % 256 == 0
+            and wq.stride() == wk.stride() == wv.stride()
+            and (rows_adjacent(weights) or (wq.shape[0] % 128 == 0 and wk.shape[0] % 128 == 0))):
+        out = torch.empty((m, n), dtype=torch.bfloat16, device=x2.device)
+        ws = [stack_rows(weights)] if rows_adjacent(weights) else weights
+        return _gemm_rope(x2, ws, out, (cos, sin, s, rope_cols, hd))
+    qkv = gemm_rows(x2, weights)
+    qkv4 = qkv.view(m // s, s, n // hd, hd)
+    rope(qkv4, cos, sin, rope_cols // hd, inverse=False, out=qkv4)
+    return qkv
+
+
+def block_decode(y: torch.Tensor, attn_ptrs, mlp_ptrs, cache_ptrs, table_ptrs, dims, scalars, foreign=None) -> None:
+    """One new token per sequence through a block (``mlp_ptrs`` None: its attention half) as one native call.  ``y`` (B, 1, D)
+    receives the output; k and v of the new position go into the cache.  The pointers and sizes are those of
+    ``kf_block_decode_bf16``, handed over as two arrays (32 separate arguments cost ctypes more than the launches' set-up).
+
+    Attention runs on the kernel split over the cache for head dim 128.  With head dim 64 it stays on what the op-by-op path
+    uses: the 128-row tile kernel for one sequence, ``foreign(q)`` (B, H hd) -> (B, H hd) between two native calls for more.
+    Those heads are the small presets' (12 of 64, one query head per KV head: 1 of the 16 MMA rows in use), where the split
+    kernel measured no faster (10.2 us, library 8.6, at 301 positions), and a small model's logits stay bit for bit the same."""
+    b, d, h, _, hd, f = dims[:6]
+    tile = hd == 64 and b == 1
+    # one buffer for every intermediate: n (D) | q (H hd) | hidden (F) | h1 (D) | attention (H hd) | rstd, scratch: rows 16-byte sized
+    scratch = torch.empty(b * (2 * d + 2 * h * hd + f) + 2 * b + 2 * h, dtype=torch.bfloat16, device=y.device)
+    base = scratch.data_ptr()
+    att = base + 2 * b * (2 * d + h * hd + f)
+    rstd = att + 2 * b * h * hd
+    yp = y.data_ptr()
+    h1 = base + 2 * b * (d + h * hd + f) if mlp_ptrs else yp
+    ints = array("q", (*attn_ptrs, *(mlp_ptrs or (0, 0, 0, 0)), *cache_ptrs, base, rstd, h1, yp, *table_ptrs, *dims, sm_count(),
+                       7, int(tile), att, rstd + 4 * b))
+    reals = array("d", scalars)
+    fn, ip, rp = lib().kf_block_decode_bf16, ints.buffer_info()[0], reals.buffer_info()[0]
+    if hd == 64 and b > 1:
+        ints[27] = 1
+        _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 2)
+        out = foreign(scratch[b * d : b * (d + h * hd)].view(b, h * hd))
+        ints[27], ints[29] = 4, out.data_ptr()
+        _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 4 if mlp_ptrs else 1)
+        return
+    _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 7 if mlp_ptrs else 4)
 
 
 # --------------------------------------------------------------------------- norm / rope / swiglu / embedding
@@ -370,12 +501,20 @@ def sumsq(x: torch.Tensor, out: torch.Tensor, accumulate: bool = False) -> torch
 def gemm_swiglu(x2: torch.Tensor, w_gate_up: torch.Tensor, want_gu: bool = True):
     """(h, gu): h = silu(x Wgᵀ) * (x Wuᵀ) computed in the epilogue of one tcgen05 GEMM over the stacked weight
     ``w_gate_up`` = [Wg ; Wu] of shape (2F, K); ``gu`` (M, 2F) holds the pre-activations when ``want_gu``."""
-    m, k = x2.shape
     f = w_gate_up.shape[0] // 2
+    return gemm_swiglu_pair(x2, w_gate_up[:f], w_gate_up[f:], want_gu)
+
+
+def gemm_swiglu_pair(x2: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, want_gu: bool = True):
+    """:func:`gemm_swiglu` over a gate and an up weight (F, K) of one row pitch, read where they are."""
+    m, k = x2.shape
+    f = wg.shape[0]
+    assert wg.shape == wu.shape and wg.stride() == wu.stride()
     h = torch.empty((m, f), dtype=torch.bfloat16, device=x2.device)
     gu = torch.empty((m, 2 * f), dtype=torch.bfloat16, device=x2.device) if want_gu else None
-    _check(lib().kf_gemm_swiglu_bf16(x2.data_ptr(), w_gate_up.data_ptr(), h.data_ptr(), gu.data_ptr() if want_gu else None,
-                                     m, f, k, x2.stride(0), w_gate_up.stride(0), f, 2 * f, sm_count(), _stream()),
+    _check(lib().kf_gemm_swiglu_bf16(x2.data_ptr(), wg.data_ptr(), wu.data_ptr(), h.data_ptr(),
+                                     gu.data_ptr() if want_gu else None, m, f, k, x2.stride(0), wg.stride(0), f, 2 * f,
+                                     sm_count(), _stream()),
            "kf_gemm_swiglu_bf16")
     return h, gu
 
@@ -425,10 +564,14 @@ def gemm_swiglu_bwd_supported(dy2: torch.Tensor, w_down: torch.Tensor, gu: torch
 
 
 def gemm_swiglu_supported(x2: torch.Tensor, w_gate_up: torch.Tensor) -> bool:
-    f = w_gate_up.shape[0] // 2
+    return gemm_swiglu_pair_supported(x2, w_gate_up, w_gate_up.shape[0] // 2)
+
+
+def gemm_swiglu_pair_supported(x2: torch.Tensor, w: torch.Tensor, f: int) -> bool:
+    """``f`` hidden units; ``w``: the gate weight (the up weight has its strides) or both stacked."""
     return (getattr(lib(), "kf_gemm_swiglu_bf16", None) is not None and not os.environ.get("KF_DISABLE_SWIGLU_EPILOGUE")
-            and f % 128 == 0 and x2.shape[0] >= 256 and x2.stride(1) == 1 and w_gate_up.stride(1) == 1
-            and x2.stride(0) % 8 == 0 and w_gate_up.stride(0) % 8 == 0 and x2.dtype == torch.bfloat16)
+            and f % 128 == 0 and x2.shape[0] >= 256 and x2.stride(1) == 1 and w.stride(1) == 1
+            and x2.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x2.dtype == torch.bfloat16)
 
 
 # --------------------------------------------------------------------------- fp8
