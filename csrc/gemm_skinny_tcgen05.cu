@@ -54,9 +54,8 @@ struct Args {
   // epilogue 2
   __nv_bfloat16 *kc, *vc;        // cache rows [batch][position][kv_dim], already offset to the first new position
   long long cache_batch;         // elements between batch entries
-  const float *cosT, *sinT;      // [S][hd / 2], row 0 = first new position
-  int S, hd;
-  int q_cols, kv_cols;
+  const float *cosT, *sinT;      // [S][64], row 0 = first new position
+  int S, kv_cols;
   int pdl;
 };
 
@@ -272,21 +271,17 @@ kf_gemm_skinny(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       store8(a.out + size_t(t) * a.ldo + row0 + n, g);
     }
   } else {
-    // heads of hd columns (64 or 128) lie inside the tile: pairs (d, d + hd / 2).  Tokens t = (batch, new position).
-    const int valid = min(WROWS, a.rows[seg] - row0);
-    const int half = a.hd >> 1, vec = half >> 3;  // 8-wide pieces of a half head
-    const int per_row = WROWS / 16;
-    for (int i = first; i < a.M * per_row; i += step) {
-      const int t = i / per_row, j = i % per_row;
-      const int n = (j / vec) * a.hd + (j % vec) * 8;  // row of the first half inside the tile
-      if (n >= valid) continue;
+    // one head of 128 columns per tile: pairs (n, n + 64).  Tokens t = (batch, new position).
+    constexpr int half = WROWS / 2, vec = half / 8;  // 8-wide pieces of a half head
+    for (int i = first; i < a.M * vec; i += step) {
+      const int t = i / vec, n = (i % vec) * 8;
       const int b = t / a.S, pos = t - b * a.S;
       float lo[8], hi[8];
       sum8(t, n, lo);
       sum8(t, n + half, hi);
       if (seg < 2) {
-        const float* cs = a.cosT + size_t(pos) * half + (j % vec) * 8;
-        const float* sn = a.sinT + size_t(pos) * half + (j % vec) * 8;
+        const float* cs = a.cosT + size_t(pos) * half + n;
+        const float* sn = a.sinT + size_t(pos) * half + n;
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           // the projection is rounded to bf16 before the rotation, like the separate kernels do
@@ -419,14 +414,15 @@ int kf_gemm_skinny_swiglu_bf16(const void* x, const void* wg, const void* wu, vo
 
 // Fused q | k | v projection of M = B * S new tokens with the rotary embedding: q (rotated) -> q_out [M][ldq], k (rotated)
 // and v -> cache rows kc / vc ([B][..][kv_cols], `cache_batch` elements between batch entries, pointing at the first new
-// position).  cosT / sinT: fp32 [S][hd / 2] of the new positions.  hd 64 or 128; q_cols and kv_cols multiples of hd.
+// position).  cosT / sinT: fp32 [S][64] of the new positions.  Head dim 128; q_cols and kv_cols multiples of it.
 int kf_gemm_skinny_qkv_bf16(const void* x, const void* wq, const void* wk, const void* wv, void* q_out, void* kc, void* vc,
-                            int M, int S, int K, int q_cols, int kv_cols, int hd, int ldx, int ldwq, int ldwk, int ldwv,
-                            int ldq, long long cache_batch, const void* cosT, const void* sinT, int pdl, int num_sms,
+                            int M, int S, int K, int q_cols, int kv_cols, int ldx, int ldwq, int ldwk, int ldwv, int ldq,
+                            long long cache_batch, const void* cosT, const void* sinT, int pdl, int num_sms,
                             void* stream) {
   using namespace kf::skinny;
+  constexpr int hd = WROWS;  // a tile of W rows is one head
   if (M < 1 || M > 256 || S < 1 || M % S || K < 8 || ((K | ldx | ldwq | ldwk | ldwv | ldq) & 7) || (cache_batch & 7) ||
-      (hd != 64 && hd != 128) || q_cols % hd || kv_cols % hd || q_cols < hd || kv_cols < hd)
+      q_cols % hd || kv_cols % hd || q_cols < hd || kv_cols < hd)
     return 5;
   const void* w[3] = {wq, wk, wv};
   const int ldw[3] = {ldwq, ldwk, ldwv}, n[3] = {q_cols, kv_cols, kv_cols};
@@ -438,7 +434,7 @@ int kf_gemm_skinny_qkv_bf16(const void* x, const void* wq, const void* wk, const
   a.cache_batch = cache_batch;
   a.cosT = (const float*)cosT;
   a.sinT = (const float*)sinT;
-  a.S = S; a.hd = hd; a.q_cols = q_cols; a.kv_cols = kv_cols;
+  a.S = S; a.kv_cols = kv_cols;
   int tiles = 0;
   for (a.n_seg = 0; a.n_seg < 3; ++a.n_seg) {
     a.tile0[a.n_seg] = tiles;

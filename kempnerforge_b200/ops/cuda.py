@@ -56,7 +56,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "kf_gemm_dgrad_stacked_bf16": [vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, i, vp],
         "kf_gemm_skinny_bf16": [vp] * 6 + [i] * 14 + [vp],
         "kf_gemm_skinny_swiglu_bf16": [vp] * 4 + [i] * 9 + [vp],
-        "kf_gemm_skinny_qkv_bf16": [vp] * 7 + [i] * 11 + [ll, vp, vp, i, i, vp],
+        "kf_gemm_skinny_qkv_bf16": [vp] * 7 + [i] * 10 + [ll, vp, vp, i, i, vp],
         "kf_rmsnorm_fwd_pdl_bf16": [vp, vp, vp, vp, i, i, f, i, vp],
         "kf_attn_decode_bf16": [vp] * 4 + [i] * 5 + [ll] * 5 + [f, i, i, i, vp],
         "kf_block_decode_bf16": [vp, vp, vp],
@@ -349,30 +349,33 @@ def block_decode(y: torch.Tensor, attn_ptrs, mlp_ptrs, cache_ptrs, table_ptrs, d
     ``kf_block_decode_bf16``, handed over as two arrays (32 separate arguments cost ctypes more than the launches' set-up).
 
     Attention runs on the kernel split over the cache for head dim 128.  With head dim 64 it stays on what the op-by-op path
-    uses: the 128-row tile kernel for one sequence, ``foreign(q)`` (B, H hd) -> (B, H hd) between two native calls for more.
+    uses: the 128-row tile kernel for one sequence, ``foreign(q)`` (rows of H hd) -> dense (B, H hd) between two native calls
+    for more; the rotation is the separate kernel's too.
     Those heads are the small presets' (12 of 64, one query head per KV head: 1 of the 16 MMA rows in use), where the split
     kernel measured no faster (10.2 us, library 8.6, at 301 positions), and a small model's logits stay bit for bit the same."""
-    b, d, h, _, hd, f = dims[:6]
+    b, d, h, hkv, hd, f = dims[:6]
     tile = hd == 64 and b == 1
-    # one buffer for every intermediate: n (D) | q (H hd) | hidden (F) | h1 (D) | attention (H hd) | rstd, scratch: rows 16-byte sized
-    scratch = torch.empty(b * (2 * d + 2 * h * hd + f) + 2 * b + 2 * h, dtype=torch.bfloat16, device=y.device)
+    qc, row = h * hd, (h + 2 * hkv) * hd
+    # one buffer for all intermediates: n (D) | q, or q | k | v | hidden (F) | h1 (D) | attention (H hd) | rstd, lse
+    scratch = torch.empty(b * (2 * d + row + qc + f) + 2 * b + 2 * h, dtype=torch.bfloat16, device=y.device)
     base = scratch.data_ptr()
-    att = base + 2 * b * (2 * d + h * hd + f)
-    rstd = att + 2 * b * h * hd
+    att = base + 2 * b * (2 * d + row + f)
+    rstd = att + 2 * b * qc
     yp = y.data_ptr()
-    h1 = base + 2 * b * (d + h * hd + f) if mlp_ptrs else yp
+    h1 = base + 2 * b * (d + row + f) if mlp_ptrs else yp
     ints = array("q", (*attn_ptrs, *(mlp_ptrs or (0, 0, 0, 0)), *cache_ptrs, base, rstd, h1, yp, *table_ptrs, *dims, sm_count(),
                        7, int(tile), att, rstd + 4 * b))
     reals = array("d", scalars)
     fn, ip, rp = lib().kf_block_decode_bf16, ints.buffer_info()[0], reals.buffer_info()[0]
+    extra = 2 if hd == 64 else 0
     if hd == 64 and b > 1:
         ints[27] = 1
-        _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 2)
-        out = foreign(scratch[b * d : b * (d + h * hd)].view(b, h * hd))
+        _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 2 + extra)
+        out = foreign(scratch[b * d : b * (d + row)].view(b, row)[:, :qc])
         ints[27], ints[29] = 4, out.data_ptr()
         _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 4 if mlp_ptrs else 1)
         return
-    _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 7 if mlp_ptrs else 4)
+    _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", (7 if mlp_ptrs else 4) + extra)
 
 
 # --------------------------------------------------------------------------- norm / rope / swiglu / embedding

@@ -117,7 +117,7 @@ def run(block, x, cos, sin, cache):
         y = torch.empty((b, 1, d), dtype=_BF16, device=x.device)
 
         def foreign(q2):
-            out = F.attention(q2.view(b, 1, h, hd), k[:, : past + 1], v[:, : past + 1], causal=False)
+            out = F.attention(q2.unflatten(1, (h, hd)).unsqueeze(1), k[:, : past + 1], v[:, : past + 1], causal=False)
             return out.reshape(b, qc)   # SDPA's output is a transposed view
 
         kc.block_decode(y, (xp, g1, pq, pk, pv, po), (g2, pg, pu, pd) if g2 else None, (kp, vp), (cp, sp),
