@@ -16,6 +16,7 @@
 // Masks, lazy rescaling and outputs are those of the single-tile kernel in attention_tcgen05.cu, which remains the
 // path for short sequences.  Replaces F.scaled_dot_product_attention (kempnerforge/model/attention.py:227-231).
 #include "attention_common.cuh"
+#include "doc_blocks.cuh"
 #include <stdlib.h>
 
 namespace kf {
@@ -35,7 +36,7 @@ struct Cfg {
   static constexpr int TILE_BYTES = BLK_N * HD * 2;
   static constexpr int BLOCK_BYTES = BLK_N * 128;
   static constexpr int N_TILES_SMEM = 2 + 2 * KV_STAGES;  // Q_A, Q_B, K ring, V ring
-  static constexpr size_t SMEM = N_TILES_SMEM * size_t(TILE_BYTES) + 1024 + 4352;
+  static constexpr size_t SMEM = N_TILES_SMEM * size_t(TILE_BYTES) + 1024 + 256 + 2048 + docblk::MASK_BYTES;
 };
 
 __device__ __forceinline__ void tile_group_sync(int tile) {
@@ -49,7 +50,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                      const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ O,
                      float* __restrict__ LSE, const int* __restrict__ doc_ids, int Sq, int Sk, int H, int group,
-                     long long ldo, float scale_log2, int* status, int n_super, int n_batch) {
+                     long long ldo, float scale_log2, int* status, int n_super, int n_batch,
+                     const int2* __restrict__ doc_range) {
   using C = Cfg<HD>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -73,6 +75,7 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
   uint8_t* bar_generic = smem_raw + (smem_base - smem_u32(smem_raw)) + C::N_TILES_SMEM * C::TILE_BYTES;
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(bar_generic + 8 * 18);
   int* doc_smem = reinterpret_cast<int*>(bar_generic + 256);  // [2 tiles][2][128] key doc ids
+  uint32_t* act = reinterpret_cast<uint32_t*>(bar_generic + 256 + 2048);  // active key tiles (one bit each)
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -89,7 +92,16 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
   // key tiles each query tile walks (tile B is absent when the sequence ends inside tile A)
   const int n_a = CAUSAL ? min(kv_all, (m0 + BLK_M + BLK_N - 1) / BLK_N) : kv_all;
   const int n_b = (m0 + BLK_M >= Sq) ? 0 : (CAUSAL ? min(kv_all, (m0 + 2 * BLK_M + BLK_N - 1) / BLK_N) : kv_all);
-  const int n_max = max(n_a, n_b);
+  int n_max = max(n_a, n_b);
+  // packed documents: key tiles whose id range meets neither query tile's are left out by every role alike.  The ids
+  // may be in any order (ranges only overlap more often then); a query's own tile is always kept.
+  const bool skip = HAS_DOC && doc_range != nullptr && docblk::fits(n_max);
+  if (HAS_DOC && skip) {
+    const int n64 = docblk::n_blocks(Sq);
+    const int2* rg = doc_range + size_t(b) * n64;
+    docblk::build_mask(act, n_max, docblk::merged(rg, n64, m0 / docblk::ROWS, 2 * BLK_M / docblk::ROWS),
+                       [&](int j) { return docblk::merged(rg, n64, j * (BLK_N / docblk::ROWS), BLK_N / docblk::ROWS); });
+  }
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -118,6 +130,9 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  // i-th key tile that is walked / its successor
+  auto first_tile = [&]() { return skip ? docblk::next(act, 0, n_max) : 0; };
+  auto next_tile = [&](int j) { return skip ? docblk::next(act, j + 1, n_max) : j + 1; };
   auto s_col = [&](int tile) { return tmem_base + uint32_t(tile * BLK_N); };
   auto o_col = [&](int tile) { return tmem_base + uint32_t(256 + tile * 128); };
 
@@ -133,8 +148,9 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
         for (int c = 0; c < C::BLOCKS; ++c)
           tma_load_2d(q_smem + tile * C::TILE_BYTES + c * C::BLOCK_BYTES, &map_q, q_full, h * HD + 64 * c,
                       b * Sq + m0 + tile * BLK_M);
-      for (int j = 0; j < n_max; ++j) {
-        const int st = j & 1, use = j >> 1;
+      int i = 0;
+      for (int j = first_tile(); j < n_max; j = next_tile(j), ++i) {
+        const int st = i & 1, use = i >> 1;
         if (use > 0 && !mbar_wait(k_empty(st), (use - 1) & 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
         mbar_expect_tx(k_full(st), C::TILE_BYTES);
 #pragma unroll
@@ -150,8 +166,9 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
     } else if (lane == 1) {
       bool ok = true;
       int issued = 0;
-      for (int j = 0; j < n_max; ++j) {
-        const int st = j & 1, use = j >> 1;
+      int i = 0;
+      for (int j = first_tile(); j < n_max; j = next_tile(j), ++i) {
+        const int st = i & 1, use = i >> 1;
         if (use > 0 && !mbar_wait(v_empty(st), (use - 1) & 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
         mbar_expect_tx(v_full(st), C::TILE_BYTES);
 #pragma unroll
@@ -169,10 +186,10 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
       constexpr uint32_t idesc_s = umma_idesc_bf16(BLK_M, BLK_N, false, false);
       constexpr uint32_t idesc_o = umma_idesc_bf16(BLK_M, HD, false, true);
       bool ok = mbar_wait(q_full, 0, status, KF_ERR_WAIT_FULL);
-      const int n_of[2] = {n_a, n_b};
-      // S_tile = Q_tile K_t^T ; the caller has made sure K_t landed
-      auto issue_s = [&](int tile, int t) {
-        const int st = t & 1;
+      const int lim[2] = {n_a, n_b};                    // key tiles below lim[tile] belong to the query tile
+      // S_tile = Q_tile K^T with the i-th walked key tile; the caller has made sure it landed
+      auto issue_s = [&](int tile, int i) {
+        const int st = i & 1;
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) {
           const uint32_t off = (kk / 4) * C::BLOCK_BYTES + (kk % 4) * 32;
@@ -181,53 +198,55 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
         }
         tc_commit(s_full(tile));
       };
-      if (ok && n_max > 0) {
+      int j = first_tile();
+      if (ok && j < n_max) {
         ok = mbar_wait(k_full(0), 0, status, KF_ERR_WAIT_FULL);
         if (ok) {
           tc_fence_after();
-          if (n_a > 0) issue_s(0, 0);
-          if (n_b > 0) issue_s(1, 0);
+          if (j < n_a) issue_s(0, 0);
+          if (j < n_b) issue_s(1, 0);
           tc_commit(k_empty(0));
         }
       }
-      for (int j = 0; j < n_max && ok; ++j) {
-        const int st = j & 1;
+      for (int i = 0; j < n_max && ok; ++i) {
+        const int st = i & 1, jn = next_tile(j);
         bool k_next_ready = false;
         for (int tile = 0; tile < 2 && ok; ++tile) {
-          if (j >= n_of[tile]) continue;
+          if (j >= lim[tile]) continue;
           // O_tile += P_tile V_j : A = P from tensor memory, B = V with the head dim contiguous (MN-major).  The
           // softmax warps hand P over in two halves: the products over the first 64 keys run while the
           // exponentials of the last 64 are still being computed.
-          if (!mbar_wait(p_half(tile), j & 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
-          if (!mbar_wait(v_full(st), (j >> 1) & 1, status, KF_ERR_WAIT_FULL)) { ok = false; break; }
+          if (!mbar_wait(p_half(tile), i & 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
+          if (!mbar_wait(v_full(st), (i >> 1) & 1, status, KF_ERR_WAIT_FULL)) { ok = false; break; }
           tc_fence_after();
 #pragma unroll
           for (int kk = 0; kk < BLK_N / 32; ++kk)
             tc_mma_f16_ts(o_col(tile), s_col(tile) + kk * 8,
                           umma_desc_sw128(v_smem + st * C::TILE_BYTES + kk * 2048, C::BLOCK_BYTES, 1024), idesc_o,
-                          (j | kk) != 0);
-          if (!mbar_wait(p_full(tile), j & 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
+                          (i | kk) != 0);
+          if (!mbar_wait(p_full(tile), i & 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
           tc_fence_after();
 #pragma unroll
           for (int kk = BLK_N / 32; kk < BLK_N / 16; ++kk)
             tc_mma_f16_ts(o_col(tile), s_col(tile) + kk * 8,
                           umma_desc_sw128(v_smem + st * C::TILE_BYTES + kk * 2048, C::BLOCK_BYTES, 1024), idesc_o, 1u);
           tc_commit(pv_done(tile));
-          if (j + 1 == n_of[tile]) tc_commit(o_final(tile));  // a phase of its own: cannot be mistaken for an earlier tile
+          if (jn >= lim[tile]) tc_commit(o_final(tile));  // a phase of its own: cannot be mistaken for an earlier tile
           // the next score tile of this query tile follows at once (its buffer's P was read by the MMAs just issued)
-          if (j + 1 < n_of[tile]) {
+          if (jn < lim[tile]) {
             if (!k_next_ready) {
-              if (!mbar_wait(k_full((j + 1) & 1), ((j + 1) >> 1) & 1, status, KF_ERR_WAIT_FULL)) { ok = false; break; }
+              if (!mbar_wait(k_full((i + 1) & 1), ((i + 1) >> 1) & 1, status, KF_ERR_WAIT_FULL)) { ok = false; break; }
               tc_fence_after();
               k_next_ready = true;
             }
-            issue_s(tile, j + 1);
+            issue_s(tile, i + 1);
           }
         }
         if (ok) {
           tc_commit(v_empty(st));                               // V_j read by both query tiles
-          if (j + 1 < n_max) tc_commit(k_empty((j + 1) & 1));   // K_{j+1} read by every S that needs it
+          if (jn < n_max) tc_commit(k_empty((i + 1) & 1));      // the next K tile read by every S that needs it
         }
+        j = jn;
       }
       if (!ok) {
         tc_commit(drain_bar);
@@ -250,18 +269,19 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
     int doc_q = 0;
     if (HAS_DOC) doc_q = row < Sq ? doc_ids[size_t(b) * Sq + row] : -1;
     bool ok = true;
-    for (int j = 0; j < n_tiles; ++j) {
+    int walked = 0;
+    for (int j = first_tile(); j < n_tiles; j = next_tile(j), ++walked) {
       const int n0 = j * BLK_N;
       const int* dk = nullptr;
       if (HAS_DOC) {
-        int* buf = doc_smem + tile * 256 + (j & 1) * BLK_N;
+        int* buf = doc_smem + tile * 256 + (walked & 1) * BLK_N;
         const int kpos = n0 + r_local;
         buf[r_local] = kpos < Sk ? doc_ids[size_t(b) * Sk + kpos] : -2;
         tile_group_sync(tile);
         dk = buf;
       }
       const bool tile_masked = HAS_DOC || (CAUSAL && n0 + BLK_N - 1 > t0) || (n0 + BLK_N > Sk);
-      if (ok && !mbar_wait(s_full(tile), j & 1, status, KF_ERR_WAIT_TMEM_FULL)) ok = false;
+      if (ok && !mbar_wait(s_full(tile), walked & 1, status, KF_ERR_WAIT_TMEM_FULL)) ok = false;
       tc_fence_after();
       uint32_t sv[BLK_N];
 #pragma unroll
@@ -291,8 +311,8 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
       const bool grow = m_new > m_run + RESCALE_THRESHOLD;
       if (__any_sync(0xffffffffu, grow)) {
         const float alpha = grow ? (m_run == NEG_INF ? 0.f : fast_exp2(m_run - m_new)) : 1.f;
-        if (j > 0) {
-          if (ok && !mbar_wait(pv_done(tile), (j - 1) & 1, status, KF_ERR_WAIT_TMEM_FULL)) ok = false;
+        if (walked > 0) {
+          if (ok && !mbar_wait(pv_done(tile), (walked - 1) & 1, status, KF_ERR_WAIT_TMEM_FULL)) ok = false;
           tc_fence_after();
 #pragma unroll 1
           for (int c = 0; c < HD / 32; ++c) {
@@ -349,7 +369,7 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full(tile));
     }
-    if (n_tiles > 0) {
+    if (walked > 0) {
       if (ok && !mbar_wait(o_final(tile), 0, status, KF_ERR_WAIT_TMEM_FULL)) ok = false;
       if (ok) {
         tc_fence_after();
@@ -388,7 +408,8 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
 
 template <int HD, bool CAUSAL, bool HAS_DOC, int POLY = 0>
 static int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, void* O, float* LSE, const int* doc,
-                  int B, int Sq, int Sk, int H, int Hkv, long long ldo, float scale, int* status, cudaStream_t stream) {
+                  int B, int Sq, int Sk, int H, int Hkv, long long ldo, float scale, int* status, cudaStream_t stream,
+                  const int2* doc_range) {
   auto kern = kf_attn_fwd2_tcgen05<HD, CAUSAL, HAS_DOC, POLY>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -399,9 +420,37 @@ static int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMa
   const int n_super = (Sq + 2 * BLK_M - 1) / (2 * BLK_M);
   dim3 grid((unsigned)(n_super * H * B));
   kern<<<grid, THREADS, Cfg<HD>::SMEM, stream>>>(mq, mk, mv, reinterpret_cast<__nv_bfloat16*>(O), LSE, doc, Sq, Sk, H,
-                                                 H / Hkv, ldo, scale * 1.4426950408889634f, status, n_super, B);
+                                                 H / Hkv, ldo, scale * 1.4426950408889634f, status, n_super, B, doc_range);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
+}
+
+// Smallest and largest id of every 64 positions (one warp each) and the ids as int32, in one pass over them.  With them the
+// attention kernels leave out tiles without a visible pair: 3000 packed tokens in 7 documents, 40 heads of 128: forward
+// 175 -> 92 us, backward 419 -> 196 us.
+template <typename T>
+__global__ void kf_doc_blocks_kernel(const T* __restrict__ ids, int* __restrict__ out, int2* __restrict__ range, int S,
+                                     int n64, int total) {
+  const int blk = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (blk >= total) return;
+  const int b = blk / n64, s0 = (blk % n64) * docblk::ROWS;
+  int lo = 0x7fffffff, hi = -0x7fffffff - 1;
+#pragma unroll
+  for (int i = 0; i < docblk::ROWS / 32; ++i) {
+    const int s = s0 + i * 32 + lane;
+    if (s < S) {
+      const int v = int(ids[size_t(b) * S + s]);
+      out[size_t(b) * S + s] = v;
+      lo = min(lo, v);
+      hi = max(hi, v);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if (lane == 0) range[blk] = make_int2(lo, hi);
 }
 
 }  // namespace attn2
@@ -411,10 +460,27 @@ extern "C" void* kf_status_device_ptr();
 
 extern "C" {
 
-// Same contract as kf_attn_fwd_bf16 (attention_tcgen05.cu); two query tiles per CTA.
-int kf_attn_fwd2_bf16(const void* q, const void* k, const void* v, void* o, void* lse, const void* doc, int B, int Sq,
-                      int Sk, int H, int Hkv, int hd, long long ldq, long long ldk, long long ldv, long long ldo,
-                      float scale, int causal, void* stream) {
+// ids [B][S] (int64, or int32 with wide == 0) -> out int32 [B][S] and range int32 [B][ceil(S / 64)][2].
+int kf_doc_blocks(const void* ids, int wide, void* out, void* range, int B, int S, void* stream) {
+  using namespace kf;
+  if (B < 1 || S < 1) return 1;
+  const int n64 = docblk::n_blocks(S), total = B * n64;
+  const int blocks = (total + 7) / 8;
+  if (wide)
+    attn2::kf_doc_blocks_kernel<long long><<<blocks, 256, 0, (cudaStream_t)stream>>>((const long long*)ids, (int*)out,
+                                                                                    (int2*)range, S, n64, total);
+  else
+    attn2::kf_doc_blocks_kernel<int><<<blocks, 256, 0, (cudaStream_t)stream>>>((const int*)ids, (int*)out, (int2*)range, S,
+                                                                              n64, total);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 400 + (int)e;
+}
+
+// Same contract as kf_attn_fwd_bf16 (attention_tcgen05.cu); two query tiles per CTA.  doc_range (optional): the id ranges
+// kf_doc_blocks wrote for `doc`; key tiles without a visible pair are skipped with it.
+int kf_attn_fwd2_bf16(const void* q, const void* k, const void* v, void* o, void* lse, const void* doc,
+                      const void* doc_range, int B, int Sq, int Sk, int H, int Hkv, int hd, long long ldq, long long ldk,
+                      long long ldv, long long ldo, float scale, int causal, void* stream) {
   using namespace kf;
   using namespace kf::attn2;
   if ((hd != 64 && hd != 128) || Hkv <= 0 || H % Hkv != 0) return 3;
@@ -431,8 +497,9 @@ int kf_attn_fwd2_bf16(const void* q, const void* k, const void* v, void* o, void
   cudaStream_t st = (cudaStream_t)stream;
   float* L = reinterpret_cast<float*>(lse);
   const int* D = reinterpret_cast<const int*>(doc);
-#define KF_ATTN2_LAUNCH(HD_, C_, D_) return launch<HD_, C_, D_>(mq, mk, mv, o, L, D, B, Sq, Sk, H, Hkv, ldo, scale, status, st)
-#define KF_ATTN2_POLY(C_, P_) return launch<128, C_, false, P_>(mq, mk, mv, o, L, D, B, Sq, Sk, H, Hkv, ldo, scale, status, st)
+  const int2* DR = reinterpret_cast<const int2*>(doc_range);
+#define KF_ATTN2_LAUNCH(HD_, C_, D_) return launch<HD_, C_, D_>(mq, mk, mv, o, L, D, B, Sq, Sk, H, Hkv, ldo, scale, status, st, DR)
+#define KF_ATTN2_POLY(C_, P_) return launch<128, C_, false, P_>(mq, mk, mv, o, L, D, B, Sq, Sk, H, Hkv, ldo, scale, status, st, DR)
   if (hd == 128 && !doc) {
     // share of the exponentials on the FMA pipe (of 16): KF_ATTN_EXP_POLY = 0 (default), 4, 6 or 8.  On the 8B
     // shape the variants measured 0.307 / 0.313 / 0.313 / 0.320 ms: the two-tile kernel is paced by the per-tile

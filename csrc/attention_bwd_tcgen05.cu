@@ -26,6 +26,7 @@
 // Replaces the backward of F.scaled_dot_product_attention (kempnerforge/model/attention.py:227-231) for the
 // causal / document-masked training path, without expanding grouped KV heads.
 #include "common.cuh"
+#include "doc_blocks.cuh"
 
 namespace kf {
 namespace attnb {
@@ -97,7 +98,7 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     const __grid_constant__ CUtensorMap map_dq, int dq_tma, const float* __restrict__ LSE, const float* __restrict__ Dsum, const int* __restrict__ doc_ids,
                     float* __restrict__ dQacc, __nv_bfloat16* __restrict__ dK, __nv_bfloat16* __restrict__ dV, int Sq,
                     int Sk, int H, int group, long long lddk, long long lddv, float scale, int* status,
-                    const float* __restrict__ cosT, const float* __restrict__ sinT) {
+                    const float* __restrict__ cosT, const float* __restrict__ sinT, const int2* __restrict__ doc_range) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -120,6 +121,7 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(bar_gen + 128);
   float* stat_smem = reinterpret_cast<float*>(bar_gen + 256);       // [2][lse2 | D][64]
   int* docq_smem = reinterpret_cast<int*>(bar_gen + 256 + 1024);    // [2][64]
+  uint32_t* act = reinterpret_cast<uint32_t*>(bar_gen + 256 + 1024 + 512);  // active query tiles (one bit each)
   const uint32_t dq_stage = bar_base + AUX_BYTES;                   // only allocated when dq_tma
 
   const int warp = threadIdx.x >> 5;
@@ -133,8 +135,15 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   const int k0 = kt * BLK_K;
   const int n_q_tiles = (Sq + BLK_Q - 1) / BLK_Q;
   const int i_start = CAUSAL ? min(n_q_tiles, k0 / BLK_Q) : 0;
-  const int n_i = n_q_tiles - i_start;
-  const int n_iter = n_i * group;
+  // packed documents: query tiles whose id range misses the key tile's are left out by every role alike
+  const bool skip = HAS_DOC && doc_range != nullptr && docblk::fits(n_q_tiles);
+  if (HAS_DOC && skip) {
+    static_assert(BLK_Q == docblk::ROWS, "one id range per query tile");
+    const int n64 = docblk::n_blocks(Sk);
+    const int2* rg = doc_range + size_t(b) * n64;
+    docblk::build_mask(act, n_q_tiles, docblk::merged(rg, n64, k0 / docblk::ROWS, BLK_K / docblk::ROWS),
+                       [&](int j) { return j >= i_start ? rg[j] : make_int2(1, 0); });
+  }
   const float scale_log2 = scale * 1.4426950408889634f;
 
   if (threadIdx.x == 0) {
@@ -166,6 +175,21 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  const int n_i = skip ? docblk::count(act, n_q_tiles) : n_q_tiles - i_start;
+  const int n_iter = n_i * group;
+  // iteration -> (query head, first query): every role walks the active query tiles of each head in order
+  struct Walk {
+    int i, head;
+  };
+  auto walk_begin = [&]() { return Walk{skip ? docblk::next(act, 0, n_q_tiles) : i_start, hk * group}; };
+  auto walk_next = [&](Walk w) {
+    w.i = skip ? docblk::next(act, w.i + 1, n_q_tiles) : w.i + 1;
+    if (w.i >= n_q_tiles) {
+      w.i = skip ? docblk::next(act, 0, n_q_tiles) : i_start;
+      ++w.head;
+    }
+    return w;
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -178,12 +202,13 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         tma_load_2d(k_smem + c * KV_BLOCK_BYTES, &map_k, kv_full, hk * HD + 64 * c, b * Sk + k0);
         tma_load_2d(v_smem + c * KV_BLOCK_BYTES, &map_v, kv_full, hk * HD + 64 * c, b * Sk + k0);
       }
-      for (int it = 0; it < n_iter; ++it) {
+      Walk wk = walk_begin();
+      for (int it = 0; it < n_iter; ++it, wk = walk_next(wk)) {
         const int st = it % STAGES;
         const int use = it / STAGES;
         if (use > 0 && !mbar_wait(stage_free(st), (use - 1) & 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
-        const int hq = hk * group + it / n_i;
-        const int q0 = (i_start + it % n_i) * BLK_Q;
+        const int hq = wk.head;
+        const int q0 = wk.i * BLK_Q;
         mbar_expect_tx(qdo_full(st), 2 * Q_TILE_BYTES);
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
@@ -284,18 +309,18 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     bool ok = true;
     // statistics of the 64 queries of iteration `t` (lse in log2 units for threads 0..63, D for 64..127), fetched one
     // iteration ahead so that the global-memory latency hides under the arithmetic of the current tile
-    auto fetch_stat = [&](int t) -> float {
+    auto fetch_stat = [&](int t, const Walk& w) -> float {
       if (t128 >= 128 || t >= n_iter) return 0.f;
-      const int hq_t = hk * group + t / n_i;
-      const int qq = (i_start + t % n_i) * BLK_Q + (t128 & 63);
-      const size_t idx = (size_t(b) * H + hq_t) * Sq + qq;
+      const int qq = w.i * BLK_Q + (t128 & 63);
+      const size_t idx = (size_t(b) * H + w.head) * Sq + qq;
       if (t128 < 64) return qq < Sq ? LSE[idx] * 1.4426950408889634f : INFINITY;  // +inf -> P = 0 for padding rows
       return qq < Sq ? Dsum[idx] : 0.f;
     };
-    float stat_next = fetch_stat(0);
+    Walk ahead = walk_begin();
+    float stat_next = fetch_stat(0, ahead);
     for (int it = 0; it < n_iter; ++it) {
-      const int hq = hk * group + it / n_i;
-      const int q0 = (i_start + it % n_i) * BLK_Q;
+      const int q0 = ahead.i * BLK_Q;
+      ahead = walk_next(ahead);
       float* stat = stat_smem + (it & 1) * 128;
       int* dq_doc = docq_smem + (it & 1) * 64;
       if (t128 < 128) {
@@ -306,7 +331,7 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
       }
       group_sync(1, 256);
-      stat_next = fetch_stat(it + 1);
+      stat_next = fetch_stat(it + 1, ahead);
       if (ok && !mbar_wait(sdp_full, it & 1, status, KF_ERR_WAIT_TMEM_FULL)) ok = false;
       tc_fence_after();
       const uint32_t t_s = t_lane + ST_COL + (it & 1) * BLK_Q;
@@ -442,9 +467,10 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const uint32_t t_lane = tmem_base + (uint32_t(quarter * 32) << 16);
     const bool elected = threadIdx.x == 192;  // issues, commits and waits for the bulk reductions
     bool ok = true;
-    for (int it = 0; it < n_iter; ++it) {
-      const int hq = hk * group + it / n_i;
-      const int q0 = (i_start + it % n_i) * BLK_Q;
+    Walk wk = walk_begin();
+    for (int it = 0; it < n_iter; ++it, wk = walk_next(wk)) {
+      const int hq = wk.head;
+      const int q0 = wk.i * BLK_Q;
       if (ok && !mbar_wait(mma_done, it & 1, status, KF_ERR_WAIT_TMEM_FULL)) ok = false;
       tc_fence_after();
       uint32_t v[BLK_Q];
@@ -594,12 +620,13 @@ int kf_attn_bwd_dq_mode(int mode) {
 // slices of one fused gradient buffer).  doc: optional int32 [B][S].  Requires Sq == Sk when causal or doc.
 // kf_attn_bwd_rope_bf16: the same, and dq / dk additionally pass through the inverse rotary embedding (cosT / sinT:
 // fp32 [Sq][64], position = index inside the sequence), i.e. they are gradients with respect to the un-rotated
-// projections when q / k were rotated after the projection.  Null tables = no rotation.
+// projections when q / k were rotated after the projection.  Null tables = no rotation.  doc_range (optional): the id
+// ranges kf_doc_blocks wrote for `doc`; query tiles without a visible pair are skipped with it.
 int kf_attn_bwd_rope_bf16(const void* q, const void* k, const void* v, const void* o, const void* d_o, const void* lse,
                           void* dsum, void* dq_acc, void* dq, void* dk, void* dv, const void* doc, int B, int Sq, int Sk,
                           int H, int Hkv, int hd, long long ldq, long long ldk, long long ldv, long long ldo,
                           long long lddo, long long lddq, long long lddk, long long lddv, float scale, int causal,
-                          const void* cosT, const void* sinT, void* stream) {
+                          const void* cosT, const void* sinT, const void* doc_range, void* stream) {
   using namespace kf;
   using namespace kf::attnb;
   if (hd != HD || Hkv <= 0 || H % Hkv != 0) return 3;
@@ -647,7 +674,8 @@ int kf_attn_bwd_rope_bf16(const void* q, const void* k, const void* v, const voi
                                       reinterpret_cast<float*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dk),      \
                                       reinterpret_cast<__nv_bfloat16*>(dv), Sq, Sk, H, H / Hkv, lddk, lddv, scale, \
                                       status, reinterpret_cast<const float*>(cosT),                                \
-                                      reinterpret_cast<const float*>(sinT));                                       \
+                                      reinterpret_cast<const float*>(sinT),                                        \
+                                      reinterpret_cast<const int2*>(doc_range));                                   \
   }
   if (doc) {
     if (causal) KF_BWD_LAUNCH(true, true) else KF_BWD_LAUNCH(false, true)
@@ -676,7 +704,7 @@ int kf_attn_bwd_bf16(const void* q, const void* k, const void* v, const void* o,
                      long long lddo, long long lddq, long long lddk, long long lddv, float scale, int causal,
                      void* stream) {
   return kf_attn_bwd_rope_bf16(q, k, v, o, d_o, lse, dsum, dq_acc, dq, dk, dv, doc, B, Sq, Sk, H, Hkv, hd, ldq, ldk, ldv,
-                               ldo, lddo, lddq, lddk, lddv, scale, causal, nullptr, nullptr, stream);
+                               ldo, lddo, lddq, lddk, lddv, scale, causal, nullptr, nullptr, nullptr, stream);
 }
 
 }  // extern "C"

@@ -99,10 +99,11 @@ def _declare(L: ctypes.CDLL) -> None:
         "kf_ag_gemm_bf16": [vp, vp, vp, vp, vp, i, i, i, i, ll, ll, ll, i, i, i, i, i, vp],
         "kf_gemm_rs_bf16": [vp, vp, vp, vp, vp, vp, i, i, i, i, ll, ll, i, i, i, i, i, vp],
         "kf_attn_bwd_bf16": [vp] * 12 + [i] * 6 + [ll] * 8 + [f, i, vp],
-        "kf_attn_bwd_rope_bf16": [vp] * 12 + [i] * 6 + [ll] * 8 + [f, i, vp, vp, vp],
+        "kf_attn_bwd_rope_bf16": [vp] * 12 + [i] * 6 + [ll] * 8 + [f, i, vp, vp, vp, vp],
+        "kf_doc_blocks": [vp, i, vp, vp, i, i, vp],
         "kf_attn_bwd_dq_mode": [i],
         "kf_grouped_pair_mode": [i],
-        "kf_attn_fwd2_bf16": [vp, vp, vp, vp, vp, vp, i, i, i, i, i, i, ll, ll, ll, ll, f, i, vp],
+        "kf_attn_fwd2_bf16": [vp] * 7 + [i] * 6 + [ll] * 4 + [f, i, vp],
         "kf_attn_fwd_bf16": [vp, vp, vp, vp, vp, vp, i, i, i, i, i, i, ll, ll, ll, ll, f, i, vp],
         "kf_symm_rs_norm_bf16": [vp, vp, i, i, ll, ll, vp, vp, i, i, vp],
         "kf_symm_adamw_bcast_bf16": [vp, vp, i, i, vp, vp, vp, ll, ll, ll, f, f, f, f, f, f, f, vp, vp, i, vp],
@@ -646,23 +647,37 @@ def attn_supported(q, k, v, causal: bool, needs_grad: bool = False) -> bool:
     return _attn_rows_ok(q) and _attn_rows_ok(k) and _attn_rows_ok(v)
 
 
+def doc_blocks(doc_ids: torch.Tensor):
+    """(int32 ids (B, S), int32 (B, ceil(S / 64), 2) smallest and largest id of every 64 positions): what the attention
+    kernels read of a document mask.  Pass the pair in place of the ids to reuse it for the backward."""
+    ids = doc_ids if doc_ids.dtype in (torch.int32, torch.int64) else doc_ids.to(torch.int32)
+    ids = ids.contiguous()
+    b, s = ids.shape
+    out = torch.empty((b, s), dtype=torch.int32, device=ids.device)
+    rng = torch.empty((b, (s + 63) // 64, 2), dtype=torch.int32, device=ids.device)
+    _check(lib().kf_doc_blocks(ids.data_ptr(), int(ids.dtype == torch.int64), out.data_ptr(), rng.data_ptr(), b, s, _stream()),
+           "kf_doc_blocks")
+    return out, rng
+
+
 def attn_fwd(q, k, v, causal: bool, doc_ids, scale: float):
-    """q (B, Sq, H, hd), k / v (B, Sk, Hkv, hd) -> out (B, Sq, H, hd) bf16 and lse (B, H, Sq) fp32."""
+    """q (B, Sq, H, hd), k / v (B, Sk, Hkv, hd) -> out (B, Sq, H, hd) bf16 and lse (B, H, Sq) fp32.  ``doc_ids``: (B, S)
+    ids, or what :func:`doc_blocks` made of them."""
     b, sq, h, hd = q.shape
     sk, hkv = k.shape[1], k.shape[2]
     out = torch.empty((b, sq, h, hd), dtype=q.dtype, device=q.device)
     lse = torch.empty((b, h, sq), dtype=torch.float32, device=q.device)
-    doc = None
+    doc = rng = None
     if doc_ids is not None:
-        doc = doc_ids.to(torch.int32).contiguous()
+        doc, rng = doc_ids if isinstance(doc_ids, tuple) else doc_blocks(doc_ids)
     # two query tiles per CTA (interleaved softmax) once there are at least two tiles; KF_ATTN_FWD=1 forces the
     # single-tile kernel
     L = lib()
     two = sq > 128 and getattr(L, "kf_attn_fwd2_bf16", None) is not None and os.environ.get("KF_ATTN_FWD", "2") != "1"
     fn = L.kf_attn_fwd2_bf16 if two else L.kf_attn_fwd_bf16
+    mask = (_ptr(doc), _ptr(rng)) if two else (_ptr(doc),)
     _check(
-        fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
-                               doc.data_ptr() if doc is not None else None, b, sq, sk, h, hkv, hd, q.stride(1),
+        fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), *mask, b, sq, sk, h, hkv, hd, q.stride(1),
            k.stride(1), v.stride(1), h * hd, float(scale), int(causal), _stream()),
         "kf_attn_fwd2_bf16" if two else "kf_attn_fwd_bf16",
     )
@@ -937,7 +952,9 @@ def attn_bwd(dout, q, k, v, out, lse, causal: bool, doc_ids, scale: float, dq=No
         assert _attn_rows_ok(t), "attention gradients need evenly pitched rows with adjacent heads"
     dsum = torch.empty((b, h, sq), dtype=torch.float32, device=q.device)
     dq_acc = torch.empty((b, sq, h, hd), dtype=torch.float32, device=q.device)
-    doc = doc_ids.to(torch.int32).contiguous() if doc_ids is not None else None
+    doc = rng = None
+    if doc_ids is not None:
+        doc, rng = doc_ids if isinstance(doc_ids, tuple) else doc_blocks(doc_ids)
     cos = sin = None
     if rope is not None:
         cos, sin = rope
@@ -950,7 +967,7 @@ def attn_bwd(dout, q, k, v, out, lse, causal: bool, doc_ids, scale: float, dq=No
                                     q.stride(1), k.stride(1), v.stride(1), out.stride(1), dout.stride(1), dq.stride(1),
                                     dk.stride(1), dv.stride(1), float(scale), int(causal),
                                     cos.data_ptr() if cos is not None else None,
-                                    sin.data_ptr() if sin is not None else None, _stream()),
+                                    sin.data_ptr() if sin is not None else None, _ptr(rng), _stream()),
         "kf_attn_bwd_rope_bf16",
     )
     return dq, dk, dv

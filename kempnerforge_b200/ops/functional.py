@@ -290,18 +290,17 @@ class _FlashAttnFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, causal, doc_ids, scale):
         cu = _cuda()
-        out, lse = cu.attn_fwd(q, k, v, causal, doc_ids, scale)
-        ctx.save_for_backward(q, k, v, out, lse, doc_ids if doc_ids is not None else torch.empty(0))
-        ctx.causal, ctx.scale, ctx.has_doc = causal, scale, doc_ids is not None
+        mask = cu.doc_blocks(doc_ids) if doc_ids is not None else None
+        out, lse = cu.attn_fwd(q, k, v, causal, mask, scale)
+        ctx.save_for_backward(q, k, v, out, lse, *(mask or ()))
+        ctx.causal, ctx.scale = causal, scale
         return out
 
     @staticmethod
     def backward(ctx, dout):
         cu = _cuda()
-        q, k, v, out, lse, doc = ctx.saved_tensors
-        dq, dk, dv = cu.attn_bwd(
-            dout, q, k, v, out, lse, ctx.causal, doc if ctx.has_doc else None, ctx.scale
-        )
+        q, k, v, out, lse, *mask = ctx.saved_tensors
+        dq, dk, dv = cu.attn_bwd(dout, q, k, v, out, lse, ctx.causal, tuple(mask) or None, ctx.scale)
         return dq, dk, dv, None, None, None
 
 
