@@ -581,7 +581,7 @@ def gemm_swiglu_pair_supported(x2: torch.Tensor, w: torch.Tensor, f: int) -> boo
 # --------------------------------------------------------------------------- fp8
 def fp8_scale(x2: torch.Tensor, e5m2: bool = False) -> torch.Tensor:
     """Device scalar fp8_max / absmax(x) (fp32, shape (1,))."""
-    scratch = torch.empty(2, dtype=torch.float32, device=x2.device)
+    scratch = torch.empty(1 + 1024, dtype=torch.float32, device=x2.device)   # the scale, then partial maxima
     if not x2.is_contiguous():
         x2 = x2.contiguous()
     _check(lib().kf_fp8_scale_bf16(x2.data_ptr(), x2.numel(), int(e5m2), scratch[1:].data_ptr(), scratch.data_ptr(),
