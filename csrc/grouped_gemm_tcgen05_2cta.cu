@@ -16,6 +16,13 @@
 //
 // EPI == 2: SwiGLU backward in the epilogue of the down projection's input-gradient product (see the launcher).
 //
+// EPI == 3: C = A_1 B_e + A_2 B2_e with A = [A_1 | A_2] side by side (the input gradient of the gate and up projections as
+// one product over K = 2 F): no second pass over C, and the sum is rounded once.
+//
+// NE > 1: every expert's weight has a tensor map of its own (up to NE of them, kernel parameters), so the weights of
+// separate Linear modules are read where they are; NE == 1: one packed (E, .., ..) tensor.  For 8 experts of 2048 x 7168
+// the copies this saves move 1.4 GB per forward pass.
+//
 // Synchronisation as in gemm_tcgen05_2cta.cu (all waits bounded); TMA loads carry no cluster multicast.
 // Replaces the padded torch._grouped_mm calls of the reference (kempnerforge/model/moe.py:20-145).
 #include "common.cuh"
@@ -36,10 +43,16 @@ constexpr size_t SMEM = size_t(STAGES) * STAGE_BYTES + 1024 + 256 + (MAX_EXPERTS
 
 using Tile = tilemath::GroupedTile;
 
-template <bool B_MN, int EPI>
+template <int NE>
+struct Maps {
+  CUtensorMap m[NE];
+};
+constexpr int MAX_SEPARATE = 32;  // experts with a tensor map of their own (two operands: 8 KB of kernel parameters)
+
+template <bool B_MN, int EPI, int NE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
-kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                             const __grid_constant__ CUtensorMap map_b2, __nv_bfloat16* __restrict__ C,
+kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ Maps<NE> maps_b,
+                             const __grid_constant__ Maps<(EPI & 1) ? NE : 1> maps_b2, __nv_bfloat16* __restrict__ C,
                              __nv_bfloat16* __restrict__ GU, const int* __restrict__ offsets, int E, int N, int K,
                              long long ldc, long long ldgu, int accumulate, int* status) {
   extern __shared__ uint8_t smem_raw[];
@@ -77,8 +90,10 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
     mbar_init(drain_bar, 1);
     mbar_fence_init();
     tma_prefetch_desc(&map_a);
-    tma_prefetch_desc(&map_b);
-    if (SWIGLU) tma_prefetch_desc(&map_b2);
+    if (NE == 1) {
+      tma_prefetch_desc(&maps_b.m[0]);
+      if (EPI & 1) tma_prefetch_desc(&maps_b2.m[0]);
+    }
     tilemath::grouped_tile_starts(offsets, E, TILE_M, tile_start);  // both CTAs of a pair compute the same table
   }
   if (warp == 1) {
@@ -98,11 +113,13 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
       int it = 0;
       bool ok = true;
       // the leader fetches the gate weights (or the first 128 columns), the peer the up weights (or the last 128)
-      const CUtensorMap* my_b = (SWIGLU && !leader) ? &map_b2 : &map_b;
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
         const Tile tl = tilemath::grouped_decode(t, n_blocks, tile_start, offsets, E, TILE_M);
         const int m0 = tl.row0 + int(rank) * CTA_M;
         const int n0 = SWIGLU ? tl.nb * TN : tl.nb * TN + int(rank) * HALF_N;
+        const int me = NE > 1 ? tl.e : 0;              // tensor map and first row of the expert's weight inside it
+        const int e_n = NE > 1 ? 0 : tl.e * N, e_k = NE > 1 ? 0 : tl.e * (EPI == 3 ? K / 2 : K);
+        const CUtensorMap* my_b = (SWIGLU && !leader) ? &maps_b2.m[me] : &maps_b.m[me];
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
@@ -113,12 +130,17 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
           if (leader) mbar_expect_tx(full_bar(s), 2 * STAGE_BYTES);
           const int k0 = kb * BK;
           tma_load_2d_pair(a_dst, &map_a, lead_full, k0, m0);
+          int kw = k0;                                 // reduction index inside the weight
+          if (EPI == 3 && k0 >= K / 2) {
+            my_b = &maps_b2.m[me];
+            kw = k0 - K / 2;
+          }
           if (!B_MN) {
-            tma_load_2d_pair(b_dst, my_b, lead_full, k0, tl.e * N + n0);
+            tma_load_2d_pair(b_dst, my_b, lead_full, kw, e_n + n0);
           } else {
 #pragma unroll
             for (int c = 0; c < HALF_N / 64; ++c)
-              tma_load_2d_pair(b_dst + c * (64 * BK * 2), my_b, lead_full, n0 + 64 * c, tl.e * K + k0);
+              tma_load_2d_pair(b_dst + c * (64 * BK * 2), my_b, lead_full, n0 + 64 * c, e_k + kw);
           }
         }
       }
@@ -235,10 +257,11 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
   }
 }
 
-template <bool B_MN, int EPI>
-static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mb2, void* C, void* GU, const void* offsets,
-                  int E, int N, int K, long long ldc, long long ldgu, int accumulate, int pairs, cudaStream_t st, int* status) {
-  auto kern = kf_grouped_gemm_tcgen05_2cta<B_MN, EPI>;
+template <bool B_MN, int EPI, int NE>
+static int launch(const CUtensorMap& ma, const Maps<NE>& mb, const Maps<(EPI & 1) ? NE : 1>& mb2, void* C, void* GU,
+                  const void* offsets, int E, int N, int K, long long ldc, long long ldgu, int accumulate, int pairs,
+                  cudaStream_t st, int* status) {
+  auto kern = kf_grouped_gemm_tcgen05_2cta<B_MN, EPI, NE>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
@@ -251,40 +274,52 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMa
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
+// Weight operand: the packed tensor (NE == 1, *w) or one pointer per expert.  Each expert's matrix is [N][K] (K
+// contiguous, boxes of 128 rows) or, b_mn, [K][N] (N contiguous, 64 x 64 boxes).
+template <int NE>
+static int make_weight_maps(Maps<NE>& m, const void* const* w, int E, int N, int K, int b_mn) {
+  for (int e = 0; e < (NE > 1 ? E : 1); ++e) {
+    const uint64_t n = NE > 1 ? 1 : E;
+    const int rc = b_mn ? make_map_2d_bf16(&m.m[e], w[e], n * K, N, N, 64, BK) : make_map_2d_bf16(&m.m[e], w[e], n * N, K, K, BK, HALF_N);
+    if (rc) return rc;
+  }
+  return 0;
+}
+
+static int pair_count(int rows, int E, int n_blocks, int num_sms) {
+  const int upper = ((rows + TILE_M - 1) / TILE_M + E) * n_blocks;  // at most one partial tile per expert
+  return upper < num_sms / 2 ? upper : num_sms / 2;
+}
+
+template <int EPI, int NE>
+static int run(const void* A, const void* const* W, const void* const* W2, void* C, void* GU, const void* offsets, int rows,
+               int E, int N, int K, int KW, long long lda, long long ldc, long long ldgu, int b_mn, int accumulate, int num_sms,
+               cudaStream_t st, int* status) {
+  CUtensorMap ma;
+  Maps<NE> mb;
+  Maps<(EPI & 1) ? NE : 1> mb2;
+  int rc = make_map_2d_bf16(&ma, A, rows, K, lda, BK, CTA_M);
+  if (rc) return 100 + rc;
+  rc = make_weight_maps<NE>(mb, W, E, N, KW, b_mn);
+  if (!rc && (EPI & 1)) rc = make_weight_maps<(EPI & 1) ? NE : 1>(mb2, W2, E, N, KW, b_mn);
+  if (rc) return 200 + rc;
+  if (!(EPI & 1)) mb2.m[0] = mb.m[0];
+  const int tn = EPI == 1 ? HALF_N : TILE_N;
+  const int pairs = pair_count(rows, E, (N + tn - 1) / tn, num_sms);
+  return b_mn ? launch<true, EPI, NE>(ma, mb, mb2, C, GU, offsets, E, N, K, ldc, ldgu, accumulate, pairs, st, status)
+              : launch<false, EPI, NE>(ma, mb, mb2, C, GU, offsets, E, N, K, ldc, ldgu, accumulate, pairs, st, status);
+}
+
 // Contracts of kf_grouped_gemm_acc_bf16 / kf_grouped_swiglu_bf16 (grouped_gemm_tcgen05.cu), which dispatch here.
 int launch_grouped_gemm_2cta(const void* A, const void* B, void* C, const void* offsets, int rows, int E, int N, int K,
                              long long lda, long long ldc, int b_mn, int accumulate, int num_sms, cudaStream_t st, int* status) {
-  CUtensorMap ma, mb;
-  int rc = make_map_2d_bf16(&ma, A, rows, K, lda, BK, CTA_M);
-  if (rc) return 100 + rc;
-  rc = b_mn ? make_map_2d_bf16(&mb, B, uint64_t(E) * K, N, N, 64, BK) : make_map_2d_bf16(&mb, B, uint64_t(E) * N, K, K, BK, HALF_N);
-  if (rc) return 200 + rc;
-  const int upper = ((rows + TILE_M - 1) / TILE_M + E) * ((N + TILE_N - 1) / TILE_N);  // at most one partial tile per expert
-  int pairs = num_sms / 2;
-  if (upper < pairs) pairs = upper;
-  return b_mn ? launch<true, 0>(ma, mb, mb, C, nullptr, offsets, E, N, K, ldc, 0, accumulate, pairs, st, status)
-              : launch<false, 0>(ma, mb, mb, C, nullptr, offsets, E, N, K, ldc, 0, accumulate, pairs, st, status);
+  return run<0, 1>(A, &B, nullptr, C, nullptr, offsets, rows, E, N, K, K, lda, ldc, 0, b_mn, accumulate, num_sms, st, status);
 }
 
 int launch_grouped_swiglu_2cta(const void* A, const void* Wg, const void* Wu, void* H, void* GU, const void* offsets, int rows,
                                int E, int F, int K, long long lda, long long ldh, long long ldgu, int b_mn, int num_sms,
                                cudaStream_t st, int* status) {
-  CUtensorMap ma, mg, mu;
-  int rc = make_map_2d_bf16(&ma, A, rows, K, lda, BK, CTA_M);
-  if (rc) return 100 + rc;
-  if (b_mn) {
-    rc = make_map_2d_bf16(&mg, Wg, uint64_t(E) * K, F, F, 64, BK);
-    if (!rc) rc = make_map_2d_bf16(&mu, Wu, uint64_t(E) * K, F, F, 64, BK);
-  } else {
-    rc = make_map_2d_bf16(&mg, Wg, uint64_t(E) * F, K, K, BK, HALF_N);
-    if (!rc) rc = make_map_2d_bf16(&mu, Wu, uint64_t(E) * F, K, K, BK, HALF_N);
-  }
-  if (rc) return 200 + rc;
-  const int upper = ((rows + TILE_M - 1) / TILE_M + E) * ((F + HALF_N - 1) / HALF_N);
-  int pairs = num_sms / 2;
-  if (upper < pairs) pairs = upper;
-  return b_mn ? launch<true, 1>(ma, mg, mu, H, GU, offsets, E, F, K, ldh, ldgu, 0, pairs, st, status)
-              : launch<false, 1>(ma, mg, mu, H, GU, offsets, E, F, K, ldh, ldgu, 0, pairs, st, status);
+  return run<1, 1>(A, &Wg, &Wu, H, GU, offsets, rows, E, F, K, K, lda, ldh, ldgu, b_mn, 0, num_sms, st, status);
 }
 
 // d[gate | up] (rows x 2F, may alias GU) from dy (rows x K) and the down weights: W [E][F][K] (b_mn == 0: K
@@ -292,18 +327,43 @@ int launch_grouped_swiglu_2cta(const void* A, const void* Wg, const void* Wu, vo
 int launch_grouped_swiglu_bwd_2cta(const void* DY, const void* W, const void* GU, void* DGU, const void* offsets, int rows,
                                    int E, int F, int K, long long lda, long long ldgu, int b_mn, int num_sms, cudaStream_t st,
                                    int* status) {
-  CUtensorMap ma, mb;
-  int rc = make_map_2d_bf16(&ma, DY, rows, K, lda, BK, CTA_M);
-  if (rc) return 100 + rc;
-  rc = b_mn ? make_map_2d_bf16(&mb, W, uint64_t(E) * K, F, F, 64, BK) : make_map_2d_bf16(&mb, W, uint64_t(E) * F, K, K, BK, HALF_N);
-  if (rc) return 200 + rc;
-  const int upper = ((rows + TILE_M - 1) / TILE_M + E) * ((F + TILE_N - 1) / TILE_N);
-  int pairs = num_sms / 2;
-  if (upper < pairs) pairs = upper;
-  void* gu = const_cast<void*>(GU);
-  return b_mn ? launch<true, 2>(ma, mb, mb, DGU, gu, offsets, E, F, K, ldgu, ldgu, 0, pairs, st, status)
-              : launch<false, 2>(ma, mb, mb, DGU, gu, offsets, E, F, K, ldgu, ldgu, 0, pairs, st, status);
+  return run<2, 1>(DY, &W, nullptr, DGU, const_cast<void*>(GU), offsets, rows, E, F, K, K, lda, ldgu, ldgu, b_mn, 0, num_sms, st,
+                   status);
 }
 
 }  // namespace grp2
 }  // namespace kf
+
+extern "C" void* kf_status_device_ptr();
+
+extern "C" {
+
+// The grouped products of an expert feed-forward with either packed weights (separate == 0: w[0] is the (E, .., ..) tensor)
+// or one matrix per expert (separate != 0: w[e], E <= 32; host arrays of device pointers).  CTA-pair tiles; rows >= 1.
+//   kind 0: C = A W_e;  1: C = silu(A W_e) * (A W2_e), GU (optional) the pre-activations;  2: C = SwiGLU'(GU) * (A W_e);
+//   kind 3: C = A[:, :K/2] W_e + A[:, K/2:] W2_e  (K / 2 a multiple of 64).
+// W_e: [N][K] (b_mn == 0) or [K][N] (b_mn == 1, K % 64 == 0); kind 3: K / 2 in its place.  Pitches multiples of 8.
+int kf_grouped_experts_bf16(int kind, const void* A, const void* const* w, const void* const* w2, int separate, void* C,
+                            void* GU, const void* offsets, int rows, int E, int N, int K, long long lda, long long ldc,
+                            long long ldgu, int b_mn, int num_sms, void* stream) {
+  using namespace kf::grp2;
+  const int KW = kind == 3 ? K / 2 : K;
+  if (E < 1 || E > (separate ? MAX_SEPARATE : MAX_EXPERTS) || (lda & 7) || (ldc & 7) || (GU && (ldgu & 7)) || (K & 7) ||
+      (N & 7) || ((b_mn || kind == 3) && (KW % BK)) || num_sms < 2 || kind < 0 || kind > 3)
+    return 5;
+  if (rows <= 0) return 0;
+  int* status = reinterpret_cast<int*>(kf_status_device_ptr());
+  cudaStream_t st = (cudaStream_t)stream;
+#define KF_EXPERTS(EPI_)                                                                                                      \
+  return separate ? run<EPI_, MAX_SEPARATE>(A, w, w2, C, GU, offsets, rows, E, N, K, KW, lda, ldc, ldgu, b_mn, 0, num_sms, st, status) \
+                  : run<EPI_, 1>(A, w, w2, C, GU, offsets, rows, E, N, K, KW, lda, ldc, ldgu, b_mn, 0, num_sms, st, status)
+  switch (kind) {
+    case 0: KF_EXPERTS(0);
+    case 1: KF_EXPERTS(1);
+    case 2: KF_EXPERTS(2);
+    default: KF_EXPERTS(3);
+  }
+#undef KF_EXPERTS
+}
+
+}  // extern "C"

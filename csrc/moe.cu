@@ -124,62 +124,210 @@ kf_router_topk(const T* __restrict__ logits, const float* __restrict__ bias, int
   if (lane == 0 && zacc != 0.f) atomicAdd(lse_sq_sum, zacc);
 }
 
+// ------------------------------------------------------------------ backward of the router
+// dlogits from the gradients of the renormalised weights, of the mean scores and of the z-loss; one warp per token, every
+// score recomputed from the logits (two reads and one write of the (tokens, E) matrix instead of about twenty element-wise
+// passes over it, which were 0.1 ms of launches at 1777 tokens).
+//   w_j = s_j / sum(s)        ->  ds_j = (dw_j - sum_i dw_i w_i) / sum(s)  at the selected experts
+//   mean_e = sum_t s_te / T   ->  ds_e += dmean_e / T
+//   s = sigmoid(l + b)        ->  dl = ds s (1 - s);      s = softmax(l)  ->  dl = s (ds - sum_e ds_e s_e)
+//   z = sum_t lse_t^2 / T     ->  dl += 2 dz / T lse softmax(l)
+// partial (optional, [gridDim.x][E]): this block's sum of the unrounded dl over its tokens (the bias gradient).
+template <typename T, bool SIGMOID>
+__global__ void __launch_bounds__(256)
+kf_router_bwd(const T* __restrict__ logits, const float* __restrict__ bias, const long long* __restrict__ idx,
+              const float* __restrict__ w, const float* __restrict__ dw, const float* __restrict__ dmean,
+              const float* __restrict__ dz, int tokens, int E, int k, T* __restrict__ dlogits, float* __restrict__ partial) {
+  extern __shared__ float sh[];  // [warps][E] sums of dl
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  float* mine = sh + warp * E;
+  if (partial)
+    for (int e = lane; e < E; e += 32) mine[e] = 0.f;
+  const float inv_t = 1.f / tokens;
+  const float dzv = dz ? dz[0] : 0.f;
+  for (int t = blockIdx.x * warps + warp; t < tokens; t += gridDim.x * warps) {
+    float raw[MAX_E_PER_LANE], sc[MAX_E_PER_LANE], ds[MAX_E_PER_LANE];
+    float mx = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < MAX_E_PER_LANE; ++j) {
+      const int e = lane + 32 * j;
+      raw[j] = e < E ? to_f<T>(logits[size_t(t) * E + e]) : -INFINITY;
+      mx = fmaxf(mx, raw[j]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    float se = 0.f;
+#pragma unroll
+    for (int j = 0; j < MAX_E_PER_LANE; ++j) se += (lane + 32 * j) < E ? __expf(raw[j] - mx) : 0.f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
+    const float lse = mx + __logf(se);
+#pragma unroll
+    for (int j = 0; j < MAX_E_PER_LANE; ++j) {
+      const int e = lane + 32 * j;
+      sc[j] = 0.f;
+      ds[j] = 0.f;
+      if (e < E) {
+        sc[j] = SIGMOID ? 1.f / (1.f + __expf(-(raw[j] + (bias ? bias[e] : 0.f)))) : __expf(raw[j] - mx) / se;
+        ds[j] = dmean ? dmean[e] * inv_t : 0.f;
+      }
+    }
+    // selected experts: sum of their scores, and <dw, w>
+    float ssum = 0.f, dot = 0.f;
+#pragma unroll
+    for (int r = 0; r < MAX_K; ++r)
+      if (r < k) {
+        const int e = (int)idx[size_t(t) * k + r];
+#pragma unroll
+        for (int j = 0; j < MAX_E_PER_LANE; ++j)
+          if (lane + 32 * j == e) ssum += sc[j];
+        dot += dw[size_t(t) * k + r] * w[size_t(t) * k + r];
+      }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, o);
+#pragma unroll
+    for (int r = 0; r < MAX_K; ++r)
+      if (r < k) {
+        const int e = (int)idx[size_t(t) * k + r];
+        const float d = (dw[size_t(t) * k + r] - dot) / ssum;
+#pragma unroll
+        for (int j = 0; j < MAX_E_PER_LANE; ++j)
+          if (lane + 32 * j == e) ds[j] += d;
+      }
+    float dots = 0.f;
+    if (!SIGMOID) {
+#pragma unroll
+      for (int j = 0; j < MAX_E_PER_LANE; ++j) dots += ds[j] * sc[j];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) dots += __shfl_xor_sync(0xffffffffu, dots, o);
+    }
+#pragma unroll
+    for (int j = 0; j < MAX_E_PER_LANE; ++j) {
+      const int e = lane + 32 * j;
+      if (e < E) {
+        float dl = SIGMOID ? ds[j] * sc[j] * (1.f - sc[j]) : sc[j] * (ds[j] - dots);
+        if (dzv != 0.f) dl += 2.f * dzv * inv_t * lse * (SIGMOID ? __expf(raw[j] - mx) / se : sc[j]);
+        if (partial) mine[e] += dl;
+        if constexpr (sizeof(T) == 2) dlogits[size_t(t) * E + e] = __float2bfloat16(dl);
+        else dlogits[size_t(t) * E + e] = dl;
+      }
+    }
+  }
+  if (!partial) return;
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    float v = 0.f;
+    for (int i = 0; i < warps; ++i) v += sh[i * E + e];
+    partial[size_t(blockIdx.x) * E + e] = v;
+  }
+}
+
+// out[e] = sum over the blocks of partial[b][e] (fixed order)
+__global__ void __launch_bounds__(256) kf_router_bias_grad(const float* __restrict__ partial, int blocks, int E, float* __restrict__ out) {
+  const int e = blockIdx.x, lane = threadIdx.x & 31;
+  __shared__ float red[8];
+  float v = 0.f;
+  for (int b = threadIdx.x; b < blocks; b += 256) v += partial[size_t(b) * E + e];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int i = 1; i < 8; ++i) v += red[i];
+    out[e] = v;
+  }
+}
+
 // ------------------------------------------------------------------ stable counting sort by expert
-constexpr int SORT_BLOCK = 256;
+// Latency-bound (a few tens of KB): what counts is the number of launches and of dependent memory round trips.  Two
+// launches: histograms of 1024 assignments per block, then every block sums the histogram rows it needs (its
+// predecessors' for the first destination rows, all of them for the expert offsets) with independent loads, instead of one
+// block walking all rows as a serial chain between the two.  Ranks inside a block come from warp matches and a prefix over
+// the 32 warps.
+constexpr int SORT_BLOCK = 1024;
+constexpr int SORT_MAX_E = 256;
 
 __global__ void __launch_bounds__(SORT_BLOCK)
 kf_moe_sort_hist(const long long* __restrict__ expert_of_slot, int slots, int E, int* __restrict__ block_hist) {
-  extern __shared__ int h[];
-  for (int i = threadIdx.x; i < E; i += blockDim.x) h[i] = 0;
+  __shared__ int h[SORT_MAX_E];
+  for (int i = threadIdx.x; i < E; i += SORT_BLOCK) h[i] = 0;
   __syncthreads();
   const int s = blockIdx.x * SORT_BLOCK + threadIdx.x;
-  if (s < slots) atomicAdd(&h[(int)expert_of_slot[s]], 1);
+  const int mine = s < slots ? (int)expert_of_slot[s] : -1;
+  const unsigned same = __match_any_sync(0xffffffffu, mine);
+  if (mine >= 0 && (int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&h[mine], __popc(same));
   __syncthreads();
-  for (int i = threadIdx.x; i < E; i += blockDim.x) block_hist[size_t(blockIdx.x) * E + i] = h[i];
-}
-
-// one block: offsets[e] (exclusive scan of the expert totals) and, in place, block_hist[b][e] -> first
-// destination row of block b's assignments to expert e
-__global__ void __launch_bounds__(256)
-kf_moe_sort_scan(int* __restrict__ block_hist, int n_blocks, int E, int* __restrict__ offsets) {
-  __shared__ int total[256];
-  const int e = threadIdx.x;
-  int sum = 0;
-  if (e < E)
-    for (int b = 0; b < n_blocks; ++b) {
-      const int v = block_hist[size_t(b) * E + e];
-      block_hist[size_t(b) * E + e] = sum;
-      sum += v;
-    }
-  total[e] = e < E ? sum : 0;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int i = 0; i < E; ++i) {
-      const int v = total[i];
-      total[i] = acc;
-      offsets[i] = acc;
-      acc += v;
-    }
-    offsets[E] = acc;
-  }
-  __syncthreads();
-  if (e < E)
-    for (int b = 0; b < n_blocks; ++b) block_hist[size_t(b) * E + e] += total[e];
+  for (int i = threadIdx.x; i < E; i += SORT_BLOCK) block_hist[size_t(blockIdx.x) * E + i] = h[i];
 }
 
 __global__ void __launch_bounds__(SORT_BLOCK)
-kf_moe_sort_place(const long long* __restrict__ expert_of_slot, int slots, int E, const int* __restrict__ block_base,
-                  int* __restrict__ row_of_slot, int* __restrict__ slot_of_row) {
-  __shared__ int ex[SORT_BLOCK];
+kf_moe_sort_place(const long long* __restrict__ expert_of_slot, int slots, int E, const int* __restrict__ block_hist,
+                  int n_blocks, int* __restrict__ offsets, int* __restrict__ row_of_slot, int* __restrict__ slot_of_row) {
+  __shared__ unsigned short wcnt[32][SORT_MAX_E];  // assignments of warp w to expert e, then their prefix over the warps
+  __shared__ int before[SORT_MAX_E], total[SORT_MAX_E], base[SORT_MAX_E];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i < 32 * E; i += SORT_BLOCK) wcnt[i / E][i % E] = 0;
+  for (int i = threadIdx.x; i < E; i += SORT_BLOCK) before[i] = total[i] = 0;
   const int s = blockIdx.x * SORT_BLOCK + threadIdx.x;
   const int mine = s < slots ? (int)expert_of_slot[s] : -1;
-  ex[threadIdx.x] = mine;
+  __syncthreads();
+  // column sums of the histogram: 1024 / E groups of rows per expert
+  {
+    const int groups = SORT_BLOCK / E, g = threadIdx.x / E, e = threadIdx.x % E;
+    if (g < groups) {
+      int lo = 0, all = 0;
+      for (int b = g; b < n_blocks; b += groups) {
+        const int v = block_hist[size_t(b) * E + e];
+        all += v;
+        if (b < (int)blockIdx.x) lo += v;
+      }
+      if (lo) atomicAdd(&before[e], lo);
+      if (all) atomicAdd(&total[e], all);
+    }
+  }
+  const unsigned same = __match_any_sync(0xffffffffu, mine);
+  const int rank = __popc(same & ((1u << lane) - 1u));
+  if (mine >= 0 && rank == 0) wcnt[warp][mine] = (unsigned short)__popc(same);
+  __syncthreads();
+  if (threadIdx.x < E) {
+    int acc = 0;
+    for (int w = 0; w < 32; ++w) {
+      const int v = wcnt[w][threadIdx.x];
+      wcnt[w][threadIdx.x] = (unsigned short)acc;
+      acc += v;
+    }
+  }
+  // exclusive scan of the expert totals by the last warp (up to 8 experts per lane)
+  if (warp == 31) {
+    int v[SORT_MAX_E / 32], sum = 0;
+#pragma unroll
+    for (int j = 0; j < SORT_MAX_E / 32; ++j) {
+      const int e = lane * (SORT_MAX_E / 32) + j;
+      v[j] = e < E ? total[e] : 0;
+      sum += v[j];
+    }
+    int pre = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, pre, o);
+      if (lane >= o) pre += u;
+    }
+    int at = pre - sum;
+#pragma unroll
+    for (int j = 0; j < SORT_MAX_E / 32; ++j) {
+      const int e = lane * (SORT_MAX_E / 32) + j;
+      if (e < E) {
+        base[e] = at;
+        if (blockIdx.x == 0) offsets[e] = at;
+        at += v[j];
+        if (blockIdx.x == 0 && e == E - 1) offsets[E] = at;
+      }
+    }
+  }
   __syncthreads();
   if (mine < 0) return;
-  int rank = 0;  // assignments to the same expert earlier in this block (keeps the sort stable)
-  for (int i = 0; i < threadIdx.x; ++i) rank += ex[i] == mine;
-  const int row = block_base[size_t(blockIdx.x) * E + mine] + rank;
+  const int row = base[mine] + before[mine] + wcnt[warp][mine] + rank;
   row_of_slot[s] = row;
   slot_of_row[row] = s;
 }
@@ -282,12 +430,42 @@ int kf_router_topk(const void* logits, int dt, const void* bias, int sigmoid, in
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
-// Stable sort of `slots` assignments by expert.  scratch: int32 [ceil(slots / 256) * E].  Outputs: offsets int32
+// Gradient of the logits of kf_router_topk.  w, dw fp32 [tokens][k]; dmean fp32 [E], dz fp32 [1] (each may be null);
+// dlogits in the type of the logits.  dbias (optional, fp32 [E], with partial fp32 [KF_ROUTER_BWD_BLOCKS = 592][E] scratch):
+// the sum of dlogits over the tokens.
+int kf_router_bwd(const void* logits, int dt, const void* bias, int sigmoid, const void* idx, const void* w, const void* dw,
+                  const void* dmean, const void* dz, int tokens, int E, int k, void* dlogits, void* dbias, void* partial,
+                  void* stream) {
+  using namespace kf::moe;
+  if (E < 1 || E > 32 * MAX_E_PER_LANE || k < 1 || k > MAX_K || k > E || (dbias && !partial)) return 3;
+  cudaStream_t st = (cudaStream_t)stream;
+  int blocks = (tokens + 7) / 8;
+  if (blocks > 592) blocks = 592;
+  if (blocks < 1) blocks = 1;
+#define KF_ROUTER_BWD(T_, S_)                                                                                           \
+  kf_router_bwd<T_, S_><<<blocks, 256, dbias ? 8 * size_t(E) * sizeof(float) : 0, st>>>(                                \
+      reinterpret_cast<const T_*>(logits), reinterpret_cast<const float*>(bias), reinterpret_cast<const long long*>(idx), \
+      reinterpret_cast<const float*>(w), reinterpret_cast<const float*>(dw), reinterpret_cast<const float*>(dmean),     \
+      reinterpret_cast<const float*>(dz), tokens, E, k, reinterpret_cast<T_*>(dlogits),                                 \
+      dbias ? reinterpret_cast<float*>(partial) : nullptr)
+  if (dt == 0) {
+    if (sigmoid) KF_ROUTER_BWD(__nv_bfloat16, true); else KF_ROUTER_BWD(__nv_bfloat16, false);
+  } else {
+    if (sigmoid) KF_ROUTER_BWD(float, true); else KF_ROUTER_BWD(float, false);
+  }
+#undef KF_ROUTER_BWD
+  if (dbias)
+    kf_router_bias_grad<<<E, 256, 0, st>>>(reinterpret_cast<const float*>(partial), blocks, E, reinterpret_cast<float*>(dbias));
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 400 + (int)e;
+}
+
+// Stable sort of `slots` assignments by expert.  scratch: int32 [ceil(slots / 1024) * E].  Outputs: offsets int32
 // [E + 1], row_of_slot int32 [slots], slot_of_row int32 [slots].
 int kf_moe_sort(const void* expert_of_slot, int slots, int E, void* scratch, void* offsets, void* row_of_slot,
                 void* slot_of_row, void* stream) {
   using namespace kf::moe;
-  if (E < 1 || E > 256) return 3;
+  if (E < 1 || E > SORT_MAX_E) return 3;
   cudaStream_t st = (cudaStream_t)stream;
   const int nb = (slots + SORT_BLOCK - 1) / SORT_BLOCK;
   if (nb == 0) {
@@ -295,10 +473,10 @@ int kf_moe_sort(const void* expert_of_slot, int slots, int E, void* scratch, voi
     return 0;
   }
   auto ex = reinterpret_cast<const long long*>(expert_of_slot);
-  kf_moe_sort_hist<<<nb, SORT_BLOCK, E * sizeof(int), st>>>(ex, slots, E, reinterpret_cast<int*>(scratch));
-  kf_moe_sort_scan<<<1, 256, 0, st>>>(reinterpret_cast<int*>(scratch), nb, E, reinterpret_cast<int*>(offsets));
-  kf_moe_sort_place<<<nb, SORT_BLOCK, 0, st>>>(ex, slots, E, reinterpret_cast<const int*>(scratch),
-                                               reinterpret_cast<int*>(row_of_slot), reinterpret_cast<int*>(slot_of_row));
+  kf_moe_sort_hist<<<nb, SORT_BLOCK, 0, st>>>(ex, slots, E, reinterpret_cast<int*>(scratch));
+  kf_moe_sort_place<<<nb, SORT_BLOCK, 0, st>>>(ex, slots, E, reinterpret_cast<const int*>(scratch), nb,
+                                               reinterpret_cast<int*>(offsets), reinterpret_cast<int*>(row_of_slot),
+                                               reinterpret_cast<int*>(slot_of_row));
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }

@@ -139,9 +139,15 @@ class MoEMLP(nn.Module):
         ex = self.experts
         return list(ex.values()) if isinstance(ex, nn.ModuleDict) else list(ex)
 
-    def run_experts(self, x_sorted: torch.Tensor, counts: torch.Tensor, offsets: torch.Tensor | None = None) -> torch.Tensor:
+    def run_experts(self, x_sorted: torch.Tensor, counts: torch.Tensor | None, offsets: torch.Tensor | None = None) -> torch.Tensor:
         """Grouped expert FFN over rows already sorted by (local) expert.  ``offsets`` (int32 (E + 1), device): the
-        row ranges when they are already known; ``x_sorted`` may then be longer than ``offsets[-1]``."""
+        row ranges when they are already known (``counts`` may then be None); ``x_sorted`` may then be longer than
+        ``offsets[-1]``."""
+        if offsets is not None and not self.packed_experts and self._is_swiglu:
+            ex = self.expert_modules()
+            y = grouped.separate_ffn(x_sorted, offsets, *([getattr(e, n).weight for e in ex] for n in ("gate_proj", "up_proj", "down_proj")))
+            if y is not None:
+                return y
         gate, up, down, layout = self.expert_weights()
         return grouped.grouped_ffn(x_sorted, counts, gate, up, down, layout, self._activation(), offsets=offsets)
 
@@ -153,9 +159,8 @@ class MoEMLP(nn.Module):
                 and x_flat.shape[1] % 8 == 0 and not (self.gradient_scale and self.training)):
             # device-side stable sort by expert, row gather, grouped expert GEMMs, weighted combine
             offsets, row_of_slot, slot_of_row = moe_ops.sort_by_expert(indices, self.num_experts)
-            counts = (offsets[1:] - offsets[:-1]).to(torch.int64)
             x_sorted = moe_ops.gather_rows(x_flat, slot_of_row, row_of_slot, k)
-            y = self.run_experts(x_sorted, counts, offsets=offsets)
+            y = self.run_experts(x_sorted, None, offsets=offsets)
             return moe_ops.combine_rows(y, weights, row_of_slot, slot_of_row)
         flat_e = indices.reshape(-1)
         order = torch.argsort(flat_e, stable=True)

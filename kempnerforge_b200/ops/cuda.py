@@ -85,6 +85,8 @@ def _declare(L: ctypes.CDLL) -> None:
         "kf_ep_layout": [vp, i, i, vp, vp, vp, vp, vp],
         "kf_ep_move_bf16": [vp, vp, vp, vp, vp, i, i, i, ll, i, vp, vp],
         "kf_router_topk": [vp, i, vp, i, i, i, i, vp, vp, vp, vp, vp, vp],
+        "kf_router_bwd": [vp, i, vp, i, vp, vp, vp, vp, vp, i, i, i, vp, vp, vp, vp],
+        "kf_grouped_experts_bf16": [i, vp, vp, vp, i, vp, vp, vp, i, i, i, i, ll, ll, ll, i, i, vp],
         "kf_moe_sort": [vp, i, i, vp, vp, vp, vp, vp],
         "kf_moe_capacity_mask": [vp, i, i, i, i, vp, vp],
         "kf_moe_gather_bf16": [vp, vp, i, i, i, vp, vp],
@@ -723,6 +725,20 @@ def router_topk(logits: torch.Tensor, bias: torch.Tensor | None, sigmoid: bool, 
     return w, idx, acc[:e], acc[e:2 * e], acc[2 * e:]
 
 
+def router_bwd(logits, bias, sigmoid: bool, idx, w, dw, dmean, dz, want_dbias: bool):
+    """(dlogits, dbias fp32 or None) of :func:`router_topk`: ``dw`` (T, k), ``dmean`` (E) of the mean scores and ``dz`` of the
+    mean squared logsumexp, all fp32."""
+    t, e = logits.shape
+    k = idx.shape[1]
+    dlogits = torch.empty_like(logits)
+    dbias = torch.empty(e, dtype=torch.float32, device=logits.device) if want_dbias else None
+    partial = torch.empty(592 * e, dtype=torch.float32, device=logits.device) if want_dbias else None
+    _check(lib().kf_router_bwd(logits.data_ptr(), 0 if logits.dtype == torch.bfloat16 else 1, _ptr(bias), int(sigmoid),
+                               idx.data_ptr(), w.data_ptr(), dw.data_ptr(), _ptr(dmean), _ptr(dz), t, e, k,
+                               dlogits.data_ptr(), _ptr(dbias), _ptr(partial), _stream()), "kf_router_bwd")
+    return dlogits, dbias
+
+
 def moe_capacity_mask(indices: torch.Tensor, num_experts: int, cap: int) -> torch.Tensor:
     """fp32 (T, k) mask: 1 for the first ``cap`` tokens (sequence order) of every (slot, expert) pair, else 0."""
     t, k = indices.shape
@@ -738,7 +754,7 @@ def moe_sort(indices: torch.Tensor, num_experts: int):
     flat = indices.reshape(-1)
     assert flat.dtype == torch.int64 and flat.is_contiguous()
     slots = flat.numel()
-    nb = (slots + 255) // 256
+    nb = (slots + 1023) // 1024
     scratch = torch.empty(max(nb, 1) * num_experts, dtype=torch.int32, device=flat.device)
     offsets = torch.empty(num_experts + 1, dtype=torch.int32, device=flat.device)
     row_of_slot = torch.empty(slots, dtype=torch.int32, device=flat.device)
@@ -852,6 +868,31 @@ def grouped_gemm_supported(a: torch.Tensor, b: torch.Tensor, b_mn: bool) -> bool
             and a.stride(0) % 8 == 0 and b.is_contiguous())
 
 
+MAX_SEPARATE_EXPERTS = 32   # experts whose weights the grouped kernels read through a tensor map each
+_GROUPED_PAIR = os.environ.get("KF_GROUPED_PAIR", "1") != "0"
+
+
+def grouped_pair_tiles() -> bool:
+    return _GROUPED_PAIR and sm_count() >= 2
+
+
+def grouped_experts(kind: int, a: torch.Tensor, w, w2, offsets: torch.Tensor, n: int, b_mn: bool, out: torch.Tensor,
+                    gu: torch.Tensor | None = None) -> torch.Tensor:
+    """Grouped products over expert rows on CTA-pair tiles: 0 ``a @ W_e``; 1 ``silu(a @ W_e) * (a @ W2_e)`` (``gu``: receives
+    the pre-activations); 2 the SwiGLU gradient of ``a @ W_e`` given ``gu``; 3 ``a[:, :K/2] @ W_e + a[:, K/2:] @ W2_e``.
+    ``w`` / ``w2``: one packed (E, .., ..) tensor or a list with one matrix per expert, (N, K) or, ``b_mn``, (K, N)."""
+    rows, k = a.shape
+    separate = isinstance(w, (list, tuple))
+    e = offsets.numel() - 1
+    arr = (c_void_p * e) if separate else (c_void_p * 1)
+    wp = arr(*[t.data_ptr() for t in w]) if separate else arr(w.data_ptr())
+    w2p = None if w2 is None else arr(*[t.data_ptr() for t in w2]) if separate else arr(w2.data_ptr())
+    _check(lib().kf_grouped_experts_bf16(kind, a.data_ptr(), wp, w2p, int(separate), out.data_ptr(), _ptr(gu), offsets.data_ptr(),
+                                         rows, e, n, k, a.stride(0), out.stride(0), gu.stride(0) if gu is not None else 0,
+                                         int(b_mn), sm_count(), _stream()), "kf_grouped_experts_bf16")
+    return out
+
+
 def grouped_wgrad(a: torch.Tensor, b: torch.Tensor, offsets: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     """Per-expert ``a_e^T @ b_e`` over the ragged row ranges ``offsets[e]:offsets[e+1]``: (E, a.shape[1], b.shape[1])
     in bf16.  The weight gradient of :func:`grouped_gemm`; experts without rows get zeros."""
@@ -920,6 +961,8 @@ def gemm_reduce_scatter(x2: torch.Tensor, w: torch.Tensor, ctx, seq_len: int, ou
 
 def grouped_pair_mode(mode: int) -> None:
     """1: the ragged grouped GEMMs run on CTA-pair tiles (default); 0: single-CTA 128 x 256 tiles."""
+    global _GROUPED_PAIR
+    _GROUPED_PAIR = bool(mode)
     lib().kf_grouped_pair_mode(int(mode))
 
 

@@ -10,6 +10,8 @@ pack/unpack loops of kempnerforge/model/moe.py:20-145.
 
 from __future__ import annotations
 
+import os
+
 import torch
 import torch.nn.functional as F
 
@@ -134,11 +136,74 @@ class _GroupedFFNFn(torch.autograd.Function):
         dgate, dup = dgu[:, :f], dgu[:, f:]
         dx = dwg = dwu = None
         if ctx.needs_input_grad[0]:
-            dx = kc.grouped_gemm(dgate, wg, offsets, b_mn=not kn)
-            kc.grouped_gemm(dup, wu, offsets, b_mn=not kn, out=dx, accumulate=True)
+            if f % 64 == 0 and kc.grouped_pair_tiles():   # one product over the 2 F gradient columns
+                dx = kc.grouped_experts(3, dgu, wg, wu, offsets, x.shape[1], not kn, torch.empty_like(x))
+            else:
+                dx = kc.grouped_gemm(dgate, wg, offsets, b_mn=not kn)
+                kc.grouped_gemm(dup, wu, offsets, b_mn=not kn, out=dx, accumulate=True)
         if ctx.needs_input_grad[1] or ctx.needs_input_grad[2]:
             dwg, dwu = wgrad(x, dgate), wgrad(x, dup)
         return dx, dwg, dwu, dwd, None, None
+
+
+class _SeparateFFNFn(torch.autograd.Function):
+    """:class:`_GroupedFFNFn` over one (F, D) gate, (F, D) up and (D, F) down matrix per expert, read where they are: the
+    kernels take a tensor map per expert, so nothing is stacked in the forward and the gate and up weight gradients come from
+    one reduction over the 2 F columns of d[gate | up]."""
+
+    @staticmethod
+    def forward(ctx, x, offsets, *weights):
+        kc = _cuda_binding
+        e = len(weights) // 3
+        gates, ups, downs = weights[:e], weights[e : 2 * e], weights[2 * e :]
+        rows, d = x.shape
+        f = gates[0].shape[0]
+        h = torch.empty((rows, f), dtype=x.dtype, device=x.device)
+        gu = torch.empty((rows, 2 * f), dtype=x.dtype, device=x.device)
+        kc.grouped_experts(1, x, gates, ups, offsets, f, False, h, gu)
+        y = kc.grouped_experts(0, h, downs, None, offsets, d, False, torch.empty_like(x))
+        ctx.save_for_backward(x, offsets, gu, h, *weights)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        kc = _cuda_binding
+        x, offsets, gu, h, *weights = ctx.saved_tensors
+        e = len(weights) // 3
+        gates, ups, downs = weights[:e], weights[e : 2 * e], weights[2 * e :]
+        f = h.shape[1]
+        if not dy.is_contiguous():
+            dy = dy.contiguous()
+        need = ctx.needs_input_grad[2:]
+        dwd = kc.grouped_wgrad(dy, h, offsets) if any(need[2 * e :]) else [None] * e
+        dgu = kc.grouped_experts(2, dy, downs, None, offsets, f, True, gu, gu)   # gu is dead after this; reuse its storage
+        dx = kc.grouped_experts(3, dgu, gates, ups, offsets, x.shape[1], True, torch.empty_like(x)) if ctx.needs_input_grad[0] else None
+        dwg = dwu = [None] * e
+        if any(need[: 2 * e]):
+            dw = kc.grouped_wgrad(dgu, x, offsets)                                # (E, 2 F, D)
+            dwg, dwu = [dw[i, :f] for i in range(e)], [dw[i, f:] for i in range(e)]
+        grads = [*dwg, *dwu, *(dwd[i] for i in range(e))]
+        return (dx, None, *(g if n else None for g, n in zip(grads, need)))
+
+
+def separate_ffn(x_sorted: torch.Tensor, offsets: torch.Tensor, gates, ups, downs) -> torch.Tensor | None:
+    """SwiGLU experts with separate Linear weights over expert-sorted rows, or None when the kernels do not cover them."""
+    from kempnerforge_b200.ops import functional as _F
+
+    kc = _cuda_binding
+    if (_F._FORCE_REF or not x_sorted.is_cuda or x_sorted.dtype != torch.bfloat16 or x_sorted.shape[0] < 256
+            or not kc.available() or len(gates) > kc.MAX_SEPARATE_EXPERTS or not kc.grouped_pair_tiles()
+            or os.environ.get("KF_DISABLE_GROUPED_SWIGLU") or os.environ.get("KF_SWIGLU_BWD_EPILOGUE", "1") != "1"
+            or os.environ.get("KF_GROUPED_WGRAD", "1") == "0"):
+        return None
+    d, f = x_sorted.shape[1], gates[0].shape[0]
+    if d % 64 or f % 64 or offsets.numel() != len(gates) + 1:
+        return None
+    for w, shape in [(w, (f, d)) for w in (*gates, *ups)] + [(w, (d, f)) for w in downs]:
+        if w.shape != shape or w.dtype != torch.bfloat16 or not w.is_cuda or not w.is_contiguous() or w.data_ptr() % 16:
+            return None
+    x = x_sorted if x_sorted.is_contiguous() else x_sorted.contiguous()
+    return _SeparateFFNFn.apply(x, offsets, *gates, *ups, *downs)
 
 
 def _native_ok(x: torch.Tensor, w: torch.Tensor, layout: str) -> bool:
@@ -185,7 +250,7 @@ def offsets_of(counts: torch.Tensor) -> torch.Tensor:
 
 def grouped_ffn(x_sorted, counts, gate_w, up_w, down_w, layout: str, activation=None, offsets=None) -> torch.Tensor:
     """Expert feed-forward over expert-sorted rows: SwiGLU when ``gate_w`` is given, else act(up) -> down.
-    ``offsets`` (int32 (E + 1) on the device) may be passed instead of being derived from ``counts``; ``x_sorted`` may
+    ``offsets`` (int32 (E + 1) on the device) may be passed instead of ``counts`` (then None); ``x_sorted`` may
     then have more rows than ``offsets[-1]`` (the extra rows are ignored)."""
     if (gate_w is not None and _native_ok(x_sorted, up_w, layout) and _native_ok(x_sorted, gate_w, layout)
             and _cuda_binding.grouped_swiglu_supported(x_sorted, gate_w, layout == "kn")):
@@ -200,6 +265,8 @@ def grouped_ffn(x_sorted, counts, gate_w, up_w, down_w, layout: str, activation=
                 return _GroupedFFNFn.apply(xs, gate_w, up_w, down_w, off, layout)
             hidden = _GroupedSwiGLUFn.apply(xs, gate_w, up_w, off, layout)
             return _GroupedLinearFn.apply(hidden, down_w, off, layout)
+    if counts is None:
+        counts = (offsets[1:] - offsets[:-1]).to(torch.int64)
     up = grouped_linear(x_sorted, up_w, counts, layout)
     if gate_w is not None:
         hidden = F.silu(grouped_linear(x_sorted, gate_w, counts, layout)) * up

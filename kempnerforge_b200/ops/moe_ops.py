@@ -1,6 +1,5 @@
 """Autograd wrappers of the native mixture-of-experts kernels: fused router, stable sort by expert, row gather and
-weighted combine.  Every piece stays on the device; the router's backward is a handful of element-wise PyTorch ops
-on the (tokens, experts) score matrix, everything else has a native backward.
+weighted combine.  Every piece stays on the device and has a native backward.
 
 Parity: kempnerforge/model/router.py:45-72,157-200 and kempnerforge/model/moe.py:256-349 (same mathematics: softmax
 or sigmoid(+bias) scores, top-k, renormalised weights, Switch load-balancing loss E * sum(f_e * P_e), z-loss
@@ -41,6 +40,13 @@ class _RouterFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dw, _didx, _dcounts, dmean, dz):
         logits, bias, idx, w = ctx.saved_tensors
+        if not torch.is_grad_enabled():
+            dlogits, dbias = kc.router_bwd(
+                logits, bias.float().contiguous() if ctx.has_bias else None, ctx.sigmoid, idx, w, dw.float().contiguous(),
+                dmean.float().contiguous() if dmean is not None else None, dz.float() if dz is not None else None,
+                ctx.has_bias and ctx.needs_input_grad[1])
+            return dlogits, dbias.to(bias.dtype) if dbias is not None else None, None, None
+        # create_graph: the same formulas as differentiable element-wise ops
         lf = logits.float()
         t = lf.shape[0]
         if ctx.sigmoid:

@@ -1,0 +1,91 @@
+"""Sort, router gradient and the expert feed-forward over separate weights at the edges of their ranges."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+def _gen(seed):
+    return torch.Generator(device=DEV).manual_seed(seed)
+
+
+@pytest.mark.parametrize("slots,e", [(1, 1), (31, 8), (1024, 64), (1025, 8), (10662, 64), (5000, 256), (70000, 3)])
+@pytest.mark.parametrize("skew", [False, True])
+def test_stable_sort_by_expert(native_lib, slots, e, skew):
+    ex = torch.randint(0, e, (slots,), device=DEV, generator=_gen(slots))
+    if skew:
+        ex = torch.where(torch.rand(slots, device=DEV, generator=_gen(1)) < 0.9, e - 1, ex)
+    off, row, slot = native_lib.moe_sort(ex, e)
+    order = torch.argsort(ex, stable=True)
+    assert torch.equal(slot.long(), order)
+    assert torch.equal(row.long()[order], torch.arange(slots, device=DEV))
+    assert torch.equal(off.long(), torch.cat([torch.zeros(1, dtype=torch.long, device=DEV), torch.bincount(ex, minlength=e).cumsum(0)]))
+
+
+@pytest.mark.parametrize("sigmoid", [False, True])
+@pytest.mark.parametrize("t,e,k,dtype", [(1, 2, 1, torch.float32), (77, 8, 2, torch.bfloat16), (1777, 64, 6, torch.bfloat16),
+                                         (5000, 160, 8, torch.float32), (333, 256, 8, torch.float32)])
+def test_router_gradient_matches_autograd_of_the_formulas(native_lib, sigmoid, t, e, k, dtype):
+    """Against the differentiable formulas (taken with create_graph) in the same fp32 arithmetic; the native scores use the
+    fast exponential (2^-21 relative)."""
+    from kempnerforge_b200.ops import moe_ops
+
+    logits = torch.randn(t, e, device=DEV, generator=_gen(1)).to(dtype).requires_grad_(True)
+    bias = (0.1 * torch.randn(e, device=DEV, generator=_gen(2))).to(dtype).requires_grad_(True) if sigmoid else None
+    w, idx, counts, mean, z = moe_ops.route(logits, bias, sigmoid, k)
+    loss = (w * torch.randn(t, k, device=DEV, generator=_gen(3))).sum() + 50 * (mean * torch.arange(e, device=DEV)).sum() + z * t
+    wrt = [logits] + ([bias] if sigmoid else [])
+    got = torch.autograd.grad(loss, wrt, retain_graph=True)
+    want = torch.autograd.grad(loss, wrt, create_graph=True)
+    for a, b in zip(got, want):
+        assert a.dtype == b.dtype
+        tol = 2.0**-8 if dtype == torch.bfloat16 else 2.0**-14
+        assert float((a.float() - b.float()).norm()) <= tol * float(b.float().norm())
+
+
+@pytest.mark.parametrize("counts", [[256], [128, 128, 128, 128], [5, 0, 300, 77, 130, 1], [0, 0, 513], [400, 17] + [3] * 30])
+@pytest.mark.parametrize("extra", [0, 64])
+def test_experts_with_separate_weights_match_the_packed_path(native_lib, counts, extra):
+    """Same rows, same matrices: stacked into packed tensors against one tensor map per expert (bit for bit where the
+    reduction is the same: everything but the input gradient's accumulation)."""
+    from kempnerforge_b200.ops import grouped
+
+    e, d, f = len(counts), 192, 320
+    rows = sum(counts)
+    x = torch.randn(rows + extra, d, device=DEV, generator=_gen(1)).bfloat16()
+    ws = [[(torch.randn(*s, device=DEV, generator=_gen(9 * i + j)) * 0.05).bfloat16().requires_grad_(True) for i in range(e)]
+          for j, s in enumerate(((f, d), (f, d), (d, f)))]
+    off = grouped.offsets_of(torch.tensor(counts, device=DEV))
+    dy = torch.randn(rows + extra, d, device=DEV, generator=_gen(3)).bfloat16()
+    xa = x.clone().requires_grad_(True)
+    ya = grouped.separate_ffn(xa, off, *ws)
+    assert ya is not None
+    ga = torch.autograd.grad(ya, [xa, *ws[0], *ws[1], *ws[2]], dy)
+    xb = x.clone().requires_grad_(True)
+    packed = [torch.stack([w.detach() for w in g]).requires_grad_(True) for g in ws]
+    yb = grouped.grouped_ffn(xb, None, *packed, "nk", offsets=off)
+    gb = torch.autograd.grad(yb, [xb, *packed], dy)
+    assert native_lib.read_status() == 0
+    assert torch.equal(ya[:rows], yb[:rows])
+    assert torch.equal(ga[0][:rows], gb[0][:rows])
+    for j in range(3):
+        assert torch.equal(torch.stack(ga[1 + j * e : 1 + (j + 1) * e]), gb[1 + j])
+
+
+def test_forms_the_separate_path_does_not_cover_return_none(native_lib):
+    from kempnerforge_b200.ops import grouped
+
+    def weights(e, f, d, dtype=torch.bfloat16):
+        return [[torch.zeros(s, device=DEV, dtype=dtype) for _ in range(e)] for s in ((f, d), (f, d), (d, f))]
+
+    off = lambda e: torch.zeros(e + 1, dtype=torch.int32, device=DEV)  # noqa: E731
+    x = torch.zeros(256, 128, device=DEV, dtype=torch.bfloat16)
+    assert grouped.separate_ffn(x[:255], off(2), *weights(2, 128, 128)) is None          # too few rows
+    assert grouped.separate_ffn(x, off(33), *weights(33, 64, 128)) is None               # too many experts
+    assert grouped.separate_ffn(x, off(2), *weights(2, 72, 128)) is None                 # F off the block
+    assert grouped.separate_ffn(x, off(2), *weights(2, 128, 128, torch.float32)) is None
+    g, u, dn = weights(2, 128, 128)
+    assert grouped.separate_ffn(x, off(2), [torch.zeros(128, 256, device=DEV, dtype=torch.bfloat16)[:, ::2]] * 2, u, dn) is None
