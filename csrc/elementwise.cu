@@ -419,6 +419,24 @@ kf_ce_fwd_bwd(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ 
   }
 }
 
+// x *= factor (one fp32 device scalar, rounded to bf16 like the tensor it scales).  A factor of exactly one, the gradient
+// that loss.backward() starts from, leaves x untouched and costs one scalar read per block.  Out of place, the pass over the
+// gradient of a 128 256 x 4096 weight (1 GB) took 1328 us of a 6413 us loss over 2047 tokens.
+__global__ void __launch_bounds__(256) kf_scale(__nv_bfloat16* __restrict__ x, long long n, const float* __restrict__ factor) {
+  const float f = __bfloat162float(__float2bfloat16(*factor));
+  if (f == 1.f) return;
+  const long long nvec = n >> 3;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
+    F8 t = load8(x + i * 8);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t.v[k] *= f;
+    store8(x + i * 8, t);
+  }
+  if (blockIdx.x == 0)
+    for (long long i = nvec * 8 + threadIdx.x; i < n; i += blockDim.x)
+      x[i] = __float2bfloat16(__bfloat162float(x[i]) * f);
+}
+
 // ------------------------------------------------------------------ vocabulary-parallel cross entropy
 // The vocabulary dimension of the logits is sharded over the tensor-parallel ranks (this rank holds columns
 // [vocab_start, vocab_start + V)).  Phase 1 produces, per row, the local maximum, the local sum of exponentials
@@ -706,6 +724,14 @@ int kf_embedding_fwd_bf16(const void* ids, const void* table, void* out, long lo
   if (D % 8) return 1;
   kf_embedding_fwd<<<grid_for(tokens * (D / 8), 256), 256, 0, (cudaStream_t)stream>>>(
       (const long long*)ids, (const __nv_bfloat16*)table, (__nv_bfloat16*)out, tokens, D, vocab);
+  KF_LAUNCH_CHECK();
+}
+
+// x[n] bf16 (16-byte aligned) *= *factor, in place.
+int kf_scale_bf16(void* x, long long n, const void* factor, void* stream) {
+  using namespace kf;
+  if (n <= 0) return 0;
+  kf_scale<<<grid_for(n / 8 + 1, 256, 148 * 8), 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)x, n, (const float*)factor);
   KF_LAUNCH_CHECK();
 }
 

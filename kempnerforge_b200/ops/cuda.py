@@ -71,6 +71,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "kf_embedding_fwd_bf16": [vp, vp, vp, ll, i, i, vp],
         "kf_embedding_bwd_bf16": [vp, vp, vp, ll, i, i, vp],
         "kf_ce_fwd_bwd_bf16": [vp, vp, vp, vp, vp, f, i, i, i, vp],
+        "kf_scale_bf16": [vp, ll, vp, vp],
         "kf_ce_vp_stats_bf16": [vp, vp, ll, vp, vp, vp, i, i, i, vp],
         "kf_ce_vp_bwd_bf16": [vp, vp, ll, vp, vp, vp, f, i, i, i, vp],
         "kf_adamw_flat": [vp, vp, vp, vp, ll, ll, f, f, f, f, f, f, f, vp, vp, i, i, i, vp],
@@ -475,6 +476,13 @@ def ce_fwd_bwd(logits: torch.Tensor, labels: torch.Tensor, stats: torch.Tensor, 
     )
     stats[0] += row_nll.sum()
     stats[1] += row_lse2.sum()
+
+
+def scale_(x: torch.Tensor, factor: torch.Tensor) -> torch.Tensor:
+    """x *= factor in place (contiguous bf16 x, one fp32 device scalar); costs nothing on the device when it is one."""
+    assert x.is_contiguous() and x.dtype == torch.bfloat16 and factor.dtype == torch.float32 and factor.numel() == 1
+    _check(lib().kf_scale_bf16(x.data_ptr(), x.numel(), factor.data_ptr(), _stream()), "kf_scale_bf16")
+    return x
 
 
 # --------------------------------------------------------------------------- optimizer
