@@ -127,6 +127,104 @@ kf_rmsnorm_fwd(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
   }
 }
 
+// Many rows: one warp per row, the whole row in registers (VPL 16-byte vectors per lane, all loads issued before the first
+// use), reduction by shuffles only.  The block-per-row kernel above spends two block barriers per row with one 16-byte load
+// in flight per thread; at 8192 x 4096 it took 36 us (134 MB: 20 us at the copy rate), this one 30 us.  It stays for
+// few rows (decoding), where a row spread over a block finishes sooner, and for rows longer than 32 * 8 * 16 = 4096.
+constexpr int ROWS_PER_BLOCK = 4;
+constexpr int WARP_ROWS_MIN = 1024;  // rows from which warps per row fill the machine (148 SMs x 8 rows in flight)
+
+__device__ __forceinline__ F8 unpack8(const uint4 u) {
+  F8 r;
+  const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), c = unpack_bf16(u.z), d = unpack_bf16(u.w);
+  r.v[0] = a.x; r.v[1] = a.y; r.v[2] = b.x; r.v[3] = b.y;
+  r.v[4] = c.x; r.v[5] = c.y; r.v[6] = d.x; r.v[7] = d.y;
+  return r;
+}
+
+template <int VPL>
+__global__ void __launch_bounds__(32 * ROWS_PER_BLOCK)
+kf_rmsnorm_fwd_warp(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                    __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, int rows, int D, float eps) {
+  const int row = blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int nvec = D >> 3;
+  grid_dep_wait();
+  grid_dep_launch();
+  if (row >= rows) return;
+  const uint4* xr = reinterpret_cast<const uint4*>(x + size_t(row) * D);
+  uint4 v[VPL];
+#pragma unroll
+  for (int c = 0; c < VPL; ++c) v[c] = lane + c * 32 < nvec ? xr[lane + c * 32] : make_uint4(0, 0, 0, 0);
+  float ss = 0.f;
+#pragma unroll
+  for (int c = 0; c < VPL; ++c) {
+    const F8 t = unpack8(v[c]);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ss += t.v[i] * t.v[i];
+  }
+  const float r = rsqrtf(warp_sum(ss) / D + eps);
+  if (lane == 0 && rstd) rstd[row] = r;
+  __nv_bfloat16* yr = y + size_t(row) * D;
+#pragma unroll
+  for (int c = 0; c < VPL; ++c)
+    if (lane + c * 32 < nvec) {
+      const F8 g = load8(w + (lane + c * 32) * 8);
+      F8 t = unpack8(v[c]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) t.v[i] = t.v[i] * r * g.v[i];
+      store8(yr + (lane + c * 32) * 8, t);
+    }
+}
+
+// dx = [dx_in +] r*g - x*r^3*mean(g*x), one warp per row, up to 2048 columns (at 4096 both rows take 128 registers and the
+// occupancy with them: 116 us against the block kernel's 85 at 8192 x 4096); every read of dy and dx_in precedes the writes of the same
+// elements by the same thread, so dx may alias either.
+template <int VPL>
+__global__ void __launch_bounds__(32 * ROWS_PER_BLOCK)
+kf_rmsnorm_bwd_dx_warp(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                       const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd, __nv_bfloat16* dx, int rows, int D,
+                       const __nv_bfloat16* dx_in) {
+  const int row = blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int nvec = D >> 3;
+  if (row >= rows) return;
+  const uint4* xr = reinterpret_cast<const uint4*>(x + size_t(row) * D);
+  const uint4* gr = reinterpret_cast<const uint4*>(dy + size_t(row) * D);
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  uint4 xv[VPL], gv[VPL];
+#pragma unroll
+  for (int c = 0; c < VPL; ++c) {
+    const bool in = lane + c * 32 < nvec;
+    xv[c] = in ? xr[lane + c * 32] : zero;
+    gv[c] = in ? gr[lane + c * 32] : zero;
+  }
+  const float r = rstd[row];
+  float dot = 0.f;
+#pragma unroll
+  for (int c = 0; c < VPL; ++c)
+    if (lane + c * 32 < nvec) {
+      const F8 a = unpack8(xv[c]), g = unpack8(gv[c]), ww = load8(w + (lane + c * 32) * 8);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) dot += g.v[i] * ww.v[i] * a.v[i];
+    }
+  const float coef = warp_sum(dot) / D * r * r * r;
+  __nv_bfloat16* dxr = dx + size_t(row) * D;
+  const __nv_bfloat16* dir = dx_in ? dx_in + size_t(row) * D : nullptr;
+#pragma unroll
+  for (int c = 0; c < VPL; ++c)
+    if (lane + c * 32 < nvec) {
+      const int e = (lane + c * 32) * 8;
+      const F8 a = unpack8(xv[c]), g = unpack8(gv[c]), ww = load8(w + e);
+      F8 o;
+      if (dir) o = load8(dir + e);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float d = r * g.v[i] * ww.v[i] - a.v[i] * coef;
+        o.v[i] = dir ? o.v[i] + d : d;
+      }
+      store8(dxr + e, o);
+    }
+}
+
 // RMSNorm backward in two streaming passes (dw first, so that dx may overwrite dy in place):
 //   kf_rmsnorm_bwd_dw   dw partial[chunk][d] = sum over the chunk's rows of dy * x * rstd   (column-parallel, fp32)
 //   kf_rmsnorm_bwd_dx   dx = [dx_in +] r*g - x*r^3*mean(g*x) with g = dy*w                   (one block per row)
@@ -143,19 +241,21 @@ kf_rmsnorm_bwd_dw(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __r
   const int r1 = min(rows, r0 + rows_per_chunk);
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   int row = r0;
-  for (; row + 4 <= r1; row += 4) {  // four rows in flight per thread
-    F8 g[4], a[4];
-    float r[4];
+  for (; row + 8 <= r1; row += 8) {  // eight rows in flight per thread, packed until they are used
+    uint4 g[8], a[8];
+    float r[8];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      g[u] = load8(dy + size_t(row + u) * D + v * 8);
-      a[u] = load8(x + size_t(row + u) * D + v * 8);
+    for (int u = 0; u < 8; ++u) {
+      g[u] = *reinterpret_cast<const uint4*>(dy + size_t(row + u) * D + v * 8);
+      a[u] = *reinterpret_cast<const uint4*>(x + size_t(row + u) * D + v * 8);
       r[u] = rstd[row + u];
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < 8; ++u) {
+      const F8 gg = unpack8(g[u]), aa = unpack8(a[u]);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] += g[u].v[i] * a[u].v[i] * r[u];
+      for (int i = 0; i < 8; ++i) acc[i] += gg.v[i] * aa.v[i] * r[u];
+    }
   }
   for (; row < r1; ++row) {
     const F8 g = load8(dy + size_t(row) * D + v * 8), a = load8(x + size_t(row) * D + v * 8);
@@ -234,15 +334,25 @@ kf_rmsnorm_bwd_dx(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __r
   }
 }
 
-// dw[d] = sum_b partial[b][d]  (fixed order -> deterministic)
-__global__ void kf_colsum_partials(const float* __restrict__ partial, __nv_bfloat16* __restrict__ out_bf16,
-                                   float* __restrict__ out_f32, int nblocks, int D) {
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= D) return;
+// dw[d] = sum_b partial[b][d]  (fixed order -> deterministic): 32 columns x 8 interleaved row groups per block, so that the
+// chain of dependent additions is nblocks / 8 long and the loads of a group are independent of it.
+__global__ void __launch_bounds__(256) kf_colsum_partials(const float* __restrict__ partial, __nv_bfloat16* __restrict__ out_bf16,
+                                                          float* __restrict__ out_f32, int nblocks, int D) {
+  __shared__ float red[8][33];
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5, d = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int b = 0; b < nblocks; ++b) s += partial[size_t(b) * D + d];
-  if (out_bf16) out_bf16[d] = __float2bfloat16(s);
-  if (out_f32) out_f32[d] = s;
+  if (d < D) {
+#pragma unroll 8
+    for (int b = g; b < nblocks; b += 8) s += partial[size_t(b) * D + d];
+  }
+  red[g][lane] = s;
+  __syncthreads();
+  if (g == 0 && d < D) {
+#pragma unroll
+    for (int i = 1; i < 8; ++i) s += red[i][lane];
+    if (out_bf16) out_bf16[d] = __float2bfloat16(s);
+    if (out_f32) out_f32[d] = s;
+  }
 }
 
 // ------------------------------------------------------------------ RoPE (half-split pairs)
@@ -640,16 +750,18 @@ int kf_rmsnorm_fwd_pdl_bf16(const void* x, const void* w, void* y, void* rstd, i
                             void* stream) {
   using namespace kf;
   if (D % 8) return 1;
+  const bool warps = rows >= WARP_ROWS_MIN && D <= 4096;
+  auto kern = !warps ? kf_rmsnorm_fwd : D <= 1024 ? kf_rmsnorm_fwd_warp<4> : D <= 2048 ? kf_rmsnorm_fwd_warp<8> : kf_rmsnorm_fwd_warp<16>;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(rows < 148 * 8 ? rows : 148 * 8);
-  cfg.blockDim = dim3(NORM_THREADS);
+  cfg.gridDim = dim3(warps ? (rows + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK : rows < 148 * 8 ? rows : 148 * 8);
+  cfg.blockDim = dim3(warps ? 32 * ROWS_PER_BLOCK : NORM_THREADS);
   cfg.stream = (cudaStream_t)stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kf_rmsnorm_fwd, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
                                      (__nv_bfloat16*)y, (float*)rstd, rows, D, eps);
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
@@ -674,8 +786,15 @@ int kf_rmsnorm_bwd_bf16(const void* dy, const void* x, const void* w, const void
   // dw first: the dx pass may overwrite dy
   kf_rmsnorm_bwd_dw<<<dim3((nvec + 255) / 256, chunks), 256, 0, st>>>(
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const float*)rstd, (float*)dw_partial, rows, D, rows_per_chunk);
-  kf_colsum_partials<<<(D + 255) / 256, 256, 0, st>>>((const float*)dw_partial, (__nv_bfloat16*)dw_bf16,
-                                                      (float*)dw_f32, chunks, D);
+  kf_colsum_partials<<<(D + 31) / 32, 256, 0, st>>>((const float*)dw_partial, (__nv_bfloat16*)dw_bf16,
+                                                    (float*)dw_f32, chunks, D);
+  if (rows >= WARP_ROWS_MIN && D <= 2048) {
+    auto kern = D <= 1024 ? kf_rmsnorm_bwd_dx_warp<4> : kf_rmsnorm_bwd_dx_warp<8>;
+    kern<<<(rows + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK, 32 * ROWS_PER_BLOCK, 0, st>>>(
+        (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const float*)rstd, (__nv_bfloat16*)dx,
+        rows, D, (const __nv_bfloat16*)dx_in);
+    KF_LAUNCH_CHECK();
+  }
   kf_rmsnorm_bwd_dx<<<rows < 148 * 8 ? rows : 148 * 8, NORM_THREADS, 0, st>>>(
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const float*)rstd,
       (__nv_bfloat16*)dx, rows, D, (const __nv_bfloat16*)dx_in);
