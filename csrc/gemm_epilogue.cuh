@@ -75,18 +75,31 @@ __device__ __forceinline__ void swiglu_chunk(uint32_t (&g)[32], const uint32_t (
   }
 }
 
+// The saved pre-activations of one 32-column chunk of one row (loaded ahead of their use).
+struct GuChunk {
+  uint4 g[4], u[4];
+};
+__device__ __forceinline__ GuChunk load_gu_chunk(const __nv_bfloat16* gate_row, const __nv_bfloat16* up_row, int valid_cols) {
+  GuChunk r;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const bool in = q * 8 < valid_cols;
+    r.g[q] = in ? *reinterpret_cast<const uint4*>(gate_row + q * 8) : make_uint4(0, 0, 0, 0);
+    r.u[q] = in ? *reinterpret_cast<const uint4*>(up_row + q * 8) : make_uint4(0, 0, 0, 0);
+  }
+  return r;
+}
+
 // SwiGLU backward on one 32-column chunk: `dh` holds the gradient of the hidden activation (fp32 accumulator values),
-// gate_row / up_row point at the saved bf16 pre-activations of these 32 hidden units, dgate_row / dup_row receive the
-// gradients (they may be the same memory as gate_row / up_row: every element is read and written by one thread).
+// `gu` the saved bf16 pre-activations of these 32 hidden units, dgate_row / dup_row receive the gradients (they may be the
+// memory `gu` was loaded from: every element is read and written by one thread).
 // The incoming gradient is rounded to bf16 first, like the two-kernel path.
-__device__ __forceinline__ void swiglu_bwd_chunk(const uint32_t (&dh)[32], const __nv_bfloat16* gate_row,
-                                                 const __nv_bfloat16* up_row, __nv_bfloat16* dgate_row,
+__device__ __forceinline__ void swiglu_bwd_chunk(const uint32_t (&dh)[32], const GuChunk& gu, __nv_bfloat16* dgate_row,
                                                  __nv_bfloat16* dup_row, int valid_cols) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     if (q * 8 >= valid_cols) break;
-    const uint4 gq = *reinterpret_cast<const uint4*>(gate_row + q * 8);
-    const uint4 uq = *reinterpret_cast<const uint4*>(up_row + q * 8);
+    const uint4 gq = gu.g[q], uq = gu.u[q];
     const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w}, uw[4] = {uq.x, uq.y, uq.z, uq.w};
     uint32_t dg[4], du[4];
 #pragma unroll

@@ -280,9 +280,14 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
       const TileCoord tc = tile_at(t);
       const int acc = tile_iter & 1;
       const uint32_t acc_ph = (tile_iter >> 1) & 1;
+      const int row = tc.m * TILE_M + int(rank) * CTA_M + quarter * 32 + lane;
+      GuChunk gu_next;
+      if constexpr (SWIGLU == 3) {  // the first pre-activations travel while the tile's products are still running
+        const __nv_bfloat16* gu_row = reinterpret_cast<const __nv_bfloat16*>(R) + size_t(row) * ldr + tc.n * TILE_N;
+        gu_next = load_gu_chunk(gu_row, gu_row + N, row < M ? N - tc.n * TILE_N : 0);
+      }
       if (!mbar_wait(tfull_bar(acc), acc_ph, status, KF_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
-      const int row = tc.m * TILE_M + int(rank) * CTA_M + quarter * 32 + lane;
       const uint32_t t_row = tmem_base + (uint32_t(quarter * 32) << 16) + acc * TILE_N;
       if constexpr (SWIGLU == 3) {
         // SwiGLU backward in the epilogue of the down projection's input-gradient GEMM: the accumulator is
@@ -295,11 +300,14 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
         for (int c = 0; c < TILE_N / 32; ++c) {
           uint32_t v[32];
           tmem_ld_32x32(t_row + c * 32, v);
+          // chunk c + 1 is fetched while chunk c is worked on: without it the eight load latencies of a row, not the
+          // products, set the pace of a K = 4096 tile
+          const GuChunk gu_now = gu_next;
+          if (c + 1 < TILE_N / 32)
+            gu_next = load_gu_chunk(gu_row + (c + 1) * 32, gu_row + N + (c + 1) * 32, row < M ? N - (col0 + (c + 1) * 32) : 0);
           tmem_ld_wait();
           const int valid = min(32, N - (col0 + c * 32));
-          if (row < M && valid > 0) {
-            swiglu_bwd_chunk(v, gu_row + c * 32, gu_row + N + c * 32, d_row + c * 32, d_row + N + c * 32, valid);
-          }
+          if (row < M && valid > 0) swiglu_bwd_chunk(v, gu_now, d_row + c * 32, d_row + N + c * 32, valid);
         }
         tc_fence_before();
         __syncwarp();

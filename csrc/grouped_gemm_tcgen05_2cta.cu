@@ -192,10 +192,15 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
     for (int t = pair; t < num_tiles && ok; t += num_pairs, ++tile_iter) {
       const Tile tl = tilemath::grouped_decode(t, n_blocks, tile_start, offsets, E, TILE_M);
       const int acc = tile_iter & 1;
-      if (!mbar_wait(tfull_bar(acc), (tile_iter >> 1) & 1, status, KF_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
-      tc_fence_after();
       const int r = int(rank) * CTA_M + quarter * 32 + lane;  // row inside the 256-row tile
       const int col0 = tl.nb * TN;
+      GuChunk gu_next;
+      if constexpr (EPI == 2) {  // the first pre-activations travel while the tile's products are still running
+        const __nv_bfloat16* gu_row = GU + size_t(tl.row0 + r) * ldgu + col0;
+        gu_next = load_gu_chunk(gu_row, gu_row + N, r < tl.valid ? N - col0 : 0);
+      }
+      if (!mbar_wait(tfull_bar(acc), (tile_iter >> 1) & 1, status, KF_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+      tc_fence_after();
       const uint32_t t_row = tmem_base + (uint32_t(quarter * 32) << 16) + acc * TILE_N;
       __nv_bfloat16* c_row = C + size_t(tl.row0 + r) * ldc + col0;
       if constexpr (EPI == 2) {
@@ -207,11 +212,12 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
         for (int c = 0; c < TILE_N / 32; ++c) {
           uint32_t v[32];
           tmem_ld_32x32(t_row + c * 32, v);
+          const GuChunk gu_now = gu_next;  // chunk c + 1 is fetched while chunk c is worked on
+          if (c + 1 < TILE_N / 32)
+            gu_next = load_gu_chunk(gu_row + (c + 1) * 32, gu_row + N + (c + 1) * 32, r < tl.valid ? N - (col0 + (c + 1) * 32) : 0);
           tmem_ld_wait();
           const int valid_cols = min(32, N - (col0 + c * 32));
-          if (r < tl.valid && valid_cols > 0) {
-            swiglu_bwd_chunk(v, gu_row + c * 32, gu_row + N + c * 32, c_row + c * 32, c_row + N + c * 32, valid_cols);
-          }
+          if (r < tl.valid && valid_cols > 0) swiglu_bwd_chunk(v, gu_now, c_row + c * 32, c_row + N + c * 32, valid_cols);
         }
       } else if constexpr (SWIGLU) {
         __nv_bfloat16* gu_row = GU ? GU + size_t(tl.row0 + r) * ldgu + col0 : nullptr;
