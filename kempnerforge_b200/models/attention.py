@@ -83,6 +83,11 @@ class Attention(nn.Module):
         key_padding_mask: torch.Tensor | None = None,
     ) -> torch.Tensor:
         qkv_w = [self.q_proj.weight, self.k_proj.weight, self.v_proj.weight]
+        if (x.is_cuda and self.tp is None and self.q_norm is None and kv_cache is None and key_padding_mask is None
+                and not self.capture_attention_weights):
+            out = F.qkv_attention(x, *qkv_w, rope_cos, rope_sin, doc_ids, self.head_dim)
+            if out is not None:
+                return F.linear(out, self.o_proj.weight)
         qkv = None
         if self.tp is not None:
             qkv = self.tp.column_linear(x, qkv_w)  # gathers the sequence shards (inside the GEMM when it can)

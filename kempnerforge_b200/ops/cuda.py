@@ -281,6 +281,14 @@ def gemm_rows(x2: torch.Tensor, weights, residual: torch.Tensor | None = None, o
     """x2 (M, K) times up to three (n_i, K) weights stacked along the output (+ ``residual``) -> bf16 (M, sum n_i).  With few
     rows the weights are read where they are; otherwise they are stacked for the tile kernels."""
     m, k = x2.shape
+    if len(weights) > 1 and residual is None and out is None and _separate_ok(x2, weights, 128) and not rows_adjacent(weights):
+        # the rotary kernel with nothing to rotate: one tensor map per weight
+        n = sum(w.shape[0] for w in weights)
+        out = torch.empty((m, n), dtype=torch.bfloat16, device=x2.device)
+        ptrs, rows, pitch = _weights3(weights)
+        _check(lib().kf_gemm_rope_bf16(x2.data_ptr(), *ptrs, out.data_ptr(), m, *rows, k, x2.stride(0), pitch[0], n, None, None,
+                                       1, 0, 64, sm_count(), _stream()), "kf_gemm_rope_bf16")
+        return out
     if not _few_rows(m, sum(w.shape[0] for w in weights)) or any(w.shape[0] % 8 or w.stride(0) % 8 or w.data_ptr() % 16 for w in weights) or k % 8:
         return gemm(x2, stack_rows(weights), residual=residual, out=out)
     ptrs, rows, pitch = _weights3(weights)
@@ -299,6 +307,32 @@ def gemm_rows(x2: torch.Tensor, weights, residual: torch.Tensor | None = None, o
                                      m, k, *rows, x2.stride(0), *pitch, out.stride(0), ldr, 0, 0, sm_count(), _stream()),
            "kf_gemm_skinny_bf16")
     return out
+
+
+def _separate_ok(x2: torch.Tensor, weights, step: int) -> bool:
+    """The CTA-pair kernel may read the weights through a tensor map each: enough 256 x 256 tiles for it, one pitch, all but
+    the last matrix a multiple of ``step`` rows, heads of 64 columns throughout."""
+    m, n = x2.shape[0], sum(w.shape[0] for w in weights)
+    tiles = -(-m // 256) * (-(-n // 256))
+    return (tiles >= 2 * (sm_count() // 2) and n % 64 == 0 and x2.stride(0) % 8 == 0 and x2.data_ptr() % 16 == 0
+            and all(w.shape[0] % step == 0 for w in weights[:-1])
+            and all(w.stride() == weights[0].stride() and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0 for w in weights))
+
+
+def dgrad_rows(dy2: torch.Tensor, weights) -> torch.Tensor:
+    """dy2 (M, sum n_i) times the (n_i, K) weights stacked along n: the input gradient of :func:`gemm_rows`."""
+    m, n = dy2.shape
+    k = weights[0].shape[1]
+    tiles = -(-m // 256) * (-(-k // 256))
+    if (len(weights) in (2, 3) and not rows_adjacent(weights) and tiles >= 2 * (sm_count() // 2) and k % 8 == 0
+            and dy2.stride(0) % 8 == 0 and dy2.data_ptr() % 16 == 0 and all(w.shape[0] % 64 == 0 for w in weights[:-1])
+            and all(w.stride() == weights[0].stride() and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0 for w in weights)):
+        out = torch.empty((m, k), dtype=torch.bfloat16, device=dy2.device)
+        ptrs, rows, pitch = _weights3(weights)
+        _check(lib().kf_gemm_dgrad_stacked_bf16(dy2.data_ptr(), *ptrs, out.data_ptr(), m, k, *rows, dy2.stride(0), pitch[0], k,
+                                                sm_count(), _stream()), "kf_gemm_dgrad_stacked_bf16")
+        return out
+    return gemm(dy2, stack_rows(weights), a_kmajor=True, b_kmajor=False)
 
 
 def swiglu_rows(x2: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor) -> torch.Tensor:

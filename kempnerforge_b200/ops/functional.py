@@ -77,26 +77,24 @@ class _LinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, *weights):
         cu = _cuda()
-        w = cu.stack_rows(weights)
         x2 = x.reshape(-1, x.shape[-1])
         if not x2.is_contiguous():
             x2 = x2.contiguous()
-        y = cu.gemm(x2, w, a_kmajor=True, b_kmajor=True)
+        y = cu.gemm(x2, weights[0]) if len(weights) == 1 or len(weights) > 3 else cu.gemm_rows(x2, weights)
         ctx.save_for_backward(x2, *weights)
         ctx.x_shape = x.shape
-        return y.view(*x.shape[:-1], w.shape[0])
+        return y.view(*x.shape[:-1], y.shape[-1])
 
     @staticmethod
     def backward(ctx, dy):
         cu = _cuda()
         x2, *weights = ctx.saved_tensors
-        w = cu.stack_rows(weights)
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
         dx = None
         if ctx.needs_input_grad[0]:
-            dx = cu.gemm(dy2, w, a_kmajor=True, b_kmajor=False).view(ctx.x_shape)
+            dx = cu.dgrad_rows(dy2, weights).view(ctx.x_shape)
         wgrads = _linear_weight_grads(cu, dy2, x2, weights, ctx.needs_input_grad[1:])
         return (dx, *wgrads)
 
@@ -333,6 +331,64 @@ def attention(
         )
         return out.transpose(1, 2)
     return ref.attention(q, k, v, causal, doc_ids, key_padding_mask, scale)
+
+
+class _QKVAttnFn(torch.autograd.Function):
+    """Attention(rotate(x Wqᵀ), rotate(x Wkᵀ), x Wvᵀ) as one node: the projection of all three weights in one GEMM with the
+    rotation in its epilogue, and a backward whose attention kernel writes dq | dk | dv into one gradient matrix, already
+    through the inverse rotation.  As separate ops the three head ranges of the projection cost autograd a zero fill, a copy
+    and an addition of the whole matrix each."""
+
+    @staticmethod
+    def forward(ctx, x, wq, wk, wv, cos, sin, doc_ids, hd):
+        cu = _cuda()
+        b, s, d = x.shape
+        x2 = x.reshape(b * s, d)
+        if not x2.is_contiguous():
+            x2 = x2.contiguous()
+        h, hkv = wq.shape[0] // hd, wk.shape[0] // hd
+        qkv = cu.qkv_rope(x2, [wq, wk, wv], cos, sin, s, hd).view(b, s, h + 2 * hkv, hd)
+        mask = cu.doc_blocks(doc_ids) if doc_ids is not None else None
+        scale = 1.0 / math.sqrt(hd)
+        out, lse = cu.attn_fwd(qkv[:, :, :h], qkv[:, :, h : h + hkv], qkv[:, :, h + hkv :], True, mask, scale)
+        ctx.save_for_backward(x2, wq, wk, wv, cos, sin, qkv, out, lse, *(mask or ()))
+        ctx.meta = (b, s, d, h, hkv, hd, scale)
+        return out.view(b, s, h * hd)
+
+    @staticmethod
+    def backward(ctx, dout):
+        cu = _cuda()
+        x2, wq, wk, wv, cos, sin, qkv, out, lse, *mask = ctx.saved_tensors
+        b, s, d, h, hkv, hd, scale = ctx.meta
+        dqkv = torch.empty_like(qkv)
+        cu.attn_bwd(dout.reshape(b, s, h, hd), qkv[:, :, :h], qkv[:, :, h : h + hkv], qkv[:, :, h + hkv :], out, lse, True,
+                    tuple(mask) or None, scale, dq=dqkv[:, :, :h], dk=dqkv[:, :, h : h + hkv], dv=dqkv[:, :, h + hkv :],
+                    rope=(cos, sin))
+        dqkv2 = dqkv.view(b * s, (h + 2 * hkv) * hd)
+        dx = cu.dgrad_rows(dqkv2, [wq, wk, wv]).view(b, s, d) if ctx.needs_input_grad[0] else None
+        wgrads = _linear_weight_grads(cu, dqkv2, x2, [wq, wk, wv], ctx.needs_input_grad[1:4])
+        return (dx, *wgrads, None, None, None, None)
+
+
+def qkv_attention(x, wq, wk, wv, cos, sin, doc_ids, hd: int) -> torch.Tensor | None:
+    """Causal self-attention of x (B, S, D) up to the output projection -> (B, S, H hd), or None when the fused node does not
+    cover the call (head dim 128, bf16 on a GPU, gradients wanted, fp32 tables of this sequence, no fp8)."""
+    if (hd != 128 or not use_native(x) or not torch.is_grad_enabled() or x.dim() != 3 or x.shape[0] * x.shape[1] < 128
+            or cos.dtype != torch.float32 or sin.dtype != torch.float32 or cos.dim() != 2 or cos.shape != sin.shape
+            or cos.requires_grad or sin.requires_grad or cos.shape[0] < x.shape[1] or cos.shape[1] != hd // 2
+            or not (cos.is_cuda and cos.is_contiguous() and sin.is_contiguous()) or cos.data_ptr() % 16 or sin.data_ptr() % 16
+            or (doc_ids is not None and doc_ids.shape != x.shape[:2])):
+        return None
+    cu = _cuda()
+    d = x.shape[-1]
+    for w in (wq, wk, wv):
+        if (w.dtype != torch.bfloat16 or not w.is_cuda or w.dim() != 2 or w.shape[1] != d or w.shape[0] % hd or not w.is_contiguous()
+                or w.data_ptr() % 16 or getattr(w, "_kf_fp8", False)):
+            return None
+    if (d % 8 or wk.shape != wv.shape or wk.shape[0] == 0 or wq.shape[0] % wk.shape[0] or cu.attn_policy() != "native"
+            or getattr(cu.lib(), "kf_attn_bwd_bf16", None) is None):
+        return None
+    return _QKVAttnFn.apply(x, wq, wk, wv, cos, sin, doc_ids, hd)
 
 
 # --------------------------------------------------------------------------- swiglu
