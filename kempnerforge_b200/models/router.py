@@ -139,8 +139,9 @@ class SigmoidTopKRouter(nn.Module):
             counts = _counts(indices, self.num_experts)
             smean = None
         self.expert_counts = counts.detach()
-        util = counts / (x.shape[0] * self.top_k + 1e-8)
-        if self.training and may_update:
+        update = self.training and may_update
+        util = counts / (x.shape[0] * self.top_k + 1e-8) if update or self.sequence_aux_loss_weight > 0 else None
+        if update:
             with torch.no_grad():
                 self.expert_ema.lerp_(util.to(self.expert_ema.dtype), 1.0 - self.ema_decay)
                 nudge = self._effective_bias_rate() * (1.0 / self.num_experts - self.expert_ema.float())

@@ -129,7 +129,8 @@ def _declare(L: ctypes.CDLL) -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the raw handle of the current stream of the current device, without building a Stream object around it
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _check(code: int, what: str, launches: int = 1) -> None:
@@ -143,10 +144,11 @@ _SM_COUNT: dict[int, int] = {}
 
 
 def sm_count() -> int:
-    dev = torch.cuda.current_device()
-    if dev not in _SM_COUNT:
-        _SM_COUNT[dev] = torch.cuda.get_device_properties(dev).multi_processor_count
-    return _SM_COUNT[dev]
+    n = _SM_COUNT.get(torch._C._cuda_getDevice())
+    if n is None:
+        dev = torch.cuda.current_device()
+        n = _SM_COUNT[dev] = torch.cuda.get_device_properties(dev).multi_processor_count
+    return n
 
 
 def read_status() -> int:

@@ -29,28 +29,31 @@ class _RouterFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits, bias, sigmoid, k):
         logits = logits.contiguous()
-        w, idx, counts, prob_sum, lse_sq = kc.router_topk(logits, bias, sigmoid, k)
+        # the sigmoid router nudges its bias in place right after routing: a private fp32 copy serves both passes
+        bf = None if bias is None else bias.detach().to(torch.float32, copy=True)
+        w, idx, counts, prob_sum, lse_sq = kc.router_topk(logits, bf, sigmoid, k)
         t = logits.shape[0]
-        # the sigmoid router nudges its bias in place right after routing: keep a private copy for the backward
-        ctx.save_for_backward(logits, bias.detach().clone() if bias is not None else torch.empty(0), idx, w)
+        ctx.save_for_backward(logits, idx, w, *(() if bf is None else (bf,)))
         ctx.sigmoid, ctx.has_bias = sigmoid, bias is not None
+        ctx.bias_dtype = bias.dtype if bias is not None else None
         ctx.mark_non_differentiable(idx, counts)
         return w, idx, counts, prob_sum / t, lse_sq.reshape(()) / t
 
     @staticmethod
     def backward(ctx, dw, _didx, _dcounts, dmean, dz):
-        logits, bias, idx, w = ctx.saved_tensors
+        logits, idx, w, *rest = ctx.saved_tensors
+        bias = rest[0] if rest else None
         if not torch.is_grad_enabled():
             dlogits, dbias = kc.router_bwd(
-                logits, bias.float().contiguous() if ctx.has_bias else None, ctx.sigmoid, idx, w, dw.float().contiguous(),
+                logits, bias, ctx.sigmoid, idx, w, dw.float().contiguous(),
                 dmean.float().contiguous() if dmean is not None else None, dz.float() if dz is not None else None,
                 ctx.has_bias and ctx.needs_input_grad[1])
-            return dlogits, dbias.to(bias.dtype) if dbias is not None else None, None, None
+            return dlogits, dbias.to(ctx.bias_dtype) if dbias is not None else None, None, None
         # create_graph: the same formulas as differentiable element-wise ops
         lf = logits.float()
         t = lf.shape[0]
         if ctx.sigmoid:
-            scores = torch.sigmoid(lf + bias.float()) if ctx.has_bias else torch.sigmoid(lf)
+            scores = torch.sigmoid(lf + bias) if ctx.has_bias else torch.sigmoid(lf)
         else:
             scores = torch.softmax(lf, dim=-1)
         sel = scores.gather(1, idx)
@@ -69,7 +72,7 @@ class _RouterFn(torch.autograd.Function):
             dlogits = dlogits + (dz.float() * 2.0 / t) * lse * torch.softmax(lf, dim=-1)
         # expert_bias is nudged by its own rule, never by gradients through the scores (the reference detaches
         # nothing here either, but its bias update overwrites any gradient step); keep autograd's answer
-        dbias = dlogits.sum(dim=0).to(bias.dtype) if (ctx.has_bias and ctx.needs_input_grad[1]) else None
+        dbias = dlogits.sum(dim=0).to(ctx.bias_dtype) if (ctx.has_bias and ctx.needs_input_grad[1]) else None
         return dlogits.to(logits.dtype), dbias, None, None
 
 
