@@ -248,6 +248,7 @@ namespace kf2 {
 int launch_gemm_2cta(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb,
                      int ldc, int ldr, int a_mn, int b_mn, int out_f32, int accumulate, int num_sms,
                      cudaStream_t stream, int* status);
+float gemm_pair_cost(int M, int N, int num_sms);
 }
 
 namespace kf2 {
@@ -375,6 +376,13 @@ int kf_gemm_bf16(const void* A, const void* B, void* C, const void* R, int M, in
     // pairs pay off once there are enough 256x256 tiles to fill the machine a few times over
     const long long pair_tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
     mode = pair_tiles >= 2LL * (num_sms / 2) ? 2 : 1;
+    // Between one and two rounds of pairs, K-major B: both forms take two rounds, and a narrower pair tile makes them shorter
+    // (1554 x 4096 from 4096 and 11008: 250 -> 223 us for the two).  With at most one round the single-CTA tiles stay ahead
+    // (1777 rows, 2048 columns: 60 us against 68 for a layer's products).
+    if (mode == 1 && !b_mn && pair_tiles > num_sms / 2) {
+      const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+      if (kf2::gemm_pair_cost(M, N, num_sms) < 1.1f * BN * float((tiles + num_sms - 1) / num_sms)) mode = 2;
+    }
   }
   if (mode == 2)
     return kf2::launch_gemm_2cta(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, out_f32, accumulate, num_sms,

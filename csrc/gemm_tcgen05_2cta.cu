@@ -7,6 +7,12 @@
 // Per CTA and k-block only 32 KB are loaded (half of what the single-CTA 128x256 tile needs for the
 // same math per SM), which leaves room for 6 pipeline stages.
 //
+// With B in its K-major form the tile of a plain product is tile_n columns wide (a multiple of 32 from 128 to 256, chosen per
+// launch): with 256-wide tiles a product of, say, 7 x 16 tiles takes two rounds of the 74 pairs and leaves half of the second one
+// idle; 224 columns make it 133 tiles of 0.88 the length in the same two rounds.  The order of every sum over K is the same for all
+// widths.  An MN-major B keeps 256: half a narrower tile is no whole number of its 64-column chunks, and the loads of the
+// neighbour's columns cost more than the fuller last round gave (weight gradients of a 7B block 2640 -> 3175 us).
+//
 // Synchronisation (all waits bounded, see common.cuh):
 //   full[s]    leader only: armed by the leader's producer with the bytes of BOTH CTAs; the peer's TMA
 //              loads complete on the leader's barrier (peer bit of the barrier address cleared)
@@ -113,7 +119,7 @@ template <bool A_MN, bool B_MN, typename OutT, int SWIGLU = 0, bool GATHER = fal
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GATHER ? THREADS_GATHER : THREADS, 1)
 kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ WeightSegs ws,
                           OutT* __restrict__ C, const OutT* __restrict__ R, int M, int N, int K, int ldc, int ldr,
-                          int accumulate, int* status, RopeArgs rope, const __grid_constant__ GatherArgs ga) {
+                          int accumulate, int* status, RopeArgs rope, int tile_n_arg, const __grid_constant__ GatherArgs ga) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t bar_base = smem_base + STAGES * STAGE_BYTES;
@@ -132,7 +138,9 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
   const int pair = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
   const int m_blocks = (M + TILE_M - 1) / TILE_M;
-  const int n_blocks = SWIGLU == 1 ? (N + HALF_N - 1) / HALF_N : (N + TILE_N - 1) / TILE_N;
+  const int tile_n = SWIGLU == 0 && !B_MN && !GATHER ? tile_n_arg : TILE_N;
+  const int half_n = tile_n >> 1;  // columns (rows of B) each CTA of the pair loads
+  const int n_blocks = SWIGLU == 1 ? (N + HALF_N - 1) / HALF_N : (N + tile_n - 1) / tile_n;
   const int num_tiles = SWIGLU == 4 ? m_blocks * (m_blocks + 1) / 2 : m_blocks * n_blocks;
   const int k_blocks = (K + BK - 1) / BK;
   // gathering variant: column tiles are the slow index (a weight row block is consumed completely soon after it
@@ -191,7 +199,7 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
         const TileCoord tc = tile_at(t);
         const int m0 = tc.m * TILE_M + int(rank) * CTA_M;
         const int n_op = SWIGLU == 1 ? tc.n * HALF_N + int(rank) * N  // leader: gate rows, peer: the matching up rows
-                                     : tc.n * TILE_N + int(rank) * HALF_N;
+                                     : tc.n * tile_n + int(rank) * half_n;
         // matrix that holds these operand rows, and the first of them inside it
         const int sg = B_MN ? 0 : int(n_op >= ws.start[1]) + int(n_op >= ws.start[2]);
         const CUtensorMap* map_b = &ws.map[sg];
@@ -210,7 +218,7 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
           const uint32_t a_dst = smem_base + s * STAGE_BYTES;
           const uint32_t b_dst = a_dst + A_BYTES;
           const uint32_t lead_full = full_bar(s) & PEER_BIT_MASK;
-          if (leader) mbar_expect_tx(full_bar(s), 2 * STAGE_BYTES);
+          if (leader) mbar_expect_tx(full_bar(s), 2 * (A_BYTES + half_n * BK * 2));
           const int k0 = kb * BK;
           if (!A_MN) {
             tma_load_2d_pair(a_dst, &map_a, lead_full, k0, m0);
@@ -238,7 +246,7 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
     if (lane == 0 && leader) {
-      constexpr uint32_t idesc = umma_idesc_bf16(TILE_M, TILE_N, A_MN, B_MN);
+      const uint32_t idesc = umma_idesc_bf16(TILE_M, tile_n, A_MN, B_MN);
       int it = 0, tile_iter = 0;
       bool ok = true;
       for (int t = pair; t < num_tiles && ok; t += num_pairs, ++tile_iter) {
@@ -283,8 +291,8 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
       const int row = tc.m * TILE_M + int(rank) * CTA_M + quarter * 32 + lane;
       GuChunk gu_next;
       if constexpr (SWIGLU == 3) {  // the first pre-activations travel while the tile's products are still running
-        const __nv_bfloat16* gu_row = reinterpret_cast<const __nv_bfloat16*>(R) + size_t(row) * ldr + tc.n * TILE_N;
-        gu_next = load_gu_chunk(gu_row, gu_row + N, row < M ? N - tc.n * TILE_N : 0);
+        const __nv_bfloat16* gu_row = reinterpret_cast<const __nv_bfloat16*>(R) + size_t(row) * ldr + tc.n * tile_n;
+        gu_next = load_gu_chunk(gu_row, gu_row + N, row < M ? min(tile_n, N - tc.n * tile_n) : 0);
       }
       if (!mbar_wait(tfull_bar(acc), acc_ph, status, KF_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
@@ -293,20 +301,20 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
         // SwiGLU backward in the epilogue of the down projection's input-gradient GEMM: the accumulator is
         // dh[rows, F] (never written); R = the saved pre-activations [rows, 2F] (gate | up), C = d[gate | up]
         // [rows, 2F] (may be the same buffer: every element is read and written by one thread).
-        const int col0 = tc.n * TILE_N;
+        const int col0 = tc.n * tile_n, width = min(tile_n, N - col0);
         const __nv_bfloat16* gu_row = reinterpret_cast<const __nv_bfloat16*>(R) + size_t(row) * ldr + col0;
         __nv_bfloat16* d_row = reinterpret_cast<__nv_bfloat16*>(C) + size_t(row) * ldc + col0;
 #pragma unroll 1
-        for (int c = 0; c < TILE_N / 32; ++c) {
+        for (int c = 0; c * 32 < width; ++c) {
           uint32_t v[32];
           tmem_ld_32x32(t_row + c * 32, v);
           // chunk c + 1 is fetched while chunk c is worked on: without it the eight load latencies of a row, not the
           // products, set the pace of a K = 4096 tile
           const GuChunk gu_now = gu_next;
-          if (c + 1 < TILE_N / 32)
-            gu_next = load_gu_chunk(gu_row + (c + 1) * 32, gu_row + N + (c + 1) * 32, row < M ? N - (col0 + (c + 1) * 32) : 0);
+          if ((c + 1) * 32 < width)
+            gu_next = load_gu_chunk(gu_row + (c + 1) * 32, gu_row + N + (c + 1) * 32, row < M ? width - (c + 1) * 32 : 0);
           tmem_ld_wait();
-          const int valid = min(32, N - (col0 + c * 32));
+          const int valid = min(32, width - c * 32);
           if (row < M && valid > 0) swiglu_bwd_chunk(v, gu_now, d_row + c * 32, d_row + N + c * 32, valid);
         }
         tc_fence_before();
@@ -431,15 +439,15 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
         if (lane == 0) arrive_on_cta(tempty_bar(acc), 0);
         continue;
       }
-      const int col0 = tc.n * TILE_N;
+      const int col0 = tc.n * tile_n, width = min(tile_n, N - col0);
       OutT* c_row = C + size_t(row) * ldc + col0;
       const OutT* r_row = R ? R + size_t(row) * ldr + col0 : nullptr;
 #pragma unroll 1
-      for (int c = 0; c < TILE_N / 32; ++c) {
+      for (int c = 0; c * 32 < width; ++c) {
         uint32_t v[32];
         tmem_ld_32x32(t_row + c * 32, v);
         tmem_ld_wait();
-        const int valid = min(32, N - (col0 + c * 32));
+        const int valid = min(32, width - c * 32);
         if (row < M && valid > 0)
           store_chunk<OutT>(c_row + c * 32, v, valid, accumulate != 0, r_row ? r_row + c * 32 : nullptr);
       }
@@ -511,6 +519,34 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
   }
 }
 
+// Tile width for an (M, N) product and what it costs: rounds of tiles over the pairs, times the columns of a tile, times a
+// penalty for narrow tiles, whose operand bytes per MMA cycle exceed those of a 256-wide tile (64 per SM and clock): 10 % for
+// the 96 of a 128-wide one, which is what a single-CTA 128 x 256 tile needs and loses against a pair.  A narrower tile has to
+// save 4 %: less is within what the model leaves out.
+static int pick_tile_n(int M, int N, int pairs, float* cost_out) {
+  const int m_blocks = (M + TILE_M - 1) / TILE_M;
+  int best = TILE_N;
+  float best_cost = 3.4e38f;
+  for (int tn = TILE_N; tn >= 128; tn -= 32) {
+    const long long tiles = (long long)m_blocks * ((N + tn - 1) / tn);
+    const long long rounds = (tiles + pairs - 1) / pairs;
+    const float bytes_per_clk = (128.f + 0.5f * tn) * 64.f / tn;
+    const float cost = float(rounds) * tn * (1.f + 0.1f * (bytes_per_clk - 64.f) / 32.f);
+    if (cost < best_cost * (best == TILE_N ? 0.96f : 1.f)) {
+      best = tn;
+      best_cost = cost;
+    }
+  }
+  if (cost_out) *cost_out = best_cost;
+  return best;
+}
+// The same measure for the best pair launch of an (M, N) product (one column of a 256-row tile per pair = 1).
+float gemm_pair_cost(int M, int N, int num_sms) {
+  float c = 3.4e38f;
+  if (num_sms >= 2) pick_tile_n(M, N, num_sms / 2, &c);
+  return c;
+}
+
 static WeightSegs one_piece(const CUtensorMap& m) {
   return WeightSegs{{m, m, m}, {0, 0x7fffffff, 0x7fffffff}};
 }
@@ -521,7 +557,9 @@ static int launch(const void* A, const void* B, void* C, const void* R, int M, i
   CUtensorMap ma, mb;
   int rc = A_MN ? make_map_2d_bf16(&ma, A, K, M, lda, 64, BK) : make_map_2d_bf16(&ma, A, M, K, lda, BK, CTA_M);
   if (rc) return 100 + rc;
-  rc = B_MN ? make_map_2d_bf16(&mb, B, K, N, ldb, 64, BK) : make_map_2d_bf16(&mb, B, N, K, ldb, BK, HALF_N);
+  int pairs = num_sms / 2;
+  const int tile_n = B_MN ? TILE_N : pick_tile_n(M, N, pairs, nullptr);
+  rc = B_MN ? make_map_2d_bf16(&mb, B, K, N, ldb, 64, BK) : make_map_2d_bf16(&mb, B, N, K, ldb, BK, tile_n / 2);
   if (rc) return 200 + rc;
   auto kern = kf_gemm_bf16_tcgen05_2cta<A_MN, B_MN, OutT>;
   static bool attr_set = false;
@@ -530,12 +568,12 @@ static int launch(const void* A, const void* B, void* C, const void* R, int M, i
     if (e != cudaSuccess) return 300 + (int)e;
     attr_set = true;
   }
-  const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N);
-  int pairs = num_sms / 2;
+  const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + tile_n - 1) / tile_n);
   if (tiles < pairs) pairs = tiles;
   kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, one_piece(mb), reinterpret_cast<OutT*>(C),
                                                    reinterpret_cast<const OutT*>(R), M, N, K, ldc, ldr, accumulate,
-                                                   status, RopeArgs{nullptr, nullptr, 1, 0, 64}, GatherArgs{});
+                                                   status, RopeArgs{nullptr, nullptr, 1, 0, 64}, tile_n,
+                                                   GatherArgs{});
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
@@ -566,7 +604,7 @@ int launch_gemm_swiglu_2cta(const void* A, const void* Wg, const void* Wu, void*
   if (tiles < pairs) pairs = tiles;
   kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, ws, reinterpret_cast<__nv_bfloat16*>(H),
                                                    reinterpret_cast<const __nv_bfloat16*>(GU), M, F, K, ldh, ldgu, 0, status,
-                                                   RopeArgs{nullptr, nullptr, 1, 0, 64}, GatherArgs{});
+                                                   RopeArgs{nullptr, nullptr, 1, 0, 64}, TILE_N, GatherArgs{});
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
@@ -606,7 +644,7 @@ int launch_gemm_rope_2cta(const void* A, const void* const* W, const int* rows, 
   int pairs = num_sms / 2;
   if (tiles < pairs) pairs = tiles;
   kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, ws, reinterpret_cast<__nv_bfloat16*>(C), nullptr, M, N, K, ldc, 0, 0,
-                                                   status, RopeArgs{cosT, sinT, S, rope_cols, hd}, GatherArgs{});
+                                                   status, RopeArgs{cosT, sinT, S, rope_cols, hd}, TILE_N, GatherArgs{});
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
@@ -638,7 +676,7 @@ int launch_gemm_symm_2cta(int x_mn, const void* X, void* C, const void* R, int n
     }                                                                                                                \
     kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, one_piece(mb), reinterpret_cast<__nv_bfloat16*>(C),                    \
                                                      reinterpret_cast<const __nv_bfloat16*>(R), n, n, K, ldc, ldr, 0, \
-                                                     status, ra, GatherArgs{});                                      \
+                                                     status, ra, TILE_N, GatherArgs{});                              \
   }
   if (x_mn) KF2_SYMM_LAUNCH(true) else KF2_SYMM_LAUNCH(false)
 #undef KF2_SYMM_LAUNCH
@@ -701,7 +739,7 @@ int launch_gemm_gather_2cta(int epi, const void* A, void* C, const void* R, int 
     }                                                                                                                \
     kern<<<pairs * 2, THREADS_GATHER, SMEM_BYTES, stream>>>(ma, one_piece(mb), reinterpret_cast<__nv_bfloat16*>(C),  \
                                                             reinterpret_cast<const __nv_bfloat16*>(R), M, N, K, ldc, ldr, \
-                                                            0, status, ra, ga);                                      \
+                                                            0, status, ra, TILE_N, ga);                              \
   }
   if (epi == 0) KF2_GATHER_LAUNCH(0) else if (epi == 1) KF2_GATHER_LAUNCH(1) else if (epi == 2) KF2_GATHER_LAUNCH(2) else return 6;
 #undef KF2_GATHER_LAUNCH
@@ -730,7 +768,7 @@ int launch_gemm_swiglu_bwd_2cta(const void* DY, const void* W, const void* GU, v
   if (tiles < pairs) pairs = tiles;
   kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, one_piece(mb), reinterpret_cast<__nv_bfloat16*>(DGU),
                                                    reinterpret_cast<const __nv_bfloat16*>(GU), M, F, K, ldgu, ldgu, 0, status,
-                                                   RopeArgs{nullptr, nullptr, 1, 0, 64}, GatherArgs{});
+                                                   RopeArgs{nullptr, nullptr, 1, 0, 64}, TILE_N, GatherArgs{});
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
@@ -767,7 +805,7 @@ int launch_gemm_stacked_k_2cta(const void* A, const void* const* W, const int* r
   int pairs = num_sms / 2;
   if (tiles < pairs) pairs = tiles;
   kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, ws, reinterpret_cast<__nv_bfloat16*>(C), nullptr, M, N, K, ldc, 0, 0,
-                                                   status, RopeArgs{nullptr, nullptr, 1, 0, 64}, GatherArgs{});
+                                                   status, RopeArgs{nullptr, nullptr, 1, 0, 64}, TILE_N, GatherArgs{});
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
