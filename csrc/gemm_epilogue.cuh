@@ -75,44 +75,87 @@ __device__ __forceinline__ void swiglu_chunk(uint32_t (&g)[32], const uint32_t (
   }
 }
 
-// The saved pre-activations of one 32-column chunk of one row (loaded ahead of their use).
-struct GuChunk {
-  uint4 g[4], u[4];
+// ---- 32 rows x 32 columns of a warp between registers (one row per lane) and global memory, through shared memory.
+// A lane that reads or writes its own row touches 32 different lines per 16-byte instruction and half a sector of each;
+// four lanes per row move 64 contiguous bytes, eight rows per instruction.  `box`: 2 KB of shared memory of this warp,
+// 16-byte chunk q of row r at slot q ^ (r / 2 % 4) of its 64 bytes (no bank conflicts either way).  Grouped products: SwiGLU
+// gradients of 8 experts of 2048 x 7168 over 4096 rows 156 -> 142 us, of 64 of 2048 x 1408 over 10 662 rows 133 -> 122.
+__device__ __forceinline__ uint32_t box_row_chunk(uint32_t box, int row, int q) {
+  return box + uint32_t(row * 64 + ((q ^ ((row >> 1) & 3)) << 4));
+}
+__device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+struct Rows32 {
+  uint4 q[4];  // as moved: chunk lane % 4 of rows lane / 4 + 8 i; or, after an exchange, the four chunks of row `lane`
 };
-__device__ __forceinline__ GuChunk load_gu_chunk(const __nv_bfloat16* gate_row, const __nv_bfloat16* up_row, int valid_cols) {
-  GuChunk r;
+// `src`: first row and column of the box; rows / cols: how many of the 32 exist (the rest reads as zero).
+__device__ __forceinline__ Rows32 load_rows32(const __nv_bfloat16* src, size_t ld, int lane, int rows, int cols) {
+  Rows32 r;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = i * 8 + (lane >> 2), ch = lane & 3;
+    r.q[i] = row < rows && ch * 8 < cols ? *reinterpret_cast<const uint4*>(src + row * ld + ch * 8) : make_uint4(0, 0, 0, 0);
+  }
+  return r;
+}
+// moved layout -> the lane's own row
+__device__ __forceinline__ Rows32 to_own_row(uint32_t box, int lane, const Rows32& m) {
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) sts128(box_row_chunk(box, i * 8 + (lane >> 2), lane & 3), m.q[i]);
+  __syncwarp();
+  Rows32 r;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) r.q[q] = lds128(box_row_chunk(box, lane, q));
+  return r;
+}
+__device__ __forceinline__ void store_rows32(uint32_t box, int lane, const Rows32& own, __nv_bfloat16* dst, size_t ld, int rows,
+                                             int cols) {
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < 4; ++q) sts128(box_row_chunk(box, lane, q), own.q[q]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = i * 8 + (lane >> 2), ch = lane & 3;
+    if (row < rows && ch * 8 < cols) *reinterpret_cast<uint4*>(dst + row * ld + ch * 8) = lds128(box_row_chunk(box, row, ch));
+  }
+}
+__device__ __forceinline__ Rows32 pack_row32(const uint32_t (&v)[32]) {
+  Rows32 r;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const bool in = q * 8 < valid_cols;
-    r.g[q] = in ? *reinterpret_cast<const uint4*>(gate_row + q * 8) : make_uint4(0, 0, 0, 0);
-    r.u[q] = in ? *reinterpret_cast<const uint4*>(up_row + q * 8) : make_uint4(0, 0, 0, 0);
+    const uint32_t* f = v + q * 8;
+    r.q[q] = make_uint4(pack_bf16(__uint_as_float(f[0]), __uint_as_float(f[1])), pack_bf16(__uint_as_float(f[2]), __uint_as_float(f[3])),
+                        pack_bf16(__uint_as_float(f[4]), __uint_as_float(f[5])), pack_bf16(__uint_as_float(f[6]), __uint_as_float(f[7])));
   }
   return r;
 }
 
-// SwiGLU backward on one 32-column chunk: `dh` holds the gradient of the hidden activation (fp32 accumulator values),
-// `gu` the saved bf16 pre-activations of these 32 hidden units, dgate_row / dup_row receive the gradients (they may be the
-// memory `gu` was loaded from: every element is read and written by one thread).
-// The incoming gradient is rounded to bf16 first, like the two-kernel path.
-__device__ __forceinline__ void swiglu_bwd_chunk(const uint32_t (&dh)[32], const GuChunk& gu, __nv_bfloat16* dgate_row,
-                                                 __nv_bfloat16* dup_row, int valid_cols) {
+// SwiGLU backward on one 32-column chunk of one row: `dh` holds the gradient of the hidden activation (fp32 accumulator
+// values), gate / up the saved bf16 pre-activations; they are replaced by the gradients.  The incoming gradient is rounded to
+// bf16 first, like the two-kernel path.
+__device__ __forceinline__ void swiglu_bwd_row(const uint32_t (&dh)[32], Rows32& gate, Rows32& up) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    if (q * 8 >= valid_cols) break;
-    const uint4 gq = gu.g[q], uq = gu.u[q];
-    const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w}, uw[4] = {uq.x, uq.y, uq.z, uq.w};
-    uint32_t dg[4], du[4];
+    uint32_t gw[4] = {gate.q[q].x, gate.q[q].y, gate.q[q].z, gate.q[q].w}, uw[4] = {up.q[q].x, up.q[q].y, up.q[q].z, up.q[q].w};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float2 g2 = unpack_bf16(gw[e]), u2 = unpack_bf16(uw[e]);
       const float d0 = __bfloat162float(__float2bfloat16(__uint_as_float(dh[q * 8 + 2 * e])));
       const float d1 = __bfloat162float(__float2bfloat16(__uint_as_float(dh[q * 8 + 2 * e + 1])));
       const float s0 = 1.f / (1.f + __expf(-g2.x)), s1 = 1.f / (1.f + __expf(-g2.y));
-      du[e] = pack_bf16(d0 * g2.x * s0, d1 * g2.y * s1);
-      dg[e] = pack_bf16(d0 * u2.x * s0 * (1.f + g2.x * (1.f - s0)), d1 * u2.y * s1 * (1.f + g2.y * (1.f - s1)));
+      uw[e] = pack_bf16(d0 * g2.x * s0, d1 * g2.y * s1);
+      gw[e] = pack_bf16(d0 * u2.x * s0 * (1.f + g2.x * (1.f - s0)), d1 * u2.y * s1 * (1.f + g2.y * (1.f - s1)));
     }
-    *reinterpret_cast<uint4*>(dgate_row + q * 8) = make_uint4(dg[0], dg[1], dg[2], dg[3]);
-    *reinterpret_cast<uint4*>(dup_row + q * 8) = make_uint4(du[0], du[1], du[2], du[3]);
+    gate.q[q] = make_uint4(gw[0], gw[1], gw[2], gw[3]);
+    up.q[q] = make_uint4(uw[0], uw[1], uw[2], uw[3]);
   }
 }
 

@@ -39,7 +39,8 @@ constexpr int CTA_M = 128, TILE_M = 256, TILE_N = 256, HALF_N = 128, BK = 64, ST
 constexpr int A_BYTES = CTA_M * BK * 2, B_BYTES = HALF_N * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int THREADS = 192, TMEM_COLS = 512;
 constexpr int MAX_EXPERTS = 256;
-constexpr size_t SMEM = size_t(STAGES) * STAGE_BYTES + 1024 + 256 + (MAX_EXPERTS + 1) * 4;
+constexpr int BOX_BYTES = 2048;  // rows of an epilogue warp on their way to or from global memory; two per warp
+constexpr size_t SMEM = size_t(STAGES) * STAGE_BYTES + 8 * BOX_BYTES + 1024 + 256 + (MAX_EXPERTS + 1) * 4;
 
 using Tile = tilemath::GroupedTile;
 
@@ -57,7 +58,8 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
                              long long ldc, long long ldgu, int accumulate, int* status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t bar_base = smem_base + STAGES * STAGE_BYTES;
+  const uint32_t box_smem = smem_base + STAGES * STAGE_BYTES;
+  const uint32_t bar_base = box_smem + 8 * BOX_BYTES;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
   auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + a); };
@@ -192,60 +194,59 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
     for (int t = pair; t < num_tiles && ok; t += num_pairs, ++tile_iter) {
       const Tile tl = tilemath::grouped_decode(t, n_blocks, tile_start, offsets, E, TILE_M);
       const int acc = tile_iter & 1;
-      const int r = int(rank) * CTA_M + quarter * 32 + lane;  // row inside the 256-row tile
-      const int col0 = tl.nb * TN;
-      GuChunk gu_next;
+      const int r0 = int(rank) * CTA_M + quarter * 32;  // first row of this warp inside the 256-row tile
+      const int rows = max(0, min(32, tl.valid - r0));  // how many of its 32 rows belong to the expert
+      const int col0 = tl.nb * TN, width = min(TN, N - col0);
+      const uint32_t box = box_smem + uint32_t(quarter * 2) * BOX_BYTES, box2 = box + BOX_BYTES;
+      __nv_bfloat16* c0 = C + size_t(tl.row0 + r0) * ldc + col0;
+      __nv_bfloat16* gu0 = GU ? GU + size_t(tl.row0 + r0) * ldgu + col0 : nullptr;
+      Rows32 g_next, u_next;
       if constexpr (EPI == 2) {  // the first pre-activations travel while the tile's products are still running
-        const __nv_bfloat16* gu_row = GU + size_t(tl.row0 + r) * ldgu + col0;
-        gu_next = load_gu_chunk(gu_row, gu_row + N, r < tl.valid ? N - col0 : 0);
+        g_next = load_rows32(gu0, ldgu, lane, rows, width);
+        u_next = load_rows32(gu0 + N, ldgu, lane, rows, width);
       }
       if (!mbar_wait(tfull_bar(acc), (tile_iter >> 1) & 1, status, KF_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       const uint32_t t_row = tmem_base + (uint32_t(quarter * 32) << 16) + acc * TILE_N;
-      __nv_bfloat16* c_row = C + size_t(tl.row0 + r) * ldc + col0;
-      if constexpr (EPI == 2) {
-        // SwiGLU backward: the accumulator is dh[rows, F] (never written); GU = the saved pre-activations [rows, 2F]
-        // (gate | up), C = d[gate | up] [rows, 2F] (may be the same buffer: every element is read and written by one
-        // thread)
-        const __nv_bfloat16* gu_row = GU + size_t(tl.row0 + r) * ldgu + col0;
 #pragma unroll 1
-        for (int c = 0; c < TILE_N / 32; ++c) {
+      for (int c = 0; c * 32 < width; ++c) {
+        const int cols = min(32, width - c * 32);
+        if constexpr (EPI == 2) {
+          // SwiGLU backward: the accumulator is dh[rows, F] (never written); GU = the saved pre-activations [rows, 2F]
+          // (gate | up), C = d[gate | up] [rows, 2F] (may be the same buffer: a warp reads a chunk before it writes it, and
+          // no other warp touches its rows)
           uint32_t v[32];
           tmem_ld_32x32(t_row + c * 32, v);
-          const GuChunk gu_now = gu_next;  // chunk c + 1 is fetched while chunk c is worked on
-          if (c + 1 < TILE_N / 32)
-            gu_next = load_gu_chunk(gu_row + (c + 1) * 32, gu_row + N + (c + 1) * 32, r < tl.valid ? N - (col0 + (c + 1) * 32) : 0);
+          const Rows32 g_now = g_next, u_now = u_next;  // chunk c + 1 is fetched while chunk c is worked on
+          if ((c + 1) * 32 < width) {
+            g_next = load_rows32(gu0 + (c + 1) * 32, ldgu, lane, rows, width - (c + 1) * 32);
+            u_next = load_rows32(gu0 + N + (c + 1) * 32, ldgu, lane, rows, width - (c + 1) * 32);
+          }
+          Rows32 g = to_own_row(box, lane, g_now), u = to_own_row(box2, lane, u_now);
           tmem_ld_wait();
-          const int valid_cols = min(32, N - (col0 + c * 32));
-          if (r < tl.valid && valid_cols > 0) swiglu_bwd_chunk(v, gu_now, c_row + c * 32, c_row + N + c * 32, valid_cols);
-        }
-      } else if constexpr (SWIGLU) {
-        __nv_bfloat16* gu_row = GU ? GU + size_t(tl.row0 + r) * ldgu + col0 : nullptr;
-#pragma unroll 1
-        for (int c = 0; c < TN / 32; ++c) {
+          swiglu_bwd_row(v, g, u);
+          store_rows32(box, lane, g, c0 + c * 32, ldc, rows, cols);
+          store_rows32(box2, lane, u, c0 + N + c * 32, ldc, rows, cols);
+        } else if constexpr (SWIGLU) {
           uint32_t g[32], u[32];
           tmem_ld_32x32(t_row + c * 32, g);
           tmem_ld_32x32(t_row + TN + c * 32, u);
           tmem_ld_wait();
-          const int valid_cols = min(32, N - (col0 + c * 32));
-          if (r < tl.valid && valid_cols > 0) {
-            if (gu_row) {
-              store_chunk<__nv_bfloat16>(gu_row + c * 32, g, valid_cols, false, nullptr);
-              store_chunk<__nv_bfloat16>(gu_row + N + c * 32, u, valid_cols, false, nullptr);
-            }
-            swiglu_chunk(g, u);
-            store_chunk<__nv_bfloat16>(c_row + c * 32, g, valid_cols, false, nullptr);
+          if (gu0) {
+            store_rows32(box, lane, pack_row32(g), gu0 + c * 32, ldgu, rows, cols);
+            store_rows32(box2, lane, pack_row32(u), gu0 + N + c * 32, ldgu, rows, cols);
           }
-        }
-      } else {
-#pragma unroll 1
-        for (int c = 0; c < TILE_N / 32; ++c) {
+          swiglu_chunk(g, u);
+          store_rows32(box, lane, pack_row32(g), c0 + c * 32, ldc, rows, cols);
+        } else {
           uint32_t v[32];
           tmem_ld_32x32(t_row + c * 32, v);
           tmem_ld_wait();
-          const int valid_cols = min(32, N - (col0 + c * 32));
-          if (r < tl.valid && valid_cols > 0)
-            store_chunk<__nv_bfloat16>(c_row + c * 32, v, valid_cols, accumulate != 0, nullptr);
+          if (accumulate) {
+            if (lane < rows) store_chunk<__nv_bfloat16>(c0 + size_t(lane) * ldc + c * 32, v, cols, true, nullptr);
+          } else {
+            store_rows32(box, lane, pack_row32(v), c0 + c * 32, ldc, rows, cols);
+          }
         }
       }
       tc_fence_before();
