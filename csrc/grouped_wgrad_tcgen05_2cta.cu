@@ -10,15 +10,18 @@
 // The ragged tail: the last 64-row block of an expert usually runs into the next expert's rows, and every CTA has to
 // zero those rows of ITS OWN shared-memory stage before the MMAs read it.  Two hand-over protocols therefore:
 //   full 64-row blocks   as in gemm_tcgen05_2cta.cu: both CTAs' TMA bytes are counted on the leader's full[s]
-//   the tail block       (at most one per tile) each CTA's loads complete on its own full[s]; the peer's MMA warp waits
-//                        for it, zeroes its tail rows, fences them towards the async proxy and arrives (remote,
-//                        release) on the leader's ready[s]; the leader does the same with its own stage and its
-//                        issuing thread then waits for ready[s] (cluster-scope acquire) before the MMAs
+//   the tail block       (at most one per tile) each CTA's loads complete on its own tail[s]; warp 6 of each CTA waits
+//                        for it, zeroes the foreign rows of its own stage up to the next multiple of 16 (only those
+//                        k-steps are issued), fences them towards the async proxy and arrives (release) on the leader's
+//                        ready[s]; the issuing thread waits for both arrivals (cluster-scope acquire) before the MMAs.
+//                        The ring runs ahead of the MMAs, so the rows are usually clear before their turn; zeroing all
+//                        64 rows inside the issuing warp held up every tile by about as long as a k-block (64 experts of
+//                        2048 x 1408 over 10 662 rows: 484 -> 397 us for three gradients; 8 of 2048 x 7168: 464 -> 414).
 //   empty[s]             both CTAs: released by the leader's tcgen05.commit, multicast to the pair
 //   tfull[a] / tempty[a] as in gemm_tcgen05_2cta.cu (8 epilogue-warp arrivals on the leader)
-// The peer's full[s] and the leader's ready[s] complete one phase per TAIL use of stage s only; both sides keep one
-// parity bit per stage for them.  (Relaying every block through the peer's warp was measured 2.4x slower than the
-// single-CTA kernel.)
+// full[s] completes a phase per full block in stage s, tail[s] and ready[s] one per tail block; every side waits for all
+// phases of its barriers in order and keeps one parity bit per stage for each.
+// (Relaying every block through the peer's warp was measured 2.4x slower than the single-CTA kernel.)
 // All waits are bounded; TMA loads carry no cluster multicast.
 //
 // Epilogue.  An expert's reduction is short (167 rows = 3 k-blocks of 0.4 us for 64 experts over 10 662 rows), so the tile's
@@ -26,7 +29,7 @@
 // lines: 5.5 us per tile.  Each epilogue warp therefore stages 32 rows x 64 columns in shared memory (two 4 KB buffers,
 // 128-byte swizzle: no bank conflicts) and one lane stores them with TMA: whole lines, asynchronously, clipped at the
 // expert's last row and column by the 3-D tensor map.  The sixth ring stage paid for the buffers.  Three gradients of 64 experts of
-// 2048 x 1408 over 10 662 rows: 685 -> 480 us; of 8 experts of 2048 x 7168 over 4096 rows: 530 -> 441 us.
+// 2048 x 1408 over 10 662 rows: 685 -> 480 us with this; of 8 experts of 2048 x 7168 over 4096 rows: 530 -> 441 us.
 //
 // Replaces the per-expert weight-gradient products that autograd derives for the padded `torch._grouped_mm`
 // call of the reference (kempnerforge/model/moe.py:20-145).
@@ -44,7 +47,7 @@ constexpr int CTA_M = 128, TILE_M = 256, TILE_N = 256, HALF_N = 128, BK = 64, ST
 constexpr int BLOCK_BYTES = 64 * BK * 2;  // one {64 columns, BK rows} box
 constexpr int A_BYTES = (CTA_M / 64) * BLOCK_BYTES, B_BYTES = (HALF_N / 64) * BLOCK_BYTES;
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int THREADS = 192, TMEM_COLS = 512;
+constexpr int THREADS = 224, TMEM_COLS = 512;
 constexpr int OUT_BYTES = 32 * 64 * 2;  // one staged box: 32 rows x 64 columns of one epilogue warp
 constexpr size_t SMEM = size_t(STAGES) * STAGE_BYTES + 4 * 2 * OUT_BYTES + 1024 + 256;
 
@@ -61,10 +64,11 @@ kf_grouped_wgrad_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const _
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
   auto ready_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + s); };
-  auto tfull_bar = [&](int a) { return bar_base + 8u * (3 * STAGES + a); };
-  auto tempty_bar = [&](int a) { return bar_base + 8u * (3 * STAGES + 2 + a); };
-  const uint32_t drain_bar = bar_base + 8u * (3 * STAGES + 4);
-  const uint32_t tmem_slot = bar_base + 8u * (3 * STAGES + 5);
+  auto tail_bar = [&](int s) { return bar_base + 8u * (3 * STAGES + s); };
+  auto tfull_bar = [&](int a) { return bar_base + 8u * (4 * STAGES + a); };
+  auto tempty_bar = [&](int a) { return bar_base + 8u * (4 * STAGES + 2 + a); };
+  const uint32_t drain_bar = bar_base + 8u * (4 * STAGES + 4);
+  const uint32_t tmem_slot = bar_base + 8u * (4 * STAGES + 5);
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -79,7 +83,8 @@ kf_grouped_wgrad_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const _
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
-      mbar_init(ready_bar(s), 1);
+      mbar_init(ready_bar(s), 2);  // the tail warps of both CTAs
+      mbar_init(tail_bar(s), 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);
@@ -104,7 +109,8 @@ kf_grouped_wgrad_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const _
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (one per CTA)
     if (lane == 0) {
-      int it = 0, peer_tails = 0;
+      int it = 0;
+      uint32_t full_parity = 0, tail_parity = 0, last_tail = 0;  // bit s: next phases of stage s, kind of its last use
       bool ok = true;
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
         const Tile tl = tilemath::wgrad_decode(t, m_blocks, n_blocks, TILE_M, TILE_N, offsets);
@@ -116,14 +122,17 @@ kf_grouped_wgrad_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const _
           const uint32_t a_dst = smem_base + s * STAGE_BYTES, b_dst = a_dst + A_BYTES;
           const int row = tl.row0 + kb * BK;
           if (tl.rows - kb * BK < BK) {
-            // tail block: every CTA's bytes complete on its own barrier (its MMA warp zeroes the foreign rows)
-            mbar_expect_tx(full_bar(s), STAGE_BYTES);
+            // tail block: every CTA's bytes complete on its own tail barrier (its warp 6 zeroes the foreign rows)
+            mbar_expect_tx(tail_bar(s), STAGE_BYTES);
 #pragma unroll
-            for (int c = 0; c < CTA_M / 64; ++c) tma_load_2d(a_dst + c * BLOCK_BYTES, &map_a, full_bar(s), m0 + 64 * c, row);
+            for (int c = 0; c < CTA_M / 64; ++c) tma_load_2d(a_dst + c * BLOCK_BYTES, &map_a, tail_bar(s), m0 + 64 * c, row);
 #pragma unroll
-            for (int c = 0; c < HALF_N / 64; ++c) tma_load_2d(b_dst + c * BLOCK_BYTES, &map_b, full_bar(s), n0 + 64 * c, row);
-            if (!leader) ++peer_tails;
+            for (int c = 0; c < HALF_N / 64; ++c) tma_load_2d(b_dst + c * BLOCK_BYTES, &map_b, tail_bar(s), n0 + 64 * c, row);
+            tail_parity ^= 1u << s;
+            last_tail |= 1u << s;
           } else {
+            full_parity ^= 1u << s;
+            last_tail &= ~(1u << s);
             const uint32_t lead_full = full_bar(s) & PEER_BIT_MASK;
             if (leader) mbar_expect_tx(full_bar(s), 2 * STAGE_BYTES);
 #pragma unroll
@@ -135,78 +144,45 @@ kf_grouped_wgrad_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const _
       }
       // Copies into this CTA's shared memory are complete once the stages they filled were consumed (empty flipped)
       // or, on the error path, once the barrier that counts them flipped.
-      if (leader)
-        for (int j = max(0, it - STAGES); j < it; ++j)
-          mbar_wait(full_bar(j % STAGES), (j / STAGES) & 1, status, KF_ERR_WAIT_DRAIN);
-      (void)peer_tails;
+      for (int s = 0; s < min(it, STAGES); ++s) {
+        if ((last_tail >> s) & 1) mbar_wait(tail_bar(s), ((tail_parity >> s) & 1) ^ 1, status, KF_ERR_WAIT_DRAIN);
+        else if (leader) mbar_wait(full_bar(s), ((full_parity >> s) & 1) ^ 1, status, KF_ERR_WAIT_DRAIN);
+      }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ stage preparation (both CTAs) + MMA issue (leader)
-    // the whole warp walks the loop (the tail rows of a stage are zeroed by all lanes); the peer's warp only acts on
-    // tail blocks
-    constexpr uint32_t idesc = umma_idesc_bf16(TILE_M, TILE_N, true, true);
-    int it = 0, tile_iter = 0;
-    uint32_t tail_parity = 0;  // bit s: parity of the next tail use of stage s (peer: its full[s]; leader: ready[s])
-    bool ok = true;
-    auto zero_tail = [&](uint32_t a_src, int valid) {
-      // rows valid..63 of every 64-column block belong to another expert (or to nobody)
-      constexpr int BLOCKS = STAGE_BYTES / BLOCK_BYTES;
-      for (int i = lane; i < tilemath::tail_chunks(valid, BK, BLOCKS); i += 32) {
-        const uint32_t addr = a_src + tilemath::tail_chunk_offset(i, valid, BK, BLOCK_BYTES);
-        asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(0u) : "memory");
-      }
-      fence_async_smem();
-      __syncwarp();
-    };
-    for (int t = pair; t < num_tiles && ok; t += num_pairs, ++tile_iter) {
-      const Tile tl = tilemath::wgrad_decode(t, m_blocks, n_blocks, TILE_M, TILE_N, offsets);
-      const int k_blocks = (tl.rows + BK - 1) / BK;
-      const int acc = tile_iter & 1;
-      if (!leader) {
-        // peer: only the tail block (the last one, when the expert's row count is not a multiple of 64)
-        const int valid = tl.rows - (k_blocks - 1) * BK;
-        if (k_blocks > 0 && valid < BK) {
-          const int s = (it + k_blocks - 1) % STAGES;
-          ok = __all_sync(0xffffffffu, mbar_wait(full_bar(s), (tail_parity >> s) & 1, status, KF_ERR_WAIT_FULL));
-          if (!ok) break;
-          tail_parity ^= 1u << s;
-          zero_tail(smem_base + s * STAGE_BYTES, valid);
-          if (lane == 0) arrive_on_cta(ready_bar(s), 0);  // this CTA's half of the stage is in place
-        }
-        it += k_blocks;
-        continue;
-      }
-      ok = __all_sync(0xffffffffu, mbar_wait(tempty_bar(acc), ((tile_iter >> 1) & 1) ^ 1, status, KF_ERR_WAIT_TMEM_EMPTY));
-      if (!ok) break;
-      tc_fence_after();
-      const uint32_t d_tmem = tmem_base + acc * TILE_N;
-      for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-        const int s = it % STAGES;
-        const uint32_t ph = (it / STAGES) & 1;
-        ok = __all_sync(0xffffffffu, mbar_wait(full_bar(s), ph, status, KF_ERR_WAIT_FULL));
-        if (!ok) break;
-        const uint32_t a_src = smem_base + s * STAGE_BYTES, b_src = a_src + A_BYTES;
-        const int valid = tl.rows - kb * BK;
-        const bool tail = valid < BK;
-        if (tail) zero_tail(a_src, valid);
-        if (lane == 0) {
-          if (tail && !mbar_wait_cluster(ready_bar(s), (tail_parity >> s) & 1, status, KF_ERR_WAIT_FULL)) ok = false;
-          if (ok) {
-            tc_fence_after();
-#pragma unroll
-            for (int k = 0; k < BK / UMMA_K; ++k)
-              mma_pair_f16(d_tmem, umma_desc_sw128(a_src + k * (UMMA_K * 128), BLOCK_BYTES, 1024),
-                           umma_desc_sw128(b_src + k * (UMMA_K * 128), BLOCK_BYTES, 1024), idesc, (kb | k) != 0);
-            commit_pair(empty_bar(s));
+    // ------------------------------------------------------------ MMA issuer (leader CTA only)
+    if (leader && lane == 0) {
+      constexpr uint32_t idesc = umma_idesc_bf16(TILE_M, TILE_N, true, true);
+      int it = 0, tile_iter = 0;
+      uint32_t full_parity = 0, ready_parity = 0;  // bit s: parity of the next full / tail use of stage s
+      bool ok = true;
+      for (int t = pair; t < num_tiles && ok; t += num_pairs, ++tile_iter) {
+        const Tile tl = tilemath::wgrad_decode(t, m_blocks, n_blocks, TILE_M, TILE_N, offsets);
+        const int k_blocks = (tl.rows + BK - 1) / BK;
+        const int acc = tile_iter & 1;
+        if (!mbar_wait(tempty_bar(acc), ((tile_iter >> 1) & 1) ^ 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + acc * TILE_N;
+        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+          const int s = it % STAGES;
+          const int valid = tl.rows - kb * BK;
+          if (valid >= BK) {
+            if (!mbar_wait(full_bar(s), (full_parity >> s) & 1, status, KF_ERR_WAIT_FULL)) { ok = false; break; }
+            full_parity ^= 1u << s;
+          } else {
+            if (!mbar_wait_cluster(ready_bar(s), (ready_parity >> s) & 1, status, KF_ERR_WAIT_FULL)) { ok = false; break; }
+            ready_parity ^= 1u << s;
           }
+          tc_fence_after();
+          const uint32_t a_src = smem_base + s * STAGE_BYTES, b_src = a_src + A_BYTES;
+          const int steps = valid < BK ? (valid + UMMA_K - 1) / UMMA_K : BK / UMMA_K;
+          for (int k = 0; k < steps; ++k)
+            mma_pair_f16(d_tmem, umma_desc_sw128(a_src + k * (UMMA_K * 128), BLOCK_BYTES, 1024),
+                         umma_desc_sw128(b_src + k * (UMMA_K * 128), BLOCK_BYTES, 1024), idesc, (kb | k) != 0);
+          commit_pair(empty_bar(s));
         }
-        if (tail) {
-          tail_parity ^= 1u << s;
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-        }
+        if (ok) commit_pair(tfull_bar(acc));
       }
-      if (ok && lane == 0) commit_pair(tfull_bar(acc));
     }
     if (leader && lane == 0) {
       // every MMA must have retired before either CTA gives up its shared or tensor memory
@@ -215,6 +191,30 @@ kf_grouped_wgrad_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const _
       mbar_wait(drain_bar, 0, status, KF_ERR_WAIT_DRAIN);
     }
     __syncwarp();
+  } else if (warp == 6) {
+    // ------------------------------------------------------------ tail rows of this CTA's stages (both CTAs)
+    int it = 0;
+    uint32_t tail_parity = 0;  // bit s: parity of the next tail use of stage s
+    for (int t = pair; t < num_tiles; t += num_pairs) {
+      const Tile tl = tilemath::wgrad_decode(t, m_blocks, n_blocks, TILE_M, TILE_N, offsets);
+      const int k_blocks = (tl.rows + BK - 1) / BK;
+      const int valid = tl.rows - (k_blocks - 1) * BK;
+      if (k_blocks > 0 && valid < BK) {
+        const int s = (it + k_blocks - 1) % STAGES;
+        if (!__all_sync(0xffffffffu, mbar_wait(tail_bar(s), (tail_parity >> s) & 1, status, KF_ERR_WAIT_FULL))) break;
+        tail_parity ^= 1u << s;
+        constexpr int BLOCKS = STAGE_BYTES / BLOCK_BYTES;
+        const int end = (valid + UMMA_K - 1) / UMMA_K * UMMA_K;  // rows the MMAs will read
+        for (int i = lane; i < tilemath::tail_chunks(valid, end, BLOCKS); i += 32) {
+          const uint32_t addr = smem_base + s * STAGE_BYTES + tilemath::tail_chunk_offset(i, valid, end, BLOCK_BYTES);
+          asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(0u) : "memory");
+        }
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) arrive_on_cta(ready_bar(s), 0);  // this CTA's half of the stage is in place
+      }
+      it += k_blocks;
+    }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5 of both CTAs)
     const int quarter = warp & 3;
