@@ -3,9 +3,16 @@
 //   C[M,N] (+)= alpha * A8[M,K] * B8[N,K]^T      alpha = 1 / (scale_a * scale_b), read from device memory
 //
 // A8 / B8 are e4m3 or e5m2 bytes with the reduction dim contiguous ("K-major"); tensorwise scales are
-// computed on the device (abs-max -> scale) and never visit the host.  Same persistent warp-specialised
-// structure as the bf16 kernel: TMA producer warp, one MMA-issuing thread, four epilogue warps, 4-stage
-// 128B-swizzled ring (128 K-elements per stage), double-buffered fp32 accumulators in tensor memory.
+// computed on the device (abs-max -> scale) and never visit the host.  Structure and synchronisation of the bf16
+// pair kernel (gemm_tcgen05_2cta.cu): a CTA pair owns a 256 x tile_n tile, each CTA loads 128 rows of A and half of
+// B's rows (128 K-bytes per stage, 6 stages, 128B swizzle), the leader issues tcgen05.mma cta_group::2, both
+// epilogues read their own tensor memory (two accumulators) and store through shared memory.
+//
+// What bounds it: the operand stream.  8-bit products take half the tensor cycles of 16-bit ones per byte pair, so a
+// 128 x 256 tile of a single CTA asks for 96 bytes per SM and clock; the pair needs 64.  tile_n follows the rounds of
+// tiles over the pairs (2000 x 14 336: 448 tiles of 256 columns are 6.05 rounds, 512 of 224 are 6.9).
+// Single-CTA 128 x 256 tiles -> pairs: 2000 x 14 336 from 4096 103 -> 88 us, 14 336 x 4096 from 2000 163 -> 115, 8192 x 6144 from
+// 4096 154 -> 135 (3.05 PFLOP/s), 1 x 4096 from 4096 20.5 -> 20.5; the same bits.
 // The transposed operands that dgrad / wgrad need are written by the cast kernel itself (one read of the
 // bf16 source produces the row-major and the transposed fp8 copy), so every GEMM runs K-major.
 //
@@ -13,24 +20,29 @@
 // kempnerforge/distributed/parallel.py:125-174): e4m3 for activations and weights, e5m2 for gradients.
 #include "common.cuh"
 #include "gemm_epilogue.cuh"
+#include "pair_common.cuh"
 #include "tile_math.h"
 #include <cuda_fp8.h>
 
 namespace kf {
 namespace f8 {
 
-constexpr int BM = 128;
-constexpr int BN = 256;
+using namespace kf::pairops;
+
+constexpr int CTA_M = 128;    // rows of A per CTA
+constexpr int TILE_M = 256;   // rows per CTA pair
+constexpr int MAX_N = 256;    // columns of the widest tile
 constexpr int BK = 128;       // fp8 elements = bytes per row of a stage
 constexpr int UMMA_K = 32;    // K per tcgen05.mma for 8-bit inputs
-constexpr int STAGES = 4;
-constexpr int A_STAGE_BYTES = BM * BK;  // 16 KB
-constexpr int B_STAGE_BYTES = BN * BK;  // 32 KB
-constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
+constexpr int STAGES = 6;
+constexpr int A_BYTES = CTA_M * BK;            // 16 KB
+constexpr int B_BYTES = (MAX_N / 2) * BK;      // 16 KB
+constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int THREADS = 192;
 constexpr int TMEM_COLS = 512;
 constexpr int GROUP_M = 8;
-constexpr size_t SMEM = size_t(STAGES) * STAGE_BYTES + 1024 + 256;
+constexpr int BOX_BYTES = 2048;  // one staged 32 x 32 box per epilogue warp
+constexpr size_t SMEM = size_t(STAGES) * STAGE_BYTES + 4 * BOX_BYTES + 1024 + 256;
 
 // Instruction descriptor for kind::f8f6f4: fp32 accumulate, A/B format 0 = e4m3, 1 = e5m2, both K-major.
 __host__ __device__ constexpr uint32_t idesc_f8(int m, int n, int a_fmt, int b_fmt) {
@@ -38,27 +50,14 @@ __host__ __device__ constexpr uint32_t idesc_f8(int m, int n, int a_fmt, int b_f
          (uint32_t(m >> 4) << 24);
 }
 
-__device__ __forceinline__ void tc_mma_f8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void tile_coord(int t, int m_blocks, int n_blocks, int& tile_m, int& tile_n) {
-  tilemath::raster(t, m_blocks, n_blocks, GROUP_M, tile_m, tile_n);
-}
-
-__global__ void __launch_bounds__(THREADS, 1)
-kf_gemm_fp8_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                    __nv_bfloat16* __restrict__ C, int M, int N, int K, int ldc, int accumulate, int a_fmt,
-                    int b_fmt, const float* __restrict__ scale_a, const float* __restrict__ scale_b, int* status) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+kf_gemm_fp8_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                         __nv_bfloat16* __restrict__ C, int M, int N, int K, int ldc, int accumulate, int a_fmt, int b_fmt,
+                         int tile_n, const float* __restrict__ scale_a, const float* __restrict__ scale_b, int* status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t bar_base = smem_base + STAGES * STAGE_BYTES;
+  const uint32_t box_smem = smem_base + STAGES * STAGE_BYTES;
+  const uint32_t bar_base = box_smem + 4 * BOX_BYTES;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
   auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + a); };
@@ -70,8 +69,12 @@ kf_gemm_fp8_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int m_blocks = (M + BM - 1) / BM;
-  const int n_blocks = (N + BN - 1) / BN;
+  const uint32_t rank = cluster_ctarank();
+  const bool leader = rank == 0;
+  const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+  const int half_n = tile_n >> 1;
+  const int m_blocks = (M + TILE_M - 1) / TILE_M;
+  const int n_blocks = (N + tile_n - 1) / tile_n;
   const int num_tiles = m_blocks * n_blocks;
   const int k_blocks = (K + BK - 1) / BK;
 
@@ -82,7 +85,7 @@ kf_gemm_fp8_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);
-      mbar_init(tempty_bar(a), 4);
+      mbar_init(tempty_bar(a), 8);  // four epilogue warps of each CTA
     }
     mbar_init(drain_bar, 1);
     mbar_fence_init();
@@ -90,102 +93,119 @@ kf_gemm_fp8_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     tma_prefetch_desc(&map_b);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, TMEM_COLS);
-    tmem_relinquish();
+    tmem_alloc_pair(tmem_slot, TMEM_COLS);
+    tmem_relinquish_pair();
   }
   tc_fence_before();
   __syncthreads();
+  cluster_sync_all();  // both CTAs' barriers exist before anyone signals across the pair
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
 
   if (warp == 0) {
+    // ------------------------------------------------------------ TMA producer (one per CTA)
     if (lane == 0) {
       int it = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      for (int t = pair; t < num_tiles && ok; t += num_pairs) {
         int tm, tn;
-        tile_coord(t, m_blocks, n_blocks, tm, tn);
+        tilemath::raster(t, m_blocks, n_blocks, GROUP_M, tm, tn);
+        const int m0 = tm * TILE_M + int(rank) * CTA_M, n0 = tn * tile_n + int(rank) * half_n;
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait(empty_bar(s), ph ^ 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
           const uint32_t a_dst = smem_base + s * STAGE_BYTES;
-          mbar_expect_tx(full_bar(s), STAGE_BYTES);
-          tma_load_2d(a_dst, &map_a, full_bar(s), kb * BK, tm * BM);
-          tma_load_2d(a_dst + A_STAGE_BYTES, &map_b, full_bar(s), kb * BK, tn * BN);
+          const uint32_t lead_full = full_bar(s) & PEER_BIT_MASK;
+          if (leader) mbar_expect_tx(full_bar(s), 2 * (A_BYTES + half_n * BK));
+          tma_load_2d_pair(a_dst, &map_a, lead_full, kb * BK, m0);
+          tma_load_2d_pair(a_dst + A_BYTES, &map_b, lead_full, kb * BK, n0);
         }
       }
-      for (int j = max(0, it - STAGES); j < it; ++j)
-        mbar_wait(full_bar(j % STAGES), (j / STAGES) & 1, status, KF_ERR_WAIT_DRAIN);
+      // copies into this CTA's shared memory are complete once their stages were consumed or, on the error path, once
+      // the leader's full barrier flipped
+      if (leader)
+        for (int j = max(0, it - STAGES); j < it; ++j)
+          mbar_wait(full_bar(j % STAGES), (j / STAGES) & 1, status, KF_ERR_WAIT_DRAIN);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = idesc_f8(BM, BN, a_fmt, b_fmt);
+    // ------------------------------------------------------------ MMA issuer (leader CTA only)
+    if (lane == 0 && leader) {
+      const uint32_t idesc = idesc_f8(TILE_M, tile_n, a_fmt, b_fmt);
       int it = 0, tile_iter = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tile_iter) {
+      for (int t = pair; t < num_tiles && ok; t += num_pairs, ++tile_iter) {
         const int acc = tile_iter & 1;
         const uint32_t acc_ph = (tile_iter >> 1) & 1;
         if (!mbar_wait(tempty_bar(acc), acc_ph ^ 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const uint32_t d_tmem = tmem_base + acc * MAX_N;
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait(full_bar(s), ph, status, KF_ERR_WAIT_FULL)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_src = smem_base + s * STAGE_BYTES;
-          const uint32_t b_src = a_src + A_STAGE_BYTES;
+          const uint32_t b_src = a_src + A_BYTES;
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             // 32 one-byte elements per step = 32 B along the swizzled 128 B row
-            tc_mma_f8(d_tmem, umma_desc_sw128(a_src + k * UMMA_K, 16, 1024),
-                      umma_desc_sw128(b_src + k * UMMA_K, 16, 1024), idesc, (kb | k) != 0);
+            mma_pair_f8(d_tmem, umma_desc_sw128(a_src + k * UMMA_K, 16, 1024),
+                        umma_desc_sw128(b_src + k * UMMA_K, 16, 1024), idesc, (kb | k) != 0);
           }
-          tc_commit(empty_bar(s));
+          commit_pair(empty_bar(s));
         }
-        if (ok) tc_commit(tfull_bar(acc));
+        if (ok) commit_pair(tfull_bar(acc));
       }
-      tc_commit(drain_bar);
+      // every MMA must have retired before either CTA gives up its shared or tensor memory
+      asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(drain_bar)
+                   : "memory");
       mbar_wait(drain_bar, 0, status, KF_ERR_WAIT_DRAIN);
     }
   } else {
+    // ------------------------------------------------------------ epilogue (warps 2..5 of both CTAs)
     const int quarter = warp & 3;
+    const uint32_t box = box_smem + uint32_t(quarter) * BOX_BYTES;
     const float alpha = 1.0f / (scale_a[0] * scale_b[0]);
     int tile_iter = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tile_iter) {
+    for (int t = pair; t < num_tiles && ok; t += num_pairs, ++tile_iter) {
       int tm, tn;
-      tile_coord(t, m_blocks, n_blocks, tm, tn);
+      tilemath::raster(t, m_blocks, n_blocks, GROUP_M, tm, tn);
       const int acc = tile_iter & 1;
       const uint32_t acc_ph = (tile_iter >> 1) & 1;
       if (!mbar_wait(tfull_bar(acc), acc_ph, status, KF_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
-      const int row = tm * BM + quarter * 32 + lane;
-      const int col0 = tn * BN;
-      const uint32_t t_row = tmem_base + (uint32_t(quarter * 32) << 16) + acc * BN;
-      __nv_bfloat16* c_row = C + size_t(row) * ldc + col0;
+      const int row0 = tm * TILE_M + int(rank) * CTA_M + quarter * 32;  // this warp's rows, and how many exist
+      const int rows = max(0, min(32, M - row0));
+      const int col0 = tn * tile_n, width = min(tile_n, N - col0);
+      const uint32_t t_row = tmem_base + (uint32_t(quarter * 32) << 16) + acc * MAX_N;
+      __nv_bfloat16* c0 = C + size_t(row0) * ldc + col0;
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = 0; c * 32 < width; ++c) {
         uint32_t v[32];
         tmem_ld_32x32(t_row + c * 32, v);
         tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-        const int valid = min(32, N - (col0 + c * 32));
-        if (row < M && valid > 0) store_chunk<__nv_bfloat16>(c_row + c * 32, v, valid, accumulate != 0, nullptr);
+        const int valid = min(32, width - c * 32);
+        if (!accumulate)
+          store_rows32(box, lane, pack_row32(v), c0 + c * 32, ldc, rows, valid);
+        else if (lane < rows)
+          store_chunk<__nv_bfloat16>(c0 + size_t(lane) * ldc + c * 32, v, valid, true, nullptr);
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(tempty_bar(acc));
+      if (lane == 0) arrive_on_cta(tempty_bar(acc), 0);
     }
   }
 
   tc_fence_before();
   __syncthreads();
+  cluster_sync_all();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    tmem_dealloc_pair(tmem_base, TMEM_COLS);
   }
 }
 
@@ -377,21 +397,24 @@ int kf_gemm_fp8(const void* A, const void* B, void* C, int M, int N, int K, long
   using namespace kf;
   using namespace kf::f8;
   if ((lda & 15) || (ldb & 15) || (ldc & 7) || M <= 0 || N <= 0 || K <= 0) return 5;
+  if (num_sms < 2) return 5;
+  int pairs = num_sms / 2;
+  const int tile_n = pair_tile_width(M, N, pairs, nullptr);
   CUtensorMap ma, mb;
-  int rc = make_map_2d_u8(&ma, A, M, K, lda, BM);
+  int rc = make_map_2d_u8(&ma, A, M, K, lda, CTA_M);
   if (rc) return 100 + rc;
-  rc = make_map_2d_u8(&mb, B, N, K, ldb, BN);
+  rc = make_map_2d_u8(&mb, B, N, K, ldb, tile_n / 2);
   if (rc) return 200 + rc;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kf_gemm_fp8_tcgen05, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+    cudaError_t e = cudaFuncSetAttribute(kf_gemm_fp8_tcgen05_2cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
     if (e != cudaSuccess) return 300 + (int)e;
     attr_set = true;
   }
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  const int grid = tiles < num_sms ? tiles : num_sms;
-  kf_gemm_fp8_tcgen05<<<grid, THREADS, SMEM, (cudaStream_t)stream>>>(
-      ma, mb, reinterpret_cast<__nv_bfloat16*>(C), M, N, K, ldc, accumulate, a_fmt, b_fmt,
+  const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + tile_n - 1) / tile_n);
+  if (tiles < pairs) pairs = tiles;
+  kf_gemm_fp8_tcgen05_2cta<<<pairs * 2, THREADS, SMEM, (cudaStream_t)stream>>>(
+      ma, mb, reinterpret_cast<__nv_bfloat16*>(C), M, N, K, ldc, accumulate, a_fmt, b_fmt, tile_n,
       reinterpret_cast<const float*>(scale_a), reinterpret_cast<const float*>(scale_b),
       reinterpret_cast<int*>(kf_status_device_ptr()));
   cudaError_t e = cudaGetLastError();

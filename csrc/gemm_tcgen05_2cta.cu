@@ -533,31 +533,10 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
   }
 }
 
-// Tile width for an (M, N) product and what it costs: rounds of tiles over the pairs, times the columns of a tile, times a
-// penalty for narrow tiles, whose operand bytes per MMA cycle exceed those of a 256-wide tile (64 per SM and clock): 10 % for
-// the 96 of a 128-wide one, which is what a single-CTA 128 x 256 tile needs and loses against a pair.  A narrower tile has to
-// save 4 %: less is within what the model leaves out.
-static int pick_tile_n(int M, int N, int pairs, float* cost_out) {
-  const int m_blocks = (M + TILE_M - 1) / TILE_M;
-  int best = TILE_N;
-  float best_cost = 3.4e38f;
-  for (int tn = TILE_N; tn >= 128; tn -= 32) {
-    const long long tiles = (long long)m_blocks * ((N + tn - 1) / tn);
-    const long long rounds = (tiles + pairs - 1) / pairs;
-    const float bytes_per_clk = (128.f + 0.5f * tn) * 64.f / tn;
-    const float cost = float(rounds) * tn * (1.f + 0.1f * (bytes_per_clk - 64.f) / 32.f);
-    if (cost < best_cost * (best == TILE_N ? 0.96f : 1.f)) {
-      best = tn;
-      best_cost = cost;
-    }
-  }
-  if (cost_out) *cost_out = best_cost;
-  return best;
-}
 // The same measure for the best pair launch of an (M, N) product (one column of a 256-row tile per pair = 1).
 float gemm_pair_cost(int M, int N, int num_sms) {
   float c = 3.4e38f;
-  if (num_sms >= 2) pick_tile_n(M, N, num_sms / 2, &c);
+  if (num_sms >= 2) pair_tile_width(M, N, num_sms / 2, &c);
   return c;
 }
 
@@ -572,7 +551,7 @@ static int launch(const void* A, const void* B, void* C, const void* R, int M, i
   int rc = A_MN ? make_map_2d_bf16(&ma, A, K, M, lda, 64, BK) : make_map_2d_bf16(&ma, A, M, K, lda, BK, CTA_M);
   if (rc) return 100 + rc;
   int pairs = num_sms / 2;
-  const int tile_n = B_MN ? TILE_N : pick_tile_n(M, N, pairs, nullptr);
+  const int tile_n = B_MN ? TILE_N : pair_tile_width(M, N, pairs, nullptr);
   rc = B_MN ? make_map_2d_bf16(&mb, B, K, N, ldb, 64, BK) : make_map_2d_bf16(&mb, B, N, K, ldb, BK, tile_n / 2);
   if (rc) return 200 + rc;
   auto kern = kf_gemm_bf16_tcgen05_2cta<A_MN, B_MN, OutT>;

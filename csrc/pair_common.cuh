@@ -36,6 +36,15 @@ __device__ __forceinline__ void mma_pair_f16(uint32_t d_tmem, uint64_t adesc, ui
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+__device__ __forceinline__ void mma_pair_f8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // Arrive on the barrier at the same shared-memory offset in both CTAs of the pair once all MMAs retired.
 __device__ __forceinline__ void commit_pair(uint32_t bar) {
   asm volatile(
@@ -84,6 +93,29 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
       }
     }
   }
+}
+
+// Tile width of a pair launch for an (M, N) product and what it costs: rounds of tiles over the pairs, times the columns of a
+// tile (multiples of 32 from 128 to 256, 256 rows), times a
+// penalty for narrow tiles, whose operand bytes per MMA cycle exceed those of a 256-wide tile (64 per SM and clock): 10 % for
+// the 96 of a 128-wide one, which is what a single-CTA 128 x 256 tile needs and loses against a pair.  A narrower tile has to
+// save 4 %: less is within what the model leaves out.
+inline int pair_tile_width(int M, int N, int pairs, float* cost_out) {
+  const int m_blocks = (M + 255) / 256;
+  int best = 256;
+  float best_cost = 3.4e38f;
+  for (int tn = 256; tn >= 128; tn -= 32) {
+    const long long tiles = (long long)m_blocks * ((N + tn - 1) / tn);
+    const long long rounds = (tiles + pairs - 1) / pairs;
+    const float bytes_per_clk = (128.f + 0.5f * tn) * 64.f / tn;
+    const float cost = float(rounds) * tn * (1.f + 0.1f * (bytes_per_clk - 64.f) / 32.f);
+    if (cost < best_cost * (best == 256 ? 0.96f : 1.f)) {
+      best = tn;
+      best_cost = cost;
+    }
+  }
+  if (cost_out) *cost_out = best_cost;
+  return best;
 }
 
 }  // namespace pairops
