@@ -99,11 +99,16 @@ __device__ __forceinline__ TileCoord tile_coord(int t, int m_blocks, int n_block
 // (or X^T X with MN-major operands), N = M.  Only the tiles on and above the diagonal are computed; every tile
 // above the diagonal is stored twice, as it is and transposed, so C comes out exactly symmetric at about half the
 // tensor-core work.  R must be symmetric as well (it is read at the untransposed position only).
+//
+// SWIGLU == 5 (fp32 partial sums, K-major A, MN-major B): the product of every tile is cut along K into `splits` units; unit
+// u = piece * tiles + tile writes its sum to C + piece * M * ldc.  The piece is the slow index, so the pairs work on (nearly) the
+// same k at a time and share the operand panels in L2; a cut of the last round alone puts them at different k and lost 40 %.
 struct RopeArgs {
   const float* cosT;  // [S][hd / 2]
   const float* sinT;
   int S, cols, hd;
   float alpha, beta, diag;  // SWIGLU == 4 only
+  int splits;               // SWIGLU == 5 only
 };
 
 // Weight operand made of up to three matrices stacked along N (q | k | v; SwiGLU == 1: gate and up): one tensor map each,
@@ -143,8 +148,12 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
   const int tile_n = SWIGLU == 0 && !B_MN && !GATHER ? tile_n_arg : TILE_N;
   const int half_n = tile_n >> 1;  // columns (rows of B) each CTA of the pair loads
   const int n_blocks = SWIGLU == 1 ? (N + HALF_N - 1) / HALF_N : (N + tile_n - 1) / tile_n;
-  const int num_tiles = SWIGLU == 4 ? m_blocks * (m_blocks + 1) / 2 : m_blocks * n_blocks;
+  const int num_tiles = SWIGLU == 4 ? m_blocks * (m_blocks + 1) / 2 : m_blocks * n_blocks * (SWIGLU == 5 ? rope.splits : 1);
   const int k_blocks = (K + BK - 1) / BK;
+  // k-blocks [k_begin(t), k_begin(t) + k_count(t)) of unit t
+  auto piece_of = [&](int t) { return SWIGLU == 5 ? t / (m_blocks * n_blocks) : 0; };
+  auto k_begin = [&](int t) { return SWIGLU == 5 ? int((long long)piece_of(t) * k_blocks / rope.splits) : 0; };
+  auto k_end = [&](int t) { return SWIGLU == 5 ? int((long long)(piece_of(t) + 1) * k_blocks / rope.splits) : k_blocks; };
   // gathering variant: column tiles are the slow index (a weight row block is consumed completely soon after it
   // arrived), rotated so that the tile holding this rank's own rows comes first
   auto tile_at = [&](int t) {
@@ -163,7 +172,7 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
       tc.n = nr + ga.n_tile_start;
       if (tc.n >= n_blocks) tc.n -= n_blocks;
     } else {
-      tc = tile_coord(t, m_blocks, n_blocks);
+      tc = tile_coord(SWIGLU == 5 ? t % (m_blocks * n_blocks) : t, m_blocks, n_blocks);
     }
     return tc;
   };
@@ -213,7 +222,7 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
             asm volatile("fence.proxy.async;" ::: "memory");  // generic-proxy stores -> this thread's TMA reads
           }
         }
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        for (int kb = k_begin(t), kb_end = k_end(t); kb < kb_end; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait(empty_bar(s), ph ^ 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
@@ -257,7 +266,7 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
         if (!mbar_wait(tempty_bar(acc), acc_ph ^ 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * TILE_N;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        for (int kb = k_begin(t), kb_end = k_end(t); kb < kb_end; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait(full_bar(s), ph, status, KF_ERR_WAIT_FULL)) { ok = false; break; }
@@ -270,7 +279,7 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
                                      : umma_desc_sw128(a_src + k * (UMMA_K * 2), 16, 1024);
             const uint64_t bd = B_MN ? umma_desc_sw128(b_src + k * (UMMA_K * 128), 64 * BK * 2, 1024)
                                      : umma_desc_sw128(b_src + k * (UMMA_K * 2), 16, 1024);
-            mma_pair_f16(d_tmem, ad, bd, idesc, (kb | k) != 0);
+            mma_pair_f16(d_tmem, ad, bd, idesc, ((kb - k_begin(t)) | k) != 0);
           }
           commit_pair(empty_bar(s));
         }
@@ -448,7 +457,7 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
         continue;
       }
       const int col0 = tc.n * tile_n, width = min(tile_n, N - col0);
-      OutT* c_row = C + size_t(row) * ldc + col0;
+      OutT* c_row = C + (SWIGLU == 5 ? size_t(piece_of(t)) * M * ldc : 0) + size_t(row) * ldc + col0;
       const OutT* r_row = R ? R + size_t(row) * ldr + col0 : nullptr;
 #pragma unroll 1
       for (int c = 0; c * 32 < width; ++c) {
@@ -803,6 +812,76 @@ int launch_gemm_stacked_k_2cta(const void* A, const void* const* W, const int* r
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
+// out[M][ldo] = bf16(sum over the pieces of ws[piece][M][N]), pieces in ascending order; 8 columns per thread.
+__global__ void __launch_bounds__(256) kf_sum_pieces(const float* __restrict__ ws, __nv_bfloat16* __restrict__ out, int M, int N,
+                                                     int ldo, int splits) {
+  const size_t per_row = N / 8, total = size_t(M) * per_row, plane = size_t(M) * N;
+  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
+    const size_t row = i / per_row, col = (i % per_row) * 8;
+    const float* p = ws + row * N + col;
+    float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+    for (int s = 1; s < splits; ++s) {
+      const float4 c = *reinterpret_cast<const float4*>(p + s * plane), d = *reinterpret_cast<const float4*>(p + s * plane + 4);
+      a.x += c.x; a.y += c.y; a.z += c.z; a.w += c.w;
+      b.x += d.x; b.y += d.y; b.z += d.z; b.w += d.w;
+    }
+    *reinterpret_cast<uint4*>(out + row * ldo + col) =
+        make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+  }
+}
+
+// Pieces along K for C[M, N] = A[M, K] B[K, N] (1 = leave it whole).  In clocks: a round of 256 x 256 tiles takes 8 per k on a
+// pair, a piece's partial sums cross memory twice (4 + 4 bytes at about 3500 bytes per clock).  At least 4096 k per piece, so
+// that filling and draining the ring stays below 2 %, and 5 % to gain.  2047 x 4096 over a vocabulary of 128 256: 128 tiles are
+// two rounds of 74 pairs, 86 % full; 4 pieces make it 7 quarter rounds, 99 % full: 1653 -> 1408 us, the 24 us of the sum included;
+// 100 x 4096 from 32 000 (16 tiles) 193 -> 77 us, 1 x 4096 from 128 256 702 -> 184.
+static int k_pieces(int M, int N, int K, int num_sms) {
+  if (num_sms < 2 || (N & 7)) return 1;
+  const int pairs = num_sms / 2;
+  const long long tiles = (long long)((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N);
+  const long long single = (long long)((M + CTA_M - 1) / CTA_M) * ((N + TILE_N - 1) / TILE_N);
+  const long long r_pair = (tiles + pairs - 1) / pairs, r_single = (single + num_sms - 1) / num_sms;
+  float best_cost = 0.95f * 8.f * float(K) * float(r_pair < r_single ? r_pair : r_single);
+  int best = 1;
+  for (int s = 2; s <= 8 && K / s >= 4096; ++s) {
+    const float cost = 8.f * float(K) * float((tiles * s + pairs - 1) / pairs) / float(s) + float(s) * float(M) * float(N) * (8.f / 3500.f);
+    if (cost < best_cost) {
+      best = s;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
+// C[M, N] (bf16) = A[M, K] B[K, N] by way of ws[splits][M][N] fp32.
+static int launch_split_k(const void* A, const void* B, void* C, void* ws, int M, int N, int K, int lda, int ldb, int ldc,
+                          int splits, int num_sms, cudaStream_t stream, int* status) {
+  CUtensorMap ma, mb;
+  int rc = make_map_2d_bf16(&ma, A, M, K, lda, BK, CTA_M);
+  if (rc) return 100 + rc;
+  rc = make_map_2d_bf16(&mb, B, K, N, ldb, 64, BK);
+  if (rc) return 200 + rc;
+  auto kern = kf_gemm_bf16_tcgen05_2cta<false, true, float, 5>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    if (e != cudaSuccess) return 300 + (int)e;
+    attr_set = true;
+  }
+  const int units = ((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N) * splits;
+  int pairs = num_sms / 2;
+  if (units < pairs) pairs = units;
+  RopeArgs ra{};
+  ra.splits = splits;
+  kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, one_piece(mb), reinterpret_cast<float*>(ws), nullptr, M, N, K, N, 0, 0, status,
+                                                   ra, TILE_N, GatherArgs{});
+  const size_t chunks = size_t(M) * (N / 8), blocks = (chunks + 255) / 256;
+  kf_sum_pieces<<<(int)(blocks < size_t(num_sms) * 8 ? blocks : size_t(num_sms) * 8), 256, 0, stream>>>(
+      reinterpret_cast<const float*>(ws), reinterpret_cast<__nv_bfloat16*>(C), M, N, ldc, splits);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 400 + (int)e;
+}
+
 int launch_gemm_2cta(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb,
                      int ldc, int ldr, int a_mn, int b_mn, int out_f32, int accumulate, int num_sms,
                      cudaStream_t stream, int* status) {
@@ -817,3 +896,18 @@ int launch_gemm_2cta(const void* A, const void* B, void* C, const void* R, int M
 }
 
 }  // namespace kf2
+
+extern "C" {
+void* kf_status_device_ptr();
+
+// Number of pieces along K that kf_gemm_split_k_bf16 should be given for this product (1: use kf_gemm_bf16).
+int kf_gemm_k_pieces(int M, int N, int K, int num_sms) { return kf2::k_pieces(M, N, K, num_sms); }
+
+// C[M][ldc] (bf16) = A[M][lda] B[K][ldb]; ws: fp32 [splits][M][N].  N a multiple of 8, 2 <= splits <= K / 64.
+int kf_gemm_split_k_bf16(const void* A, const void* B, void* C, void* ws, int M, int N, int K, int lda, int ldb, int ldc, int splits,
+                         int num_sms, void* stream) {
+  if (M < 1 || N < 8 || K < 1 || (N & 7) || ((lda | ldb | ldc) & 7) || splits < 2 || splits > (K + 63) / 64 || num_sms < 2) return 5;
+  return kf2::launch_split_k(A, B, C, ws, M, N, K, lda, ldb, ldc, splits, num_sms, (cudaStream_t)stream,
+                             (int*)kf_status_device_ptr());
+}
+}

@@ -50,6 +50,8 @@ def available() -> bool:
 def _declare(L: ctypes.CDLL) -> None:
     vp, i, ll, f = c_void_p, c_int, c_longlong, c_float
     sigs = {
+        "kf_gemm_k_pieces": [i, i, i, i],
+        "kf_gemm_split_k_bf16": [vp, vp, vp, vp, i, i, i, i, i, i, i, i, vp],
         "kf_gemm_bf16": [vp, vp, vp, vp, i, i, i, i, i, i, i, i, i, i, i, i, i, vp],
         "kf_gemm_swiglu_bf16": [vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, vp],
         "kf_gemm_rope_bf16": [vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, vp, vp, i, i, i, i, vp],
@@ -194,6 +196,11 @@ def stack_rows(tensors):
 
 
 # --------------------------------------------------------------------------- GEMM
+# From this reduction length on (the input gradient of a vocabulary projection) the native rule for a split along K is asked; it
+# never splits into pieces shorter than half of it.
+SPLIT_K_MIN = 8192
+
+
 def gemm(
     a: torch.Tensor,
     b: torch.Tensor,
@@ -246,6 +253,14 @@ def gemm(
         ldr = residual.stride(0)
         if ldr % (4 if out_f32 else 8) or residual.data_ptr() % 16:
             raise NativeKernelError("gemm residual must be 16-byte aligned")
+    if (K >= SPLIT_K_MIN and mode in (None, 0) and GEMM_MODE == 0 and a_kmajor and not b_kmajor and not out_f32 and not accumulate
+            and residual is None):
+        pieces = lib().kf_gemm_k_pieces(M, N, K, sm_count())
+        if pieces > 1:
+            ws = torch.empty((pieces, M, N), dtype=torch.float32, device=a.device)
+            _check(lib().kf_gemm_split_k_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), ws.data_ptr(), M, N, K, lda, ldb, ldc, pieces,
+                                              sm_count(), _stream()), "kf_gemm_split_k_bf16", 2)
+            return out
     code = lib().kf_gemm_bf16(
         a.data_ptr(), b.data_ptr(), out.data_ptr(), residual.data_ptr() if residual is not None else None,
         M, N, K, lda, ldb, ldc, ldr, 0 if a_kmajor else 1, 0 if b_kmajor else 1, int(out_f32), int(accumulate),
