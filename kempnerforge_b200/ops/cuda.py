@@ -297,6 +297,7 @@ def _weights3(weights):
 def gemm_rows(x2: torch.Tensor, weights, residual: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
     """x2 (M, K) times up to three (n_i, K) weights stacked along the output (+ ``residual``) -> bf16 (M, sum n_i).  With few
     rows the weights are read where they are; otherwise they are stacked for the tile kernels."""
+    assert 1 <= len(weights) <= 3, "more than three matrices have to be stacked first"
     m, k = x2.shape
     if len(weights) > 1 and residual is None and out is None and _separate_ok(x2, weights, 128) and not rows_adjacent(weights):
         # the rotary kernel with nothing to rotate: one tensor map per weight

@@ -80,7 +80,8 @@ class _LinearFn(torch.autograd.Function):
         x2 = x.reshape(-1, x.shape[-1])
         if not x2.is_contiguous():
             x2 = x2.contiguous()
-        y = cu.gemm(x2, weights[0]) if len(weights) == 1 or len(weights) > 3 else cu.gemm_rows(x2, weights)
+        # one matrix after stacking, or up to three that the kernels can read where they are
+        y = cu.gemm_rows(x2, weights) if len(weights) in (2, 3) else cu.gemm(x2, cu.stack_rows(weights))
         ctx.save_for_backward(x2, *weights)
         ctx.x_shape = x.shape
         return y.view(*x.shape[:-1], y.shape[-1])
