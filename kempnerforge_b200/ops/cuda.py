@@ -229,6 +229,7 @@ def gemm(
     M, K = (a.shape[0], a.shape[1]) if a_kmajor else (a.shape[1], a.shape[0])
     N, Kb = (b.shape[0], b.shape[1]) if b_kmajor else (b.shape[1], b.shape[0])
     assert K == Kb, f"inner dimensions differ: {K} vs {Kb}"
+    assert a.device == b.device, f"operands on {a.device} and {b.device}"
     lda, ldb = a.stride(0), b.stride(0)
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype or torch.bfloat16, device=a.device)
@@ -246,7 +247,7 @@ def gemm(
         return _gemm_rope(a, [b], out, rope)
     if (mode in (None, 0) and GEMM_MODE == 0 and _few_rows(M, N) and a_kmajor and b_kmajor and not out_f32
             and not accumulate and N % 8 == 0 and K % 8 == 0):
-        return gemm_rows(a, [b], residual, out)
+        return _stream_rows(a, [b], residual, out)
     ldr = 0
     if residual is not None:
         assert residual.shape == (M, N) and residual.dtype == out.dtype and residual.stride(1) == 1
@@ -287,6 +288,14 @@ def _ptr(t: torch.Tensor | None):
     return t.data_ptr() if t is not None else None
 
 
+def _plain_rows(w: torch.Tensor, device: torch.device) -> bool:
+    """A kernel can read the matrix by its address and row pitch: on its GPU, adjacent columns, rows that do not overlap, 16-byte
+    steps.  Anything else is left to the copy that stacks the matrices: the pitch alone would name other elements, the address
+    other memory."""
+    return (w.device == device and w.stride(1) == 1 and w.stride(0) >= w.shape[1] and w.stride(0) % 8 == 0
+            and w.data_ptr() % 16 == 0)
+
+
 def _weights3(weights):
     """(pointers, rows, row pitches) of up to three stacked matrices, padded with empty ones."""
     n = 3 - len(weights)
@@ -307,8 +316,14 @@ def gemm_rows(x2: torch.Tensor, weights, residual: torch.Tensor | None = None, o
         _check(lib().kf_gemm_rope_bf16(x2.data_ptr(), *ptrs, out.data_ptr(), m, *rows, k, x2.stride(0), pitch[0], n, None, None,
                                        1, 0, 64, sm_count(), _stream()), "kf_gemm_rope_bf16")
         return out
-    if not _few_rows(m, sum(w.shape[0] for w in weights)) or any(w.shape[0] % 8 or w.stride(0) % 8 or w.data_ptr() % 16 for w in weights) or k % 8:
+    if not _few_rows(m, sum(w.shape[0] for w in weights)) or any(w.shape[0] % 8 or not _plain_rows(w, x2.device) for w in weights) or k % 8:
         return gemm(x2, stack_rows(weights), residual=residual, out=out)
+    return _stream_rows(x2, weights, residual, out)
+
+
+def _stream_rows(x2: torch.Tensor, weights, residual: torch.Tensor | None, out: torch.Tensor | None) -> torch.Tensor:
+    """:func:`gemm_rows` on the weight-streaming kernel."""
+    m, k = x2.shape
     ptrs, rows, pitch = _weights3(weights)
     n = sum(rows)
     if out is None:
@@ -334,7 +349,7 @@ def _separate_ok(x2: torch.Tensor, weights, step: int) -> bool:
     tiles = -(-m // 256) * (-(-n // 256))
     return (tiles >= 2 * (sm_count() // 2) and n % 64 == 0 and x2.stride(0) % 8 == 0 and x2.data_ptr() % 16 == 0
             and all(w.shape[0] % step == 0 for w in weights[:-1])
-            and all(w.stride() == weights[0].stride() and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0 for w in weights))
+            and all(w.stride() == weights[0].stride() and _plain_rows(w, x2.device) for w in weights))
 
 
 def dgrad_rows(dy2: torch.Tensor, weights) -> torch.Tensor:
@@ -344,7 +359,7 @@ def dgrad_rows(dy2: torch.Tensor, weights) -> torch.Tensor:
     tiles = -(-m // 256) * (-(-k // 256))
     if (len(weights) in (2, 3) and not rows_adjacent(weights) and tiles >= 2 * (sm_count() // 2) and k % 8 == 0
             and dy2.stride(0) % 8 == 0 and dy2.data_ptr() % 16 == 0 and all(w.shape[0] % 64 == 0 for w in weights[:-1])
-            and all(w.stride() == weights[0].stride() and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0 for w in weights)):
+            and all(w.stride() == weights[0].stride() and _plain_rows(w, dy2.device) for w in weights)):
         out = torch.empty((m, k), dtype=torch.bfloat16, device=dy2.device)
         ptrs, rows, pitch = _weights3(weights)
         _check(lib().kf_gemm_dgrad_stacked_bf16(dy2.data_ptr(), *ptrs, out.data_ptr(), m, k, *rows, dy2.stride(0), pitch[0], k,

@@ -1,5 +1,7 @@
-"""Projections over several weight matrices.  On the CPU the native entries are replaced by functions that read memory as the
-kernels do: by address and row pitch."""
+"""Projections over several weight matrices: how many there are and how they lie in memory.
+
+The kernels read a matrix by its address and row pitch alone, so a weight they cannot describe has to be copied first.  On the
+CPU the native entries are replaced by functions that read memory exactly as the kernels do."""
 
 import ctypes
 
@@ -78,6 +80,14 @@ def _weights(form, rows, k, device="cpu"):
     for n in rows:
         if form == "dense":
             w = torch.randn(n, k, device=device, generator=g).bfloat16()
+        elif form == "columns":        # every second column: the row pitch alone says nothing about it
+            w = torch.randn(n, 2 * k, device=device, generator=g).bfloat16()[:, ::2]
+        elif form == "transposed":
+            w = torch.randn(k, n, 8, device=device, generator=g).bfloat16()[..., 0].t()
+        elif form == "one row":        # a row pitch of zero
+            w = torch.randn(1, k, device=device, generator=g).bfloat16().expand(n, k)
+        else:                          # rows cut out of a wider matrix
+            w = torch.randn(n, k + 24, device=device, generator=g).bfloat16()[:, 8 : 8 + k]
         out.append(w)
     return out
 
@@ -103,7 +113,7 @@ def _check(x, ws):
     assert _bounded(torch.cat(got[1:]), dy.t(), x)
 
 
-FORMS = ["dense"]
+FORMS = ["dense", "columns", "transposed", "one row", "cut"]
 
 
 @pytest.mark.parametrize("rows", [(16,) * 4, (8, 16, 24, 8, 8), (128, 64), (128, 128, 64)])
@@ -116,6 +126,9 @@ def test_every_weight_counts_whatever_its_layout(fake, rows, form, m):
 def test_dense_weights_are_still_read_where_they_are(fake):
     _check(torch.randn(600, 64).bfloat16(), _weights("dense", (128, 64), 64))
     assert fake.calls[0] == "separate"
+    fake.calls.clear()
+    _check(torch.randn(3, 64).bfloat16(), _weights("cut", (128, 64), 64))
+    assert fake.calls[0] == "few rows"
 
 
 def test_more_than_three_matrices_are_refused_by_the_kernels_front_end(fake):
@@ -123,6 +136,18 @@ def test_more_than_three_matrices_are_refused_by_the_kernels_front_end(fake):
 
     with pytest.raises(AssertionError):
         kc.gemm_rows(torch.randn(3, 64).bfloat16(), _weights("dense", (16,) * 4, 64))
+
+
+def test_a_matrix_on_another_device_is_refused_before_any_kernel(fake):
+    from kempnerforge_b200.ops import cuda as kc
+
+    x, w = torch.randn(3, 64).bfloat16(), _weights("dense", (128, 64), 64)
+    for ws in ([w[0], w[1].to("meta")], [w[0].to("meta"), w[1].to("meta")]):
+        with pytest.raises((AssertionError, RuntimeError, NotImplementedError)):
+            kc.gemm_rows(x, ws)
+        with pytest.raises((AssertionError, RuntimeError, NotImplementedError)):
+            kc.dgrad_rows(torch.randn(600, 192).bfloat16(), ws)
+    assert not fake.calls
 
 
 @pytest.mark.gpu
