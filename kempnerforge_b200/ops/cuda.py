@@ -383,11 +383,18 @@ def swiglu_rows(x2: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor) -> torch.T
     return swiglu_fwd(gemm_rows(x2, [wg, wu]))
 
 
+def rope_tables_ok(cos: torch.Tensor, sin: torch.Tensor) -> bool:
+    """The kernels with the rotation in their epilogue read fp32 tables 16 bytes at a time; tables that start elsewhere (slices
+    of a packed buffer) are left to the separate rotary kernel, which reads single values."""
+    return (cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
+            and (cos.data_ptr() | sin.data_ptr()) % 16 == 0)
+
+
 def _gemm_rope(x2: torch.Tensor, weights, out: torch.Tensor, rope: tuple) -> torch.Tensor:
     cos, sin, seq_len, rope_cols, hd = rope
     m, k = x2.shape
     assert out.dtype == torch.bfloat16
-    assert cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
+    assert rope_tables_ok(cos, sin)
     assert cos.shape[-1] == hd // 2 and cos.numel() >= seq_len * (hd // 2) and m % seq_len == 0
     ptrs, rows, pitch = _weights3(weights)
     _check(lib().kf_gemm_rope_bf16(x2.data_ptr(), *ptrs, out.data_ptr(), m, *rows, k, x2.stride(0), pitch[0], out.stride(0),
@@ -402,7 +409,7 @@ def qkv_rope(x2: torch.Tensor, weights, cos, sin, s: int, hd: int) -> torch.Tens
     m = x2.shape[0]
     n = wq.shape[0] + wk.shape[0] + wv.shape[0]
     rope_cols = wq.shape[0] + wk.shape[0]
-    if (m > SKINNY_MAX_ROWS and gemm_rope_supported(x2, wq, hd) and wk.shape[0] % hd == 0 and n % 256 == 0
+    if (m > SKINNY_MAX_ROWS and gemm_rope_supported(x2, wq, hd) and rope_tables_ok(cos, sin) and wk.shape[0] % hd == 0 and n % 256 == 0
             and wq.stride() == wk.stride() == wv.stride()
             and (rows_adjacent(weights) or (wq.shape[0] % 128 == 0 and wk.shape[0] % 128 == 0))):
         out = torch.empty((m, n), dtype=torch.bfloat16, device=x2.device)
@@ -1076,7 +1083,7 @@ def attn_bwd(dout, q, k, v, out, lse, causal: bool, doc_ids, scale: float, dq=No
     cos = sin = None
     if rope is not None:
         cos, sin = rope
-        assert sq == sk and cos.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
+        assert sq == sk and rope_tables_ok(cos, sin)
         assert cos.shape[-1] == hd // 2 and cos.numel() >= sq * (hd // 2)
     _check(
         lib().kf_attn_bwd_rope_bf16(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),

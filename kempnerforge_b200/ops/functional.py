@@ -377,7 +377,7 @@ def qkv_attention(x, wq, wk, wv, cos, sin, doc_ids, hd: int) -> torch.Tensor | N
     if (hd != 128 or not use_native(x) or not torch.is_grad_enabled() or x.dim() != 3 or x.shape[0] * x.shape[1] < 128
             or cos.dtype != torch.float32 or sin.dtype != torch.float32 or cos.dim() != 2 or cos.shape != sin.shape
             or cos.requires_grad or sin.requires_grad or cos.shape[0] < x.shape[1] or cos.shape[1] != hd // 2
-            or not (cos.is_cuda and cos.is_contiguous() and sin.is_contiguous()) or cos.data_ptr() % 16 or sin.data_ptr() % 16
+            or not (cos.is_cuda and _cuda().rope_tables_ok(cos, sin))
             or (doc_ids is not None and doc_ids.shape != x.shape[:2])):
         return None
     cu = _cuda()

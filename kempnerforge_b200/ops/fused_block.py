@@ -126,8 +126,8 @@ def _gather_plan(g, key: str, weights, x2):
 def _rope_fused(n1, w_qkv, cos, sin, s: int, hd: int) -> bool:
     """The rotary epilogue of the CTA-pair GEMM applies: fp32 (S, hd / 2) tables, whole sequences per row block,
     and a problem large enough for that kernel (small ones keep the separate in-place pass)."""
-    return (os.environ.get("KF_ROPE_EPILOGUE", "1") != "0" and cos.dtype == torch.float32 and cos.is_contiguous()
-            and sin.is_contiguous() and cos.dim() == 2 and cos.shape[0] >= s and cos.shape[1] == hd // 2
+    return (os.environ.get("KF_ROPE_EPILOGUE", "1") != "0" and kc.rope_tables_ok(cos, sin)
+            and cos.dim() == 2 and cos.shape[0] >= s and cos.shape[1] == hd // 2
             and n1.shape[0] % s == 0 and n1.shape[0] >= 256 and w_qkv.shape[0] % 256 == 0
             and kc.gemm_rope_supported(n1, w_qkv, hd))
 
@@ -265,7 +265,7 @@ class DenseBlockFn(torch.autograd.Function):
         dqkv4 = torch.empty_like(qkv4)
         if it["actx"][0] == "native":
             # dq | dk | dv land in their head ranges of the fused gradient, already through the inverse rotation
-            fused_rope = hd == 128 and cos.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
+            fused_rope = hd == 128 and kc.rope_tables_ok(cos, sin)
             kc.attn_bwd(dattn.view(b, s, h, hd), q, k, v, attn, it["actx"][1], True, None, 1.0 / math.sqrt(hd),
                         dq=dqkv4[:, :, :h], dk=dqkv4[:, :, h : h + hkv], dv=dqkv4[:, :, h + hkv :],
                         rope=(cos, sin) if fused_rope else None)
@@ -337,7 +337,7 @@ class AttnHalfFn(torch.autograd.Function):
         qkv4 = qkv.view(b, s, h + 2 * hkv, hd)
         q, k, v = qkv4[:, :, :h], qkv4[:, :, h : h + hkv], qkv4[:, :, h + hkv :]
         dqkv4 = torch.empty_like(qkv4)
-        fused_rope = hd == 128 and cos.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
+        fused_rope = hd == 128 and kc.rope_tables_ok(cos, sin)
         kc.attn_bwd(dattn.view(b, s, h, hd), q, k, v, attn2.view(b, s, h, hd), lse, True, None, 1.0 / math.sqrt(hd),
                     dq=dqkv4[:, :, :h], dk=dqkv4[:, :, h : h + hkv], dv=dqkv4[:, :, h + hkv :],
                     rope=(cos, sin) if fused_rope else None)

@@ -150,6 +150,54 @@ def test_a_matrix_on_another_device_is_refused_before_any_kernel(fake):
     assert not fake.calls
 
 
+def _tables(s, half, shift, device="cpu"):
+    """cos | sin of one packed buffer that starts ``shift`` values late."""
+    g = torch.Generator(device=device).manual_seed(2)
+    ang = torch.rand(s, half, device=device, generator=g)
+    buf = torch.empty(2 * s * half + shift, device=device)
+    cos, sin = buf[shift : shift + s * half].view(s, half), buf[shift + s * half :].view(s, half)
+    cos.copy_(ang.cos())
+    sin.copy_(ang.sin())
+    return cos, sin
+
+
+@pytest.mark.parametrize("shift", [0, 1, 2, 4])
+def test_rotary_tables_off_16_bytes_take_the_separate_rotation(fake, shift):
+    from kempnerforge_b200.ops import cuda as kc
+    from kempnerforge_b200.ops import fused_block
+
+    x, ws = torch.randn(512, 64).bfloat16(), _weights("dense", (256, 128, 128), 64)
+    cos, sin = _tables(256, 64, shift)
+    kc.qkv_rope(x, ws, cos, sin, 256, 128)
+    assert ("rope" in fake.calls) == (shift % 4 == 0) and ("rotation" in fake.calls) == (shift % 4 != 0)
+    assert fused_block._rope_fused(x, torch.cat(ws), cos, sin, 256, 128) == (shift % 4 == 0)
+    if shift % 4:
+        with pytest.raises(AssertionError):
+            kc.gemm(x, torch.cat(ws), rope=(cos, sin, 256, 384, 128))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("grad", [False, True])
+def test_a_block_takes_rotary_tables_from_anywhere(native_lib, grad):
+    from kempnerforge_b200.config import ModelConfig
+    from kempnerforge_b200.models.transformer import TransformerBlock
+
+    torch.manual_seed(0)
+    block = TransformerBlock(ModelConfig(dim=512, n_layers=1, n_heads=4, n_kv_heads=2, vocab_size=256, ffn_hidden_dim=512,
+                                         max_seq_len=512), 0).to(DEV, torch.bfloat16)
+    x = torch.randn(2, 300, 512, device=DEV).bfloat16()
+    out = []
+    for shift in (0, 1):
+        cos, sin = _tables(300, 64, shift, DEV)
+        xl = x.clone().requires_grad_(grad)
+        with torch.set_grad_enabled(grad):
+            y = block(xl, cos, sin)
+        out.append([y.detach()] + ([torch.autograd.grad(y.float().square().sum(), xl)[0]] if grad else []))
+    assert native_lib.read_status() == 0
+    for a, b in zip(*out):   # q, k and their gradients are rounded once more around the separate rotation (2^-9 each)
+        assert float((a.float() - b.float()).norm()) <= 2.0**-6 * float(a.float().norm())
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("rows", [(64,) * 4, (128, 256, 64, 8, 512), (1024, 256, 256), (640, 640)])
 @pytest.mark.parametrize("form", FORMS)
