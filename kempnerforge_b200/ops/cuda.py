@@ -893,18 +893,21 @@ def grouped_swiglu_supported(a: torch.Tensor, wg: torch.Tensor, b_mn: bool) -> b
         and not os.environ.get("KF_DISABLE_GROUPED_SWIGLU")
 
 
-def grouped_swiglu_bwd(dy: torch.Tensor, w_down: torch.Tensor, gu: torch.Tensor, offsets: torch.Tensor, b_mn: bool) -> torch.Tensor:
-    """d[gate | up] (rows, 2F), written over ``gu``: the input-gradient product of the experts' down projection
+def grouped_swiglu_bwd(dy: torch.Tensor, w_down: torch.Tensor, gu: torch.Tensor, offsets: torch.Tensor, b_mn: bool,
+                       out: torch.Tensor | None = None) -> torch.Tensor:
+    """d[gate | up] (rows, 2F), written to ``out`` (default: over ``gu``): the input-gradient product of the experts' down projection
     (``dy`` (rows, K) times ``w_down``: (E, F, K), or (E, K, F) with ``b_mn``) with the SwiGLU gradient in its epilogue;
     the gradient of the hidden activation is never written to memory.  Rows past ``offsets[E]`` stay untouched."""
     rows, k = dy.shape
     e = w_down.shape[0]
     f = w_down.shape[2] if b_mn else w_down.shape[1]
+    out = gu if out is None else out
     assert gu.shape == (rows, 2 * f) and gu.is_contiguous() and w_down.is_contiguous() and dy.stride(1) == 1
-    _check(lib().kf_grouped_swiglu_bwd_bf16(dy.data_ptr(), w_down.data_ptr(), gu.data_ptr(), gu.data_ptr(), offsets.data_ptr(),
+    assert out.shape == gu.shape and out.dtype == gu.dtype and out.is_contiguous()
+    _check(lib().kf_grouped_swiglu_bwd_bf16(dy.data_ptr(), w_down.data_ptr(), gu.data_ptr(), out.data_ptr(), offsets.data_ptr(),
                                             rows, e, f, k, dy.stride(0), 2 * f, int(b_mn), sm_count(), _stream()),
            "kf_grouped_swiglu_bwd_bf16")
-    return gu
+    return out
 
 
 def grouped_swiglu_bwd_supported(dy: torch.Tensor, w_down: torch.Tensor, b_mn: bool) -> bool:

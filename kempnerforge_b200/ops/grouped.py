@@ -96,12 +96,19 @@ class _GroupedSwiGLUFn(torch.autograd.Function):
         return dx, dwg, dwu, None, None
 
 
+def _gradient_buffer(saved: torch.Tensor) -> torch.Tensor:
+    """Where the gradient of a saved activation goes inside a backward pass: over the activation when the graph is released
+    after this pass, a buffer of its own when it is kept (the kernels write through raw pointers, so autograd's version check
+    would not notice that a later pass reads gradients as activations)."""
+    return torch.empty_like(saved) if torch._C._autograd._get_current_graph_task_keep_graph() else saved
+
+
 class _GroupedFFNFn(torch.autograd.Function):
     """The whole expert feed-forward, down(silu(x @ Wg_e) * (x @ Wu_e)), over ragged expert rows as one node.
 
     Forward: the gate / up grouped GEMM with the SwiGLU epilogue, then the down projection.  Backward: the down
     projection's input-gradient product with the SwiGLU gradient in its epilogue (the gradient of the hidden
-    activation never reaches memory; d[gate | up] overwrites the saved pre-activations), two input-gradient grouped
+    activation never reaches memory; d[gate | up] overwrites the saved pre-activations unless the graph is kept), two input-gradient grouped
     GEMMs (the second accumulating into the first's output) and three ragged weight-gradient reductions."""
 
     @staticmethod
@@ -132,7 +139,7 @@ class _GroupedFFNFn(torch.autograd.Function):
 
         dwd = wgrad(h, dy) if ctx.needs_input_grad[3] else None
         # dh = dy @ Wd_e^T: 'kn' stores Wd_e as (F, D), read with the reduction index D contiguous
-        dgu = kc.grouped_swiglu_bwd(dy, wd, gu, offsets, b_mn=not kn)   # gu is dead after this; reuse its storage
+        dgu = kc.grouped_swiglu_bwd(dy, wd, gu, offsets, b_mn=not kn, out=_gradient_buffer(gu))
         dgate, dup = dgu[:, :f], dgu[:, f:]
         dx = dwg = dwu = None
         if ctx.needs_input_grad[0]:
@@ -176,7 +183,7 @@ class _SeparateFFNFn(torch.autograd.Function):
             dy = dy.contiguous()
         need = ctx.needs_input_grad[2:]
         dwd = kc.grouped_wgrad(dy, h, offsets) if any(need[2 * e :]) else [None] * e
-        dgu = kc.grouped_experts(2, dy, downs, None, offsets, f, True, gu, gu)   # gu is dead after this; reuse its storage
+        dgu = kc.grouped_experts(2, dy, downs, None, offsets, f, True, _gradient_buffer(gu), gu)
         dx = kc.grouped_experts(3, dgu, gates, ups, offsets, x.shape[1], True, torch.empty_like(x)) if ctx.needs_input_grad[0] else None
         dwg = dwu = [None] * e
         if any(need[: 2 * e]):
