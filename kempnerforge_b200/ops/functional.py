@@ -486,13 +486,13 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dloss):
         dh, dw = ctx.saved_tensors
-        if (not torch._C._autograd._get_current_graph_task_keep_graph() and not torch.is_grad_enabled()
-                and dloss.dtype == torch.float32 and getattr(ctx.weight, "_kf_grad", None) is None):
-            # nobody reads the saved gradients again: scale them where they are and hand them out
+        # a released graph: nobody reads the saved gradients again, they are scaled where they are and handed out
+        released = not torch._C._autograd._get_current_graph_task_keep_graph() and not torch.is_grad_enabled()
+        if released and dloss.dtype == torch.float32 and getattr(ctx.weight, "_kf_grad", None) is None:
             cu = _cuda()
             return cu.scale_(dh, dloss).view(ctx.h_shape), cu.scale_(dw, dloss), None, None, None
         factor = dloss.to(dh.dtype)
-        dh = dh.mul_(factor).view(ctx.h_shape)
+        dh = (dh.mul_(factor) if released else dh * factor).view(ctx.h_shape)
 
         def compute(out, accumulate):
             if accumulate:

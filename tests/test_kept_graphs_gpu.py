@@ -39,3 +39,31 @@ def test_experts_give_the_same_gradients_again(native_lib, form, counts):
     assert all(bool((g != 0).any()) for g in (first[0], *first[1 : 1 + (form == "separate")]))
     for a, b, c in zip(first, again, last):
         assert torch.equal(a, b) and torch.equal(a, c)
+
+
+@pytest.mark.parametrize("slot", [False, True])
+@pytest.mark.parametrize("factor", [1.0, 0.37])
+def test_loss_gives_the_same_gradients_again(native_lib, slot, factor):
+    from kempnerforge_b200.ops import functional as F
+
+    t, v, d = 300, 1000, 128
+    h = torch.randn(t, d, device=DEV, generator=_gen(0)).bfloat16().requires_grad_(True)
+    w = (torch.randn(v, d, device=DEV, generator=_gen(1)) * 0.05).bfloat16().requires_grad_(True)
+    lab = torch.randint(0, v, (t,), device=DEV, generator=_gen(2))
+    one = torch.autograd.grad(F.linear_cross_entropy(h, w, lab, 1e-3), [h, w])
+    f = float(torch.tensor(factor).bfloat16())
+    want = [(g.float() * f).bfloat16() for g in one]
+    if slot:
+        w._kf_grad = torch.zeros_like(w)
+
+    def grads(loss, **kw):
+        if not slot:
+            return torch.autograd.grad(loss, [h, w], **kw)
+        w._kf_grad_live = False
+        return torch.autograd.grad(loss, [h], **kw)[0], w._kf_grad.clone()
+
+    loss = F.linear_cross_entropy(h, w, lab, 1e-3) * factor
+    for keep in (True, True, False):
+        for a, b in zip(grads(loss, retain_graph=keep), want):
+            assert torch.equal(a, b)
+    assert native_lib.read_status() == 0
