@@ -99,8 +99,10 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
   if (HAS_DOC && skip) {
     const int n64 = docblk::n_blocks(Sq);
     const int2* rg = doc_range + size_t(b) * n64;
-    docblk::build_mask(act, n_max, docblk::merged(rg, n64, m0 / docblk::ROWS, 2 * BLK_M / docblk::ROWS),
-                       [&](int j) { return docblk::merged(rg, n64, j * (BLK_N / docblk::ROWS), BLK_N / docblk::ROWS); });
+    const tilemath::IdRange own = docblk::ids(docblk::merged(rg, n64, m0 / docblk::ROWS, 2 * BLK_M / docblk::ROWS));
+    docblk::build_mask(act, n_max, [&](int j) {
+      return tilemath::ids_meet(docblk::ids(docblk::merged(rg, n64, j * (BLK_N / docblk::ROWS), BLK_N / docblk::ROWS)), own);
+    });
   }
 
   if (threadIdx.x == 0) {

@@ -131,8 +131,8 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     static_assert(BLK_Q == docblk::ROWS, "one id range per query tile");
     const int n64 = docblk::n_blocks(Sk);
     const int2* rg = doc_range + size_t(b) * n64;
-    docblk::build_mask(act, n_q_tiles, docblk::merged(rg, n64, k0 / docblk::ROWS, BLK_K / docblk::ROWS),
-                       [&](int j) { return j >= i_start ? rg[j] : make_int2(1, 0); });
+    const tilemath::IdRange own = docblk::ids(docblk::merged(rg, n64, k0 / docblk::ROWS, BLK_K / docblk::ROWS));
+    docblk::build_mask(act, n_q_tiles, [&](int j) { return tilemath::query_tile_walked(j, i_start, docblk::ids(rg[j]), own); });
   }
   const float scale_log2 = scale * 1.4426950408889634f;
 

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "tile_math.h"
+
 namespace kf {
 namespace docblk {
 
@@ -25,18 +27,15 @@ __device__ __forceinline__ int2 merged(const int2* rg, int n64, int first, int n
   return r;
 }
 
-// One bit per tile whose range meets `own`; called by all threads of the block, which synchronise before the mask is read.
-template <typename RangeOf>
-__device__ __forceinline__ void build_mask(uint32_t* mask, int tiles, int2 own, RangeOf range_of) {
+__device__ __forceinline__ tilemath::IdRange ids(int2 r) { return {r.x, r.y}; }
+
+// One bit per tile for which walked(j) holds; called by all threads of the block, which synchronise before the mask is read.
+template <typename Walked>
+__device__ __forceinline__ void build_mask(uint32_t* mask, int tiles, Walked walked) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   for (int w = warp; w * 32 < tiles; w += warps) {
     const int j = w * 32 + lane;
-    bool on = false;
-    if (j < tiles) {
-      const int2 r = range_of(j);
-      on = r.x <= own.y && own.x <= r.y;
-    }
-    const uint32_t bits = __ballot_sync(0xffffffffu, on);
+    const uint32_t bits = __ballot_sync(0xffffffffu, j < tiles && walked(j));
     if (lane == 0) mask[w] = bits;
   }
 }

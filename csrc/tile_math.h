@@ -29,6 +29,17 @@ KF_TM_HD void raster(int t, int m_blocks, int n_blocks, int group_m, int& m, int
   n = r / rows;
 }
 
+// Smallest and largest document id of a run of positions.  Two runs whose ranges do not meet hold no visible (query, key)
+// pair, whatever the order of the ids.
+struct IdRange {
+  int lo, hi;
+};
+KF_TM_HD bool ids_meet(IdRange a, IdRange b) { return a.lo <= b.hi && b.lo <= a.hi; }
+
+// Attention backward: whether the walk of a key tile with ids `own` visits query tile j with ids `range`; tiles before `first`
+// lie above the causal diagonal.
+KF_TM_HD bool query_tile_walked(int j, int first, IdRange range, IdRange own) { return j >= first && ids_meet(range, own); }
+
 // Ragged grouped GEMM.  tile_start[e] = number of row tiles (of `bm` rows) of experts 0..e-1, tile_start[E] the
 // total; offsets[e] .. offsets[e+1] are expert e's rows.  Fills tile_start and returns the total.
 KF_TM_HD int grouped_tile_starts(const int* offsets, int E, int bm, int* tile_start) {
