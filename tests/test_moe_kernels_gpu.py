@@ -46,6 +46,28 @@ def test_router_gradient_matches_autograd_of_the_formulas(native_lib, sigmoid, t
         assert float((a.float() - b.float()).norm()) <= tol * float(b.float().norm())
 
 
+@pytest.mark.parametrize("sigmoid", [False, True])
+@pytest.mark.parametrize("t,e,k,std", [(1777, 64, 6, 1.0), (5000, 160, 8, 3.0), (2048, 8, 2, 5.0)])
+@pytest.mark.parametrize("zloss", [0.0, 0.5])
+def test_router_gradient_of_fp32_logits_is_as_close_to_64_bits_as_fp32_operations(native_lib, sigmoid, t, e, k, std, zloss):
+    from kempnerforge_b200.ops import moe_ops
+
+    logits = (std * torch.randn(t, e, device=DEV, generator=_gen(1))).requires_grad_(True)
+    bias = 0.1 * torch.randn(e, device=DEV, generator=_gen(2)) if sigmoid else None
+    w, idx, _, mean, z = moe_ops.route(logits, bias, sigmoid, k)
+    dw, dm = torch.randn(t, k, device=DEV, generator=_gen(3)), torch.randn(e, device=DEV, generator=_gen(4))
+    loss = (w * dw).sum() + (mean * dm).sum() + z * zloss
+    got = torch.autograd.grad(loss, logits, retain_graph=True)[0]
+    fp32 = torch.autograd.grad(loss, logits, create_graph=True)[0].detach()
+    x = logits.detach().double().requires_grad_(True)
+    s = torch.sigmoid(x + bias.double()) if sigmoid else torch.softmax(x, -1)
+    sel = s.gather(1, idx)
+    total = (sel / sel.sum(-1, keepdim=True) * dw.double()).sum() + (s.mean(0) * dm.double()).sum()
+    want = torch.autograd.grad(total + zloss * torch.logsumexp(x, -1).square().mean(), x)[0]
+    # the two differ in the order of their sums alone: 5 % of the error (the fast exponential adds 7 %)
+    assert float((got.double() - want).norm()) <= 1.05 * float((fp32.double() - want).norm())
+
+
 @pytest.mark.parametrize("counts", [[256], [128, 128, 128, 128], [5, 0, 300, 77, 130, 1], [0, 0, 513], [400, 17] + [3] * 30])
 @pytest.mark.parametrize("extra", [0, 64])
 def test_experts_with_separate_weights_match_the_packed_path(native_lib, counts, extra):
