@@ -6,10 +6,12 @@
 // query head), i.e. 32 blocks that each walk the whole cache and read every key `group` times.  Here
 //   * one cluster per (batch, KV head): all query heads of the group are the 16 rows of an m16n8k16 MMA, so K and V
 //     are read once; the keys are split over the cluster's CTAs (up to 8) and over the four warps of each CTA;
-//   * K and V tiles of 64 keys move through a three-stage cp.async ring (two CTAs per SM: 190 KB in flight per SM),
-//     16-byte chunks XOR-swizzled so that ldmatrix is free of bank conflicts;
+//   * K and V tiles of 64 keys move through a three-stage cp.async ring, two stages of which are in flight while the third is
+//     read (head dim 128, two CTAs per SM: 128 KB in flight per SM), 16-byte chunks XOR-swizzled so that ldmatrix is free of
+//     bank conflicts;
 //   * the partial (max, sum, output) triples are merged in shared memory and then across the cluster through
 //     distributed shared memory, in a fixed order: one launch, no workspace, bit-reproducible.
+// Generation uses the form for head dim 128; with 64 the block keeps the bits of the separate ops (ops/cuda.py, block_decode).
 // The cache may be a view of a larger one (any batch stride; rows 16-byte aligned), so growing caches need no copy.
 //
 // Replaces F.scaled_dot_product_attention for the cached step of the reference (kempnerforge/model/attention.py:213-231).

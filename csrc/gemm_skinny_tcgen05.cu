@@ -300,8 +300,10 @@ kf_gemm_skinny(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
 }
 
 // Number of CTAs a K range is split over: enough of them to fill the SMs, at least MIN_KB ring steps each.  Weights of less
-// than 8 MB (512 blocks of 128 x 64) are not split: a CTA streams its share in 2 - 5 us either way (768 x 768: 10.3 us with and
-// without, launch included), and with the unsplit sum over K the projections of small models keep the bits of the tile kernels.
+// than 8 MB (512 blocks of 128 x 64) are not split, so that the projections of small models sum over K in the order of the tile
+// kernels and keep their bits: in a model of a few layers every rounding travels on, and one that falls differently moves the
+// logits by as much as all of them together are off.  That costs time: one row, L2 flushed, unsplit / split: 768 x 768 7.0 / 5.6
+// us, 2304 x 768 7.3 / 6.1, 768 x 2048 12.7 / 6.6, 1024 x 3072 17.6 / 7.9.
 static int pick_splits(int tiles, int k_blocks, int num_sms, int per_sm) {
   constexpr int MIN_KB = 4;
   if (tiles * k_blocks < 512) return 1;

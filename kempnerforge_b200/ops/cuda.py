@@ -428,9 +428,11 @@ def block_decode(y: torch.Tensor, attn_ptrs, mlp_ptrs, cache_ptrs, table_ptrs, d
 
     Attention runs on the kernel split over the cache for head dim 128.  With head dim 64 it stays on what the op-by-op path
     uses: the 128-row tile kernel for one sequence, ``foreign(q)`` (rows of H hd) -> dense (B, H hd) between two native calls
-    for more; the rotation is the separate kernel's too.
-    Those heads are the small presets' (12 of 64, one query head per KV head: 1 of the 16 MMA rows in use), where the split
-    kernel measured no faster (10.2 us, library 8.6, at 301 positions), and a small model's logits stay bit for bit the same."""
+    for more; the rotation is the separate kernel's too.  The reason is that a small model's logits stay bit for bit the same, not
+    speed.  Measured (12 heads of 64, one query head per KV head, us, at 300 / 1000 / 2000 / 4000 positions): one sequence, split
+    kernel 5.2 / 6.3 / 7.7 / 10.1, tile kernel 7.7 / 12.3 / 19.7 / 34.7, library 4.9 / 6.5 / 7.9 / 8.8; four sequences, split
+    6.1 / 8.2 / 11.1 / 17.3, library 5.4 / 7.2 / 9.6 / 14.6; sixteen, split 9.7 / 18.9 / 31.2 / 54.8, library 9.2 / 16.9 / 25.6 /
+    40.4."""
     b, d, h, hkv, hd, f = dims[:6]
     tile = hd == 64 and b == 1
     qc, row = h * hd, (h + 2 * hkv) * hd

@@ -1,4 +1,5 @@
-"""The fused head and loss under the gradients it can be handed: one, another scalar, a kept graph, a flat gradient slot."""
+"""The fused head and loss under the gradients it can be handed: one, another scalar, and the weight gradient of a kept graph
+(repeated passes and flat gradient slots: test_kept_graphs_gpu.py)."""
 
 import pytest
 import torch
