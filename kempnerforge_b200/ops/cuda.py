@@ -733,10 +733,15 @@ def attn_supported(q, k, v, causal: bool, needs_grad: bool = False) -> bool:
     return _attn_rows_ok(q) and _attn_rows_ok(k) and _attn_rows_ok(v)
 
 
-def doc_blocks(doc_ids: torch.Tensor):
+def doc_blocks(doc_ids: torch.Tensor, like: torch.Tensor | None = None):
     """(int32 ids (B, S), int32 (B, ceil(S / 64), 2) smallest and largest id of every 64 positions): what the attention
-    kernels read of a document mask.  Pass the pair in place of the ids to reuse it for the backward."""
+    kernels read of a document mask.  Pass the pair in place of the ids to reuse it for the backward.  ``like`` (B, S, ..): the
+    keys they belong to; ids of as many positions in another shape and one row for all sequences are taken, any others refused."""
     ids = doc_ids if doc_ids.dtype in (torch.int32, torch.int64) else doc_ids.to(torch.int32)
+    if like is not None:
+        assert ids.device == like.device, f"document ids on {ids.device}, keys on {like.device}"
+        if ids.shape != like.shape[:2]:
+            ids = ids.reshape(like.shape[:2]) if ids.numel() == like.shape[0] * like.shape[1] else ids.expand(like.shape[:2])
     ids = ids.contiguous()
     b, s = ids.shape
     out = torch.empty((b, s), dtype=torch.int32, device=ids.device)
@@ -747,7 +752,7 @@ def doc_blocks(doc_ids: torch.Tensor):
 
 
 def attn_fwd(q, k, v, causal: bool, doc_ids, scale: float):
-    """q (B, Sq, H, hd), k / v (B, Sk, Hkv, hd) -> out (B, Sq, H, hd) bf16 and lse (B, H, Sq) fp32.  ``doc_ids``: (B, S)
+    """q (B, Sq, H, hd), k / v (B, Sk, Hkv, hd) -> out (B, Sq, H, hd) bf16 and lse (B, H, Sq) fp32.  ``doc_ids``: (B, Sk)
     ids, or what :func:`doc_blocks` made of them."""
     b, sq, h, hd = q.shape
     sk, hkv = k.shape[1], k.shape[2]
@@ -755,7 +760,7 @@ def attn_fwd(q, k, v, causal: bool, doc_ids, scale: float):
     lse = torch.empty((b, h, sq), dtype=torch.float32, device=q.device)
     doc = rng = None
     if doc_ids is not None:
-        doc, rng = doc_ids if isinstance(doc_ids, tuple) else doc_blocks(doc_ids)
+        doc, rng = doc_ids if isinstance(doc_ids, tuple) else doc_blocks(doc_ids, k)
     # two query tiles per CTA (interleaved softmax) once there are at least two tiles; KF_ATTN_FWD=1 forces the
     # single-tile kernel
     L = lib()
@@ -1084,7 +1089,7 @@ def attn_bwd(dout, q, k, v, out, lse, causal: bool, doc_ids, scale: float, dq=No
     dq_acc = torch.empty((b, sq, h, hd), dtype=torch.float32, device=q.device)
     doc = rng = None
     if doc_ids is not None:
-        doc, rng = doc_ids if isinstance(doc_ids, tuple) else doc_blocks(doc_ids)
+        doc, rng = doc_ids if isinstance(doc_ids, tuple) else doc_blocks(doc_ids, k)
     cos = sin = None
     if rope is not None:
         cos, sin = rope

@@ -289,7 +289,7 @@ class _FlashAttnFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, causal, doc_ids, scale):
         cu = _cuda()
-        mask = cu.doc_blocks(doc_ids) if doc_ids is not None else None
+        mask = cu.doc_blocks(doc_ids, k) if doc_ids is not None else None
         out, lse = cu.attn_fwd(q, k, v, causal, mask, scale)
         ctx.save_for_backward(q, k, v, out, lse, *(mask or ()))
         ctx.causal, ctx.scale = causal, scale
@@ -349,7 +349,7 @@ class _QKVAttnFn(torch.autograd.Function):
             x2 = x2.contiguous()
         h, hkv = wq.shape[0] // hd, wk.shape[0] // hd
         qkv = cu.qkv_rope(x2, [wq, wk, wv], cos, sin, s, hd).view(b, s, h + 2 * hkv, hd)
-        mask = cu.doc_blocks(doc_ids) if doc_ids is not None else None
+        mask = cu.doc_blocks(doc_ids, qkv) if doc_ids is not None else None
         scale = 1.0 / math.sqrt(hd)
         out, lse = cu.attn_fwd(qkv[:, :, :h], qkv[:, :, h : h + hkv], qkv[:, :, h + hkv :], True, mask, scale)
         ctx.save_for_backward(x2, wq, wk, wv, cos, sin, qkv, out, lse, *(mask or ()))
