@@ -289,10 +289,10 @@ def _ptr(t: torch.Tensor | None):
 
 
 def _plain_rows(w: torch.Tensor, device: torch.device) -> bool:
-    """A kernel can read the matrix by its address and row pitch: on its GPU, adjacent columns, rows that do not overlap, 16-byte
-    steps.  Anything else is left to the copy that stacks the matrices: the pitch alone would name other elements, the address
+    """A kernel can read the matrix by its address and row pitch: on its GPU, not empty (an empty one ends the kernels' list),
+    adjacent columns, rows that do not overlap, 16-byte steps.  Anything else is left to the copy that stacks the matrices: the pitch alone would name other elements, the address
     other memory."""
-    return (w.device == device and w.stride(1) == 1 and w.stride(0) >= w.shape[1] and w.stride(0) % 8 == 0
+    return (w.device == device and w.shape[0] > 0 and w.stride(1) == 1 and w.stride(0) >= w.shape[1] and w.stride(0) % 8 == 0
             and w.data_ptr() % 16 == 0)
 
 

@@ -22,7 +22,8 @@ class _FakeLibrary:
         self.calls = []
 
     def _stack(self, ptrs, rows, cols, pitches):
-        ws = [(p, n, ld) for p, n, ld in zip(ptrs, rows, pitches) if n]
+        rows = list(rows) + [0]
+        ws = list(zip(ptrs, rows, pitches))[: rows.index(0)]   # the first empty matrix ends the list
         if any(ld < cols or ld % 8 for _, _, ld in ws):   # a tensor map refuses these
             return None
         return torch.cat([_read(p, n, cols, ld) for p, n, ld in ws])
@@ -116,7 +117,7 @@ def _check(x, ws):
 FORMS = ["dense", "columns", "transposed", "one row", "cut"]
 
 
-@pytest.mark.parametrize("rows", [(16,) * 4, (8, 16, 24, 8, 8), (128, 64), (128, 128, 64)])
+@pytest.mark.parametrize("rows", [(16,) * 4, (8, 16, 24, 8, 8), (128, 64), (128, 128, 64), (128, 0, 64), (0, 64)])
 @pytest.mark.parametrize("form", FORMS)
 @pytest.mark.parametrize("m", [3, 600])
 def test_every_weight_counts_whatever_its_layout(fake, rows, form, m):
@@ -199,7 +200,7 @@ def test_a_block_takes_rotary_tables_from_anywhere(native_lib, grad):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("rows", [(64,) * 4, (128, 256, 64, 8, 512), (1024, 256, 256), (640, 640)])
+@pytest.mark.parametrize("rows", [(64,) * 4, (128, 256, 64, 8, 512), (1024, 256, 256), (640, 640), (1024, 0, 512)])
 @pytest.mark.parametrize("form", FORMS)
 @pytest.mark.parametrize("m", [5, 300, 4100])
 def test_several_weights_on_the_gpu(native_lib, rows, form, m):
