@@ -1,4 +1,4 @@
-// Flash attention backward on the 5th-generation tensor cores (head dim 128).
+// Flash attention backward on the 5th-generation tensor cores (head dim 64 or 128; the sizes below are those of 128).
 //
 // One CTA owns a tile of 128 keys of one (batch, KV head) and walks over every query head of the group and
 // every 64-row query tile that can see those keys.  All five GEMMs of the backward pass run on tcgen05 with
@@ -24,6 +24,9 @@
 //   warps 6-9  : dQ reduction (TMEM -> shared-memory tile -> one cp.reduce.async.bulk.tensor add per tile;
 //                or, as a fallback mode, red.global.add.f32 per element)
 //
+// Head dim 64 has half the products per score and the same softmax, so it is bound by the softmax warps: 100 positions of 12
+// heads 15 us, 3 x 333 23 us, 2048 65 us (the library's backward 16, 19 and 40, before the copies around it).
+//
 // D_i = rowsum(dO_i * O_i) comes from a small pre-pass; a post-pass converts the fp32 dQ to bf16.
 // Replaces the backward of F.scaled_dot_product_attention (kempnerforge/model/attention.py:227-231) for the
 // causal / document-masked training path, without expanding grouped KV heads.
@@ -33,7 +36,6 @@
 namespace kf {
 namespace attnb {
 
-constexpr int HD = 128;
 constexpr int BLK_K = 128;  // keys per CTA
 constexpr int BLK_Q = 64;   // queries per iteration
 constexpr int THREADS = 448;
@@ -41,19 +43,24 @@ constexpr int TMEM_COLS = 512;
 constexpr int ST_COL = 0;     // S^T buffers 0 / 1 (fp32, 64 cols each); P^T (bf16 pairs, 32 cols) aliases each start
 constexpr int DPT_COL = 128;  // dP^T (fp32, 64 cols)
 constexpr int DQT_COL = 192;  // dQ^T (fp32, 64 cols)
-constexpr int DV_COL = 256;   // dV accumulator (fp32, 128 cols)
-constexpr int DK_COL = 384;   // dK accumulator (fp32, 128 cols)
-constexpr int KV_TILE_BYTES = BLK_K * HD * 2;   // 32 KB: two blocks of [128 rows x 128 B]
-constexpr int KV_BLOCK_BYTES = BLK_K * 128;     // 16 KB
-constexpr int Q_TILE_BYTES = BLK_Q * HD * 2;    // 16 KB: two blocks of [64 rows x 128 B]
-constexpr int Q_BLOCK_BYTES = BLK_Q * 128;      // 8 KB
+constexpr int DV_COL = 256;   // dV accumulator (fp32, HD cols)
+constexpr int DK_COL = 384;   // dK accumulator (fp32, HD cols)
+constexpr int KV_BLOCK_BYTES = BLK_K * 128;     // 16 KB: [128 rows x 128 B], HD / 64 of them per K / V tile
+constexpr int Q_BLOCK_BYTES = BLK_Q * 128;      // 8 KB: [64 rows x 128 B], HD / 64 of them per Q_i / dO_i tile
 constexpr int DS_BYTES = BLK_K * BLK_Q * 2;     // 16 KB: [128 key rows x 128 B]
 constexpr int STAGES = 3;  // Q_i / dO_i ring: a tile is loaded one whole iteration before its scores are issued
 constexpr int AUX_BYTES = 2048;  // barriers, row statistics, doc ids
-constexpr size_t SMEM = 2 * size_t(KV_TILE_BYTES) + STAGES * 2 * size_t(Q_TILE_BYTES) + 2 * DS_BYTES + 1024 /*align*/ +
-                        AUX_BYTES;
-constexpr int DQ_STAGE_BYTES = BLK_Q * HD * 4;  // 32 KB: one dQ tile [64 queries][128] fp32 for the bulk reduction
-constexpr size_t SMEM_DQ_TMA = SMEM + DQ_STAGE_BYTES;
+
+template <int HD>
+struct Cfg {
+  static constexpr int BLOCKS = HD / 64;
+  static constexpr int KV_TILE_BYTES = BLOCKS * KV_BLOCK_BYTES;
+  static constexpr int Q_TILE_BYTES = BLOCKS * Q_BLOCK_BYTES;
+  static constexpr size_t SMEM =
+      2 * size_t(KV_TILE_BYTES) + STAGES * 2 * size_t(Q_TILE_BYTES) + 2 * DS_BYTES + 1024 /*align*/ + AUX_BYTES;
+  static constexpr int DQ_STAGE_BYTES = BLK_Q * HD * 4;  // one dQ tile [64 queries][HD] fp32 for the bulk reduction
+  static constexpr size_t SMEM_DQ_TMA = SMEM + DQ_STAGE_BYTES;
+};
 
 using attn::fadd2;
 using attn::fast_exp2;
@@ -81,7 +88,7 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
-template <bool CAUSAL, bool HAS_DOC>
+template <int HD, bool CAUSAL, bool HAS_DOC>
 __global__ void __launch_bounds__(THREADS, 1)
 kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
@@ -89,6 +96,7 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     float* __restrict__ dQacc, __nv_bfloat16* __restrict__ dK, __nv_bfloat16* __restrict__ dV, int Sq,
                     int Sk, int H, int group, long long lddk, long long lddv, float scale, int* status,
                     const float* __restrict__ cosT, const float* __restrict__ sinT, const int2* __restrict__ doc_range) {
+  constexpr int KV_TILE_BYTES = Cfg<HD>::KV_TILE_BYTES, Q_TILE_BYTES = Cfg<HD>::Q_TILE_BYTES, BLOCKS = Cfg<HD>::BLOCKS;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -188,7 +196,7 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       int issued = 0;
       mbar_expect_tx(kv_full, 2 * KV_TILE_BYTES);
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
+      for (int c = 0; c < BLOCKS; ++c) {
         tma_load_2d(k_smem + c * KV_BLOCK_BYTES, &map_k, kv_full, hk * HD + 64 * c, b * Sk + k0);
         tma_load_2d(v_smem + c * KV_BLOCK_BYTES, &map_v, kv_full, hk * HD + 64 * c, b * Sk + k0);
       }
@@ -201,7 +209,7 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const int q0 = wk.i * BLK_Q;
         mbar_expect_tx(qdo_full(st), 2 * Q_TILE_BYTES);
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < BLOCKS; ++c) {
           tma_load_2d(q_smem + st * Q_TILE_BYTES + c * Q_BLOCK_BYTES, &map_q, qdo_full(st), hq * HD + 64 * c,
                       b * Sq + q0);
           tma_load_2d(do_smem + st * Q_TILE_BYTES + c * Q_BLOCK_BYTES, &map_do, qdo_full(st), hq * HD + 64 * c,
@@ -270,7 +278,8 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         for (int kk = 0; kk < BLK_Q / 16; ++kk)
           tc_mma_f16(tmem_base + DK_COL, umma_desc_sw128(dss + kk * 32, 16, 1024),
                      umma_desc_sw128(qs + kk * 2048, Q_BLOCK_BYTES, 1024), idesc_acc, (it | kk) != 0);
-        // dQ_i^T = K^T dS : A = K rows read with the head dim as M, B = dS^T rows read with the query dim as N
+        // dQ_i^T = K^T dS : A = K rows read with the head dim as M, B = dS^T rows read with the query dim as N.  With 64
+        // head dims the upper half of M is whatever follows K in shared memory (V): those 64 lanes are never read.
 #pragma unroll
         for (int kk = 0; kk < BLK_K / 16; ++kk)
           tc_mma_f16(tmem_base + DQT_COL, umma_desc_sw128(k_smem + kk * 2048, KV_BLOCK_BYTES, 1024),
@@ -486,14 +495,15 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         group_sync(2, 128);
 #pragma unroll
         for (int c = 0; c < BLK_Q; ++c)
-          asm volatile("st.shared.b32 [%0], %1;" ::"r"(dq_stage + uint32_t(c * HD + d) * 4u), "r"(v[c]) : "memory");
+          if (HD == 128 || d < HD)
+            asm volatile("st.shared.b32 [%0], %1;" ::"r"(dq_stage + uint32_t(c * HD + d) * 4u), "r"(v[c]) : "memory");
         fence_async_smem();
         group_sync(2, 128);
         if (elected && ok) {
           tma_reduce_add_2d(&map_dq, dq_stage, hq * HD, b * Sq + q0);
           bulk_commit();
         }
-      } else if (ok) {
+      } else if (ok && (HD == 128 || d < HD)) {
         float* base = dQacc + ((size_t(b) * Sq + q0) * H + hq) * HD + d;
 #pragma unroll
         for (int c = 0; c < BLK_Q; ++c)
@@ -511,24 +521,26 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   }
 }
 
-// D[b, h, s] = sum_d O[b, s, h, d] * dO[b, s, h, d]: 16 lanes x 16 bytes per (b, s, h) row, eight rows per warp with all
+// D[b, h, s] = sum_d O[b, s, h, d] * dO[b, s, h, d]: HD / 8 lanes x 16 bytes per (b, s, h) row, 8 (16) rows per warp with all
 // eight loads of a lane in flight.  Memory-bound; one row per warp with one 8-byte load per lane and operand ran at a quarter
 // of the copy rate (80 us at 8192 x 32 heads, 134 MB), this form takes 35 us.
-__global__ void __launch_bounds__(256) kf_attn_bwd_dot128(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __restrict__ dO,
+template <int HD>
+__global__ void __launch_bounds__(256) kf_attn_bwd_dot(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __restrict__ dO,
                                                           float* __restrict__ D, int B, int S, int H, long long ldo,
                                                           long long lddo) {
   const long long rows = (long long)B * S * H;
-  const long long r0 = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * 8;
-  const int lane = threadIdx.x & 31, half = lane >> 4, c = (lane & 15) * 8;
+  constexpr int LANES = HD / 8, PER = 32 / LANES;  // lanes per row, rows per warp and load
+  const long long r0 = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * (4 * PER);
+  const int lane = threadIdx.x & 31, sub = lane / LANES, c = (lane % LANES) * 8;
   if (r0 >= rows) return;
   uint4 a[4], g[4];
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    const long long row = r0 + u * 2 + half < rows ? r0 + u * 2 + half : rows - 1;
+    const long long row = r0 + u * PER + sub < rows ? r0 + u * PER + sub : rows - 1;
     const long long bs = row / H;
     const int h = int(row - bs * H);
-    a[u] = *reinterpret_cast<const uint4*>(O + bs * ldo + (long long)h * 128 + c);
-    g[u] = *reinterpret_cast<const uint4*>(dO + bs * lddo + (long long)h * 128 + c);
+    a[u] = *reinterpret_cast<const uint4*>(O + bs * ldo + (long long)h * HD + c);
+    g[u] = *reinterpret_cast<const uint4*>(dO + bs * lddo + (long long)h * HD + c);
   }
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
@@ -540,9 +552,9 @@ __global__ void __launch_bounds__(256) kf_attn_bwd_dot128(const __nv_bfloat16* _
       acc += x.x * y.x + x.y * y.y;
     }
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    const long long row = r0 + u * 2 + half;
-    if ((lane & 15) == 0 && row < rows) {
+    for (int o = LANES / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    const long long row = r0 + u * PER + sub;
+    if (lane % LANES == 0 && row < rows) {
       const long long bs = row / H;
       const long long b = bs / S;
       D[(b * H + (row - bs * H)) * S + (bs - b * S)] = acc;
@@ -565,7 +577,8 @@ __global__ void kf_f32_to_bf16_rows(const float* __restrict__ src, __nv_bfloat16
   }
 }
 
-// scale * fp32 dQ [rows][H * 128] -> bf16 rows with pitch ld, through the inverse rotary embedding of position (row % S)
+// scale * fp32 dQ [rows][H * HD] -> bf16 rows with pitch ld, through the inverse rotary embedding of position (row % S)
+template <int HD>
 __global__ void kf_dq_finish_rope(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long rows, int H,
                                   long long ld, const float* __restrict__ cosT, const float* __restrict__ sinT, int S,
                                   float scale) {
@@ -619,35 +632,16 @@ inline int make_map_2d_f32_plain(CUtensorMap* map, const void* base, uint64_t ro
 }  // namespace attnb
 }  // namespace kf
 
-extern "C" {
-
-// How the backward kernel adds its dQ tiles to the fp32 accumulator: 0 = red.global per element,
-// 1 = one bulk tensor reduction per tile (default).  Returns the previous mode.
-int kf_attn_bwd_dq_mode(int mode) {
-  const int prev = kf::attnb::g_dq_mode;
-  if (mode == 0 || mode == 1) kf::attnb::g_dq_mode = mode;
-  return prev;
-}
-
-// Backward attention (head dim 128).  q / k / v / o / do: rows (b * S + s) with pitches ld*, heads side by
-// side; lse: fp32 [B][H][Sq] from the forward; dsum: fp32 scratch [B][H][Sq]; dq_acc: fp32 scratch
-// [B][Sq][H][128] (zeroed here); dq / dk / dv: bf16 outputs with pitches lddq / lddk / lddv (they may be
-// slices of one fused gradient buffer).  doc: optional int32 [B][S].  Requires Sq == Sk when causal or doc.
-// kf_attn_bwd_rope_bf16: the same, and dq / dk additionally pass through the inverse rotary embedding (cosT / sinT:
-// fp32 [Sq][64], position = index inside the sequence), i.e. they are gradients with respect to the un-rotated
-// projections when q / k were rotated after the projection.  Null tables = no rotation.  doc_range (optional): the id
-// ranges kf_doc_blocks wrote for `doc`; query tiles without a visible pair are skipped with it.
-int kf_attn_bwd_rope_bf16(const void* q, const void* k, const void* v, const void* o, const void* d_o, const void* lse,
+namespace kf {
+namespace attnb {
+template <int HD>
+static int run(const void* q, const void* k, const void* v, const void* o, const void* d_o, const void* lse,
                           void* dsum, void* dq_acc, void* dq, void* dk, void* dv, const void* doc, int B, int Sq, int Sk,
-                          int H, int Hkv, int hd, long long ldq, long long ldk, long long ldv, long long ldo,
+                          int H, int Hkv, long long ldq, long long ldk, long long ldv, long long ldo,
                           long long lddo, long long lddq, long long lddk, long long lddv, float scale, int causal,
-                          const void* cosT, const void* sinT, const void* doc_range, void* stream) {
-  using namespace kf;
-  using namespace kf::attnb;
-  if (hd != HD || Hkv <= 0 || H % Hkv != 0) return 3;
-  if ((causal || doc) && Sq != Sk) return 4;
-  if ((ldq | ldk | ldv | ldo | lddo | lddq | lddk | lddv) & 7) return 5;
-  cudaStream_t st = (cudaStream_t)stream;
+                          const void* cosT, const void* sinT, const void* doc_range, cudaStream_t st) {
+  using C = Cfg<HD>;
+  constexpr int hd = HD;
   CUtensorMap mq, mk, mv, mdo;
   int rc = make_map_2d_bf16(&mq, q, uint64_t(B) * Sq, uint64_t(H) * hd, ldq, 64, BLK_Q);
   if (rc) return 100 + rc;
@@ -661,13 +655,14 @@ int kf_attn_bwd_rope_bf16(const void* q, const void* k, const void* v, const voi
   CUtensorMap mdq;
   rc = make_map_2d_f32_plain(&mdq, dq_acc, uint64_t(B) * Sq, uint64_t(H) * hd, HD, BLK_Q);
   if (rc) return 280 + rc;
-  const size_t smem_bytes = dq_tma ? SMEM_DQ_TMA : SMEM;
+  const size_t smem_bytes = dq_tma ? C::SMEM_DQ_TMA : C::SMEM;
   // pre-pass: D = rowsum(dO * O); zero the fp32 dQ accumulator
   {
     const long long rows = (long long)B * Sq * H;
     const int threads = 256;
-    const long long blocks = ((rows + 7) / 8 * 32 + threads - 1) / threads;
-    kf_attn_bwd_dot128<<<(unsigned)blocks, threads, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(o),
+    constexpr int ROWS_PER_WARP = 4 * 32 / (HD / 8);
+    const long long blocks = ((rows + ROWS_PER_WARP - 1) / ROWS_PER_WARP * 32 + threads - 1) / threads;
+    kf_attn_bwd_dot<HD><<<(unsigned)blocks, threads, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(o),
                                                              reinterpret_cast<const __nv_bfloat16*>(d_o),
                                                              reinterpret_cast<float*>(dsum), B, Sq, H, ldo, lddo);
     cudaError_t e = cudaMemsetAsync(dq_acc, 0, size_t(B) * Sq * H * hd * sizeof(float), st);
@@ -677,10 +672,10 @@ int kf_attn_bwd_rope_bf16(const void* q, const void* k, const void* v, const voi
   dim3 grid(Hkv * B, (Sk + BLK_K - 1) / BLK_K);
 #define KF_BWD_LAUNCH(C_, D_)                                                                                      \
   {                                                                                                                \
-    auto kern = kf_attn_bwd_tcgen05<C_, D_>;                                                                       \
+    auto kern = kf_attn_bwd_tcgen05<HD, C_, D_>;                                                                       \
     static bool attr_set = false;                                                                                  \
     if (!attr_set) {                                                                                               \
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_DQ_TMA);   \
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_DQ_TMA);   \
       if (e != cudaSuccess) return 300 + (int)e;                                                                   \
       attr_set = true;                                                                                             \
     }                                                                                                              \
@@ -702,7 +697,7 @@ int kf_attn_bwd_rope_bf16(const void* q, const void* k, const void* v, const voi
     const long long rows = (long long)B * Sq;
     const int cols = H * hd;
     if (cosT)
-      kf_dq_finish_rope<<<1184, 256, 0, st>>>(reinterpret_cast<const float*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dq),
+      kf_dq_finish_rope<HD><<<1184, 256, 0, st>>>(reinterpret_cast<const float*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dq),
                                               rows, H, lddq, reinterpret_cast<const float*>(cosT),
                                               reinterpret_cast<const float*>(sinT), Sq, scale);
     else
@@ -711,6 +706,41 @@ int kf_attn_bwd_rope_bf16(const void* q, const void* k, const void* v, const voi
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
+}
+
+}  // namespace attnb
+}  // namespace kf
+
+extern "C" {
+
+// How the backward kernel adds its dQ tiles to the fp32 accumulator: 0 = red.global per element,
+// 1 = one bulk tensor reduction per tile (default).  Returns the previous mode.
+int kf_attn_bwd_dq_mode(int mode) {
+  const int prev = kf::attnb::g_dq_mode;
+  if (mode == 0 || mode == 1) kf::attnb::g_dq_mode = mode;
+  return prev;
+}
+
+// Backward attention (head dim 64 or 128).  q / k / v / o / do: rows (b * S + s) with pitches ld*, heads side by
+// side; lse: fp32 [B][H][Sq] from the forward; dsum: fp32 scratch [B][H][Sq]; dq_acc: fp32 scratch
+// [B][Sq][H][hd] (zeroed here); dq / dk / dv: bf16 outputs with pitches lddq / lddk / lddv (they may be
+// slices of one fused gradient buffer).  doc: optional int32 [B][S].  Requires Sq == Sk when causal or doc.
+// kf_attn_bwd_rope_bf16: the same, and dq / dk additionally pass through the inverse rotary embedding (cosT / sinT:
+// fp32 [Sq][hd / 2], position = index inside the sequence), i.e. they are gradients with respect to the un-rotated
+// projections when q / k were rotated after the projection.  Null tables = no rotation.  doc_range (optional): the id
+// ranges kf_doc_blocks wrote for `doc`; query tiles without a visible pair are skipped with it.
+int kf_attn_bwd_rope_bf16(const void* q, const void* k, const void* v, const void* o, const void* d_o, const void* lse,
+                          void* dsum, void* dq_acc, void* dq, void* dk, void* dv, const void* doc, int B, int Sq, int Sk,
+                          int H, int Hkv, int hd, long long ldq, long long ldk, long long ldv, long long ldo,
+                          long long lddo, long long lddq, long long lddk, long long lddv, float scale, int causal,
+                          const void* cosT, const void* sinT, const void* doc_range, void* stream) {
+  using namespace kf::attnb;
+  if ((hd != 64 && hd != 128) || Hkv <= 0 || H % Hkv != 0) return 3;
+  if ((causal || doc) && Sq != Sk) return 4;
+  if ((ldq | ldk | ldv | ldo | lddo | lddq | lddk | lddv) & 7) return 5;
+  auto fn = hd == 64 ? run<64> : run<128>;
+  return fn(q, k, v, o, d_o, lse, dsum, dq_acc, dq, dk, dv, doc, B, Sq, Sk, H, Hkv, ldq, ldk, ldv, ldo, lddo, lddq, lddk, lddv, scale,
+            causal, cosT, sinT, doc_range, (cudaStream_t)stream);
 }
 
 int kf_attn_bwd_bf16(const void* q, const void* k, const void* v, const void* o, const void* d_o, const void* lse,

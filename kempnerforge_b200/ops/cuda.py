@@ -718,19 +718,35 @@ def _attn_rows_ok(t: torch.Tensor) -> bool:
             and t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0)
 
 
-def attn_supported(q, k, v, causal: bool, needs_grad: bool = False) -> bool:
+def attn_supported(q, k, v, causal: bool, needs_grad: bool = False, docs: bool = False) -> bool:
     """Shapes the tcgen05 attention kernels cover: bf16, head dim 64 or 128, grouped KV heads, causal or full,
     optional document ids; q / k / v may be strided views of one fused projection output."""
     L = lib()
     if getattr(L, "kf_attn_fwd_bf16", None) is None or attn_policy() == "library":
         return False
-    if needs_grad and (getattr(L, "kf_attn_bwd_bf16", None) is None or q.shape[-1] != 128):
+    if needs_grad and (getattr(L, "kf_attn_bwd_bf16", None) is None
+                       or not attn_bwd_chosen(q.shape[-1], q.shape[0] * q.shape[2], q.shape[1], k.shape[1], causal, docs)):
         return False
     if q.dtype != torch.bfloat16 or q.shape[-1] not in (64, 128) or q.shape[2] % k.shape[2] != 0:
         return False
     if causal and q.shape[1] != k.shape[1]:
         return False
     return _attn_rows_ok(q) and _attn_rows_ok(k) and _attn_rows_ok(v)
+
+
+HEAD64_MAX_SCORES = 1 << 25
+
+
+def attn_bwd_chosen(hd: int, heads: int, sq: int, sk: int, causal: bool, docs: bool) -> bool:
+    """Whether attention with gradients (``heads`` = batch x query heads) runs on the native kernels.  Head dim 128: always.  64:
+    with document ids, which the library does not take; else up to ``HEAD64_MAX_SCORES`` visible scores, and unless the
+    program asked for deterministic algorithms (dQ tiles are added in the order in which they finish).  Measured, forward +
+    backward, us, native / library (12 causal heads): 100 positions 20 / 21, 3 x 333 34 / 30, 2048 101 / 66, 4 x 2048 259 / 151.
+    Around the library's kernels a block also makes three copies and a rotation of q | k | v gradients and issues a second
+    autograd graph from the host (170 us), which decides up to about the limit."""
+    if hd != 64:
+        return hd == 128
+    return docs or (heads * sq * sk // (2 if causal else 1) <= HEAD64_MAX_SCORES and not torch.are_deterministic_algorithms_enabled())
 
 
 def doc_blocks(doc_ids: torch.Tensor, like: torch.Tensor | None = None):
@@ -1074,7 +1090,7 @@ def gemm_rope_supported(x2: torch.Tensor, w: torch.Tensor, hd: int) -> bool:
 def attn_bwd(dout, q, k, v, out, lse, causal: bool, doc_ids, scale: float, dq=None, dk=None, dv=None, rope=None):
     """Gradients of ``attn_fwd``.  ``dq`` / ``dk`` / ``dv`` may be preallocated (strided) destinations, e.g. the
     three head ranges of one fused projection gradient; otherwise contiguous tensors are returned.
-    ``rope = (cos, sin)`` (fp32 (S, 64)): dq and dk leave through the inverse rotary embedding, i.e. they are the
+    ``rope = (cos, sin)`` (fp32 (S, hd / 2)): dq and dk leave through the inverse rotary embedding, i.e. they are the
     gradients of the un-rotated projections when q and k were rotated after the projection."""
     b, sq, h, hd = q.shape
     sk, hkv = k.shape[1], k.shape[2]

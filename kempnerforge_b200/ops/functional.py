@@ -320,7 +320,7 @@ def attention(
         needs_grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
         policy = cu.attn_policy()
         want = policy == "native" or (policy == "auto" and (not needs_grad or doc_ids is not None))
-        if want and (doc_ids is None or q.shape[1] == k.shape[1]) and cu.attn_supported(q, k, v, causal, needs_grad):
+        if want and (doc_ids is None or q.shape[1] == k.shape[1]) and cu.attn_supported(q, k, v, causal, needs_grad, doc_ids is not None):
             if not needs_grad:
                 return cu.attn_fwd(q, k, v, causal, doc_ids, scale)[0]
             return _FlashAttnFn.apply(q, k, v, causal, doc_ids, scale)
@@ -373,14 +373,16 @@ class _QKVAttnFn(torch.autograd.Function):
 
 def qkv_attention(x, wq, wk, wv, cos, sin, doc_ids, hd: int) -> torch.Tensor | None:
     """Causal self-attention of x (B, S, D) up to the output projection -> (B, S, H hd), or None when the fused node does not
-    cover the call (head dim 128, bf16 on a GPU, gradients wanted, fp32 tables of this sequence, no fp8)."""
-    if (hd != 128 or not use_native(x) or not torch.is_grad_enabled() or x.dim() != 3 or x.shape[0] * x.shape[1] < 128
+    cover the call (head dim 64 or 128, bf16 on a GPU, gradients wanted, fp32 tables of this sequence, no fp8)."""
+    if (hd not in (64, 128) or not use_native(x) or not torch.is_grad_enabled() or x.dim() != 3 or x.shape[0] * x.shape[1] < 128
             or cos.dtype != torch.float32 or sin.dtype != torch.float32 or cos.dim() != 2 or cos.shape != sin.shape
             or cos.requires_grad or sin.requires_grad or cos.shape[0] < x.shape[1] or cos.shape[1] != hd // 2
             or not (cos.is_cuda and _cuda().rope_tables_ok(cos, sin))
             or (doc_ids is not None and doc_ids.shape != x.shape[:2])):
         return None
     cu = _cuda()
+    if not cu.attn_bwd_chosen(hd, x.shape[0] * (wq.shape[0] // hd), x.shape[1], x.shape[1], True, doc_ids is not None):
+        return None
     d = x.shape[-1]
     for w in (wq, wk, wv):
         if (w.dtype != torch.bfloat16 or not w.is_cuda or w.dim() != 2 or w.shape[1] != d or w.shape[0] % hd or not w.is_contiguous()

@@ -265,7 +265,7 @@ class DenseBlockFn(torch.autograd.Function):
         dqkv4 = torch.empty_like(qkv4)
         if it["actx"][0] == "native":
             # dq | dk | dv land in their head ranges of the fused gradient, already through the inverse rotation
-            fused_rope = hd == 128 and kc.rope_tables_ok(cos, sin)
+            fused_rope = kc.rope_tables_ok(cos, sin)
             kc.attn_bwd(dattn.view(b, s, h, hd), q, k, v, attn, it["actx"][1], True, None, 1.0 / math.sqrt(hd),
                         dq=dqkv4[:, :, :h], dk=dqkv4[:, :, h : h + hkv], dv=dqkv4[:, :, h + hkv :],
                         rope=(cos, sin) if fused_rope else None)
@@ -337,7 +337,7 @@ class AttnHalfFn(torch.autograd.Function):
         qkv4 = qkv.view(b, s, h + 2 * hkv, hd)
         q, k, v = qkv4[:, :, :h], qkv4[:, :, h : h + hkv], qkv4[:, :, h + hkv :]
         dqkv4 = torch.empty_like(qkv4)
-        fused_rope = hd == 128 and kc.rope_tables_ok(cos, sin)
+        fused_rope = kc.rope_tables_ok(cos, sin)
         kc.attn_bwd(dattn.view(b, s, h, hd), q, k, v, attn2.view(b, s, h, hd), lse, True, None, 1.0 / math.sqrt(hd),
                     dq=dqkv4[:, :, :h], dk=dqkv4[:, :, h : h + hkv], dv=dqkv4[:, :, h + hkv :],
                     rope=(cos, sin) if fused_rope else None)
@@ -352,7 +352,7 @@ class AttnHalfFn(torch.autograd.Function):
 
 
 def attn_half_supported(block, x, kv_cache, doc_ids, key_padding_mask) -> bool:
-    """The fused attention sub-layer covers bf16 causal self-attention with head dim 128 on a GPU, without masks,
+    """The fused attention sub-layer covers bf16 causal self-attention with head dim 64 or 128 on a GPU, without masks,
     caches, q/k norms, tensor parallelism, fp8 or hooks; the feed-forward half of the block may be anything."""
     att = block.attention
     if not (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 3 and kv_cache is None and doc_ids is None
@@ -369,7 +369,7 @@ def attn_half_supported(block, x, kv_cache, doc_ids, key_padding_mask) -> bool:
         and not getattr(block, "fp8", False)
         and not getattr(block, "_kf_fp8_block", False)
         and not (unit is not None and getattr(unit, "sharded", False))
-        and att.head_dim == 128
+        and kc.attn_bwd_chosen(att.head_dim, x.shape[0] * (att.q_proj.weight.shape[0] // att.head_dim), x.shape[1], x.shape[1], True, False)
         and x.shape[-1] % 8 == 0
         and x.shape[0] * x.shape[1] >= 128
         and kc.attn_policy() == "native"
