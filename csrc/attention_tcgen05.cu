@@ -18,6 +18,7 @@
 // Replaces F.scaled_dot_product_attention and the repeat_interleave GQA expansion of the reference
 // (kempnerforge/model/attention.py:173-175,190-231) for the causal / document-masked cases.
 #include "attention_common.cuh"
+#include "skinny_common.cuh"
 
 namespace kf {
 namespace attn {
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 kf_attn_fwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ O,
                     float* __restrict__ LSE, const int* __restrict__ doc_ids, int Sq, int Sk, int H, int group,
-                    long long ldo, float scale_log2, int* status) {
+                    long long ldo, float scale_log2, int* status, int n_old) {
   using C = Cfg<HD>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -120,22 +121,32 @@ kf_attn_fwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // ------------------------------------------------------------ TMA producers
     // lane 0 feeds Q and the K ring, lane 1 the V ring: independent, so waiting for a V stage never
     // delays a K load (K_{j+1} is needed a whole tile before V_{j+1})
+    // In a programmatic launch (generation step) the tiles that hold only keys older than the previous kernel's writes
+    // travel before that kernel has finished.
+    auto old_tiles = [&](int stages) { return min(min(n_tiles, stages), n_old / BLK_N); };
     if (lane == 0) {
       bool ok = true;
       int issued = 0;
-      mbar_expect_tx(q_full, C::TILE_BYTES);
-#pragma unroll
-      for (int c = 0; c < C::BLOCKS; ++c)
-        tma_load_2d(q_smem + c * C::BLOCK_BYTES, &map_q, q_full, h * HD + 64 * c, b * Sq + m0);
-      for (int j = 0; j < n_tiles; ++j) {
+      auto load_k = [&](int j) {
         const int st = j % K_STAGES;
-        const int use = j / K_STAGES;  // how many times this stage has been filled before
-        if (use > 0 && !mbar_wait(k_empty(st), (use - 1) & 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
         mbar_expect_tx(k_full(st), C::TILE_BYTES);
 #pragma unroll
         for (int c = 0; c < C::BLOCKS; ++c)
           tma_load_2d(k_smem + st * C::TILE_BYTES + c * C::BLOCK_BYTES, &map_k, k_full(st), hk * HD + 64 * c,
                       b * Sk + j * BLK_N);
+      };
+      const int pre = old_tiles(K_STAGES);
+      for (; issued < pre; ++issued) load_k(issued);
+      grid_dep_wait();
+      mbar_expect_tx(q_full, C::TILE_BYTES);
+#pragma unroll
+      for (int c = 0; c < C::BLOCKS; ++c)
+        tma_load_2d(q_smem + c * C::BLOCK_BYTES, &map_q, q_full, h * HD + 64 * c, b * Sq + m0);
+      for (int j = pre; j < n_tiles; ++j) {
+        const int st = j % K_STAGES;
+        const int use = j / K_STAGES;  // how many times this stage has been filled before
+        if (use > 0 && !mbar_wait(k_empty(st), (use - 1) & 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
+        load_k(j);
         ++issued;
       }
       if (!ok) {
@@ -147,15 +158,22 @@ kf_attn_fwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     } else if (lane == 1) {
       bool ok = true;
       int issued = 0;
-      for (int j = 0; j < n_tiles; ++j) {
+      auto load_v = [&](int j) {
         const int st = j % V_STAGES;
-        const int use = j / V_STAGES;
-        if (use > 0 && !mbar_wait(v_empty(st), (use - 1) & 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
         mbar_expect_tx(v_full(st), C::TILE_BYTES);
 #pragma unroll
         for (int c = 0; c < C::BLOCKS; ++c)
           tma_load_2d(v_smem + st * C::TILE_BYTES + c * C::BLOCK_BYTES, &map_v, v_full(st), hk * HD + 64 * c,
                       b * Sk + j * BLK_N);
+      };
+      const int pre = old_tiles(V_STAGES);
+      for (; issued < pre; ++issued) load_v(issued);
+      grid_dep_wait();
+      for (int j = pre; j < n_tiles; ++j) {
+        const int st = j % V_STAGES;
+        const int use = j / V_STAGES;
+        if (use > 0 && !mbar_wait(v_empty(st), (use - 1) & 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
+        load_v(j);
         ++issued;
       }
       if (!ok) {
@@ -163,7 +181,12 @@ kf_attn_fwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           mbar_wait(v_full(j % V_STAGES), (j / V_STAGES) & 1, status, KF_ERR_WAIT_DRAIN);
       }
     }
+    __syncwarp();
+    grid_dep_wait();
+    grid_dep_launch();
   } else if (warp == 1) {
+    grid_dep_wait();
+    grid_dep_launch();
     // ------------------------------------------------------------ MMA issuer
     if (lane == 0) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(BLK_M, BLK_N, false, false);
@@ -217,6 +240,8 @@ kf_attn_fwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // its row maximum through shared memory once per tile; everything else (sums, O columns) is split.
     // After a failed wait a warp keeps walking the loop (without waiting) so that its partner never
     // blocks on a named barrier.
+    grid_dep_wait();  // this kernel's output may still be read, under another name, by kernels before the previous one
+    grid_dep_launch();
     const int quarter = warp & 3;
     const int half = (warp - 2) >> 2;
     const int r_local = quarter * 32 + lane;
@@ -380,7 +405,7 @@ kf_attn_fwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 template <int HD, bool CAUSAL, bool HAS_DOC>
 static int launch_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, void* O, float* LSE,
                       const int* doc, int B, int Sq, int Sk, int H, int Hkv, long long ldo, float scale,
-                      int* status, cudaStream_t stream) {
+                      int* status, int pdl, cudaStream_t stream) {
   auto kern = kf_attn_fwd_tcgen05<HD, CAUSAL, HAS_DOC>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -391,10 +416,18 @@ static int launch_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtens
     if (e != cudaSuccess) return 300 + (int)e;
     attr_set = true;
   }
-  dim3 grid((Sq + BLK_M - 1) / BLK_M, H, B);
-  kern<<<grid, THREADS, Cfg<HD>::SMEM, stream>>>(mq, mk, mv, reinterpret_cast<__nv_bfloat16*>(O), LSE, doc, Sq, Sk,
-                                                 H, H / Hkv, ldo, scale * 1.4426950408889634f, status);
-  cudaError_t e = cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((Sq + BLK_M - 1) / BLK_M, H, B);
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = Cfg<HD>::SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, reinterpret_cast<__nv_bfloat16*>(O), LSE, doc, Sq, Sk, H, H / Hkv, ldo,
+                                     scale * 1.4426950408889634f, status, pdl ? Sk - Sq : 0);
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
@@ -429,9 +462,10 @@ int kf_attn_fwd_occupancy(int hd) {
 // ids (requires Sq == Sk).  hd in {64, 128}; causal requires Sq == Sk.  Pitches must be multiples of 8
 // elements and the base pointers 16-byte aligned.  Returns 0 or an error code; errors of bounded waits go
 // to the library's status word.
-int kf_attn_fwd_bf16(const void* q, const void* k, const void* v, void* o, void* lse, const void* doc, int B,
-                     int Sq, int Sk, int H, int Hkv, int hd, long long ldq, long long ldk, long long ldv,
-                     long long ldo, float scale, int causal, void* stream) {
+// pdl: a programmatic launch behind a kernel that wrote q and the last Sq keys and values only (the older ones are read early).
+int kf_attn_fwd_pdl_bf16(const void* q, const void* k, const void* v, void* o, void* lse, const void* doc, int B,
+                         int Sq, int Sk, int H, int Hkv, int hd, long long ldq, long long ldk, long long ldv,
+                         long long ldo, float scale, int causal, int pdl, void* stream) {
   using namespace kf;
   using namespace kf::attn;
   if ((hd != 64 && hd != 128) || Hkv <= 0 || H % Hkv != 0) return 3;
@@ -449,7 +483,7 @@ int kf_attn_fwd_bf16(const void* q, const void* k, const void* v, void* o, void*
   float* L = reinterpret_cast<float*>(lse);
   const int* D = reinterpret_cast<const int*>(doc);
 #define KF_ATTN_LAUNCH(HD_, C_, D_) \
-  return launch_fwd<HD_, C_, D_>(mq, mk, mv, o, L, D, B, Sq, Sk, H, Hkv, ldo, scale, status, st)
+  return launch_fwd<HD_, C_, D_>(mq, mk, mv, o, L, D, B, Sq, Sk, H, Hkv, ldo, scale, status, pdl, st)
   if (hd == 128) {
     if (doc) { if (causal) KF_ATTN_LAUNCH(128, true, true); else KF_ATTN_LAUNCH(128, false, true); }
     if (causal) KF_ATTN_LAUNCH(128, true, false); else KF_ATTN_LAUNCH(128, false, false);
@@ -458,6 +492,12 @@ int kf_attn_fwd_bf16(const void* q, const void* k, const void* v, void* o, void*
     if (causal) KF_ATTN_LAUNCH(64, true, false); else KF_ATTN_LAUNCH(64, false, false);
   }
 #undef KF_ATTN_LAUNCH
+}
+
+int kf_attn_fwd_bf16(const void* q, const void* k, const void* v, void* o, void* lse, const void* doc, int B,
+                     int Sq, int Sk, int H, int Hkv, int hd, long long ldq, long long ldk, long long ldv,
+                     long long ldo, float scale, int causal, void* stream) {
+  return kf_attn_fwd_pdl_bf16(q, k, v, o, lse, doc, B, Sq, Sk, H, Hkv, hd, ldq, ldk, ldv, ldo, scale, causal, 0, stream);
 }
 
 }  // extern "C"

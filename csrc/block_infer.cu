@@ -4,22 +4,9 @@
 // output allocation) 5 - 15 us, so the block is launch-bound from Python.  This entry issues the whole chain
 //   RMSNorm -> q|k|v projection (rotary embedding, k and v into the cache) -> attention over the cache
 //   -> o projection (+ x) -> RMSNorm -> gate|up projection (SwiGLU) -> down projection (+ residual)
-// as programmatic launches: each kernel sets up (and streams its first weight tiles) while its predecessor drains.
+// as programmatic launches: each kernel sets up (and streams its first weight tiles) while its predecessor drains.  Up to
+// kf_skinny_norm_rows() sequences the projections take their norms along: five kernels in the chain instead of seven.
 #include "common.cuh"
-
-namespace kf {
-// k and v columns of q | k | v [B][qc + 2 kvc] -> one cache row per batch entry; 16 bytes per thread.
-__global__ void kf_kv_append(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict__ kc, __nv_bfloat16* __restrict__ vc,
-                             int B, int qc, int kvc, long long cache_batch) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, per = kvc / 4;  // k and v chunks of one entry
-  const int b = i / per, j = i % per;
-  if (b >= B) return;
-  const bool is_v = j >= kvc / 8;
-  const int c = (is_v ? j - kvc / 8 : j) * 8;
-  const uint4 w = *reinterpret_cast<const uint4*>(qkv + (size_t)b * (qc + 2 * kvc) + qc + (is_v ? kvc : 0) + c);
-  *reinterpret_cast<uint4*>((is_v ? vc : kc) + (size_t)b * cache_batch + c) = w;
-}
-}  // namespace kf
 
 extern "C" {
 int kf_rmsnorm_fwd_pdl_bf16(const void* x, const void* w, void* y, void* rstd, int rows, int D, float eps, int pdl,
@@ -27,26 +14,25 @@ int kf_rmsnorm_fwd_pdl_bf16(const void* x, const void* w, void* y, void* rstd, i
 int kf_gemm_skinny_bf16(const void* x, const void* w0, const void* w1, const void* w2, void* out, const void* residual,
                         int M, int K, int n0, int n1, int n2, int ldx, int ldw0, int ldw1, int ldw2, int ldo, int ldr,
                         int round_first, int pdl, int num_sms, void* stream);
-int kf_gemm_skinny_swiglu_bf16(const void* x, const void* wg, const void* wu, void* h, int M, int F, int K, int ldx,
-                               int ldwg, int ldwu, int ldh, int pdl, int num_sms, void* stream);
-int kf_gemm_skinny_qkv_bf16(const void* x, const void* wq, const void* wk, const void* wv, void* q_out, void* kc, void* vc,
-                            int M, int S, int K, int q_cols, int kv_cols, int ldx, int ldwq, int ldwk, int ldwv, int ldq,
-                            long long cache_batch, const void* cosT, const void* sinT, int pdl, int num_sms,
-                            void* stream);
+int kf_skinny_norm_rows();
+int kf_gemm_skinny_norm_swiglu_bf16(const void* x, const void* gain, float eps, const void* wg, const void* wu, void* h, int M,
+                                    int F, int K, int ldx, int ldwg, int ldwu, int ldh, int pdl, int num_sms, void* stream);
+int kf_gemm_skinny_norm_qkv_bf16(const void* x, const void* gain, float eps, const void* wq, const void* wk, const void* wv,
+                                 void* q_out, void* kc, void* vc, int M, int S, int K, int q_cols, int kv_cols, int hd, int ldx,
+                                 int ldwq, int ldwk, int ldwv, int ldq, long long cache_batch, const void* cosT,
+                                 const void* sinT, int pdl, int num_sms, void* stream);
 int kf_attn_decode_bf16(const void* q, const void* k, const void* v, void* o, int B, int Sk, int H, int Hkv, int hd,
                         long long ldq, long long ldo, long long kv_row, long long k_batch, long long v_batch, float scale,
                         int n_old, int pdl, int num_sms, void* stream);
-int kf_rope_bf16(const void* x, void* y, const void* cosT, const void* sinT, long long tokens, int S, int Htot, int n_rot,
-                 int hd, int inverse, void* stream);
-int kf_attn_fwd_bf16(const void* q, const void* k, const void* v, void* o, void* lse, const void* doc, int B, int Sq, int Sk,
-                     int H, int Hkv, int hd, long long ldq, long long ldk, long long ldv, long long ldo, float scale, int causal,
-                     void* stream);
+int kf_attn_fwd_pdl_bf16(const void* q, const void* k, const void* v, void* o, void* lse, const void* doc, int B, int Sq, int Sk,
+                         int H, int Hkv, int hd, long long ldq, long long ldk, long long ldv, long long ldo, float scale,
+                         int causal, int pdl, void* stream);
 
 // Attention half of a block for one new token in each of B sequences: h1 = x + Attention(RMSNorm(x)); with wd != null
 // also the SwiGLU half: y = h1 + MLP(RMSNorm(h1)).  All matrices [out][in] contiguous; x, h1, y [B][D] contiguous.
 // a: x, wn1, wq, wk, wv, wo, wn2, wg, wu, wd, kc, vc, scratch, rstd, h1, y, cosT, sinT (device pointers), then
 //    B, D, H, Hkv, hd, F, pos, cache_batch, num_sms;  r: eps1, eps2, scale
-//   scratch: bf16, B * (D + (H + 2 * Hkv) * hd) elements (+ B * F with wd), kept between calls for separate parts; rstd: fp32 [B]
+//   scratch: bf16, B * (D + H * hd) elements (+ B * F with wd), kept between calls for separate parts; rstd: fp32 [B]
 //   kc / vc: cache [B][positions][Hkv][hd], cache_batch elements between batch entries; `pos` = index of the new token
 //   cosT / sinT: fp32 [1][hd / 2], the row of the new position
 //   a[27]: parts to run (1 = up to the cache, 2 = attention, 4 = the rest); a[28]: attention kernel (0 = split over the cache,
@@ -67,34 +53,23 @@ int kf_block_decode_bf16(const long long* a, const double* r, void* stream) {
   const int qc = H * hd, kvc = Hkv * hd;
   bf* n = (bf*)scratch;                 // [B][D]
   bf* q = n + (size_t)B * D;            // [B][qc]
-  bf* hid = q + (size_t)B * (qc + 2 * kvc);  // [B][F]; q: [B][qc], or q | k | v for head dim 64
+  bf* hid = q + (size_t)B * qc;         // [B][F]
+  const bool norm_along = B <= kf_skinny_norm_rows();
   void* att = reinterpret_cast<void*>(a[29]);
   int rc;
   if (parts & 1) {
     const long long row = (long long)pos * kvc;
-    rc = kf_rmsnorm_fwd_pdl_bf16(x, wn1, n, rstd, B, D, eps1, 1, stream);
-    if (rc) return 1000 + rc;
-    if (hd == 128) {
-      rc = kf_gemm_skinny_qkv_bf16(n, wq, wk, wv, q, (bf*)kc + row, (bf*)vc + row, B, 1, D, qc, kvc, D, D, D, D, qc, cache_batch,
-                                   cosT, sinT, 1, num_sms, stream);
-    } else {
-      // Head dim 64: q | k | v [B][qc + 2 kvc], rotated by the rotary kernel of the op-by-op path.  The rotary epilogue gives
-      // the same values except for about one rounding in 10^5 (the compiler contracts a c - b s differently there), and one
-      // such bit decides over all later roundings of a small model.
-      rc = kf_gemm_skinny_bf16(n, wq, wk, wv, q, nullptr, B, D, qc, kvc, kvc, D, D, D, D, qc + 2 * kvc, 0, 0, 1, num_sms, stream);
-      if (!rc) rc = kf_rope_bf16(q, q, cosT, sinT, B, 1, H + 2 * Hkv, H + Hkv, hd, 0, stream);
-      if (!rc) {
-        const int chunks = B * kvc / 4;  // 16-byte pieces of k and of v
-        kf::kf_kv_append<<<(chunks + 255) / 256, 256, 0, (cudaStream_t)stream>>>(q, (bf*)kc + row, (bf*)vc + row, B, qc, kvc,
-                                                                               cache_batch);
-        rc = (int)cudaGetLastError();
-      }
+    if (!norm_along) {
+      rc = kf_rmsnorm_fwd_pdl_bf16(x, wn1, n, rstd, B, D, eps1, 1, stream);
+      if (rc) return 1000 + rc;
     }
+    rc = kf_gemm_skinny_norm_qkv_bf16(norm_along ? x : n, norm_along ? wn1 : nullptr, eps1, wq, wk, wv, q, (bf*)kc + row, (bf*)vc + row,
+                                      B, 1, D, qc, kvc, hd, D, D, D, D, qc, cache_batch, cosT, sinT, 1, num_sms, stream);
     if (rc) return 2000 + rc;
   }
   if (parts & 2) {
-    rc = tile_attention ? kf_attn_fwd_bf16(q, kc, vc, att, reinterpret_cast<void*>(a[30]), nullptr, 1, 1, pos + 1, H, Hkv, hd,
-                                           qc + 2 * kvc, kvc, kvc, qc, scale, 0, stream)
+    rc = tile_attention ? kf_attn_fwd_pdl_bf16(q, kc, vc, att, reinterpret_cast<void*>(a[30]), nullptr, 1, 1, pos + 1, H, Hkv, hd,
+                                               qc, kvc, kvc, qc, scale, 0, 1, stream)
                         : kf_attn_decode_bf16(q, kc, vc, att, B, pos + 1, H, Hkv, hd, qc, qc, kvc, cache_batch, cache_batch,
                                               scale, pos, 1, num_sms, stream);
     if (rc) return 3000 + rc;
@@ -105,9 +80,12 @@ int kf_block_decode_bf16(const long long* a, const double* r, void* stream) {
                            stream);
   if (rc) return 4000 + rc;
   if (!wd) return 0;
-  rc = kf_rmsnorm_fwd_pdl_bf16(h1, wn2, n, rstd, B, D, eps2, 1, stream);
-  if (rc) return 5000 + rc;
-  rc = kf_gemm_skinny_swiglu_bf16(n, wg, wu, hid, B, F, D, D, D, D, F, 1, num_sms, stream);
+  if (!norm_along) {
+    rc = kf_rmsnorm_fwd_pdl_bf16(h1, wn2, n, rstd, B, D, eps2, 1, stream);
+    if (rc) return 5000 + rc;
+  }
+  rc = kf_gemm_skinny_norm_swiglu_bf16(norm_along ? h1 : n, norm_along ? wn2 : nullptr, eps2, wg, wu, hid, B, F, D, D, D, D, F, 1,
+                                       num_sms, stream);
   if (rc) return 6000 + rc;
   rc = kf_gemm_skinny_bf16(hid, wd, nullptr, nullptr, y, h1, B, F, D, 0, 0, F, F, 0, 0, D, D, 1, 1, num_sms, stream);
   return rc ? 7000 + rc : 0;

@@ -380,8 +380,7 @@ __global__ void kf_rope(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __re
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const float c = cp[i], s = inverse ? -sp[i] : sp[i];
-        oa.v[i] = a.v[i] * c - b.v[i] * s;
-        ob.v[i] = b.v[i] * c + a.v[i] * s;
+        rotate_pair(a.v[i], b.v[i], c, s, oa.v[i], ob.v[i]);
       }
       a = oa;
       b = ob;

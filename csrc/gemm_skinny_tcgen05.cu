@@ -14,14 +14,19 @@
 //     triggers its dependents does so after its own wait, so when a block of this grid starts, all work before the
 //     immediately preceding kernel is complete and visible; that kernel itself never writes weights.)
 //
+// With NORM the operand is RMSNorm(x) and x comes in as it is: the four epilogue warps, idle until the accumulator is done,
+// compute each row's scale and write the normalised 64-column blocks into the ring, in the arithmetic and order of
+// kf_rmsnorm_fwd (the same bits).  A norm kernel of its own is a link of 2 - 3 us in the chain of a generation step (wait,
+// load, two block barriers, drain); up to NORM_ROWS rows every CTA repeats that work from L2 for less (a 7B block on one token
+// 95.7 -> 92.0 us).
+//
 // Epilogues: 0 = (+ residual); 1 = SwiGLU over W = [gate ; up] (64 gate and the matching 64 up rows share a tile);
-// 2 = rotary embedding of the q and k heads with k and v stored straight into the KV cache.
+// 2 = rotary embedding of the q and k heads (64 or 128 wide) with k and v stored straight into the KV cache.
 //
 //   warp 0: TMA producer; warp 1: MMA issuer, owns TMEM; warps 2-5: accumulator -> shared memory; all: reduction + store
 //
 // Covers the Linear call sites of the reference during generation (kempnerforge/model/generate.py:66-131).
-#include "common.cuh"
-#include "skinny_common.cuh"
+#include "skinny_args.cuh"
 
 namespace kf {
 namespace skinny {
@@ -30,6 +35,7 @@ constexpr int WROWS = 128;
 constexpr int BK = 64;
 constexpr int THREADS = 192;
 constexpr int W_BYTES = WROWS * BK * 2;  // 16 KB
+static_assert(NORM_ROWS <= 4, "a warp writes one ring stage: 8 lanes per row");
 
 template <int NT>
 struct Cfg {
@@ -40,23 +46,6 @@ struct Cfg {
   static constexpr int RED_BYTES = NT * WROWS * 4;  // reduction buffer, aliases the ring
   static constexpr int BODY = STAGES * STAGE > RED_BYTES ? STAGES * STAGE : RED_BYTES;
   static constexpr size_t SMEM = size_t(BODY) + 1024 + 256;
-};
-
-struct Args {
-  __nv_bfloat16* out;            // [M][ldo]
-  const __nv_bfloat16* residual; // [M][ldr] or null (epilogue 0)
-  int M, K, ldo, ldr;
-  int round_first;               // residual: round the product to bf16 before adding, as separate kernels do
-  int n_seg;
-  int tile0[4];   // first tile of each segment (epilogue 1: of the hidden dimension)
-  int rows[3];    // rows of each segment
-  int col[3];     // output column of each segment's first row
-  // epilogue 2
-  __nv_bfloat16 *kc, *vc;        // cache rows [batch][position][kv_dim], already offset to the first new position
-  long long cache_batch;         // elements between batch entries
-  const float *cosT, *sinT;      // [S][64], row 0 = first new position
-  int S, kv_cols;
-  int pdl;
 };
 
 __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t cta) {
@@ -70,7 +59,7 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
   return v;
 }
 
-template <int NT, int EPI>
+template <int NT, int EPI, bool NORM>
 __global__ void __launch_bounds__(THREADS)
 kf_gemm_skinny(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w0,
                const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_w2,
@@ -84,6 +73,8 @@ kf_gemm_skinny(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   const uint32_t acc_bar = bar_base + 8u * (2 * C::STAGES);
   const uint32_t tmem_slot = bar_base + 8u * (2 * C::STAGES + 1);
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
+  float* norm_red = reinterpret_cast<float*>(smem_raw + (bar_base + 128 - smem_u32(smem_raw)));  // [NORM_ROWS][8]
+  static_assert(8 * (2 * C::STAGES + 1) + 4 <= 128 && NORM_ROWS * 8 * 4 <= 128, "barriers, then the partial sums");
   float* red = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw)));
   constexpr int TMEM_COLS = NT < 32 ? 32 : NT;
 
@@ -102,12 +93,12 @@ kf_gemm_skinny(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
-      mbar_init(full_bar(s), 1);
+      mbar_init(full_bar(s), NORM ? 2 : 1);  // NORM: and the warp that wrote the x block
       mbar_init(empty_bar(s), 1);
     }
     mbar_init(acc_bar, 1);
     mbar_fence_init();
-    tma_prefetch_desc(&map_x);
+    if (!NORM) tma_prefetch_desc(&map_x);
     tma_prefetch_desc(seg == 0 ? &map_w0 : seg == 1 ? &map_w1 : &map_w2);
     if (EPI == 1) tma_prefetch_desc(&map_w1);
   }
@@ -127,7 +118,7 @@ kf_gemm_skinny(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       auto load_w = [&](int i) {
         const int s = i % C::STAGES, k0 = (kb0 + i) * BK;
         const uint32_t dst = smem_base + s * C::STAGE;
-        mbar_expect_tx(full_bar(s), C::STAGE);
+        mbar_expect_tx(full_bar(s), NORM ? W_BYTES : C::STAGE);
         if (EPI == 1) {
           tma_load_2d(dst, &map_w0, full_bar(s), k0, row0);
           tma_load_2d(dst + W_BYTES / 2, &map_w1, full_bar(s), k0, row0);
@@ -141,14 +132,16 @@ kf_gemm_skinny(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       };
       const int pre = min(n_kb, C::STAGES);
       for (int i = 0; i < pre; ++i) load_w(i);
-      grid_dep_wait();
-      for (int i = 0; i < pre; ++i) load_x(i);
+      if (!NORM) {
+        grid_dep_wait();
+        for (int i = 0; i < pre; ++i) load_x(i);
+      }
       int i = pre;
       for (; i < n_kb; ++i) {
         const int s = i % C::STAGES;
         if (!mbar_wait(empty_bar(s), ((i / C::STAGES) - 1) & 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
         load_w(i);
-        load_x(i);
+        if (!NORM) load_x(i);
       }
       // on the error path nobody consumes the stages: wait for the copies still landing in this CTA's shared memory
       if (!ok)
@@ -181,6 +174,43 @@ kf_gemm_skinny(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     // ------------------------------------------------------------ accumulator -> reduction buffer [token][W row]
     const int quarter = warp & 3;
     grid_dep_wait();
+    if constexpr (NORM) {
+      const int t = threadIdx.x - 64, nvec = a.K >> 3;  // threads t and t + 128 of the norm kernel's 256
+      for (int r = 0; r < a.M; ++r) {
+        const __nv_bfloat16* xr = a.x + size_t(r) * a.ldx;
+        float ss[2] = {0.f, 0.f};
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          for (int v = t + 128 * h; v < nvec; v += 256) add_squares(*reinterpret_cast<const uint4*>(xr + v * 8), ss[h]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          ss[h] = norm_warp_sum(ss[h]);
+          if (lane == 0) norm_red[r * 8 + (t >> 5) + 4 * h] = ss[h];
+        }
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      const int r = lane >> 3, ch = lane & 7;  // this lane's row and 16-byte chunk of a block
+      float rstd = 0.f;
+      for (int i = 0; i < a.M; ++i) {
+        const float ri = norm_rstd(norm_red + i * 8, lane, a.K, a.eps);
+        if (i == r) rstd = ri;
+      }
+      const __nv_bfloat16* xr = a.x + size_t(r < a.M ? r : 0) * a.ldx;
+      for (int i = t >> 5; i < n_kb; i += 4) {
+        const int s = i % C::STAGES, col = (kb0 + i) * BK + ch * 8;
+        uint4 u = make_uint4(0, 0, 0, 0);
+        if (r < a.M && col < a.K)
+          u = norm_vec(*reinterpret_cast<const uint4*>(xr + col), *reinterpret_cast<const uint4*>(a.gain + col), rstd);
+        if (i >= C::STAGES && !mbar_wait(empty_bar(s), ((i / C::STAGES) - 1) & 1, status, KF_ERR_WAIT_EMPTY)) break;
+        if (r < a.M) {  // rows past M feed accumulator columns that nobody reads
+          const uint32_t dst = smem_base + s * C::STAGE + W_BYTES + uint32_t(r * 128 + ((ch ^ (r & 7)) << 4));
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(u.x), "r"(u.y), "r"(u.z), "r"(u.w) : "memory");
+        }
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full_bar(s));
+      }
+    }
     ok = mbar_wait(acc_bar, 0, status, KF_ERR_WAIT_TMEM_FULL);
     tc_fence_after();
     const uint32_t t_row = tmem_base + (uint32_t(quarter * 32) << 16);
@@ -271,23 +301,23 @@ kf_gemm_skinny(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       store8(a.out + size_t(t) * a.ldo + row0 + n, g);
     }
   } else {
-    // one head of 128 columns per tile: pairs (n, n + 64).  Tokens t = (batch, new position).
-    constexpr int half = WROWS / 2, vec = half / 8;  // 8-wide pieces of a half head
-    for (int i = first; i < a.M * vec; i += step) {
-      const int t = i / vec, n = (i % vec) * 8;
+    // one head of 128 columns or two of 64 per tile: pairs (n, n + half).  Tokens t = (batch, new position).
+    const int half = a.hd >> 1, vec = half >> 3;  // 8-wide pieces of a half head; 8 pairs of pieces per token and tile
+    for (int i = first; i < a.M * 8; i += step) {
+      const int t = i >> 3, head = (i & 7) / vec, m = (i & 7) % vec * 8, n = head * a.hd + m;
       const int b = t / a.S, pos = t - b * a.S;
+      if (row0 + n >= a.rows[seg]) continue;
       float lo[8], hi[8];
       sum8(t, n, lo);
       sum8(t, n + half, hi);
       if (seg < 2) {
-        const float* cs = a.cosT + size_t(pos) * half + n;
-        const float* sn = a.sinT + size_t(pos) * half + n;
+        const float* cs = a.cosT + size_t(pos) * half + m;
+        const float* sn = a.sinT + size_t(pos) * half + m;
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           // the projection is rounded to bf16 before the rotation, like the separate kernels do
           const float x = __bfloat162float(__float2bfloat16(lo[e])), y = __bfloat162float(__float2bfloat16(hi[e]));
-          lo[e] = x * cs[e] - y * sn[e];
-          hi[e] = y * cs[e] + x * sn[e];
+          rotate_pair(x, y, cs[e], sn[e], lo[e], hi[e]);
         }
       }
       __nv_bfloat16* p = seg == 0 ? a.out + size_t(t) * a.ldo + row0 + n
@@ -302,21 +332,23 @@ kf_gemm_skinny(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
 // Number of CTAs a K range is split over: enough of them to fill the SMs, at least MIN_KB ring steps each.  Weights of less
 // than 8 MB (512 blocks of 128 x 64) are not split, so that the projections of small models sum over K in the order of the tile
 // kernels and keep their bits: in a model of a few layers every rounding travels on, and one that falls differently moves the
-// logits by as much as all of them together are off.  That costs time: one row, L2 flushed, unsplit / split: 768 x 768 7.0 / 5.6
-// us, 2304 x 768 7.3 / 6.1, 768 x 2048 12.7 / 6.6, 1024 x 3072 17.6 / 7.9.
+// logits by as much as all of them together are off.  That costs time (one row, L2 flushed, unsplit / split: 768 x 768 7.0 / 5.6
+// us, 2304 x 768 7.3 / 6.1, 768 x 2048 12.7 / 6.6, 1024 x 3072 17.6 / 7.9), which gemm_small.cu gets back for up to 16 rows.
+static bool small_weight(int tiles, int k_blocks) { return tiles * k_blocks < 512; }
+
 static int pick_splits(int tiles, int k_blocks, int num_sms, int per_sm) {
   constexpr int MIN_KB = 4;
-  if (tiles * k_blocks < 512) return 1;
+  if (small_weight(tiles, k_blocks)) return 1;
   int s = 1;
   while (s < 8 && tiles * s * 2 <= num_sms * per_sm && k_blocks >= 2 * s * MIN_KB) s *= 2;
   return s;
 }
 
-template <int NT, int EPI>
+template <int NT, int EPI, bool NORM = false>
 static int launch(const CUtensorMap& mx, const CUtensorMap (&mw)[3], const Args& a, int tiles, int num_sms, int* status,
                   cudaStream_t stream) {
   using C = Cfg<NT>;
-  auto kern = kf_gemm_skinny<NT, EPI>;
+  auto kern = kf_gemm_skinny<NT, EPI, NORM>;
   static bool attr_set[16] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -348,13 +380,21 @@ static int dispatch(const void* x, int ldx, const void* const* w, const int* ldw
                     int* status, cudaStream_t stream) {
   const int nt = a.M <= 16 ? 16 : a.M <= 32 ? 32 : a.M <= 64 ? 64 : a.M <= 128 ? 128 : 256;
   CUtensorMap mx, mw[3];
-  int rc = make_map_2d_bf16(&mx, x, a.M, a.K, ldx, BK, nt);
+  int rc = 0;
+  a.x = (const __nv_bfloat16*)x;
+  a.ldx = ldx;
+  if (a.gain && a.M > NORM_ROWS) return 5;
+  if (small_fits(a, EPI, small_weight(tiles, (a.K + BK - 1) / BK), num_sms)) return run_small(EPI, w, ldw, a, status, stream);
+  if (!a.gain) rc = make_map_2d_bf16(&mx, x, a.M, a.K, ldx, BK, nt);
   if (rc) return 100 + rc;
   for (int i = 0; i < a.n_seg; ++i) {
     rc = make_map_2d_bf16(&mw[i], w[i], a.rows[i], a.K, ldw[i], BK, EPI == 1 ? 64 : WROWS);
     if (rc) return 200 + rc;
   }
   for (int i = a.n_seg; i < 3; ++i) mw[i] = mw[0];  // never read
+  if constexpr (EPI != 0) {
+    if (a.gain) return launch<16, EPI, true>(mw[0], mw, a, tiles, num_sms, status, stream);
+  }
   switch (nt) {
     case 16: return launch<16, EPI>(mx, mw, a, tiles, num_sms, status, stream);
     case 32: return launch<32, EPI>(mx, mw, a, tiles, num_sms, status, stream);
@@ -399,9 +439,12 @@ int kf_gemm_skinny_bf16(const void* x, const void* w0, const void* w1, const voi
   return dispatch<0>(x, ldx, w, ldw, a, tiles, num_sms, (int*)kf_status_device_ptr(), (cudaStream_t)stream);
 }
 
-// h[M, F] = silu(x Wg^T) * (x Wu^T); 1 <= M <= 256.
-int kf_gemm_skinny_swiglu_bf16(const void* x, const void* wg, const void* wu, void* h, int M, int F, int K, int ldx,
-                               int ldwg, int ldwu, int ldh, int pdl, int num_sms, void* stream) {
+// Rows up to which kf_gemm_skinny_norm_* take the norm of their input along.
+int kf_skinny_norm_rows() { return kf::skinny::NORM_ROWS; }
+
+// h[M, F] = silu(n Wg^T) * (n Wu^T); 1 <= M <= 256.  gain null: n = x; else n = RMSNorm(x) with it, M <= kf_skinny_norm_rows().
+int kf_gemm_skinny_norm_swiglu_bf16(const void* x, const void* gain, float eps, const void* wg, const void* wu, void* h, int M,
+                                    int F, int K, int ldx, int ldwg, int ldwu, int ldh, int pdl, int num_sms, void* stream) {
   using namespace kf::skinny;
   if (M < 1 || M > 256 || K < 8 || F < 8 || ((K | F | ldx | ldwg | ldwu | ldh) & 7)) return 5;
   const void* w[3] = {wg, wu, nullptr};
@@ -409,22 +452,29 @@ int kf_gemm_skinny_swiglu_bf16(const void* x, const void* wg, const void* wu, vo
   Args a{};
   a.out = (__nv_bfloat16*)h;
   a.M = M; a.K = K; a.ldo = ldh; a.pdl = pdl;
+  a.gain = (const __nv_bfloat16*)gain;
+  a.eps = eps;
   a.n_seg = 2;
   a.rows[0] = a.rows[1] = F;
   return dispatch<1>(x, ldx, w, ldw, a, (F + 63) / 64, num_sms, (int*)kf_status_device_ptr(), (cudaStream_t)stream);
 }
 
+int kf_gemm_skinny_swiglu_bf16(const void* x, const void* wg, const void* wu, void* h, int M, int F, int K, int ldx,
+                               int ldwg, int ldwu, int ldh, int pdl, int num_sms, void* stream) {
+  return kf_gemm_skinny_norm_swiglu_bf16(x, nullptr, 0.f, wg, wu, h, M, F, K, ldx, ldwg, ldwu, ldh, pdl, num_sms, stream);
+}
+
 // Fused q | k | v projection of M = B * S new tokens with the rotary embedding: q (rotated) -> q_out [M][ldq], k (rotated)
 // and v -> cache rows kc / vc ([B][..][kv_cols], `cache_batch` elements between batch entries, pointing at the first new
-// position).  cosT / sinT: fp32 [S][64] of the new positions.  Head dim 128; q_cols and kv_cols multiples of it.
-int kf_gemm_skinny_qkv_bf16(const void* x, const void* wq, const void* wk, const void* wv, void* q_out, void* kc, void* vc,
-                            int M, int S, int K, int q_cols, int kv_cols, int ldx, int ldwq, int ldwk, int ldwv, int ldq,
-                            long long cache_batch, const void* cosT, const void* sinT, int pdl, int num_sms,
-                            void* stream) {
+// position).  cosT / sinT: fp32 [S][hd / 2] of the new positions.  hd 64 or 128; q_cols and kv_cols multiples of it.
+// gain null: of x itself; else of RMSNorm(x) with it, M <= kf_skinny_norm_rows().
+int kf_gemm_skinny_norm_qkv_bf16(const void* x, const void* gain, float eps, const void* wq, const void* wk, const void* wv,
+                                 void* q_out, void* kc, void* vc, int M, int S, int K, int q_cols, int kv_cols, int hd, int ldx,
+                                 int ldwq, int ldwk, int ldwv, int ldq, long long cache_batch, const void* cosT,
+                                 const void* sinT, int pdl, int num_sms, void* stream) {
   using namespace kf::skinny;
-  constexpr int hd = WROWS;  // a tile of W rows is one head
-  if (M < 1 || M > 256 || S < 1 || M % S || K < 8 || ((K | ldx | ldwq | ldwk | ldwv | ldq) & 7) || (cache_batch & 7) ||
-      q_cols % hd || kv_cols % hd || q_cols < hd || kv_cols < hd)
+  if ((hd != 64 && hd != 128) || M < 1 || M > 256 || S < 1 || M % S || K < 8 || ((K | ldx | ldwq | ldwk | ldwv | ldq) & 7) ||
+      (cache_batch & 7) || q_cols % hd || kv_cols % hd || q_cols < hd || kv_cols < hd)
     return 5;
   const void* w[3] = {wq, wk, wv};
   const int ldw[3] = {ldwq, ldwk, ldwv}, n[3] = {q_cols, kv_cols, kv_cols};
@@ -436,7 +486,9 @@ int kf_gemm_skinny_qkv_bf16(const void* x, const void* wq, const void* wk, const
   a.cache_batch = cache_batch;
   a.cosT = (const float*)cosT;
   a.sinT = (const float*)sinT;
-  a.S = S; a.kv_cols = kv_cols;
+  a.S = S; a.kv_cols = kv_cols; a.hd = hd;
+  a.gain = (const __nv_bfloat16*)gain;
+  a.eps = eps;
   int tiles = 0;
   for (a.n_seg = 0; a.n_seg < 3; ++a.n_seg) {
     a.tile0[a.n_seg] = tiles;
@@ -444,6 +496,14 @@ int kf_gemm_skinny_qkv_bf16(const void* x, const void* wq, const void* wk, const
     tiles += (n[a.n_seg] + WROWS - 1) / WROWS;
   }
   return dispatch<2>(x, ldx, w, ldw, a, tiles, num_sms, (int*)kf_status_device_ptr(), (cudaStream_t)stream);
+}
+
+int kf_gemm_skinny_qkv_bf16(const void* x, const void* wq, const void* wk, const void* wv, void* q_out, void* kc, void* vc,
+                            int M, int S, int K, int q_cols, int kv_cols, int ldx, int ldwq, int ldwk, int ldwv, int ldq,
+                            long long cache_batch, const void* cosT, const void* sinT, int pdl, int num_sms,
+                            void* stream) {
+  return kf_gemm_skinny_norm_qkv_bf16(x, nullptr, 0.f, wq, wk, wv, q_out, kc, vc, M, S, K, q_cols, kv_cols, 128, ldx, ldwq, ldwk,
+                                      ldwv, ldq, cache_batch, cosT, sinT, pdl, num_sms, stream);
 }
 
 }  // extern "C"

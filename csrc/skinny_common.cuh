@@ -25,4 +25,18 @@ __device__ __forceinline__ void cluster_sync_all() {
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+
+// (x, y) rotated by the angle of (c, s), spelled out so that the rotary kernel and the epilogues of generation steps give the same
+// bits: left to the compiler, which of the two products is fused with the sum differs between kernels, one bf16 value in 10^5.
+__device__ __forceinline__ void rotate_pair(float x, float y, float c, float s, float& rx, float& ry) {
+  rx = __fmaf_rn(x, c, -__fmul_rn(y, s));
+  ry = __fmaf_rn(y, c, __fmul_rn(x, s));
+}
+
+__device__ __forceinline__ float norm_warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 }  // namespace kf

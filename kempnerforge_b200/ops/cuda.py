@@ -59,6 +59,10 @@ def _declare(L: ctypes.CDLL) -> None:
         "kf_gemm_skinny_bf16": [vp] * 6 + [i] * 14 + [vp],
         "kf_gemm_skinny_swiglu_bf16": [vp] * 4 + [i] * 9 + [vp],
         "kf_gemm_skinny_qkv_bf16": [vp] * 7 + [i] * 10 + [ll, vp, vp, i, i, vp],
+        "kf_skinny_norm_rows": [],
+        "kf_gemm_skinny_norm_swiglu_bf16": [vp, vp, f, vp, vp, vp] + [i] * 9 + [vp],
+        "kf_gemm_skinny_norm_qkv_bf16": [vp, vp, f] + [vp] * 6 + [i] * 11 + [ll, vp, vp, i, i, vp],
+        "kf_attn_fwd_pdl_bf16": [vp] * 6 + [i] * 6 + [ll] * 4 + [f, i, i, vp],
         "kf_rmsnorm_fwd_pdl_bf16": [vp, vp, vp, vp, i, i, f, i, vp],
         "kf_attn_decode_bf16": [vp] * 4 + [i] * 5 + [ll] * 5 + [f, i, i, i, vp],
         "kf_block_decode_bf16": [vp, vp, vp],
@@ -428,34 +432,34 @@ def block_decode(y: torch.Tensor, attn_ptrs, mlp_ptrs, cache_ptrs, table_ptrs, d
 
     Attention runs on the kernel split over the cache for head dim 128.  With head dim 64 it stays on what the op-by-op path
     uses: the 128-row tile kernel for one sequence, ``foreign(q)`` (rows of H hd) -> dense (B, H hd) between two native calls
-    for more; the rotation is the separate kernel's too.  The reason is that a small model's logits stay bit for bit the same, not
+    for more.  The reason is that a small model's logits stay bit for bit the same, not
     speed.  Measured (12 heads of 64, one query head per KV head, us, at 300 / 1000 / 2000 / 4000 positions): one sequence, split
     kernel 5.2 / 6.3 / 7.7 / 10.1, tile kernel 7.7 / 12.3 / 19.7 / 34.7, library 4.9 / 6.5 / 7.9 / 8.8; four sequences, split
     6.1 / 8.2 / 11.1 / 17.3, library 5.4 / 7.2 / 9.6 / 14.6; sixteen, split 9.7 / 18.9 / 31.2 / 54.8, library 9.2 / 16.9 / 25.6 /
     40.4."""
     b, d, h, hkv, hd, f = dims[:6]
     tile = hd == 64 and b == 1
-    qc, row = h * hd, (h + 2 * hkv) * hd
-    # one buffer for all intermediates: n (D) | q, or q | k | v | hidden (F) | h1 (D) | attention (H hd) | rstd, lse
-    scratch = torch.empty(b * (2 * d + row + qc + f) + 2 * b + 2 * h, dtype=torch.bfloat16, device=y.device)
+    qc = h * hd
+    # one buffer for all intermediates: n (D) | q (H hd) | hidden (F) | h1 (D) | attention (H hd) | rstd, lse
+    scratch = torch.empty(b * (2 * d + 2 * qc + f) + 2 * b + 2 * h, dtype=torch.bfloat16, device=y.device)
     base = scratch.data_ptr()
-    att = base + 2 * b * (2 * d + row + f)
+    att = base + 2 * b * (2 * d + qc + f)
     rstd = att + 2 * b * qc
     yp = y.data_ptr()
-    h1 = base + 2 * b * (d + row + f) if mlp_ptrs else yp
+    h1 = base + 2 * b * (d + qc + f) if mlp_ptrs else yp
     ints = array("q", (*attn_ptrs, *(mlp_ptrs or (0, 0, 0, 0)), *cache_ptrs, base, rstd, h1, yp, *table_ptrs, *dims, sm_count(),
                        7, int(tile), att, rstd + 4 * b))
     reals = array("d", scalars)
     fn, ip, rp = lib().kf_block_decode_bf16, ints.buffer_info()[0], reals.buffer_info()[0]
-    extra = 2 if hd == 64 else 0
+    norms = 0 if b <= lib().kf_skinny_norm_rows() else 1   # norm kernels per half of the block
     if hd == 64 and b > 1:
         ints[27] = 1
-        _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 2 + extra)
-        out = foreign(scratch[b * d : b * (d + row)].view(b, row)[:, :qc])
+        _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 1 + norms)
+        out = foreign(scratch[b * d : b * (d + qc)].view(b, qc))
         ints[27], ints[29] = 4, out.data_ptr()
-        _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 4 if mlp_ptrs else 1)
+        _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 3 + norms if mlp_ptrs else 1)
         return
-    _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", (7 if mlp_ptrs else 4) + extra)
+    _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 5 + 2 * norms if mlp_ptrs else 3 + norms)
 
 
 # --------------------------------------------------------------------------- norm / rope / swiglu / embedding

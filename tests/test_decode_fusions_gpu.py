@@ -1,0 +1,74 @@
+"""Projections of a generation step that take the norm and the rotation along: bit for bit the separate kernels."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+def _rand(*shape, scale=1.0, seed=0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return (torch.randn(*shape, device=DEV, generator=g) * scale).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("m,f,k", [(1, 64, 8), (1, 200, 72), (2, 2048, 768), (3, 136, 2056), (4, 14336, 4096), (4, 1024, 5120), (1, 64, 9000)])
+def test_norm_along_with_swiglu(native_lib, m, f, k):
+    kc, L = native_lib, native_lib.lib()
+    assert m <= L.kf_skinny_norm_rows()
+    x = _rand(m + 1, k + 8, scale=3.0, seed=1)[:m, :k]                       # a row pitch of its own
+    gain, wg, wu = 1 + 0.1 * _rand(k, seed=2), _rand(f, k, scale=k**-0.5, seed=3), _rand(f, k, scale=k**-0.5, seed=4)
+    n, _ = kc.rmsnorm_fwd(x.contiguous(), gain, 1e-5)
+    out = []
+    for src, g in ((n, None), (x, gain.data_ptr())):
+        h = torch.empty(m, f, dtype=torch.bfloat16, device=DEV)
+        kc._check(L.kf_gemm_skinny_norm_swiglu_bf16(src.data_ptr(), g, 1e-5, wg.data_ptr(), wu.data_ptr(), h.data_ptr(), m, f, k,
+                                                    src.stride(0), k, k, f, 0, kc.sm_count(), kc._stream()), "swiglu")
+        out.append(h)
+    assert native_lib.read_status() == 0
+    assert torch.equal(*out)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("b,heads,kv,k", [(1, 12, 12, 768), (2, 3, 1, 264), (4, 16, 4, 2048), (5, 6, 3, 520), (33, 4, 2, 768)])
+def test_projection_rotation_and_cache(native_lib, b, heads, kv, k, hd):
+    kc, L = native_lib, native_lib.lib()
+    qc, kvc = heads * hd, kv * hd
+    x, gain = _rand(b, k, seed=1), 1 + 0.1 * _rand(k, seed=2)
+    ws = [_rand(n, k, scale=k**-0.5, seed=3 + i) for i, n in enumerate((qc, kvc, kvc))]
+    ang = torch.rand(1, hd // 2, device=DEV, generator=torch.Generator(device=DEV).manual_seed(9)) * 6.0
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    n, _ = kc.rmsnorm_fwd(x, gain, 1e-5)
+    qkv = kc.gemm_rows(n, ws).view(b, 1, heads + 2 * kv, hd)
+    kc.rope(qkv, cos, sin, heads + kv, inverse=False, out=qkv)
+    want = qkv.view(b, -1).split([qc, kvc, kvc], 1)
+    for src, g in ((n, None), (x, gain.data_ptr())) if b <= L.kf_skinny_norm_rows() else ((n, None),):
+        q = torch.empty(b, qc, dtype=torch.bfloat16, device=DEV)
+        cache = torch.full((2, b, 3, kvc), 7.0, dtype=torch.bfloat16, device=DEV)
+        kc._check(L.kf_gemm_skinny_norm_qkv_bf16(src.data_ptr(), g, 1e-5, *(w.data_ptr() for w in ws), q.data_ptr(),
+                                                 cache[0, 0, 1].data_ptr(), cache[1, 0, 1].data_ptr(), b, 1, k, qc, kvc, hd, k, k, k, k, qc,
+                                                 3 * kvc, cos.data_ptr(), sin.data_ptr(), 0, kc.sm_count(), kc._stream()), "qkv")
+        assert native_lib.read_status() == 0
+        for got, w in zip((q, cache[0, :, 1], cache[1, :, 1]), want):
+            assert torch.equal(got, w)
+        assert bool((cache[:, :, 0] == 7).all()) and bool((cache[:, :, 2] == 7).all())
+    assert L.kf_gemm_skinny_norm_qkv_bf16(x.data_ptr(), gain.data_ptr(), 1e-5, *(w.data_ptr() for w in ws), q.data_ptr(),
+                                          cache.data_ptr(), cache.data_ptr(), L.kf_skinny_norm_rows() + 1, 1, k, qc, kvc, hd, k, k, k, k,
+                                          qc, 3 * kvc, cos.data_ptr(), sin.data_ptr(), 0, kc.sm_count(), kc._stream()) == 5
+
+
+@pytest.mark.parametrize("m", [1, 2, 7, 8, 9, 16])
+@pytest.mark.parametrize("rows,k", [([8], 32), ([768], 768), ([24, 40, 8], 96), ([768], 2048), ([256, 64], 1504), ([512], 4096)])
+def test_small_weights_keep_the_bits_of_the_tile_kernel(native_lib, m, rows, k):
+    kc = native_lib
+    x = _rand(m, k + 8, seed=1)[:, :k]
+    ws = [_rand(n, k + 16, scale=0.3, seed=2 + i)[:, :k] for i, n in enumerate(rows)]
+    res = _rand(m, sum(rows), seed=7)
+    frame = torch.full((m + 1, sum(rows) + 8), 7.0, dtype=torch.bfloat16, device=DEV)
+    out = kc._stream_rows(x, ws, None, frame[:m, : sum(rows)])
+    with_res = kc._stream_rows(x, ws, res, None)
+    assert kc.read_status() == 0
+    w = torch.cat(ws)
+    assert torch.equal(out, kc.gemm(x, w, mode=1)) and torch.equal(with_res, kc.gemm(x, w, residual=res, mode=1))
+    assert bool((frame[m:] == 7).all()) and bool((frame[:, sum(rows):] == 7).all())
