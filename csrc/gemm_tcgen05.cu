@@ -44,9 +44,16 @@ __device__ __forceinline__ TileCoord tile_coord(int t, int m_blocks, int n_block
   return tc;
 }
 
+// B operand.  An MN-major one may be up to three matrices stacked along K (the weights of a fused projection read for their
+// input gradient): start[i] = first k of matrix i, a multiple of BK; one piece: start[1] = start[2] = INT_MAX.
+struct BSegs {
+  CUtensorMap map[3];
+  int start[3];
+};
+
 template <bool A_MN, bool B_MN, typename OutT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-kf_gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+kf_gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ BSegs bs,
                      OutT* __restrict__ C, const OutT* __restrict__ R, int M, int N, int K, int ldc, int ldr, int accumulate,
                      int* status) {
   extern __shared__ uint8_t smem_raw[];
@@ -82,7 +89,7 @@ kf_gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_con
     mbar_init(drain_bar, 1);
     mbar_fence_init();
     tma_prefetch_desc(&map_a);
-    tma_prefetch_desc(&map_b);
+    tma_prefetch_desc(&bs.map[0]);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, TMEM_COLS);
@@ -117,11 +124,12 @@ kf_gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_con
               tma_load_2d(a_dst + c * (64 * BK * 2), &map_a, full_bar(s), m0 + 64 * c, k0);
           }
           if (!B_MN) {
-            tma_load_2d(b_dst, &map_b, full_bar(s), k0, n0);
+            tma_load_2d(b_dst, &bs.map[0], full_bar(s), k0, n0);
           } else {
+            const int ks = int(k0 >= bs.start[1]) + int(k0 >= bs.start[2]);
 #pragma unroll
             for (int c = 0; c < BN / 64; ++c)
-              tma_load_2d(b_dst + c * (64 * BK * 2), &map_b, full_bar(s), n0 + 64 * c, k0);
+              tma_load_2d(b_dst + c * (64 * BK * 2), &bs.map[ks], full_bar(s), n0 + 64 * c, k0 - bs.start[ks]);
           }
         }
       }
@@ -216,16 +224,28 @@ static int* status_ptr() {
   return g_status[dev];
 }
 
+// B: one matrix, or (B_MN) up to three with rows[i] rows each.
 template <bool A_MN, bool B_MN, typename OutT>
-static int launch_gemm(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb,
-                       int ldc, int ldr, int accumulate, int num_sms, cudaStream_t stream) {
-  CUtensorMap ma, mb;
-  int rc;
+static int launch_gemm(const void* A, const void* const* B, const int* rows, void* C, const void* R, int M, int N, int K, int lda,
+                       int ldb, int ldc, int ldr, int accumulate, int num_sms, cudaStream_t stream) {
+  CUtensorMap ma;
+  BSegs mb;
+  int rc, at = 0, n = 0;
   // K-major: rows = M (or N), cols = K, one (64 x rows) box.  MN-major: rows = K, cols = M (or N), 64x64 boxes.
   rc = A_MN ? make_map_2d_bf16(&ma, A, K, M, lda, 64, BK) : make_map_2d_bf16(&ma, A, M, K, lda, BK, BM);
   if (rc) return 100 + rc;
-  rc = B_MN ? make_map_2d_bf16(&mb, B, K, N, ldb, 64, BK) : make_map_2d_bf16(&mb, B, N, K, ldb, BK, BN);
-  if (rc) return 200 + rc;
+  for (; n < (B_MN ? 3 : 1) && rows[n] > 0; ++n) {
+    if (at % BK) return 6;
+    rc = B_MN ? make_map_2d_bf16(&mb.map[n], B[n], rows[n], N, ldb, 64, BK) : make_map_2d_bf16(&mb.map[n], B[n], N, K, ldb, BK, BN);
+    if (rc) return 200 + rc;
+    mb.start[n] = at;
+    at += rows[n];
+  }
+  if (n == 0 || at != K) return 6;
+  for (; n < 3; ++n) {
+    mb.map[n] = mb.map[0];
+    mb.start[n] = 0x7fffffff;
+  }
   auto kern = kf_gemm_bf16_tcgen05<A_MN, B_MN, OutT>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -298,11 +318,16 @@ int kf_gemm_swiglu_bwd_bf16(const void* dy, const void* w, const void* gu, void*
 
 // Input gradient of a projection whose weight is up to three matrices [n_i][K] stacked along the output (n1 = n2 = 0: one):
 // out[M, K] = dy[M, n0 + n1 + n2] * [w0 ; w1 ; w2].  All but the last n_i a multiple of 64; pitches multiples of 8.
+// The weights of separate Linear modules need no copy that stacks them (10 us of host time each, and 2 x the weight's bytes).
 int kf_gemm_dgrad_stacked_bf16(const void* dy, const void* w0, const void* w1, const void* w2, void* out, int M, int K,
                                int n0, int n1, int n2, int lda, int ldw, int ldc, int num_sms, void* stream) {
   if ((lda & 7) || (ldw & 7) || (ldc & 7) || M <= 0 || K <= 0) return 5;
   const void* w[3] = {w0, w1, w2};
   const int rows[3] = {n0, n1, n2};
+  // the rule of kf_gemm_bf16 for an MN-major B: pairs once their tiles are two rounds
+  if ((long long)((M + 255) / 256) * ((K + 255) / 256) < 2LL * (num_sms / 2))
+    return kf::launch_gemm<false, true, __nv_bfloat16>(dy, w, rows, out, nullptr, M, K, n0 + n1 + n2, lda, ldw, ldc, 0, 0, num_sms,
+                                                       (cudaStream_t)stream);
   return kf2::launch_gemm_stacked_k_2cta(dy, w, rows, out, M, K, n0 + n1 + n2, lda, ldw, ldc, num_sms, (cudaStream_t)stream,
                                          kf::status_ptr());
 }
@@ -387,9 +412,11 @@ int kf_gemm_bf16(const void* A, const void* B, void* C, const void* R, int M, in
   if (mode == 2)
     return kf2::launch_gemm_2cta(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, out_f32, accumulate, num_sms,
                                  st, status_ptr());
-#define KF_DISPATCH(AM, BM_)                                                                                  \
-  (out_f32 ? launch_gemm<AM, BM_, float>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, accumulate, num_sms, st)    \
-           : launch_gemm<AM, BM_, __nv_bfloat16>(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, accumulate, num_sms, st))
+  const void* b[3] = {B, nullptr, nullptr};
+  const int k_rows[3] = {K, 0, 0};
+#define KF_DISPATCH(AM, BM_)                                                                                          \
+  (out_f32 ? launch_gemm<AM, BM_, float>(A, b, k_rows, C, R, M, N, K, lda, ldb, ldc, ldr, accumulate, num_sms, st)    \
+           : launch_gemm<AM, BM_, __nv_bfloat16>(A, b, k_rows, C, R, M, N, K, lda, ldb, ldc, ldr, accumulate, num_sms, st))
   if (!a_mn && !b_mn) return KF_DISPATCH(false, false);
   if (!a_mn && b_mn) return KF_DISPATCH(false, true);
   if (a_mn && !b_mn) return KF_DISPATCH(true, false);

@@ -66,6 +66,8 @@ def _declare(L: ctypes.CDLL) -> None:
         "kf_rmsnorm_fwd_pdl_bf16": [vp, vp, vp, vp, i, i, f, i, vp],
         "kf_attn_decode_bf16": [vp] * 4 + [i] * 5 + [ll] * 5 + [f, i, i, i, vp],
         "kf_block_decode_bf16": [vp, vp, vp],
+        "kf_block_train_fwd_bf16": [vp, vp, vp],
+        "kf_block_train_bwd_bf16": [vp, vp, vp],
         "kf_gemm_swiglu_bwd_bf16": [vp, vp, vp, vp, i, i, i, i, i, i, i, vp],
         "kf_gemm_symm_bf16": [i, vp, vp, vp, i, i, i, i, i, f, f, f, i, vp],
         "kf_rmsnorm_fwd_bf16": [vp, vp, vp, vp, i, i, f, vp],
@@ -360,9 +362,8 @@ def dgrad_rows(dy2: torch.Tensor, weights) -> torch.Tensor:
     """dy2 (M, sum n_i) times the (n_i, K) weights stacked along n: the input gradient of :func:`gemm_rows`."""
     m, n = dy2.shape
     k = weights[0].shape[1]
-    tiles = -(-m // 256) * (-(-k // 256))
-    if (len(weights) in (2, 3) and not rows_adjacent(weights) and tiles >= 2 * (sm_count() // 2) and k % 8 == 0
-            and dy2.stride(0) % 8 == 0 and dy2.data_ptr() % 16 == 0 and all(w.shape[0] % 64 == 0 for w in weights[:-1])
+    if (len(weights) in (2, 3) and not rows_adjacent(weights) and m > 0 and k > 0 and k % 8 == 0 and GEMM_MODE == 0
+            and (n < SPLIT_K_MIN or lib().kf_gemm_k_pieces(m, k, n, sm_count()) == 1) and dy2.stride(0) % 8 == 0 and dy2.data_ptr() % 16 == 0 and all(w.shape[0] % 64 == 0 for w in weights[:-1])
             and all(w.stride() == weights[0].stride() and _plain_rows(w, dy2.device) for w in weights)):
         out = torch.empty((m, k), dtype=torch.bfloat16, device=dy2.device)
         ptrs, rows, pitch = _weights3(weights)

@@ -19,6 +19,10 @@ epilogue), so neither a copy nor a separate rotary pass exists in either directi
 block at the 8B shape) so that the recomputation skips the attention forward; the default keeps
 only the block input, which is what "full" checkpointing means in the reference.
 
+Shapes that the fused epilogues cover throughout are issued by one native call per direction (``csrc/block_train.cu``): the same
+kernels in the same order on one buffer for everything the backward needs.  The rest (few rows, odd widths, sharded parameters,
+gradient slots in different states) is issued op by op.
+
 Semantics are those of kempnerforge/model/transformer.py:82-103 with the activation
 checkpointing of kempnerforge/distributed/parallel.py:90-122.
 """
@@ -27,10 +31,12 @@ from __future__ import annotations
 
 import math
 import os
+from array import array
 
 import torch
 
 from kempnerforge_b200.ops import cuda as kc
+from kempnerforge_b200.ops.fused_infer import _matrix
 
 
 def _wgrad(dy2: torch.Tensor, x2: torch.Tensor, weights) -> list:
@@ -132,6 +138,133 @@ def _rope_fused(n1, w_qkv, cos, sin, s: int, hd: int) -> bool:
             and kc.gemm_rope_supported(n1, w_qkv, hd))
 
 
+# --------------------------------------------------------------------------- one native call per direction
+# variables that select parts of the op-by-op path: any of them set leaves the block to it
+_SWITCHES = ("KF_ROPE_EPILOGUE", "KF_DISABLE_SWIGLU_EPILOGUE", "KF_SWIGLU_BWD_EPILOGUE", "KF_ATTN_FWD", "KF_AC_KEEP_ATTN")
+
+
+def _vector(w, d: int, device) -> bool:
+    return (w.dtype is torch.bfloat16 and w.dim() == 1 and w.size(0) == d and w.is_contiguous() and w.data_ptr() % 16 == 0
+            and w.device == device)
+
+
+def _chain_dims(x2, cos, sin, weights, b: int, s: int, d: int, hd: int):
+    """(B, S, D, H, Hkv, hd, F) when both directions of the block can be issued natively, else None."""
+    wn1, wq, wk, wv, wo, wn2, wg, wu, wd = weights
+    if b * s <= kc.SKINNY_MAX_ROWS or d % 64 or hd not in (64, 128) or wq.dim() != 2 or wk.dim() != 2 or wg.dim() != 2:
+        return None
+    qc, kvc, f = wq.size(0), wk.size(0), wg.size(0)
+    if (kvc == 0 or f == 0 or f % 256 or qc % 128 or kvc % 128 or (qc + 2 * kvc) % 256 or qc % hd or qc % kvc or kc.GEMM_MODE
+            or any(k in os.environ for k in _SWITCHES) or kc.attn_policy() != "native"
+            or not kc.attn_bwd_chosen(hd, b * (qc // hd), s, s, True, False)):
+        return None
+    dev = x2.device
+    for w, rows, cols in ((wq, qc, d), (wk, kvc, d), (wv, kvc, d), (wo, d, qc), (wg, f, d), (wu, f, d), (wd, d, f)):
+        if not _matrix(w, rows, cols) or w.device != dev or _sharded_unit(w) is not None:
+            return None
+    if (not _vector(wn1, d, dev) or not _vector(wn2, d, dev) or x2.data_ptr() % 16 or not kc.rope_tables_ok(cos, sin) or cos.device != dev
+            or sin.device != dev or cos.dim() != 2 or cos.shape != sin.shape or cos.size(0) < s or cos.size(1) != hd // 2):
+        return None
+    return b, s, d, qc // hd, kvc // hd, hd, f
+
+
+class _ChainState:
+    """What a natively issued forward left for its backward: one buffer, and where its parts start."""
+
+    def __init__(self, x2, cos, sin, weights, dims, eps, keep: bool, need_output: bool) -> None:
+        b, s, d, h, hkv, hd, f = dims
+        t, qc, nq = b * s, h * hd, (h + 2 * hkv) * hd
+        # n1, rstd1, qkv, attention, lse, h1, n2, rstd2, gate | up, hidden
+        sizes = (2 * t * d, 4 * t, 2 * t * nq, 2 * t * qc, 4 * t * h, 2 * t * d, 2 * t * d, 4 * t, 4 * t * f if keep else 0, 2 * t * f)
+        at = [0]
+        for n in sizes:
+            at.append(at[-1] + (n + 255) // 256 * 256)
+        self.dims, self.at, self.scalars = dims, at, array("d", (eps, 1.0 / math.sqrt(hd)))
+        self.buf = torch.empty(at[-1], dtype=torch.uint8, device=x2.device)
+        base = self.buf.data_ptr()
+        parts = [base + o for o in at[:-1]]
+        if not keep:
+            parts[8] = 0
+        self.y = torch.empty((t, d), dtype=torch.bfloat16, device=x2.device) if need_output else None
+        self.ptrs = [t_.data_ptr() for t_ in (x2, *weights, cos, sin)] + parts + [*dims, kc.sm_count()]
+        ints = array("q", (*self.ptrs, self.y.data_ptr() if need_output else 0))
+        kc._check(kc.lib().kf_block_train_fwd_bf16(ints.buffer_info()[0], self.scalars.buffer_info()[0], kc._stream()),
+                  "kf_block_train_fwd_bf16", 7 if need_output else 6)
+
+    def views(self) -> dict:
+        """The parts as the tensors that the op-by-op backward reads."""
+        b, s, d, h, hkv, hd, f = self.dims
+        t = b * s
+
+        def part(i, shape, dtype=torch.bfloat16):
+            n = math.prod(shape) * dtype.itemsize
+            return self.buf[self.at[i] : self.at[i] + n].view(dtype).view(shape)
+
+        return dict(n1=part(0, (t, d)), rstd1=part(1, (t,), torch.float32), qkv4=part(2, (b, s, h + 2 * hkv, hd)), attn2=part(3, (t, h * hd)),
+                    actx=("native", part(4, (b, h, s), torch.float32)), h1=part(5, (t, d)), n2=part(6, (t, d)),
+                    rstd2=part(7, (t,), torch.float32), gu=part(8, (t, 2 * f)), hmid=part(9, (t, f)))
+
+
+def _grad_target(weights):
+    """Where the gradient of row-stacked weights goes: (stacked flat slot or None for a tensor of its own, accumulate); None when
+    the slots are of several kinds."""
+    slots = [getattr(w, "_kf_grad", None) for w in weights]
+    if all(s is None for s in slots):
+        return None, 0
+    live = [getattr(w, "_kf_grad_live", False) for w in weights]
+    if (any(s is None or s.dtype is not torch.bfloat16 or s.shape != w.shape or s.data_ptr() % 16 or s.device != w.device
+            for s, w in zip(slots, weights)) or any(live) != all(live) or not kc.rows_adjacent(slots)):
+        return None
+    return slots[0], int(live[0])
+
+
+def _chain_backward(it: _ChainState, dy2, x2, weights):
+    """(dx, gradients of the nine weights) of a natively issued forward, or None when the gradient slots do not fit."""
+    wn1, wq, wk, wv, wo, wn2, wg, wu, wd = weights
+    groups = ((wq, wk, wv), (wo,), (wg, wu), (wd,))
+    targets = [_grad_target(g) for g in groups]
+    if any(t is None for t in targets) or dy2.dtype is not torch.bfloat16:
+        return None
+    if dy2.data_ptr() % 16:
+        dy2 = dy2.clone()
+    b, s, d, h, hkv, hd, f = it.dims
+    t, qc, nq, dev = b * s, h * hd, (h + 2 * hkv) * hd, x2.device
+    own = [torch.empty((rows, cols), dtype=torch.bfloat16, device=dev) if tg[0] is None else None
+           for tg, (rows, cols) in zip(targets, ((nq, d), (d, qc), (2 * f, d), (d, f)))]
+    dx = torch.empty((t, d), dtype=torch.bfloat16, device=dev)
+    dwn = torch.empty((2, d), dtype=torch.bfloat16, device=dev)
+    L = kc.lib()
+    # dh1, dattn, dqkv, dq_acc, dsum, partial
+    at = [0]
+    for n in (2 * t * d, 2 * t * qc, 2 * t * nq, 4 * t * qc, 4 * t * h, 4 * L.kf_rmsnorm_bwd_blocks(t) * d):
+        at.append(at[-1] + (n + 255) // 256 * 256)
+    scratch = torch.empty(at[-1], dtype=torch.uint8, device=dev)
+    base = scratch.data_ptr()
+    pieces = L.kf_gemm_k_pieces(t, d, 2 * f, kc.sm_count()) if 2 * f >= kc.SPLIT_K_MIN else 1
+    stack_gu, ws = kc.rows_adjacent((wg, wu)), None
+    ptrs = list(it.ptrs)
+    if pieces > 1:
+        ws = torch.empty((pieces, t, d), dtype=torch.float32, device=dev)
+        if not stack_gu:
+            w_gu = kc.stack_rows([wg, wu])
+            ptrs[7] = w_gu.data_ptr()
+    outs = [(tg[0] if o is None else o).data_ptr() for tg, o in zip(targets, own)]
+    ints = array("q", (*ptrs, dy2.data_ptr(), dx.data_ptr(), *outs, dwn.data_ptr(), dwn.data_ptr() + 2 * d, *(base + o for o in at[:-1]),
+                       *(tg[1] for tg in targets), int(kc.rows_adjacent((wq, wk, wv))), int(stack_gu),
+                       ws.data_ptr() if ws is not None else 0, pieces))
+    kc._check(L.kf_block_train_bwd_bf16(ints.buffer_info()[0], it.scalars.buffer_info()[0], kc._stream()), "kf_block_train_bwd_bf16",
+              11 + (pieces > 1))
+    g_w = []
+    for group, o in zip(groups, own):
+        row = 0
+        for w in group:
+            if o is None:
+                w._kf_grad_live = True
+            g_w.append(None if o is None else o[row : row + w.size(0)] if len(group) > 1 else o)
+            row += w.size(0)
+    return dx, (_norm_wgrad(wn1, dwn[0]), *g_w[:4], _norm_wgrad(wn2, dwn[1]), *g_w[4:])
+
+
 class DenseBlockFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, cos, sin, wn1, wq, wk, wv, wo, wn2, wg, wu, wd, eps, head_dim, recompute):
@@ -141,11 +274,18 @@ class DenseBlockFn(torch.autograd.Function):
             x2 = x2.contiguous()
         ctx.meta = (b, s, d, eps, head_dim, recompute)
         ctx.weights = (wn1, wq, wk, wv, wo, wn2, wg, wu, wd)
+        ctx.attn_saved = None
+        dims = _chain_dims(x2, cos, sin, ctx.weights, b, s, d, head_dim)
+        if dims is not None:
+            it = _ChainState(x2, cos, sin, ctx.weights, dims, eps, keep=not recompute, need_output=True)
+            ctx.save_for_backward(x2, cos, sin)
+            y, it.y = it.y, None
+            ctx.inter = None if recompute else it
+            return y.view(b, s, d)
         keep_attn = recompute and os.environ.get("KF_AC_KEEP_ATTN", "0") == "1"
         inter = DenseBlockFn._run_forward(x2, cos, sin, ctx.weights, ctx.meta, need_output=True, keep=not recompute,
                                           keep_attn=keep_attn)
         y = inter.pop("y")
-        ctx.attn_saved = None
         if recompute:
             ctx.save_for_backward(x2, cos, sin)
             ctx.inter = None
@@ -230,6 +370,17 @@ class DenseBlockFn(torch.autograd.Function):
         if unit is not None:
             unit.engine.prepare_backward(unit)  # parameter staging is ours again; gradient staging slot is free
         it = ctx.inter
+        if it is None and unit is None and ctx.attn_saved is None:
+            dims = _chain_dims(x2, cos, sin, ctx.weights, b, s, d, hd)
+            if dims is not None:
+                it = _ChainState(x2, cos, sin, ctx.weights, dims, eps, keep=True, need_output=False)
+        if isinstance(it, _ChainState):
+            dy2 = dy.reshape(b * s, d)
+            done = _chain_backward(it, dy2 if dy2.is_contiguous() else dy2.contiguous(), x2, ctx.weights)
+            if done is not None:
+                ctx.inter = None
+                return (done[0].view(b, s, d), None, None, *done[1], None, None, None)
+            it = it.views()
         if it is None:
             it = DenseBlockFn._run_forward(x2, cos, sin, ctx.weights, ctx.meta, need_output=False, keep=True,
                                            attn_saved=ctx.attn_saved)
