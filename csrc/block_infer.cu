@@ -91,4 +91,14 @@ int kf_block_decode_bf16(const long long* a, const double* r, void* stream) {
   return rc ? 7000 + rc : 0;
 }
 
+// n blocks in a row: a holds 31 values per block, r three.  The blocks may share their intermediates (scratch, rstd, h1, attention):
+// a kernel of the chain writes only after all kernels before it are complete.
+int kf_blocks_decode_bf16(const long long* a, const double* r, int n, void* stream) {
+  for (int i = 0; i < n; ++i) {
+    const int rc = kf_block_decode_bf16(a + 31 * i, r + 3 * i, stream);
+    if (rc) return rc;
+  }
+  return 0;
+}
+
 }  // extern "C"

@@ -312,7 +312,15 @@ class Transformer(nn.Module):
         else:
             ca_blocks = list(self.cross_attention_layers.values()) if self._ca_cadence else []
             image_features = ctx.image_features
-            for pos, (key, layer) in enumerate(self.layers.items()):
+            done = None
+            if (kv_caches is not None and seq_len == 1 and not ca_blocks and h.is_cuda and doc_ids is None and kpm is None and tp is None
+                    and not _FUSED_BLOCK_OFF and not torch.is_grad_enabled() and F.use_native(h)
+                    and all(type(layer) is TransformerBlock for layer in self.layers.values())):
+                from kempnerforge_b200.ops import fused_infer
+
+                done = fused_infer.run_layers(list(self.layers.values()), h, cos, sin, kv_caches)
+            h = h if done is None else done
+            for pos, (key, layer) in enumerate(self.layers.items() if done is None else ()):
                 i = int(key)
                 cache = kv_caches[pos] if kv_caches is not None else None
                 h = layer(h, cos, sin, kv_cache=cache, doc_ids=doc_ids, key_padding_mask=kpm)

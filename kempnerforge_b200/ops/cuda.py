@@ -66,6 +66,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "kf_rmsnorm_fwd_pdl_bf16": [vp, vp, vp, vp, i, i, f, i, vp],
         "kf_attn_decode_bf16": [vp] * 4 + [i] * 5 + [ll] * 5 + [f, i, i, i, vp],
         "kf_block_decode_bf16": [vp, vp, vp],
+        "kf_blocks_decode_bf16": [vp, vp, i, vp],
         "kf_block_train_fwd_bf16": [vp, vp, vp],
         "kf_block_train_bwd_bf16": [vp, vp, vp],
         "kf_gemm_swiglu_bwd_bf16": [vp, vp, vp, vp, i, i, i, i, i, i, i, vp],
@@ -461,6 +462,36 @@ def block_decode(y: torch.Tensor, attn_ptrs, mlp_ptrs, cache_ptrs, table_ptrs, d
         _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 3 + norms if mlp_ptrs else 1)
         return
     _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 5 + 2 * norms if mlp_ptrs else 3 + norms)
+
+
+def blocks_decode(x: torch.Tensor, xp: int, plans, table_ptrs) -> torch.Tensor:
+    """One new token per sequence through a row of blocks (``plans``: what ``fused_infer._plan`` made of them, all with an MLP and
+    an attention that ``kf_block_decode_bf16`` runs itself) as one native call.  The blocks share one buffer of intermediates and
+    hand x on through two more: each kernel of the chain writes only after all before it are complete."""
+    b, _, d = x.shape
+    n = len(plans)
+    # n (D) | q (H hd) | hidden (F) | h1 (D) | attention (H hd) | the outputs of even and of odd blocks | rstd, lse
+    cols = max(2 * d + 2 * p.h * p.hd + p.f for p in plans)
+    lse = 2 * max(p.h for p in plans)
+    scratch = torch.empty(b * cols + 2 * b + lse + 2 * b * d, dtype=torch.bfloat16, device=x.device)
+    y = torch.empty_like(x)
+    base = scratch.data_ptr()
+    hand = [base + 2 * b * cols, base + 2 * b * (cols + d)]
+    rstd = base + 2 * b * (cols + 2 * d)
+    sms = sm_count()
+    ints, reals = array("q"), array("d")
+    launches, src = 0, xp
+    norms = 0 if b <= lib().kf_skinny_norm_rows() else 1
+    for i, p in enumerate(plans):
+        h1 = base + 2 * b * (d + p.h * p.hd + p.f)
+        dst = y.data_ptr() if i == n - 1 else hand[i & 1]
+        ints.extend((src, *p.attn_ptrs, *p.mlp_ptrs, *p.cache_ptrs, base, rstd, h1, dst, *table_ptrs, b, d, p.h, p.hkv, p.hd, p.f, p.past,
+                     p.batch_step, sms, 7, int(p.hd == 64), h1 + 2 * b * d, rstd + 4 * b))
+        reals.extend((p.eps1, p.eps2, 1.0 / math.sqrt(p.hd)))
+        launches += 5 + 2 * norms
+        src = dst
+    _check(lib().kf_blocks_decode_bf16(ints.buffer_info()[0], reals.buffer_info()[0], n, _stream()), "kf_blocks_decode_bf16", launches)
+    return y
 
 
 # --------------------------------------------------------------------------- norm / rope / swiglu / embedding

@@ -6,6 +6,8 @@ o projection with the residual, RMSNorm, gate|up with SwiGLU, down with the resi
 or a plain forward pass, uses the epilogue-fused GEMMs of the training block and reads q | k | v from the projection's own
 buffer.  The weights of separate ``nn.Linear`` modules are read where they are: nothing is concatenated.
 
+All blocks of a model on one new token are one native call (:func:`run_layers`).
+
 What the fused form does not cover (masks, hooks, q/k norms, tensor parallelism, fp8, captured attention weights, a prompt
 behind a non-empty cache, foreign module types) returns None and takes the op-by-op path.
 
@@ -60,49 +62,109 @@ def _gain(norm, d: int) -> int:
     return 0 if p & 15 else p
 
 
-def run(block, x, cos, sin, cache):
-    """The block's output (new (B, S, D) tensor), or None when this path does not cover the call."""
+class _Plan:
+    """Addresses and sizes of one block's weights and cache, checked."""
+
+    __slots__ = ("mlp", "norm1", "norm2", "attn_ptrs", "mlp_ptrs", "cache_ptrs", "weights", "h", "hkv", "hd", "f", "past", "batch_step",
+                 "eps1", "eps2")
+
+
+def _plan(block, b: int, s: int, d: int, cos, sin, cache):
+    """The plan of a call of ``block`` on (b, s, d) inputs, or None when this path does not cover it."""
     sub = block._modules
     att, mlp, norm1 = sub["attention"], sub["mlp"], sub["attention_norm"]
-    if (type(att) is not Attention or x.dim() != 3 or att.tp is not None or att._modules.get("q_norm") is not None
-            or att.q_norm is not None or att.k_norm is not None or att.capture_attention_weights
-            or getattr(block, "fp8", False) or getattr(block, "_kf_fp8_block", False) or not _plain(att)
-            or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks
-            or torch.autograd.forward_ad._current_level >= 0 or kc.attn_policy() != "native"):
+    if (type(att) is not Attention or att.tp is not None or att._modules.get("q_norm") is not None or att.q_norm is not None
+            or att.k_norm is not None or att.capture_attention_weights or getattr(block, "fp8", False)
+            or getattr(block, "_kf_fp8_block", False) or not _plain(att)):
         return None
-    hd = att.head_dim
-    b, s, d = x.shape
+    p = _Plan()
+    hd = p.hd = att.head_dim
     wq, wk, wv, wo = _weight(att, "q_proj"), _weight(att, "k_proj"), _weight(att, "v_proj"), _weight(att, "o_proj")
     if hd not in (64, 128) or b * s == 0 or d % 8 or wq is None or wk is None:
         return None
     qc, kvc = wq.size(0), wk.size(0)
     if kvc == 0 or qc % hd or kvc % hd or qc % kvc or getattr(getattr(wq, "_kf_flat", None), "sharded", False):
         return None
-    pq, pk, pv, po = _matrix(wq, qc, d), _matrix(wk, kvc, d), _matrix(wv, kvc, d), _matrix(wo, d, qc)
-    g1 = _gain(norm1, d)
-    if (not (pq and pk and pv and po and g1) or cos.dtype is not torch.float32 or sin.dtype is not torch.float32
-            or cos.dim() != 2 or cos.shape != sin.shape or cos.size(0) < s or cos.size(1) != hd // 2
+    p.attn_ptrs = _gain(norm1, d), _matrix(wq, qc, d), _matrix(wk, kvc, d), _matrix(wv, kvc, d), _matrix(wo, d, qc)
+    if (not all(p.attn_ptrs) or cos.dtype is not torch.float32 or sin.dtype is not torch.float32 or cos.dim() != 2
+            or cos.shape != sin.shape or cos.size(0) < s or cos.size(1) != hd // 2
             or not (cos.is_cuda and cos.is_contiguous() and sin.is_contiguous())):
         return None
-    h, hkv = qc // hd, kvc // hd
-    past = 0
+    p.h, p.hkv, p.past = qc // hd, kvc // hd, 0
     if cache is not None:
         k, v = cache.k, cache.v
-        past = cache.seq_len
+        p.past = cache.seq_len
         if (type(cache) is not KVCache or k.dtype is not _BF16 or v.dtype is not _BF16 or k.dim() != 4 or k.shape != v.shape
-                or k.size(0) != b or k.size(2) != hkv or k.size(3) != hd or not (k.is_contiguous() and v.is_contiguous())
-                or not (k.is_cuda and v.is_cuda) or past + s > k.size(1)):
+                or k.size(0) != b or k.size(2) != p.hkv or k.size(3) != hd or not (k.is_contiguous() and v.is_contiguous())
+                or not (k.is_cuda and v.is_cuda) or p.past + s > k.size(1)):
             return None
-        kp, vp = k.data_ptr(), v.data_ptr()
-        if (kp | vp) & 15:
+        p.cache_ptrs, p.batch_step = (k.data_ptr(), v.data_ptr()), k.stride(0)
+        if (p.cache_ptrs[0] | p.cache_ptrs[1]) & 15:
             return None
-    g2, norm2 = 0, None
+    p.mlp_ptrs, p.norm2, p.f, p.eps1, p.eps2 = None, None, 0, norm1.eps, 0.0
+    wg = wu = wd = None
     if type(mlp) is SwiGLUMLP and mlp.tp is None and _plain(mlp):
         norm2 = sub["mlp_norm"]
         wg, wu, wd = _weight(mlp, "gate_proj"), _weight(mlp, "up_proj"), _weight(mlp, "down_proj")
         f = wg.size(0) if wg is not None else 0
-        pg, pu, pd = _matrix(wg, f, d), _matrix(wu, f, d), _matrix(wd, d, f)
-        g2 = _gain(norm2, d) if f and f % 8 == 0 and pg and pu and pd else 0
+        ptrs = _matrix(wg, f, d), _matrix(wu, f, d), _matrix(wd, d, f)
+        g2 = _gain(norm2, d) if f and f % 8 == 0 and all(ptrs) else 0
+        if g2:
+            p.mlp_ptrs, p.norm2, p.f, p.eps2 = (g2, *ptrs), norm2, f, norm2.eps
+    p.mlp, p.norm1, p.weights = mlp, norm1, (wq, wk, wv, wo, wg, wu, wd)
+    return p
+
+
+def _refused() -> bool:
+    return bool(_nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks
+                or torch.autograd.forward_ad._current_level >= 0 or kc.attn_policy() != "native")
+
+
+def _one_token(b: int, cos, sin) -> bool:
+    """The native generation step takes this many sequences and these tables."""
+    return b <= kc.SKINNY_MAX_ROWS and not (cos.data_ptr() | sin.data_ptr()) & 15
+
+
+def run_layers(layers, x, cos, sin, caches):
+    """One new token per sequence through all of a model's blocks as one native call: the last block's output (B, 1, D), or None
+    when some block is not covered (nothing has been done then).  Issued block by block, Python takes 50 us per block, more
+    than the 18 us that the five kernels of a small one run."""
+    if x.dim() != 3 or x.size(1) != 1 or not layers or len(caches) < len(layers) or _refused():
+        return None
+    b, _, d = x.shape
+    plans = []
+    for block, cache in zip(layers, caches):
+        if not _plain(block) or cache is None:
+            return None
+        p = _plan(block, b, 1, d, cos, sin, cache)
+        # heads of 64 for several sequences go through the library's attention, one block at a time
+        if p is None or p.mlp_ptrs is None or (p.hd == 64 and b > 1) or not _one_token(b, cos, sin):
+            return None
+        plans.append(p)
+    if len({id(c) for c in caches[: len(plans)]}) != len(plans):
+        return None
+    if not x.is_contiguous():
+        x = x.contiguous()
+    xp = x.data_ptr()
+    if xp & 15:
+        return None
+    y = kc.blocks_decode(x, xp, plans, (cos.data_ptr(), sin.data_ptr()))
+    for p, cache in zip(plans, caches):
+        cache.seq_len = p.past + 1
+    return y
+
+
+def run(block, x, cos, sin, cache):
+    """The block's output (new (B, S, D) tensor), or None when this path does not cover the call."""
+    if x.dim() != 3 or _refused():
+        return None
+    b, s, d = x.shape
+    p = _plan(block, b, s, d, cos, sin, cache)
+    if p is None:
+        return None
+    hd, h, hkv, past, g2, norm1, norm2 = p.hd, p.h, p.hkv, p.past, p.mlp_ptrs, p.norm1, p.norm2
+    wq, wk, wv, wo, wg, wu, wd = p.weights
+    mlp, qc = p.mlp, h * hd
     if not x.is_contiguous():
         x = x.contiguous()
     xp = x.data_ptr()
@@ -111,17 +173,16 @@ def run(block, x, cos, sin, cache):
     scale = 1.0 / math.sqrt(hd)
     t = b * s
     if s == 1 and cache is not None:
-        cp, sp = cos.data_ptr(), sin.data_ptr()
-        if t > kc.SKINNY_MAX_ROWS or (cp | sp) & 15:
+        if not _one_token(b, cos, sin):
             return None
         y = torch.empty((b, 1, d), dtype=_BF16, device=x.device)
 
         def foreign(q2):
-            out = F.attention(q2.unflatten(1, (h, hd)).unsqueeze(1), k[:, : past + 1], v[:, : past + 1], causal=False)
+            out = F.attention(q2.unflatten(1, (h, hd)).unsqueeze(1), cache.k[:, : past + 1], cache.v[:, : past + 1], causal=False)
             return out.reshape(b, qc)   # SDPA's output is a transposed view
 
-        kc.block_decode(y, (xp, g1, pq, pk, pv, po), (g2, pg, pu, pd) if g2 else None, (kp, vp), (cp, sp),
-                        (b, d, h, hkv, hd, f if g2 else 0, past, k.stride(0)), (norm1.eps, norm2.eps if g2 else 0.0, scale), foreign)
+        kc.block_decode(y, (xp, *p.attn_ptrs), p.mlp_ptrs, p.cache_ptrs, (cos.data_ptr(), sin.data_ptr()),
+                        (b, d, h, hkv, hd, p.f, past, p.batch_step), (p.eps1, p.eps2, scale), foreign)
         cache.seq_len = past + 1
         return y if g2 else y + mlp(block.mlp_norm(y))
     if past:

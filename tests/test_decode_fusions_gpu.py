@@ -72,3 +72,70 @@ def test_small_weights_keep_the_bits_of_the_tile_kernel(native_lib, m, rows, k):
     w = torch.cat(ws)
     assert torch.equal(out, kc.gemm(x, w, mode=1)) and torch.equal(with_res, kc.gemm(x, w, residual=res, mode=1))
     assert bool((frame[m:] == 7).all()) and bool((frame[:, sum(rows):] == 7).all())
+
+
+def _model(heads, kv, batch, ctx, layers=3, **over):
+    from kempnerforge_b200.config import ModelConfig
+    from kempnerforge_b200.models.attention import KVCache
+    from kempnerforge_b200.models.transformer import Transformer
+
+    torch.manual_seed(0)
+    cfg = ModelConfig(dim=512, n_layers=layers, n_heads=heads, n_kv_heads=kv, vocab_size=256, ffn_hidden_dim=768, max_seq_len=512, **over)
+    model = Transformer(cfg).to(DEV, torch.bfloat16).eval()
+    model._rope_cos = model._rope_sin = None
+    caches = [KVCache(batch, ctx + 8, kv, 512 // heads, torch.bfloat16, torch.device(DEV)) for _ in range(layers)]
+    for i, c in enumerate(caches):
+        c.k.copy_(_rand(*c.k.shape, seed=20 + i))
+        c.v.copy_(_rand(*c.v.shape, seed=40 + i))
+        c.seq_len = ctx
+    return model, caches
+
+
+def _steps(model, caches, batch, n=3):
+    start = [(c.k.clone(), c.v.clone(), c.seq_len) for c in caches]
+    tokens = torch.arange(batch, device=DEV)[:, None] % 256
+    with torch.no_grad():
+        out = [model(tokens + i, kv_caches=caches) for i in range(n)]
+    out += [t.clone() for c in caches for t in (c.k, c.v)] + [c.seq_len for c in caches]
+    for c, (k, v, length) in zip(caches, start):
+        c.k.copy_(k)
+        c.v.copy_(v)
+        c.seq_len = length
+    return out
+
+
+@pytest.mark.parametrize("heads,kv,batch,ctx", [(8, 8, 1, 1), (8, 2, 1, 130), (4, 4, 1, 200), (4, 2, 3, 77), (4, 2, 6, 64)])
+def test_all_blocks_in_one_call(native_lib, monkeypatch, heads, kv, batch, ctx):
+    from kempnerforge_b200.ops import fused_infer
+
+    model, caches = _model(heads, kv, batch, ctx)
+    used, native = [], fused_infer.run_layers
+    monkeypatch.setattr(fused_infer, "run_layers", lambda *a: used.append(native(*a)) or used[-1])
+    got = _steps(model, caches, batch)
+    assert len(used) == 3 and all(u is not None for u in used) and native_lib.read_status() == 0
+    monkeypatch.setattr(fused_infer, "run_layers", lambda *a: None)
+    want = _steps(model, caches, batch)
+    assert all(torch.equal(a, b) if torch.is_tensor(a) else a == b for a, b in zip(got, want))
+
+
+def test_models_that_go_block_by_block(native_lib):
+    from kempnerforge_b200.ops import fused_infer
+
+    def run(model, caches, batch=1):
+        x = _rand(batch, 1, 512)
+        cos, sin = model.rope_tables(x.device, min(c.seq_len for c in caches), 1)
+        with torch.no_grad():
+            return fused_infer.run_layers(list(model.layers.values()), x, cos, sin, caches)
+
+    model, caches = _model(8, 8, 1, 40)
+    assert run(model, caches) is not None and [c.seq_len for c in caches] == [41] * 3
+    caches[2].seq_len = caches[2].k.size(1)                                     # full: the error comes from the cache itself
+    assert run(model, caches) is None and [c.seq_len for c in caches[:2]] == [41] * 2
+    assert run(model, [caches[0]] * 3) is None and run(model, caches[:2]) is None
+    handle = model.layers["1"].register_forward_hook(lambda m, a, o: o)
+    caches[2].seq_len = 41
+    assert run(model, caches) is None
+    handle.remove()
+    assert run(model, caches) is not None
+    assert run(*_model(8, 8, 2, 40), batch=2) is None                           # heads of 64, several sequences: the library's attention
+    assert run(*_model(4, 4, 1, 40, qk_norm=True)) is None
