@@ -7,10 +7,14 @@
 // hand over, and the tensor cores alternate  O_A += P_A V_j, S_A = Q_A K_{j+1}^T, O_B += P_B V_j, S_B = Q_B K_{j+1}^T.
 // K and V tiles are fetched once for both query tiles.
 //
-//   warp 0    : TMA producers (lane 0: Q_A, Q_B and the K ring; lane 1: the V ring)
-//   warp 1    : MMA issuer
-//   warps 2-5 : softmax + epilogue of tile A (one thread per query row)
-//   warps 6-9 : softmax + epilogue of tile B
+//   warp 0     : TMA producers (lane 0: Q_A, Q_B and the K ring; lane 1: the V ring)
+//   warp 1     : MMA issuer (warps 2 and 3 only make the first warpgroup whole)
+//   warps 4-7  : softmax + epilogue of tile A (one thread per query row)
+//   warps 8-11 : softmax + epilogue of tile B
+// A softmax thread holds a row of 128 scores; at the 168 registers that an even split leaves it spilled 50 - 110 bytes per
+// tile, so the first warpgroup gives its registers to the other two.  2 x 4096 tokens, 32 query and
+// 8 key heads of 128: 290 -> 274 us; 3000 tokens, 40 heads: 124 -> 114 us; 4 x 2048 tokens, 12 heads of 64: 68.5 -> 62.5 us.
+//
 //   TMEM      : S_A | S_B | O_A | O_B   (128 fp32 columns each; bf16 P aliases the start of its S)
 //
 // Masks, lazy rescaling and outputs are those of the single-tile kernel in attention_tcgen05.cu, which remains the
@@ -25,7 +29,8 @@ namespace attn2 {
 using namespace kf::attn;
 
 constexpr int BLK_M = 128, BLK_N = 128;
-constexpr int THREADS = 320;
+constexpr int THREADS = 384;  // three warpgroups: TMA + MMA, softmax of tile A, softmax of tile B
+constexpr int REGS_ISSUE = 72, REGS_SOFTMAX = 216;  // per thread; 72 + 2 * 216 = 3 * 168, what the launch gets
 constexpr int TMEM_COLS = 512;
 constexpr int KV_STAGES = 2;
 constexpr float RESCALE_THRESHOLD = 8.0f;
@@ -38,6 +43,11 @@ struct Cfg {
   static constexpr int N_TILES_SMEM = 2 + 2 * KV_STAGES;  // Q_A, Q_B, K ring, V ring
   static constexpr size_t SMEM = N_TILES_SMEM * size_t(TILE_BYTES) + 1024 + 256 + 2048 + docblk::MASK_BYTES;
 };
+
+template <int N>
+__device__ __forceinline__ void regs_give() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void regs_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 
 __device__ __forceinline__ void tile_group_sync(int tile) {
   asm volatile("bar.sync %0, 128;" ::"r"(tile + 1) : "memory");
@@ -138,126 +148,130 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
   auto s_col = [&](int tile) { return tmem_base + uint32_t(tile * BLK_N); };
   auto o_col = [&](int tile) { return tmem_base + uint32_t(256 + tile * 128); };
 
-  if (warp == 0) {
-    // ------------------------------------------------------------ TMA producers
-    if (lane == 0) {
-      bool ok = true;
-      int issued = 0;
-      mbar_expect_tx(q_full, 2 * C::TILE_BYTES);
+  if (warp < 4) {
+    regs_give<REGS_ISSUE>();
+    if (warp == 0) {
+      // ------------------------------------------------------------ TMA producers
+      if (lane == 0) {
+        bool ok = true;
+        int issued = 0;
+        mbar_expect_tx(q_full, 2 * C::TILE_BYTES);
 #pragma unroll
-      for (int tile = 0; tile < 2; ++tile)
+        for (int tile = 0; tile < 2; ++tile)
 #pragma unroll
-        for (int c = 0; c < C::BLOCKS; ++c)
-          tma_load_2d(q_smem + tile * C::TILE_BYTES + c * C::BLOCK_BYTES, &map_q, q_full, h * HD + 64 * c,
-                      b * Sq + m0 + tile * BLK_M);
-      int i = 0;
-      for (int j = first_tile(); j < n_max; j = next_tile(j), ++i) {
-        const int st = i & 1, use = i >> 1;
-        if (use > 0 && !mbar_wait(k_empty(st), (use - 1) & 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
-        mbar_expect_tx(k_full(st), C::TILE_BYTES);
+          for (int c = 0; c < C::BLOCKS; ++c)
+            tma_load_2d(q_smem + tile * C::TILE_BYTES + c * C::BLOCK_BYTES, &map_q, q_full, h * HD + 64 * c,
+                        b * Sq + m0 + tile * BLK_M);
+        int i = 0;
+        for (int j = first_tile(); j < n_max; j = next_tile(j), ++i) {
+          const int st = i & 1, use = i >> 1;
+          if (use > 0 && !mbar_wait(k_empty(st), (use - 1) & 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
+          mbar_expect_tx(k_full(st), C::TILE_BYTES);
 #pragma unroll
-        for (int c = 0; c < C::BLOCKS; ++c)
-          tma_load_2d(k_smem + st * C::TILE_BYTES + c * C::BLOCK_BYTES, &map_k, k_full(st), hk * HD + 64 * c,
-                      b * Sk + j * BLK_N);
-        ++issued;
-      }
-      if (!ok) {
-        mbar_wait(q_full, 0, status, KF_ERR_WAIT_DRAIN);
-        for (int j = max(0, issued - 2); j < issued; ++j) mbar_wait(k_full(j & 1), (j >> 1) & 1, status, KF_ERR_WAIT_DRAIN);
-      }
-    } else if (lane == 1) {
-      bool ok = true;
-      int issued = 0;
-      int i = 0;
-      for (int j = first_tile(); j < n_max; j = next_tile(j), ++i) {
-        const int st = i & 1, use = i >> 1;
-        if (use > 0 && !mbar_wait(v_empty(st), (use - 1) & 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
-        mbar_expect_tx(v_full(st), C::TILE_BYTES);
-#pragma unroll
-        for (int c = 0; c < C::BLOCKS; ++c)
-          tma_load_2d(v_smem + st * C::TILE_BYTES + c * C::BLOCK_BYTES, &map_v, v_full(st), hk * HD + 64 * c,
-                      b * Sk + j * BLK_N);
-        ++issued;
-      }
-      if (!ok)
-        for (int j = max(0, issued - 2); j < issued; ++j) mbar_wait(v_full(j & 1), (j >> 1) & 1, status, KF_ERR_WAIT_DRAIN);
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = umma_idesc_bf16(BLK_M, BLK_N, false, false);
-      constexpr uint32_t idesc_o = umma_idesc_bf16(BLK_M, HD, false, true);
-      bool ok = mbar_wait(q_full, 0, status, KF_ERR_WAIT_FULL);
-      const int lim[2] = {n_a, n_b};                    // key tiles below lim[tile] belong to the query tile
-      // S_tile = Q_tile K^T with the i-th walked key tile; the caller has made sure it landed
-      auto issue_s = [&](int tile, int i) {
-        const int st = i & 1;
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t off = (kk / 4) * C::BLOCK_BYTES + (kk % 4) * 32;
-          tc_mma_f16(s_col(tile), umma_desc_sw128(q_smem + tile * C::TILE_BYTES + off, 16, 1024),
-                     umma_desc_sw128(k_smem + st * C::TILE_BYTES + off, 16, 1024), idesc_s, kk != 0);
+          for (int c = 0; c < C::BLOCKS; ++c)
+            tma_load_2d(k_smem + st * C::TILE_BYTES + c * C::BLOCK_BYTES, &map_k, k_full(st), hk * HD + 64 * c,
+                        b * Sk + j * BLK_N);
+          ++issued;
         }
-        tc_commit(s_full(tile));
-      };
-      int j = first_tile();
-      if (ok && j < n_max) {
-        ok = mbar_wait(k_full(0), 0, status, KF_ERR_WAIT_FULL);
-        if (ok) {
-          tc_fence_after();
-          if (j < n_a) issue_s(0, 0);
-          if (j < n_b) issue_s(1, 0);
-          tc_commit(k_empty(0));
+        if (!ok) {
+          mbar_wait(q_full, 0, status, KF_ERR_WAIT_DRAIN);
+          for (int j = max(0, issued - 2); j < issued; ++j) mbar_wait(k_full(j & 1), (j >> 1) & 1, status, KF_ERR_WAIT_DRAIN);
         }
+      } else if (lane == 1) {
+        bool ok = true;
+        int issued = 0;
+        int i = 0;
+        for (int j = first_tile(); j < n_max; j = next_tile(j), ++i) {
+          const int st = i & 1, use = i >> 1;
+          if (use > 0 && !mbar_wait(v_empty(st), (use - 1) & 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
+          mbar_expect_tx(v_full(st), C::TILE_BYTES);
+#pragma unroll
+          for (int c = 0; c < C::BLOCKS; ++c)
+            tma_load_2d(v_smem + st * C::TILE_BYTES + c * C::BLOCK_BYTES, &map_v, v_full(st), hk * HD + 64 * c,
+                        b * Sk + j * BLK_N);
+          ++issued;
+        }
+        if (!ok)
+          for (int j = max(0, issued - 2); j < issued; ++j) mbar_wait(v_full(j & 1), (j >> 1) & 1, status, KF_ERR_WAIT_DRAIN);
       }
-      for (int i = 0; j < n_max && ok; ++i) {
-        const int st = i & 1, jn = next_tile(j);
-        bool k_next_ready = false;
-        for (int tile = 0; tile < 2 && ok; ++tile) {
-          if (j >= lim[tile]) continue;
-          // O_tile += P_tile V_j : A = P from tensor memory, B = V with the head dim contiguous (MN-major).  The
-          // softmax warps hand P over in two halves: the products over the first 64 keys run while the
-          // exponentials of the last 64 are still being computed.
-          if (!mbar_wait(p_half(tile), i & 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
-          if (!mbar_wait(v_full(st), (i >> 1) & 1, status, KF_ERR_WAIT_FULL)) { ok = false; break; }
-          tc_fence_after();
+    } else if (warp == 1) {
+      // ------------------------------------------------------------ MMA issuer
+      if (lane == 0) {
+        constexpr uint32_t idesc_s = umma_idesc_bf16(BLK_M, BLK_N, false, false);
+        constexpr uint32_t idesc_o = umma_idesc_bf16(BLK_M, HD, false, true);
+        bool ok = mbar_wait(q_full, 0, status, KF_ERR_WAIT_FULL);
+        const int lim[2] = {n_a, n_b};                    // key tiles below lim[tile] belong to the query tile
+        // S_tile = Q_tile K^T with the i-th walked key tile; the caller has made sure it landed
+        auto issue_s = [&](int tile, int i) {
+          const int st = i & 1;
 #pragma unroll
-          for (int kk = 0; kk < BLK_N / 32; ++kk)
-            tc_mma_f16_ts(o_col(tile), s_col(tile) + kk * 8,
-                          umma_desc_sw128(v_smem + st * C::TILE_BYTES + kk * 2048, C::BLOCK_BYTES, 1024), idesc_o,
-                          (i | kk) != 0);
-          if (!mbar_wait(p_full(tile), i & 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
-          tc_fence_after();
-#pragma unroll
-          for (int kk = BLK_N / 32; kk < BLK_N / 16; ++kk)
-            tc_mma_f16_ts(o_col(tile), s_col(tile) + kk * 8,
-                          umma_desc_sw128(v_smem + st * C::TILE_BYTES + kk * 2048, C::BLOCK_BYTES, 1024), idesc_o, 1u);
-          tc_commit(pv_done(tile));
-          if (jn >= lim[tile]) tc_commit(o_final(tile));  // a phase of its own: cannot be mistaken for an earlier tile
-          // the next score tile of this query tile follows at once (its buffer's P was read by the MMAs just issued)
-          if (jn < lim[tile]) {
-            if (!k_next_ready) {
-              if (!mbar_wait(k_full((i + 1) & 1), ((i + 1) >> 1) & 1, status, KF_ERR_WAIT_FULL)) { ok = false; break; }
-              tc_fence_after();
-              k_next_ready = true;
-            }
-            issue_s(tile, i + 1);
+          for (int kk = 0; kk < HD / 16; ++kk) {
+            const uint32_t off = (kk / 4) * C::BLOCK_BYTES + (kk % 4) * 32;
+            tc_mma_f16(s_col(tile), umma_desc_sw128(q_smem + tile * C::TILE_BYTES + off, 16, 1024),
+                       umma_desc_sw128(k_smem + st * C::TILE_BYTES + off, 16, 1024), idesc_s, kk != 0);
+          }
+          tc_commit(s_full(tile));
+        };
+        int j = first_tile();
+        if (ok && j < n_max) {
+          ok = mbar_wait(k_full(0), 0, status, KF_ERR_WAIT_FULL);
+          if (ok) {
+            tc_fence_after();
+            if (j < n_a) issue_s(0, 0);
+            if (j < n_b) issue_s(1, 0);
+            tc_commit(k_empty(0));
           }
         }
-        if (ok) {
-          tc_commit(v_empty(st));                               // V_j read by both query tiles
-          if (jn < n_max) tc_commit(k_empty((i + 1) & 1));      // the next K tile read by every S that needs it
+        for (int i = 0; j < n_max && ok; ++i) {
+          const int st = i & 1, jn = next_tile(j);
+          bool k_next_ready = false;
+          for (int tile = 0; tile < 2 && ok; ++tile) {
+            if (j >= lim[tile]) continue;
+            // O_tile += P_tile V_j : A = P from tensor memory, B = V with the head dim contiguous (MN-major).  The
+            // softmax warps hand P over in two halves: the products over the first 64 keys run while the
+            // exponentials of the last 64 are still being computed.
+            if (!mbar_wait(p_half(tile), i & 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
+            if (!mbar_wait(v_full(st), (i >> 1) & 1, status, KF_ERR_WAIT_FULL)) { ok = false; break; }
+            tc_fence_after();
+#pragma unroll
+            for (int kk = 0; kk < BLK_N / 32; ++kk)
+              tc_mma_f16_ts(o_col(tile), s_col(tile) + kk * 8,
+                            umma_desc_sw128(v_smem + st * C::TILE_BYTES + kk * 2048, C::BLOCK_BYTES, 1024), idesc_o,
+                            (i | kk) != 0);
+            if (!mbar_wait(p_full(tile), i & 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
+            tc_fence_after();
+#pragma unroll
+            for (int kk = BLK_N / 32; kk < BLK_N / 16; ++kk)
+              tc_mma_f16_ts(o_col(tile), s_col(tile) + kk * 8,
+                            umma_desc_sw128(v_smem + st * C::TILE_BYTES + kk * 2048, C::BLOCK_BYTES, 1024), idesc_o, 1u);
+            tc_commit(pv_done(tile));
+            if (jn >= lim[tile]) tc_commit(o_final(tile));  // a phase of its own: cannot be mistaken for an earlier tile
+            // the next score tile of this query tile follows at once (its buffer's P was read by the MMAs just issued)
+            if (jn < lim[tile]) {
+              if (!k_next_ready) {
+                if (!mbar_wait(k_full((i + 1) & 1), ((i + 1) >> 1) & 1, status, KF_ERR_WAIT_FULL)) { ok = false; break; }
+                tc_fence_after();
+                k_next_ready = true;
+              }
+              issue_s(tile, i + 1);
+            }
+          }
+          if (ok) {
+            tc_commit(v_empty(st));                               // V_j read by both query tiles
+            if (jn < n_max) tc_commit(k_empty((i + 1) & 1));      // the next K tile read by every S that needs it
+          }
+          j = jn;
         }
-        j = jn;
-      }
-      if (!ok) {
-        tc_commit(drain_bar);
-        mbar_wait(drain_bar, 0, status, KF_ERR_WAIT_DRAIN);
+        if (!ok) {
+          tc_commit(drain_bar);
+          mbar_wait(drain_bar, 0, status, KF_ERR_WAIT_DRAIN);
+        }
       }
     }
   } else {
-    // ------------------------------------------------------------ softmax + epilogue: warps 2-5 tile A, 6-9 tile B
-    const int tile = (warp - 2) >> 2;
+    // ------------------------------------------------------------ softmax + epilogue: warps 4-7 tile A, 8-11 tile B
+    regs_take<REGS_SOFTMAX>();
+    const int tile = (warp >> 2) - 1;
     const int quarter = warp & 3;
     const int r_local = quarter * 32 + lane;
     const int t0 = m0 + tile * BLK_M;          // first query row of this tile
