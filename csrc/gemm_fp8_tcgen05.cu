@@ -421,6 +421,15 @@ int kf_gemm_fp8(const void* A, const void* B, void* C, int M, int N, int K, long
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
+// scale[0] = fp8_max / max(partial[0 .. blocks)).
+int kf_fp8_scale_from_partial(const void* partial, int blocks, int e5m2, void* scale, void* stream) {
+  using namespace kf::f8;
+  kf_scale_from_amax<<<1, 256, 0, (cudaStream_t)stream>>>(reinterpret_cast<const float*>(partial), blocks, reinterpret_cast<float*>(scale),
+                                                          e5m2 ? E5M2_MAX : E4M3_MAX);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 400 + (int)e;
+}
+
 // scale[0] = fp8_max / absmax(x) for n bf16 values; amax_scratch holds AMAX_BLOCKS (1024) floats.
 int kf_fp8_scale_bf16(const void* x, long long n, int e5m2, void* amax_scratch, void* scale, void* stream) {
   using namespace kf::f8;

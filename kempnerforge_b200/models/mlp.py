@@ -28,6 +28,12 @@ class SwiGLUMLP(nn.Module):
         if self.tp is not None:
             gu = self.tp.column_linear(x, [self.gate_proj.weight, self.up_proj.weight])
             return self.tp.row_linear(F.swiglu_stacked(gu), self.down_proj.weight)
+        if x.is_cuda and getattr(self.gate_proj.weight, "_kf_fp8", False):
+            from kempnerforge_b200.ops import fp8
+
+            y = fp8.swiglu_mlp(x, self.gate_proj.weight, self.up_proj.weight, self.down_proj.weight)
+            if y is not None:
+                return y
         gu = F.fused_linear(x, [self.gate_proj.weight, self.up_proj.weight])
         return F.linear(F.swiglu_stacked(gu), self.down_proj.weight)
 

@@ -88,6 +88,9 @@ def _declare(L: ctypes.CDLL) -> None:
         "kf_test_flag_timeout": [vp, i, ll],
         "kf_gemm_fp8": [vp, vp, vp, i, i, i, ll, ll, i, i, i, vp, vp, i, i, vp],
         "kf_fp8_scale_bf16": [vp, ll, i, vp, vp, vp],
+        "kf_fp8_scale_from_partial": [vp, i, i, vp, vp],
+        "kf_swiglu_fwd_scale_bf16": [vp, vp, ll, i, i, vp, vp, vp],
+        "kf_swiglu_bwd_scale_bf16": [vp, vp, vp, ll, i, i, vp, vp, vp],
         "kf_fp8_cast_bf16": [vp, i, i, ll, vp, i, vp, ll, vp, ll, vp],
         "kf_lion": [vp, vp, vp, ll, i, f, f, f, f, vp],
         "kf_sf_adamw": [vp, vp, vp, vp, vp, ll, i, f, f, f, f, f, f, f, i, vp],
@@ -549,6 +552,26 @@ def swiglu_bwd(dh: torch.Tensor, gu: torch.Tensor, out=None) -> torch.Tensor:
     dgu = torch.empty_like(gu) if out is None else out
     _check(lib().kf_swiglu_bwd_bf16(dh.data_ptr(), gu.data_ptr(), dgu.data_ptr(), rows, h, _stream()), "kf_swiglu_bwd_bf16")
     return dgu
+
+
+def swiglu_fwd_scale(gu: torch.Tensor, e5m2: bool = False):
+    """(:func:`swiglu_fwd` of gu (rows, 2H), what :func:`fp8_scale` gives for it): the maximum is taken while the values pass."""
+    rows, h = gu.shape[0], gu.shape[1] // 2
+    out = torch.empty((rows, h), dtype=gu.dtype, device=gu.device)
+    scratch = torch.empty(1 + 148 * 16, dtype=torch.float32, device=gu.device)   # the scale, then partial maxima
+    _check(lib().kf_swiglu_fwd_scale_bf16(gu.data_ptr(), out.data_ptr(), rows, h, int(e5m2), scratch.data_ptr() + 4, scratch.data_ptr(),
+                                          _stream()), "kf_swiglu_fwd_scale_bf16", 2)
+    return out, scratch[:1]
+
+
+def swiglu_bwd_scale(dh: torch.Tensor, gu: torch.Tensor, e5m2: bool = True):
+    """(:func:`swiglu_bwd` in a tensor of its own, its fp8 scale)."""
+    rows, h = gu.shape[0], gu.shape[1] // 2
+    dgu = torch.empty_like(gu)
+    scratch = torch.empty(1 + 148 * 16, dtype=torch.float32, device=gu.device)
+    _check(lib().kf_swiglu_bwd_scale_bf16(dh.data_ptr(), gu.data_ptr(), dgu.data_ptr(), rows, h, int(e5m2), scratch.data_ptr() + 4,
+                                          scratch.data_ptr(), _stream()), "kf_swiglu_bwd_scale_bf16", 2)
+    return dgu, scratch[:1]
 
 
 def embedding_fwd(ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:

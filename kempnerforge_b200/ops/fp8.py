@@ -148,6 +148,73 @@ class _Fp8LinearFn(torch.autograd.Function):
         return (dx, *wgrads)
 
 
+class _Fp8SwiGLUFn(torch.autograd.Function):
+    """down(silu(x Wgᵀ) * (x Wuᵀ)) with fp8 products as one node: the arithmetic of two :class:`_Fp8LinearFn` around the SwiGLU
+    kernel, except that the maxima of the hidden activation and of d[gate | up], which their casts wait for, come from the
+    kernels that write them."""
+
+    @staticmethod
+    def forward(ctx, x, wg, wu, wd):
+        from kempnerforge_b200.ops import cuda as cu
+
+        x2 = x.reshape(-1, x.shape[-1])
+        if not x2.is_contiguous():
+            x2 = x2.contiguous()
+        sx, x8, _ = quantize(x2)
+        s_gu, w8, _ = quantized_weight((wg, wu), want_t=False)
+        gu = scaled_mm(x8, w8, sx, s_gu)
+        h, sh = cu.swiglu_fwd_scale(gu)
+        _, h8, _ = quantize(h, scale=sh)
+        sd, d8, _ = quantized_weight((wd,), want_t=False)
+        y = scaled_mm(h8, d8, sh, sd)
+        ctx.save_for_backward(x2, sx, s_gu, gu, h, sh, sd, wg, wu, wd)
+        ctx.x_shape = x.shape
+        return y.view(*x.shape[:-1], d8.shape[0])
+
+    @staticmethod
+    def backward(ctx, dy):
+        from kempnerforge_b200.ops import cuda as cu
+        from kempnerforge_b200.ops import functional as F
+
+        x2, sx, s_gu, gu, h, sh, sd, wg, wu, wd = ctx.saved_tensors
+        dy2 = dy.reshape(-1, dy.shape[-1])
+        if not dy2.is_contiguous():
+            dy2 = dy2.contiguous()
+        need_x, need_g, need_u, need_d = ctx.needs_input_grad
+        need_h = need_x or need_g or need_u
+        sg, g8, g8t = quantize(dy2, e5m2=True, want_row=need_h, want_t=need_d)
+        dx = g_wg = g_wu = g_wd = None
+        if need_h:
+            _, _, d8t = quantized_weight((wd,), want_t=True)
+            dgu, s_dgu = cu.swiglu_bwd_scale(scaled_mm(g8, d8t, sg, sd, a_e5m2=True), gu)
+        if need_d:
+            _, _, h8t = quantize(h, want_row=False, want_t=True, scale=sh)
+            (g_wd,) = F._deposit_stacked_weight_grads(
+                [wd], (True,), lambda out, acc: scaled_mm(g8t, h8t, sg, sh, a_e5m2=True, out=out, accumulate=acc))
+        if need_h:
+            need_w = need_g or need_u
+            _, q8, q8t = quantize(dgu, e5m2=True, want_row=need_x, want_t=need_w, scale=s_dgu)
+            if need_x:
+                _, _, w8t = quantized_weight((wg, wu), want_t=True)
+                dx = scaled_mm(q8, w8t, s_dgu, s_gu, a_e5m2=True).view(ctx.x_shape)
+            if need_w:
+                _, _, x8t = quantize(x2, want_row=False, want_t=True, scale=sx)
+                g_wg, g_wu = F._deposit_stacked_weight_grads(
+                    [wg, wu], (need_g, need_u),
+                    lambda out, acc: scaled_mm(q8t, x8t, s_dgu, sx, a_e5m2=True, out=out, accumulate=acc))
+        return dx, g_wg, g_wu, g_wd
+
+
+def swiglu_mlp(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, wd: torch.Tensor) -> torch.Tensor | None:
+    """A SwiGLU feed-forward whose three weights are tagged for fp8 and that the node covers, else None."""
+    from kempnerforge_b200.ops import functional as F
+
+    if (not F.use_native(x) or x.numel() == 0 or not supported(x, [wg, wu, wd]) or wg.shape != wu.shape
+            or wd.shape[1] != wg.shape[0] or wg.shape[1] != x.shape[-1] or any(not w.is_cuda or w.dtype != torch.bfloat16 for w in (wg, wu, wd))):
+        return None
+    return _Fp8SwiGLUFn.apply(x, wg, wu, wd)
+
+
 def linear(x: torch.Tensor, weights: list[torch.Tensor]) -> torch.Tensor:
     """fp8 Linear against one weight or several weights stacked along the output dimension."""
     return _Fp8LinearFn.apply(x, *weights)
