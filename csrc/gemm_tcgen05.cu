@@ -16,6 +16,7 @@
 // SwiGLU gate/up/down, output head: kempnerforge/model/attention.py:150-152,236,
 // kempnerforge/model/mlp.py:26, kempnerforge/model/embedding.py:51) and their backward.
 #include "common.cuh"
+#include "pair_common.cuh"
 #include "gemm_epilogue.cuh"
 #include "tile_math.h"
 
@@ -269,7 +270,35 @@ int launch_gemm_2cta(const void* A, const void* B, void* C, const void* R, int M
                      int ldc, int ldr, int a_mn, int b_mn, int out_f32, int accumulate, int num_sms,
                      cudaStream_t stream, int* status);
 float gemm_pair_cost(int M, int N, int num_sms);
+int tokens_width(int T, int m_rows, int num_sms, float* cost, int* rounds);
+int launch_tokens_plain(const void* x, const void* const* w, const int* rows, int n_seg, int w_mn, void* out, const void* residual, int T,
+                        int F, int K, int ldx, int ldw, int ldo, int ldr, int tile_n, int num_sms, cudaStream_t stream, int* status);
 }
+
+namespace kf {
+// Width of the token tiles (gemm_tokens_tcgen05_2cta.cu) if they pay for x[M, K] over N columns, else 0.  The other kernels in the
+// measure of tokens_width: pairs as they are, a round of single-CTA tiles 920 (their k-block takes 1.2 times that of a pair) or,
+// over an MN-major B, 800.   Measured, token
+// tiles / the others, us: 4096 columns from 14336 over 300 rows 74 / 95, over 1200 rows 145 / 150; 5120 from 13824 over 777
+// rows, where single CTAs have one round and pairs two, 138 / 98; at equal rounds 4096 from 4096 over 2300 rows 57 / 60, from more
+// than four rounds on no difference.  Input gradients (MN-major): 5120 columns from 7168 over 1332 rows 80 / 94, over 2000 118 /
+// 119; from 2048, where the ramp shows, 17.3 / 16.7 over 1554 rows.
+static int tokens_pay(int M, int N, int K, int b_mn, int pair, int num_sms) {
+  if (num_sms < 2 || (b_mn && K < 3072)) return 0;
+  const int pairs = num_sms / 2;
+  float cost, other;
+  int rounds;
+  const int tn = kf2::tokens_width(M, N, num_sms, &cost, &rounds);
+  if (pair) {
+    const int w = b_mn ? 256 : kf::pairops::pair_tile_width(M, N, pairs, nullptr);
+    other = float(512 + w) * float(((long long)((M + 255) / 256) * ((N + w - 1) / w) + pairs - 1) / pairs);
+  } else {
+    other = (b_mn ? 800.f : 920.f) * float(((long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN) + num_sms - 1) / num_sms);
+  }
+  if (b_mn) return cost * (1.f + 160.f / float(K)) < 0.96f * other ? tn : 0;  // W is the transposed operand: ramp of 2.5 k-blocks
+  return cost <= (rounds <= 4 ? 1.f : 0.97f) * other ? tn : 0;
+}
+}  // namespace kf
 
 namespace kf2 {
 int launch_gemm_swiglu_2cta(const void* A, const void* Wg, const void* Wu, void* H, void* GU, int M, int F, int K, int lda,
@@ -324,8 +353,14 @@ int kf_gemm_dgrad_stacked_bf16(const void* dy, const void* w0, const void* w1, c
   if ((lda & 7) || (ldw & 7) || (ldc & 7) || M <= 0 || K <= 0) return 5;
   const void* w[3] = {w0, w1, w2};
   const int rows[3] = {n0, n1, n2};
-  // the rule of kf_gemm_bf16 for an MN-major B: pairs once their tiles are two rounds
-  if ((long long)((M + 255) / 256) * ((K + 255) / 256) < 2LL * (num_sms / 2))
+  // the rules of kf_gemm_bf16 for an MN-major B: pairs once their tiles are two rounds, token tiles where they are shorter
+  const int pair = (long long)((M + 255) / 256) * ((K + 255) / 256) >= 2LL * (num_sms / 2);
+  const int n_seg = n1 <= 0 ? 1 : n2 <= 0 ? 2 : 3;
+  const bool whole = n0 > 0 && (n0 % 64 == 0 || n_seg == 1) && (n1 % 64 == 0 || n_seg < 3);  // no k-block reaches over two weights
+  if (const int tn = whole ? kf::tokens_pay(M, K, n0 + n1 + n2, 1, pair, num_sms) : 0)
+    return kf2::launch_tokens_plain(dy, w, rows, n_seg, 1, out, nullptr, M, K, n0 + n1 + n2, lda, ldw, ldc, 0, tn, num_sms,
+                                    (cudaStream_t)stream, kf::status_ptr());
+  if (!pair)
     return kf::launch_gemm<false, true, __nv_bfloat16>(dy, w, rows, out, nullptr, M, K, n0 + n1 + n2, lda, ldw, ldc, 0, 0, num_sms,
                                                        (cudaStream_t)stream);
   return kf2::launch_gemm_stacked_k_2cta(dy, w, rows, out, M, K, n0 + n1 + n2, lda, ldw, ldc, num_sms, (cudaStream_t)stream,
@@ -389,7 +424,8 @@ int kf_gemm_swiglu_bf16(const void* x, const void* wg, const void* wu, void* h, 
 //   b_mn == 0: B is stored [N][ldb] (K contiguous);  b_mn == 1: B is stored [K][ldb] (N contiguous)
 //   out_f32: C (and R) are fp32 instead of bf16.  Leading dimensions in elements; A/B pitches must be
 //   multiples of 8 elements and base pointers 16-byte aligned (TMA), ldc/ldr multiples of 8 (bf16) / 4 (fp32).
-//   mode: 0 = pick automatically, 1 = one CTA per 128x256 tile, 2 = CTA pairs (cta_group::2) on 256x256 tiles.
+//   mode: 0 = pick automatically, 1 = one CTA per 128x256 tile, 2 = CTA pairs (cta_group::2) on 256x256 tiles, 3 = CTA pairs on
+//   tiles of 256 columns of C and a width of rows chosen per launch (A K-major, bf16 output, no accumulation, N % 8 == 0).
 // Returns 0 on success, otherwise a code identifying the failing step.
 int kf_gemm_bf16(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb,
                  int ldc, int ldr, int a_mn, int b_mn, int out_f32, int accumulate, int mode, int num_sms,
@@ -397,7 +433,8 @@ int kf_gemm_bf16(const void* A, const void* B, void* C, const void* R, int M, in
   using namespace kf;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (M <= 0 || N <= 0 || K <= 0) return 1;
-  if (mode == 0) {
+  const bool automatic = mode == 0;
+  if (automatic) {
     // pairs pay off once there are enough 256x256 tiles to fill the machine a few times over
     const long long pair_tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
     mode = pair_tiles >= 2LL * (num_sms / 2) ? 2 : 1;
@@ -409,6 +446,13 @@ int kf_gemm_bf16(const void* A, const void* B, void* C, const void* R, int M, in
       if (kf2::gemm_pair_cost(M, N, num_sms) < 1.1f * BN * float((tiles + num_sms - 1) / num_sms)) mode = 2;
     }
   }
+  if (!a_mn && !out_f32 && !accumulate && num_sms >= 2 && (N & 7) == 0 && (automatic || mode == 3)) {
+    const int tn = mode == 3 ? kf2::tokens_width(M, N, num_sms, nullptr, nullptr) : tokens_pay(M, N, K, b_mn, mode == 2, num_sms);
+    const void* w[3] = {B, nullptr, nullptr};
+    const int rows[3] = {b_mn ? K : N, 0, 0};
+    if (tn) return kf2::launch_tokens_plain(A, w, rows, 1, b_mn, C, R, M, N, K, lda, ldb, ldc, ldr, tn, num_sms, st, status_ptr());
+  }
+  if (mode == 3) return 6;
   if (mode == 2)
     return kf2::launch_gemm_2cta(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, out_f32, accumulate, num_sms,
                                  st, status_ptr());

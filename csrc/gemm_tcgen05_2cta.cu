@@ -30,6 +30,29 @@ namespace kf2 {
 using namespace kf;
 using namespace kf::pairops;
 
+// gemm_tokens_tcgen05_2cta.cu: the same products with tiles cut to the number of rows of A
+int tokens_width(int T, int m_rows, int num_sms, float* cost, int* rounds);
+int launch_tokens_swiglu(const void* x, const void* wg, const void* wu, void* h, const void* gu, int T, int F, int K, int ldx, int ldw,
+                         int ldh, int ldgu, int tile_n, int num_sms, cudaStream_t stream, int* status);
+int launch_tokens_rope(const void* x, const void* const* w, const int* rows, int n_seg, void* out, int T, int F, int K, int ldx, int ldw,
+                       int ldo, const float* cosT, const float* sinT, int S, int rope_cols, int hd, int tile_n, int num_sms,
+                       cudaStream_t stream, int* status);
+int launch_tokens_swiglu_bwd(const void* dy, const void* w, const void* gu, void* dgu, int T, int F, int K, int ldy, int ldw, int ldgu,
+                             int tile_n, int num_sms, cudaStream_t stream, int* status);
+
+// Width of the token tiles if they pay against 256 x 256 tiles of the same product, else 0.  m_rows: rows of the weight stack;
+// `limit`: what the modelled cost (tokens_width) must fall to.  Their epilogue turns the accumulators, so a step of one width
+// (0.96) is worth it only where enough k-blocks hide that.  Measured, token tiles / these: gate and
+// up of 14336 over 777 tokens (0.96) 162 / 167 us, 7168 over 999 from 2048 columns (0.96) 55 / 53; q | k | v of 6144 over 520 (0.92) 34 /
+// 35, over 640 (0.96) 35.2 / 34.9; the gradient 78 / 82 (520, 0.92) and 196 / 192 (2000, 0.96).
+static int tokens_pay(int M, int m_rows, int n_tiles, float limit, int num_sms) {
+  const int pairs = num_sms / 2;
+  const long long tiles = (long long)((M + 255) / 256) * n_tiles;
+  float cost;
+  const int tn = tokens_width(M, m_rows, num_sms, &cost, nullptr);
+  return cost < limit * 768.f * float((tiles + pairs - 1) / pairs) ? tn : 0;
+}
+
 constexpr int CTA_M = 128;   // rows of A per CTA
 constexpr int TILE_M = 256;  // rows per CTA pair
 constexpr int TILE_N = 256;
@@ -583,6 +606,8 @@ static int launch(const void* A, const void* B, void* C, const void* R, int M, i
 // h[M, F] = silu(x Wg^T) * (x Wu^T), Wg and Wu [F][K] each; gu (optional) receives [M, 2F] pre-activations.  F % 128 == 0.
 int launch_gemm_swiglu_2cta(const void* A, const void* Wg, const void* Wu, void* H, void* GU, int M, int F, int K, int lda,
                             int ldw, int ldh, int ldgu, int num_sms, cudaStream_t stream, int* status) {
+  if (const int tn = tokens_pay(M, 2 * F, (F + HALF_N - 1) / HALF_N, K >= 4096 ? 0.97f : 0.93f, num_sms))
+    return launch_tokens_swiglu(A, Wg, Wu, H, GU, M, F, K, lda, ldw, ldh, ldgu, tn, num_sms, stream, status);
   CUtensorMap ma;
   WeightSegs ws;
   int rc = make_map_2d_bf16(&ma, A, M, K, lda, BK, CTA_M);
@@ -618,6 +643,12 @@ int launch_gemm_rope_2cta(const void* A, const void* const* W, const int* rows, 
                           int ldw, int ldc, const float* cosT, const float* sinT, int S, int rope_cols, int hd, int num_sms,
                           cudaStream_t stream, int* status) {
   if ((hd != 64 && hd != 128 && hd != 256) || N % hd || rope_cols % hd || rope_cols > N || S <= 0) return 6;
+  if (hd != 256)
+    if (const int tn = tokens_pay(M, N, (N + TILE_N - 1) / TILE_N, 0.93f, num_sms)) {
+      const int n_seg = rows[1] <= 0 ? 1 : rows[2] <= 0 ? 2 : 3;
+      if (rows[0] <= 0 || rows[0] + (n_seg > 1 ? rows[1] : 0) + (n_seg > 2 ? rows[2] : 0) != N) return 6;
+      return launch_tokens_rope(A, W, rows, n_seg, C, M, N, K, lda, ldw, ldc, cosT, sinT, S, rope_cols, hd, tn, num_sms, stream, status);
+    }
   CUtensorMap ma;
   WeightSegs ws;
   int rc = make_map_2d_bf16(&ma, A, M, K, lda, BK, CTA_M);
@@ -753,6 +784,8 @@ int launch_gemm_gather_2cta(int epi, const void* A, void* C, const void* R, int 
 // weight read for its input gradient); gu and dgu may be the same buffer.  F % 8 == 0, K % 64 == 0.
 int launch_gemm_swiglu_bwd_2cta(const void* DY, const void* W, const void* GU, void* DGU, int M, int F, int K, int lda,
                                 int ldw, int ldgu, int num_sms, cudaStream_t stream, int* status) {
+  if (const int tn = tokens_pay(M, F, (F + TILE_N - 1) / TILE_N, 0.93f, num_sms))
+    return launch_tokens_swiglu_bwd(DY, W, GU, DGU, M, F, K, lda, ldw, ldgu, tn, num_sms, stream, status);
   CUtensorMap ma, mb;
   int rc = make_map_2d_bf16(&ma, DY, M, K, lda, BK, CTA_M);
   if (rc) return 100 + rc;
