@@ -278,10 +278,9 @@ int launch_tokens_plain(const void* x, const void* const* w, const int* rows, in
 namespace kf {
 // Width of the token tiles (gemm_tokens_tcgen05_2cta.cu) if they pay for x[M, K] over N columns, else 0.  The other kernels in the
 // measure of tokens_width: pairs as they are, a round of single-CTA tiles 920 (their k-block takes 1.2 times that of a pair) or,
-// over an MN-major B, 800.   Measured, token
-// tiles / the others, us: 4096 columns from 14336 over 300 rows 74 / 95, over 1200 rows 145 / 150; 5120 from 13824 over 777
-// rows, where single CTAs have one round and pairs two, 138 / 98; at equal rounds 4096 from 4096 over 2300 rows 57 / 60, from more
-// than four rounds on no difference.  Input gradients (MN-major): 5120 columns from 7168 over 1332 rows 80 / 94, over 2000 118 /
+// over an MN-major B, 800.  Measured, token tiles / the others, us: 4096 columns from 14336 over 300 rows 74 / 95, over 1200 rows
+// 145 / 150; 5120 from 13824 over 777 rows, where single CTAs have one round and pairs two, 138 / 98; at equal rounds 4096 from
+// 4096 over 2300 rows 57 / 60, from more than four rounds on no difference.  Input gradients (MN-major): 5120 columns from 7168 over 1332 rows 80 / 94, over 2000 118 /
 // 119; from 2048, where the ramp shows, 17.3 / 16.7 over 1554 rows.
 static int tokens_pay(int M, int N, int K, int b_mn, int pair, int num_sms) {
   if (num_sms < 2 || (b_mn && K < 3072)) return 0;
