@@ -6,6 +6,10 @@
 //   -> o projection (+ x) -> RMSNorm -> gate|up projection (SwiGLU) -> down projection (+ residual)
 // as programmatic launches: each kernel sets up (and streams its first weight tiles) while its predecessor drains.  Up to
 // kf_skinny_norm_rows() sequences the projections take their norms along: five kernels in the chain instead of seven.
+//
+// Inside the chain a kernel may fetch weights ahead of its wait, because the kernel before it writes none.  The kernel before the
+// chain is the caller's, which may have written any operand of the first one (a weight copied in, rotary tables built for this step),
+// so the first kernel either waits before it reads anything (the norm) or is an ordinary launch (the projection with its norm).
 #include "common.cuh"
 
 extern "C" {
@@ -38,7 +42,8 @@ int kf_attn_fwd_pdl_bf16(const void* q, const void* k, const void* v, void* o, v
 //   a[27]: parts to run (1 = up to the cache, 2 = attention, 4 = the rest); a[28]: attention kernel (0 = split over the cache,
 //   1 = the 128-row tile kernel, B == 1); a[29]: attention output [B][H * hd] (written by part 2, read by part 4); a[30]: fp32
 //   [H] scratch of the tile kernel
-int kf_block_decode_bf16(const long long* a, const double* r, void* stream) {
+// first: the block's first kernel follows a kernel of the caller's.
+static int block_decode(const long long* a, const double* r, bool first, void* stream) {
   void* p[18];
   for (int i = 0; i < 18; ++i) p[i] = reinterpret_cast<void*>(a[i]);
   const void *x = p[0], *wn1 = p[1], *wq = p[2], *wk = p[3], *wv = p[4], *wo = p[5], *wn2 = p[6], *wg = p[7], *wu = p[8],
@@ -64,7 +69,7 @@ int kf_block_decode_bf16(const long long* a, const double* r, void* stream) {
       if (rc) return 1000 + rc;
     }
     rc = kf_gemm_skinny_norm_qkv_bf16(norm_along ? x : n, norm_along ? wn1 : nullptr, eps1, wq, wk, wv, q, (bf*)kc + row, (bf*)vc + row,
-                                      B, 1, D, qc, kvc, hd, D, D, D, D, qc, cache_batch, cosT, sinT, 1, num_sms, stream);
+                                      B, 1, D, qc, kvc, hd, D, D, D, D, qc, cache_batch, cosT, sinT, !(first && norm_along), num_sms, stream);
     if (rc) return 2000 + rc;
   }
   if (parts & 2) {
@@ -91,11 +96,13 @@ int kf_block_decode_bf16(const long long* a, const double* r, void* stream) {
   return rc ? 7000 + rc : 0;
 }
 
+int kf_block_decode_bf16(const long long* a, const double* r, void* stream) { return block_decode(a, r, true, stream); }
+
 // n blocks in a row: a holds 31 values per block, r three.  The blocks may share their intermediates (scratch, rstd, h1, attention):
 // a kernel of the chain writes only after all kernels before it are complete.
 int kf_blocks_decode_bf16(const long long* a, const double* r, int n, void* stream) {
   for (int i = 0; i < n; ++i) {
-    const int rc = kf_block_decode_bf16(a + 31 * i, r + 3 * i, stream);
+    const int rc = block_decode(a + 31 * i, r + 3 * i, i == 0, stream);
     if (rc) return rc;
   }
   return 0;

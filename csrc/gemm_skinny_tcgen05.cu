@@ -12,7 +12,8 @@
 //   * the launch is programmatic: barriers, tensor memory and the first ring of W tiles are set up while the previous
 //     kernel of the stream drains; x is read only after griddepcontrol.wait.  (Every kernel of this library that
 //     triggers its dependents does so after its own wait, so when a block of this grid starts, all work before the
-//     immediately preceding kernel is complete and visible; that kernel itself never writes weights.)
+//     immediately preceding kernel is complete and visible; the caller asks for such a launch only where that kernel
+//     itself writes no weights, see block_infer.cu.)
 //
 // With NORM the operand is RMSNorm(x) and x comes in as it is: the four epilogue warps, idle until the accumulator is done,
 // compute each row's scale and write the normalised 64-column blocks into the ring, in the arithmetic and order of

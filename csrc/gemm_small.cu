@@ -7,8 +7,8 @@
 // 16 to 4096, 65 536 sums each).  Hence
 //   * a CTA owns 16 rows of W: the m16n8k16 tile of one warp, up to two of them for up to 16 tokens;
 //   * the CTA's whole strip of W (K <= 4096: 16 rows of at most 8 KB) is requested with one bulk copy per row before the
-//     previous kernel of the stream has finished (programmatic launch; weights are never written by that kernel), so that
-//     only x, the chain and the store remain behind it;
+//     previous kernel of the stream has finished (a programmatic launch: only behind a kernel that writes no weights and no
+//     gain, see block_infer.cu), so that only x, the chain and the store remain behind it;
 //   * the accumulator of a thread holds rows g and g + 8 of the tile, which are made gate and up of one hidden unit, or the two
 //     halves of a rotary pair: no exchange before the epilogue;
 //   * optionally the norm of x is taken along, in the arithmetic and order of kf_rmsnorm_fwd (the same bits).
@@ -98,6 +98,13 @@ kf_gemm_small(const __grid_constant__ SmallWeights sw, const __grid_constant__ A
     if (NORM) bulk_row(g_smem, a.gain, 2 * K, w_bar);
   }
   const int g = lane >> 2, t2 = (lane & 3) * 2;  // this thread's rows g and g + 8, tokens nt * 8 + t2 and t2 + 1
+  __syncthreads();
+  grid_dep_wait();
+  grid_dep_launch();
+  if (tid == 0) {
+    mbar_expect_tx(x_bar, uint32_t(a.M) * 2 * K);
+    for (int r = 0; r < a.M; ++r) bulk_row(x_smem + r * pitch, a.x + size_t(r) * a.ldx, 2 * K, x_bar);
+  }
   float cs[NT][2], sn[NT][2];
   if (EPI == 2 && warp == 0 && seg < 2) {
 #pragma unroll
@@ -109,13 +116,6 @@ kf_gemm_small(const __grid_constant__ SmallWeights sw, const __grid_constant__ A
         cs[nt][e] = a.cosT[at];
         sn[nt][e] = a.sinT[at];
       }
-  }
-  __syncthreads();
-  grid_dep_wait();
-  grid_dep_launch();
-  if (tid == 0) {
-    mbar_expect_tx(x_bar, uint32_t(a.M) * 2 * K);
-    for (int r = 0; r < a.M; ++r) bulk_row(x_smem + r * pitch, a.x + size_t(r) * a.ldx, 2 * K, x_bar);
   }
   float res[NT][4];
   if (EPI == 0 && warp == 0 && a.residual) {

@@ -139,3 +139,48 @@ def test_models_that_go_block_by_block(native_lib):
     assert run(model, caches) is not None
     assert run(*_model(8, 8, 2, 40), batch=2) is None                           # heads of 64, several sequences: the library's attention
     assert run(*_model(4, 4, 1, 40, qk_norm=True)) is None
+
+
+@pytest.mark.parametrize("written", ["weight", "gain", "tables"])
+@pytest.mark.parametrize("dim,heads,kv,ffn,batch", [(768, 12, 12, 2048, 1), (512, 4, 2, 768, 4), (512, 4, 2, 768, 6), (4096, 32, 8, 4096, 1)])
+def test_operands_written_by_the_kernel_before_the_step(native_lib, dim, heads, kv, ffn, batch, written):
+    """The kernel in front of a generation step may have written any operand of its first projection."""
+    from kempnerforge_b200.config import ModelConfig
+    from kempnerforge_b200.models.attention import KVCache
+    from kempnerforge_b200.models.transformer import TransformerBlock
+
+    torch.manual_seed(0)
+    cfg = ModelConfig(dim=dim, n_layers=1, n_heads=heads, n_kv_heads=kv, vocab_size=64, ffn_hidden_dim=ffn, max_seq_len=256)
+    block = TransformerBlock(cfg, 0).to(DEV, torch.bfloat16).eval()
+    hd, ctx = dim // heads, 100
+    cache = KVCache(batch, 128, kv, hd, torch.bfloat16, torch.device(DEV))
+    for i, t in enumerate((cache.k, cache.v)):
+        t.copy_(_rand(*t.shape, seed=20 + i))
+    x, tables = _rand(batch, 1, dim, seed=1), torch.zeros(2, 1, hd // 2, device=DEV)
+    g = torch.Generator(device=DEV).manual_seed(3)
+    if written == "tables":
+        target = tables
+        versions = [torch.rand(2, 1, hd // 2, device=DEV, generator=g) for _ in range(2)]
+    else:
+        target = block.attention.v_proj.weight if written == "weight" else block.attention_norm.weight
+        versions = [_rand(*target.shape, scale=0.05, seed=5 + i) for i in range(2)]
+
+    def step(sync):
+        cache.seq_len = ctx
+        if sync:
+            torch.cuda.synchronize()
+        y = block(x, tables[0], tables[1], kv_cache=cache)
+        return [y, cache.k[:, ctx].clone(), cache.v[:, ctx].clone()]
+
+    with torch.no_grad():
+        want = []
+        for v in versions:
+            target.copy_(v)
+            want.append(step(sync=True))
+        assert not all(torch.equal(a, b) for a, b in zip(*want))
+        got = []
+        for i in range(40):
+            target.copy_(versions[i & 1])
+            got.append(step(sync=False))
+    assert native_lib.read_status() == 0
+    assert all(torch.equal(a, b) for i, out in enumerate(got) for a, b in zip(out, want[i & 1]))
