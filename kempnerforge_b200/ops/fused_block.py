@@ -162,14 +162,16 @@ def _chain_dims(x2, cos, sin, weights, b: int, s: int, d: int, hd: int):
     for w, rows, cols in ((wq, qc, d), (wk, kvc, d), (wv, kvc, d), (wo, d, qc), (wg, f, d), (wu, f, d), (wd, d, f)):
         if not _matrix(w, rows, cols) or w.device != dev or _sharded_unit(w) is not None:
             return None
-    if (not _vector(wn1, d, dev) or not _vector(wn2, d, dev) or x2.data_ptr() % 16 or not kc.rope_tables_ok(cos, sin) or cos.device != dev
+    if (not _vector(wn1, d, dev) or not _vector(wn2, d, dev) or not x2.is_contiguous() or x2.data_ptr() % 16 or not kc.rope_tables_ok(cos, sin) or cos.device != dev
             or sin.device != dev or cos.dim() != 2 or cos.shape != sin.shape or cos.size(0) < s or cos.size(1) != hd // 2):
         return None
     return b, s, d, qc // hd, kvc // hd, hd, f
 
 
 class _ChainState:
-    """What a natively issued forward left for its backward: one buffer, and where its parts start."""
+    """What a natively issued forward left for its backward: one buffer, and where its parts start.  The block's input, tables and
+    weights are not among them: the backward takes the addresses of those that it is given itself.  Autograd may hand back another
+    tensor than the one that was saved (saved-tensor hooks, an enclosing checkpoint), and a parameter's data may have been set anew."""
 
     def __init__(self, x2, cos, sin, weights, dims, eps, keep: bool, need_output: bool) -> None:
         b, s, d, h, hkv, hd, f = dims
@@ -182,14 +184,17 @@ class _ChainState:
         self.dims, self.at, self.scalars = dims, at, array("d", (eps, 1.0 / math.sqrt(hd)))
         self.buf = torch.empty(at[-1], dtype=torch.uint8, device=x2.device)
         base = self.buf.data_ptr()
-        parts = [base + o for o in at[:-1]]
+        self.parts = [base + o for o in at[:-1]]
         if not keep:
-            parts[8] = 0
+            self.parts[8] = 0
         self.y = torch.empty((t, d), dtype=torch.bfloat16, device=x2.device) if need_output else None
-        self.ptrs = [t_.data_ptr() for t_ in (x2, *weights, cos, sin)] + parts + [*dims, kc.sm_count()]
-        ints = array("q", (*self.ptrs, self.y.data_ptr() if need_output else 0))
+        ints = array("q", (*self.block_args(x2, cos, sin, weights), self.y.data_ptr() if need_output else 0))
         kc._check(kc.lib().kf_block_train_fwd_bf16(ints.buffer_info()[0], self.scalars.buffer_info()[0], kc._stream()),
                   "kf_block_train_fwd_bf16", 7 if need_output else 6)
+
+    def block_args(self, x2, cos, sin, weights) -> list:
+        """The first values of either native call."""
+        return [*(t.data_ptr() for t in (x2, *weights, cos, sin)), *self.parts, *self.dims, kc.sm_count()]
 
     def views(self) -> dict:
         """The parts as the tensors that the op-by-op backward reads."""
@@ -218,7 +223,7 @@ def _grad_target(weights):
     return slots[0], int(live[0])
 
 
-def _chain_backward(it: _ChainState, dy2, x2, weights):
+def _chain_backward(it: _ChainState, dy2, x2, cos, sin, weights):
     """(dx, gradients of the nine weights) of a natively issued forward, or None when the gradient slots do not fit."""
     wn1, wq, wk, wv, wo, wn2, wg, wu, wd = weights
     groups = ((wq, wk, wv), (wo,), (wg, wu), (wd,))
@@ -242,7 +247,7 @@ def _chain_backward(it: _ChainState, dy2, x2, weights):
     base = scratch.data_ptr()
     pieces = L.kf_gemm_k_pieces(t, d, 2 * f, kc.sm_count()) if 2 * f >= kc.SPLIT_K_MIN else 1
     stack_gu, ws = kc.rows_adjacent((wg, wu)), None
-    ptrs = list(it.ptrs)
+    ptrs = it.block_args(x2, cos, sin, weights)
     if pieces > 1:
         ws = torch.empty((pieces, t, d), dtype=torch.float32, device=dev)
         if not stack_gu:
@@ -364,19 +369,24 @@ class DenseBlockFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x2, cos, sin = ctx.saved_tensors
+        if not x2.is_contiguous():
+            x2 = x2.contiguous()
         b, s, d, eps, hd, recompute = ctx.meta
         wn1, wq, wk, wv, wo, wn2, wg, wu, wd = ctx.weights
         unit = _sharded_unit(wq)
         if unit is not None:
             unit.engine.prepare_backward(unit)  # parameter staging is ours again; gradient staging slot is free
         it = ctx.inter
-        if it is None and unit is None and ctx.attn_saved is None:
-            dims = _chain_dims(x2, cos, sin, ctx.weights, b, s, d, hd)
-            if dims is not None:
-                it = _ChainState(x2, cos, sin, ctx.weights, dims, eps, keep=True, need_output=False)
+        dims = None
+        if isinstance(it, _ChainState) or (it is None and unit is None and ctx.attn_saved is None):
+            dims = _chain_dims(x2, cos, sin, ctx.weights, b, s, d, hd)   # of the tensors that this pass was given
+        if it is None and dims is not None:
+            it = _ChainState(x2, cos, sin, ctx.weights, dims, eps, keep=True, need_output=False)
         if isinstance(it, _ChainState):
             dy2 = dy.reshape(b * s, d)
-            done = _chain_backward(it, dy2 if dy2.is_contiguous() else dy2.contiguous(), x2, ctx.weights)
+            done = None
+            if dims == it.dims:
+                done = _chain_backward(it, dy2 if dy2.is_contiguous() else dy2.contiguous(), x2, cos, sin, ctx.weights)
             if done is not None:
                 ctx.inter = None
                 return (done[0].view(b, s, d), None, None, *done[1], None, None, None)

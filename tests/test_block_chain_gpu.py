@@ -99,6 +99,59 @@ def test_second_backward_over_a_kept_graph(native_lib):
     assert all(torch.equal(a, b) for a, b in zip(first, again))
 
 
+def _over(block, tables, x, dy, wrap=lambda f, x: f(x)):
+    """Gradients of two passes through the block in a row, their input an intermediate that nothing but the graph keeps."""
+    block.zero_grad(set_to_none=True)
+    xl = x.clone().requires_grad_(True)
+
+    def body(t):
+        return block(block(t * 1.5, *tables) * 0.5, *tables)
+
+    y = wrap(body, xl)
+    junk = [torch.full_like(x, float("nan")) for _ in range(8)]   # takes over memory that was given back
+    y.backward(dy)
+    del junk
+    return [y.detach(), xl.grad] + [p.grad.clone() for p in block.parameters()]
+
+
+@pytest.mark.parametrize("s", [100, 333])
+def test_saved_input_comes_back_as_another_tensor(native_lib, s):
+    """Saved-tensor hooks and an enclosing checkpoint hand the backward a copy, and the original is gone."""
+    from torch.utils.checkpoint import checkpoint
+
+    block, _, tables = _block(512, 4, 4, 512, s, False, False)
+    g = torch.Generator(device=DEV).manual_seed(1)
+    x, dy = (torch.randn(3, s, 512, device=DEV, generator=g).bfloat16() for _ in range(2))
+    want = _over(block, tables, x, dy)
+    assert all(bool(w.isfinite().all()) for w in want)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.clone(), lambda t: t):
+        cloned = _over(block, tables, x, dy)
+    with torch.autograd.graph.save_on_cpu():
+        offloaded = _over(block, tables, x, dy)
+    nested = _over(block, tables, x, dy, lambda f, t: checkpoint(f, t, use_reentrant=False))
+    assert native_lib.read_status() == 0
+    for got in (cloned, offloaded, nested):
+        _same(got, want, s)
+
+
+def test_weights_set_anew_between_the_passes(native_lib):
+    block, _, tables = _block(512, 4, 4, 512, 100, False, False)
+    x, dy = (torch.randn(3, 100, 512, device=DEV).bfloat16() for _ in range(2))
+
+    def run(move):
+        block.zero_grad(set_to_none=True)
+        xl = x.clone().requires_grad_(True)
+        y = block(xl, *tables)
+        if move:   # the same values elsewhere; the old place is given back and overwritten
+            for p in block.parameters():
+                p.data = p.data.clone()
+            junk = [torch.full((512 * 512,), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(16)]
+        y.backward(dy)
+        return [xl.grad] + [p.grad.clone() for p in block.parameters()]
+
+    _same(run(True), run(False), 100)
+
+
 def test_shapes_outside_it(native_lib, monkeypatch):
     from kempnerforge_b200.ops import fused_block
 
