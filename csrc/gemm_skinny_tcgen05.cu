@@ -385,6 +385,11 @@ static int dispatch(const void* x, int ldx, const void* const* w, const int* ldw
   a.x = (const __nv_bfloat16*)x;
   a.ldx = ldx;
   if (a.gain && a.M > NORM_ROWS) return 5;
+  // the bulk copies of the small kernel and the vector loads of the norm need what the encoding of a tensor map checks by itself
+  auto off16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
+  if (off16(x) || off16(a.gain)) return 101;
+  for (int i = 0; i < a.n_seg; ++i)
+    if (off16(w[i])) return 201;
   if (small_fits(a, EPI, small_weight(tiles, (a.K + BK - 1) / BK), num_sms)) return run_small(EPI, w, ldw, a, status, stream);
   if (!a.gain) rc = make_map_2d_bf16(&mx, x, a.M, a.K, ldx, BK, nt);
   if (rc) return 100 + rc;

@@ -62,6 +62,27 @@ def test_few_row_swiglu_epilogue(native_lib, m, f, k):
     assert bool(((got - want).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("m,f,k", [(2, 64, 128), (2, 72, 520), (16, 256, 768), (3, 14336, 1024)])   # small weights, tiles, a large weight
+def test_operands_off_16_bytes_are_refused(native_lib, m, f, k):
+    """The copies into shared memory need 16-byte steps whichever kernel takes the product: an error from the host, no launch."""
+    def off(*shape):   # contiguous, two bytes further
+        return torch.zeros(math.prod(shape) + 1, dtype=torch.bfloat16, device=DEV)[1:].view(shape)
+
+    L, kc = native_lib.lib(), native_lib
+    x, wg, wu, gain = _rand(m, k), _rand(f, k), _rand(f, k), _rand(k)
+    h = torch.full((m, f), 7.0, dtype=torch.bfloat16, device=DEV)
+    for bad in range(3):
+        ops = [off(*t.shape) if i == bad else t for i, t in enumerate((x, wg, wu))]
+        with pytest.raises(native_lib.NativeKernelError):
+            native_lib.swiglu_rows(*ops)
+    if m <= L.kf_skinny_norm_rows():
+        for src, g in ((x, off(k)), (off(m, k), gain)):
+            assert L.kf_gemm_skinny_norm_swiglu_bf16(src.data_ptr(), g.data_ptr(), 1e-5, wg.data_ptr(), wu.data_ptr(), h.data_ptr(), m, f, k,
+                                                     k, k, k, f, 0, kc.sm_count(), kc._stream()) != 0
+    torch.cuda.synchronize()
+    assert native_lib.read_status() == 0 and bool((h == 7).all())
+
+
 def _cache(b, room, hkv, hd, seed):
     """A cache of bounded values followed by NaNs: nothing past the visible positions may be read."""
     return _rand(b, room, hkv, hd, seed=seed), _rand(b, room, hkv, hd, seed=seed + 1)
