@@ -318,7 +318,7 @@ kf_gemm_skinny(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         for (int e = 0; e < 8; ++e) {
           // the projection is rounded to bf16 before the rotation, like the separate kernels do
           const float x = __bfloat162float(__float2bfloat16(lo[e])), y = __bfloat162float(__float2bfloat16(hi[e]));
-          rotate_pair(x, y, cs[e], sn[e], lo[e], hi[e]);
+          rotate_pair_step(a.hd, x, y, cs[e], sn[e], lo[e], hi[e]);
         }
       }
       __nv_bfloat16* p = seg == 0 ? a.out + size_t(t) * a.ldo + row0 + n

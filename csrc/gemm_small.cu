@@ -208,7 +208,7 @@ kf_gemm_small(const __grid_constant__ SmallWeights sw, const __grid_constant__ A
         if (EPI == 1) {
           a.out[size_t(tok) * a.ldo + r_lo + g] = __float2bfloat16(lo / (1.f + __expf(-lo)) * hi);
         } else {
-          if (seg < 2) rotate_pair(lo, hi, cs[nt][e], sn[nt][e], lo, hi);
+          if (seg < 2) rotate_pair_step(a.hd, lo, hi, cs[nt][e], sn[nt][e], lo, hi);
           const int b = tok / a.S, pos = tok - b * a.S;
           __nv_bfloat16* p = seg == 0 ? a.out + size_t(tok) * a.ldo
                                       : (seg == 1 ? a.kc : a.vc) + size_t(b) * a.cache_batch + size_t(pos) * a.kv_cols;

@@ -25,12 +25,19 @@ __device__ __forceinline__ void cluster_sync_all() {
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-
-// (x, y) rotated by the angle of (c, s), spelled out so that the rotary kernel and the epilogues of generation steps give the same
-// bits: left to the compiler, which of the two products is fused with the sum differs between kernels, one bf16 value in 10^5.
+// (x, y) rotated by the angle of (c, s), spelled out because which of two products is fused with their sum decides one bf16 value in
+// 10^5, and the compiler chooses differently from kernel to kernel.  This is the choice of the rotary kernel.
 __device__ __forceinline__ void rotate_pair(float x, float y, float c, float s, float& rx, float& ry) {
   rx = __fmaf_rn(x, c, -__fmul_rn(y, s));
   ry = __fmaf_rn(y, c, __fmul_rn(x, s));
+}
+
+// The same in the epilogue of a generation step.  Heads of 64 keep the bits of the rotary kernel, which rotated them before that
+// epilogue did; heads of 128 keep those that the epilogue has always had, with the other product fused in the second half.
+__device__ __forceinline__ void rotate_pair_step(int hd, float x, float y, float c, float s, float& rx, float& ry) {
+  float other;
+  rotate_pair(x, y, c, s, rx, other);
+  ry = hd == 64 ? other : __fmaf_rn(x, s, __fmul_rn(y, c));
 }
 
 __device__ __forceinline__ float norm_warp_sum(float v) {

@@ -1,4 +1,5 @@
-"""Projections of a generation step that take the norm and the rotation along: bit for bit the separate kernels."""
+"""Projections of a generation step that take the norm and the rotation along: bit for bit the separate kernels, except that the
+rotation of heads of 128 rounds the second half of a pair in another place."""
 
 import pytest
 import torch
@@ -41,7 +42,12 @@ def test_projection_rotation_and_cache(native_lib, b, heads, kv, k, hd):
     cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
     n, _ = kc.rmsnorm_fwd(x, gain, 1e-5)
     qkv = kc.gemm_rows(n, ws).view(b, 1, heads + 2 * kv, hd)
+    x2 = qkv[..., hd // 2 :].clone()
+    x1 = qkv[..., : hd // 2].clone()
     kc.rope(qkv, cos, sin, heads + kv, inverse=False, out=qkv)
+    if hd == 128:   # the second half of a pair: x1 sin in full precision, x2 cos rounded to fp32, their sum rounded once
+        hi = (x1.double() * sin.double() + (x2.double() * cos.double()).float().double()).float().bfloat16()
+        qkv[:, :, : heads + kv, hd // 2 :] = hi[:, :, : heads + kv]
     want = qkv.view(b, -1).split([qc, kvc, kvc], 1)
     for src, g in ((n, None), (x, gain.data_ptr())) if b <= L.kf_skinny_norm_rows() else ((n, None),):
         q = torch.empty(b, qc, dtype=torch.bfloat16, device=DEV)
