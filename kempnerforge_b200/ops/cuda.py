@@ -797,15 +797,16 @@ HEAD64_MAX_SCORES = 1 << 25
 
 
 def attn_bwd_chosen(hd: int, heads: int, sq: int, sk: int, causal: bool, docs: bool) -> bool:
-    """Whether attention with gradients (``heads`` = batch x query heads) runs on the native kernels.  Head dim 128: always.  64:
-    with document ids, which the library does not take; else up to ``HEAD64_MAX_SCORES`` visible scores, and unless the
-    program asked for deterministic algorithms (dQ tiles are added in the order in which they finish).  Measured, forward +
-    backward, us, native / library (12 causal heads): 100 positions 20 / 21, 3 x 333 34 / 30, 2048 101 / 66, 4 x 2048 259 / 151.
-    Around the library's kernels a block also makes three copies and a rotation of q | k | v gradients and issues a second
-    autograd graph from the host (170 us), which decides up to about the limit."""
+    """Whether a fused node runs attention with gradients (``heads`` = batch x query heads) on the native kernels.  Head dim 128:
+    always.  64: not with document ids, whose scores and probabilities the reference formulas hold in fp32; else up to
+    ``HEAD64_MAX_SCORES`` visible scores, and a program that asked for deterministic algorithms keeps the library, which knows of
+    that.  Measured, forward + backward, us, native / library (12 causal heads): 100 positions 20 / 21, 3 x 333 34 / 30, 2048 101 /
+    66, 4 x 2048 259 / 151.  Around the library's kernels a block also makes three copies and a rotation of q | k | v gradients and
+    issues a second autograd graph from the host (170 us), which decides up to about the limit."""
     if hd != 64:
         return hd == 128
-    return docs or (heads * sq * sk // (2 if causal else 1) <= HEAD64_MAX_SCORES and not torch.are_deterministic_algorithms_enabled())
+    return (not docs and heads * sq * sk // (2 if causal else 1) <= HEAD64_MAX_SCORES
+            and not torch.are_deterministic_algorithms_enabled())
 
 
 def doc_blocks(doc_ids: torch.Tensor, like: torch.Tensor | None = None):

@@ -373,7 +373,7 @@ class _QKVAttnFn(torch.autograd.Function):
 
 def qkv_attention(x, wq, wk, wv, cos, sin, doc_ids, hd: int) -> torch.Tensor | None:
     """Causal self-attention of x (B, S, D) up to the output projection -> (B, S, H hd), or None when the fused node does not
-    cover the call (head dim 64 or 128, bf16 on a GPU, gradients wanted, fp32 tables of this sequence, no fp8)."""
+    cover the call (head dim 128, or 64 without documents; bf16 on a GPU, gradients wanted, fp32 tables of this sequence, no fp8)."""
     if (hd not in (64, 128) or not use_native(x) or not torch.is_grad_enabled() or x.dim() != 3 or x.shape[0] * x.shape[1] < 128
             or cos.dtype != torch.float32 or sin.dtype != torch.float32 or cos.dim() != 2 or cos.shape != sin.shape
             or cos.requires_grad or sin.requires_grad or cos.shape[0] < x.shape[1] or cos.shape[1] != hd // 2

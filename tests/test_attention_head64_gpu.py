@@ -1,4 +1,5 @@
-"""Backward attention with heads of 64: edges of the 128-key and 64-query tiles, masks, rotation, both dQ modes."""
+"""Attention with heads of 64 and gradients: edges of the 128-key and 64-query tiles, masks, rotation, both dQ modes, and
+which calls do not take the native kernels."""
 
 import math
 
@@ -79,11 +80,36 @@ def test_what_stays_on_the_library(native_lib):
     q, k, v, _ = _inputs(1, 128, 128, 2, 2, 3)
     assert native_lib.attn_supported(q, k, v, True, needs_grad=True)
     assert native_lib.attn_bwd_chosen(64, 8, 2896, 2896, True, False) and not native_lib.attn_bwd_chosen(64, 8, 2897, 2897, True, False)
-    assert native_lib.attn_bwd_chosen(64, 99, 4096, 4096, True, True) and native_lib.attn_bwd_chosen(128, 99, 4096, 4096, True, False)
+    assert not native_lib.attn_bwd_chosen(64, 1, 128, 128, True, True) and native_lib.attn_bwd_chosen(128, 99, 4096, 4096, True, False)
+    assert not native_lib.attn_supported(q, k, v, True, needs_grad=True, docs=True) and native_lib.attn_supported(q, k, v, True, docs=True)
     assert not native_lib.attn_bwd_chosen(96, 1, 64, 64, True, True)
     torch.use_deterministic_algorithms(True)
     try:
         assert not native_lib.attn_supported(q, k, v, True, needs_grad=True)
-        assert native_lib.attn_supported(q, k, v, True, needs_grad=True, docs=True) and native_lib.attn_supported(q, k, v, True)
+        assert not native_lib.attn_supported(q, k, v, True, needs_grad=True, docs=True) and native_lib.attn_supported(q, k, v, True)
     finally:
         torch.use_deterministic_algorithms(False)
+
+
+def test_documents_with_gradients_stay_in_fp32(native_lib):
+    """Nothing but the result is rounded to bf16: 2^-9 relative per value."""
+    from kempnerforge_b200.models.attention import Attention
+    from kempnerforge_b200.ops import functional as F
+    from kempnerforge_b200.ops import ref
+
+    b, s, h, hkv = 2, 300, 4, 2
+    q, k, v, dout = _inputs(b, s, s, h, hkv, 7)
+    doc = (torch.arange(s, device=DEV) // 90).expand(b, s).contiguous()
+    ql, kl, vl = (t.clone().requires_grad_(True) for t in (q, k, v))
+    out = F.attention(ql, kl, vl, doc_ids=doc)
+    got = torch.autograd.grad(out, (ql, kl, vl), dout)
+    want64 = ref.attention(q.double(), k.double(), v.double(), doc_ids=doc)
+    for a, w in zip((out.detach(), *got), (want64, *_grads64(q, k, v, dout, True, doc))):
+        assert float((a.double() - w).norm()) <= 2.0**-9 * float(w.norm())
+    # the layer takes the same way
+    torch.manual_seed(0)
+    att = Attention(h * HD, h, hkv).to(DEV, torch.bfloat16)
+    x = torch.randn(b, s, h * HD, device=DEV).bfloat16().requires_grad_(True)
+    tables = [t.cos() if i == 0 else t.sin() for i, t in enumerate([torch.rand(s, HD // 2, device=DEV) * 6] * 2)]
+    w = [att.q_proj.weight, att.k_proj.weight, att.v_proj.weight]
+    assert F.qkv_attention(x, *w, *tables, doc, HD) is None and F.qkv_attention(x, *w, *tables, None, HD) is not None
