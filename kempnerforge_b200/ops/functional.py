@@ -320,6 +320,9 @@ def attention(
         needs_grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
         policy = cu.attn_policy()
         want = policy == "native" or (policy == "auto" and (not needs_grad or doc_ids is not None))
+        # Heads of 64 with gradients are native in the fused nodes only.  Called by itself, this is the library's attention with
+        # all that it supports (functorch transforms, the program's choice of its kernels) or the fp32 formulas.
+        want = want and not (needs_grad and hd == 64)
         if want and (doc_ids is None or q.shape[1] == k.shape[1]) and cu.attn_supported(q, k, v, causal, needs_grad, doc_ids is not None):
             if not needs_grad:
                 return cu.attn_fwd(q, k, v, causal, doc_ids, scale)[0]

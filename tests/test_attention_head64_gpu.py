@@ -113,3 +113,20 @@ def test_documents_with_gradients_stay_in_fp32(native_lib):
     tables = [t.cos() if i == 0 else t.sin() for i, t in enumerate([torch.rand(s, HD // 2, device=DEV) * 6] * 2)]
     w = [att.q_proj.weight, att.k_proj.weight, att.v_proj.weight]
     assert F.qkv_attention(x, *w, *tables, doc, HD) is None and F.qkv_attention(x, *w, *tables, None, HD) is not None
+
+
+def test_called_by_itself_it_transforms(native_lib):
+    from kempnerforge_b200.ops import functional as F
+
+    q, k, v, dout = _inputs(2, 150, 150, 2, 2, 9)
+
+    def loss(q, k, v, d):
+        return (F.attention(q, k, v) * d).float().sum()
+
+    got = torch.func.grad(loss, argnums=(0, 1, 2))(q, k, v, dout)
+    ql, kl, vl = (t.clone().requires_grad_(True) for t in (q, k, v))
+    want = torch.autograd.grad(loss(ql, kl, vl, dout), (ql, kl, vl))
+    assert all(torch.equal(a, w) for a, w in zip(got, want))
+    with torch.nn.attention.sdpa_kernel(torch.nn.attention.SDPBackend.MATH):   # the program's choice of kernel holds
+        (first,) = torch.autograd.grad(loss(ql, kl, vl, dout), ql, create_graph=True)
+        assert first.requires_grad
