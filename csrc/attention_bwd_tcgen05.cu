@@ -24,8 +24,12 @@
 //   warps 6-9  : dQ reduction (TMEM -> shared-memory tile -> one cp.reduce.async.bulk.tensor add per tile;
 //                or, as a fallback mode, red.global.add.f32 per element)
 //
-// Head dim 64 has half the products per score and the same softmax, so it is bound by the softmax warps: 100 positions of 12
-// heads 15 us, 3 x 333 23 us, 2048 65 us (the library's backward 16, 19 and 40, before the copies around it).
+// Head dim 64 adds nothing up in memory: each key tile writes its dQ tiles to a part of its own, and the post-pass adds the parts in
+// the order of the key tiles, so equal inputs give equal bits (the library's backward, which such models had before, repeats itself
+// at their usual lengths).  It has half the products per score and the same softmax, so it is bound by the softmax warps.  Backward
+// with its pre- and post-pass, 12 causal heads, us, parts / one accumulator that all tiles add to: 100 positions 16.4 / 17.3, 3 x 333
+// 26 / 27, 1024 43 / 43, 2048 74 / 70, 2 x 1600 87 / 78.  (The library's backward for 100, 3 x 333 and 2048: 16, 19 and 40, before
+// the copies around it.)
 //
 // D_i = rowsum(dO_i * O_i) comes from a small pre-pass; a post-pass converts the fp32 dQ to bf16.
 // Replaces the backward of F.scaled_dot_product_attention (kempnerforge/model/attention.py:227-231) for the
@@ -83,6 +87,10 @@ __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, uint32
   asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map),
                "r"(x), "r"(y), "r"(smem_src)
                : "memory");
+}
+// contiguous bytes, both ends on 16 bytes
+__device__ __forceinline__ void bulk_store(float* dst, uint32_t smem_src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
@@ -487,11 +495,11 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(dq_free);  // the values are in registers: the next dQ^T may be computed
-      if (dq_tma) {
-        // transpose through shared memory into the [query][head dim] tile the tensor map describes, then one
-        // bulk reduction adds the whole tile; rows past the end of the tensor are clipped by the TMA unit, rows
-        // of padding queries hold exact zeros
-        if (elected) bulk_wait_read_all();  // the previous reduction has read the staging tile
+      if (HD == 64 || dq_tma) {
+        // transpose through shared memory into a [query][head dim] tile.  Head dim 128: the tile that the tensor map describes, added
+        // by one bulk reduction; rows past the end of the tensor are clipped by the TMA unit, rows of padding queries hold exact
+        // zeros.  64: 16 KB in this key tile's own part, which has rows for padding queries
+        if (elected) bulk_wait_read_all();  // the previous copy has read the staging tile
         group_sync(2, 128);
 #pragma unroll
         for (int c = 0; c < BLK_Q; ++c)
@@ -500,17 +508,21 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         fence_async_smem();
         group_sync(2, 128);
         if (elected && ok) {
-          tma_reduce_add_2d(&map_dq, dq_stage, hq * HD, b * Sq + q0);
+          if constexpr (HD == 64)
+            bulk_store(dQacc + (((size_t(kt) * (gridDim.x / Hkv_) + b) * H + hq) * n_q_tiles + wk.i) * (BLK_Q * HD), dq_stage,
+                       BLK_Q * HD * 4);
+          else
+            tma_reduce_add_2d(&map_dq, dq_stage, hq * HD, b * Sq + q0);
           bulk_commit();
         }
-      } else if (ok && (HD == 128 || d < HD)) {
+      } else if (ok) {
         float* base = dQacc + ((size_t(b) * Sq + q0) * H + hq) * HD + d;
 #pragma unroll
         for (int c = 0; c < BLK_Q; ++c)
           if (q0 + c < Sq) red_add_f32(base + size_t(c) * H * HD, __uint_as_float(v[c]));
       }
     }
-    if (dq_tma && elected) bulk_wait_all();
+    if ((HD == 64 || dq_tma) && elected) bulk_wait_all();
   }
 
   tc_fence_before();
@@ -577,12 +589,11 @@ __global__ void kf_f32_to_bf16_rows(const float* __restrict__ src, __nv_bfloat16
   }
 }
 
-// scale * fp32 dQ [rows][H * HD] -> bf16 rows with pitch ld, through the inverse rotary embedding of position (row % S)
-template <int HD>
+// scale * fp32 dQ [rows][H * 128] -> bf16 rows with pitch ld, through the inverse rotary embedding of position (row % S)
 __global__ void kf_dq_finish_rope(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long rows, int H,
                                   long long ld, const float* __restrict__ cosT, const float* __restrict__ sinT, int S,
                                   float scale) {
-  constexpr int HALF = HD / 2;
+  constexpr int HD = 128, HALF = HD / 2;
   const long long n4 = rows * H * (HALF / 4);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
     const int j = (i % (HALF / 4)) * 4;
@@ -603,6 +614,41 @@ __global__ void kf_dq_finish_rope(const float* __restrict__ src, __nv_bfloat16* 
     hi.y = pack_bf16(b.z * c.z - a.z * s.z, b.w * c.w - a.w * s.w);
     *reinterpret_cast<uint2*>(dst + r * ld + h * HD + j) = lo;
     *reinterpret_cast<uint2*>(dst + r * ld + h * HD + HALF + j) = hi;
+  }
+}
+
+// Head dim 64: scale * the sum of the parts [key tile][b][head][query tile][64 queries][64] -> bf16 rows with pitch ld, in the order of
+// the key tiles; with cosT through the inverse rotary embedding.  causal: a query's keys end with its own tile.
+__global__ void kf_dq_add_parts(const float* __restrict__ parts, __nv_bfloat16* __restrict__ dst, int B, int S, int H, int key_tiles,
+                                int causal, long long ld, const float* __restrict__ cosT, const float* __restrict__ sinT, float scale) {
+  constexpr int HD = 64, HALF = HD / 2;
+  const int n_q_tiles = (S + BLK_Q - 1) / BLK_Q;
+  const size_t part = size_t(B) * H * n_q_tiles * (BLK_Q * HD);
+  const long long n4 = (long long)B * S * H * (HALF / 4);
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
+    const int j = (i % (HALF / 4)) * 4;
+    const long long rh = i / (HALF / 4), r = rh / H;
+    const int h = rh % H, pos = r % S, b = r / S;
+    const float* src = parts + ((size_t(b) * H + h) * n_q_tiles * BLK_Q + pos) * HD + j;
+    const int n = causal ? min(key_tiles, pos / BLK_K + 1) : key_tiles;
+    float4 a = *reinterpret_cast<const float4*>(src), c = *reinterpret_cast<const float4*>(src + HALF);
+#pragma unroll 4
+    for (int t = 1; t < n; ++t) {
+      const float4 u = *reinterpret_cast<const float4*>(src + t * part), v = *reinterpret_cast<const float4*>(src + t * part + HALF);
+      a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
+      c.x += v.x; c.y += v.y; c.z += v.z; c.w += v.w;
+    }
+    const float lo[4] = {a.x * scale, a.y * scale, a.z * scale, a.w * scale}, hi[4] = {c.x * scale, c.y * scale, c.z * scale, c.w * scale};
+    float x[4], y[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float cs = cosT ? cosT[size_t(pos) * HALF + j + e] : 1.f, sn = cosT ? sinT[size_t(pos) * HALF + j + e] : 0.f;
+      x[e] = cosT ? lo[e] * cs + hi[e] * sn : lo[e];
+      y[e] = cosT ? hi[e] * cs - lo[e] * sn : hi[e];
+    }
+    __nv_bfloat16* out = dst + r * ld + h * HD + j;
+    *reinterpret_cast<uint2*>(out) = make_uint2(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]));
+    *reinterpret_cast<uint2*>(out + HALF) = make_uint2(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]));
   }
 }
 
@@ -651,12 +697,13 @@ static int run(const void* q, const void* k, const void* v, const void* o, const
   if (rc) return 250 + rc;
   rc = make_map_2d_bf16(&mdo, d_o, uint64_t(B) * Sq, uint64_t(H) * hd, lddo, 64, BLK_Q);
   if (rc) return 270 + rc;
-  const int dq_tma = g_dq_mode;
-  CUtensorMap mdq;
-  rc = make_map_2d_f32_plain(&mdq, dq_acc, uint64_t(B) * Sq, uint64_t(H) * hd, HD, BLK_Q);
+  const int dq_tma = HD == 128 ? g_dq_mode : 1;
+  CUtensorMap mdq = mq;
+  if (HD == 128) rc = make_map_2d_f32_plain(&mdq, dq_acc, uint64_t(B) * Sq, uint64_t(H) * hd, HD, BLK_Q);
   if (rc) return 280 + rc;
   const size_t smem_bytes = dq_tma ? C::SMEM_DQ_TMA : C::SMEM;
-  // pre-pass: D = rowsum(dO * O); zero the fp32 dQ accumulator
+  const int key_tiles = (Sk + BLK_K - 1) / BLK_K, q_tiles = (Sq + BLK_Q - 1) / BLK_Q;
+  // pre-pass: D = rowsum(dO * O); zero the fp32 dQ accumulator (the parts of head dim 64 where documents leave tiles out)
   {
     const long long rows = (long long)B * Sq * H;
     const int threads = 256;
@@ -665,11 +712,13 @@ static int run(const void* q, const void* k, const void* v, const void* o, const
     kf_attn_bwd_dot<HD><<<(unsigned)blocks, threads, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(o),
                                                              reinterpret_cast<const __nv_bfloat16*>(d_o),
                                                              reinterpret_cast<float*>(dsum), B, Sq, H, ldo, lddo);
-    cudaError_t e = cudaMemsetAsync(dq_acc, 0, size_t(B) * Sq * H * hd * sizeof(float), st);
+    cudaError_t e = cudaSuccess;
+    if (HD == 128) e = cudaMemsetAsync(dq_acc, 0, size_t(B) * Sq * H * hd * sizeof(float), st);
+    else if (doc) e = cudaMemsetAsync(dq_acc, 0, size_t(key_tiles) * B * H * q_tiles * BLK_Q * hd * sizeof(float), st);
     if (e != cudaSuccess) return 400 + (int)e;
   }
   int* status = reinterpret_cast<int*>(kf_status_device_ptr());
-  dim3 grid(Hkv * B, (Sk + BLK_K - 1) / BLK_K);
+  dim3 grid(Hkv * B, key_tiles);
 #define KF_BWD_LAUNCH(C_, D_)                                                                                      \
   {                                                                                                                \
     auto kern = kf_attn_bwd_tcgen05<HD, C_, D_>;                                                                       \
@@ -696,8 +745,12 @@ static int run(const void* q, const void* k, const void* v, const void* o, const
   {
     const long long rows = (long long)B * Sq;
     const int cols = H * hd;
-    if (cosT)
-      kf_dq_finish_rope<HD><<<1184, 256, 0, st>>>(reinterpret_cast<const float*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dq),
+    if (HD == 64)
+      kf_dq_add_parts<<<1184, 256, 0, st>>>(reinterpret_cast<const float*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dq), B, Sq, H, key_tiles,
+                                            causal, lddq, reinterpret_cast<const float*>(cosT), reinterpret_cast<const float*>(sinT),
+                                            scale);
+    else if (cosT)
+      kf_dq_finish_rope<<<1184, 256, 0, st>>>(reinterpret_cast<const float*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dq),
                                               rows, H, lddq, reinterpret_cast<const float*>(cosT),
                                               reinterpret_cast<const float*>(sinT), Sq, scale);
     else
@@ -713,7 +766,7 @@ static int run(const void* q, const void* k, const void* v, const void* o, const
 
 extern "C" {
 
-// How the backward kernel adds its dQ tiles to the fp32 accumulator: 0 = red.global per element,
+// How the backward kernel adds its dQ tiles to the fp32 accumulator (head dim 128): 0 = red.global per element,
 // 1 = one bulk tensor reduction per tile (default).  Returns the previous mode.
 int kf_attn_bwd_dq_mode(int mode) {
   const int prev = kf::attnb::g_dq_mode;
@@ -722,8 +775,8 @@ int kf_attn_bwd_dq_mode(int mode) {
 }
 
 // Backward attention (head dim 64 or 128).  q / k / v / o / do: rows (b * S + s) with pitches ld*, heads side by
-// side; lse: fp32 [B][H][Sq] from the forward; dsum: fp32 scratch [B][H][Sq]; dq_acc: fp32 scratch
-// [B][Sq][H][hd] (zeroed here); dq / dk / dv: bf16 outputs with pitches lddq / lddk / lddv (they may be
+// side; lse: fp32 [B][H][Sq] from the forward; dsum: fp32 scratch [B][H][Sq]; dq_acc: fp32 scratch, [B][Sq][H][128] (zeroed
+// here) or, for head dim 64, [ceil(Sk / 128)][B][H][ceil(Sq / 64) * 64][64]; dq / dk / dv: bf16 outputs with pitches lddq / lddk / lddv (they may be
 // slices of one fused gradient buffer).  doc: optional int32 [B][S].  Requires Sq == Sk when causal or doc.
 // kf_attn_bwd_rope_bf16: the same, and dq / dk additionally pass through the inverse rotary embedding (cosT / sinT:
 // fp32 [Sq][hd / 2], position = index inside the sequence), i.e. they are gradients with respect to the un-rotated

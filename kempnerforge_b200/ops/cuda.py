@@ -794,19 +794,20 @@ def attn_supported(q, k, v, causal: bool, needs_grad: bool = False, docs: bool =
 
 
 HEAD64_MAX_SCORES = 1 << 25
+HEAD64_MAX_PARTS = 9 << 22   # 151 MB of dQ parts: what HEAD64_MAX_SCORES causal scores need, with a margin for whole tiles
 
 
 def attn_bwd_chosen(hd: int, heads: int, sq: int, sk: int, causal: bool, docs: bool) -> bool:
     """Whether a fused node runs attention with gradients (``heads`` = batch x query heads) on the native kernels.  Head dim 128:
     always.  64: not with document ids, whose scores and probabilities the reference formulas hold in fp32; else up to
-    ``HEAD64_MAX_SCORES`` visible scores, and a program that asked for deterministic algorithms keeps the library, which knows of
+    ``HEAD64_MAX_SCORES`` visible scores (many sequences shorter than a tile: ``HEAD64_MAX_PARTS`` of scratch), and a program that asked for deterministic algorithms keeps the library, which knows of
     that.  Measured, forward + backward, us, native / library (12 causal heads): 100 positions 20 / 21, 3 x 333 34 / 30, 2048 101 /
     66, 4 x 2048 259 / 151.  Around the library's kernels a block also makes three copies and a rotation of q | k | v gradients and
     issues a second autograd graph from the host (170 us), which decides up to about the limit."""
     if hd != 64:
         return hd == 128
     return (not docs and heads * sq * sk // (2 if causal else 1) <= HEAD64_MAX_SCORES
-            and not torch.are_deterministic_algorithms_enabled())
+            and attn_bwd_dq_floats(1, sq, sk, heads, hd) <= HEAD64_MAX_PARTS and not torch.are_deterministic_algorithms_enabled())
 
 
 def doc_blocks(doc_ids: torch.Tensor, like: torch.Tensor | None = None):
@@ -1147,6 +1148,11 @@ def gemm_rope_supported(x2: torch.Tensor, w: torch.Tensor, hd: int) -> bool:
             and x2.dtype == torch.bfloat16 and x2.stride(0) % 8 == 0 and w.stride(0) % 8 == 0)
 
 
+def attn_bwd_dq_floats(b: int, sq: int, sk: int, h: int, hd: int) -> int:
+    """fp32 values of dQ scratch: one accumulator, or for head dim 64 a part per tile of 128 keys."""
+    return b * sq * h * hd if hd != 64 else -(-sk // 128) * b * h * (-(-sq // 64) * 64) * 64
+
+
 def attn_bwd(dout, q, k, v, out, lse, causal: bool, doc_ids, scale: float, dq=None, dk=None, dv=None, rope=None):
     """Gradients of ``attn_fwd``.  ``dq`` / ``dk`` / ``dv`` may be preallocated (strided) destinations, e.g. the
     three head ranges of one fused projection gradient; otherwise contiguous tensors are returned.
@@ -1162,7 +1168,7 @@ def attn_bwd(dout, q, k, v, out, lse, causal: bool, doc_ids, scale: float, dq=No
     for t in (dq, dk, dv, out, dout):
         assert _attn_rows_ok(t), "attention gradients need evenly pitched rows with adjacent heads"
     dsum = torch.empty((b, h, sq), dtype=torch.float32, device=q.device)
-    dq_acc = torch.empty((b, sq, h, hd), dtype=torch.float32, device=q.device)
+    dq_acc = torch.empty(attn_bwd_dq_floats(b, sq, sk, h, hd), dtype=torch.float32, device=q.device)
     doc = rng = None
     if doc_ids is not None:
         doc, rng = doc_ids if isinstance(doc_ids, tuple) else doc_blocks(doc_ids, k)

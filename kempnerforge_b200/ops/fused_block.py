@@ -241,7 +241,7 @@ def _chain_backward(it: _ChainState, dy2, x2, cos, sin, weights):
     L = kc.lib()
     # dh1, dattn, dqkv, dq_acc, dsum, partial
     at = [0]
-    for n in (2 * t * d, 2 * t * qc, 2 * t * nq, 4 * t * qc, 4 * t * h, 4 * L.kf_rmsnorm_bwd_blocks(t) * d):
+    for n in (2 * t * d, 2 * t * qc, 2 * t * nq, 4 * kc.attn_bwd_dq_floats(b, s, s, h, hd), 4 * t * h, 4 * L.kf_rmsnorm_bwd_blocks(t) * d):
         at.append(at[-1] + (n + 255) // 256 * 256)
     scratch = torch.empty(at[-1], dtype=torch.uint8, device=dev)
     base = scratch.data_ptr()

@@ -1,4 +1,4 @@
-"""Attention with heads of 64 and gradients: edges of the 128-key and 64-query tiles, masks, rotation, both dQ modes, and
+"""Attention with heads of 64 and gradients: edges of the 128-key and 64-query tiles, masks, rotation, fixed order of the sums, and
 which calls do not take the native kernels."""
 
 import math
@@ -89,6 +89,29 @@ def test_what_stays_on_the_library(native_lib):
         assert not native_lib.attn_supported(q, k, v, True, needs_grad=True, docs=True) and native_lib.attn_supported(q, k, v, True)
     finally:
         torch.use_deterministic_algorithms(False)
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("b,s,h,hkv", [(3, 333, 12, 12), (2, 1025, 8, 2), (1, 2048, 12, 12)])
+def test_equal_inputs_give_equal_bits(native_lib, b, s, h, hkv, causal):
+    q, k, v, dout = _inputs(b, s, s, h, hkv, 2)
+    out, lse = native_lib.attn_fwd(q, k, v, causal, None, HD**-0.5)
+    first = native_lib.attn_bwd(dout, q, k, v, out, lse, causal, None, HD**-0.5)
+    for _ in range(10):
+        again = native_lib.attn_bwd(dout, q, k, v, out, lse, causal, None, HD**-0.5)
+        assert all(torch.equal(x, y) for x, y in zip(first, again))
+    assert native_lib.read_status() == 0
+
+
+def test_parts_of_the_longest_call_fit(native_lib):
+    n = native_lib.attn_bwd_dq_floats
+    assert n(3, 333, 333, 12, 128) == 3 * 333 * 12 * 128
+    assert n(3, 333, 333, 12, 64) == 3 * 3 * 12 * 384 * 64
+    for causal, s in ((True, 2896), (False, 2048)):
+        assert s * s * 8 // (1 + causal) <= native_lib.HEAD64_MAX_SCORES < (s + 1) ** 2 * 8 // (1 + causal)
+        assert n(1, s, s, 8, 64) <= native_lib.HEAD64_MAX_PARTS
+    # sequences much shorter than a tile: the tiles, not the scores, are what a call costs
+    assert native_lib.attn_bwd_chosen(64, 12 * 768, 8, 8, True, False) and not native_lib.attn_bwd_chosen(64, 12 * 769, 8, 8, True, False)
 
 
 def test_documents_with_gradients_stay_in_fp32(native_lib):
