@@ -83,9 +83,9 @@ __device__ __forceinline__ void red_add_f32(float* addr, float v) {
 }
 
 // fp32 tile in shared memory (row-major, the tensor map's box) added to global memory by the TMA unit
-__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, uint32_t smem_src, int x, int y) {
-  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map),
-               "r"(x), "r"(y), "r"(smem_src)
+__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, uint32_t smem_src, int x, int y, int z) {
+  asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(map),
+               "r"(x), "r"(y), "r"(z), "r"(smem_src)
                : "memory");
 }
 // contiguous bytes, both ends on 16 bytes
@@ -205,8 +205,8 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       mbar_expect_tx(kv_full, 2 * KV_TILE_BYTES);
 #pragma unroll
       for (int c = 0; c < BLOCKS; ++c) {
-        tma_load_2d(k_smem + c * KV_BLOCK_BYTES, &map_k, kv_full, hk * HD + 64 * c, b * Sk + k0);
-        tma_load_2d(v_smem + c * KV_BLOCK_BYTES, &map_v, kv_full, hk * HD + 64 * c, b * Sk + k0);
+        tma_load_3d(k_smem + c * KV_BLOCK_BYTES, &map_k, kv_full, hk * HD + 64 * c, k0, b);
+        tma_load_3d(v_smem + c * KV_BLOCK_BYTES, &map_v, kv_full, hk * HD + 64 * c, k0, b);
       }
       Walk wk = walk_begin();
       for (int it = 0; it < n_iter; ++it, wk = walk_next(wk)) {
@@ -218,10 +218,10 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         mbar_expect_tx(qdo_full(st), 2 * Q_TILE_BYTES);
 #pragma unroll
         for (int c = 0; c < BLOCKS; ++c) {
-          tma_load_2d(q_smem + st * Q_TILE_BYTES + c * Q_BLOCK_BYTES, &map_q, qdo_full(st), hq * HD + 64 * c,
-                      b * Sq + q0);
-          tma_load_2d(do_smem + st * Q_TILE_BYTES + c * Q_BLOCK_BYTES, &map_do, qdo_full(st), hq * HD + 64 * c,
-                      b * Sq + q0);
+          tma_load_3d(q_smem + st * Q_TILE_BYTES + c * Q_BLOCK_BYTES, &map_q, qdo_full(st), hq * HD + 64 * c,
+                      q0, b);
+          tma_load_3d(do_smem + st * Q_TILE_BYTES + c * Q_BLOCK_BYTES, &map_do, qdo_full(st), hq * HD + 64 * c,
+                      q0, b);
         }
         ++issued;
       }
@@ -497,8 +497,8 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       if (lane == 0) mbar_arrive(dq_free);  // the values are in registers: the next dQ^T may be computed
       if (HD == 64 || dq_tma) {
         // transpose through shared memory into a [query][head dim] tile.  Head dim 128: the tile that the tensor map describes, added
-        // by one bulk reduction; rows past the end of the tensor are clipped by the TMA unit, rows of padding queries hold exact
-        // zeros.  64: 16 KB in this key tile's own part, which has rows for padding queries
+        // by one bulk reduction, which leaves out the rows past the end of the sequence.  64: 16 KB in this key tile's own part,
+        // which has rows for padding queries
         if (elected) bulk_wait_read_all();  // the previous copy has read the staging tile
         group_sync(2, 128);
 #pragma unroll
@@ -512,7 +512,7 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             bulk_store(dQacc + (((size_t(kt) * (gridDim.x / Hkv_) + b) * H + hq) * n_q_tiles + wk.i) * (BLK_Q * HD), dq_stage,
                        BLK_Q * HD * 4);
           else
-            tma_reduce_add_2d(&map_dq, dq_stage, hq * HD, b * Sq + q0);
+            tma_reduce_add_3d(&map_dq, dq_stage, hq * HD, q0, b);
           bulk_commit();
         }
       } else if (ok) {
@@ -661,16 +661,16 @@ namespace kf {
 namespace attnb {
 static int g_dq_mode = 1;  // 0: red.global per element, 1: bulk tensor reduction from shared memory (1.75x faster)
 
-// fp32 [rows][cols] row-major -> tensor map with an unswizzled (box_cols x box_rows) box
-inline int make_map_2d_f32_plain(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_cols,
-                                 uint32_t box_rows) {
+// fp32 [planes][rows][cols] without gaps -> tensor map with an unswizzled (box_cols x box_rows x 1) box
+inline int make_map_3d_f32_plain(CUtensorMap* map, const void* base, uint64_t planes, uint64_t rows, uint64_t cols,
+                                 uint32_t box_cols, uint32_t box_rows) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return -1;
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {cols * 4};
-  cuuint32_t box[2] = {box_cols, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr,
+  cuuint64_t dims[3] = {cols, rows, planes};
+  cuuint64_t strides[2] = {cols * 4, rows * cols * 4};
+  cuuint32_t box[3] = {box_cols, box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : (int)r;
@@ -689,17 +689,17 @@ static int run(const void* q, const void* k, const void* v, const void* o, const
   using C = Cfg<HD>;
   constexpr int hd = HD;
   CUtensorMap mq, mk, mv, mdo;
-  int rc = make_map_2d_bf16(&mq, q, uint64_t(B) * Sq, uint64_t(H) * hd, ldq, 64, BLK_Q);
+  int rc = make_map_3d_bf16(&mq, q, B, Sq, uint64_t(H) * hd, 64, BLK_Q, ldq);
   if (rc) return 100 + rc;
-  rc = make_map_2d_bf16(&mk, k, uint64_t(B) * Sk, uint64_t(Hkv) * hd, ldk, 64, BLK_K);
+  rc = make_map_3d_bf16(&mk, k, B, Sk, uint64_t(Hkv) * hd, 64, BLK_K, ldk);
   if (rc) return 200 + rc;
-  rc = make_map_2d_bf16(&mv, v, uint64_t(B) * Sk, uint64_t(Hkv) * hd, ldv, 64, BLK_K);
+  rc = make_map_3d_bf16(&mv, v, B, Sk, uint64_t(Hkv) * hd, 64, BLK_K, ldv);
   if (rc) return 250 + rc;
-  rc = make_map_2d_bf16(&mdo, d_o, uint64_t(B) * Sq, uint64_t(H) * hd, lddo, 64, BLK_Q);
+  rc = make_map_3d_bf16(&mdo, d_o, B, Sq, uint64_t(H) * hd, 64, BLK_Q, lddo);
   if (rc) return 270 + rc;
   const int dq_tma = HD == 128 ? g_dq_mode : 1;
   CUtensorMap mdq = mq;
-  if (HD == 128) rc = make_map_2d_f32_plain(&mdq, dq_acc, uint64_t(B) * Sq, uint64_t(H) * hd, HD, BLK_Q);
+  if (HD == 128) rc = make_map_3d_f32_plain(&mdq, dq_acc, B, Sq, uint64_t(H) * hd, HD, BLK_Q);
   if (rc) return 280 + rc;
   const size_t smem_bytes = dq_tma ? C::SMEM_DQ_TMA : C::SMEM;
   const int key_tiles = (Sk + BLK_K - 1) / BLK_K, q_tiles = (Sq + BLK_Q - 1) / BLK_Q;

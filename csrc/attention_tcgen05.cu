@@ -132,8 +132,8 @@ kf_attn_fwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         mbar_expect_tx(k_full(st), C::TILE_BYTES);
 #pragma unroll
         for (int c = 0; c < C::BLOCKS; ++c)
-          tma_load_2d(k_smem + st * C::TILE_BYTES + c * C::BLOCK_BYTES, &map_k, k_full(st), hk * HD + 64 * c,
-                      b * Sk + j * BLK_N);
+          tma_load_3d(k_smem + st * C::TILE_BYTES + c * C::BLOCK_BYTES, &map_k, k_full(st), hk * HD + 64 * c,
+                      j * BLK_N, b);
       };
       const int pre = old_tiles(K_STAGES);
       for (; issued < pre; ++issued) load_k(issued);
@@ -141,7 +141,7 @@ kf_attn_fwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       mbar_expect_tx(q_full, C::TILE_BYTES);
 #pragma unroll
       for (int c = 0; c < C::BLOCKS; ++c)
-        tma_load_2d(q_smem + c * C::BLOCK_BYTES, &map_q, q_full, h * HD + 64 * c, b * Sq + m0);
+        tma_load_3d(q_smem + c * C::BLOCK_BYTES, &map_q, q_full, h * HD + 64 * c, m0, b);
       for (int j = pre; j < n_tiles; ++j) {
         const int st = j % K_STAGES;
         const int use = j / K_STAGES;  // how many times this stage has been filled before
@@ -163,8 +163,8 @@ kf_attn_fwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         mbar_expect_tx(v_full(st), C::TILE_BYTES);
 #pragma unroll
         for (int c = 0; c < C::BLOCKS; ++c)
-          tma_load_2d(v_smem + st * C::TILE_BYTES + c * C::BLOCK_BYTES, &map_v, v_full(st), hk * HD + 64 * c,
-                      b * Sk + j * BLK_N);
+          tma_load_3d(v_smem + st * C::TILE_BYTES + c * C::BLOCK_BYTES, &map_v, v_full(st), hk * HD + 64 * c,
+                      j * BLK_N, b);
       };
       const int pre = old_tiles(V_STAGES);
       for (; issued < pre; ++issued) load_v(issued);
@@ -472,11 +472,11 @@ int kf_attn_fwd_pdl_bf16(const void* q, const void* k, const void* v, void* o, v
   if ((causal || doc) && Sq != Sk) return 4;
   if ((ldq | ldk | ldv | ldo) & 7) return 5;
   CUtensorMap mq, mk, mv;
-  int rc = make_map_2d_bf16(&mq, q, uint64_t(B) * Sq, uint64_t(H) * hd, ldq, 64, BLK_M);
+  int rc = make_map_3d_bf16(&mq, q, B, Sq, uint64_t(H) * hd, 64, BLK_M, ldq);
   if (rc) return 100 + rc;
-  rc = make_map_2d_bf16(&mk, k, uint64_t(B) * Sk, uint64_t(Hkv) * hd, ldk, 64, BLK_N);
+  rc = make_map_3d_bf16(&mk, k, B, Sk, uint64_t(Hkv) * hd, 64, BLK_N, ldk);
   if (rc) return 200 + rc;
-  rc = make_map_2d_bf16(&mv, v, uint64_t(B) * Sk, uint64_t(Hkv) * hd, ldv, 64, BLK_N);
+  rc = make_map_3d_bf16(&mv, v, B, Sk, uint64_t(Hkv) * hd, 64, BLK_N, ldv);
   if (rc) return 250 + rc;
   int* status = reinterpret_cast<int*>(kf_status_device_ptr());
   cudaStream_t st = (cudaStream_t)stream;

@@ -326,13 +326,14 @@ inline int make_map_2d_bf16(CUtensorMap* map, const void* base, uint64_t rows, u
   return r == CUDA_SUCCESS ? 0 : (int)r;
 }
 
-// Contiguous bf16 [planes][rows][cols] -> tensor map with a (box_cols x box_rows x 1) box and 128-byte swizzle.
+// bf16 [planes][rows][cols] -> tensor map with a (box_cols x box_rows x 1) box and 128-byte swizzle.  Rows lie `ld` elements apart,
+// planes follow one another.  A box that reaches over the end of a plane is filled with zeros.
 inline int make_map_3d_bf16(CUtensorMap* map, const void* base, uint64_t planes, uint64_t rows, uint64_t cols,
-                            uint32_t box_cols, uint32_t box_rows) {
+                            uint32_t box_cols, uint32_t box_rows, uint64_t ld) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return -1;
   cuuint64_t dims[3] = {cols, rows, planes};
-  cuuint64_t strides[2] = {cols * 2, rows * cols * 2};
+  cuuint64_t strides[2] = {ld * 2, rows * ld * 2};
   cuuint32_t box[3] = {box_cols, box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,

@@ -285,7 +285,7 @@ int launch_grouped_wgrad_2cta(const void* A, const void* B, void* Out, const voi
   rc = make_map_2d_bf16(&mb, B, rows, N, ldb, 64, BK);
   if (rc) return 200 + rc;
   CUtensorMap mo;
-  rc = make_map_3d_bf16(&mo, Out, E, M, N, 64, 32);
+  rc = make_map_3d_bf16(&mo, Out, E, M, N, 64, 32, N);
   if (rc) return 300 + rc;
   const long long tiles = (long long)E * ((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N);
   int pairs = num_sms / 2;
