@@ -88,7 +88,7 @@ class TransformerBlock(nn.Module):
             if x.is_cuda and not _FUSED_BLOCK_OFF and F.use_native(x):
                 from kempnerforge_b200.ops import fused_block
 
-                if fused_block.attn_half_supported(self, x, kv_cache, doc_ids, key_padding_mask):
+                if fused_block.attn_half_supported(self, x, kv_cache, doc_ids, key_padding_mask, cos, sin):
                     # blocks the whole-block node does not cover (mixture-of-experts layers): the attention
                     # sub-layer as one node, residual included
                     x = fused_block.attn_half(self, x, cos, sin)

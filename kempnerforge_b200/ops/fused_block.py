@@ -34,7 +34,9 @@ import os
 from array import array
 
 import torch
+from torch.nn.modules import module as _nn_module
 
+from kempnerforge_b200.models.attention import Attention
 from kempnerforge_b200.ops import cuda as kc
 from kempnerforge_b200.ops.fused_infer import _matrix
 
@@ -512,10 +514,19 @@ class AttnHalfFn(torch.autograd.Function):
         return dx.view(b, s, d), None, None, g_wn1, g_wq, g_wk, g_wv, g_wo, None, None
 
 
-def attn_half_supported(block, x, kv_cache, doc_ids, key_padding_mask) -> bool:
+def _unhooked(mod) -> bool:
+    """Leaving out the call of the module leaves out nothing but its class's own forward."""
+    return not (mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks or mod._backward_pre_hooks
+                or "forward" in mod.__dict__)
+
+
+def attn_half_supported(block, x, kv_cache, doc_ids, key_padding_mask, cos=None, sin=None) -> bool:
     """The fused attention sub-layer covers bf16 causal self-attention with head dim 64 or 128 on a GPU, without masks,
-    caches, q/k norms, tensor parallelism, fp8 or hooks; the feed-forward half of the block may be anything."""
+    caches, q/k norms, tensor parallelism, fp8 or hooks; the feed-forward half of the block may be anything.  ``cos`` / ``sin``:
+    the tables of the call, one row per position."""
     att = block.attention
+    if cos is not None and (cos.dim() != 2 or cos.shape != sin.shape or cos.size(0) < x.shape[1] or cos.size(1) != att.head_dim // 2):
+        return False
     if not (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 3 and kv_cache is None and doc_ids is None
             and key_padding_mask is None and torch.is_grad_enabled()):
         return False
@@ -537,8 +548,10 @@ def attn_half_supported(block, x, kv_cache, doc_ids, key_padding_mask) -> bool:
         and getattr(kc.lib(), "kf_attn_bwd_bf16", None) is not None
         and att.q_proj.weight.dtype == torch.bfloat16
         and not block._forward_hooks
-        and not att._forward_hooks
-        and not block.attention_norm._forward_hooks
+        and type(att).forward is Attention.forward
+        and _unhooked(att)
+        and _unhooked(block.attention_norm)
+        and not (_nn_module._has_any_global_hook() or torch.autograd.forward_ad._current_level >= 0)
     )
 
 

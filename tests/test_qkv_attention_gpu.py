@@ -86,3 +86,46 @@ def test_linear_over_weights_that_are_not_adjacent(native_lib, rows):
     check(y, x.detach().double(), w.t())
     check(got[0], dy.double(), w)
     check(torch.cat(got[1:]), dy.double().t(), x.detach().double())
+
+
+@pytest.mark.parametrize("heads", [8, 4])   # heads of 64 and of 128
+def test_attention_half_of_an_expert_block_keeps_what_surrounds_it(native_lib, monkeypatch, heads):
+    """Tables and hooks that the attention module serves: the same result as without the fused sub-layer."""
+    from kempnerforge_b200.config import ModelConfig
+    from kempnerforge_b200.models.position import precompute_rope_frequencies
+    from kempnerforge_b200.models.transformer import TransformerBlock
+    from kempnerforge_b200.ops import fused_block
+
+    torch.manual_seed(0)
+    cfg = ModelConfig(dim=512, n_layers=1, n_heads=heads, n_kv_heads=2, vocab_size=64, ffn_hidden_dim=256, max_seq_len=256,
+                      num_experts=4, moe_top_k=2, moe_packed_experts=True)
+    with torch.device(DEV):
+        block = TransformerBlock(cfg, 0).to(torch.bfloat16)
+    s, hd = 200, 512 // heads
+    cos, sin = precompute_rope_frequencies(hd, s, 10000.0, device=DEV)
+    x = torch.randn(2, s, 512, device=DEV).bfloat16()
+    calls = []
+    half = fused_block.attn_half
+    monkeypatch.setattr(fused_block, "attn_half", lambda *a: calls.append(1) or half(*a))
+
+    def run(c, sn):
+        xl = x.clone().requires_grad_(True)
+        y = block(xl, c, sn)
+        (g,) = torch.autograd.grad(y.float().square().sum(), xl)
+        return y.detach(), g
+
+    want = run(cos, sin)
+    assert len(calls) == 1
+    n = len(calls)
+    per_row = run(cos.expand(2, *cos.shape), sin.expand(2, *sin.shape))      # a table for every sequence: the formulas
+    assert all(float((a.float() - w.float()).norm()) <= 2.0**-6 * float(w.float().norm()) for a, w in zip(per_row, want))
+    seen = []
+    for mod in (block.attention, block.attention_norm):
+        for register in ("register_forward_pre_hook", "register_full_backward_hook"):
+            handle = getattr(mod, register)(lambda *a, at=(mod, register): seen.append(at))
+            run(cos, sin)
+            handle.remove()
+            assert seen[-1] == (mod, register)
+    assert len(seen) == 4 and len(calls) == n
+    run(cos, sin)
+    assert len(calls) == n + 1 and native_lib.read_status() == 0
