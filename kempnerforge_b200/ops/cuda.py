@@ -531,6 +531,7 @@ def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, n_rot: int, inve
     b, s, h, hd = x.shape
     y = torch.empty_like(x) if out is None else out
     assert cos.dtype == torch.float32 and cos.shape[0] >= s and cos.shape[1] == hd // 2
+    cos, sin = cos.contiguous(), sin.contiguous()   # the kernel steps from row to row by the width
     _check(
         lib().kf_rope_bf16(x.data_ptr(), y.data_ptr(), cos.data_ptr(), sin.data_ptr(), b * s, s, h, n_rot, hd, int(inverse), _stream()),
         "kf_rope_bf16",

@@ -116,6 +116,9 @@ def test_attention_half_of_an_expert_block_keeps_what_surrounds_it(native_lib, m
 
     want = run(cos, sin)
     assert len(calls) == 1
+    packed = torch.stack([cos, sin], 1)                      # tables that are not contiguous
+    apart = run(packed[:, 0], packed[:, 1])
+    assert all(torch.equal(a, w) or float((a.float() - w.float()).norm()) <= 2.0**-6 * float(w.float().norm()) for a, w in zip(apart, want))
     n = len(calls)
     per_row = run(cos.expand(2, *cos.shape), sin.expand(2, *sin.shape))      # a table for every sequence: the formulas
     assert all(float((a.float() - w.float()).norm()) <= 2.0**-6 * float(w.float().norm()) for a, w in zip(per_row, want))
