@@ -367,8 +367,11 @@ def dgrad_rows(dy2: torch.Tensor, weights) -> torch.Tensor:
     m, n = dy2.shape
     k = weights[0].shape[1]
     if (len(weights) in (2, 3) and not rows_adjacent(weights) and m > 0 and k > 0 and k % 8 == 0 and GEMM_MODE == 0
-            and (n < SPLIT_K_MIN or lib().kf_gemm_k_pieces(m, k, n, sm_count()) == 1) and dy2.stride(0) % 8 == 0 and dy2.data_ptr() % 16 == 0 and all(w.shape[0] % 64 == 0 for w in weights[:-1])
-            and all(w.stride() == weights[0].stride() and _plain_rows(w, dy2.device) for w in weights)):
+            and (n < SPLIT_K_MIN or lib().kf_gemm_k_pieces(m, k, n, sm_count()) == 1)
+            and dy2.dtype == torch.bfloat16 and dy2.stride(1) == 1 and dy2.stride(0) % 8 == 0 and dy2.data_ptr() % 16 == 0
+            and n == sum(w.shape[0] for w in weights) and all(w.shape[0] % 64 == 0 for w in weights[:-1])
+            and all(w.dtype == torch.bfloat16 and w.shape[1] == k and w.stride() == weights[0].stride() and _plain_rows(w, dy2.device)
+                    for w in weights)):
         out = torch.empty((m, k), dtype=torch.bfloat16, device=dy2.device)
         ptrs, rows, pitch = _weights3(weights)
         _check(lib().kf_gemm_dgrad_stacked_bf16(dy2.data_ptr(), *ptrs, out.data_ptr(), m, k, *rows, dy2.stride(0), pitch[0], k,

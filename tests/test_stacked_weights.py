@@ -151,6 +151,19 @@ def test_a_matrix_on_another_device_is_refused_before_any_kernel(fake):
     assert not fake.calls
 
 
+@pytest.mark.parametrize("m", [8, 600])
+def test_input_gradient_wants_rows_of_its_weights_width(fake, m):
+    from kempnerforge_b200.ops import cuda as kc
+
+    ws = _weights("dense", (128, 64), 64)
+    for dy in (torch.randn(192, m).bfloat16().t(), torch.randn(m, 200).bfloat16(), torch.randn(m, 192).half()):
+        with pytest.raises(AssertionError):
+            kc.dgrad_rows(dy, ws)
+    with pytest.raises((AssertionError, RuntimeError)):
+        kc.dgrad_rows(torch.randn(m, 192).bfloat16(), [w.float() for w in ws])
+    assert not fake.calls
+
+
 def _tables(s, half, shift, device="cpu"):
     """cos | sin of one packed buffer that starts ``shift`` values late."""
     g = torch.Generator(device=device).manual_seed(2)
