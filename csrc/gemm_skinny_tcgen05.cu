@@ -504,12 +504,4 @@ int kf_gemm_skinny_norm_qkv_bf16(const void* x, const void* gain, float eps, con
   return dispatch<2>(x, ldx, w, ldw, a, tiles, num_sms, (int*)kf_status_device_ptr(), (cudaStream_t)stream);
 }
 
-int kf_gemm_skinny_qkv_bf16(const void* x, const void* wq, const void* wk, const void* wv, void* q_out, void* kc, void* vc,
-                            int M, int S, int K, int q_cols, int kv_cols, int ldx, int ldwq, int ldwk, int ldwv, int ldq,
-                            long long cache_batch, const void* cosT, const void* sinT, int pdl, int num_sms,
-                            void* stream) {
-  return kf_gemm_skinny_norm_qkv_bf16(x, nullptr, 0.f, wq, wk, wv, q_out, kc, vc, M, S, K, q_cols, kv_cols, 128, ldx, ldwq, ldwk,
-                                      ldwv, ldq, cache_batch, cosT, sinT, pdl, num_sms, stream);
-}
-
 }  // extern "C"

@@ -4,9 +4,9 @@
 // piece (pick_splits in gemm_skinny_tcgen05.cu says why), so a generation step of a small model is a chain of K / 16 dependent
 // MMAs after another.  One tcgen05.mma that adds to the accumulator of the one before it takes 70 ns at 16 columns, whatever
 // the rows; mma.sync m16n8k16 takes a quarter of that and gives the same fp32 bits (compared with the tile kernels over K from
-// 16 to 4096, 65 536 sums each).  Hence
+// 16 to 4800).  Hence
 //   * a CTA owns 16 rows of W: the m16n8k16 tile of one warp, up to two of them for up to 16 tokens;
-//   * the CTA's whole strip of W (K <= 4096: 16 rows of at most 8 KB) is requested with one bulk copy per row before the
+//   * the CTA's whole strip of W (16 rows; beside x it has room for K up to 4800 with 8 rows of x, 3616 with 16) is requested with one bulk copy per row before the
 //     previous kernel of the stream has finished (a programmatic launch: only behind a kernel that writes no weights and no
 //     gain, see block_infer.cu), so that only x, the chain and the store remain behind it;
 //   * the accumulator of a thread holds rows g and g + 8 of the tile, which are made gate and up of one hidden unit, or the two
@@ -244,13 +244,14 @@ static int launch_small(const SmallWeights& sw, const Args& a, int tiles, int* s
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
-// Up to 16 rows, sums that stay in one piece, and every CTA's strip in shared memory at once (1 KB per CTA is the system's).
+// Up to 16 rows, sums that stay in one piece, and all CTAs resident at once: their strips in shared memory (1 KB per CTA is the
+// system's), their threads within the 2048 of an SM.
 bool small_fits(const Args& a, int epi, bool one_piece, int num_sms) {
   if (a.M > 16 || a.K % 32 || !one_piece) return false;
   const size_t smem = small_smem(a.K, (a.M + 7) / 8, a.gain != nullptr);
   int tiles = 0;
   for (int i = 0; i < a.n_seg; ++i) tiles += (a.rows[i] + SMALL_ROWS - 1) / SMALL_ROWS;
-  return smem <= 232448 && tiles <= num_sms * int(233472 / (smem + 1024));
+  return smem <= 232448 && tiles <= num_sms * min(int(233472 / (smem + 1024)), 2048 / SMALL_THREADS);
 }
 
 int run_small(int epi, const void* const* w, const int* ldw, Args& a, int* status, cudaStream_t stream) {

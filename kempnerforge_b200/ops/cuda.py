@@ -58,7 +58,6 @@ def _declare(L: ctypes.CDLL) -> None:
         "kf_gemm_dgrad_stacked_bf16": [vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, i, vp],
         "kf_gemm_skinny_bf16": [vp] * 6 + [i] * 14 + [vp],
         "kf_gemm_skinny_swiglu_bf16": [vp] * 4 + [i] * 9 + [vp],
-        "kf_gemm_skinny_qkv_bf16": [vp] * 7 + [i] * 10 + [ll, vp, vp, i, i, vp],
         "kf_skinny_norm_rows": [],
         "kf_gemm_skinny_norm_swiglu_bf16": [vp, vp, f, vp, vp, vp] + [i] * 9 + [vp],
         "kf_gemm_skinny_norm_qkv_bf16": [vp, vp, f] + [vp] * 6 + [i] * 11 + [ll, vp, vp, i, i, vp],

@@ -32,7 +32,8 @@ def test_norm_along_with_swiglu(native_lib, m, f, k):
 
 
 @pytest.mark.parametrize("hd", [64, 128])
-@pytest.mark.parametrize("b,heads,kv,k", [(1, 12, 12, 768), (2, 3, 1, 264), (4, 16, 4, 2048), (5, 6, 3, 520), (33, 4, 2, 768)])
+@pytest.mark.parametrize("b,heads,kv,k", [(1, 12, 12, 768), (2, 3, 1, 264), (4, 16, 4, 2048), (5, 6, 3, 520), (9, 4, 2, 768), (16, 6, 2, 3616),
+                                            (33, 4, 2, 768)])
 def test_projection_rotation_and_cache(native_lib, b, heads, kv, k, hd):
     kc, L = native_lib, native_lib.lib()
     qc, kvc = heads * hd, kv * hd
@@ -65,7 +66,8 @@ def test_projection_rotation_and_cache(native_lib, b, heads, kv, k, hd):
 
 
 @pytest.mark.parametrize("m", [1, 2, 7, 8, 9, 16])
-@pytest.mark.parametrize("rows,k", [([8], 32), ([768], 768), ([24, 40, 8], 96), ([768], 2048), ([256, 64], 1504), ([512], 4096)])
+@pytest.mark.parametrize("rows,k", [([8], 32), ([768], 768), ([24, 40, 8], 96), ([768], 2048), ([256, 64], 1504), ([512], 4096),
+                                    ([136], 3616), ([64], 4800)])
 def test_small_weights_keep_the_bits_of_the_tile_kernel(native_lib, m, rows, k):
     kc = native_lib
     x = _rand(m, k + 8, seed=1)[:, :k]
@@ -78,6 +80,24 @@ def test_small_weights_keep_the_bits_of_the_tile_kernel(native_lib, m, rows, k):
     w = torch.cat(ws)
     assert torch.equal(out, kc.gemm(x, w, mode=1)) and torch.equal(with_res, kc.gemm(x, w, residual=res, mode=1))
     assert bool((frame[m:] == 7).all()) and bool((frame[:, sum(rows):] == 7).all())
+
+
+@pytest.mark.parametrize("m", [1, 4, 8, 9, 15, 16])
+@pytest.mark.parametrize("f,k", [(8, 32), (2048, 768), (136, 3616), (64, 4608)])
+def test_small_weights_with_swiglu_against_the_tile_kernel(native_lib, m, f, k):
+    """Gate and up on single-CTA tiles, then the SwiGLU kernel; with the norm along, the norm kernel first."""
+    kc, L = native_lib, native_lib.lib()
+    x, gain = _rand(m, k, scale=2.0, seed=1), 1 + 0.1 * _rand(k, seed=2)
+    wg, wu = _rand(f, k, scale=k**-0.5, seed=3), _rand(f, k, scale=k**-0.5, seed=4)
+    w = torch.cat([wg, wu])
+    frame = torch.full((m + 1, f + 8), 7.0, dtype=torch.bfloat16, device=DEV)
+    for g in (None, gain) if m <= L.kf_skinny_norm_rows() else (None,):
+        n = x if g is None else kc.rmsnorm_fwd(x, g, 1e-5)[0]
+        kc._check(L.kf_gemm_skinny_norm_swiglu_bf16(x.data_ptr(), kc._ptr(g), 1e-5, wg.data_ptr(), wu.data_ptr(), frame.data_ptr(), m, f, k,
+                                                    k, k, k, f + 8, 0, kc.sm_count(), kc._stream()), "swiglu")
+        assert native_lib.read_status() == 0
+        assert torch.equal(frame[:m, :f], kc.swiglu_fwd(kc.gemm(n, w, mode=1)))
+    assert bool((frame[m:] == 7).all()) and bool((frame[:, f:] == 7).all())
 
 
 def _model(heads, kv, batch, ctx, layers=3, **over):
