@@ -280,9 +280,9 @@ namespace kf {
 // measure of tokens_width: pairs as they are, a round of single-CTA tiles 920 (their k-block takes 1.2 times that of a pair) or,
 // over an MN-major B, 800.  Measured, token tiles / the others, us: 4096 columns from 14336 over 300 rows 74 / 95, over 1200 rows
 // 145 / 150; 5120 from 13824 over 777 rows, where single CTAs have one round and pairs two, 138 / 98; at equal rounds 4096 from
-// 4096 over 2300 rows 57 / 60, from more than four rounds on no difference.  Input gradients (MN-major): 5120 columns from 7168 over 1332 rows 80 / 94, over 2000 118 /
-// 119; from 2048, where the ramp shows, 17.3 / 16.7 over 1554 rows.
-static int tokens_pay(int M, int N, int K, int b_mn, int pair, int num_sms) {
+// 4096 over 2300 rows 57 / 60, from more than four rounds on no difference.  Input gradients (MN-major): 5120 columns from 7168 over
+// 1332 rows 80 / 94, over 2000 118 / 119; from 2048, where the ramp shows, 17.3 / 16.7 over 1554 rows.
+static int plain_tokens(int M, int N, int K, int b_mn, int pair, int num_sms) {
   if (num_sms < 2 || (b_mn && K < 3072)) return 0;
   const int pairs = num_sms / 2;
   float cost, other;
@@ -297,9 +297,26 @@ static int tokens_pay(int M, int N, int K, int b_mn, int pair, int num_sms) {
   if (b_mn) return cost * (1.f + 160.f / float(K)) < 0.96f * other ? tn : 0;  // W is the transposed operand: ramp of 2.5 k-blocks
   return cost <= (rounds <= 4 ? 1.f : 0.97f) * other ? tn : 0;
 }
+
+// 2: CTA pairs, 1: one CTA per tile.  Pairs pay off once there are enough 256 x 256 tiles to fill the machine a few times over.
+static int plain_mode(int M, int N, int b_mn, int num_sms) {
+  const long long pair_tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
+  if (pair_tiles >= 2LL * (num_sms / 2)) return 2;
+  // Between one and two rounds of pairs, K-major B: both forms take two rounds, and a narrower pair tile makes them shorter
+  // (1554 x 4096 from 4096 and 11008: 250 -> 223 us for the two).  With at most one round the single-CTA tiles stay ahead
+  // (1777 rows, 2048 columns: 60 us against 68 for a layer's products).
+  if (!b_mn && pair_tiles > num_sms / 2) {
+    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+    if (kf2::gemm_pair_cost(M, N, num_sms) < 1.1f * BN * float((tiles + num_sms - 1) / num_sms)) return 2;
+  }
+  return 1;
+}
 }  // namespace kf
 
 namespace kf2 {
+int swiglu_tokens(int M, int F, int K, int num_sms);
+int rope_tokens(int M, int N, int hd, int num_sms);
+int swiglu_bwd_tokens(int M, int F, int num_sms);
 int launch_gemm_swiglu_2cta(const void* A, const void* Wg, const void* Wu, void* H, void* GU, int M, int F, int K, int lda,
                             int ldw, int ldh, int ldgu, int num_sms, cudaStream_t stream, int* status);
 }
@@ -353,10 +370,10 @@ int kf_gemm_dgrad_stacked_bf16(const void* dy, const void* w0, const void* w1, c
   const void* w[3] = {w0, w1, w2};
   const int rows[3] = {n0, n1, n2};
   // the rules of kf_gemm_bf16 for an MN-major B: pairs once their tiles are two rounds, token tiles where they are shorter
-  const int pair = (long long)((M + 255) / 256) * ((K + 255) / 256) >= 2LL * (num_sms / 2);
+  const int pair = kf::plain_mode(M, K, 1, num_sms) == 2;
   const int n_seg = n1 <= 0 ? 1 : n2 <= 0 ? 2 : 3;
   const bool whole = n0 > 0 && (n0 % 64 == 0 || n_seg == 1) && (n1 % 64 == 0 || n_seg < 3);  // no k-block reaches over two weights
-  if (const int tn = whole ? kf::tokens_pay(M, K, n0 + n1 + n2, 1, pair, num_sms) : 0)
+  if (const int tn = whole ? kf::plain_tokens(M, K, n0 + n1 + n2, 1, pair, num_sms) : 0)
     return kf2::launch_tokens_plain(dy, w, rows, n_seg, 1, out, nullptr, M, K, n0 + n1 + n2, lda, ldw, ldc, 0, tn, num_sms,
                                     (cudaStream_t)stream, kf::status_ptr());
   if (!pair)
@@ -418,6 +435,16 @@ int kf_gemm_swiglu_bf16(const void* x, const void* wg, const void* wu, void* h, 
                                       kf::status_ptr());
 }
 
+// Rows of A per tile when a product takes the tiles cut to their number, 0 when it takes another kernel: plain products over a
+// K-major (kind 0) or an MN-major B (1), SwiGLU with N hidden units (2), rotary embedding with heads of `hd` (3), SwiGLU gradient
+// with N hidden units (4).
+int kf_gemm_tokens_width(int kind, int M, int N, int K, int hd, int num_sms) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (kind <= 1) return kf::plain_tokens(M, N, K, kind, kf::plain_mode(M, N, kind, num_sms) == 2, num_sms);
+  return kind == 2 ? kf2::swiglu_tokens(M, N, K, num_sms) : kind == 3 ? kf2::rope_tokens(M, N, hd, num_sms)
+                                                                     : kf2::swiglu_bwd_tokens(M, N, num_sms);
+}
+
 // C[M,N] = op(A) * op(B)^T (+ C if accumulate) (+ R if given), bf16 inputs, fp32 accumulation.
 //   a_mn == 0: A is stored [M][lda] (K contiguous);  a_mn == 1: A is stored [K][lda] (M contiguous)
 //   b_mn == 0: B is stored [N][ldb] (K contiguous);  b_mn == 1: B is stored [K][ldb] (N contiguous)
@@ -433,20 +460,9 @@ int kf_gemm_bf16(const void* A, const void* B, void* C, const void* R, int M, in
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (M <= 0 || N <= 0 || K <= 0) return 1;
   const bool automatic = mode == 0;
-  if (automatic) {
-    // pairs pay off once there are enough 256x256 tiles to fill the machine a few times over
-    const long long pair_tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
-    mode = pair_tiles >= 2LL * (num_sms / 2) ? 2 : 1;
-    // Between one and two rounds of pairs, K-major B: both forms take two rounds, and a narrower pair tile makes them shorter
-    // (1554 x 4096 from 4096 and 11008: 250 -> 223 us for the two).  With at most one round the single-CTA tiles stay ahead
-    // (1777 rows, 2048 columns: 60 us against 68 for a layer's products).
-    if (mode == 1 && !b_mn && pair_tiles > num_sms / 2) {
-      const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-      if (kf2::gemm_pair_cost(M, N, num_sms) < 1.1f * BN * float((tiles + num_sms - 1) / num_sms)) mode = 2;
-    }
-  }
+  if (automatic) mode = plain_mode(M, N, b_mn, num_sms);
   if (!a_mn && !out_f32 && !accumulate && num_sms >= 2 && (N & 7) == 0 && (automatic || mode == 3)) {
-    const int tn = mode == 3 ? kf2::tokens_width(M, N, num_sms, nullptr, nullptr) : tokens_pay(M, N, K, b_mn, mode == 2, num_sms);
+    const int tn = mode == 3 ? kf2::tokens_width(M, N, num_sms, nullptr, nullptr) : plain_tokens(M, N, K, b_mn, mode == 2, num_sms);
     const void* w[3] = {B, nullptr, nullptr};
     const int rows[3] = {b_mn ? K : N, 0, 0};
     if (tn) return kf2::launch_tokens_plain(A, w, rows, 1, b_mn, C, R, M, N, K, lda, ldb, ldc, ldr, tn, num_sms, st, status_ptr());

@@ -45,7 +45,7 @@ int launch_tokens_swiglu_bwd(const void* dy, const void* w, const void* gu, void
 // (0.96) is worth it only where enough k-blocks hide that.  Measured, token tiles / these, us: gate and up of 14336 over 777 tokens
 // (0.96) 162 / 167, 7168 over 999 from 2048 columns (0.96) 55 / 53; q | k | v of 6144 over 520 (0.92) 34 / 35, over 640 (0.96)
 // 35.2 / 34.9; the gradient of 14336 over 520 (0.92) 78 / 82, over 2000 (0.96) 196 / 192.
-static int tokens_pay(int M, int m_rows, int n_tiles, float limit, int num_sms) {
+static int fused_tokens(int M, int m_rows, int n_tiles, float limit, int num_sms) {
   if (num_sms < 2) return 0;
   const int pairs = num_sms / 2;
   const long long tiles = (long long)((M + 255) / 256) * n_tiles;
@@ -58,6 +58,16 @@ constexpr int CTA_M = 128;   // rows of A per CTA
 constexpr int TILE_M = 256;  // rows per CTA pair
 constexpr int TILE_N = 256;
 constexpr int HALF_N = 128;  // rows of B per CTA
+
+// The rule for each epilogue: SwiGLU over 2F rows of gate and up, rotary embedding over N rows of q | k | v, SwiGLU gradient.
+int swiglu_tokens(int M, int F, int K, int num_sms) {
+  return fused_tokens(M, 2 * F, (F + HALF_N - 1) / HALF_N, K >= 4096 ? 0.97f : 0.93f, num_sms);
+}
+int rope_tokens(int M, int N, int hd, int num_sms) {
+  return hd == 256 ? 0 : fused_tokens(M, N, (N + TILE_N - 1) / TILE_N, 0.93f, num_sms);
+}
+int swiglu_bwd_tokens(int M, int F, int num_sms) { return fused_tokens(M, F, (F + TILE_N - 1) / TILE_N, 0.93f, num_sms); }
+
 constexpr int BK = 64;
 constexpr int STAGES = 6;
 constexpr int UMMA_K = 16;
@@ -607,7 +617,7 @@ static int launch(const void* A, const void* B, void* C, const void* R, int M, i
 // h[M, F] = silu(x Wg^T) * (x Wu^T), Wg and Wu [F][K] each; gu (optional) receives [M, 2F] pre-activations.  F % 128 == 0.
 int launch_gemm_swiglu_2cta(const void* A, const void* Wg, const void* Wu, void* H, void* GU, int M, int F, int K, int lda,
                             int ldw, int ldh, int ldgu, int num_sms, cudaStream_t stream, int* status) {
-  if (const int tn = tokens_pay(M, 2 * F, (F + HALF_N - 1) / HALF_N, K >= 4096 ? 0.97f : 0.93f, num_sms))
+  if (const int tn = swiglu_tokens(M, F, K, num_sms))
     return launch_tokens_swiglu(A, Wg, Wu, H, GU, M, F, K, lda, ldw, ldh, ldgu, tn, num_sms, stream, status);
   CUtensorMap ma;
   WeightSegs ws;
@@ -644,12 +654,11 @@ int launch_gemm_rope_2cta(const void* A, const void* const* W, const int* rows, 
                           int ldw, int ldc, const float* cosT, const float* sinT, int S, int rope_cols, int hd, int num_sms,
                           cudaStream_t stream, int* status) {
   if ((hd != 64 && hd != 128 && hd != 256) || N % hd || rope_cols % hd || rope_cols > N || S <= 0) return 6;
-  if (hd != 256)
-    if (const int tn = tokens_pay(M, N, (N + TILE_N - 1) / TILE_N, 0.93f, num_sms)) {
-      const int n_seg = rows[1] <= 0 ? 1 : rows[2] <= 0 ? 2 : 3;
-      if (rows[0] <= 0 || rows[0] + (n_seg > 1 ? rows[1] : 0) + (n_seg > 2 ? rows[2] : 0) != N) return 6;
-      return launch_tokens_rope(A, W, rows, n_seg, C, M, N, K, lda, ldw, ldc, cosT, sinT, S, rope_cols, hd, tn, num_sms, stream, status);
-    }
+  if (const int tn = rope_tokens(M, N, hd, num_sms)) {
+    const int n_seg = rows[1] <= 0 ? 1 : rows[2] <= 0 ? 2 : 3;
+    if (rows[0] <= 0 || rows[0] + (n_seg > 1 ? rows[1] : 0) + (n_seg > 2 ? rows[2] : 0) != N) return 6;
+    return launch_tokens_rope(A, W, rows, n_seg, C, M, N, K, lda, ldw, ldc, cosT, sinT, S, rope_cols, hd, tn, num_sms, stream, status);
+  }
   CUtensorMap ma;
   WeightSegs ws;
   int rc = make_map_2d_bf16(&ma, A, M, K, lda, BK, CTA_M);
@@ -785,7 +794,7 @@ int launch_gemm_gather_2cta(int epi, const void* A, void* C, const void* R, int 
 // weight read for its input gradient); gu and dgu may be the same buffer.  F % 8 == 0, K % 64 == 0.
 int launch_gemm_swiglu_bwd_2cta(const void* DY, const void* W, const void* GU, void* DGU, int M, int F, int K, int lda,
                                 int ldw, int ldgu, int num_sms, cudaStream_t stream, int* status) {
-  if (const int tn = tokens_pay(M, F, (F + TILE_N - 1) / TILE_N, 0.93f, num_sms))
+  if (const int tn = swiglu_bwd_tokens(M, F, num_sms))
     return launch_tokens_swiglu_bwd(DY, W, GU, DGU, M, F, K, lda, ldw, ldgu, tn, num_sms, stream, status);
   CUtensorMap ma, mb;
   int rc = make_map_2d_bf16(&ma, DY, M, K, lda, BK, CTA_M);

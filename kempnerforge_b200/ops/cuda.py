@@ -51,6 +51,7 @@ def _declare(L: ctypes.CDLL) -> None:
     vp, i, ll, f = c_void_p, c_int, c_longlong, c_float
     sigs = {
         "kf_gemm_k_pieces": [i, i, i, i],
+        "kf_gemm_tokens_width": [i, i, i, i, i, i],
         "kf_gemm_split_k_bf16": [vp, vp, vp, vp, i, i, i, i, i, i, i, i, vp],
         "kf_gemm_bf16": [vp, vp, vp, vp, i, i, i, i, i, i, i, i, i, i, i, i, i, vp],
         "kf_gemm_swiglu_bf16": [vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, vp],
@@ -228,7 +229,8 @@ def gemm(
     projection): the heads inside the first ``rope_cols`` output columns are rotated by the angle of position
     ``row % seq_len``; ``cos`` / ``sin`` are fp32 (seq_len, head_dim / 2).  Needs K-major operands, bf16 output.
 
-    ``mode``: None/0 = automatic, 1 = single-CTA 128x256 tiles, 2 = CTA pairs (cta_group::2) on 256x256 tiles.
+    ``mode``: None/0 = automatic, 1 = single-CTA 128x256 tiles, 2 = CTA pairs (cta_group::2) on 256x256 tiles, 3 = CTA pairs
+    on tiles cut to the number of rows.
 
     ``a_kmajor``: a is stored (M, K); otherwise (K, M).  ``b_kmajor``: b is stored (N, K); otherwise (K, N).
     Rows may be strided (row pitch a multiple of 8 elements); columns must be contiguous.
