@@ -132,6 +132,7 @@ kf_gemm_skinny(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         tma_load_2d(smem_base + s * C::STAGE + W_BYTES, &map_x, full_bar(s), (kb0 + i) * BK, 0);
       };
       const int pre = min(n_kb, C::STAGES);
+      if (a.pdl == PDL_WAIT_FIRST) grid_dep_wait();
       for (int i = 0; i < pre; ++i) load_w(i);
       if (!NORM) {
         grid_dep_wait();

@@ -89,6 +89,7 @@ kf_gemm_small(const __grid_constant__ SmallWeights sw, const __grid_constant__ A
     mbar_init(w_bar, 1);
     mbar_init(x_bar, 1);
     mbar_fence_init();
+    if (a.pdl == PDL_WAIT_FIRST) grid_dep_wait();
     mbar_expect_tx(w_bar, uint32_t(has_hi ? 16 : 8) * 2 * K + (NORM ? 2 * K : 0));
     for (int r = 0; r < 8; ++r)
       bulk_row(w_smem + r * pitch, sw.w[seg] + size_t(r_lo + r) * sw.ldw[seg], 2 * K, w_bar);

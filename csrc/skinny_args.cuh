@@ -6,6 +6,11 @@
 namespace kf {
 namespace skinny {
 
+// Args::pdl.  0: an ordinary launch.  PDL_EARLY_WEIGHTS: a programmatic launch behind a kernel that writes no weights and no gain; they
+// are fetched while it runs.  PDL_WAIT_FIRST: a programmatic launch behind any kernel; nothing is read before the wait, only barriers and
+// tensor memory are set up.
+constexpr int PDL_EARLY_WEIGHTS = 1, PDL_WAIT_FIRST = 2;
+
 constexpr int NORM_ROWS = 4;  // rows up to which a projection takes the norm of its input along
 
 struct Args {
@@ -25,7 +30,7 @@ struct Args {
   const __nv_bfloat16 *x, *gain; // [M][ldx]; [K] with the norm, else null
   int ldx;
   float eps;
-  int pdl;
+  int pdl;                       // how the launch follows the previous kernel, see above
 };
 
 // The arithmetic of kf_rmsnorm_fwd, whose block of 256 threads adds the squares of every 256th vector of 8 per thread, then
