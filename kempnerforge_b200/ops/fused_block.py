@@ -38,7 +38,6 @@ from torch.nn.modules import module as _nn_module
 
 from kempnerforge_b200.models.attention import Attention
 from kempnerforge_b200.ops import cuda as kc
-from kempnerforge_b200.ops.fused_infer import _matrix
 
 
 def _wgrad(dy2: torch.Tensor, x2: torch.Tensor, weights) -> list:
@@ -145,9 +144,21 @@ def _rope_fused(n1, w_qkv, cos, sin, s: int, hd: int) -> bool:
 _SWITCHES = ("KF_ROPE_EPILOGUE", "KF_DISABLE_SWIGLU_EPILOGUE", "KF_SWIGLU_BWD_EPILOGUE", "KF_ATTN_FWD", "KF_AC_KEEP_ATTN")
 
 
-def _vector(w, d: int, device) -> bool:
-    return (w.dtype is torch.bfloat16 and w.dim() == 1 and w.size(0) == d and w.is_contiguous() and w.data_ptr() % 16 == 0
-            and w.device == device)
+def _chain_operands(dims, x2, cos, sin, weights):
+    """Addresses of a block's operands if they lie as the kernels read them, else None.  Both passes ask: a backward pass may be
+    given other tensors than the forward pass was."""
+    b, s, d, h, hkv, hd, f = dims
+    qc, kvc = h * hd, hkv * hd
+    ptrs, low, dev = [], 0, x2.get_device()
+    for t, shape in zip((x2, *weights), ((b * s, d), (d,), (qc, d), (kvc, d), (kvc, d), (d, qc), (d,), (f, d), (f, d), (d, f))):
+        if t.shape != shape or t.dtype is not torch.bfloat16 or not t.is_contiguous() or t.get_device() != dev:
+            return None
+        ptrs.append(t.data_ptr())
+        low |= ptrs[-1]
+    if (low & 15 or not kc.rope_tables_ok(cos, sin) or cos.dim() != 2 or cos.shape != sin.shape or cos.size(0) < s
+            or cos.size(1) != hd // 2 or cos.get_device() != dev or sin.get_device() != dev):
+        return None
+    return ptrs + [cos.data_ptr(), sin.data_ptr()]
 
 
 def _chain_dims(x2, cos, sin, weights, b: int, s: int, d: int, hd: int):
@@ -160,14 +171,12 @@ def _chain_dims(x2, cos, sin, weights, b: int, s: int, d: int, hd: int):
             or any(k in os.environ for k in _SWITCHES) or kc.attn_policy() != "native"
             or not kc.attn_bwd_chosen(hd, b * (qc // hd), s, s, True, False)):
         return None
-    dev = x2.device
-    for w, rows, cols in ((wq, qc, d), (wk, kvc, d), (wv, kvc, d), (wo, d, qc), (wg, f, d), (wu, f, d), (wd, d, f)):
-        if not _matrix(w, rows, cols) or w.device != dev or _sharded_unit(w) is not None:
+    for w in weights:
+        tags = w.__dict__
+        if "_kf_fp8" in tags or getattr(tags.get("_kf_flat"), "sharded", False):
             return None
-    if (not _vector(wn1, d, dev) or not _vector(wn2, d, dev) or not x2.is_contiguous() or x2.data_ptr() % 16 or not kc.rope_tables_ok(cos, sin) or cos.device != dev
-            or sin.device != dev or cos.dim() != 2 or cos.shape != sin.shape or cos.size(0) < s or cos.size(1) != hd // 2):
-        return None
-    return b, s, d, qc // hd, kvc // hd, hd, f
+    dims = b, s, d, qc // hd, kvc // hd, hd, f
+    return None if _chain_operands(dims, x2, cos, sin, weights) is None else dims
 
 
 class _ChainState:
@@ -190,13 +199,14 @@ class _ChainState:
         if not keep:
             self.parts[8] = 0
         self.y = torch.empty((t, d), dtype=torch.bfloat16, device=x2.device) if need_output else None
-        ints = array("q", (*self.block_args(x2, cos, sin, weights), self.y.data_ptr() if need_output else 0))
+        operands = [w.data_ptr() for w in (x2, *weights, cos, sin)]
+        ints = array("q", (*self.block_args(operands), self.y.data_ptr() if need_output else 0))
         kc._check(kc.lib().kf_block_train_fwd_bf16(ints.buffer_info()[0], self.scalars.buffer_info()[0], kc._stream()),
                   "kf_block_train_fwd_bf16", 7 if need_output else 6)
 
-    def block_args(self, x2, cos, sin, weights) -> list:
+    def block_args(self, operands) -> list:
         """The first values of either native call."""
-        return [*(t.data_ptr() for t in (x2, *weights, cos, sin)), *self.parts, *self.dims, kc.sm_count()]
+        return [*operands, *self.parts, *self.dims, kc.sm_count()]
 
     def views(self) -> dict:
         """The parts as the tensors that the op-by-op backward reads."""
@@ -226,8 +236,12 @@ def _grad_target(weights):
 
 
 def _chain_backward(it: _ChainState, dy2, x2, cos, sin, weights):
-    """(dx, gradients of the nine weights) of a natively issued forward, or None when the gradient slots do not fit."""
+    """(dx, gradients of the nine weights) of a natively issued forward, or None when the operands or the gradient slots do not
+    fit."""
     wn1, wq, wk, wv, wo, wn2, wg, wu, wd = weights
+    operands = _chain_operands(it.dims, x2, cos, sin, weights)
+    if operands is None:
+        return None
     groups = ((wq, wk, wv), (wo,), (wg, wu), (wd,))
     targets = [_grad_target(g) for g in groups]
     if any(t is None for t in targets) or dy2.dtype is not torch.bfloat16:
@@ -249,7 +263,7 @@ def _chain_backward(it: _ChainState, dy2, x2, cos, sin, weights):
     base = scratch.data_ptr()
     pieces = L.kf_gemm_k_pieces(t, d, 2 * f, kc.sm_count()) if 2 * f >= kc.SPLIT_K_MIN else 1
     stack_gu, ws = kc.rows_adjacent((wg, wu)), None
-    ptrs = it.block_args(x2, cos, sin, weights)
+    ptrs = it.block_args(operands)
     if pieces > 1:
         ws = torch.empty((pieces, t, d), dtype=torch.float32, device=dev)
         if not stack_gu:
@@ -379,16 +393,13 @@ class DenseBlockFn(torch.autograd.Function):
         if unit is not None:
             unit.engine.prepare_backward(unit)  # parameter staging is ours again; gradient staging slot is free
         it = ctx.inter
-        dims = None
-        if isinstance(it, _ChainState) or (it is None and unit is None and ctx.attn_saved is None):
-            dims = _chain_dims(x2, cos, sin, ctx.weights, b, s, d, hd)   # of the tensors that this pass was given
-        if it is None and dims is not None:
-            it = _ChainState(x2, cos, sin, ctx.weights, dims, eps, keep=True, need_output=False)
+        if it is None and unit is None and ctx.attn_saved is None:
+            dims = _chain_dims(x2, cos, sin, ctx.weights, b, s, d, hd)
+            if dims is not None:
+                it = _ChainState(x2, cos, sin, ctx.weights, dims, eps, keep=True, need_output=False)
         if isinstance(it, _ChainState):
             dy2 = dy.reshape(b * s, d)
-            done = None
-            if dims == it.dims:
-                done = _chain_backward(it, dy2 if dy2.is_contiguous() else dy2.contiguous(), x2, cos, sin, ctx.weights)
+            done = _chain_backward(it, dy2 if dy2.is_contiguous() else dy2.contiguous(), x2, cos, sin, ctx.weights)
             if done is not None:
                 ctx.inter = None
                 return (done[0].view(b, s, d), None, None, *done[1], None, None, None)
