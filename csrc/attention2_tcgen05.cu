@@ -12,8 +12,9 @@
 //   warps 4-7  : softmax + epilogue of tile A (one thread per query row)
 //   warps 8-11 : softmax + epilogue of tile B
 // A softmax thread holds a row of 128 scores; at the 168 registers that an even split leaves it spilled 50 - 110 bytes per
-// tile, so the first warpgroup gives its registers to the other two.  2 x 4096 tokens, 32 query and
-// 8 key heads of 128: 290 -> 274 us; 3000 tokens, 40 heads: 124 -> 114 us; 4 x 2048 tokens, 12 heads of 64: 68.5 -> 62.5 us.
+// tile, so the first warpgroup gives its registers to the other two.  The kernel alone: 2 x 4096 tokens, 32 query and 8 key heads
+// of 128, 290 -> 274 us; 3000 tokens, 40 heads, 124 -> 114; 4 x 2048 tokens, 12 heads of 64, 68.5 -> 62.5.  In a whole training
+// step of these sizes, which the power cap paces, that is below the spread of the runs.
 //
 //   TMEM      : S_A | S_B | O_A | O_B   (128 fp32 columns each; bf16 P aliases the start of its S)
 //
