@@ -746,9 +746,9 @@ static int run(const void* q, const void* k, const void* v, const void* o, const
     const long long rows = (long long)B * Sq;
     const int cols = H * hd;
     if (HD == 64)
-      kf_dq_add_parts<<<1184, 256, 0, st>>>(reinterpret_cast<const float*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dq), B, Sq, H, key_tiles,
-                                            causal, lddq, reinterpret_cast<const float*>(cosT), reinterpret_cast<const float*>(sinT),
-                                            scale);
+      kf_dq_add_parts<<<1184, 256, 0, st>>>(reinterpret_cast<const float*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dq), B, Sq, H,
+                                            key_tiles, causal, lddq, reinterpret_cast<const float*>(cosT),
+                                            reinterpret_cast<const float*>(sinT), scale);
     else if (cosT)
       kf_dq_finish_rope<<<1184, 256, 0, st>>>(reinterpret_cast<const float*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dq),
                                               rows, H, lddq, reinterpret_cast<const float*>(cosT),
@@ -776,8 +776,8 @@ int kf_attn_bwd_dq_mode(int mode) {
 
 // Backward attention (head dim 64 or 128).  q / k / v / o / do: rows (b * S + s) with pitches ld*, heads side by
 // side; lse: fp32 [B][H][Sq] from the forward; dsum: fp32 scratch [B][H][Sq]; dq_acc: fp32 scratch, [B][Sq][H][128] (zeroed
-// here) or, for head dim 64, [ceil(Sk / 128)][B][H][ceil(Sq / 64) * 64][64]; dq / dk / dv: bf16 outputs with pitches lddq / lddk / lddv (they may be
-// slices of one fused gradient buffer).  doc: optional int32 [B][S].  Requires Sq == Sk when causal or doc.
+// here) or, for head dim 64, [ceil(Sk / 128)][B][H][ceil(Sq / 64) * 64][64]; dq / dk / dv: bf16 outputs with pitches lddq / lddk /
+// lddv (they may be slices of one fused gradient buffer).  doc: optional int32 [B][S].  Requires Sq == Sk when causal or doc.
 // kf_attn_bwd_rope_bf16: the same, and dq / dk additionally pass through the inverse rotary embedding (cosT / sinT:
 // fp32 [Sq][hd / 2], position = index inside the sequence), i.e. they are gradients with respect to the un-rotated
 // projections when q / k were rotated after the projection.  Null tables = no rotation.  doc_range (optional): the id

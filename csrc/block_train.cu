@@ -102,8 +102,8 @@ int kf_block_train_fwd_bf16(const long long* a, const double* r, void* st) {
 }
 
 // Gradients of the above.  a: as there, then dy [T][D], dx [T][D], dWqkv [qc + 2 kvc][D], dWo [D][qc], dWgu [2F][D], dWd [D][F],
-// dwn1 [D], dwn2 [D]; dh1 [T][D], dattn [T][qc], dqkv [T][qc + 2 kvc], dq_acc fp32 (as kf_attn_bwd_rope_bf16 wants it), dsum fp32 [B][H][S], partial
-// (kf_rmsnorm_bwd_blocks(T) * D fp32); accumulate into dWqkv, dWo, dWgu, dWd (0 or 1 each); stacked: q | k | v and gate | up each lie
+// dwn1 [D], dwn2 [D]; dh1 [T][D], dattn [T][qc], dqkv [T][qc + 2 kvc], dq_acc fp32 (as kf_attn_bwd_rope_bf16 wants it),
+// dsum fp32 [B][H][S], partial (kf_rmsnorm_bwd_blocks(T) * D fp32); accumulate into dWqkv, dWo, dWgu, dWd (0 or 1 each); stacked: q | k | v and gate | up each lie
 // back to back; ws and pieces of a split gate | up input gradient (stacked only; 0 and 1: not split).  gu is overwritten.
 int kf_block_train_bwd_bf16(const long long* a, const double* r, void* st) {
   using namespace kf::blocktrain;

@@ -6,9 +6,9 @@
 // the rows; mma.sync m16n8k16 takes a quarter of that and gives the same fp32 bits (compared with the tile kernels over K from
 // 16 to 4800).  Hence
 //   * a CTA owns 16 rows of W: the m16n8k16 tile of one warp, up to two of them for up to 16 tokens;
-//   * the CTA's whole strip of W (16 rows; beside x it has room for K up to 4800 with 8 rows of x, 3616 with 16) is requested with one bulk copy per row before the
-//     previous kernel of the stream has finished (a programmatic launch: only behind a kernel that writes no weights and no
-//     gain, see block_infer.cu), so that only x, the chain and the store remain behind it;
+//   * the CTA's whole strip of W (16 rows; beside x it has room for K up to 4800 with 8 rows of x, 3616 with 16) is requested with
+//     one bulk copy per row before the previous kernel of the stream has finished (a programmatic launch: only behind a kernel
+//     that writes no weights and no gain, see block_infer.cu), so that only x, the chain and the store remain behind it;
 //   * the accumulator of a thread holds rows g and g + 8 of the tile, which are made gate and up of one hidden unit, or the two
 //     halves of a rotary pair: no exchange before the epilogue;
 //   * optionally the norm of x is taken along, in the arithmetic and order of kf_rmsnorm_fwd (the same bits).

@@ -440,6 +440,7 @@ int kf_gemm_swiglu_bf16(const void* x, const void* wg, const void* wu, void* h, 
 // with N hidden units (4).
 int kf_gemm_tokens_width(int kind, int M, int N, int K, int hd, int num_sms) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (kind <= 1 && (N & 7)) return 0;
   if (kind <= 1) return kf::plain_tokens(M, N, K, kind, kf::plain_mode(M, N, kind, num_sms) == 2, num_sms);
   return kind == 2 ? kf2::swiglu_tokens(M, N, K, num_sms) : kind == 3 ? kf2::rope_tokens(M, N, hd, num_sms)
                                                                      : kf2::swiglu_bwd_tokens(M, N, num_sms);
