@@ -7,8 +7,9 @@
 // hand over, and the tensor cores alternate  O_A += P_A V_j, S_A = Q_A K_{j+1}^T, O_B += P_B V_j, S_B = Q_B K_{j+1}^T.
 // K and V tiles are fetched once for both query tiles.
 //
-//   warp 0     : TMA producers (lane 0: Q_A, Q_B and the K ring; lane 1: the V ring)
-//   warp 1     : MMA issuer (warps 2 and 3 only make the first warpgroup whole)
+//   warp 0     : TMA producer (Q_A, Q_B and the K ring)
+//   warp 1     : MMA issuer
+//   warp 2     : TMA producer of the V ring (warp 3 only makes the first warpgroup whole)
 //   warps 4-7  : softmax + epilogue of tile A (one thread per query row)
 //   warps 8-11 : softmax + epilogue of tile B
 // A softmax thread holds a row of 128 scores; at the 168 registers that an even split leaves it spilled 50 - 110 bytes per
@@ -88,7 +89,7 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
   int* doc_smem = reinterpret_cast<int*>(bar_generic + 256);  // [2 tiles][2][128] key doc ids
   uint32_t* act = reinterpret_cast<uint32_t*>(bar_generic + 256 + 2048);  // active key tiles (one bit each)
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   // 1-D grid, query super-tile slowest: blocks are handed out in index order, so with a causal mask ALL the longest
   // rows (of every head and batch entry) start first and the short ones fill the tail of the last wave; the heads
@@ -152,8 +153,8 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
   if (warp < 4) {
     regs_give<REGS_ISSUE>();
     if (warp == 0) {
-      // ------------------------------------------------------------ TMA producers
-      if (lane == 0) {
+      // ------------------------------------------------------------ TMA producer of Q and K
+      if (elect_one()) {
         bool ok = true;
         int issued = 0;
         mbar_expect_tx(q_full, 2 * C::TILE_BYTES);
@@ -178,7 +179,10 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
           mbar_wait(q_full, 0, status, KF_ERR_WAIT_DRAIN);
           for (int j = max(0, issued - 2); j < issued; ++j) mbar_wait(k_full(j & 1), (j >> 1) & 1, status, KF_ERR_WAIT_DRAIN);
         }
-      } else if (lane == 1) {
+      }
+    } else if (warp == 2) {
+      // ------------------------------------------------------------ TMA producer of V
+      if (elect_one()) {
         bool ok = true;
         int issued = 0;
         int i = 0;
@@ -197,7 +201,7 @@ kf_attn_fwd2_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_con
       }
     } else if (warp == 1) {
       // ------------------------------------------------------------ MMA issuer
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t idesc_s = umma_idesc_bf16(BLK_M, BLK_N, false, false);
         constexpr uint32_t idesc_o = umma_idesc_bf16(BLK_M, HD, false, true);
         bool ok = mbar_wait(q_full, 0, status, KF_ERR_WAIT_FULL);

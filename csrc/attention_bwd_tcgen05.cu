@@ -130,7 +130,7 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   uint32_t* act = reinterpret_cast<uint32_t*>(bar_gen + 256 + 1024 + 512);  // active query tiles (one bit each)
   const uint32_t dq_stage = bar_base + AUX_BYTES;                   // only allocated when dq_tma
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   // grid: x = (batch, KV head), y = key tile.  Blocks are handed out x-fastest, so with a causal mask all the
   // heaviest key tiles (the earliest: every query sees them) start first and the lightest ones fill the tail.
@@ -199,7 +199,7 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       int issued = 0;
       mbar_expect_tx(kv_full, 2 * KV_TILE_BYTES);
@@ -233,7 +233,7 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_st = umma_idesc_bf16(128, BLK_Q, false, false);  // S^T, dP^T
       constexpr uint32_t idesc_acc = umma_idesc_bf16(128, HD, false, true);     // dV, dK (B = rows of Q_i / dO_i)
       constexpr uint32_t idesc_dq = umma_idesc_bf16(128, BLK_Q, true, true);    // dQ^T = K^T dS

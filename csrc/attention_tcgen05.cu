@@ -78,7 +78,7 @@ kf_attn_fwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   int* doc_smem = reinterpret_cast<int*>(bar_generic + 256);            // [2][128] key doc ids
   float* xch_smem = reinterpret_cast<float*>(bar_generic + 256 + 1024);  // [2][2][128] maxima, [2][128] sums
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int n_q_tiles = gridDim.x;
   const int qt = n_q_tiles - 1 - blockIdx.x;  // the longest (last) causal rows are scheduled first
@@ -188,7 +188,7 @@ kf_attn_fwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     grid_dep_wait();
     grid_dep_launch();
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(BLK_M, BLK_N, false, false);
       constexpr uint32_t idesc_o = umma_idesc_bf16(BLK_M, HD, false, true);
       bool ok = mbar_wait(q_full, 0, status, KF_ERR_WAIT_FULL);

@@ -67,7 +67,7 @@ kf_gemm_fp8_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid
   volatile uint32_t* tmem_slot_ptr =
       reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
@@ -104,7 +104,7 @@ kf_gemm_fp8_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (one per CTA)
-    if (lane == 0) {
+    if (elect_one()) {
       int it = 0;
       bool ok = true;
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
@@ -130,7 +130,7 @@ kf_gemm_fp8_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       const uint32_t idesc = idesc_f8(TILE_M, tile_n, a_fmt, b_fmt);
       int it = 0, tile_iter = 0;
       bool ok = true;

@@ -79,7 +79,7 @@ kf_gemm_skinny(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   float* red = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw)));
   constexpr int TMEM_COLS = NT < 32 ? 32 : NT;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int splits = int(cluster_nctaid()), rank = int(cluster_ctarank());
   const int tile = int(blockIdx.x) / splits;
   const int k_blocks = (a.K + BK - 1) / BK;
@@ -115,7 +115,7 @@ kf_gemm_skinny(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   bool ok = true;
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       auto load_w = [&](int i) {
         const int s = i % C::STAGES, k0 = (kb0 + i) * BK;
         const uint32_t dst = smem_base + s * C::STAGE;
@@ -154,7 +154,7 @@ kf_gemm_skinny(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     grid_dep_wait();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(WROWS, NT, false, false);
       for (int i = 0; i < n_kb; ++i) {
         const int s = i % C::STAGES;

@@ -71,7 +71,7 @@ kf_gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_con
   volatile uint32_t* tmem_slot_ptr =
       reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int m_blocks = (M + BM - 1) / BM;
   const int n_blocks = (N + BN - 1) / BN;
@@ -103,7 +103,7 @@ kf_gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_con
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int it = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
@@ -140,7 +140,7 @@ kf_gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_con
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, A_MN, B_MN);
       int it = 0, tile_iter = 0;
       bool ok = true;

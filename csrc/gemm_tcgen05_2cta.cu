@@ -172,7 +172,7 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
   const uint32_t tmem_slot = bar_base + 8u * (2 * STAGES + 5);
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
   const bool leader = rank == 0;
@@ -237,7 +237,7 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (one per CTA)
-    if (lane == 0) {
+    if (elect_one()) {
       int it = 0;
       bool ok = true;
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
@@ -290,7 +290,7 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       const uint32_t idesc = umma_idesc_bf16(TILE_M, tile_n, A_MN, B_MN);
       int it = 0, tile_iter = 0;
       bool ok = true;

@@ -100,7 +100,7 @@ kf_gemm_tokens_2cta(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   const uint32_t tmem_slot = bar_base + 8u * (2 * MAX_STAGES + 5);
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
   const bool leader = rank == 0;
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
@@ -142,7 +142,7 @@ kf_gemm_tokens_2cta(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (one per CTA)
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0, fills = 0;  // stage, and how many were filled altogether
       uint32_t phase = 0;
       bool ok = true;
@@ -183,7 +183,7 @@ kf_gemm_tokens_2cta(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       int s = 0, tile_iter = 0;
       uint32_t phase = 0;
       bool ok = true;

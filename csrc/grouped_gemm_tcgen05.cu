@@ -56,7 +56,7 @@ kf_grouped_gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(bar_gen + 8 * (2 * STAGES + 5));
   int* tile_start = reinterpret_cast<int*>(bar_gen + 256);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   constexpr int TN = SWIGLU ? BN / 2 : BN;  // output columns (hidden units) per tile
   const int n_blocks = (N + TN - 1) / TN;
   const int k_blocks = (K + BK - 1) / BK;
@@ -79,7 +79,7 @@ kf_grouped_gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_
   const int num_tiles = tile_start[E] * n_blocks;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int it = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
@@ -115,7 +115,7 @@ kf_grouped_gemm_tcgen05(const __grid_constant__ CUtensorMap map_a, const __grid_
         mbar_wait(full_bar(j % STAGES), (j / STAGES) & 1, status, KF_ERR_WAIT_DRAIN);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, false, B_MN);
       int it = 0, tile_iter = 0;
       bool ok = true;

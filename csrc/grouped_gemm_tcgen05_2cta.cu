@@ -70,7 +70,7 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(bar_gen + 8 * (2 * STAGES + 5));
   int* tile_start = reinterpret_cast<int*>(bar_gen + 256);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
   const bool leader = rank == 0;
   const int pair = blockIdx.x >> 1;
@@ -111,7 +111,7 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (one per CTA)
-    if (lane == 0) {
+    if (elect_one()) {
       int it = 0;
       bool ok = true;
       // the leader fetches the gate weights (or the first 128 columns), the peer the up weights (or the last 128)
@@ -154,7 +154,7 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(TILE_M, TILE_N, false, B_MN);
       int it = 0, tile_iter = 0;
       bool ok = true;

@@ -71,7 +71,7 @@ kf_grouped_wgrad_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const _
   const uint32_t tmem_slot = bar_base + 8u * (4 * STAGES + 5);
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
   const bool leader = rank == 0;
   const int pair = blockIdx.x >> 1;
@@ -108,7 +108,7 @@ kf_grouped_wgrad_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const _
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (one per CTA)
-    if (lane == 0) {
+    if (elect_one()) {
       int it = 0;
       uint32_t full_parity = 0, tail_parity = 0, last_tail = 0;  // bit s: next phases of stage s, kind of its last use
       bool ok = true;
@@ -151,7 +151,7 @@ kf_grouped_wgrad_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const _
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (leader && lane == 0) {
+    if (leader && elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(TILE_M, TILE_N, true, true);
       int it = 0, tile_iter = 0;
       uint32_t full_parity = 0, ready_parity = 0;  // bit s: parity of the next full / tail use of stage s
@@ -183,8 +183,6 @@ kf_grouped_wgrad_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const _
         }
         if (ok) commit_pair(tfull_bar(acc));
       }
-    }
-    if (leader && lane == 0) {
       // every MMA must have retired before either CTA gives up its shared or tensor memory
       asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(drain_bar)
                    : "memory");
