@@ -11,7 +11,7 @@
 //                                       the factor `scale` of dS is applied to the finished dK and dQ instead:
 //                                       1250 -> 1085 us at 2 x 4096 tokens, 32 heads)
 //   dV  += P^T  dO_i                     (A from TMEM, 128 x 128 accumulator, lives in TMEM for the whole CTA)
-//   dK  += dS^T Q_i                      (A from smem, 128 x 128 accumulator)
+//   dK  += dS^T Q_i                      (A from TMEM, 128 x 128 accumulator)
 //   dQ_i^T = K^T dS                      (128 head-dim rows x 64 queries; added to an fp32 dQ by a bulk reduction)
 //
 //   warp 0     : TMA producer (K, V once; Q_i / dO_i ring of three stages)
@@ -23,6 +23,14 @@
 //                cycles of an iteration)
 //   warps 6-9  : dQ reduction (TMEM -> shared-memory tile -> one cp.reduce.async.bulk.tensor add per tile;
 //                or, as a fallback mode, red.global.add.f32 per element)
+//
+// What bounds an iteration is the shared-memory port (128 bytes per clock).  The MMAs read their operands through it (176 KB: a
+// 128 x 64 tile of 16 k takes the 48 clocks of its 6 KB, not the 32 of its products), the copies of Q_i and dO_i write 32 KB, dS^T
+// 16 KB, and the fp32 dQ tile crosses it twice: 2300 clocks of the 2500 that one takes.  Hence dS^T comes from tensor memory for dK,
+// where it lies behind P^T of the same 32 queries in the columns of S^T that only their own warp has read; no warp has to wait for
+// another before it writes there.  The two halves of the queries synchronise apart (128 threads), so a scheduler's two warps drift
+// into different phases.  With the statistics fetched untouched (see fetch_stat), backward with its pre- and post-pass, us:
+// 2 x 4096 tokens, 32 query and 8 key heads of 128: 831 -> 779; 3000, 40 heads: 386 -> 363; 4 x 2048, 12 heads of 64: 230 -> 197.
 //
 // Head dim 64 adds nothing up in memory: each key tile writes its dQ tiles to a part of its own, and the post-pass adds the parts in
 // the order of the key tiles, so equal inputs give equal bits (the library's backward, which such models had before, repeats itself
@@ -121,12 +129,14 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   auto qdo_full = [&](int st) { return bar_base + 8u * (1 + st); };     // 3
   auto stage_free = [&](int st) { return bar_base + 8u * (4 + st); };   // 3
   auto ds_free = [&](int buf) { return bar_base + 8u * (7 + buf); };    // 2
-  const uint32_t sdp_full = bar_base + 8u * 9, ds_ready = bar_base + 8u * 10, mma_done = bar_base + 8u * 11,
+  // one per dS^T buffer: a warp may arrive for tile t + 1 before another has for t (but not for t + 2, whose scores wait for both)
+  auto ds_ready = [&](int buf) { return bar_base + 8u * (buf ? 17 : 10); };
+  const uint32_t sdp_full = bar_base + 8u * 9, mma_done = bar_base + 8u * 11,
                  dq_free = bar_base + 8u * 12, drain_bar = bar_base + 8u * 13, sdp_taken = bar_base + 8u * 14,
                  final_bar = bar_base + 8u * 15, tmem_slot = bar_base + 8u * 16;
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(bar_gen + 128);
-  float* stat_smem = reinterpret_cast<float*>(bar_gen + 256);       // [2][lse2 | D][64]
-  int* docq_smem = reinterpret_cast<int*>(bar_gen + 256 + 1024);    // [2][64]
+  float* stat_smem = reinterpret_cast<float*>(bar_gen + 256);       // [2][half][lse2 | D][32]
+  int* docq_smem = reinterpret_cast<int*>(bar_gen + 256 + 1024);    // [2][half][32]
   uint32_t* act = reinterpret_cast<uint32_t*>(bar_gen + 256 + 1024 + 512);  // active query tiles (one bit each)
   const uint32_t dq_stage = bar_base + AUX_BYTES;                   // only allocated when dq_tma
 
@@ -159,7 +169,8 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       mbar_init(stage_free(st), 1);
     }
     mbar_init(sdp_full, 1);
-    mbar_init(ds_ready, 8);
+    mbar_init(ds_ready(0), 8);
+    mbar_init(ds_ready(1), 8);
     mbar_init(mma_done, 1);
     mbar_init(dq_free, 4);
     mbar_init(sdp_taken, 8);
@@ -273,19 +284,20 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           if (!mbar_wait(sdp_taken, it & 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
           if (!issue_scores(it + 1)) { ok = false; break; }
         }
-        if (!mbar_wait(ds_ready, it & 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
+        if (!mbar_wait(ds_ready(buf), (it >> 1) & 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
         if (it > 0 && !mbar_wait(dq_free, (it - 1) & 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
         tc_fence_after();
-        // dV += P^T dO_i : A = P^T from TMEM (8 columns per 16 queries), B = dO_i rows (head dim contiguous)
+        // dV += P^T dO_i : A = P^T from TMEM (8 columns per 16 queries, the second half of the queries 32 columns on),
+        // B = dO_i rows (head dim contiguous)
 #pragma unroll
         for (int kk = 0; kk < BLK_Q / 16; ++kk)
-          tc_mma_f16_ts(tmem_base + DV_COL, tmem_base + ST_COL + buf * BLK_Q + kk * 8,
+          tc_mma_f16_ts(tmem_base + DV_COL, tmem_base + ST_COL + buf * BLK_Q + (kk >> 1) * (BLK_Q / 2) + (kk & 1) * 8,
                         umma_desc_sw128(dos + kk * 2048, Q_BLOCK_BYTES, 1024), idesc_acc, (it | kk) != 0);
-        // dK += dS^T Q_i : A = dS^T from smem (query dim contiguous), B = Q_i rows
+        // dK += dS^T Q_i : A = dS^T from TMEM (behind P^T of the same queries), B = Q_i rows
 #pragma unroll
         for (int kk = 0; kk < BLK_Q / 16; ++kk)
-          tc_mma_f16(tmem_base + DK_COL, umma_desc_sw128(dss + kk * 32, 16, 1024),
-                     umma_desc_sw128(qs + kk * 2048, Q_BLOCK_BYTES, 1024), idesc_acc, (it | kk) != 0);
+          tc_mma_f16_ts(tmem_base + DK_COL, tmem_base + ST_COL + buf * BLK_Q + (kk >> 1) * (BLK_Q / 2) + 16 + (kk & 1) * 8,
+                        umma_desc_sw128(qs + kk * 2048, Q_BLOCK_BYTES, 1024), idesc_acc, (it | kk) != 0);
         // dQ_i^T = K^T dS : A = K rows read with the head dim as M, B = dS^T rows read with the query dim as N.  With 64
         // head dims the upper half of M is whatever follows K in shared memory (V): those 64 lanes are never read.
 #pragma unroll
@@ -310,18 +322,20 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const int r_local = quarter * 32 + lane;  // key row of this thread
     const int kpos = k0 + r_local;
     const uint32_t t_lane = tmem_base + (uint32_t(quarter * 32) << 16);
-    const int t128 = half == 0 ? threadIdx.x - 64 : 128;   // the first group's 128 threads fetch the row statistics
+    const int t128 = quarter * 32 + lane;     // 0 .. 31 of a half fetch -lse (log2 units), 32 .. 63 -D, 64 .. 95 document ids
     int doc_k = 0;
     if (HAS_DOC) doc_k = kpos < Sk ? doc_ids[size_t(b) * Sk + kpos] : -2;
     bool ok = true;
-    // statistics of the 64 queries of iteration `t` (-lse in log2 units for threads 0..63, -D for 64..127), fetched one
-    // iteration ahead so that the global-memory latency hides under the arithmetic of the current tile
+    // the statistics of this half's queries of iteration `t`, fetched one iteration ahead so that the global-memory latency
+    // hides under the arithmetic of the current tile: as they lie in memory, because the first instruction that touches a loaded
+    // value waits for it (the factor applied here held every tile up by 800 cycles)
     auto fetch_stat = [&](int t, const Walk& w) -> float {
-      if (t128 >= 128 || t >= n_iter) return 0.f;
-      const int qq = w.i * BLK_Q + (t128 & 63);
+      if (t128 >= (HAS_DOC ? 96 : 64) || t >= n_iter) return 0.f;
+      const int qq = w.i * BLK_Q + half * HQ + lane;
       const size_t idx = (size_t(b) * H + w.head) * Sq + qq;
-      if (t128 < 64) return qq < Sq ? LSE[idx] * -1.4426950408889634f : -INFINITY;  // -inf -> P = 0 for padding rows
-      return qq < Sq ? -Dsum[idx] : 0.f;
+      if (t128 < 32) return qq < Sq ? LSE[idx] : INFINITY;  // P = 0 for padding rows
+      if (t128 < 64) return qq < Sq ? Dsum[idx] : 0.f;
+      return __int_as_float(qq < Sq ? doc_ids[size_t(b) * Sq + qq] : -1);
     };
     Walk ahead = walk_begin();
     float stat_next = fetch_stat(0, ahead);
@@ -329,16 +343,11 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     for (int it = 0; it < n_iter; ++it) {
       const int q0 = ahead.i * BLK_Q;
       ahead = walk_next(ahead);
-      float* stat = stat_smem + (it & 1) * 128;
-      int* dq_doc = docq_smem + (it & 1) * 64;
-      if (t128 < 128) {
-        stat[t128] = stat_next;
-        if (HAS_DOC && t128 < 64) {
-          const int qq = q0 + t128;
-          dq_doc[t128] = qq < Sq ? doc_ids[size_t(b) * Sq + qq] : -1;
-        }
-      }
-      group_sync(1, 256);
+      float* stat = stat_smem + ((it & 1) * 2 + half) * (2 * HQ);
+      int* dq_doc = docq_smem + ((it & 1) * 2 + half) * HQ;
+      if (t128 < 64) stat[t128] = stat_next * (t128 < 32 ? -1.4426950408889634f : -1.f);
+      else if (HAS_DOC && t128 < 96) dq_doc[lane] = __float_as_int(stat_next);
+      group_sync(half == 0 ? 1 : 3, 128);  // the halves run apart: a scheduler holds one warp of each
       stat_next = fetch_stat(it + 1, ahead);
       if (ok && !mbar_wait(sdp_full, it & 1, status, KF_ERR_WAIT_TMEM_FULL)) ok = false;
       tc_fence_after();
@@ -350,16 +359,13 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(sdp_taken);  // dP^T is in registers: the next tile's dP^T may be computed
-      // P^T overwrites the first 32 columns of S^T: nobody may store before both warps of a key-row quarter have
-      // loaded their scores
-      group_sync(3, 256);
       const bool tile_masked = HAS_DOC || (CAUSAL && q0 < k0 + BLK_K - 1) || (k0 + BLK_K > Sk) || (q0 + BLK_Q > Sq);
       uint32_t pk[HQ / 2], dsk[HQ / 2];
 #pragma unroll
       for (int i4 = 0; i4 < HQ / 4; ++i4) {
         // four queries per step: their -lse / -D come as two 16-byte broadcast reads of two pairs each
-        const ulonglong2 l4 = *reinterpret_cast<const ulonglong2*>(stat + half * HQ + 4 * i4);
-        const ulonglong2 d4 = *reinterpret_cast<const ulonglong2*>(stat + 64 + half * HQ + 4 * i4);
+        const ulonglong2 l4 = *reinterpret_cast<const ulonglong2*>(stat + 4 * i4);
+        const ulonglong2 d4 = *reinterpret_cast<const ulonglong2*>(stat + HQ + 4 * i4);
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           const int c = 4 * i4 + 2 * u;       // index inside this thread's half
@@ -375,8 +381,8 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
               v1 = v1 && kpos <= qpos + 1;
             }
             if (HAS_DOC) {
-              v0 = v0 && dq_doc[half * HQ + c] == doc_k;
-              v1 = v1 && dq_doc[half * HQ + c + 1] == doc_k;
+              v0 = v0 && dq_doc[c] == doc_k;
+              v1 = v1 && dq_doc[c + 1] == doc_k;
             }
             p0 = v0 ? p0 : 0.f;
             p1 = v1 ? p1 : 0.f;
@@ -387,8 +393,10 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           dsk[2 * i4 + u] = pack_bf16(s0, s1);
         }
       }
-      // P^T over the start of S^T (bf16 pairs: 16 columns per 32 queries)
-      tmem_st_32x16(t_s + half * (HQ / 2), pk);
+      // P^T over the start of this half of S^T (bf16 pairs: 16 columns for 32 queries), which this warp alone has read
+      // and dS^T behind it
+      tmem_st_32x16(t_s + half * HQ, pk);
+      tmem_st_32x16(t_s + half * HQ + HQ / 2, dsk);
       // dS^T into shared memory, 128B-swizzled rows (16-byte chunk c of row r lives at chunk c ^ (r % 8));
       // the previous iteration's dK / dQ MMAs must have finished reading it
       // (two buffers: the MMAs of iteration it-2 were the last readers of this one)
@@ -405,7 +413,7 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(ds_ready);
+      if (lane == 0) mbar_arrive(ds_ready(it & 1));
     }
     // ---- epilogue: dK / dV accumulators -> bf16 rows of the key tile (first softmax group: one thread per key row)
     if (half != 0) ok = false;
