@@ -12,8 +12,8 @@
 //   full 64-row blocks   as in gemm_tcgen05_2cta.cu: both CTAs' TMA bytes are counted on the leader's full[s]
 //   the tail block       (at most one per tile) each CTA's loads complete on its own tail[s]; warp 6 of each CTA waits
 //                        for it, zeroes the foreign rows of its own stage up to the next multiple of 16 (only those
-//                        k-steps are issued), fences them towards the async proxy and arrives (release) on the leader's
-//                        ready[s]; the issuing thread waits for both arrivals (cluster-scope acquire) before the MMAs.
+//                        k-steps are issued), fences them towards the async proxy and arrives on the leader's
+//                        ready[s]; the issuing thread waits for both arrivals before the MMAs.
 //                        The ring runs ahead of the MMAs, so the rows are usually clear before their turn; zeroing all
 //                        64 rows inside the issuing warp held up every tile by about as long as a k-block (64 experts of
 //                        2048 x 1408 over 10 662 rows: 484 -> 397 us for three gradients; 8 of 2048 x 7168: 464 -> 414).
@@ -28,8 +28,12 @@
 // way out, not its products, sets the pace.  With one row per thread every 16-byte store of a warp touched 32 different
 // lines: 5.5 us per tile.  Each epilogue warp therefore stages 32 rows x 64 columns in shared memory (two 4 KB buffers,
 // 128-byte swizzle: no bank conflicts) and one lane stores them with TMA: whole lines, asynchronously, clipped at the
-// expert's last row and column by the 3-D tensor map.  The sixth ring stage paid for the buffers.  Three gradients of 64 experts of
-// 2048 x 1408 over 10 662 rows: 685 -> 480 us with this; of 8 experts of 2048 x 7168 over 4096 rows: 530 -> 441 us.
+// expert's last row and column by the 3-D tensor map.  Three gradients of 64 experts of 2048 x 1408 over 10 662 rows: 685 -> 480 us
+// with this; of 8 experts of 2048 x 7168 over 4096 rows: 530 -> 441 us.
+//
+// What held such short tiles up after that was synchronisation: arrivals that waited for the warp's stores (see arrive_on_cta), row
+// offsets read from global memory by every role of every tile (400 clocks each), and the cleared rows' addresses.  The three
+// gradients, 64 experts: 417 -> 304 us (3.7 TB/s of gradients written); 8 experts: 374 -> 304 us (1190 TFLOP/s), sixth stage included.
 //
 // Replaces the per-expert weight-gradient products that autograd derives for the padded `torch._grouped_mm`
 // call of the reference (kempnerforge/model/moe.py:20-145).
@@ -43,19 +47,20 @@ namespace gwg2 {
 
 using namespace kf::pairops;
 
-constexpr int CTA_M = 128, TILE_M = 256, TILE_N = 256, HALF_N = 128, BK = 64, STAGES = 5, UMMA_K = 16;
+constexpr int CTA_M = 128, TILE_M = 256, TILE_N = 256, HALF_N = 128, BK = 64, STAGES = 6, UMMA_K = 16;
 constexpr int BLOCK_BYTES = 64 * BK * 2;  // one {64 columns, BK rows} box
 constexpr int A_BYTES = (CTA_M / 64) * BLOCK_BYTES, B_BYTES = (HALF_N / 64) * BLOCK_BYTES;
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int THREADS = 224, TMEM_COLS = 512;
 constexpr int OUT_BYTES = 32 * 64 * 2;  // one staged box: 32 rows x 64 columns of one epilogue warp
-constexpr size_t SMEM = size_t(STAGES) * STAGE_BYTES + 4 * 2 * OUT_BYTES + 1024 + 256;
+constexpr int MAX_TABLE = 256;           // up to so many experts the row offsets are kept in shared memory
+constexpr size_t SMEM = size_t(STAGES) * STAGE_BYTES + 4 * 2 * OUT_BYTES + 1024 + 256 + (MAX_TABLE + 1) * 4;
 
 using Tile = tilemath::WgradTile;
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 kf_grouped_wgrad_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                              const __grid_constant__ CUtensorMap map_o, const int* __restrict__ offsets, int E, int M, int N,
+                              const __grid_constant__ CUtensorMap map_o, const int* __restrict__ row_offsets, int E, int M, int N,
                               int* status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -79,6 +84,11 @@ kf_grouped_wgrad_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const _
   const int m_blocks = (M + TILE_M - 1) / TILE_M, n_blocks = (N + TILE_N - 1) / TILE_N;
   const int num_tiles = E * m_blocks * n_blocks;
 
+  // Every role of every tile looks its expert's rows up; from global memory that held each of them up by 400 clocks.
+  int* table = reinterpret_cast<int*>(smem_raw + (bar_base + 256 - smem_u32(smem_raw)));
+  const int* offsets = E <= MAX_TABLE ? table : row_offsets;
+  if (E <= MAX_TABLE)
+    for (int i = threadIdx.x; i <= E; i += THREADS) table[i] = row_offsets[i];
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full_bar(s), 1);
@@ -201,12 +211,11 @@ kf_grouped_wgrad_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const _
         const int s = (it + k_blocks - 1) % STAGES;
         if (!__all_sync(0xffffffffu, mbar_wait(tail_bar(s), (tail_parity >> s) & 1, status, KF_ERR_WAIT_FULL))) break;
         tail_parity ^= 1u << s;
-        constexpr int BLOCKS = STAGE_BYTES / BLOCK_BYTES;
+        static_assert(STAGE_BYTES == 4 * BLOCK_BYTES, "a lane owns one 16-byte chunk of the rows of one of four blocks");
         const int end = (valid + UMMA_K - 1) / UMMA_K * UMMA_K;  // rows the MMAs will read
-        for (int i = lane; i < tilemath::tail_chunks(valid, end, BLOCKS); i += 32) {
-          const uint32_t addr = smem_base + s * STAGE_BYTES + tilemath::tail_chunk_offset(i, valid, end, BLOCK_BYTES);
-          asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(0u) : "memory");
-        }
+        const uint32_t chunk = smem_base + s * STAGE_BYTES + (lane >> 3) * BLOCK_BYTES + (lane & 7) * 16;
+        for (int r = valid; r < end; ++r)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(chunk + r * 128), "r"(0u) : "memory");
         fence_async_smem();
         __syncwarp();
         if (lane == 0) arrive_on_cta(ready_bar(s), 0);  // this CTA's half of the stage is in place

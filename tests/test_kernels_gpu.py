@@ -569,6 +569,36 @@ def test_grouped_wgrad_matches_per_expert_products(native_lib, counts, grouped_t
         start += c
 
 
+@pytest.mark.parametrize("experts", [255, 256, 257, 600])
+def test_grouped_wgrad_of_many_experts_with_ragged_tails(native_lib, experts):
+    """Row ranges kept in shared memory (up to 256 experts) and read where they are; every tail of a block of 16 rows, next to rows of
+    NaN that must have been cleared before the product reads them, the same bits each time."""
+    torch.manual_seed(0)
+    m, n = 72, 264
+    counts = [(i * 7) % 33 for i in range(experts)]
+    rows = sum(counts)
+    a, b = _rand(rows, m), _rand(rows, n)
+    offsets = torch.zeros(experts + 1, dtype=torch.int32, device="cuda")
+    offsets[1:] = torch.tensor(counts, device="cuda").cumsum(0)
+    expert = torch.repeat_interleave(torch.arange(experts, device="cuda"), torch.tensor(counts, device="cuda"))
+    want = torch.zeros(experts, m, n, device="cuda")
+    for e in range(experts):
+        want[e] = a[expert == e].float().t() @ b[expert == e].float()
+    # bf16 products of up to 32 rows in fp32, one rounding: 2^-9 of the value and of what cancels in its sum
+    bound = torch.zeros(experts, m, n, device="cuda")
+    for e in range(experts):
+        bound[e] = (a[expert == e].float().abs().t() @ b[expert == e].float().abs()) * 2**-20 + want[e].abs() * 2**-8
+    first = native_lib.grouped_wgrad(a, b, offsets)
+    assert ((first.float() - want).abs() <= bound).all()
+    odd = (expert % 2 == 1)[:, None]
+    nan = float("nan")
+    a2, b2 = a.masked_fill(odd, nan), b.masked_fill(odd, nan)   # every second expert's rows, which follow another's tail
+    for _ in range(8):
+        got = native_lib.grouped_wgrad(a2, b2, offsets)
+        assert torch.equal(got[0::2], first[0::2])
+    assert native_lib.read_status() == 0
+
+
 # --------------------------------------------------------------------------- Newton-Schulz on the tensor cores
 @pytest.mark.parametrize("shape", [(256, 256), (128, 512), (512, 128), (1024, 384), (64, 4096)])
 def test_newton_schulz_matches_the_fp32_formulation_for_wide_and_tall_matrices(native_lib, shape):
