@@ -2,7 +2,10 @@
 //
 //   kf_router_topk      one warp per token: softmax or sigmoid(+bias) over the expert logits, top-k by repeated
 //                       warp arg-max, renormalised weights, per-expert token counts, per-expert probability sums
-//                       (load-balancing loss) and the sum of logsumexp^2 (router z-loss) in one pass.
+//                       (load-balancing loss) and the sum of logsumexp^2 (router z-loss) in one pass.  What a layer makes
+//                       of them (means, the balancing loss, weights in bf16, a private copy of the bias) leaves the same
+//                       launch: as tensor operations on a few hundred values these were nine launches of 2 us forward
+//                       and nine backward, each of which costs the host 5 to 15 us.
 //   kf_moe_sort_*       stable counting sort of the (token, k) assignments by expert: per-block histograms,
 //                       a scan, then ranks -> `row_of_slot` (destination row of every assignment),
 //                       `slot_of_row` (its inverse) and the expert offsets the grouped GEMM consumes.
@@ -27,11 +30,31 @@ __device__ __forceinline__ float to_f<float>(float v) { return v; }
 template <>
 __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
+// fp32 or bf16 (`half`), or none.
+struct RouterBias {
+  const void* p;
+  int half;
+  __device__ __forceinline__ float at(int e) const {
+    return p == nullptr ? 0.f : half ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[e]) : reinterpret_cast<const float*>(p)[e];
+  }
+};
+
+// What the router leaves beside the choice: counts [E], mean scores [E], mean logsumexp^2, and for softmax scores the balancing loss
+// E sum_e (counts_e / (tokens k)) mean_e (else 0).  keep [E]: what the backward reads and the program may change in the meantime,
+// the bias as it was (sigmoid) or the counts (softmax).  The block that finishes last writes them from acc: counts [E], sums of the
+// scores [E], of logsumexp^2 [1], finished blocks [1], zeros on entry.
+struct RouterStats {
+  float *counts, *mean, *z, *balance, *keep, *acc;
+};
+
+// w_half (optional): the weights rounded to bf16.
 template <typename T, bool SIGMOID>
 __global__ void __launch_bounds__(256)
-kf_router_topk(const T* __restrict__ logits, const float* __restrict__ bias, int tokens, int E, int k,
-               long long* __restrict__ idx_out, float* __restrict__ w_out, float* __restrict__ counts,
-               float* __restrict__ prob_sum, float* __restrict__ lse_sq_sum) {
+kf_router_topk(const T* __restrict__ logits, RouterBias bias, int tokens, int E, int k, long long* __restrict__ idx_out,
+               float* __restrict__ w_out, __nv_bfloat16* __restrict__ w_half, RouterStats out) {
+  float *counts = out.acc, *prob_sum = counts + E, *lse_sq_sum = counts + 2 * E;
+  if (SIGMOID && blockIdx.x == 0)
+    for (int e = threadIdx.x; e < E; e += blockDim.x) out.keep[e] = bias.at(e);
   extern __shared__ float sh[];  // [E] probability sums of this block, [E] counts
   float* sh_prob = sh;
   float* sh_cnt = sh + E;
@@ -63,7 +86,7 @@ kf_router_topk(const T* __restrict__ logits, const float* __restrict__ bias, int
       const int e = lane + 32 * j;
       if (e < E) {
         if (SIGMOID) {
-          score[j] = 1.f / (1.f + __expf(-(raw[j] + (bias ? bias[e] : 0.f))));
+          score[j] = 1.f / (1.f + __expf(-(raw[j] + bias.at(e))));
         } else {
           score[j] = __expf(raw[j] - mx) / se;
         }
@@ -109,6 +132,7 @@ kf_router_topk(const T* __restrict__ logits, const float* __restrict__ bias, int
         if (r < k) {
           idx_out[size_t(t) * k + r] = isel[r];
           w_out[size_t(t) * k + r] = wsel[r] * inv;
+          if (w_half) w_half[size_t(t) * k + r] = __float2bfloat16(wsel[r] * inv);
           atomicAdd(&sh_cnt[isel[r]], 1.f);
         }
       }
@@ -122,6 +146,29 @@ kf_router_topk(const T* __restrict__ logits, const float* __restrict__ bias, int
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) zacc += __shfl_xor_sync(0xffffffffu, zacc, o);
   if (lane == 0 && zacc != 0.f) atomicAdd(lse_sq_sum, zacc);
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(reinterpret_cast<int*>(out.acc + 2 * E + 1), 1) == int(gridDim.x) - 1;
+  __syncthreads();
+  if (!last || threadIdx.x >= 32) return;
+  __threadfence();
+  float loss = 0.f;
+  for (int e = lane; e < E; e += 32) {
+    const float mean = __fdiv_rn(__ldcg(prob_sum + e), float(tokens)), count = __ldcg(counts + e);
+    if (!SIGMOID) {
+      out.keep[e] = count;
+      loss += __fdiv_rn(count, float(tokens) * float(k)) * mean;
+    }
+    out.counts[e] = count;
+    out.mean[e] = mean;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+  if (lane == 0) {
+    *out.z = __fdiv_rn(__ldcg(lse_sq_sum), float(tokens));
+    *out.balance = float(E) * loss;
+  }
 }
 
 // ------------------------------------------------------------------ backward of the router
@@ -132,6 +179,7 @@ kf_router_topk(const T* __restrict__ logits, const float* __restrict__ bias, int
 //   mean_e = sum_t s_te / T   ->  ds_e += dmean_e / T
 //   s = sigmoid(l + b)        ->  dl = ds s (1 - s);      s = softmax(l)  ->  dl = s (ds - sum_e ds_e s_e)
 //   z = sum_t lse_t^2 / T     ->  dl += 2 dz / T lse softmax(l)
+//   balance = E sum_e (counts_e / (T k)) mean_e   ->  dmean_e += dbalance E counts_e / (T k)
 // partial (optional, [gridDim.x][E]): this block's sum of the unrounded dl over its tokens (the bias gradient).
 //
 // The scores are recomputed with correctly rounded divisions and with exponentials and logarithms in 64 bits: the fast forms (and
@@ -144,8 +192,15 @@ __device__ __forceinline__ float log_f32(float x) { return float(log(double(x)))
 template <typename T, bool SIGMOID>
 __global__ void __launch_bounds__(256)
 kf_router_bwd(const T* __restrict__ logits, const float* __restrict__ bias, const long long* __restrict__ idx,
-              const float* __restrict__ w, const float* __restrict__ dw, const float* __restrict__ dmean,
-              const float* __restrict__ dz, int tokens, int E, int k, T* __restrict__ dlogits, float* __restrict__ partial) {
+              const float* __restrict__ w, const void* __restrict__ dw_any, int dw_half, const float* __restrict__ dmean,
+              const float* __restrict__ dz, const float* __restrict__ dbalance, const float* __restrict__ counts, int tokens, int E,
+              int k, T* __restrict__ dlogits, float* __restrict__ partial) {
+  auto dw = [&](size_t i) {
+    return dw_any == nullptr ? 0.f
+           : dw_half         ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(dw_any)[i])
+                             : reinterpret_cast<const float*>(dw_any)[i];
+  };
+  const float balance = dbalance ? __fdiv_rn(dbalance[0] * float(E), float(tokens) * float(k)) : 0.f;
   extern __shared__ float sh[];  // [warps][E] sums of dl
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   float* mine = sh + warp * E;
@@ -183,6 +238,7 @@ kf_router_bwd(const T* __restrict__ logits, const float* __restrict__ bias, cons
       if (e < E) {
         sc[j] = SIGMOID ? __fdiv_rn(1.f, 1.f + exp_f32(-(raw[j] + (bias ? bias[e] : 0.f)))) : __fdiv_rn(ex[j], se);
         ds[j] = dmean ? dmean[e] * inv_t : 0.f;
+        if (balance != 0.f) ds[j] += balance * counts[e] * inv_t;
       }
     }
     // selected experts: sum of their scores, and <dw, w>
@@ -194,7 +250,7 @@ kf_router_bwd(const T* __restrict__ logits, const float* __restrict__ bias, cons
 #pragma unroll
         for (int j = 0; j < MAX_E_PER_LANE; ++j)
           if (lane + 32 * j == e) ssum += sc[j];
-        dot += dw[size_t(t) * k + r] * w[size_t(t) * k + r];
+        dot += dw(size_t(t) * k + r) * w[size_t(t) * k + r];
       }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, o);
@@ -202,7 +258,7 @@ kf_router_bwd(const T* __restrict__ logits, const float* __restrict__ bias, cons
     for (int r = 0; r < MAX_K; ++r)
       if (r < k) {
         const int e = (int)idx[size_t(t) * k + r];
-        const float d = __fdiv_rn(dw[size_t(t) * k + r] - dot, ssum);
+        const float d = __fdiv_rn(dw(size_t(t) * k + r) - dot, ssum);
 #pragma unroll
         for (int j = 0; j < MAX_E_PER_LANE; ++j)
           if (lane + 32 * j == e) ds[j] += d;
@@ -235,8 +291,8 @@ kf_router_bwd(const T* __restrict__ logits, const float* __restrict__ bias, cons
   }
 }
 
-// out[e] = sum over the blocks of partial[b][e] (fixed order)
-__global__ void __launch_bounds__(256) kf_router_bias_grad(const float* __restrict__ partial, int blocks, int E, float* __restrict__ out) {
+// out[e] = sum over the blocks of partial[b][e] (fixed order), in fp32 or bf16
+__global__ void __launch_bounds__(256) kf_router_bias_grad(const float* __restrict__ partial, int blocks, int E, void* __restrict__ out, int half) {
   const int e = blockIdx.x, lane = threadIdx.x & 31;
   __shared__ float red[8];
   float v = 0.f;
@@ -248,7 +304,8 @@ __global__ void __launch_bounds__(256) kf_router_bias_grad(const float* __restri
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int i = 1; i < 8; ++i) v += red[i];
-    out[e] = v;
+    if (half) reinterpret_cast<__nv_bfloat16*>(out)[e] = __float2bfloat16(v);
+    else reinterpret_cast<float*>(out)[e] = v;
   }
 }
 
@@ -358,9 +415,11 @@ __global__ void kf_moe_gather(const __nv_bfloat16* __restrict__ src, const int* 
   }
 }
 
-// out[t] = sum_j w[t, j] * y[row_of_slot[t * k + j]]   (w == nullptr: plain sum, the gradient of the gather)
+// out[t] = sum_j w[t, j] * y[row_of_slot[t * k + j]] (+ plus[t])   (w == nullptr: plain sum, the gradient of the gather)
+template <typename W>
 __global__ void kf_moe_combine(const __nv_bfloat16* __restrict__ y, const int* __restrict__ row_of_slot,
-                               const float* __restrict__ w, int tokens, int k, int cols, __nv_bfloat16* __restrict__ out) {
+                               const W* __restrict__ w, const __nv_bfloat16* __restrict__ plus, int tokens, int k, int cols,
+                               __nv_bfloat16* __restrict__ out) {
   const int vec = cols / 8;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)tokens * vec;
        i += (long long)gridDim.x * blockDim.x) {
@@ -368,11 +427,18 @@ __global__ void kf_moe_combine(const __nv_bfloat16* __restrict__ y, const int* _
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int j = 0; j < k; ++j) {
       const int row = row_of_slot[size_t(t) * k + j];
-      const float wj = w ? w[size_t(t) * k + j] : 1.f;
+      const float wj = w ? to_f<W>(w[size_t(t) * k + j]) : 1.f;
       const uint4 v = *reinterpret_cast<const uint4*>(y + size_t(row) * cols + c);
       const float2 a = unpack_bf16(v.x), b = unpack_bf16(v.y), cc = unpack_bf16(v.z), d = unpack_bf16(v.w);
       acc[0] += wj * a.x; acc[1] += wj * a.y; acc[2] += wj * b.x; acc[3] += wj * b.y;
       acc[4] += wj * cc.x; acc[5] += wj * cc.y; acc[6] += wj * d.x; acc[7] += wj * d.y;
+    }
+    if (plus) {  // the sum over the experts is rounded first, like an addition of two tensors
+      const uint4 v = *reinterpret_cast<const uint4*>(plus + size_t(t) * cols + c);
+      const float2 a = unpack_bf16(v.x), b = unpack_bf16(v.y), cc = unpack_bf16(v.z), d = unpack_bf16(v.w);
+      const float p[8] = {a.x, a.y, b.x, b.y, cc.x, cc.y, d.x, d.y};
+#pragma unroll
+      for (int i8 = 0; i8 < 8; ++i8) acc[i8] = __bfloat162float(__float2bfloat16(acc[i8])) + p[i8];
     }
     uint4 o;
     o.x = pack_bf16(acc[0], acc[1]); o.y = pack_bf16(acc[2], acc[3]);
@@ -382,15 +448,16 @@ __global__ void kf_moe_combine(const __nv_bfloat16* __restrict__ y, const int* _
 }
 
 // backward of the combine, one warp per sorted row: dy[row] = w[slot] * dout[token],  dw[slot] = <dout[token], y[row]>
+template <typename W>
 __global__ void kf_moe_combine_bwd(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ y,
-                                   const int* __restrict__ slot_of_row, const float* __restrict__ w, int rows, int k, int cols,
-                                   __nv_bfloat16* __restrict__ dy, float* __restrict__ dw) {
+                                   const int* __restrict__ slot_of_row, const W* __restrict__ w, int rows, int k, int cols,
+                                   __nv_bfloat16* __restrict__ dy, W* __restrict__ dw) {
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
     const int slot = slot_of_row[r];
     const int tok = slot / k;
-    const float ws = w[slot];
+    const float ws = to_f<W>(w[slot]);
     float dot = 0.f;
     for (int c = lane * 8; c < cols; c += 256) {
       const uint4 g = *reinterpret_cast<const uint4*>(dout + size_t(tok) * cols + c);
@@ -405,7 +472,10 @@ __global__ void kf_moe_combine_bwd(const __nv_bfloat16* __restrict__ dout, const
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-    if (lane == 0) dw[slot] = dot;
+    if (lane == 0) {
+      if constexpr (sizeof(W) == 2) dw[slot] = __float2bfloat16(dot);
+      else dw[slot] = dot;
+    }
   }
 }
 
@@ -414,41 +484,45 @@ __global__ void kf_moe_combine_bwd(const __nv_bfloat16* __restrict__ dout, const
 
 extern "C" {
 
-// logits [tokens][E] (dt 0 = bf16, 1 = fp32); bias fp32 [E] or null (sigmoid mode); outputs: idx int64 [tokens][k],
-// w fp32 [tokens][k] (renormalised), and ACCUMULATED into: counts fp32 [E], prob_sum fp32 [E], lse_sq_sum fp32 [1]
-// (zero them first).  E <= 256, k <= 8.
-int kf_router_topk(const void* logits, int dt, const void* bias, int sigmoid, int tokens, int E, int k, void* idx, void* w,
-                   void* counts, void* prob_sum, void* lse_sq_sum, void* stream) {
+// logits [tokens][E] (dt 0 = bf16, 1 = fp32); bias [E] fp32 or (bias_half) bf16 or null (sigmoid mode);
+// outputs: idx int64 [tokens][k], w fp32 [tokens][k] (renormalised), w_half bf16 [tokens][k] or null, keep fp32 [E] for the
+// backward (the bias, or zeros, with sigmoid scores; the counts with softmax), counts and mean scores fp32 [E], mean logsumexp^2 and
+// balancing loss fp32 [1].  acc: fp32 [2 E + 2] of scratch.  E <= 256, k <= 8.
+int kf_router_topk(const void* logits, int dt, const void* bias, int bias_half, int sigmoid, int tokens, int E, int k, void* idx, void* w,
+                   void* w_half, void* keep, void* counts, void* mean, void* z, void* balance, void* acc, void* stream) {
   using namespace kf::moe;
   if (E < 1 || E > 32 * MAX_E_PER_LANE || k < 1 || k > MAX_K || k > E) return 3;
+  cudaStream_t st = (cudaStream_t)stream;
   if (tokens <= 0) return 0;
+  cudaError_t e = cudaMemsetAsync(acc, 0, (2 * size_t(E) + 2) * sizeof(float), st);
+  if (e != cudaSuccess) return 350 + (int)e;
   const int threads = 256, wpb = threads / 32;
   int blocks = (tokens + wpb - 1) / wpb;
   if (blocks > 1184) blocks = 1184;
   const size_t sh = 2 * size_t(E) * sizeof(float);
-  cudaStream_t st = (cudaStream_t)stream;
+  const RouterBias rb{bias, bias_half};
+  const RouterStats rs{(float*)counts, (float*)mean, (float*)z, (float*)balance, (float*)keep, (float*)acc};
 #define KF_ROUTER(T_, S_)                                                                                              \
-  kf_router_topk<T_, S_><<<blocks, threads, sh, st>>>(reinterpret_cast<const T_*>(logits),                              \
-                                                      reinterpret_cast<const float*>(bias), tokens, E, k,               \
+  kf_router_topk<T_, S_><<<blocks, threads, sh, st>>>(reinterpret_cast<const T_*>(logits), rb, tokens, E, k,            \
                                                       reinterpret_cast<long long*>(idx), reinterpret_cast<float*>(w),   \
-                                                      reinterpret_cast<float*>(counts), reinterpret_cast<float*>(prob_sum), \
-                                                      reinterpret_cast<float*>(lse_sq_sum))
+                                                      reinterpret_cast<__nv_bfloat16*>(w_half), rs)
   if (dt == 0) {
     if (sigmoid) KF_ROUTER(__nv_bfloat16, true); else KF_ROUTER(__nv_bfloat16, false);
   } else {
     if (sigmoid) KF_ROUTER(float, true); else KF_ROUTER(float, false);
   }
 #undef KF_ROUTER
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
-// Gradient of the logits of kf_router_topk.  w, dw fp32 [tokens][k]; dmean fp32 [E], dz fp32 [1] (each may be null);
-// dlogits in the type of the logits.  dbias (optional, fp32 [E], with partial fp32 [KF_ROUTER_BWD_BLOCKS = 592][E] scratch):
+// Gradient of the logits of kf_router_topk.  w fp32 [tokens][k], dw fp32 or (dw_half) bf16 [tokens][k]; dmean fp32 [E], dz fp32 [1],
+// dbalance fp32 [1] with counts fp32 [E] (each gradient may be null); dlogits in the type of the logits.  dbias (optional,
+// [E] fp32 or, dbias_half, bf16, with partial fp32 [KF_ROUTER_BWD_BLOCKS = 592][E] scratch):
 // the sum of dlogits over the tokens.
-int kf_router_bwd(const void* logits, int dt, const void* bias, int sigmoid, const void* idx, const void* w, const void* dw,
-                  const void* dmean, const void* dz, int tokens, int E, int k, void* dlogits, void* dbias, void* partial,
-                  void* stream) {
+int kf_router_bwd(const void* logits, int dt, const void* bias, int sigmoid, const void* idx, const void* w, const void* dw, int dw_half,
+                  const void* dmean, const void* dz, const void* dbalance, const void* counts, int tokens, int E, int k, void* dlogits,
+                  void* dbias, int dbias_half, void* partial, void* stream) {
   using namespace kf::moe;
   if (E < 1 || E > 32 * MAX_E_PER_LANE || k < 1 || k > MAX_K || k > E || (dbias && !partial)) return 3;
   cudaStream_t st = (cudaStream_t)stream;
@@ -458,8 +532,9 @@ int kf_router_bwd(const void* logits, int dt, const void* bias, int sigmoid, con
 #define KF_ROUTER_BWD(T_, S_)                                                                                           \
   kf_router_bwd<T_, S_><<<blocks, 256, dbias ? 8 * size_t(E) * sizeof(float) : 0, st>>>(                                \
       reinterpret_cast<const T_*>(logits), reinterpret_cast<const float*>(bias), reinterpret_cast<const long long*>(idx), \
-      reinterpret_cast<const float*>(w), reinterpret_cast<const float*>(dw), reinterpret_cast<const float*>(dmean),     \
-      reinterpret_cast<const float*>(dz), tokens, E, k, reinterpret_cast<T_*>(dlogits),                                 \
+      reinterpret_cast<const float*>(w), dw, dw_half, reinterpret_cast<const float*>(dmean),                            \
+      reinterpret_cast<const float*>(dz), reinterpret_cast<const float*>(dbalance),                                     \
+      reinterpret_cast<const float*>(counts), tokens, E, k, reinterpret_cast<T_*>(dlogits),                             \
       dbias ? reinterpret_cast<float*>(partial) : nullptr)
   if (dt == 0) {
     if (sigmoid) KF_ROUTER_BWD(__nv_bfloat16, true); else KF_ROUTER_BWD(__nv_bfloat16, false);
@@ -468,7 +543,7 @@ int kf_router_bwd(const void* logits, int dt, const void* bias, int sigmoid, con
   }
 #undef KF_ROUTER_BWD
   if (dbias)
-    kf_router_bias_grad<<<E, 256, 0, st>>>(reinterpret_cast<const float*>(partial), blocks, E, reinterpret_cast<float*>(dbias));
+    kf_router_bias_grad<<<E, 256, 0, st>>>(reinterpret_cast<const float*>(partial), blocks, E, dbias, dbias_half);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
@@ -507,31 +582,38 @@ int kf_moe_gather_bf16(const void* src, const void* slot_of_row, int rows, int k
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
-int kf_moe_combine_bf16(const void* y, const void* row_of_slot, const void* w, int tokens, int k, int cols, void* out,
-                        void* stream) {
+// w: [tokens][k] fp32 or (w_half) bf16, or null; plus: bf16 [tokens][cols] added to the sum, or null.
+int kf_moe_combine_bf16(const void* y, const void* row_of_slot, const void* w, int w_half, const void* plus, int tokens, int k, int cols,
+                        void* out, void* stream) {
   using namespace kf::moe;
   if (cols & 7) return 5;
   if (tokens <= 0) return 0;
   long long work = (long long)tokens * (cols / 8);
   int blocks = (int)((work + 255) / 256 < 2368 ? (work + 255) / 256 : 2368);
-  kf_moe_combine<<<blocks, 256, 0, (cudaStream_t)stream>>>(reinterpret_cast<const __nv_bfloat16*>(y),
-                                                         reinterpret_cast<const int*>(row_of_slot),
-                                                         reinterpret_cast<const float*>(w), tokens, k, cols,
-                                                         reinterpret_cast<__nv_bfloat16*>(out));
+#define KF_COMBINE(W_)                                                                                                        \
+  kf_moe_combine<W_><<<blocks, 256, 0, (cudaStream_t)stream>>>(                                                               \
+      reinterpret_cast<const __nv_bfloat16*>(y), reinterpret_cast<const int*>(row_of_slot), reinterpret_cast<const W_*>(w),   \
+      reinterpret_cast<const __nv_bfloat16*>(plus), tokens, k, cols, reinterpret_cast<__nv_bfloat16*>(out))
+  if (w && w_half) KF_COMBINE(__nv_bfloat16); else KF_COMBINE(float);
+#undef KF_COMBINE
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
-int kf_moe_combine_bwd_bf16(const void* dout, const void* y, const void* slot_of_row, const void* w, int rows, int k,
+// w and dw: [rows] in slot order, fp32 or (w_half) bf16.
+int kf_moe_combine_bwd_bf16(const void* dout, const void* y, const void* slot_of_row, const void* w, int w_half, int rows, int k,
                             int cols, void* dy, void* dw, void* stream) {
   using namespace kf::moe;
   if (cols & 7) return 5;
   if (rows <= 0) return 0;
   int blocks = (rows + 7) / 8 < 2368 ? (rows + 7) / 8 : 2368;
-  kf_moe_combine_bwd<<<blocks, 256, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(dout), reinterpret_cast<const __nv_bfloat16*>(y),
-      reinterpret_cast<const int*>(slot_of_row), reinterpret_cast<const float*>(w), rows, k, cols,
-      reinterpret_cast<__nv_bfloat16*>(dy), reinterpret_cast<float*>(dw));
+#define KF_COMBINE_BWD(W_)                                                                                                    \
+  kf_moe_combine_bwd<W_><<<blocks, 256, 0, (cudaStream_t)stream>>>(                                                           \
+      reinterpret_cast<const __nv_bfloat16*>(dout), reinterpret_cast<const __nv_bfloat16*>(y),                                \
+      reinterpret_cast<const int*>(slot_of_row), reinterpret_cast<const W_*>(w), rows, k, cols,                               \
+      reinterpret_cast<__nv_bfloat16*>(dy), reinterpret_cast<W_*>(dw))
+  if (w_half) KF_COMBINE_BWD(__nv_bfloat16); else KF_COMBINE_BWD(float);
+#undef KF_COMBINE_BWD
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }

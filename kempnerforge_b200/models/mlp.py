@@ -1,8 +1,7 @@
 """Feed-forward blocks.
 
-``SwiGLUMLP`` issues one GEMM for gate and up (their weights sit back to back in
-the block's flat parameter buffer, so the stacked (2H, D) matrix is a view), a
-fused SwiGLU kernel, and the down GEMM.
+``SwiGLUMLP`` is one GEMM over the gate and up weights, read where they are, with the SwiGLU in its epilogue, and the
+down GEMM; sizes the fused epilogues do not cover take a GEMM over the stacked weights, a SwiGLU kernel and the down GEMM.
 Parity: kempnerforge/model/mlp.py:12-77 (module/parameter names, registry keys
 ``swiglu`` / ``standard_gelu`` / ``standard_relu``, ``build_mlp`` dispatch).
 """
@@ -34,6 +33,9 @@ class SwiGLUMLP(nn.Module):
             y = fp8.swiglu_mlp(x, self.gate_proj.weight, self.up_proj.weight, self.down_proj.weight)
             if y is not None:
                 return y
+        y = F.swiglu_mlp(x, self.gate_proj.weight, self.up_proj.weight, self.down_proj.weight)
+        if y is not None:
+            return y
         gu = F.fused_linear(x, [self.gate_proj.weight, self.up_proj.weight])
         return F.linear(F.swiglu_stacked(gu), self.down_proj.weight)
 

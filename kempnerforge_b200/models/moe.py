@@ -151,7 +151,8 @@ class MoEMLP(nn.Module):
         gate, up, down, layout = self.expert_weights()
         return grouped.grouped_ffn(x_sorted, counts, gate, up, down, layout, self._activation(), offsets=offsets)
 
-    def _local_forward(self, x_flat, weights, indices):
+    def _local_forward(self, x_flat, weights, indices, shared=None):
+        """The experts' output, and ``shared`` (the shared expert's, or None) added to it."""
         t, k = indices.shape
         from kempnerforge_b200.ops import moe_ops
 
@@ -161,7 +162,7 @@ class MoEMLP(nn.Module):
             offsets, row_of_slot, slot_of_row = moe_ops.sort_by_expert(indices, self.num_experts)
             x_sorted = moe_ops.gather_rows(x_flat, slot_of_row, row_of_slot, k)
             y = self.run_experts(x_sorted, None, offsets=offsets)
-            return moe_ops.combine_rows(y, weights, row_of_slot, slot_of_row)
+            return moe_ops.combine_rows(y, weights, row_of_slot, slot_of_row, shared)
         flat_e = indices.reshape(-1)
         order = torch.argsort(flat_e, stable=True)
         token_of_row = order // k
@@ -174,7 +175,8 @@ class MoEMLP(nn.Module):
         inverse = torch.empty_like(order)
         inverse[order] = torch.arange(order.numel(), device=order.device)
         y = y.index_select(0, inverse).view(t, k, -1)
-        return (y * weights.unsqueeze(-1).to(y.dtype)).sum(dim=1)
+        out = (y * weights.unsqueeze(-1).to(y.dtype)).sum(dim=1)
+        return out if shared is None else out + shared
 
     @property
     def aux_loss(self) -> torch.Tensor:
@@ -198,10 +200,11 @@ class MoEMLP(nn.Module):
             from kempnerforge_b200.parallel.expert_parallel import ep_dispatch_and_compute
 
             out = ep_dispatch_and_compute(x_flat, weights, indices, self)
+            if self.shared_expert is not None:
+                out = out + self.shared_expert(x_flat)
         else:
-            out = self._local_forward(x_flat, weights, indices)
-        if self.shared_expert is not None:
-            out = out + self.shared_expert(x_flat)
+            shared = self.shared_expert(x_flat) if self.shared_expert is not None else None
+            out = self._local_forward(x_flat, weights, indices, shared)
         return out.view(b, s, d)
 
 

@@ -43,13 +43,10 @@ class SoftmaxTopKRouter(nn.Module):
         from kempnerforge_b200.ops import moe_ops
 
         if moe_ops.native_ok(logits, self.num_experts, self.top_k):
-            # one kernel: softmax, top-k, renormalised weights, counts, mean probabilities, z-loss
-            weights, indices, counts, pmean, z = moe_ops.route(logits, None, False, self.top_k)
+            # one kernel: softmax, top-k, renormalised weights, counts, balancing loss, z-loss
+            weights, indices, counts, _, self.z_loss, self.aux_loss = moe_ops.route_layer(logits, None, False, self.top_k, x.dtype)
             self.expert_counts = counts.detach()
-            frac = counts / (x.shape[0] * self.top_k)
-            self.aux_loss = self.num_experts * (frac.detach() * pmean).sum()
-            self.z_loss = z
-            return weights.to(x.dtype), indices
+            return weights, indices
         probs = torch.softmax(logits.float(), dim=-1)
         weights, indices = torch.topk(probs, self.top_k, dim=-1)
         weights = (weights / weights.sum(dim=-1, keepdim=True)).to(x.dtype)
@@ -130,8 +127,7 @@ class SigmoidTopKRouter(nn.Module):
         bias, may_update = self._bias_for_this_pass()
         native = moe_ops.native_ok(logits, self.num_experts, self.top_k)
         if native:
-            weights, indices, counts, smean, z = moe_ops.route(logits, bias, True, self.top_k)
-            weights = weights.to(x.dtype)
+            weights, indices, counts, smean, z, zero = moe_ops.route_layer(logits, bias, True, self.top_k, x.dtype)
         else:
             scores = torch.sigmoid(logits.float() + bias.float())
             weights, indices = torch.topk(scores, self.top_k, dim=-1)
@@ -151,7 +147,7 @@ class SigmoidTopKRouter(nn.Module):
             balance = self.num_experts * (util.detach() * mean_scores).sum()
             self.aux_loss = self.sequence_aux_loss_weight * balance
         else:
-            self.aux_loss = torch.zeros((), device=x.device)
+            self.aux_loss = zero if native else torch.zeros((), device=x.device)
         self.z_loss = z if native else torch.logsumexp(logits.float(), dim=-1).pow(2).mean()
         return weights, indices
 

@@ -97,14 +97,14 @@ def _declare(L: ctypes.CDLL) -> None:
         "kf_ep_put_bf16": [vp, vp, i, vp, i, i, i, i, ll, vp, vp, i, vp],
         "kf_ep_layout": [vp, i, i, vp, vp, vp, vp, vp],
         "kf_ep_move_bf16": [vp, vp, vp, vp, vp, i, i, i, ll, i, vp, vp],
-        "kf_router_topk": [vp, i, vp, i, i, i, i, vp, vp, vp, vp, vp, vp],
-        "kf_router_bwd": [vp, i, vp, i, vp, vp, vp, vp, vp, i, i, i, vp, vp, vp, vp],
+        "kf_router_topk": [vp, i, vp, i, i, i, i, i] + [vp] * 10,
+        "kf_router_bwd": [vp, i, vp, i, vp, vp, vp, i, vp, vp, vp, vp, i, i, i, vp, vp, i, vp, vp],
         "kf_grouped_experts_bf16": [i, vp, vp, vp, i, vp, vp, vp, i, i, i, i, ll, ll, ll, i, i, vp],
         "kf_moe_sort": [vp, i, i, vp, vp, vp, vp, vp],
         "kf_moe_capacity_mask": [vp, i, i, i, i, vp, vp],
         "kf_moe_gather_bf16": [vp, vp, i, i, i, vp, vp],
-        "kf_moe_combine_bf16": [vp, vp, vp, i, i, i, vp, vp],
-        "kf_moe_combine_bwd_bf16": [vp, vp, vp, vp, i, i, i, vp, vp, vp],
+        "kf_moe_combine_bf16": [vp, vp, vp, i, vp, i, i, i, vp, vp],
+        "kf_moe_combine_bwd_bf16": [vp, vp, vp, vp, i, i, i, i, vp, vp, vp],
         "kf_grouped_gemm_bf16": [vp, vp, vp, vp, i, i, i, i, ll, ll, i, i, vp],
         "kf_grouped_gemm_acc_bf16": [vp, vp, vp, vp, i, i, i, i, ll, ll, i, i, i, vp],
         "kf_grouped_swiglu_bf16": [vp, vp, vp, vp, vp, vp, i, i, i, i, ll, ll, ll, i, i, vp],
@@ -673,17 +673,19 @@ def gemm_swiglu_pair(x2: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, want_
     return h, gu
 
 
-def gemm_swiglu_bwd(dy2: torch.Tensor, w_down: torch.Tensor, gu: torch.Tensor) -> torch.Tensor:
-    """d[gate | up] (M, 2F), written over ``gu``: the input-gradient GEMM of the down projection (``dy2`` (M, K) times
+def gemm_swiglu_bwd(dy2: torch.Tensor, w_down: torch.Tensor, gu: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+    """d[gate | up] (M, 2F), written to ``out`` (default: over ``gu``): the input-gradient GEMM of the down projection (``dy2`` (M, K) times
     ``w_down`` (K, F) as stored) with the SwiGLU gradient in its epilogue; the gradient of the hidden activation is
     never written to memory."""
     m, k = dy2.shape
     f = w_down.shape[1]
     assert w_down.shape[0] == k and gu.shape == (m, 2 * f) and gu.is_contiguous() and w_down.stride(1) == 1
-    _check(lib().kf_gemm_swiglu_bwd_bf16(dy2.data_ptr(), w_down.data_ptr(), gu.data_ptr(), gu.data_ptr(), m, f, k,
+    out = gu if out is None else out
+    assert out.shape == gu.shape and out.dtype == gu.dtype and out.is_contiguous()
+    _check(lib().kf_gemm_swiglu_bwd_bf16(dy2.data_ptr(), w_down.data_ptr(), gu.data_ptr(), out.data_ptr(), m, f, k,
                                          dy2.stride(0), w_down.stride(0), 2 * f, sm_count(), _stream()),
            "kf_gemm_swiglu_bwd_bf16")
-    return gu
+    return out
 
 
 def gemm_symm(x: torch.Tensor, tall: bool = False, residual: torch.Tensor | None = None, alpha: float = 1.0,
@@ -881,32 +883,46 @@ def sf_adamw_step(y, g, z, v, x, lr, b1, b2, eps, wd, bc2, ck, first: bool) -> b
 
 
 # --------------------------------------------------------------------------- mixture of experts
-def router_topk(logits: torch.Tensor, bias: torch.Tensor | None, sigmoid: bool, k: int):
-    """(weights fp32 (T, k), indices int64 (T, k), counts fp32 (E), prob_sum fp32 (E), sum of logsumexp² fp32 (1))."""
+def router_topk(logits: torch.Tensor, bias: torch.Tensor | None, sigmoid: bool, k: int, half: bool = False):
+    """(weights fp32 (T, k), the same in bf16 or None, indices int64 (T, k), what :func:`router_bwd` needs of the bias or the
+    counts, token counts fp32 (E), mean scores fp32 (E), mean logsumexp² fp32 (), balance fp32 ()): ``balance`` = E sum(counts /
+    (T k) * mean) of softmax scores, 0 of sigmoid ones.  ``half``: also the bf16 weights.  ``bias``: fp32 or bf16 (E)."""
     t, e = logits.shape
     assert logits.is_contiguous() and logits.dtype in (torch.bfloat16, torch.float32)
-    idx = torch.empty((t, k), dtype=torch.int64, device=logits.device)
-    w = torch.empty((t, k), dtype=torch.float32, device=logits.device)
-    acc = torch.zeros(2 * e + 1, dtype=torch.float32, device=logits.device)
-    b = bias.float().contiguous() if bias is not None else None
-    _check(lib().kf_router_topk(logits.data_ptr(), 0 if logits.dtype == torch.bfloat16 else 1,
-                                b.data_ptr() if b is not None else None, int(sigmoid), t, e, k, idx.data_ptr(),
-                                w.data_ptr(), acc.data_ptr(), acc[e:].data_ptr(), acc[2 * e:].data_ptr(), _stream()),
-           "kf_router_topk")
-    return w, idx, acc[:e], acc[e:2 * e], acc[2 * e:]
+    dev = logits.device
+    idx = torch.empty((t, k), dtype=torch.int64, device=dev)
+    w = torch.empty((t, k), dtype=torch.float32, device=dev)
+    w16 = torch.empty((t, k), dtype=torch.bfloat16, device=dev) if half else None
+    # tensors of their own: a program may change any of them in place
+    counts, mean, keep = (torch.empty(e, dtype=torch.float32, device=dev) for _ in range(3))
+    z, balance = (torch.empty((), dtype=torch.float32, device=dev) for _ in range(2))
+    acc = torch.empty(2 * e + 2, dtype=torch.float32, device=dev)
+    assert bias is None or (bias.shape == (e,) and bias.is_contiguous() and bias.dtype in (torch.bfloat16, torch.float32))
+    _check(lib().kf_router_topk(logits.data_ptr(), 0 if logits.dtype == torch.bfloat16 else 1, _ptr(bias),
+                                int(bias is not None and bias.dtype == torch.bfloat16), int(sigmoid), t, e, k,
+                                idx.data_ptr(), w.data_ptr(), _ptr(w16), keep.data_ptr(), counts.data_ptr(), mean.data_ptr(), z.data_ptr(),
+                                balance.data_ptr(), acc.data_ptr(), _stream()), "kf_router_topk")
+    if t == 0:   # no token, no launch: means over nothing
+        counts.zero_(), keep.zero_(), mean.fill_(float("nan")), z.fill_(float("nan")), balance.fill_(0.0 if sigmoid else float("nan"))
+    return w, w16, idx, keep, counts, mean, z, balance
 
 
-def router_bwd(logits, bias, sigmoid: bool, idx, w, dw, dmean, dz, want_dbias: bool):
-    """(dlogits, dbias fp32 or None) of :func:`router_topk`: ``dw`` (T, k), ``dmean`` (E) of the mean scores and ``dz`` of the
-    mean squared logsumexp, all fp32."""
+def router_bwd(logits, keep, sigmoid: bool, idx, w, dw, dmean, dz, dbalance, dbias_dtype: torch.dtype | None):
+    """(dlogits, dbias or None) of :func:`router_topk`: ``dw`` (T, k) fp32 or bf16, ``dmean`` (E) of the mean scores, ``dz`` of the
+    mean squared logsumexp and ``dbalance`` of the balancing loss, all fp32 (each may be None).  ``dbias_dtype``: fp32 or bf16,
+    None for no gradient of the bias."""
     t, e = logits.shape
     k = idx.shape[1]
     dlogits = torch.empty_like(logits)
-    dbias = torch.empty(e, dtype=torch.float32, device=logits.device) if want_dbias else None
-    partial = torch.empty(592 * e, dtype=torch.float32, device=logits.device) if want_dbias else None
-    _check(lib().kf_router_bwd(logits.data_ptr(), 0 if logits.dtype == torch.bfloat16 else 1, _ptr(bias), int(sigmoid),
-                               idx.data_ptr(), w.data_ptr(), dw.data_ptr(), _ptr(dmean), _ptr(dz), t, e, k,
-                               dlogits.data_ptr(), _ptr(dbias), _ptr(partial), _stream()), "kf_router_bwd")
+    dbias = partial = None
+    if dbias_dtype is not None:
+        dbias = torch.empty(e, dtype=dbias_dtype, device=logits.device)
+        partial = torch.empty(592 * e, dtype=torch.float32, device=logits.device)
+    _check(lib().kf_router_bwd(logits.data_ptr(), 0 if logits.dtype == torch.bfloat16 else 1, keep.data_ptr(), int(sigmoid),
+                               idx.data_ptr(), w.data_ptr(), _ptr(dw), int(dw is not None and dw.dtype == torch.bfloat16),
+                               _ptr(dmean), _ptr(dz), _ptr(dbalance), keep.data_ptr(), t, e, k, dlogits.data_ptr(), _ptr(dbias),
+                               int(dbias_dtype == torch.bfloat16), _ptr(partial), _stream()), "kf_router_bwd",
+           2 if dbias is not None else 1)
     return dlogits, dbias
 
 
@@ -943,20 +959,26 @@ def moe_gather(x: torch.Tensor, slot_of_row: torch.Tensor, k: int) -> torch.Tens
     return out
 
 
-def moe_combine(y: torch.Tensor, row_of_slot: torch.Tensor, w: torch.Tensor | None, tokens: int, k: int) -> torch.Tensor:
+def moe_combine(y: torch.Tensor, row_of_slot: torch.Tensor, w: torch.Tensor | None, tokens: int, k: int,
+                plus: torch.Tensor | None = None) -> torch.Tensor:
+    """(T, D) sum over the k rows of every token, weighted by ``w`` (T, k) fp32 or bf16, and ``plus`` (T, D) added to it."""
     cols = y.shape[1]
     out = torch.empty((tokens, cols), dtype=y.dtype, device=y.device)
-    _check(lib().kf_moe_combine_bf16(y.data_ptr(), row_of_slot.data_ptr(), w.data_ptr() if w is not None else None,
-                                     tokens, k, cols, out.data_ptr(), _stream()), "kf_moe_combine_bf16")
+    assert w is None or w.dtype in (torch.float32, torch.bfloat16)
+    _check(lib().kf_moe_combine_bf16(y.data_ptr(), row_of_slot.data_ptr(), _ptr(w), int(w is not None and w.dtype == torch.bfloat16),
+                                     _ptr(plus), tokens, k, cols, out.data_ptr(), _stream()), "kf_moe_combine_bf16")
     return out
 
 
 def moe_combine_bwd(dout: torch.Tensor, y: torch.Tensor, slot_of_row: torch.Tensor, w: torch.Tensor, k: int):
+    """(dy, dw) of the weighted :func:`moe_combine`; ``dw`` in the type of ``w`` (fp32 or bf16), in slot order."""
     rows, cols = y.shape
+    assert w.dtype in (torch.float32, torch.bfloat16)
     dy = torch.empty_like(y)
-    dw = torch.empty(rows, dtype=torch.float32, device=y.device)
-    _check(lib().kf_moe_combine_bwd_bf16(dout.data_ptr(), y.data_ptr(), slot_of_row.data_ptr(), w.data_ptr(), rows, k, cols,
-                                         dy.data_ptr(), dw.data_ptr(), _stream()), "kf_moe_combine_bwd_bf16")
+    dw = torch.empty(rows, dtype=w.dtype, device=y.device)
+    _check(lib().kf_moe_combine_bwd_bf16(dout.data_ptr(), y.data_ptr(), slot_of_row.data_ptr(), w.data_ptr(),
+                                         int(w.dtype == torch.bfloat16), rows, k, cols, dy.data_ptr(), dw.data_ptr(), _stream()),
+           "kf_moe_combine_bwd_bf16")
     return dy, dw
 
 

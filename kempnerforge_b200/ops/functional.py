@@ -15,6 +15,7 @@ the optimizer and the reduce-scatter read the flat buffer directly.
 from __future__ import annotations
 
 import math
+import os
 
 import torch
 
@@ -422,6 +423,62 @@ def swiglu_stacked(gu: torch.Tensor) -> torch.Tensor:
     if use_native(gu) and gu.is_contiguous() and h % 8 == 0:
         return _SwiGLUFn.apply(gu)
     return ref.swiglu(gu[..., :h], gu[..., h:])
+
+
+class _SwiGLUMLPFn(torch.autograd.Function):
+    """A whole SwiGLU MLP: gate | up GEMM with the activation in its epilogue, down GEMM; backward with the SwiGLU gradient in
+    the epilogue of the down projection's input gradient, one input-gradient and one weight-gradient GEMM for gate and up.
+    The same roundings as :class:`_LinearFn` and :class:`_SwiGLUFn` in a row."""
+
+    @staticmethod
+    def forward(ctx, x, wg, wu, wd):
+        cu = _cuda()
+        x2 = x.reshape(-1, x.shape[-1])
+        if not x2.is_contiguous():
+            x2 = x2.contiguous()
+        h, gu = cu.gemm_swiglu_pair(x2, wg, wu, want_gu=any(ctx.needs_input_grad))
+        y = cu.gemm_rows(h, [wd])
+        if gu is not None:
+            ctx.save_for_backward(x2, wg, wu, wd, gu, h)
+            ctx.x_shape = x.shape
+        return y.view(*x.shape[:-1], y.shape[-1])
+
+    @staticmethod
+    def backward(ctx, dy):
+        from kempnerforge_b200.ops.grouped import _gradient_buffer
+
+        cu = _cuda()
+        x2, wg, wu, wd, gu, h = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        dy2 = dy.reshape(-1, dy.shape[-1])
+        if not dy2.is_contiguous():
+            dy2 = dy2.contiguous()
+        dwd = _linear_weight_grads(cu, dy2, h, [wd], need[3:])
+        if not any(need[:3]):
+            return (None, None, None, *dwd)
+        dgu = cu.gemm_swiglu_bwd(dy2, wd, gu, out=_gradient_buffer(gu))
+        dx = cu.dgrad_rows(dgu, [wg, wu]).view(ctx.x_shape) if need[0] else None
+        return (dx, *_linear_weight_grads(cu, dgu, x2, [wg, wu], need[1:3]), *dwd)
+
+
+def swiglu_mlp(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, wd: torch.Tensor) -> torch.Tensor | None:
+    """down(silu(x Wgᵀ) * (x Wuᵀ)) as one node on the fused GEMMs, or None when they do not cover the call."""
+    if not (use_native(x) and x.dim() >= 2 and x.numel() and torch.autograd.forward_ad._current_level < 0):
+        return None
+    cu = _cuda()
+    d, f = x.shape[-1], wg.shape[0]
+    rows = x.numel() // d
+    if rows < 256 or d % 64 or f % 256 or wg.shape != (f, d) or wu.shape != (f, d) or wd.shape != (d, f):
+        return None
+    for w in (wg, wu, wd):
+        if (w.dtype != torch.bfloat16 or w.device != x.device or not w.is_contiguous() or w.data_ptr() % 16
+                or hasattr(w, "_kf_fp8") or getattr(getattr(w, "_kf_flat", None), "sharded", False)):
+            return None
+    if os.environ.get("KF_DISABLE_SWIGLU_EPILOGUE") or os.environ.get("KF_SWIGLU_BWD_EPILOGUE", "1") != "1" or cu.GEMM_MODE:
+        return None
+    if x.is_contiguous() and x.data_ptr() % 16:
+        return None
+    return _SwiGLUMLPFn.apply(x, wg, wu, wd)
 
 
 # --------------------------------------------------------------------------- embedding

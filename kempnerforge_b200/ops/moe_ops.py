@@ -23,61 +23,84 @@ def native_ok(x: torch.Tensor, num_experts: int, top_k: int) -> bool:
 
 
 class _RouterFn(torch.autograd.Function):
-    """(weights, indices, counts, score_mean, z_loss) from logits.  ``score_mean`` (mean score per expert) and
-    ``z_loss`` are differentiable, like ``weights``; ``indices`` and ``counts`` are not."""
+    """(weights, indices, counts, score_mean, z_loss, balance) from logits; weights in ``dtype``.  ``score_mean`` (mean score per
+    expert), ``z_loss`` and, for softmax scores, ``balance`` = E sum(counts / (T k) * score_mean) are differentiable, like
+    ``weights``; ``indices`` and ``counts`` are not."""
 
     @staticmethod
-    def forward(ctx, logits, bias, sigmoid, k):
+    def forward(ctx, logits, bias, sigmoid, k, dtype):
+        ctx.set_materialize_grads(False)   # a layer that trains on the weights alone gets None for the rest
         logits = logits.contiguous()
-        # the sigmoid router nudges its bias in place right after routing: a private fp32 copy serves both passes
-        bf = None if bias is None else bias.detach().to(torch.float32, copy=True)
-        w, idx, counts, prob_sum, lse_sq = kc.router_topk(logits, bf, sigmoid, k)
-        t = logits.shape[0]
-        ctx.save_for_backward(logits, idx, w, *(() if bf is None else (bf,)))
+        b = bias
+        if b is not None:
+            b = b.detach()
+            if b.dtype not in (torch.float32, torch.bfloat16):
+                b = b.to(torch.float32)
+            b = b.contiguous()
+        # the sigmoid router nudges its bias in place right after routing: the fp32 copy in ``keep`` serves the backward
+        w, w16, idx, keep, counts, mean, z, balance = kc.router_topk(logits, b, sigmoid, k, dtype is torch.bfloat16)
+        ctx.save_for_backward(logits, idx, w, keep)
         ctx.sigmoid, ctx.has_bias = sigmoid, bias is not None
         ctx.bias_dtype = bias.dtype if bias is not None else None
-        ctx.mark_non_differentiable(idx, counts)
-        return w, idx, counts, prob_sum / t, lse_sq.reshape(()) / t
+        ctx.mark_non_differentiable(idx, counts, *((balance,) if sigmoid else ()))
+        out = w16 if dtype is torch.bfloat16 else w.to(dtype)
+        return out, idx, counts, mean, z, balance
 
     @staticmethod
-    def backward(ctx, dw, _didx, _dcounts, dmean, dz):
-        logits, idx, w, *rest = ctx.saved_tensors
-        bias = rest[0] if rest else None
+    def backward(ctx, dw, _didx, _dcounts, dmean, dz, dbalance):
+        logits, idx, w, keep = ctx.saved_tensors   # keep: the bias (sigmoid) or the counts (softmax)
+        t, e = logits.shape
+        if dw is None and dmean is None and dz is None and dbalance is None:
+            return None, None, None, None, None
+        dmean, dz, dbalance = (None if g is None else g.float().contiguous() for g in (dmean, dz, dbalance))
         if not torch.is_grad_enabled():
-            dlogits, dbias = kc.router_bwd(
-                logits, bias, ctx.sigmoid, idx, w, dw.float().contiguous(),
-                dmean.float().contiguous() if dmean is not None else None, dz.float() if dz is not None else None,
-                ctx.has_bias and ctx.needs_input_grad[1])
-            return dlogits, dbias.to(ctx.bias_dtype) if dbias is not None else None, None, None
+            if dw is not None:
+                dw = (dw if dw.dtype in (torch.float32, torch.bfloat16) else dw.float()).contiguous()
+            bias_grad = ctx.bias_dtype if ctx.has_bias and ctx.needs_input_grad[1] else None
+            half = bias_grad is torch.bfloat16
+            dlogits, dbias = kc.router_bwd(logits, keep, ctx.sigmoid, idx, w, dw, dmean, dz, dbalance,
+                                           None if bias_grad is None else torch.bfloat16 if half else torch.float32)
+            return dlogits, dbias.to(bias_grad) if dbias is not None else None, None, None, None
         # create_graph: the same formulas as differentiable element-wise ops
         lf = logits.float()
-        t = lf.shape[0]
         if ctx.sigmoid:
-            scores = torch.sigmoid(lf + bias) if ctx.has_bias else torch.sigmoid(lf)
+            scores = torch.sigmoid(lf + keep)
         else:
             scores = torch.softmax(lf, dim=-1)
-        sel = scores.gather(1, idx)
-        ssum = sel.sum(dim=1, keepdim=True)
-        # w = sel / ssum
-        dsel = (dw - (dw * w).sum(dim=1, keepdim=True)) / ssum
-        dscores = torch.zeros_like(scores).scatter_(1, idx, dsel)
+        dscores = torch.zeros_like(scores)
+        if dw is not None:
+            sel = scores.gather(1, idx)
+            ssum = sel.sum(dim=1, keepdim=True)
+            # w = sel / ssum
+            dw = dw.float()
+            dsel = (dw - (dw * (sel / ssum)).sum(dim=1, keepdim=True)) / ssum
+            dscores = dscores.scatter(1, idx, dsel)
+        if dbalance is not None:
+            per_expert = dbalance * e * keep / (t * idx.shape[1])
+            dmean = per_expert if dmean is None else dmean + per_expert
         if dmean is not None:
-            dscores = dscores + dmean.float()[None, :] / t
+            dscores = dscores + dmean[None, :] / t
         if ctx.sigmoid:
             dlogits = dscores * scores * (1.0 - scores)
         else:
             dlogits = scores * (dscores - (dscores * scores).sum(dim=1, keepdim=True))
         if dz is not None:
             lse = torch.logsumexp(lf, dim=-1, keepdim=True)
-            dlogits = dlogits + (dz.float() * 2.0 / t) * lse * torch.softmax(lf, dim=-1)
+            dlogits = dlogits + (dz * 2.0 / t) * lse * torch.softmax(lf, dim=-1)
         # expert_bias is nudged by its own rule, never by gradients through the scores (the reference detaches
         # nothing here either, but its bias update overwrites any gradient step); keep autograd's answer
         dbias = dlogits.sum(dim=0).to(ctx.bias_dtype) if (ctx.has_bias and ctx.needs_input_grad[1]) else None
-        return dlogits.to(logits.dtype), dbias, None, None
+        return dlogits.to(logits.dtype), dbias, None, None, None
 
 
 def route(logits: torch.Tensor, bias: torch.Tensor | None, sigmoid: bool, k: int):
-    return _RouterFn.apply(logits, bias, sigmoid, k)
+    """(weights fp32, indices, counts, score_mean, z_loss)."""
+    return _RouterFn.apply(logits, bias, sigmoid, k, torch.float32)[:5]
+
+
+def route_layer(logits: torch.Tensor, bias: torch.Tensor | None, sigmoid: bool, k: int, dtype: torch.dtype):
+    """(weights in ``dtype``, indices, counts, score_mean, z_loss, balance) of :class:`_RouterFn`."""
+    return _RouterFn.apply(logits, bias, sigmoid, k, dtype)
 
 
 class _GatherFn(torch.autograd.Function):
@@ -96,23 +119,23 @@ class _GatherFn(torch.autograd.Function):
 
 
 class _CombineFn(torch.autograd.Function):
-    """out[t] = sum_j w[t, j] * y_sorted[row_of_slot[t, j]]."""
+    """out[t] = sum_j w[t, j] * y_sorted[row_of_slot[t, j]] (+ plus[t])."""
 
     @staticmethod
-    def forward(ctx, y, w, row_of_slot, slot_of_row):
+    def forward(ctx, y, w, row_of_slot, slot_of_row, plus):
         t, k = w.shape
-        wf = w.float().contiguous()
-        ctx.save_for_backward(y, wf, row_of_slot, slot_of_row)
+        wk = (w if w.dtype in (torch.float32, torch.bfloat16) else w.float()).contiguous()
+        ctx.save_for_backward(y, wk, row_of_slot, slot_of_row)
         ctx.w_dtype = w.dtype
-        return kc.moe_combine(y.contiguous(), row_of_slot, wf, t, k)
+        return kc.moe_combine(y.contiguous(), row_of_slot, wk, t, k, plus)
 
     @staticmethod
     def backward(ctx, dout):
-        y, wf, row_of_slot, slot_of_row = ctx.saved_tensors
-        t, k = wf.shape
-        dy, dw_rows = kc.moe_combine_bwd(dout.contiguous(), y.contiguous(), slot_of_row, wf.reshape(-1), k)
+        y, wk, row_of_slot, slot_of_row = ctx.saved_tensors
+        t, k = wk.shape
+        dy, dw_rows = kc.moe_combine_bwd(dout.contiguous(), y.contiguous(), slot_of_row, wk.reshape(-1), k)
         # dw comes out per sorted row (indexed by slot inside the kernel): it is already in slot order
-        return dy, dw_rows.view(t, k).to(ctx.w_dtype), None, None
+        return dy, dw_rows.view(t, k).to(ctx.w_dtype), None, None, dout if ctx.needs_input_grad[4] else None
 
 
 def sort_by_expert(indices: torch.Tensor, num_experts: int):
@@ -123,5 +146,9 @@ def gather_rows(x, slot_of_row, row_of_slot, k):
     return _GatherFn.apply(x, slot_of_row, row_of_slot, k)
 
 
-def combine_rows(y, w, row_of_slot, slot_of_row):
-    return _CombineFn.apply(y, w, row_of_slot, slot_of_row)
+def combine_rows(y, w, row_of_slot, slot_of_row, plus=None):
+    """``plus`` (T, D): another contribution to every token (a shared expert), added to the rounded sum in the same pass."""
+    if plus is not None and not (plus.is_cuda and plus.dtype == y.dtype and plus.shape == (w.shape[0], y.shape[1])
+                                 and plus.is_contiguous() and plus.data_ptr() % 16 == 0):
+        return _CombineFn.apply(y, w, row_of_slot, slot_of_row, None) + plus
+    return _CombineFn.apply(y, w, row_of_slot, slot_of_row, plus)
