@@ -742,13 +742,17 @@ def fp8_scale(x2: torch.Tensor, e5m2: bool = False) -> torch.Tensor:
 
 
 def fp8_cast(x2: torch.Tensor, scale: torch.Tensor, e5m2: bool, want_row: bool = True, want_t: bool = False):
-    """fp8 bytes of x * scale: (rows, cols) and / or the transposed (cols, rows) copy, as uint8 tensors."""
+    """fp8 bytes of x * scale: (rows, cols) and / or the transposed (cols, rows) copy, as uint8 tensors.  The rows of the transposed
+    copy start on 128 bytes."""
     rows, cols = x2.shape
     assert x2.stride(1) == 1
     row = torch.empty((rows, cols), dtype=torch.uint8, device=x2.device) if want_row else None
-    t = torch.empty((cols, rows), dtype=torch.uint8, device=x2.device) if want_t else None
+    # A product over the rows of x reads 128 bytes of every row of the copy at a time: at a pitch of 2000 each of those reads spans two
+    # lines.  Weight gradients of a 7B feed-forward over 2000 tokens, us: gate | up 216 -> 151, down 107 -> 77
+    pitch = -(-rows // 128) * 128
+    t = torch.empty((cols, pitch), dtype=torch.uint8, device=x2.device)[:, :rows] if want_t else None
     _check(lib().kf_fp8_cast_bf16(x2.data_ptr(), rows, cols, x2.stride(0), scale.data_ptr(), int(e5m2),
-                                  row.data_ptr() if want_row else None, cols, t.data_ptr() if want_t else None, rows,
+                                  row.data_ptr() if want_row else None, cols, t.data_ptr() if want_t else None, pitch,
                                   _stream()), "kf_fp8_cast_bf16")
     return row, t
 
