@@ -2,21 +2,27 @@
 //
 //   C[rows of expert e, :N] (+)= A[rows of expert e, :K] * op(B_e)          for every expert e
 //
-// Same contract as the single-CTA kernel in grouped_gemm_tcgen05.cu (expert-sorted rows, int32 `offsets` on the
-// device, nothing padded, no host read), with the tiling of the dense CTA-pair GEMM: two CTAs on neighbouring SMs own
-// a 256 x 256 output tile, CTA r loads 128 of the tile's rows of A and 128 of its rows / columns of B, the leader
-// issues 256 x 256 x 16 MMAs that read both CTAs' shared memory.  Per CTA and k-block 32 KB are loaded instead of the
-// 48 KB of the 128 x 256 single-CTA tile, which leaves six pipeline stages and takes the shared-memory read port off
-// the critical path.  A row tile never crosses an expert boundary: tiles are counted per expert (256 rows each, the
-// last one partial) and the epilogue stores only the rows that belong to the expert.
+// Same contract as the single-CTA kernel in grouped_gemm_tcgen05.cu: expert-sorted rows, int32 `offsets` on the device, nothing padded,
+// no host read.
 //
-// SWIGLU: two weight operands (gate: map_b, up: map_b2) of N = F hidden units each; a tile covers 128 hidden units,
-// the leader CTA loads their gate weights and the peer the matching up weights, so every CTA's accumulator holds
-// [gate 128 | up 128] for its 128 rows; the epilogue writes h = silu(gate) * up and optionally the pre-activations.
+// Tiles.  The weights are the M side of the MMA (256 rows of B_e per pair, 128 per CTA) and the tokens its N side, as in
+// gemm_tokens_tcgen05_2cta.cu: an expert's rows are cut into equal tiles of a multiple of 32, up to 256, and never cross its end.  An
+// MMA's time follows its N side (see warp_index in common.cuh; a k-block of a pair takes about 1.45 ns per token and 70 ns), so a tile costs what
+// its tokens do.  With the tokens as the M side every tile was 256 rows: 167 rows per expert (64 experts, top 6 of 1777 tokens) paid for
+// 256, and 520 for 768.  The widest tile allowed is chosen on the device, once per CTA, so that rounds of tiles over the pairs times the
+// average tile are least: 8 experts of about 512 rows and 2048 output columns are 160 tiles of 256, three rounds of the 74 pairs, or
+// 192 tiles of 192 in the same three.
+// All token tiles of a block of 256 weight rows are neighbours in the tile order, so the weights cross the L2 cache once.
+// What bounds them now: 64 experts stream their weights (gate and up 738 MB: 113 us at the copy rate), 8 experts run the tensor cores at
+// the clock that the power cap leaves (518 clocks per k-block of 512).  Measured, us, tokens as M side / as N side, in the order
+// gate | up, down, SwiGLU gradient, input gradient: 64 experts of 2048 x 1408 over 10 662 rows 166, 90, 141, 156 / 160, 90, 118, 149;
+// whole layers, forward and backward: 64 experts over 598 tokens 860 / 769, over 1457 1200 / 1071; 8 experts of 2048 x 7168 over 2048
+// tokens, where some experts have more than 512 rows, 1270 / 1216, over 1484 1429 / 1362.
 //
-// EPI == 2: SwiGLU backward in the epilogue of the down projection's input-gradient product (see the launcher).
-//
-// EPI == 3: C = A_1 B_e + A_2 B2_e with A = [A_1 | A_2] side by side (the input gradient of the gate and up projections as
+// kind 1, SwiGLU: gate (maps_b) and up weights (maps_b2), 128 hidden units per tile: a CTA's accumulator lanes hold 64 gate and the 64
+// matching up units; h = silu(gate) * up and optionally the pre-activations are written.
+// kind 2: SwiGLU backward in the epilogue of the down projection's input-gradient product (see the launcher).
+// kind 3: C = A_1 B_e + A_2 B2_e with A = [A_1 | A_2] side by side (the input gradient of the gate and up projections as
 // one product over K = 2 F): no second pass over C, and the sum is rounded once.
 //
 // NE > 1: every expert's weight has a tensor map of its own (up to NE of them, kernel parameters), so the weights of
@@ -25,24 +31,24 @@
 //
 // Synchronisation as in gemm_tcgen05_2cta.cu (all waits bounded); TMA loads carry no cluster multicast.
 // Replaces the padded torch._grouped_mm calls of the reference (kempnerforge/model/moe.py:20-145).
-#include "common.cuh"
-#include "gemm_epilogue.cuh"
-#include "tile_math.h"
 #include "pair_common.cuh"
+#include "tile_math.h"
+#include "tokens_epilogue.cuh"
 
 namespace kf {
 namespace grp2 {
 
 using namespace kf::pairops;
+using kf2::tokens::Output;
+using kf2::tokens::WARP_BYTES;
+using tilemath::TokenTiles;
 
-constexpr int CTA_M = 128, TILE_M = 256, TILE_N = 256, HALF_N = 128, BK = 64, STAGES = 6, UMMA_K = 16;
-constexpr int A_BYTES = CTA_M * BK * 2, B_BYTES = HALF_N * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr int CTA_M = 128, TILE_M = 256, MAX_N = 256, BK = 64, STAGES = 6, UMMA_K = 16;
+constexpr int A_BYTES = CTA_M * BK * 2, B_BYTES = MAX_N / 2 * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int THREADS = 192, TMEM_COLS = 512;
 constexpr int MAX_EXPERTS = 256;
-constexpr int BOX_BYTES = 2048;  // rows of an epilogue warp on their way to or from global memory; two per warp
-constexpr size_t SMEM = size_t(STAGES) * STAGE_BYTES + 8 * BOX_BYTES + 1024 + 256 + (MAX_EXPERTS + 1) * 4;
-
-using Tile = tilemath::GroupedTile;
+constexpr int BAR_BYTES = 192;
+constexpr size_t SMEM = size_t(STAGES) * STAGE_BYTES + 4 * WARP_BYTES + 1024 + BAR_BYTES + (MAX_EXPERTS + 1) * 4;
 
 template <int NE>
 struct Maps {
@@ -50,16 +56,16 @@ struct Maps {
 };
 constexpr int MAX_SEPARATE = 32;  // experts with a tensor map of their own (two operands: 8 KB of kernel parameters)
 
-template <bool B_MN, int EPI, int NE>
+// map_a.m[i]: boxes of 16 (i + 1) token rows, what a CTA of the pair loads of a tile of 32 (i + 1).
+template <bool B_MN, int KIND, int NE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
-kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ Maps<NE> maps_b,
-                             const __grid_constant__ Maps<(EPI & 1) ? NE : 1> maps_b2, __nv_bfloat16* __restrict__ C,
-                             __nv_bfloat16* __restrict__ GU, const int* __restrict__ offsets, int E, int N, int K,
-                             long long ldc, long long ldgu, int accumulate, int* status) {
+kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ Maps<8> map_a, const __grid_constant__ Maps<NE> maps_b,
+                             const __grid_constant__ Maps<(KIND & 1) ? NE : 1> maps_b2, const __grid_constant__ Output out,
+                             const int* __restrict__ row_offsets, int E, int N, int K, int* status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t box_smem = smem_base + STAGES * STAGE_BYTES;
-  const uint32_t bar_base = box_smem + 8 * BOX_BYTES;
+  const uint32_t bar_base = box_smem + 4 * WARP_BYTES;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
   auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + a); };
@@ -68,18 +74,21 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
   const uint32_t tmem_slot = bar_base + 8u * (2 * STAGES + 5);
   uint8_t* bar_gen = smem_raw + (bar_base - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(bar_gen + 8 * (2 * STAGES + 5));
-  int* tile_start = reinterpret_cast<int*>(bar_gen + 256);
+  volatile int* widest_ptr = reinterpret_cast<volatile int*>(bar_gen + 8 * (2 * STAGES + 6));
+  static_assert(8 * (2 * STAGES + 7) <= BAR_BYTES, "barriers, tensor-memory address, widest tile and number of tiles");
+  int* offsets = reinterpret_cast<int*>(bar_gen + BAR_BYTES);
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
   const bool leader = rank == 0;
   const int pair = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
-  constexpr bool SWIGLU = EPI == 1;
-  constexpr int TN = SWIGLU ? HALF_N : TILE_N;  // output columns (hidden units) per tile
-  const int n_blocks = (N + TN - 1) / TN;
+  constexpr bool SWIGLU = KIND == 1;
+  constexpr int TILE_F = SWIGLU ? TILE_M / 2 : TILE_M, CTA_F = TILE_F / 2;  // features (hidden units) per tile and per CTA
+  const int f_blocks = (N + TILE_F - 1) / TILE_F;
   const int k_blocks = (K + BK - 1) / BK;
 
+  for (int i = threadIdx.x; i <= E; i += THREADS) offsets[i] = row_offsets[i];
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full_bar(s), 1);
@@ -91,12 +100,35 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
     }
     mbar_init(drain_bar, 1);
     mbar_fence_init();
-    tma_prefetch_desc(&map_a);
     if (NE == 1) {
       tma_prefetch_desc(&maps_b.m[0]);
-      if (EPI & 1) tma_prefetch_desc(&maps_b2.m[0]);
+      if (KIND & 1) tma_prefetch_desc(&maps_b2.m[0]);
     }
-    tilemath::grouped_tile_starts(offsets, E, TILE_M, tile_start);  // both CTAs of a pair compute the same table
+  }
+  __syncthreads();  // the offsets are in place
+  if (warp == 0) {  // widest token tile: the same choice in every CTA
+    int best = MAX_N, total = 0;
+    float best_cost = 3.4e38f;
+    for (int widest = MAX_N; widest >= tilemath::NARROWEST_TOKENS; widest -= 32) {
+      int tiles = 0, clocks = 0;
+      for (int e = lane; e < E; e += 32) {
+        const int rows = offsets[e + 1] - offsets[e], n = tilemath::ceil_div(rows, widest);
+        tiles += n;
+        clocks += n * tilemath::token_tile_cost(tilemath::token_tile_width(rows, n));
+      }
+      tiles = __reduce_add_sync(0xffffffffu, tiles);
+      clocks = __reduce_add_sync(0xffffffffu, clocks);
+      const float cost = tilemath::token_rounds_cost(tiles, clocks, f_blocks, num_pairs);
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = widest;
+        total = tiles * f_blocks;
+      }
+    }
+    if (lane == 0) {
+      widest_ptr[0] = best;
+      widest_ptr[1] = total;
+    }
   }
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, TMEM_COLS);
@@ -107,42 +139,45 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
   cluster_sync_all();  // both CTAs' barriers exist before anyone signals across the pair
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
-  const int num_tiles = tile_start[E] * n_blocks;
+  const int widest = widest_ptr[0], num_tiles = widest_ptr[1];
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (one per CTA)
     if (elect_one()) {
       int it = 0;
       bool ok = true;
-      // the leader fetches the gate weights (or the first 128 columns), the peer the up weights (or the last 128)
+      TokenTiles walk(offsets, f_blocks, widest);
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
-        const Tile tl = tilemath::grouped_decode(t, n_blocks, tile_start, offsets, E, TILE_M);
-        const int m0 = tl.row0 + int(rank) * CTA_M;
-        const int n0 = SWIGLU ? tl.nb * TN : tl.nb * TN + int(rank) * HALF_N;
+        const auto tl = walk.at(t);
+        const int half = tl.width >> 1;
+        const int n0 = tl.row0 + int(rank) * half, f0 = tl.fb * TILE_F + int(rank) * CTA_F;
+        const CUtensorMap* my_a = &map_a.m[(tl.width >> 5) - 1];
         const int me = NE > 1 ? tl.e : 0;              // tensor map and first row of the expert's weight inside it
-        const int e_n = NE > 1 ? 0 : tl.e * N, e_k = NE > 1 ? 0 : tl.e * (EPI == 3 ? K / 2 : K);
-        const CUtensorMap* my_b = (SWIGLU && !leader) ? &maps_b2.m[me] : &maps_b.m[me];
+        const int e_n = NE > 1 ? 0 : tl.e * N, e_k = NE > 1 ? 0 : tl.e * (KIND == 3 ? K / 2 : K);
+        const CUtensorMap* my_b = &maps_b.m[me];
+        const uint32_t bytes = 2u * (A_BYTES + half * BK * 2);
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(empty_bar(s), ph ^ 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
-          const uint32_t a_dst = smem_base + s * STAGE_BYTES;
-          const uint32_t b_dst = a_dst + A_BYTES;
+          if (!mbar_wait(empty_bar(s), ((it / STAGES) & 1) ^ 1, status, KF_ERR_WAIT_EMPTY)) { ok = false; break; }
+          const uint32_t w_dst = smem_base + s * STAGE_BYTES;
           const uint32_t lead_full = full_bar(s) & PEER_BIT_MASK;
-          if (leader) mbar_expect_tx(full_bar(s), 2 * STAGE_BYTES);
+          if (leader) mbar_expect_tx(full_bar(s), bytes);
           const int k0 = kb * BK;
-          tma_load_2d_pair(a_dst, &map_a, lead_full, k0, m0);
+          tma_load_2d_pair(w_dst + A_BYTES, my_a, lead_full, k0, n0);
           int kw = k0;                                 // reduction index inside the weight
-          if (EPI == 3 && k0 >= K / 2) {
+          if (KIND == 3 && k0 >= K / 2) {
             my_b = &maps_b2.m[me];
             kw = k0 - K / 2;
           }
-          if (!B_MN) {
-            tma_load_2d_pair(b_dst, my_b, lead_full, kw, e_n + n0);
+          if constexpr (B_MN) {  // two boxes of 64 features; SwiGLU: 64 gate units, the 64 matching up units
+            tma_load_2d_pair(w_dst, my_b, lead_full, f0, e_k + kw);
+            if constexpr (SWIGLU) tma_load_2d_pair(w_dst + A_BYTES / 2, &maps_b2.m[me], lead_full, f0, e_k + kw);
+            else tma_load_2d_pair(w_dst + A_BYTES / 2, my_b, lead_full, f0 + 64, e_k + kw);
+          } else if constexpr (SWIGLU) {
+            tma_load_2d_pair(w_dst, my_b, lead_full, kw, e_n + f0);
+            tma_load_2d_pair(w_dst + A_BYTES / 2, &maps_b2.m[me], lead_full, kw, e_n + f0);
           } else {
-#pragma unroll
-            for (int c = 0; c < HALF_N / 64; ++c)
-              tma_load_2d_pair(b_dst + c * (64 * BK * 2), my_b, lead_full, n0 + 64 * c, e_k + kw);
+            tma_load_2d_pair(w_dst, my_b, lead_full, kw, e_n + f0);
           }
         }
       }
@@ -155,27 +190,25 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
     if (leader && elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(TILE_M, TILE_N, false, B_MN);
       int it = 0, tile_iter = 0;
       bool ok = true;
+      TokenTiles walk(offsets, f_blocks, widest);
       for (int t = pair; t < num_tiles && ok; t += num_pairs, ++tile_iter) {
+        const uint32_t idesc = umma_idesc_bf16(TILE_M, walk.at(t).width, B_MN, false);
         const int acc = tile_iter & 1;
-        const uint32_t acc_ph = (tile_iter >> 1) & 1;
-        if (!mbar_wait(tempty_bar(acc), acc_ph ^ 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
+        if (!mbar_wait(tempty_bar(acc), ((tile_iter >> 1) & 1) ^ 1, status, KF_ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * TILE_N;
+        const uint32_t d_tmem = tmem_base + acc * MAX_N;
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(full_bar(s), ph, status, KF_ERR_WAIT_FULL)) { ok = false; break; }
+          if (!mbar_wait(full_bar(s), (it / STAGES) & 1, status, KF_ERR_WAIT_FULL)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t a_src = smem_base + s * STAGE_BYTES;
-          const uint32_t b_src = a_src + A_BYTES;
+          const uint32_t w_src = smem_base + s * STAGE_BYTES, a_src = w_src + A_BYTES;
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t bd = B_MN ? umma_desc_sw128(b_src + k * (UMMA_K * 128), 64 * BK * 2, 1024)
-                                     : umma_desc_sw128(b_src + k * (UMMA_K * 2), 16, 1024);
-            mma_pair_f16(d_tmem, umma_desc_sw128(a_src + k * (UMMA_K * 2), 16, 1024), bd, idesc, (kb | k) != 0);
+            const uint64_t wd = B_MN ? umma_desc_sw128(w_src + k * (UMMA_K * 128), 64 * BK * 2, 1024)
+                                     : umma_desc_sw128(w_src + k * (UMMA_K * 2), 16, 1024);
+            mma_pair_f16(d_tmem, wd, umma_desc_sw128(a_src + k * (UMMA_K * 2), 16, 1024), idesc, (kb | k) != 0);
           }
           commit_pair(empty_bar(s));
         }
@@ -190,65 +223,15 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
     // ------------------------------------------------------------ epilogue (warps 2..5 of both CTAs)
     const int quarter = warp & 3;
     int tile_iter = 0;
-    bool ok = true;
-    for (int t = pair; t < num_tiles && ok; t += num_pairs, ++tile_iter) {
-      const Tile tl = tilemath::grouped_decode(t, n_blocks, tile_start, offsets, E, TILE_M);
+    TokenTiles walk(offsets, f_blocks, widest);
+    for (int t = pair; t < num_tiles; t += num_pairs, ++tile_iter) {
+      const auto tl = walk.at(t);
       const int acc = tile_iter & 1;
-      const int r0 = int(rank) * CTA_M + quarter * 32;  // first row of this warp inside the 256-row tile
-      const int rows = max(0, min(32, tl.valid - r0));  // how many of its 32 rows belong to the expert
-      const int col0 = tl.nb * TN, width = min(TN, N - col0);
-      const uint32_t box = box_smem + uint32_t(quarter * 2) * BOX_BYTES, box2 = box + BOX_BYTES;
-      __nv_bfloat16* c0 = C + size_t(tl.row0 + r0) * ldc + col0;
-      __nv_bfloat16* gu0 = GU ? GU + size_t(tl.row0 + r0) * ldgu + col0 : nullptr;
-      Rows32 g_next, u_next;
-      if constexpr (EPI == 2) {  // the first pre-activations travel while the tile's products are still running
-        g_next = load_rows32(gu0, ldgu, lane, rows, width);
-        u_next = load_rows32(gu0 + N, ldgu, lane, rows, width);
-      }
-      if (!mbar_wait(tfull_bar(acc), (tile_iter >> 1) & 1, status, KF_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
-      tc_fence_after();
-      const uint32_t t_row = tmem_base + (uint32_t(quarter * 32) << 16) + acc * TILE_N;
-#pragma unroll 1
-      for (int c = 0; c * 32 < width; ++c) {
-        const int cols = min(32, width - c * 32);
-        if constexpr (EPI == 2) {
-          // SwiGLU backward: the accumulator is dh[rows, F] (never written); GU = the saved pre-activations [rows, 2F]
-          // (gate | up), C = d[gate | up] [rows, 2F] (may be the same buffer: a warp reads a chunk before it writes it, and
-          // no other warp touches its rows)
-          uint32_t v[32];
-          tmem_ld_32x32(t_row + c * 32, v);
-          const Rows32 g_now = g_next, u_now = u_next;  // chunk c + 1 is fetched while chunk c is worked on
-          if ((c + 1) * 32 < width) {
-            g_next = load_rows32(gu0 + (c + 1) * 32, ldgu, lane, rows, width - (c + 1) * 32);
-            u_next = load_rows32(gu0 + N + (c + 1) * 32, ldgu, lane, rows, width - (c + 1) * 32);
-          }
-          Rows32 g = to_own_row(box, lane, g_now), u = to_own_row(box2, lane, u_now);
-          tmem_ld_wait();
-          swiglu_bwd_row(v, g, u);
-          store_rows32(box, lane, g, c0 + c * 32, ldc, rows, cols);
-          store_rows32(box2, lane, u, c0 + N + c * 32, ldc, rows, cols);
-        } else if constexpr (SWIGLU) {
-          uint32_t g[32], u[32];
-          tmem_ld_32x32(t_row + c * 32, g);
-          tmem_ld_32x32(t_row + TN + c * 32, u);
-          tmem_ld_wait();
-          if (gu0) {
-            store_rows32(box, lane, pack_row32(g), gu0 + c * 32, ldgu, rows, cols);
-            store_rows32(box2, lane, pack_row32(u), gu0 + N + c * 32, ldgu, rows, cols);
-          }
-          swiglu_chunk(g, u);
-          store_rows32(box, lane, pack_row32(g), c0 + c * 32, ldc, rows, cols);
-        } else {
-          uint32_t v[32];
-          tmem_ld_32x32(t_row + c * 32, v);
-          tmem_ld_wait();
-          if (accumulate) {
-            if (lane < rows) store_chunk<__nv_bfloat16>(c0 + size_t(lane) * ldc + c * 32, v, cols, true, nullptr);
-          } else {
-            store_rows32(box, lane, pack_row32(v), c0 + c * 32, ldc, rows, cols);
-          }
-        }
-      }
+      const bool ok = kf2::tokens::tile_epilogue<KIND == 1 ? 1 : KIND == 2 ? 3 : 0>(
+          out, box_smem, quarter, lane, tl.fb * TILE_F + int(rank) * CTA_F, tl.row0, tl.valid,
+          tmem_base + (uint32_t(quarter * 32) << 16) + acc * MAX_N,
+          [&] { return mbar_wait(tfull_bar(acc), (tile_iter >> 1) & 1, status, KF_ERR_WAIT_TMEM_FULL); });
+      if (!ok) break;
       tc_fence_before();
       __syncwarp();
       if (lane == 0) arrive_on_cta(tempty_bar(acc), 0);
@@ -264,57 +247,60 @@ kf_grouped_gemm_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __
   }
 }
 
-template <bool B_MN, int EPI, int NE>
-static int launch(const CUtensorMap& ma, const Maps<NE>& mb, const Maps<(EPI & 1) ? NE : 1>& mb2, void* C, void* GU,
-                  const void* offsets, int E, int N, int K, long long ldc, long long ldgu, int accumulate, int pairs,
-                  cudaStream_t st, int* status) {
-  auto kern = kf_grouped_gemm_tcgen05_2cta<B_MN, EPI, NE>;
+template <bool B_MN, int KIND, int NE>
+static int launch(const Maps<8>& ma, const Maps<NE>& mb, const Maps<(KIND & 1) ? NE : 1>& mb2, const Output& out,
+                  const void* offsets, int E, int N, int K, int pairs, cudaStream_t st, int* status) {
+  auto kern = kf_grouped_gemm_tcgen05_2cta<B_MN, KIND, NE>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
     if (e != cudaSuccess) return 300 + (int)e;
     attr_set = true;
   }
-  kern<<<pairs * 2, THREADS, SMEM, st>>>(ma, mb, mb2, reinterpret_cast<__nv_bfloat16*>(C), reinterpret_cast<__nv_bfloat16*>(GU),
-                                         reinterpret_cast<const int*>(offsets), E, N, K, ldc, ldgu, accumulate, status);
+  kern<<<pairs * 2, THREADS, SMEM, st>>>(ma, mb, mb2, out, reinterpret_cast<const int*>(offsets), E, N, K, status);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
 // Weight operand: the packed tensor (NE == 1, *w) or one pointer per expert.  Each expert's matrix is [N][K] (K
-// contiguous, boxes of 128 rows) or, b_mn, [K][N] (N contiguous, 64 x 64 boxes).
+// contiguous, boxes of `box` rows) or, b_mn, [K][N] (N contiguous, 64 x 64 boxes).
 template <int NE>
-static int make_weight_maps(Maps<NE>& m, const void* const* w, int E, int N, int K, int b_mn) {
+static int make_weight_maps(Maps<NE>& m, const void* const* w, int E, int N, int K, int b_mn, int box) {
   for (int e = 0; e < (NE > 1 ? E : 1); ++e) {
     const uint64_t n = NE > 1 ? 1 : E;
-    const int rc = b_mn ? make_map_2d_bf16(&m.m[e], w[e], n * K, N, N, 64, BK) : make_map_2d_bf16(&m.m[e], w[e], n * N, K, K, BK, HALF_N);
+    const int rc = b_mn ? make_map_2d_bf16(&m.m[e], w[e], n * K, N, N, 64, BK) : make_map_2d_bf16(&m.m[e], w[e], n * N, K, K, BK, box);
     if (rc) return rc;
   }
   return 0;
 }
 
-static int pair_count(int rows, int E, int n_blocks, int num_sms) {
-  const int upper = ((rows + TILE_M - 1) / TILE_M + E) * n_blocks;  // at most one partial tile per expert
-  return upper < num_sms / 2 ? upper : num_sms / 2;
-}
-
-template <int EPI, int NE>
+template <int KIND, int NE>
 static int run(const void* A, const void* const* W, const void* const* W2, void* C, void* GU, const void* offsets, int rows,
                int E, int N, int K, int KW, long long lda, long long ldc, long long ldgu, int b_mn, int accumulate, int num_sms,
                cudaStream_t st, int* status) {
-  CUtensorMap ma;
+  if (ldc > 0x7fffffffll || ldgu > 0x7fffffffll) return 6;
+  Maps<8> ma;
   Maps<NE> mb;
-  Maps<(EPI & 1) ? NE : 1> mb2;
-  int rc = make_map_2d_bf16(&ma, A, rows, K, lda, BK, CTA_M);
+  Maps<(KIND & 1) ? NE : 1> mb2;
+  int rc = 0;
+  for (int i = 0; i < 8 && !rc; ++i) rc = make_map_2d_bf16(&ma.m[i], A, rows, K, lda, BK, 16 * (i + 1));
   if (rc) return 100 + rc;
-  rc = make_weight_maps<NE>(mb, W, E, N, KW, b_mn);
-  if (!rc && (EPI & 1)) rc = make_weight_maps<(EPI & 1) ? NE : 1>(mb2, W2, E, N, KW, b_mn);
+  rc = make_weight_maps<NE>(mb, W, E, N, KW, b_mn, KIND == 1 ? CTA_M / 2 : CTA_M);
+  if (!rc && (KIND & 1)) rc = make_weight_maps<(KIND & 1) ? NE : 1>(mb2, W2, E, N, KW, b_mn, KIND == 1 ? CTA_M / 2 : CTA_M);
   if (rc) return 200 + rc;
-  if (!(EPI & 1)) mb2.m[0] = mb.m[0];
-  const int tn = EPI == 1 ? HALF_N : TILE_N;
-  const int pairs = pair_count(rows, E, (N + tn - 1) / tn, num_sms);
-  return b_mn ? launch<true, EPI, NE>(ma, mb, mb2, C, GU, offsets, E, N, K, ldc, ldgu, accumulate, pairs, st, status)
-              : launch<false, EPI, NE>(ma, mb, mb2, C, GU, offsets, E, N, K, ldc, ldgu, accumulate, pairs, st, status);
+  if (!(KIND & 1)) mb2.m[0] = mb.m[0];
+  Output out{};
+  out.out = reinterpret_cast<__nv_bfloat16*>(C);
+  out.aux = reinterpret_cast<const __nv_bfloat16*>(KIND == 1 || KIND == 2 ? GU : accumulate ? C : nullptr);
+  out.F = N;
+  out.ldo = (int)ldc;
+  out.lda = (int)(KIND == 1 || KIND == 2 ? ldgu : ldc);
+  const int tile_f = KIND == 1 ? TILE_M / 2 : TILE_M;
+  // at most so many tiles: the narrowest, one partial tile per expert
+  const long long upper = ((long long)(rows / tilemath::NARROWEST_TOKENS) + E) * ((N + tile_f - 1) / tile_f);
+  const int pairs = upper < num_sms / 2 ? (int)upper : num_sms / 2;
+  return b_mn ? launch<true, KIND, NE>(ma, mb, mb2, out, offsets, E, N, K, pairs, st, status)
+              : launch<false, KIND, NE>(ma, mb, mb2, out, offsets, E, N, K, pairs, st, status);
 }
 
 // Contracts of kf_grouped_gemm_acc_bf16 / kf_grouped_swiglu_bf16 (grouped_gemm_tcgen05.cu), which dispatch here.

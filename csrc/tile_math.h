@@ -77,6 +77,55 @@ KF_TM_HD GroupedTile grouped_decode(int t, int n_blocks, const int* tile_start, 
   return x;
 }
 
+// Ragged grouped GEMM with tokens as the N side of the MMA: expert e's rows are cut into n = ceil(rows / widest) tiles of
+// token_tile_width(rows, n) tokens (the last one may hold fewer, never none), each met by every block of weight rows.
+constexpr int NARROWEST_TOKENS = 96;  // below, a tile takes no less time
+KF_TM_HD int token_tile_width(int rows, int n) { return n > 0 ? ceil_div(ceil_div(rows, n), 32) * 32 : 0; }
+
+// What a tile takes, in units of one token's share of a k-block on a CTA pair.  Measured, ns per k-block of 64: 96 tokens 210, 128 245, 160
+// 285, 192 330, 224 390, 256 430 (products of 4096 and 28 672 rows with 4096 columns, back to back).
+KF_TM_HD int token_tile_cost(int width) { return 48 + (width < NARROWEST_TOKENS ? NARROWEST_TOKENS : width); }
+
+// Rounds of `tiles` x `f_blocks` tiles over the pairs, times the average tile.
+KF_TM_HD float token_rounds_cost(int tiles, int cost, int f_blocks, int pairs) {
+  if (tiles == 0) return 0.f;
+  const long long all = (long long)tiles * f_blocks;
+  return float((all + pairs - 1) / pairs) * (float(cost) / float(tiles));
+}
+
+struct TokenTile {
+  int e, fb;       // expert and block of weight rows
+  int row0;        // first row of the tile in the sorted activation matrix
+  int valid;       // rows of the tile that belong to the expert (1 .. width)
+  int width;       // tokens of the tile as computed (a multiple of 32 up to the widest)
+};
+
+// Walks the tiles in ascending order of their linear index (experts slowest, token tiles fastest); experts without rows own none.
+struct TokenTiles {
+  const int* offsets;
+  int f_blocks, widest;
+  int e, first, n;  // current expert, its first tile, its token tiles
+  KF_TM_HD TokenTiles(const int* off, int fb, int w) : offsets(off), f_blocks(fb), widest(w), e(0), first(0) {
+    n = ceil_div(off[1] - off[0], w);
+  }
+  KF_TM_HD TokenTile at(int t) {
+    while (t >= first + n * f_blocks) {
+      first += n * f_blocks;
+      ++e;
+      n = ceil_div(offsets[e + 1] - offsets[e], widest);
+    }
+    const int r = t - first, rows = offsets[e + 1] - offsets[e];
+    TokenTile x;
+    x.e = e;
+    x.fb = r / n;
+    x.width = token_tile_width(rows, n);
+    const int at = (r - x.fb * n) * x.width;
+    x.row0 = offsets[e] + at;
+    x.valid = imin(x.width, rows - at);
+    return x;
+  }
+};
+
 struct WgradTile {
   int e, m0, n0;  // expert, first output row / column of the tile
   int row0, rows; // the expert's range of the reduction dimension

@@ -468,7 +468,7 @@ def swiglu_mlp(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, wd: torch.Te
     cu = _cuda()
     d, f = x.shape[-1], wg.shape[0]
     rows = x.numel() // d
-    if rows < 256 or d % 64 or f % 256 or wg.shape != (f, d) or wu.shape != (f, d) or wd.shape != (d, f):
+    if rows < 256 or d % 64 or f % 128 or wg.shape != (f, d) or wu.shape != (f, d) or wd.shape != (d, f):
         return None
     for w in (wg, wu, wd):
         if (w.dtype != torch.bfloat16 or w.device != x.device or not w.is_contiguous() or w.data_ptr() % 16

@@ -99,6 +99,41 @@ static void test_wgrad() {
     }
 }
 
+// every row of every expert meets every block of weight rows once, in tiles of the walk; the tiles of an expert are equal but the last
+static void test_token_tiles() {
+  std::vector<std::vector<int>> cases = {{0}, {1}, {256}, {257}, {0, 0, 513, 0}, {5, 0, 300, 77, 130, 1}, {1000, 24, 31, 32, 33},
+                                         {95, 96, 97, 191, 192, 193, 287, 288, 289}};
+  cases.emplace_back(256, 3);
+  for (const auto& counts : cases)
+    for (int widest = 256; widest >= NARROWEST_TOKENS; widest -= 32)
+      for (int f_blocks : {1, 3, 11}) {
+        const int E = int(counts.size());
+        std::vector<int> offsets(static_cast<size_t>(E) + 1, 0);
+        int tiles = 0;
+        for (int e = 0; e < E; ++e) {
+          offsets[e + 1] = offsets[e] + counts[e];
+          tiles += ceil_div(counts[e], widest);
+        }
+        const size_t cells = static_cast<size_t>(offsets[E]) * static_cast<size_t>(f_blocks);
+        std::vector<int> seen(cells, 0);
+        for (int start = 0; start < 3; ++start) {   // a walk that skips tiles, as one pair of several does
+          TokenTiles walk(offsets.data(), f_blocks, widest);
+          for (int t = start; t < tiles * f_blocks; t += 3) {
+            const TokenTile x = walk.at(t);
+            CHECK(x.e >= 0 && x.e < E && x.fb >= 0 && x.fb < f_blocks);
+            if (x.e < 0 || x.e >= E || x.fb < 0 || x.fb >= f_blocks) return;
+            CHECK(x.width % 32 == 0 && x.width >= 32 && x.width <= widest && x.valid >= 1 && x.valid <= x.width);
+            CHECK(x.row0 >= offsets[x.e] && x.row0 + x.valid <= offsets[x.e + 1]);
+            CHECK(x.valid == x.width || x.row0 + x.valid == offsets[x.e + 1]);
+            if (x.row0 < offsets[x.e] || x.row0 + x.valid > offsets[x.e + 1]) return;
+            for (int r = 0; r < x.valid; ++r) seen[size_t(x.row0 + r) * f_blocks + x.fb] += 1;
+          }
+        }
+        for (int v : seen) CHECK(v == 1);
+      }
+  CHECK(token_rounds_cost(0, 0, 5, 74) == 0.f && token_rounds_cost(74, 74 * 10, 1, 74) == 10.f && token_rounds_cost(75, 750, 1, 74) == 20.f);
+}
+
 // the chunks cleared at the ragged end of a reduction range are exactly the rows valid..bk-1 of every block
 static void test_tail_chunks() {
   const int bk = 64, blocks = 6, block_bytes = 64 * bk * 2;
@@ -126,6 +161,7 @@ int main() {
   test_raster();
   test_grouped();
   test_wgrad();
+  test_token_tiles();
   test_tail_chunks();
   if (failures) {
     std::fprintf(stderr, "%d check(s) failed\n", failures);

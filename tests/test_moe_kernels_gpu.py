@@ -111,3 +111,61 @@ def test_forms_the_separate_path_does_not_cover_return_none(native_lib):
     assert grouped.separate_ffn(x, off(2), *weights(2, 128, 128, torch.float32)) is None
     g, u, dn = weights(2, 128, 128)
     assert grouped.separate_ffn(x, off(2), [torch.zeros(128, 256, device=DEV, dtype=torch.bfloat16)[:, ::2]] * 2, u, dn) is None
+
+
+@pytest.mark.parametrize("counts", [[1], [32, 31, 33], [96, 97, 95, 0], [256, 257, 255], [0, 513, 0, 289, 2], [192, 193, 161, 160] * 4, [7] * 250])
+@pytest.mark.parametrize("b_mn", [False, True])
+@pytest.mark.parametrize("n,k", [(136, 128), (264, 192)])
+def test_grouped_products_on_token_tiles(native_lib, counts, b_mn, n, k):
+    """All four products against fp32 at the edges of the token tiles and with partial blocks of weight rows; rows that belong to no
+    expert are not written, and what they hold (NaN) reaches no other row."""
+    e, rows = len(counts), sum(counts)
+    extra = 40
+    off = torch.zeros(e + 1, dtype=torch.int32, device=DEV)
+    off[1:] = torch.tensor(counts, device=DEV).cumsum(0)
+    expert = torch.repeat_interleave(torch.arange(e, device=DEV), torch.tensor(counts, device=DEV))
+    gen = _gen(rows)
+
+    def rand(*s, std=1.0):
+        return (std * torch.randn(*s, device=DEV, generator=gen)).bfloat16()
+
+    def padded(t):
+        return torch.cat([t, torch.full((extra, t.shape[1]), float("nan"), device=DEV, dtype=t.dtype)])
+
+    shape = (e, k, n) if b_mn else (e, n, k)
+    w, w2 = rand(*shape, std=0.1), rand(*shape, std=0.1)
+    mats = [(v if b_mn else v.transpose(1, 2)).float() for v in (w, w2)]   # (E, K, N)
+    a = rand(rows, 2 * k)
+    gu = rand(rows, 2 * n)
+    by = lambda x, m: torch.bmm(x.float()[:, None], m[expert])[:, 0]      # noqa: E731
+
+    def fresh(cols):
+        return torch.full((rows + extra, cols), 77.0, device=DEV, dtype=torch.bfloat16)
+
+    def check(got, want, size, rel=2.0**-7):
+        # a rounding to bf16 (2^-8 of the value) and the sum: every 16 products are added to an accumulator that keeps 23 bits of the
+        # larger one, 2 k / 16 <= 24 times at most, so 2^-18 of the sum of magnitudes
+        assert ((got[:rows].float() - want).abs() <= want.abs() * rel + size * 2.0**-18).all()
+        assert (got[rows:] == 77.0).all()
+
+    a1 = a[:, :k].contiguous()
+    big = [by(v.abs(), m.abs()) for v, m in ((a1, mats[0]), (a1, mats[1]), (a[:, k:], mats[1]))]
+    y = fresh(n)
+    native_lib.grouped_experts(0, padded(a1), w, None, off, n, b_mn, y)
+    want = by(a1, mats[0])
+    check(y, want, big[0])
+    h, pre = fresh(n), fresh(2 * n)
+    native_lib.grouped_experts(1, padded(a1), w, w2, off, n, b_mn, h, pre)
+    up = by(a1, mats[1])
+    check(pre, torch.cat([want, up], 1), torch.cat(big[:2], 1))
+    check(h, torch.nn.functional.silu(pre[:rows, :n].float()) * pre[:rows, n:].float(), 1e-2)
+    d = fresh(2 * n)
+    native_lib.grouped_experts(2, padded(a1), w, None, off, n, b_mn, d, padded(gu))
+    g, u, dh = gu[:, :n].float(), gu[:, n:].float(), want.bfloat16().float()
+    s = torch.sigmoid(g)
+    check(d, torch.cat([dh * u * s * (1 + g * (1 - s)), dh * g * s], 1), 5 * torch.cat([big[0]] * 2, 1),   # |u|, |g| up to 5
+          rel=2.0**-6)   # a whole step of dh (2^-7) where the two sums round apart, and the rounding of the product
+    dx = fresh(n)
+    native_lib.grouped_experts(3, padded(a), w, w2, off, n, b_mn, dx)
+    check(dx, want + by(a[:, k:], mats[1]), big[0] + big[2])
+    assert native_lib.read_status() == 0
