@@ -9,6 +9,7 @@ no silent fallback to library kernels.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import math
 import os
 from array import array
@@ -16,7 +17,7 @@ from ctypes import c_float, c_int, c_longlong, c_void_p
 
 import torch
 
-from kempnerforge_b200.ops.build import LIB_PATH
+from kempnerforge_b200.ops.build import LIB_PATH, STEPS_PATH
 
 _lib = None
 GEMM_MODE = int(os.environ.get("KF_GEMM_MODE", "0"))  # 0 = automatic, 1 = single CTA tiles, 2 = CTA pairs
@@ -471,34 +472,40 @@ def block_decode(y: torch.Tensor, attn_ptrs, mlp_ptrs, cache_ptrs, table_ptrs, d
     _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 5 + 2 * norms if mlp_ptrs else 3 + norms)
 
 
-def blocks_decode(x: torch.Tensor, xp: int, plans, table_ptrs) -> torch.Tensor:
-    """One new token per sequence through a row of blocks (``plans``: what ``fused_infer._plan`` made of them, all with an MLP and
-    an attention that ``kf_block_decode_bf16`` runs itself) as one native call.  The blocks share one buffer of intermediates and
-    hand x on through two more: each kernel of the chain writes only after all before it are complete."""
-    b, _, d = x.shape
-    n = len(plans)
-    # n (D) | q (H hd) | hidden (F) | h1 (D) | attention (H hd) | the outputs of even and of odd blocks | rstd, lse
-    cols = max(2 * d + 2 * p.h * p.hd + p.f for p in plans)
-    lse = 2 * max(p.h for p in plans)
-    scratch = torch.empty(b * cols + 2 * b + lse + 2 * b * d, dtype=torch.bfloat16, device=x.device)
-    y = torch.empty_like(x)
-    base = scratch.data_ptr()
-    hand = [base + 2 * b * cols, base + 2 * b * (cols + d)]
-    rstd = base + 2 * b * (cols + 2 * d)
-    sms = sm_count()
-    ints, reals = array("q"), array("d")
-    launches, src = 0, xp
-    norms = 0 if b <= lib().kf_skinny_norm_rows() else 1
-    for i, p in enumerate(plans):
-        h1 = base + 2 * b * (d + p.h * p.hd + p.f)
-        dst = y.data_ptr() if i == n - 1 else hand[i & 1]
-        ints.extend((src, *p.attn_ptrs, *p.mlp_ptrs, *p.cache_ptrs, base, rstd, h1, dst, *table_ptrs, b, d, p.h, p.hkv, p.hd, p.f, p.past,
-                     p.batch_step, sms, 7, int(p.hd == 64), h1 + 2 * b * d, rstd + 4 * b))
-        reals.extend((p.eps1, p.eps2, 1.0 / math.sqrt(p.hd)))
-        launches += 5 + 2 * norms
-        src = dst
-    _check(lib().kf_blocks_decode_bf16(ints.buffer_info()[0], reals.buffer_info()[0], n, _stream()), "kf_blocks_decode_bf16", launches)
-    return y
+_steps = None
+
+
+def _load_steps():
+    """The CPython module of ``csrc/steps.cpp``, told the classes it looks for and the native entry."""
+    global _steps
+    if not STEPS_PATH.exists():
+        raise NativeKernelError(f"native module {STEPS_PATH} is missing; run `python -m kempnerforge_b200.ops.build`")
+    from kempnerforge_b200.models.attention import Attention, KVCache
+    from kempnerforge_b200.models.mlp import SwiGLUMLP
+    from kempnerforge_b200.models.norm import RMSNorm
+
+    spec = importlib.util.spec_from_file_location("kf_steps", STEPS_PATH)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    mod.configure(Attention, SwiGLUMLP, RMSNorm, KVCache, torch.nn.Parameter,
+                  ctypes.cast(lib().kf_blocks_decode_bf16, c_void_p).value, SKINNY_MAX_ROWS, lib().kf_skinny_norm_rows())
+    _steps = mod
+    return mod
+
+
+def blocks_decode(blocks: list, caches: list, x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, foreign=None):
+    """One new token per sequence through a row of plain blocks (attention on our kernels and a SwiGLU MLP) as one native call that
+    checks them as well (``csrc/steps.cpp``): the last block's output (B, 1, D), or None when one of them is not plainly
+    covered.  Without ``foreign`` the call stands for the blocks themselves, so hooks on them count; a block that calls it
+    gives its ``foreign(q (B, H hd), H, hd, position)`` -> (B, H hd) for the attention of heads of 64 over several sequences."""
+    r = (_steps or _load_steps()).decode(blocks, caches, x, cos, sin, foreign, _stream(), sm_count())
+    if r is None:
+        return None
+    if type(r) is int:
+        raise NativeKernelError(f"kf_blocks_decode_bf16 failed with code {r}")
+    global LAUNCH_COUNT
+    LAUNCH_COUNT += r[1]
+    return r[0]
 
 
 # --------------------------------------------------------------------------- norm / rope / swiglu / embedding

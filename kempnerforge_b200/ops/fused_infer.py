@@ -6,7 +6,8 @@ o projection with the residual, RMSNorm, gate|up with SwiGLU, down with the resi
 or a plain forward pass, uses the epilogue-fused GEMMs of the training block and reads q | k | v from the projection's own
 buffer.  The weights of separate ``nn.Linear`` modules are read where they are: nothing is concatenated.
 
-All blocks of a model on one new token are one native call (:func:`run_layers`).
+All blocks of a model on one new token are one native call (:func:`run_layers`).  A step through plain blocks is checked in
+native code too (``csrc/steps.cpp``), by the rules of :func:`_plan`, which decides about every other call.
 
 What the fused form does not cover (masks, hooks, q/k norms, tensor parallelism, fp8, captured attention weights, a prompt
 behind a non-empty cache, foreign module types) returns None and takes the op-by-op path.
@@ -126,32 +127,12 @@ def _one_token(b: int, cos, sin) -> bool:
 
 
 def run_layers(layers, x, cos, sin, caches):
-    """One new token per sequence through all of a model's blocks as one native call: the last block's output (B, 1, D), or None
-    when some block is not covered (nothing has been done then).  Issued block by block, Python takes 50 us per block, more
-    than the 18 us that the five kernels of a small one run."""
+    """One new token per sequence through all of a model's blocks as one native call, checks included: the last block's output
+    (B, 1, D), or None when some block is not plainly covered (nothing has been done then).  Issued block by block, Python takes
+    50 us per block, more than the 18 us that the five kernels of a small one run."""
     if x.dim() != 3 or x.size(1) != 1 or not layers or len(caches) < len(layers) or _refused():
         return None
-    b, _, d = x.shape
-    plans = []
-    for block, cache in zip(layers, caches):
-        if not _plain(block) or cache is None:
-            return None
-        p = _plan(block, b, 1, d, cos, sin, cache)
-        # heads of 64 for several sequences go through the library's attention, one block at a time
-        if p is None or p.mlp_ptrs is None or (p.hd == 64 and b > 1) or not _one_token(b, cos, sin):
-            return None
-        plans.append(p)
-    if len({id(c) for c in caches[: len(plans)]}) != len(plans):
-        return None
-    if not x.is_contiguous():
-        x = x.contiguous()
-    xp = x.data_ptr()
-    if xp & 15:
-        return None
-    y = kc.blocks_decode(x, xp, plans, (cos.data_ptr(), sin.data_ptr()))
-    for p, cache in zip(plans, caches):
-        cache.seq_len = p.past + 1
-    return y
+    return kc.blocks_decode(list(layers), list(caches), x if x.is_contiguous() else x.contiguous(), cos, sin)
 
 
 def run(block, x, cos, sin, cache):
@@ -159,6 +140,14 @@ def run(block, x, cos, sin, cache):
     if x.dim() != 3 or _refused():
         return None
     b, s, d = x.shape
+    if s == 1 and type(cache) is KVCache:   # a generation step of a plain block is checked and issued by one native call
+        def foreign(q2, h, hd, past):
+            out = F.attention(q2.unflatten(1, (h, hd)).unsqueeze(1), cache.k[:, : past + 1], cache.v[:, : past + 1], causal=False)
+            return out.reshape(b, h * hd)   # SDPA's output is a transposed view
+
+        y = kc.blocks_decode([block], [cache], x if x.is_contiguous() else x.contiguous(), cos, sin, foreign)
+        if y is not None:
+            return y
     p = _plan(block, b, s, d, cos, sin, cache)
     if p is None:
         return None
@@ -177,12 +166,9 @@ def run(block, x, cos, sin, cache):
             return None
         y = torch.empty((b, 1, d), dtype=_BF16, device=x.device)
 
-        def foreign(q2):
-            out = F.attention(q2.unflatten(1, (h, hd)).unsqueeze(1), cache.k[:, : past + 1], cache.v[:, : past + 1], causal=False)
-            return out.reshape(b, qc)   # SDPA's output is a transposed view
-
         kc.block_decode(y, (xp, *p.attn_ptrs), p.mlp_ptrs, p.cache_ptrs, (cos.data_ptr(), sin.data_ptr()),
-                        (b, d, h, hkv, hd, p.f, past, p.batch_step), (p.eps1, p.eps2, scale), foreign)
+                        (b, d, h, hkv, hd, p.f, past, p.batch_step), (p.eps1, p.eps2, scale),
+                        lambda q2: foreign(q2, h, hd, past))
         cache.seq_len = past + 1
         return y if g2 else y + mlp(block.mlp_norm(y))
     if past:
