@@ -391,26 +391,10 @@ __global__ void kf_rope(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __re
 }
 
 // ------------------------------------------------------------------ SwiGLU on stacked [gate | up]
-// amax (optional, [gridDim.x]): largest magnitude that each block stored, for a tensor that is cast to fp8 next.  A pass of its
-// own would read it again: 57 MB of hidden activations forward and 115 MB of gradients backward at 2000 tokens x 14 336 (42 -> 12 us
-// for the maxima of an fp8 feed-forward with its backward).  The whole call: 1253 -> 1234 and 1260 -> 1242 us in two comparisons, in which
-// the runs of one side differed by 1.3 and 1.7 %.
-__device__ __forceinline__ float absmax_stored(const F8& v, float m) {  // of the values after rounding to bf16
-#pragma unroll
-  for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(__bfloat162float(__float2bfloat16(v.v[i]))));
-  return m;
-}
-__device__ __forceinline__ void store_block_max(float m, float* amax) {
-  __shared__ float red[40];
-  m = block_max(m, red);
-  if (threadIdx.x == 0) amax[blockIdx.x] = m;
-}
-
 __global__ void kf_swiglu_fwd(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h,
-                              long long rows, int H, float* __restrict__ amax) {
+                              long long rows, int H) {
   const int vec = H >> 3;
   const long long total = rows * vec;
-  float m = 0.f;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
     const long long r = idx / vec;
@@ -420,18 +404,14 @@ __global__ void kf_swiglu_fwd(const __nv_bfloat16* __restrict__ gu, __nv_bfloat1
 #pragma unroll
     for (int i = 0; i < 8; ++i) o.v[i] = a.v[i] / (1.f + __expf(-a.v[i])) * b.v[i];
     store8(h + size_t(r) * H + v * 8, o);
-    if (amax) m = absmax_stored(o, m);
   }
-  if (amax) store_block_max(m, amax);
 }
 
 // rows_ptr (optional, device int): only the first min(rows, *rows_ptr) rows are touched (ragged expert activations
 // whose buffers are sized by an upper bound known on the host).
 __global__ void kf_swiglu_bwd(const __nv_bfloat16* __restrict__ dh, const __nv_bfloat16* __restrict__ gu,
-                              __nv_bfloat16* __restrict__ dgu, long long rows, int H, const int* __restrict__ rows_ptr,
-                              float* __restrict__ amax) {
+                              __nv_bfloat16* __restrict__ dgu, long long rows, int H, const int* __restrict__ rows_ptr) {
   const int vec = H >> 3;
-  float m = 0.f;
   if (rows_ptr) rows = min(rows, (long long)*rows_ptr);
   const long long total = rows * vec;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
@@ -449,9 +429,7 @@ __global__ void kf_swiglu_bwd(const __nv_bfloat16* __restrict__ dh, const __nv_b
     }
     store8(dgu + off, da);
     store8(dgu + off + H, db);
-    if (amax) m = absmax_stored(db, absmax_stored(da, m));
   }
-  if (amax) store_block_max(m, amax);
 }
 
 // ------------------------------------------------------------------ embedding
@@ -837,37 +815,15 @@ int kf_swiglu_fwd_bf16(const void* gu, void* h, long long rows, int H, void* str
   using namespace kf;
   if (H % 8) return 1;
   kf_swiglu_fwd<<<grid_for(rows * (H / 8), 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)gu, (__nv_bfloat16*)h, rows, H, nullptr);
+      (const __nv_bfloat16*)gu, (__nv_bfloat16*)h, rows, H);
   KF_LAUNCH_CHECK();
-}
-
-// The SwiGLU passes followed by scale[0] = fp8_max / (largest magnitude of what they stored), as kf_fp8_scale_bf16 gives it.
-// partial: 2368 floats (one per block).
-int kf_fp8_scale_from_partial(const void* partial, int blocks, int e5m2, void* scale, void* stream);
-
-int kf_swiglu_fwd_scale_bf16(const void* gu, void* h, long long rows, int H, int e5m2, void* partial, void* scale, void* stream) {
-  using namespace kf;
-  if (H % 8) return 1;
-  const int grid = grid_for(rows * (H / 8), 256);
-  kf_swiglu_fwd<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)h, rows, H, (float*)partial);
-  return kf_fp8_scale_from_partial(partial, grid, e5m2, scale, stream);
-}
-
-int kf_swiglu_bwd_scale_bf16(const void* dh, const void* gu, void* dgu, long long rows, int H, int e5m2, void* partial, void* scale,
-                             void* stream) {
-  using namespace kf;
-  if (H % 8) return 1;
-  const int grid = grid_for(rows * (H / 8), 256);
-  kf_swiglu_bwd<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)dh, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu,
-                                                        rows, H, nullptr, (float*)partial);
-  return kf_fp8_scale_from_partial(partial, grid, e5m2, scale, stream);
 }
 
 int kf_swiglu_bwd_bf16(const void* dh, const void* gu, void* dgu, long long rows, int H, void* stream) {
   using namespace kf;
   if (H % 8) return 1;
   kf_swiglu_bwd<<<grid_for(rows * (H / 8), 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)dh, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, rows, H, nullptr, nullptr);
+      (const __nv_bfloat16*)dh, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, rows, H, nullptr);
   KF_LAUNCH_CHECK();
 }
 
@@ -876,7 +832,7 @@ int kf_swiglu_bwd_ragged_bf16(const void* dh, const void* gu, void* dgu, long lo
   using namespace kf;
   if (H % 8) return 1;
   kf_swiglu_bwd<<<grid_for(rows_bound * (H / 8), 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)dh, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, rows_bound, H, (const int*)rows_ptr, nullptr);
+      (const __nv_bfloat16*)dh, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, rows_bound, H, (const int*)rows_ptr);
   KF_LAUNCH_CHECK();
 }
 

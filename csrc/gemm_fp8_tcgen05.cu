@@ -38,11 +38,25 @@ constexpr int STAGES = 6;
 constexpr int A_BYTES = CTA_M * BK;            // 16 KB
 constexpr int B_BYTES = (MAX_N / 2) * BK;      // 16 KB
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int THREADS = 192;
 constexpr int TMEM_COLS = 512;
 constexpr int GROUP_M = 8;
 constexpr int BOX_BYTES = 2048;  // one staged 32 x 32 box per epilogue warp
-constexpr size_t SMEM = size_t(STAGES) * STAGE_BYTES + 4 * BOX_BYTES + 1024 + 256;
+
+// What the epilogue makes of the product.  SWIGLU: B is [gate ; up] with N rows each; the leader's half of a tile is gate rows and the
+// peer's the matching up rows, C[M, N] = silu(gate) * up, and G[M, 2N] (optional) receives the pre-activations.  SWIGLU_BWD: the product
+// is the gradient of the hidden activation (never stored), G[M, 2N] holds the saved pre-activations and C[M, 2N] receives their
+// gradients.  Both round where the separate passes store bf16, in the same order of operations, and leave the largest magnitude that
+// each warp stored in amax[block * 8 + warp], which the cast to fp8 that follows waits for.
+//
+// In place of the product, a pass over 2N + N columns and a maximum, us (gate | up and the gradient, the latter's product from 4096):
+// 2000 x 14 336 from 4096 201 -> 180 and 132 -> 113, 256 rows 45 -> 40 and 33 -> 29, 2448 x 8192 from 2048 91 -> 75 and 72 -> 61,
+// 4096 x 3584 from 1024 52 -> 43 and 49 -> 46.  Where K is short the epilogue is what is waited for (five boxes of shared-memory traffic
+// per chunk next to the operands'): eight warps (four: 3584 units from 1024 45 and 50) that each take every other chunk, and rows of G
+// loaded 32 bytes per lane straight to their owners (through the boxes 52).
+enum Kind { PLAIN = 0, SWIGLU = 1, SWIGLU_BWD = 2 };
+template <int KIND> constexpr int EPI_WARPS = KIND == PLAIN ? 4 : 8;  // one or two for each quarter of the tensor memory
+template <int KIND> constexpr int THREADS = 64 + 32 * EPI_WARPS<KIND>;
+template <int KIND> constexpr size_t SMEM = size_t(STAGES) * STAGE_BYTES + EPI_WARPS<KIND> * BOX_BYTES + 1024 + 256;
 
 // Instruction descriptor for kind::f8f6f4: fp32 accumulate, A/B format 0 = e4m3, 1 = e5m2, both K-major.
 __host__ __device__ constexpr uint32_t idesc_f8(int m, int n, int a_fmt, int b_fmt) {
@@ -50,14 +64,83 @@ __host__ __device__ constexpr uint32_t idesc_f8(int m, int n, int a_fmt, int b_f
          (uint32_t(m >> 4) << 24);
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+// of the eight bf16 values of a 16-byte word
+__device__ __forceinline__ float absmax8(const uint4 v) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  float m = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 f = unpack_bf16(w[j]);
+    m = fmaxf(m, fmaxf(fabsf(f.x), fabsf(f.y)));
+  }
+  return m;
+}
+// of the first `valid` (a multiple of eight) values of a row
+__device__ __forceinline__ float absmax_row(const Rows32& r, int valid, float m) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (q * 8 < valid) m = fmaxf(m, absmax8(r.q[q]));
+  return m;
+}
+// the lane's own row of a box of 32 x 32 (rows, cols: how many exist, cols a multiple of 16; the rest is zero); src and ld on 32 bytes
+__device__ __forceinline__ Rows32 load_own_row(const __nv_bfloat16* src, size_t ld, int lane, int rows, int cols) {
+  Rows32 r;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint4 &a = r.q[2 * h], &b = r.q[2 * h + 1];
+    a = b = make_uint4(0, 0, 0, 0);
+    if (lane < rows && h * 16 < cols)
+      asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                   : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                   : "l"(src + lane * ld + h * 16));
+  }
+  return r;
+}
+// bf16 row of silu(gate) * up, operation for operation what kf_swiglu_fwd computes
+__device__ __forceinline__ Rows32 swiglu_row(const Rows32& gate, const Rows32& up) {
+  Rows32 h;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint32_t gw[4] = {gate.q[q].x, gate.q[q].y, gate.q[q].z, gate.q[q].w}, uw[4] = {up.q[q].x, up.q[q].y, up.q[q].z, up.q[q].w};
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 g = unpack_bf16(gw[e]), u = unpack_bf16(uw[e]);
+      o[e] = pack_bf16(g.x / (1.f + __expf(-g.x)) * u.x, g.y / (1.f + __expf(-g.y)) * u.y);
+    }
+    h.q[q] = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+  return h;
+}
+// gate and up are replaced by their gradients, operation for operation what kf_swiglu_bwd computes
+__device__ __forceinline__ void swiglu_grad_row(const Rows32& dh, Rows32& gate, Rows32& up) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint32_t dw[4] = {dh.q[q].x, dh.q[q].y, dh.q[q].z, dh.q[q].w};
+    uint32_t gw[4] = {gate.q[q].x, gate.q[q].y, gate.q[q].z, gate.q[q].w}, uw[4] = {up.q[q].x, up.q[q].y, up.q[q].z, up.q[q].w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 a = unpack_bf16(gw[e]), b = unpack_bf16(uw[e]), d = unpack_bf16(dw[e]);
+      const float s0 = 1.f / (1.f + __expf(-a.x)), s1 = 1.f / (1.f + __expf(-a.y));
+      const float silu0 = a.x * s0, silu1 = a.y * s1;
+      uw[e] = pack_bf16(d.x * silu0, d.y * silu1);
+      gw[e] = pack_bf16(d.x * b.x * s0 * (1.f + a.x * (1.f - s0)), d.y * b.y * s1 * (1.f + a.y * (1.f - s1)));
+    }
+    gate.q[q] = make_uint4(gw[0], gw[1], gw[2], gw[3]);
+    up.q[q] = make_uint4(uw[0], uw[1], uw[2], uw[3]);
+  }
+}
+
+template <int KIND>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS<KIND>, 1)
 kf_gemm_fp8_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          __nv_bfloat16* __restrict__ C, int M, int N, int K, int ldc, int accumulate, int a_fmt, int b_fmt,
-                         int tile_n, const float* __restrict__ scale_a, const float* __restrict__ scale_b, int* status) {
+                         int tile_n, const float* __restrict__ scale_a, const float* __restrict__ scale_b,
+                         __nv_bfloat16* __restrict__ G, int ldg, float* __restrict__ amax, int* status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t box_smem = smem_base + STAGES * STAGE_BYTES;
-  const uint32_t bar_base = box_smem + 4 * BOX_BYTES;
+  const uint32_t bar_base = box_smem + EPI_WARPS<KIND> * BOX_BYTES;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
   auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + a); };
@@ -74,7 +157,8 @@ kf_gemm_fp8_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const int half_n = tile_n >> 1;
   const int m_blocks = (M + TILE_M - 1) / TILE_M;
-  const int n_blocks = (N + tile_n - 1) / tile_n;
+  const int cols = KIND == SWIGLU ? half_n : tile_n;  // columns of 0 .. N that a tile covers
+  const int n_blocks = (N + cols - 1) / cols;
   const int num_tiles = m_blocks * n_blocks;
   const int k_blocks = (K + BK - 1) / BK;
 
@@ -85,7 +169,7 @@ kf_gemm_fp8_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);
-      mbar_init(tempty_bar(a), 8);  // four epilogue warps of each CTA
+      mbar_init(tempty_bar(a), 2 * EPI_WARPS<KIND>);  // the epilogue warps of both CTAs
     }
     mbar_init(drain_bar, 1);
     mbar_fence_init();
@@ -110,7 +194,7 @@ kf_gemm_fp8_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
         int tm, tn;
         tilemath::raster(t, m_blocks, n_blocks, GROUP_M, tm, tn);
-        const int m0 = tm * TILE_M + int(rank) * CTA_M, n0 = tn * tile_n + int(rank) * half_n;
+        const int m0 = tm * TILE_M + int(rank) * CTA_M, n0 = tn * cols + int(rank) * (KIND == SWIGLU ? N : half_n);
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
@@ -163,10 +247,12 @@ kf_gemm_fp8_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid
       mbar_wait(drain_bar, 0, status, KF_ERR_WAIT_DRAIN);
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5 of both CTAs)
-    const int quarter = warp & 3;
-    const uint32_t box = box_smem + uint32_t(quarter) * BOX_BYTES;
+    // ------------------------------------------------------------ epilogue (warps 2.. of both CTAs)
+    const int quarter = warp & 3, first = (warp - 2) >> 2;
+    constexpr int STEP = EPI_WARPS<KIND> / 4;
+    const uint32_t box = box_smem + uint32_t(warp - 2) * BOX_BYTES;
     const float alpha = 1.0f / (scale_a[0] * scale_b[0]);
+    float largest = 0.f;
     int tile_iter = 0;
     bool ok = true;
     for (int t = pair; t < num_tiles && ok; t += num_pairs, ++tile_iter) {
@@ -178,18 +264,45 @@ kf_gemm_fp8_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid
       tc_fence_after();
       const int row0 = tm * TILE_M + int(rank) * CTA_M + quarter * 32;  // this warp's rows, and how many exist
       const int rows = max(0, min(32, M - row0));
-      const int col0 = tn * tile_n, width = min(tile_n, N - col0);
+      const int col0 = tn * cols, width = min(cols, N - col0);
       const uint32_t t_row = tmem_base + (uint32_t(quarter * 32) << 16) + acc * MAX_N;
       __nv_bfloat16* c0 = C + size_t(row0) * ldc + col0;
+      __nv_bfloat16* g0 = KIND == PLAIN || G == nullptr ? nullptr : G + size_t(row0) * ldg + col0;
+      Rows32 g_next, u_next;  // saved pre-activations of the chunk that follows: under way while this one is worked on
+      if (KIND == SWIGLU_BWD) {
+        g_next = load_own_row(g0 + first * 32, ldg, lane, rows, width - first * 32);
+        u_next = load_own_row(g0 + N + first * 32, ldg, lane, rows, width - first * 32);
+      }
 #pragma unroll 1
-      for (int c = 0; c * 32 < width; ++c) {
-        uint32_t v[32];
+      for (int c = first; c * 32 < width; c += STEP) {
+        uint32_t v[32], w[32];
         tmem_ld_32x32(t_row + c * 32, v);
+        if (KIND == SWIGLU) tmem_ld_32x32(t_row + half_n + c * 32, w);
         tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
         const int valid = min(32, width - c * 32);
-        if (!accumulate)
+        if (KIND == SWIGLU) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) w[i] = __float_as_uint(__uint_as_float(w[i]) * alpha);
+          const Rows32 gate = pack_row32(v), up = pack_row32(w), h = swiglu_row(gate, up);
+          largest = absmax_row(h, valid, largest);
+          if (g0 != nullptr) {
+            store_rows32(box, lane, gate, g0 + c * 32, ldg, rows, valid);
+            store_rows32(box, lane, up, g0 + N + c * 32, ldg, rows, valid);
+          }
+          store_rows32(box, lane, h, c0 + c * 32, ldc, rows, valid);
+        } else if (KIND == SWIGLU_BWD) {
+          Rows32 gate = g_next, up = u_next;
+          if (const int n = (c + STEP) * 32; n < width) {
+            g_next = load_own_row(g0 + n, ldg, lane, rows, width - n);
+            u_next = load_own_row(g0 + N + n, ldg, lane, rows, width - n);
+          }
+          swiglu_grad_row(pack_row32(v), gate, up);
+          largest = absmax_row(up, valid, absmax_row(gate, valid, largest));
+          store_rows32(box, lane, gate, c0 + c * 32, ldc, rows, valid);
+          store_rows32(box, lane, up, c0 + N + c * 32, ldc, rows, valid);
+        } else if (!accumulate)
           store_rows32(box, lane, pack_row32(v), c0 + c * 32, ldc, rows, valid);
         else if (lane < rows)
           store_chunk<__nv_bfloat16>(c0 + size_t(lane) * ldc + c * 32, v, valid, true, nullptr);
@@ -197,6 +310,11 @@ kf_gemm_fp8_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid
       tc_fence_before();
       __syncwarp();
       if (lane == 0) arrive_on_cta(tempty_bar(acc), 0);
+    }
+    if (KIND != PLAIN) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, o));
+      if (lane == 0) amax[blockIdx.x * EPI_WARPS<KIND> + warp - 2] = largest;
     }
   }
 
@@ -229,17 +347,6 @@ constexpr float E4M3_MAX = 448.f;
 constexpr float E5M2_MAX = 57344.f;
 
 constexpr int AMAX_BLOCKS = 1024;  // partial maxima (and the size of their buffer)
-
-__device__ __forceinline__ float absmax8(const uint4 v) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-  float m = 0.f;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 f = unpack_bf16(w[j]);
-    m = fmaxf(m, fmaxf(fabsf(f.x), fabsf(f.y)));
-  }
-  return m;
-}
 
 // partial[block] = max |x| over the block's share; four independent 16-byte loads in flight per thread
 __global__ void __launch_bounds__(256) kf_absmax_bf16(const __nv_bfloat16* __restrict__ x, long long n, float* __restrict__ partial) {
@@ -283,6 +390,12 @@ __global__ void __launch_bounds__(256) kf_scale_from_amax(const float* __restric
     for (int w = 1; w < 8; ++w) m = fmaxf(m, red[w]);
     scale[0] = fp8_max / fmaxf(m, 1e-12f);
   }
+}
+
+static int launch_scale(const void* partial, int n, float fp8_max, void* scale, void* stream) {
+  kf_scale_from_amax<<<1, 256, 0, (cudaStream_t)stream>>>(reinterpret_cast<const float*>(partial), n, reinterpret_cast<float*>(scale), fp8_max);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
 template <bool E5M2>
@@ -382,6 +495,39 @@ kf_cast_fp8(const __nv_bfloat16* __restrict__ x, int rows, int cols, long long l
   }
 }
 
+// One product; rows of B: N, or 2N for SWIGLU.  With a SwiGLU: N a multiple of 16, G and its rows on 32 bytes.
+template <int KIND>
+static int launch(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, int ldc, int a_fmt, int b_fmt,
+                  const void* scale_a, const void* scale_b, int accumulate, void* G, int ldg, void* amax, int* blocks, int num_sms,
+                  void* stream, int* status) {
+  if ((lda & 15) || (ldb & 15) || (ldc & 7) || (ldg & 7) || M <= 0 || N <= 0 || K <= 0) return 5;
+  if (num_sms < 2 || (KIND != PLAIN && ((N & 15) || (ldg & 15) || (reinterpret_cast<uintptr_t>(G) & 31)))) return 5;
+  const int b_rows = KIND == SWIGLU ? 2 * N : N;
+  int pairs = num_sms / 2;
+  const int tile_n = pair_tile_width(M, b_rows, pairs, nullptr);
+  const int cols = KIND == SWIGLU ? tile_n / 2 : tile_n;
+  CUtensorMap ma, mb;
+  int rc = make_map_2d_u8(&ma, A, M, K, lda, CTA_M);
+  if (rc) return 100 + rc;
+  rc = make_map_2d_u8(&mb, B, b_rows, K, ldb, tile_n / 2);
+  if (rc) return 200 + rc;
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(kf_gemm_fp8_tcgen05_2cta<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM<KIND>);
+    if (e != cudaSuccess) return 300 + (int)e;
+    attr_set = true;
+  }
+  const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + cols - 1) / cols);
+  if (tiles < pairs) pairs = tiles;
+  if (blocks != nullptr) *blocks = pairs * 2;
+  kf_gemm_fp8_tcgen05_2cta<KIND><<<pairs * 2, THREADS<KIND>, SMEM<KIND>, (cudaStream_t)stream>>>(
+      ma, mb, reinterpret_cast<__nv_bfloat16*>(C), M, N, K, ldc, accumulate, a_fmt, b_fmt, tile_n,
+      reinterpret_cast<const float*>(scale_a), reinterpret_cast<const float*>(scale_b), reinterpret_cast<__nv_bfloat16*>(G), ldg,
+      reinterpret_cast<float*>(amax), status);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 400 + (int)e;
+}
+
 }  // namespace f8
 }  // namespace kf
 
@@ -394,40 +540,31 @@ extern "C" {
 int kf_gemm_fp8(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, int ldc,
                 int a_fmt, int b_fmt, const void* scale_a, const void* scale_b, int accumulate, int num_sms,
                 void* stream) {
-  using namespace kf;
   using namespace kf::f8;
-  if ((lda & 15) || (ldb & 15) || (ldc & 7) || M <= 0 || N <= 0 || K <= 0) return 5;
-  if (num_sms < 2) return 5;
-  int pairs = num_sms / 2;
-  const int tile_n = pair_tile_width(M, N, pairs, nullptr);
-  CUtensorMap ma, mb;
-  int rc = make_map_2d_u8(&ma, A, M, K, lda, CTA_M);
-  if (rc) return 100 + rc;
-  rc = make_map_2d_u8(&mb, B, N, K, ldb, tile_n / 2);
-  if (rc) return 200 + rc;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kf_gemm_fp8_tcgen05_2cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
-    if (e != cudaSuccess) return 300 + (int)e;
-    attr_set = true;
-  }
-  const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + tile_n - 1) / tile_n);
-  if (tiles < pairs) pairs = tiles;
-  kf_gemm_fp8_tcgen05_2cta<<<pairs * 2, THREADS, SMEM, (cudaStream_t)stream>>>(
-      ma, mb, reinterpret_cast<__nv_bfloat16*>(C), M, N, K, ldc, accumulate, a_fmt, b_fmt, tile_n,
-      reinterpret_cast<const float*>(scale_a), reinterpret_cast<const float*>(scale_b),
-      reinterpret_cast<int*>(kf_status_device_ptr()));
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : 400 + (int)e;
+  return launch<PLAIN>(A, B, C, M, N, K, lda, ldb, ldc, a_fmt, b_fmt, scale_a, scale_b, accumulate, nullptr, 0, nullptr, nullptr, num_sms,
+                       stream, reinterpret_cast<int*>(kf_status_device_ptr()));
 }
 
-// scale[0] = fp8_max / max(partial[0 .. blocks)).
-int kf_fp8_scale_from_partial(const void* partial, int blocks, int e5m2, void* scale, void* stream) {
+// H[M,F] = silu(gate) * up of [gate | up] = A8 * B8^T / (scale_a * scale_b), B8 = [gate ; up] (2F rows), and scale[0] = fp8_max / absmax(H)
+// for a cast to e4m3.  GU[M,2F] (optional) receives the pre-activations.  partial: eight floats per SM.
+int kf_gemm_fp8_swiglu(const void* A, const void* B, void* H, void* GU, int M, int F, int K, long long lda, long long ldb, int ldh, int ldgu,
+                       const void* scale_a, const void* scale_b, void* partial, void* scale, int num_sms, void* stream) {
   using namespace kf::f8;
-  kf_scale_from_amax<<<1, 256, 0, (cudaStream_t)stream>>>(reinterpret_cast<const float*>(partial), blocks, reinterpret_cast<float*>(scale),
-                                                          e5m2 ? E5M2_MAX : E4M3_MAX);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : 400 + (int)e;
+  int blocks = 0;
+  const int rc = launch<SWIGLU>(A, B, H, M, F, K, lda, ldb, ldh, 0, 0, scale_a, scale_b, 0, GU, ldgu, partial, &blocks, num_sms, stream,
+                                reinterpret_cast<int*>(kf_status_device_ptr()));
+  return rc ? rc : launch_scale(partial, blocks * EPI_WARPS<SWIGLU>, E4M3_MAX, scale, stream);
+}
+
+// DGU[M,2F] = SwiGLU'(GU) * (A8 * B8^T / (scale_a * scale_b)), A8 e5m2 (the incoming gradient), B8 e4m3 with F rows, and
+// scale[0] = fp8_max / absmax(DGU) for a cast to e5m2.  partial: eight floats per SM.
+int kf_gemm_fp8_swiglu_bwd(const void* A, const void* B, const void* GU, void* DGU, int M, int F, int K, long long lda, long long ldb, int ldgu,
+                           const void* scale_a, const void* scale_b, void* partial, void* scale, int num_sms, void* stream) {
+  using namespace kf::f8;
+  int blocks = 0;
+  const int rc = launch<SWIGLU_BWD>(A, B, DGU, M, F, K, lda, ldb, ldgu, 1, 0, scale_a, scale_b, 0, const_cast<void*>(GU), ldgu, partial, &blocks,
+                                    num_sms, stream, reinterpret_cast<int*>(kf_status_device_ptr()));
+  return rc ? rc : launch_scale(partial, blocks * EPI_WARPS<SWIGLU_BWD>, E5M2_MAX, scale, stream);
 }
 
 // scale[0] = fp8_max / absmax(x) for n bf16 values; amax_scratch holds AMAX_BLOCKS (1024) floats.
@@ -439,10 +576,7 @@ int kf_fp8_scale_bf16(const void* x, long long n, int e5m2, void* amax_scratch, 
   if (blocks > AMAX_BLOCKS) blocks = AMAX_BLOCKS;
   kf_absmax_bf16<<<(int)blocks, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(x), n,
                                               reinterpret_cast<float*>(amax_scratch));
-  kf_scale_from_amax<<<1, 256, 0, st>>>(reinterpret_cast<const float*>(amax_scratch), (int)blocks,
-                                        reinterpret_cast<float*>(scale), e5m2 ? E5M2_MAX : E4M3_MAX);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : 400 + (int)e;
+  return launch_scale(amax_scratch, (int)blocks, e5m2 ? E5M2_MAX : E4M3_MAX, scale, stream);
 }
 
 // fp8(x * scale) row-major into out (optional) and transposed into out_t (optional).

@@ -89,9 +89,8 @@ def _declare(L: ctypes.CDLL) -> None:
         "kf_test_flag_timeout": [vp, i, ll],
         "kf_gemm_fp8": [vp, vp, vp, i, i, i, ll, ll, i, i, i, vp, vp, i, i, vp],
         "kf_fp8_scale_bf16": [vp, ll, i, vp, vp, vp],
-        "kf_fp8_scale_from_partial": [vp, i, i, vp, vp],
-        "kf_swiglu_fwd_scale_bf16": [vp, vp, ll, i, i, vp, vp, vp],
-        "kf_swiglu_bwd_scale_bf16": [vp, vp, vp, ll, i, i, vp, vp, vp],
+        "kf_gemm_fp8_swiglu": [vp, vp, vp, vp, i, i, i, ll, ll, i, i, vp, vp, vp, vp, i, vp],
+        "kf_gemm_fp8_swiglu_bwd": [vp, vp, vp, vp, i, i, i, ll, ll, i, vp, vp, vp, vp, i, vp],
         "kf_fp8_cast_bf16": [vp, i, i, ll, vp, i, vp, ll, vp, ll, vp],
         "kf_lion": [vp, vp, vp, ll, i, f, f, f, f, vp],
         "kf_sf_adamw": [vp, vp, vp, vp, vp, ll, i, f, f, f, f, f, f, f, i, vp],
@@ -566,26 +565,6 @@ def swiglu_bwd(dh: torch.Tensor, gu: torch.Tensor, out=None) -> torch.Tensor:
     return dgu
 
 
-def swiglu_fwd_scale(gu: torch.Tensor, e5m2: bool = False):
-    """(:func:`swiglu_fwd` of gu (rows, 2H), what :func:`fp8_scale` gives for it): the maximum is taken while the values pass."""
-    rows, h = gu.shape[0], gu.shape[1] // 2
-    out = torch.empty((rows, h), dtype=gu.dtype, device=gu.device)
-    scratch = torch.empty(1 + 148 * 16, dtype=torch.float32, device=gu.device)   # the scale, then partial maxima
-    _check(lib().kf_swiglu_fwd_scale_bf16(gu.data_ptr(), out.data_ptr(), rows, h, int(e5m2), scratch.data_ptr() + 4, scratch.data_ptr(),
-                                          _stream()), "kf_swiglu_fwd_scale_bf16", 2)
-    return out, scratch[:1]
-
-
-def swiglu_bwd_scale(dh: torch.Tensor, gu: torch.Tensor, e5m2: bool = True):
-    """(:func:`swiglu_bwd` in a tensor of its own, its fp8 scale)."""
-    rows, h = gu.shape[0], gu.shape[1] // 2
-    dgu = torch.empty_like(gu)
-    scratch = torch.empty(1 + 148 * 16, dtype=torch.float32, device=gu.device)
-    _check(lib().kf_swiglu_bwd_scale_bf16(dh.data_ptr(), gu.data_ptr(), dgu.data_ptr(), rows, h, int(e5m2), scratch.data_ptr() + 4,
-                                          scratch.data_ptr(), _stream()), "kf_swiglu_bwd_scale_bf16", 2)
-    return dgu, scratch[:1]
-
-
 def embedding_fwd(ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
     ids = ids.contiguous()
     if ids.dtype != torch.int64:
@@ -778,6 +757,37 @@ def gemm_fp8(a8: torch.Tensor, b8: torch.Tensor, sa: torch.Tensor, sb: torch.Ten
                              out.stride(0), int(a_e5m2), int(b_e5m2), sa.data_ptr(), sb.data_ptr(), int(accumulate),
                              sm_count(), _stream()), "kf_gemm_fp8")
     return out
+
+
+def gemm_fp8_swiglu(a8: torch.Tensor, b8: torch.Tensor, sa: torch.Tensor, sb: torch.Tensor):
+    """(gu, h, s): :func:`gemm_fp8` of e4m3 operands, b8 = [gate ; up] (2F rows), :func:`swiglu_fwd` of it and :func:`fp8_scale` of that, from one
+    kernel and the small one that turns its maxima into a scale."""
+    m, k = a8.shape
+    f = b8.shape[0] // 2
+    assert b8.shape == (2 * f, k) and a8.stride(1) == 1 and b8.stride(1) == 1
+    gu = torch.empty((m, 2 * f), dtype=torch.bfloat16, device=a8.device)
+    h = torch.empty((m, f), dtype=torch.bfloat16, device=a8.device)
+    scratch = torch.empty(1 + 8 * sm_count(), dtype=torch.float32, device=a8.device)   # the scale, then partial maxima
+    _check(lib().kf_gemm_fp8_swiglu(a8.data_ptr(), b8.data_ptr(), h.data_ptr(), gu.data_ptr(), m, f, k, a8.stride(0), b8.stride(0), f, 2 * f,
+                                    sa.data_ptr(), sb.data_ptr(), scratch.data_ptr() + 4, scratch.data_ptr(), sm_count(), _stream()),
+           "kf_gemm_fp8_swiglu", 2)
+    return gu, h, scratch[:1]
+
+
+def gemm_fp8_swiglu_bwd(a8: torch.Tensor, b8: torch.Tensor, sa: torch.Tensor, sb: torch.Tensor, gu: torch.Tensor):
+    """(dgu, s): :func:`swiglu_bwd` of :func:`gemm_fp8` of an e5m2 gradient and e4m3 weights (F rows) in a tensor of its own, and its e5m2
+    :func:`fp8_scale`; the gradient of the hidden activation stays on the chip."""
+    m, k = a8.shape
+    f = b8.shape[0]
+    assert b8.shape[1] == k and a8.stride(1) == 1 and b8.stride(1) == 1 and gu.shape == (m, 2 * f)
+    if not gu.is_contiguous() or gu.data_ptr() % 32:
+        gu = gu.clone(memory_format=torch.contiguous_format)
+    dgu = torch.empty_like(gu)
+    scratch = torch.empty(1 + 8 * sm_count(), dtype=torch.float32, device=a8.device)   # the scale, then partial maxima
+    _check(lib().kf_gemm_fp8_swiglu_bwd(a8.data_ptr(), b8.data_ptr(), gu.data_ptr(), dgu.data_ptr(), m, f, k, a8.stride(0), b8.stride(0), 2 * f,
+                                        sa.data_ptr(), sb.data_ptr(), scratch.data_ptr() + 4, scratch.data_ptr(), sm_count(), _stream()),
+           "kf_gemm_fp8_swiglu_bwd", 2)
+    return dgu, scratch[:1]
 
 
 # --------------------------------------------------------------------------- attention

@@ -150,8 +150,8 @@ class _Fp8LinearFn(torch.autograd.Function):
 
 class _Fp8SwiGLUFn(torch.autograd.Function):
     """down(silu(x Wgᵀ) * (x Wuᵀ)) with fp8 products as one node: the arithmetic of two :class:`_Fp8LinearFn` around the SwiGLU
-    kernel, except that the maxima of the hidden activation and of d[gate | up], which their casts wait for, come from the
-    kernels that write them."""
+    kernel, except that the SwiGLU and its gradient, and the maxima that the casts of their results wait for, are taken in the
+    epilogues of the products before them."""
 
     @staticmethod
     def forward(ctx, x, wg, wu, wd):
@@ -162,8 +162,7 @@ class _Fp8SwiGLUFn(torch.autograd.Function):
             x2 = x2.contiguous()
         sx, x8, _ = quantize(x2)
         s_gu, w8, _ = quantized_weight((wg, wu), want_t=False)
-        gu = scaled_mm(x8, w8, sx, s_gu)
-        h, sh = cu.swiglu_fwd_scale(gu)
+        gu, h, sh = cu.gemm_fp8_swiglu(x8, w8, sx, s_gu)
         _, h8, _ = quantize(h, scale=sh)
         sd, d8, _ = quantized_weight((wd,), want_t=False)
         y = scaled_mm(h8, d8, sh, sd)
@@ -186,7 +185,7 @@ class _Fp8SwiGLUFn(torch.autograd.Function):
         dx = g_wg = g_wu = g_wd = None
         if need_h:
             _, _, d8t = quantized_weight((wd,), want_t=True)
-            dgu, s_dgu = cu.swiglu_bwd_scale(scaled_mm(g8, d8t, sg, sd, a_e5m2=True), gu)
+            dgu, s_dgu = cu.gemm_fp8_swiglu_bwd(g8, d8t, sg, sd, gu)
         if need_d:
             _, _, h8t = quantize(h, want_row=False, want_t=True, scale=sh)
             (g_wd,) = F._deposit_stacked_weight_grads(

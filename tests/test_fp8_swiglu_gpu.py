@@ -66,3 +66,38 @@ def test_second_backward_and_other_layers(native_lib):
     w = [mlp.gate_proj.weight, mlp.up_proj.weight, mlp.down_proj.weight]
     assert fp8.swiglu_mlp(x[:, :5], *w) is None and fp8.swiglu_mlp(x.float(), *w) is None   # 15 rows; fp32
     assert fp8.swiglu_mlp(x, w[0], w[1], w[2].detach().clone()) is None                     # a weight that is not tagged
+
+
+# Rows and hidden units at the edges of tiles: 16 is the fewest, 256 x 1024 one round of the narrowest tiles, and 2048 rows with 14 336,
+# 12 288 and 10 752 units take tiles of different widths (a half of 112 or 80 columns ends inside a chunk of 32).
+@pytest.mark.parametrize("t,k,f", [(16, 16, 16), (272, 144, 1024), (256, 64, 1040), (2000, 128, 14336), (2048, 256, 10752), (2544, 96, 4752), (4096, 64, 3600)])
+def test_products_with_swiglu_epilogues(native_lib, t, k, f):
+    """Bit for bit the product, the SwiGLU pass over what it stores and the scale of the result."""
+    cu = native_lib
+    torch.manual_seed(1)
+    q = lambda rows, e5m2=False: cu.fp8_cast(torch.randn(rows, k, device=DEV).bfloat16(), torch.full((1,), 30.0, device=DEV), e5m2)[0]
+    sa, sb = torch.full((1,), 30.0, device=DEV), torch.full((1,), 7.0, device=DEV)
+    x8, w8 = q(t), q(2 * f)
+    gu = cu.gemm_fp8(x8, w8, sa, sb)
+    h = cu.swiglu_fwd(gu)
+    got = cu.gemm_fp8_swiglu(x8, w8, sa, sb)
+    assert _equal(got, (gu, h, cu.fp8_scale(h)))
+    g8, d8 = q(t, True), q(f)
+    dgu = cu.swiglu_bwd(cu.gemm_fp8(g8, d8, sa, sb, a_e5m2=True), gu)
+    assert _equal(cu.gemm_fp8_swiglu_bwd(g8, d8, sa, sb, gu), (dgu, cu.fp8_scale(dgu, True)))
+    assert native_lib.read_status() == 0
+
+
+def test_saved_pre_activations_may_come_back_elsewhere(native_lib):
+    """Hooks on saved tensors return copies with other strides and on other addresses."""
+    mlp = _mlp(64, 272)
+    x, dy = (torch.randn(48, 64, device=DEV).bfloat16() for _ in range(2))
+    ref = _run(mlp, x, dy)
+
+    def moved(t):
+        if t.dim() != 2 or t.shape[0] != 48 or t.dtype != torch.bfloat16:
+            return t
+        return torch.empty(t.shape[0] * (t.shape[1] + 8) + 8, dtype=t.dtype, device=t.device)[8:].view(t.shape[0], -1)[:, : t.shape[1]].copy_(t)
+
+    with torch.autograd.graph.saved_tensors_hooks(moved, lambda t: t):
+        assert _equal(ref, _run(mlp, x, dy))
