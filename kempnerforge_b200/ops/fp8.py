@@ -151,10 +151,11 @@ class _Fp8LinearFn(torch.autograd.Function):
 class _Fp8SwiGLUFn(torch.autograd.Function):
     """down(silu(x Wgᵀ) * (x Wuᵀ)) with fp8 products as one node: the arithmetic of two :class:`_Fp8LinearFn` around the SwiGLU
     kernel, except that the SwiGLU and its gradient, and the maxima that the casts of their results wait for, are taken in the
-    epilogues of the products before them."""
+    epilogues of the products before them.  The hidden activation is cast once: where a gradient of ``wd`` will be wanted
+    (``recording``) its transposed fp8 copy is written together with the other one and kept in its stead, at half its bytes."""
 
     @staticmethod
-    def forward(ctx, x, wg, wu, wd):
+    def forward(ctx, x, wg, wu, wd, recording):
         from kempnerforge_b200.ops import cuda as cu
 
         x2 = x.reshape(-1, x.shape[-1])
@@ -163,10 +164,10 @@ class _Fp8SwiGLUFn(torch.autograd.Function):
         sx, x8, _ = quantize(x2)
         s_gu, w8, _ = quantized_weight((wg, wu), want_t=False)
         gu, h, sh = cu.gemm_fp8_swiglu(x8, w8, sx, s_gu)
-        _, h8, _ = quantize(h, scale=sh)
+        _, h8, h8t = quantize(h, scale=sh, want_t=recording and ctx.needs_input_grad[3])
         sd, d8, _ = quantized_weight((wd,), want_t=False)
         y = scaled_mm(h8, d8, sh, sd)
-        ctx.save_for_backward(x2, sx, s_gu, gu, h, sh, sd, wg, wu, wd)
+        ctx.save_for_backward(x2, sx, s_gu, gu, h8t, sh, sd, wg, wu, wd)
         ctx.x_shape = x.shape
         return y.view(*x.shape[:-1], d8.shape[0])
 
@@ -175,11 +176,11 @@ class _Fp8SwiGLUFn(torch.autograd.Function):
         from kempnerforge_b200.ops import cuda as cu
         from kempnerforge_b200.ops import functional as F
 
-        x2, sx, s_gu, gu, h, sh, sd, wg, wu, wd = ctx.saved_tensors
+        x2, sx, s_gu, gu, h8t, sh, sd, wg, wu, wd = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
-        need_x, need_g, need_u, need_d = ctx.needs_input_grad
+        need_x, need_g, need_u, need_d, _ = ctx.needs_input_grad
         need_h = need_x or need_g or need_u
         sg, g8, g8t = quantize(dy2, e5m2=True, want_row=need_h, want_t=need_d)
         dx = g_wg = g_wu = g_wd = None
@@ -187,7 +188,6 @@ class _Fp8SwiGLUFn(torch.autograd.Function):
             _, _, d8t = quantized_weight((wd,), want_t=True)
             dgu, s_dgu = cu.gemm_fp8_swiglu_bwd(g8, d8t, sg, sd, gu)
         if need_d:
-            _, _, h8t = quantize(h, want_row=False, want_t=True, scale=sh)
             (g_wd,) = F._deposit_stacked_weight_grads(
                 [wd], (True,), lambda out, acc: scaled_mm(g8t, h8t, sg, sh, a_e5m2=True, out=out, accumulate=acc))
         if need_h:
@@ -201,7 +201,7 @@ class _Fp8SwiGLUFn(torch.autograd.Function):
                 g_wg, g_wu = F._deposit_stacked_weight_grads(
                     [wg, wu], (need_g, need_u),
                     lambda out, acc: scaled_mm(q8t, x8t, s_dgu, sx, a_e5m2=True, out=out, accumulate=acc))
-        return dx, g_wg, g_wu, g_wd
+        return dx, g_wg, g_wu, g_wd, None
 
 
 def swiglu_mlp(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, wd: torch.Tensor) -> torch.Tensor | None:
@@ -211,7 +211,7 @@ def swiglu_mlp(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, wd: torch.Te
     if (not F.use_native(x) or x.numel() == 0 or not supported(x, [wg, wu, wd]) or wg.shape != wu.shape
             or wd.shape[1] != wg.shape[0] or wg.shape[1] != x.shape[-1] or any(not w.is_cuda or w.dtype != torch.bfloat16 for w in (wg, wu, wd))):
         return None
-    return _Fp8SwiGLUFn.apply(x, wg, wu, wd)
+    return _Fp8SwiGLUFn.apply(x, wg, wu, wd, torch.is_grad_enabled())
 
 
 def linear(x: torch.Tensor, weights: list[torch.Tensor]) -> torch.Tensor:

@@ -101,3 +101,24 @@ def test_saved_pre_activations_may_come_back_elsewhere(native_lib):
 
     with torch.autograd.graph.saved_tensors_hooks(moved, lambda t: t):
         assert _equal(ref, _run(mlp, x, dy))
+    with torch.autograd.graph.save_on_cpu():   # the transposed fp8 copy returns without its pitch
+        assert _equal(ref, _run(mlp, x, dy))
+
+
+def test_hidden_activation_is_kept_only_as_its_transposed_copy(native_lib):
+    """h (48, 272) in bf16 is not among the saved tensors; without a recorded graph no transposed copy is written."""
+    from kempnerforge_b200.ops import fp8
+
+    mlp = _mlp(64, 272)
+    x = torch.randn(48, 64, device=DEV).bfloat16()
+    saved, wanted, quantize = [], [], fp8.quantize
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: saved.append((tuple(t.shape), t.dtype)) or t, lambda t: t):
+        y = mlp(x)
+    assert ((48, 272), torch.bfloat16) not in saved and ((272, 48), torch.uint8) in saved
+    fp8.quantize = lambda *a, **k: wanted.append(k.get("want_t", False)) or quantize(*a, **k)
+    try:
+        with torch.no_grad():
+            assert torch.equal(mlp(x), y)
+    finally:
+        fp8.quantize = quantize
+    assert wanted and not any(wanted)
