@@ -46,7 +46,7 @@ constexpr int BOX_BYTES = 2048;  // one staged 32 x 32 box per epilogue warp
 // peer's the matching up rows, C[M, N] = silu(gate) * up, and G[M, 2N] (optional) receives the pre-activations.  SWIGLU_BWD: the product
 // is the gradient of the hidden activation (never stored), G[M, 2N] holds the saved pre-activations and C[M, 2N] receives their
 // gradients.  Both round where the separate passes store bf16, in the same order of operations, and leave the largest magnitude that
-// each warp stored in amax[block * 8 + warp], which the cast to fp8 that follows waits for.
+// each warp stored in amax[block * 8 + warp], for the cast to fp8 that follows.
 //
 // In place of the product, a pass over 2N + N columns and a maximum, us (gate | up and the gradient, the latter's product from 4096):
 // 2000 x 14 336 from 4096 201 -> 180 and 132 -> 113, 256 rows 45 -> 40 and 33 -> 29, 2448 x 8192 from 2048 91 -> 75 and 72 -> 61,
@@ -376,26 +376,22 @@ __global__ void __launch_bounds__(256) kf_absmax_bf16(const __nv_bfloat16* __res
   }
 }
 
-// scale = fp8_max / max(amax, tiny)
-__global__ void __launch_bounds__(256) kf_scale_from_amax(const float* __restrict__ partial, int blocks, float* __restrict__ scale, float fp8_max) {
-  __shared__ float red[8];
+// fp8_max / max(largest of n partial maxima, tiny), in every thread of a block of 256
+__device__ __forceinline__ float scale_of(const float* __restrict__ partial, int n, float fp8_max, float* red) {
   float m = 0.f;
-  for (int i = threadIdx.x; i < blocks; i += 256) m = fmaxf(m, partial[i]);
+  for (int i = threadIdx.x; i < n; i += 256) m = fmaxf(m, partial[i]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
   __syncthreads();
-  if (threadIdx.x == 0) {
 #pragma unroll
-    for (int w = 1; w < 8; ++w) m = fmaxf(m, red[w]);
-    scale[0] = fp8_max / fmaxf(m, 1e-12f);
-  }
+  for (int w = 0; w < 8; ++w) m = fmaxf(m, red[w]);
+  return fp8_max / fmaxf(m, 1e-12f);
 }
-
-static int launch_scale(const void* partial, int n, float fp8_max, void* scale, void* stream) {
-  kf_scale_from_amax<<<1, 256, 0, (cudaStream_t)stream>>>(reinterpret_cast<const float*>(partial), n, reinterpret_cast<float*>(scale), fp8_max);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : 400 + (int)e;
+__global__ void __launch_bounds__(256) kf_scale_from_amax(const float* __restrict__ partial, int n, float* __restrict__ scale, float fp8_max) {
+  __shared__ float red[8];
+  const float s = scale_of(partial, n, fp8_max, red);
+  if (threadIdx.x == 0) scale[0] = s;
 }
 
 template <bool E5M2>
@@ -409,12 +405,16 @@ __device__ __forceinline__ uint8_t to_fp8(float v) {
 // stores, whole 128-byte lines on every side; the tile is transposed through shared memory as 4-byte words (word w of row
 // r at w ^ 4 * (r / 16 % 8): the 32 lanes of a transposed read hit 32 different banks) and byte permutes.  The casts of an fp8
 // 7B feed-forward over 2000 tokens took 145 us with 4-byte loads and byte-wise transposes, 88 us so (their maxima 60 -> 40).
+//
+// partial (optional): n partial maxima of |x|; every block makes the scale from them while its tile is under way, and the first one
+// stores it for the products.  A kernel of one block in between was a launch and a drain: feed-forwards with their backward, of 240 rows
+// x 4096 450 -> 422 us, of 2448 x 2048 449 -> 439, of 1008 x 4096 614 -> 610; over 2000 x 4096 no change (1067: the power limit).
 template <bool E5M2>
 __global__ void __launch_bounds__(256)
-kf_cast_fp8(const __nv_bfloat16* __restrict__ x, int rows, int cols, long long ldx, const float* __restrict__ scale,
-            uint8_t* __restrict__ out, long long ld_out, uint8_t* __restrict__ out_t, long long ld_t) {
+kf_cast_fp8(const __nv_bfloat16* __restrict__ x, int rows, int cols, long long ldx, const float* __restrict__ partial, int n,
+            float* __restrict__ scale, uint8_t* __restrict__ out, long long ld_out, uint8_t* __restrict__ out_t, long long ld_t) {
   __shared__ uint32_t tile[128][32];
-  const float s = scale[0];
+  __shared__ float red[8];
   const int r0 = blockIdx.y * 128, c0 = blockIdx.x * 128;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // 16 threads x 8 columns, 16 rows per step
   const int c = c0 + tx * 8;
@@ -437,6 +437,13 @@ kf_cast_fp8(const __nv_bfloat16* __restrict__ x, int rows, int cols, long long l
         v[i] = make_uint4(w[0], w[1], w[2], w[3]);
       }
     }
+  }
+  float s;
+  if (partial != nullptr) {
+    s = scale_of(partial, n, E5M2 ? E5M2_MAX : E4M3_MAX, red);
+    if ((blockIdx.x | blockIdx.y | threadIdx.x) == 0) scale[0] = s;
+  } else {
+    s = scale[0];
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -498,7 +505,7 @@ kf_cast_fp8(const __nv_bfloat16* __restrict__ x, int rows, int cols, long long l
 // One product; rows of B: N, or 2N for SWIGLU.  With a SwiGLU: N a multiple of 16, G and its rows on 32 bytes.
 template <int KIND>
 static int launch(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, int ldc, int a_fmt, int b_fmt,
-                  const void* scale_a, const void* scale_b, int accumulate, void* G, int ldg, void* amax, int* blocks, int num_sms,
+                  const void* scale_a, const void* scale_b, int accumulate, void* G, int ldg, void* amax, int* count, int num_sms,
                   void* stream, int* status) {
   if ((lda & 15) || (ldb & 15) || (ldc & 7) || (ldg & 7) || M <= 0 || N <= 0 || K <= 0) return 5;
   if (num_sms < 2 || (KIND != PLAIN && ((N & 15) || (ldg & 15) || (reinterpret_cast<uintptr_t>(G) & 31)))) return 5;
@@ -519,7 +526,7 @@ static int launch(const void* A, const void* B, void* C, int M, int N, int K, lo
   }
   const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + cols - 1) / cols);
   if (tiles < pairs) pairs = tiles;
-  if (blocks != nullptr) *blocks = pairs * 2;
+  if (count != nullptr) *count = pairs * 2 * EPI_WARPS<KIND>;
   kf_gemm_fp8_tcgen05_2cta<KIND><<<pairs * 2, THREADS<KIND>, SMEM<KIND>, (cudaStream_t)stream>>>(
       ma, mb, reinterpret_cast<__nv_bfloat16*>(C), M, N, K, ldc, accumulate, a_fmt, b_fmt, tile_n,
       reinterpret_cast<const float*>(scale_a), reinterpret_cast<const float*>(scale_b), reinterpret_cast<__nv_bfloat16*>(G), ldg,
@@ -545,52 +552,62 @@ int kf_gemm_fp8(const void* A, const void* B, void* C, int M, int N, int K, long
                        stream, reinterpret_cast<int*>(kf_status_device_ptr()));
 }
 
-// H[M,F] = silu(gate) * up of [gate | up] = A8 * B8^T / (scale_a * scale_b), B8 = [gate ; up] (2F rows), and scale[0] = fp8_max / absmax(H)
-// for a cast to e4m3.  GU[M,2F] (optional) receives the pre-activations.  partial: eight floats per SM.
+// H[M,F] = silu(gate) * up of [gate | up] = A8 * B8^T / (scale_a * scale_b), e4m3 operands, B8 = [gate ; up] (2F rows); partial[0 .. *count)
+// = partial maxima of |H|, eight per SM at most.  GU[M,2F] (optional) receives the pre-activations.
 int kf_gemm_fp8_swiglu(const void* A, const void* B, void* H, void* GU, int M, int F, int K, long long lda, long long ldb, int ldh, int ldgu,
-                       const void* scale_a, const void* scale_b, void* partial, void* scale, int num_sms, void* stream) {
+                       const void* scale_a, const void* scale_b, void* partial, int* count, int num_sms, void* stream) {
   using namespace kf::f8;
-  int blocks = 0;
-  const int rc = launch<SWIGLU>(A, B, H, M, F, K, lda, ldb, ldh, 0, 0, scale_a, scale_b, 0, GU, ldgu, partial, &blocks, num_sms, stream,
-                                reinterpret_cast<int*>(kf_status_device_ptr()));
-  return rc ? rc : launch_scale(partial, blocks * EPI_WARPS<SWIGLU>, E4M3_MAX, scale, stream);
+  return launch<SWIGLU>(A, B, H, M, F, K, lda, ldb, ldh, 0, 0, scale_a, scale_b, 0, GU, ldgu, partial, count, num_sms, stream,
+                        reinterpret_cast<int*>(kf_status_device_ptr()));
 }
 
-// DGU[M,2F] = SwiGLU'(GU) * (A8 * B8^T / (scale_a * scale_b)), A8 e5m2 (the incoming gradient), B8 e4m3 with F rows, and
-// scale[0] = fp8_max / absmax(DGU) for a cast to e5m2.  partial: eight floats per SM.
+// DGU[M,2F] = SwiGLU'(GU) * (A8 * B8^T / (scale_a * scale_b)), A8 e5m2 (the incoming gradient), B8 e4m3 with F rows; partial and count
+// as above, of |DGU|.
 int kf_gemm_fp8_swiglu_bwd(const void* A, const void* B, const void* GU, void* DGU, int M, int F, int K, long long lda, long long ldb, int ldgu,
-                           const void* scale_a, const void* scale_b, void* partial, void* scale, int num_sms, void* stream) {
+                           const void* scale_a, const void* scale_b, void* partial, int* count, int num_sms, void* stream) {
   using namespace kf::f8;
-  int blocks = 0;
-  const int rc = launch<SWIGLU_BWD>(A, B, DGU, M, F, K, lda, ldb, ldgu, 1, 0, scale_a, scale_b, 0, const_cast<void*>(GU), ldgu, partial, &blocks,
-                                    num_sms, stream, reinterpret_cast<int*>(kf_status_device_ptr()));
-  return rc ? rc : launch_scale(partial, blocks * EPI_WARPS<SWIGLU_BWD>, E5M2_MAX, scale, stream);
+  return launch<SWIGLU_BWD>(A, B, DGU, M, F, K, lda, ldb, ldgu, 1, 0, scale_a, scale_b, 0, const_cast<void*>(GU), ldgu, partial, count,
+                            num_sms, stream, reinterpret_cast<int*>(kf_status_device_ptr()));
+}
+
+// partial[0 .. *count) = partial maxima of |x| of n bf16 values; partial holds AMAX_BLOCKS (1024) floats.
+int kf_fp8_absmax_bf16(const void* x, long long n, void* partial, int* count, void* stream) {
+  using namespace kf::f8;
+  long long blocks = (n / 8 + 1023) / 1024;  // four loads per thread before a block is added
+  if (blocks < 1) blocks = 1;
+  if (blocks > AMAX_BLOCKS) blocks = AMAX_BLOCKS;
+  *count = (int)blocks;
+  kf_absmax_bf16<<<(int)blocks, 256, 0, (cudaStream_t)stream>>>(reinterpret_cast<const __nv_bfloat16*>(x), n,
+                                                                reinterpret_cast<float*>(partial));
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
 // scale[0] = fp8_max / absmax(x) for n bf16 values; amax_scratch holds AMAX_BLOCKS (1024) floats.
 int kf_fp8_scale_bf16(const void* x, long long n, int e5m2, void* amax_scratch, void* scale, void* stream) {
   using namespace kf::f8;
-  cudaStream_t st = (cudaStream_t)stream;
-  long long blocks = (n / 8 + 1023) / 1024;  // four loads per thread before a block is added
-  if (blocks < 1) blocks = 1;
-  if (blocks > AMAX_BLOCKS) blocks = AMAX_BLOCKS;
-  kf_absmax_bf16<<<(int)blocks, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(x), n,
-                                              reinterpret_cast<float*>(amax_scratch));
-  return launch_scale(amax_scratch, (int)blocks, e5m2 ? E5M2_MAX : E4M3_MAX, scale, stream);
+  int count = 0;
+  if (const int rc = kf_fp8_absmax_bf16(x, n, amax_scratch, &count, stream)) return rc;
+  kf_scale_from_amax<<<1, 256, 0, (cudaStream_t)stream>>>(reinterpret_cast<const float*>(amax_scratch), count,
+                                                          reinterpret_cast<float*>(scale), e5m2 ? E5M2_MAX : E4M3_MAX);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
-// fp8(x * scale) row-major into out (optional) and transposed into out_t (optional).
-int kf_fp8_cast_bf16(const void* x, int rows, int cols, long long ldx, const void* scale, int e5m2, void* out,
+// fp8(x * scale) row-major into out (optional) and transposed into out_t (optional).  With n > 0 the scale is fp8_max / the largest of
+// partial[0 .. n), and is stored in scale[0]; else it is read there.
+int kf_fp8_cast_bf16(const void* x, int rows, int cols, long long ldx, const void* partial, int n, void* scale, int e5m2, void* out,
                      long long ld_out, void* out_t, long long ld_t, void* stream) {
   using namespace kf::f8;
+  auto pp = n > 0 ? reinterpret_cast<const float*>(partial) : nullptr;
   dim3 grid((cols + 127) / 128, (rows + 127) / 128);
   auto xp = reinterpret_cast<const __nv_bfloat16*>(x);
-  auto sp = reinterpret_cast<const float*>(scale);
+  auto sp = reinterpret_cast<float*>(scale);
   if (e5m2)
-    kf_cast_fp8<true><<<grid, 256, 0, (cudaStream_t)stream>>>(xp, rows, cols, ldx, sp, (uint8_t*)out, ld_out,
+    kf_cast_fp8<true><<<grid, 256, 0, (cudaStream_t)stream>>>(xp, rows, cols, ldx, pp, n, sp, (uint8_t*)out, ld_out,
                                                               (uint8_t*)out_t, ld_t);
   else
-    kf_cast_fp8<false><<<grid, 256, 0, (cudaStream_t)stream>>>(xp, rows, cols, ldx, sp, (uint8_t*)out, ld_out,
+    kf_cast_fp8<false><<<grid, 256, 0, (cudaStream_t)stream>>>(xp, rows, cols, ldx, pp, n, sp, (uint8_t*)out, ld_out,
                                                                (uint8_t*)out_t, ld_t);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;

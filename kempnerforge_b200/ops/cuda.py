@@ -14,6 +14,7 @@ import math
 import os
 from array import array
 from ctypes import c_float, c_int, c_longlong, c_void_p
+from typing import NamedTuple
 
 import torch
 
@@ -91,7 +92,8 @@ def _declare(L: ctypes.CDLL) -> None:
         "kf_fp8_scale_bf16": [vp, ll, i, vp, vp, vp],
         "kf_gemm_fp8_swiglu": [vp, vp, vp, vp, i, i, i, ll, ll, i, i, vp, vp, vp, vp, i, vp],
         "kf_gemm_fp8_swiglu_bwd": [vp, vp, vp, vp, i, i, i, ll, ll, i, vp, vp, vp, vp, i, vp],
-        "kf_fp8_cast_bf16": [vp, i, i, ll, vp, i, vp, ll, vp, ll, vp],
+        "kf_fp8_absmax_bf16": [vp, ll, vp, vp, vp],
+        "kf_fp8_cast_bf16": [vp, i, i, ll, vp, i, vp, i, vp, ll, vp, ll, vp],
         "kf_lion": [vp, vp, vp, ll, i, f, f, f, f, vp],
         "kf_sf_adamw": [vp, vp, vp, vp, vp, ll, i, f, f, f, f, f, f, f, i, vp],
         "kf_ep_put_bf16": [vp, vp, i, vp, i, i, i, i, ll, vp, vp, i, vp],
@@ -717,6 +719,23 @@ def gemm_swiglu_pair_supported(x2: torch.Tensor, w: torch.Tensor, f: int) -> boo
 
 
 # --------------------------------------------------------------------------- fp8
+class PartialMax(NamedTuple):
+    """Where |x| was taken the maximum of: a slot for the scale that :func:`fp8_cast` makes of it, then ``count`` partial maxima."""
+
+    scratch: torch.Tensor
+    count: int
+
+
+def fp8_absmax(x2: torch.Tensor) -> PartialMax:
+    """The maxima that :func:`fp8_scale` makes its scale of."""
+    scratch = torch.empty(1 + 1024, dtype=torch.float32, device=x2.device)
+    if not x2.is_contiguous():
+        x2 = x2.contiguous()
+    count = ctypes.c_int()
+    _check(lib().kf_fp8_absmax_bf16(x2.data_ptr(), x2.numel(), scratch.data_ptr() + 4, ctypes.byref(count), _stream()), "kf_fp8_absmax_bf16")
+    return PartialMax(scratch, count.value)
+
+
 def fp8_scale(x2: torch.Tensor, e5m2: bool = False) -> torch.Tensor:
     """Device scalar fp8_max / absmax(x) (fp32, shape (1,))."""
     scratch = torch.empty(1 + 1024, dtype=torch.float32, device=x2.device)   # the scale, then partial maxima
@@ -727,9 +746,12 @@ def fp8_scale(x2: torch.Tensor, e5m2: bool = False) -> torch.Tensor:
     return scratch[:1]
 
 
-def fp8_cast(x2: torch.Tensor, scale: torch.Tensor, e5m2: bool, want_row: bool = True, want_t: bool = False):
+def fp8_cast(x2: torch.Tensor, scale: torch.Tensor | PartialMax, e5m2: bool, want_row: bool = True, want_t: bool = False):
     """fp8 bytes of x * scale: (rows, cols) and / or the transposed (cols, rows) copy, as uint8 tensors.  The rows of the transposed
-    copy start on 128 bytes."""
+    copy start on 128 bytes.  Of the maxima of x the kernel makes the scale itself and leaves it in ``scratch[:1]``."""
+    partial, count = None, 0
+    if isinstance(scale, PartialMax):
+        partial, count, scale = scale.scratch.data_ptr() + 4, scale.count, scale.scratch
     rows, cols = x2.shape
     assert x2.stride(1) == 1
     row = torch.empty((rows, cols), dtype=torch.uint8, device=x2.device) if want_row else None
@@ -737,7 +759,7 @@ def fp8_cast(x2: torch.Tensor, scale: torch.Tensor, e5m2: bool, want_row: bool =
     # lines.  Weight gradients of a 7B feed-forward over 2000 tokens, us: gate | up 216 -> 151, down 107 -> 77
     pitch = -(-rows // 128) * 128
     t = torch.empty((cols, pitch), dtype=torch.uint8, device=x2.device)[:, :rows] if want_t else None
-    _check(lib().kf_fp8_cast_bf16(x2.data_ptr(), rows, cols, x2.stride(0), scale.data_ptr(), int(e5m2),
+    _check(lib().kf_fp8_cast_bf16(x2.data_ptr(), rows, cols, x2.stride(0), partial, count, scale.data_ptr(), int(e5m2),
                                   row.data_ptr() if want_row else None, cols, t.data_ptr() if want_t else None, pitch,
                                   _stream()), "kf_fp8_cast_bf16")
     return row, t
@@ -760,34 +782,36 @@ def gemm_fp8(a8: torch.Tensor, b8: torch.Tensor, sa: torch.Tensor, sb: torch.Ten
 
 
 def gemm_fp8_swiglu(a8: torch.Tensor, b8: torch.Tensor, sa: torch.Tensor, sb: torch.Tensor):
-    """(gu, h, s): :func:`gemm_fp8` of e4m3 operands, b8 = [gate ; up] (2F rows), :func:`swiglu_fwd` of it and :func:`fp8_scale` of that, from one
-    kernel and the small one that turns its maxima into a scale."""
+    """(gu, h, maxima of h): :func:`gemm_fp8` of e4m3 operands, b8 = [gate ; up] (2F rows), :func:`swiglu_fwd` of it and
+    :func:`fp8_absmax` of that, from one kernel."""
     m, k = a8.shape
     f = b8.shape[0] // 2
     assert b8.shape == (2 * f, k) and a8.stride(1) == 1 and b8.stride(1) == 1
     gu = torch.empty((m, 2 * f), dtype=torch.bfloat16, device=a8.device)
     h = torch.empty((m, f), dtype=torch.bfloat16, device=a8.device)
-    scratch = torch.empty(1 + 8 * sm_count(), dtype=torch.float32, device=a8.device)   # the scale, then partial maxima
+    scratch = torch.empty(1 + 8 * sm_count(), dtype=torch.float32, device=a8.device)
+    count = ctypes.c_int()
     _check(lib().kf_gemm_fp8_swiglu(a8.data_ptr(), b8.data_ptr(), h.data_ptr(), gu.data_ptr(), m, f, k, a8.stride(0), b8.stride(0), f, 2 * f,
-                                    sa.data_ptr(), sb.data_ptr(), scratch.data_ptr() + 4, scratch.data_ptr(), sm_count(), _stream()),
-           "kf_gemm_fp8_swiglu", 2)
-    return gu, h, scratch[:1]
+                                    sa.data_ptr(), sb.data_ptr(), scratch.data_ptr() + 4, ctypes.byref(count), sm_count(), _stream()),
+           "kf_gemm_fp8_swiglu")
+    return gu, h, PartialMax(scratch, count.value)
 
 
 def gemm_fp8_swiglu_bwd(a8: torch.Tensor, b8: torch.Tensor, sa: torch.Tensor, sb: torch.Tensor, gu: torch.Tensor):
-    """(dgu, s): :func:`swiglu_bwd` of :func:`gemm_fp8` of an e5m2 gradient and e4m3 weights (F rows) in a tensor of its own, and its e5m2
-    :func:`fp8_scale`; the gradient of the hidden activation stays on the chip."""
+    """(dgu, its maxima): :func:`swiglu_bwd` of :func:`gemm_fp8` of an e5m2 gradient and e4m3 weights (F rows) in a tensor of its own,
+    and :func:`fp8_absmax` of it; the gradient of the hidden activation stays on the chip."""
     m, k = a8.shape
     f = b8.shape[0]
     assert b8.shape[1] == k and a8.stride(1) == 1 and b8.stride(1) == 1 and gu.shape == (m, 2 * f)
     if not gu.is_contiguous() or gu.data_ptr() % 32:
         gu = gu.clone(memory_format=torch.contiguous_format)
     dgu = torch.empty_like(gu)
-    scratch = torch.empty(1 + 8 * sm_count(), dtype=torch.float32, device=a8.device)   # the scale, then partial maxima
+    scratch = torch.empty(1 + 8 * sm_count(), dtype=torch.float32, device=a8.device)
+    count = ctypes.c_int()
     _check(lib().kf_gemm_fp8_swiglu_bwd(a8.data_ptr(), b8.data_ptr(), gu.data_ptr(), dgu.data_ptr(), m, f, k, a8.stride(0), b8.stride(0), 2 * f,
-                                        sa.data_ptr(), sb.data_ptr(), scratch.data_ptr() + 4, scratch.data_ptr(), sm_count(), _stream()),
-           "kf_gemm_fp8_swiglu_bwd", 2)
-    return dgu, scratch[:1]
+                                        sa.data_ptr(), sb.data_ptr(), scratch.data_ptr() + 4, ctypes.byref(count), sm_count(), _stream()),
+           "kf_gemm_fp8_swiglu_bwd")
+    return dgu, PartialMax(scratch, count.value)
 
 
 # --------------------------------------------------------------------------- attention

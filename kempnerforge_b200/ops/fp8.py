@@ -58,15 +58,16 @@ def is_fp8_weight(w: torch.Tensor) -> bool:
 
 # --------------------------------------------------------------------------- quantisation
 def quantize(x2: torch.Tensor, e5m2: bool = False, want_row: bool = True, want_t: bool = False,
-             scale: torch.Tensor | None = None):
-    """(scale, row-major fp8 bytes or None, transposed fp8 bytes or None) of a 2-D bf16 tensor."""
+             scale=None):
+    """(scale, row-major fp8 bytes or None, transposed fp8 bytes or None) of a 2-D bf16 tensor.  ``scale``: the one to use, or (on a GPU) the
+    maxima that the kernel before took of ``x2``; else the largest magnitude is looked for."""
     from kempnerforge_b200.ops import cuda as cu
 
     if x2.is_cuda:
         if scale is None:
-            scale = cu.fp8_scale(x2, e5m2)
+            scale = cu.fp8_absmax(x2)
         row, t = cu.fp8_cast(x2, scale, e5m2, want_row, want_t)
-        return scale, row, t
+        return scale.scratch[:1] if isinstance(scale, cu.PartialMax) else scale, row, t
     fmax = E5M2_MAX if e5m2 else E4M3_MAX
     dt = torch.float8_e5m2 if e5m2 else torch.float8_e4m3fn
     if scale is None:
@@ -163,8 +164,8 @@ class _Fp8SwiGLUFn(torch.autograd.Function):
             x2 = x2.contiguous()
         sx, x8, _ = quantize(x2)
         s_gu, w8, _ = quantized_weight((wg, wu), want_t=False)
-        gu, h, sh = cu.gemm_fp8_swiglu(x8, w8, sx, s_gu)
-        _, h8, h8t = quantize(h, scale=sh, want_t=recording and ctx.needs_input_grad[3])
+        gu, h, h_max = cu.gemm_fp8_swiglu(x8, w8, sx, s_gu)
+        sh, h8, h8t = quantize(h, scale=h_max, want_t=recording and ctx.needs_input_grad[3])
         sd, d8, _ = quantized_weight((wd,), want_t=False)
         y = scaled_mm(h8, d8, sh, sd)
         ctx.save_for_backward(x2, sx, s_gu, gu, h8t, sh, sd, wg, wu, wd)
@@ -186,13 +187,13 @@ class _Fp8SwiGLUFn(torch.autograd.Function):
         dx = g_wg = g_wu = g_wd = None
         if need_h:
             _, _, d8t = quantized_weight((wd,), want_t=True)
-            dgu, s_dgu = cu.gemm_fp8_swiglu_bwd(g8, d8t, sg, sd, gu)
+            dgu, dgu_max = cu.gemm_fp8_swiglu_bwd(g8, d8t, sg, sd, gu)
         if need_d:
             (g_wd,) = F._deposit_stacked_weight_grads(
                 [wd], (True,), lambda out, acc: scaled_mm(g8t, h8t, sg, sh, a_e5m2=True, out=out, accumulate=acc))
         if need_h:
             need_w = need_g or need_u
-            _, q8, q8t = quantize(dgu, e5m2=True, want_row=need_x, want_t=need_w, scale=s_dgu)
+            s_dgu, q8, q8t = quantize(dgu, e5m2=True, want_row=need_x, want_t=need_w, scale=dgu_max)
             if need_x:
                 _, _, w8t = quantized_weight((wg, wu), want_t=True)
                 dx = scaled_mm(q8, w8t, s_dgu, s_gu, a_e5m2=True).view(ctx.x_shape)

@@ -80,11 +80,17 @@ def test_products_with_swiglu_epilogues(native_lib, t, k, f):
     x8, w8 = q(t), q(2 * f)
     gu = cu.gemm_fp8(x8, w8, sa, sb)
     h = cu.swiglu_fwd(gu)
-    got = cu.gemm_fp8_swiglu(x8, w8, sa, sb)
-    assert _equal(got, (gu, h, cu.fp8_scale(h)))
+    *got, h_max = cu.gemm_fp8_swiglu(x8, w8, sa, sb)
+    assert _equal(got, (gu, h))
+    assert _equal(cu.fp8_cast(h, h_max, False, True, True), cu.fp8_cast(h, cu.fp8_scale(h), False, True, True))
+    assert torch.equal(h_max.scratch[:1], cu.fp8_scale(h))
     g8, d8 = q(t, True), q(f)
     dgu = cu.swiglu_bwd(cu.gemm_fp8(g8, d8, sa, sb, a_e5m2=True), gu)
-    assert _equal(cu.gemm_fp8_swiglu_bwd(g8, d8, sa, sb, gu), (dgu, cu.fp8_scale(dgu, True)))
+    got, dgu_max = cu.gemm_fp8_swiglu_bwd(g8, d8, sa, sb, gu)
+    assert torch.equal(got, dgu)
+    for maxima in (dgu_max, cu.fp8_absmax(dgu)):
+        assert _equal(cu.fp8_cast(dgu, maxima, True, True, True), cu.fp8_cast(dgu, cu.fp8_scale(dgu, True), True, True, True))
+        assert torch.equal(maxima.scratch[:1], cu.fp8_scale(dgu, True))
     assert native_lib.read_status() == 0
 
 
