@@ -56,14 +56,14 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 struct F8 {
   float v[8];
 };
-__device__ __forceinline__ F8 load8(const __nv_bfloat16* p) {
-  uint4 u = *reinterpret_cast<const uint4*>(p);
+__device__ __forceinline__ F8 unpack8(const uint4 u) {
   F8 r;
   float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), c = unpack_bf16(u.z), d = unpack_bf16(u.w);
   r.v[0] = a.x; r.v[1] = a.y; r.v[2] = b.x; r.v[3] = b.y;
   r.v[4] = c.x; r.v[5] = c.y; r.v[6] = d.x; r.v[7] = d.y;
   return r;
 }
+__device__ __forceinline__ F8 load8(const __nv_bfloat16* p) { return unpack8(*reinterpret_cast<const uint4*>(p)); }
 __device__ __forceinline__ void store8(__nv_bfloat16* p, const F8& r) {
   uint4 u;
   u.x = pack_bf16(r.v[0], r.v[1]);
@@ -133,14 +133,6 @@ kf_rmsnorm_fwd(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
 // few rows (decoding), where a row spread over a block finishes sooner, and for rows longer than 32 * 8 * 16 = 4096.
 constexpr int ROWS_PER_BLOCK = 4;
 constexpr int WARP_ROWS_MIN = 1024;  // rows from which warps per row fill the machine (148 SMs x 8 rows in flight)
-
-__device__ __forceinline__ F8 unpack8(const uint4 u) {
-  F8 r;
-  const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), c = unpack_bf16(u.z), d = unpack_bf16(u.w);
-  r.v[0] = a.x; r.v[1] = a.y; r.v[2] = b.x; r.v[3] = b.y;
-  r.v[4] = c.x; r.v[5] = c.y; r.v[6] = d.x; r.v[7] = d.y;
-  return r;
-}
 
 template <int VPL>
 __global__ void __launch_bounds__(32 * ROWS_PER_BLOCK)
@@ -528,6 +520,73 @@ kf_ce_fwd_bwd(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ 
   }
 }
 
+// The same where the product that wrote the logits left (largest, sum of exponentials) of every row and tile of columns,
+// stats[tile][rows]: one small kernel joins them per row, and the gradient is one pass over the logits, four 16-byte words of a thread
+// under way at once.  2047 rows of 128 256 columns: 280 us by blocks that read their row twice, 195 so (1.05 GB: 160 at the copy rate).  A
+// row held in the registers of a cluster of blocks took 340: load, exchange and store wait for one another.
+constexpr int CE_JOIN_WARPS = 32;
+__global__ void __launch_bounds__(32 * CE_JOIN_WARPS)
+kf_ce_join(const float2* __restrict__ stats, int tiles, const __nv_bfloat16* __restrict__ logits, const long long* __restrict__ labels,
+           float* __restrict__ row_lse, float* __restrict__ row_nll, float* __restrict__ row_lse2, int rows, int V, int ld) {
+  __shared__ float2 part[CE_JOIN_WARPS][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = blockIdx.x * 32 + lane;
+  float m = -INFINITY, s = 0.f;
+  auto join = [&](const float2 p) {
+    const float m2 = fmaxf(m, p.x), base = m2 == -INFINITY ? 0.f : m2;
+    s = s * __expf(m - base) + p.y * __expf(p.x - base);
+    m = m2;
+  };
+  if (row < rows)
+    for (int t = warp; t < tiles; t += 4 * CE_JOIN_WARPS) {  // four loads under way
+      float2 p[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        p[j] = t + j * CE_JOIN_WARPS < tiles ? stats[size_t(t + j * CE_JOIN_WARPS) * rows + row] : make_float2(-INFINITY, 0.f);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) join(p[j]);
+    }
+  part[warp][lane] = make_float2(m, s);
+  __syncthreads();
+  if (warp > 0 || row >= rows) return;
+  for (int w = 1; w < CE_JOIN_WARPS; ++w) join(part[w][lane]);
+  const float lse = m + __logf(s);
+  const long long label = labels[row];
+  const bool valid = label >= 0 && label < V;
+  row_lse[row] = lse;
+  row_nll[row] = valid ? lse - __bfloat162float(logits[size_t(row) * ld + label]) : 0.f;
+  row_lse2[row] = valid ? lse * lse : 0.f;
+}
+constexpr int CE_GRAD_THREADS = 256, CE_GRAD_WORDS = 4;
+__global__ void __launch_bounds__(CE_GRAD_THREADS)
+kf_ce_grad(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ labels, const float* __restrict__ row_lse,
+           const float* __restrict__ inv_n_ptr, float z_w, int V, int ld) {
+  const int row = blockIdx.y, nvec = V >> 3, v0 = blockIdx.x * (CE_GRAD_THREADS * CE_GRAD_WORDS) + threadIdx.x;
+  __nv_bfloat16* lr = logits + size_t(row) * ld;
+  uint4 w[CE_GRAD_WORDS];
+#pragma unroll
+  for (int j = 0; j < CE_GRAD_WORDS; ++j)
+    if (v0 + j * CE_GRAD_THREADS < nvec) w[j] = *reinterpret_cast<const uint4*>(lr + size_t(v0 + j * CE_GRAD_THREADS) * 8);
+  const long long label = labels[row];
+  const float lse = row_lse[row], inv_n = *inv_n_ptr;
+  const bool valid = label >= 0 && label < V;
+  const float gscale = valid ? inv_n * (1.f + 2.f * z_w * lse) : 0.f;
+  const int picked = valid ? int(label) : -8;
+#pragma unroll
+  for (int j = 0; j < CE_GRAD_WORDS; ++j) {
+    const int v = v0 + j * CE_GRAD_THREADS;
+    if (v >= nvec) break;
+    F8 t = unpack8(w[j]);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t.v[i] = __expf(t.v[i] - lse) * gscale;
+    if ((picked >> 3) == v) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (v * 8 + i == picked) t.v[i] -= inv_n;
+    }
+    store8(lr + size_t(v) * 8, t);
+  }
+}
+
 // x *= factor (one fp32 device scalar, rounded to bf16 like the tensor it scales).  A factor of exactly one, the gradient
 // that loss.backward() starts from, leaves x untouched and costs one scalar read per block.  Out of place, the pass over the
 // gradient of a 128 256 x 4096 weight (1 GB) took 1328 us of a 6413 us loss over 2047 tokens.
@@ -869,6 +928,23 @@ int kf_ce_fwd_bwd_bf16(void* logits, const void* labels, void* row_nll, void* ro
   kf_ce_fwd_bwd<<<rows, CE_THREADS, 0, (cudaStream_t)stream>>>(
       (__nv_bfloat16*)logits, (const long long*)labels, (float*)row_nll, (float*)row_lse2,
       (const float*)inv_n, z_w, V, ld);
+  KF_LAUNCH_CHECK();
+}
+
+// kf_ce_fwd_bwd_bf16 of logits whose product left stats[tiles][rows] (kf_gemm_logits_bf16).  V a multiple of 8; row_lse: rows floats.
+int kf_ce_grad_bf16(void* logits, const void* stats, int tiles, const void* labels, void* row_lse, void* row_nll, void* row_lse2,
+                    const void* inv_n, float z_w, int rows, int V, int ld, void* stream) {
+  using namespace kf;
+  if (ld % 8 || V % 8) return 1;
+  constexpr int per_block = CE_GRAD_THREADS * CE_GRAD_WORDS;
+  kf_ce_join<<<(rows + 31) / 32, 32 * CE_JOIN_WARPS, 0, (cudaStream_t)stream>>>(
+      (const float2*)stats, tiles, (const __nv_bfloat16*)logits, (const long long*)labels, (float*)row_lse, (float*)row_nll,
+      (float*)row_lse2, rows, V, ld);
+  for (int r = 0; r < rows; r += 65535) {
+    const int n = rows - r < 65535 ? rows - r : 65535;
+    kf_ce_grad<<<dim3((V / 8 + per_block - 1) / per_block, n), CE_GRAD_THREADS, 0, (cudaStream_t)stream>>>(
+        (__nv_bfloat16*)logits + size_t(r) * ld, (const long long*)labels + r, (const float*)row_lse + r, (const float*)inv_n, z_w, V, ld);
+  }
   KF_LAUNCH_CHECK();
 }
 

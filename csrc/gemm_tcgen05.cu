@@ -314,6 +314,7 @@ static int plain_mode(int M, int N, int b_mn, int num_sms) {
 }  // namespace kf
 
 namespace kf2 {
+int gemm_pair_width(int M, int N, int num_sms);
 int swiglu_tokens(int M, int F, int K, int num_sms);
 int rope_tokens(int M, int N, int hd, int num_sms);
 int swiglu_bwd_tokens(int M, int F, int num_sms);
@@ -482,6 +483,14 @@ int kf_gemm_bf16(const void* A, const void* B, void* C, const void* R, int M, in
   if (a_mn && !b_mn) return KF_DISPATCH(true, false);
   return KF_DISPATCH(true, true);
 #undef KF_DISPATCH
+}
+
+// Width of the column tiles of kf_gemm_logits_bf16 where that kernel is the one that kf_gemm_bf16 takes for K-major operands and a
+// bf16 result, else 0.
+int kf_gemm_logits_width(int M, int N, int K, int num_sms) {
+  using namespace kf;
+  if (M <= 0 || N <= 0 || K <= 0 || num_sms < 2 || (N & 7) || plain_mode(M, N, 0, num_sms) != 2 || plain_tokens(M, N, K, 0, true, num_sms)) return 0;
+  return kf2::gemm_pair_width(M, N, num_sms);
 }
 
 // Status word shared by all kernels of this library on the current device (0 = healthy).

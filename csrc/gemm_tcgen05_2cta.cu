@@ -137,12 +137,18 @@ __device__ __forceinline__ TileCoord tile_coord(int t, int m_blocks, int n_block
 // SWIGLU == 5 (fp32 partial sums, K-major A, MN-major B): the product of every tile is cut along K into `splits` units; unit
 // u = piece * tiles + tile writes its sum to C + piece * M * ldc.  The piece is the slow index, so the pairs work on (nearly) the
 // same k at a time and share the operand panels in L2; a cut of the last round alone puts them at different k and lost 40 %.
+//
+// SWIGLU == 6 (bf16, K-major operands): C is rows of logits; for every row and tile of columns stats[tc.n * M + row] = (largest value,
+// sum of exp(value - largest)) of what was stored there, so that the cross entropy need not read the rows for them.  The exponentials
+// hide behind the next tile's products: 2047 x 128 256 from 4096 columns 1387 -> 1395 us (and the rows 280 -> 195), 4096 x 50 304
+// from 1024 289 -> 305, but from 768, twelve k-blocks, 228 -> 263.
 struct RopeArgs {
   const float* cosT;  // [S][hd / 2]
   const float* sinT;
   int S, cols, hd;
   float alpha, beta, diag;  // SWIGLU == 4 only
   int splits;               // SWIGLU == 5 only
+  float2* stats;            // SWIGLU == 6 only
 };
 
 // Weight operand made of up to three matrices stacked along N (q | k | v; SwiGLU == 1: gate and up): one tensor map each,
@@ -154,6 +160,34 @@ struct WeightSegs {
   CUtensorMap map[3];
   int start[3];
 };
+
+// The first `valid` (a multiple of eight) columns of a chunk of a row join its (largest value, sum of exponentials relative to it).
+__device__ __forceinline__ void row_stats(const Rows32& own, int valid, float& largest, float& sum) {
+  float m = largest;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    if (q * 8 >= valid) break;
+    const uint32_t w[4] = {own.q[q].x, own.q[q].y, own.q[q].z, own.q[q].w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = unpack_bf16(w[i]);
+      m = fmaxf(m, fmaxf(f.x, f.y));
+    }
+  }
+  const float base = m == -INFINITY ? 0.f : m;  // nothing but masked columns so far: their exponentials are zeros
+  sum *= __expf(largest - base);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    if (q * 8 >= valid) break;
+    const uint32_t w[4] = {own.q[q].x, own.q[q].y, own.q[q].z, own.q[q].w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = unpack_bf16(w[i]);
+      sum += __expf(f.x - base) + __expf(f.y - base);
+    }
+  }
+  largest = m;
+}
 
 template <bool A_MN, bool B_MN, typename OutT, int SWIGLU = 0, bool GATHER = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GATHER ? THREADS_GATHER : THREADS, 1)
@@ -493,12 +527,19 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
       const int col0 = tc.n * tile_n, width = min(tile_n, N - col0);
       OutT* c_row = C + (SWIGLU == 5 ? size_t(piece_of(t)) * M * ldc : 0) + size_t(row) * ldc + col0;
       const OutT* r_row = R ? R + size_t(row) * ldr + col0 : nullptr;
+      float largest = -INFINITY, sum = 0.f;  // SWIGLU == 6
 #pragma unroll 1
       for (int c = 0; c * 32 < width; ++c) {
         uint32_t v[32];
         tmem_ld_32x32(t_row + c * 32, v);
         tmem_ld_wait();
         const int valid = min(32, width - c * 32);
+        if constexpr (SWIGLU == 6) {
+          const Rows32 own = pack_row32(v);
+          row_stats(own, valid, largest, sum);
+          store_rows32(box, lane, own, reinterpret_cast<__nv_bfloat16*>(C) + size_t(row0) * ldc + col0 + c * 32, ldc, rows, valid);
+          continue;
+        }
         if constexpr (sizeof(OutT) == 2) {
           if (!accumulate && !r_row) {
             store_rows32(box, lane, pack_row32(v), reinterpret_cast<__nv_bfloat16*>(C) + size_t(row0) * ldc + col0 + c * 32, ldc,
@@ -508,6 +549,7 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
         }
         if (row < M) store_chunk<OutT>(c_row + c * 32, v, valid, accumulate != 0, r_row ? r_row + c * 32 : nullptr);
       }
+      if (SWIGLU == 6 && row < M) rope.stats[size_t(tc.n) * M + row] = make_float2(largest, sum);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) arrive_on_cta(tempty_bar(acc), 0);
@@ -925,6 +967,35 @@ static int launch_split_k(const void* A, const void* B, void* C, void* ws, int M
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
+// C[M][ldc] (bf16) = A[M, K] B[N, K]^T with stats (SWIGLU == 6): one row of M float2 for every tile of columns.
+static int launch_logits(const void* A, const void* B, void* C, void* stats, int M, int N, int K, int lda, int ldb, int ldc, int num_sms,
+                         cudaStream_t stream, int* status) {
+  CUtensorMap ma, mb;
+  int rc = make_map_2d_bf16(&ma, A, M, K, lda, BK, CTA_M);
+  if (rc) return 100 + rc;
+  int pairs = num_sms / 2;
+  const int tile_n = pair_tile_width(M, N, pairs, nullptr);
+  rc = make_map_2d_bf16(&mb, B, N, K, ldb, BK, tile_n / 2);
+  if (rc) return 200 + rc;
+  auto kern = kf_gemm_bf16_tcgen05_2cta<false, false, __nv_bfloat16, 6>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    if (e != cudaSuccess) return 300 + (int)e;
+    attr_set = true;
+  }
+  const int tiles = ((M + TILE_M - 1) / TILE_M) * ((N + tile_n - 1) / tile_n);
+  if (tiles < pairs) pairs = tiles;
+  RopeArgs ra{};
+  ra.stats = reinterpret_cast<float2*>(stats);
+  kern<<<pairs * 2, THREADS, SMEM_BYTES, stream>>>(ma, one_piece(mb), reinterpret_cast<__nv_bfloat16*>(C), nullptr, M, N, K, ldc, 0, 0,
+                                                   status, ra, tile_n, GatherArgs{});
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 400 + (int)e;
+}
+
+int gemm_pair_width(int M, int N, int num_sms) { return pair_tile_width(M, N, num_sms / 2, nullptr); }
+
 int launch_gemm_2cta(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb,
                      int ldc, int ldr, int a_mn, int b_mn, int out_f32, int accumulate, int num_sms,
                      cudaStream_t stream, int* status) {
@@ -945,6 +1016,13 @@ void* kf_status_device_ptr();
 
 // Number of pieces along K that kf_gemm_split_k_bf16 should be given for this product (1: use kf_gemm_bf16).
 int kf_gemm_k_pieces(int M, int N, int K, int num_sms) { return kf2::k_pieces(M, N, K, num_sms); }
+
+// C[M][ldc] (bf16) = A[M][lda] B[N][ldb]^T and stats[tiles of columns][M] float2, the tiles kf_gemm_logits_width columns wide.
+int kf_gemm_logits_bf16(const void* A, const void* B, void* C, void* stats, int M, int N, int K, int lda, int ldb, int ldc, int num_sms,
+                        void* stream) {
+  if (M < 1 || N < 8 || K < 1 || (N & 7) || ((lda | ldb | ldc) & 7) || num_sms < 2) return 5;
+  return kf2::launch_logits(A, B, C, stats, M, N, K, lda, ldb, ldc, num_sms, (cudaStream_t)stream, (int*)kf_status_device_ptr());
+}
 
 // C[M][ldc] (bf16) = A[M][lda] B[K][ldb]; ws: fp32 [splits][M][N].  N a multiple of 8, 2 <= splits <= K / 64.
 int kf_gemm_split_k_bf16(const void* A, const void* B, void* C, void* ws, int M, int N, int K, int lda, int ldb, int ldc, int splits,

@@ -82,6 +82,9 @@ def _declare(L: ctypes.CDLL) -> None:
         "kf_embedding_fwd_bf16": [vp, vp, vp, ll, i, i, vp],
         "kf_embedding_bwd_bf16": [vp, vp, vp, ll, i, i, vp],
         "kf_ce_fwd_bwd_bf16": [vp, vp, vp, vp, vp, f, i, i, i, vp],
+        "kf_ce_grad_bf16": [vp, vp, i, vp, vp, vp, vp, vp, f, i, i, i, vp],
+        "kf_gemm_logits_width": [i, i, i, i],
+        "kf_gemm_logits_bf16": [vp, vp, vp, vp, i, i, i, i, i, i, i, vp],
         "kf_scale_bf16": [vp, ll, vp, vp],
         "kf_ce_vp_stats_bf16": [vp, vp, ll, vp, vp, vp, i, i, i, vp],
         "kf_ce_vp_bwd_bf16": [vp, vp, ll, vp, vp, vp, f, i, i, i, vp],
@@ -588,20 +591,54 @@ def embedding_bwd(dy: torch.Tensor, ids: torch.Tensor, dtable: torch.Tensor, acc
 
 
 # --------------------------------------------------------------------------- cross entropy
-def ce_fwd_bwd(logits: torch.Tensor, labels: torch.Tensor, stats: torch.Tensor, inv_n: torch.Tensor, z_weight: float) -> None:
-    """Overwrites ``logits`` (rows, V) with d loss / d logits and adds [sum nll, sum lse²] into ``stats``."""
+# Row statistics in the epilogue of the logits pay where its exponentials hide behind the products (K) and where a second read of the rows
+# comes from HBM rather than from the 126 MB of L2 (bytes of logits).  Product and cross entropy, us, without / with: 2047 x 128 256 from
+# 4096 1613 / 1548, 1024 x 128 256 from 2048 490 / 454, 4096 x 32 000 from 2048 455 / 440 and from 1024 288 / 281, 4096 x 50 304 from 1024
+# 449 / 430; the whole loss over 1698 rows from 768 341 / 344, over 249 rows of 128 256 from 4096 949 / 952.
+LOGITS_MIN_K = 1024
+LOGITS_MIN_BYTES = 128 << 20
+
+
+def gemm_logits(h: torch.Tensor, weight: torch.Tensor):
+    """(:func:`gemm` of K-major operands, for every tile of its columns and row the largest value and the sum of exponentials relative to
+    it as (tiles, rows, 2) fp32, or None where another kernel makes the product)."""
+    (m, k), n = h.shape, weight.shape[0]
+    width = 0
+    if GEMM_MODE == 0 and k >= LOGITS_MIN_K and 2 * m * n >= LOGITS_MIN_BYTES and not _few_rows(m, n) and k % 8 == 0 and h.stride(0) % 8 == 0 and weight.stride(0) % 8 == 0:
+        width = lib().kf_gemm_logits_width(m, n, k, sm_count())
+    if width == 0 or h.data_ptr() % 16 or weight.data_ptr() % 16:
+        return gemm(h, weight, a_kmajor=True, b_kmajor=True), None
+    assert h.dtype == weight.dtype == torch.bfloat16 and weight.shape[1] == k and h.stride(1) == weight.stride(1) == 1
+    assert h.device == weight.device
+    out = torch.empty((m, n), dtype=torch.bfloat16, device=h.device)
+    stats = torch.empty((-(-n // width), m, 2), dtype=torch.float32, device=h.device)
+    _check(lib().kf_gemm_logits_bf16(h.data_ptr(), weight.data_ptr(), out.data_ptr(), stats.data_ptr(), m, n, k, h.stride(0), weight.stride(0), n,
+                                     sm_count(), _stream()), "kf_gemm_logits_bf16")
+    return out, stats
+
+
+def ce_fwd_bwd(logits: torch.Tensor, labels: torch.Tensor, stats: torch.Tensor, inv_n: torch.Tensor, z_weight: float,
+               tiles: torch.Tensor | None = None) -> None:
+    """Overwrites ``logits`` (rows, V) with d loss / d logits and adds [sum nll, sum lse²] into ``stats``.  ``tiles``: what
+    :func:`gemm_logits` returned with them."""
     rows, v = logits.shape
     assert logits.stride(1) == 1
     row_nll = torch.empty(rows, dtype=torch.float32, device=logits.device)
     row_lse2 = torch.empty(rows, dtype=torch.float32, device=logits.device)
     labels = labels.contiguous()
-    _check(
-        lib().kf_ce_fwd_bwd_bf16(
-            logits.data_ptr(), labels.data_ptr(), row_nll.data_ptr(), row_lse2.data_ptr(), inv_n.data_ptr(),
-            float(z_weight), rows, v, logits.stride(0), _stream(),
-        ),
-        "kf_ce_fwd_bwd_bf16",
-    )
+    if tiles is not None:
+        row_lse = torch.empty(rows, dtype=torch.float32, device=logits.device)
+        _check(lib().kf_ce_grad_bf16(logits.data_ptr(), tiles.data_ptr(), tiles.shape[0], labels.data_ptr(), row_lse.data_ptr(),
+                                     row_nll.data_ptr(), row_lse2.data_ptr(), inv_n.data_ptr(), float(z_weight), rows, v, logits.stride(0),
+                                     _stream()), "kf_ce_grad_bf16", 2)
+    else:
+        _check(
+            lib().kf_ce_fwd_bwd_bf16(
+                logits.data_ptr(), labels.data_ptr(), row_nll.data_ptr(), row_lse2.data_ptr(), inv_n.data_ptr(),
+                float(z_weight), rows, v, logits.stride(0), _stream(),
+            ),
+            "kf_ce_fwd_bwd_bf16",
+        )
     stats[0] += row_nll.sum()
     stats[1] += row_lse2.sum()
 

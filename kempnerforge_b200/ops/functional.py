@@ -535,9 +535,9 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
         dw = torch.empty_like(weight)
         for lo in range(0, t, chunk):
             hi = min(t, lo + chunk)
-            logits = cu.gemm(h2[lo:hi], weight, a_kmajor=True, b_kmajor=True)
+            logits, tiles = cu.gemm_logits(h2[lo:hi], weight)
             # in place: logits <- d(loss)/dlogits ; stats accumulate
-            cu.ce_fwd_bwd(logits, lab[lo:hi], stats, inv_n, z_weight)
+            cu.ce_fwd_bwd(logits, lab[lo:hi], stats, inv_n, z_weight, tiles)
             cu.gemm(logits, weight, a_kmajor=True, b_kmajor=False, out=dh[lo:hi])
             cu.gemm(logits, h2[lo:hi], a_kmajor=False, b_kmajor=False, out=dw, accumulate=lo > 0)
         ctx.save_for_backward(dh, dw)
