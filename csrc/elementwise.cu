@@ -75,28 +75,32 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const F8& r) {
 
 // ------------------------------------------------------------------ RMSNorm
 constexpr int NORM_THREADS = 256;
-constexpr int NORM_CACHE = 4;  // vectors of 8 kept in registers per thread (covers D <= 8192)
 
+// CACHE: 16-byte words of a row per thread that are all under way at once and stay in registers, packed, between the two passes: 2 for
+// D <= 4096, 4 for D <= 8192.
+template <int CACHE>
 __global__ void __launch_bounds__(NORM_THREADS)
 kf_rmsnorm_fwd(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, int rows, int D, float eps) {
   __shared__ float red[40];
   const int nvec = D >> 3;
-  constexpr int CACHED = NORM_CACHE * NORM_THREADS;  // vectors kept in registers per row
+  constexpr int CACHED = CACHE * NORM_THREADS;  // vectors kept in registers per row
   grid_dep_wait();
   grid_dep_launch();
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const __nv_bfloat16* xr = x + size_t(row) * D;
-    F8 cache[NORM_CACHE];
+    uint4 cache[CACHE];
     float ss = 0.f;
 #pragma unroll
-    for (int c = 0; c < NORM_CACHE; ++c) {
+    for (int c = 0; c < CACHE; ++c) {
       const int v = threadIdx.x + c * NORM_THREADS;
-      if (v < nvec) {
-        cache[c] = load8(xr + v * 8);
+      cache[c] = v < nvec ? *reinterpret_cast<const uint4*>(xr + v * 8) : make_uint4(0, 0, 0, 0);
+    }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) ss += cache[c].v[i] * cache[c].v[i];
-      }
+    for (int c = 0; c < CACHE; ++c) {
+      const F8 t = unpack8(cache[c]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) ss += t.v[i] * t.v[i];
     }
     for (int v = threadIdx.x + CACHED; v < nvec; v += NORM_THREADS) {
       const F8 t = load8(xr + v * 8);
@@ -107,11 +111,11 @@ kf_rmsnorm_fwd(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
     if (threadIdx.x == 0 && rstd) rstd[row] = r;
     __nv_bfloat16* yr = y + size_t(row) * D;
 #pragma unroll
-    for (int c = 0; c < NORM_CACHE; ++c) {
+    for (int c = 0; c < CACHE; ++c) {
       const int v = threadIdx.x + c * NORM_THREADS;
       if (v < nvec) {
         const F8 g = load8(w + v * 8);
-        F8 t = cache[c];
+        F8 t = unpack8(cache[c]);
 #pragma unroll
         for (int i = 0; i < 8; ++i) t.v[i] = t.v[i] * r * g.v[i];
         store8(yr + v * 8, t);
@@ -127,10 +131,11 @@ kf_rmsnorm_fwd(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
   }
 }
 
-// Many rows: one warp per row, the whole row in registers (VPL 16-byte vectors per lane, all loads issued before the first
-// use), reduction by shuffles only.  The block-per-row kernel above spends two block barriers per row with one 16-byte load
-// in flight per thread; at 8192 x 4096 it took 36 us (134 MB: 20 us at the copy rate), this one 30 us.  It stays for
-// few rows (decoding), where a row spread over a block finishes sooner, and for rows longer than 32 * 8 * 16 = 4096.
+// Many short rows: one warp per row, the whole row in registers (VPL 16-byte vectors per lane, all loads issued before the first
+// use), reduction by shuffles only; a block per row leaves threads of it without work.  us, warp / block per row, caches cold: 8192 x 768
+// 7.4 / 19.0, 4096 x 1024 5.7 / 10.9, 4096 x 2048 10.9 / 12.5, 1777 x 2048 6.9 / 7.0, but 8192 x 4096 31.9 / 28.7 (20.5 at the copy
+// rate) and 1554 x 4096 11.9 / 8.2: sixteen vectors per lane leave too few warps on an SM.  With few rows (decoding) a row spread over a
+// block finishes sooner.
 constexpr int ROWS_PER_BLOCK = 4;
 constexpr int WARP_ROWS_MIN = 1024;  // rows from which warps per row fill the machine (148 SMs x 8 rows in flight)
 
@@ -168,9 +173,10 @@ kf_rmsnorm_fwd_warp(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __
     }
 }
 
-// dx = [dx_in +] r*g - x*r^3*mean(g*x), one warp per row, up to 2048 columns (at 4096 both rows take 128 registers and the
-// occupancy with them: 116 us against the block kernel's 85 at 8192 x 4096); every read of dy and dx_in precedes the writes of the same
-// elements by the same thread, so dx may alias either.
+// dx = [dx_in +] r*g - x*r^3*mean(g*x), one warp per row, up to 1024 columns: warp / block per row, us, caches cold, 8192 x 768 10.6 / 26.5,
+// 4096 x 1024 8.1 / 14.6, but 4096 x 2048 with eight vectors per lane 26.3 / 17.9.  Every read of dy and dx_in precedes the writes of the
+// same elements by the same thread, so dx may alias either.  dx_in comes with the other two, not after the reduction: 8192 x 768
+// 12.7 -> 10.6 us.
 template <int VPL>
 __global__ void __launch_bounds__(32 * ROWS_PER_BLOCK)
 kf_rmsnorm_bwd_dx_warp(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
@@ -182,12 +188,14 @@ kf_rmsnorm_bwd_dx_warp(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16
   const uint4* xr = reinterpret_cast<const uint4*>(x + size_t(row) * D);
   const uint4* gr = reinterpret_cast<const uint4*>(dy + size_t(row) * D);
   const uint4 zero = make_uint4(0, 0, 0, 0);
-  uint4 xv[VPL], gv[VPL];
+  const uint4* ir = dx_in ? reinterpret_cast<const uint4*>(dx_in + size_t(row) * D) : nullptr;
+  uint4 xv[VPL], gv[VPL], iv[VPL];
 #pragma unroll
   for (int c = 0; c < VPL; ++c) {
     const bool in = lane + c * 32 < nvec;
     xv[c] = in ? xr[lane + c * 32] : zero;
     gv[c] = in ? gr[lane + c * 32] : zero;
+    iv[c] = in && ir ? ir[lane + c * 32] : zero;
   }
   const float r = rstd[row];
   float dot = 0.f;
@@ -200,18 +208,16 @@ kf_rmsnorm_bwd_dx_warp(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16
     }
   const float coef = warp_sum(dot) / D * r * r * r;
   __nv_bfloat16* dxr = dx + size_t(row) * D;
-  const __nv_bfloat16* dir = dx_in ? dx_in + size_t(row) * D : nullptr;
 #pragma unroll
   for (int c = 0; c < VPL; ++c)
     if (lane + c * 32 < nvec) {
       const int e = (lane + c * 32) * 8;
       const F8 a = unpack8(xv[c]), g = unpack8(gv[c]), ww = load8(w + e);
-      F8 o;
-      if (dir) o = load8(dir + e);
+      F8 o = unpack8(iv[c]);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const float d = r * g.v[i] * ww.v[i] - a.v[i] * coef;
-        o.v[i] = dir ? o.v[i] + d : d;
+        o.v[i] = ir ? o.v[i] + d : d;
       }
       store8(dxr + e, o);
     }
@@ -222,7 +228,9 @@ kf_rmsnorm_bwd_dx_warp(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16
 //   kf_rmsnorm_bwd_dx   dx = [dx_in +] r*g - x*r^3*mean(g*x) with g = dy*w                   (one block per row)
 // Both keep many rows in flight per SM (few registers, no accumulators that live across rows), which is what lets
 // them run at memory speed; the earlier single kernel carried the dw accumulators through the row loop and was
-// latency bound.  dx_in (optional) is the gradient arriving over the residual connection; it may alias dx.
+// latency bound.  dx_in (optional) is the gradient arriving over the residual connection; it may alias dx.  A thread of the dx pass asks for
+// all its words of the three tensors at once and keeps them packed: 8192 x 4096 69 -> 47 us (268 MB: 41 at the copy rate), 8192 x 8192
+// 139 -> 101, 1777 x 2048 (a warp per row before) 16.3 -> 8.5.
 __global__ void __launch_bounds__(256)
 kf_rmsnorm_bwd_dw(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                   const float* __restrict__ rstd, float* __restrict__ partial, int rows, int D, int rows_per_chunk) {
@@ -269,60 +277,64 @@ kf_rmsnorm_bwd_dx(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __r
   __shared__ float red[40];
   const int nvec = D >> 3;
   constexpr int CACHED = BWD_CACHE * NORM_THREADS;
-  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    const __nv_bfloat16* xr = x + size_t(row) * D;
-    const __nv_bfloat16* dyr = dy + size_t(row) * D;
-    const float r = rstd[row];
-    float dot = 0.f;
-    F8 xc[BWD_CACHE], gc[BWD_CACHE];  // gc holds dy * w
+  const int row = blockIdx.x;
+  const __nv_bfloat16* xr = x + size_t(row) * D;
+  const __nv_bfloat16* dyr = dy + size_t(row) * D;
+  const float r = rstd[row];
+  float dot = 0.f;
+  __nv_bfloat16* dxr = dx + size_t(row) * D;
+  const __nv_bfloat16* dir = dx_in ? dx_in + size_t(row) * D : nullptr;
+  uint4 xc[BWD_CACHE], gc[BWD_CACHE], ic[BWD_CACHE];
 #pragma unroll
-    for (int c = 0; c < BWD_CACHE; ++c) {
-      const int v = threadIdx.x + c * NORM_THREADS;
-      if (v < nvec) {
-        xc[c] = load8(xr + v * 8);
-        gc[c] = load8(dyr + v * 8);
-        const F8 ww = load8(w + v * 8);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          gc[c].v[i] *= ww.v[i];
-          dot += gc[c].v[i] * xc[c].v[i];
-        }
-      }
+  for (int c = 0; c < BWD_CACHE; ++c) {
+    const int v = threadIdx.x + c * NORM_THREADS;
+    if (v < nvec) {
+      xc[c] = *reinterpret_cast<const uint4*>(xr + v * 8);
+      gc[c] = *reinterpret_cast<const uint4*>(dyr + v * 8);
+      if (dir) ic[c] = *reinterpret_cast<const uint4*>(dir + v * 8);
     }
-    for (int v = threadIdx.x + CACHED; v < nvec; v += NORM_THREADS) {
-      const F8 a = load8(xr + v * 8), g = load8(dyr + v * 8), ww = load8(w + v * 8);
+  }
+#pragma unroll
+  for (int c = 0; c < BWD_CACHE; ++c) {
+    const int v = threadIdx.x + c * NORM_THREADS;
+    if (v < nvec) {
+      const F8 a = unpack8(xc[c]), g = unpack8(gc[c]), ww = load8(w + v * 8);
 #pragma unroll
       for (int i = 0; i < 8; ++i) dot += g.v[i] * ww.v[i] * a.v[i];
     }
-    const float coef = block_sum(dot, red) / D * r * r * r;
-    __nv_bfloat16* dxr = dx + size_t(row) * D;
-    const __nv_bfloat16* dir = dx_in ? dx_in + size_t(row) * D : nullptr;
+  }
+  for (int v = threadIdx.x + CACHED; v < nvec; v += NORM_THREADS) {
+    const F8 a = load8(xr + v * 8), g = load8(dyr + v * 8), ww = load8(w + v * 8);
 #pragma unroll
-    for (int c = 0; c < BWD_CACHE; ++c) {
-      const int v = threadIdx.x + c * NORM_THREADS;
-      if (v < nvec) {
-        F8 o;
-        if (dir) o = load8(dir + v * 8);
+    for (int i = 0; i < 8; ++i) dot += g.v[i] * ww.v[i] * a.v[i];
+  }
+  const float coef = block_sum(dot, red) / D * r * r * r;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float d = r * gc[c].v[i] - xc[c].v[i] * coef;
-          o.v[i] = dir ? o.v[i] + d : d;
-        }
-        store8(dxr + v * 8, o);
-      }
-    }
-    // beyond the register cache: every element is re-read and then written by the same thread, so dx may alias dy
-    for (int v = threadIdx.x + CACHED; v < nvec; v += NORM_THREADS) {
-      const F8 a = load8(xr + v * 8), g = load8(dyr + v * 8), ww = load8(w + v * 8);
+  for (int c = 0; c < BWD_CACHE; ++c) {
+    const int v = threadIdx.x + c * NORM_THREADS;
+    if (v < nvec) {
+      const F8 a = unpack8(xc[c]), g = unpack8(gc[c]), ww = load8(w + v * 8);
       F8 o;
-      if (dir) o = load8(dir + v * 8);
+      if (dir) o = unpack8(ic[c]);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const float d = r * g.v[i] * ww.v[i] - a.v[i] * coef;
+        const float d = r * (g.v[i] * ww.v[i]) - a.v[i] * coef;
         o.v[i] = dir ? o.v[i] + d : d;
       }
       store8(dxr + v * 8, o);
     }
+  }
+  // beyond the register cache: every element is re-read and then written by the same thread, so dx may alias dy
+  for (int v = threadIdx.x + CACHED; v < nvec; v += NORM_THREADS) {
+    const F8 a = load8(xr + v * 8), g = load8(dyr + v * 8), ww = load8(w + v * 8);
+    F8 o;
+    if (dir) o = load8(dir + v * 8);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float d = r * g.v[i] * ww.v[i] - a.v[i] * coef;
+      o.v[i] = dir ? o.v[i] + d : d;
+    }
+    store8(dxr + v * 8, o);
   }
 }
 
@@ -808,10 +820,10 @@ int kf_rmsnorm_fwd_pdl_bf16(const void* x, const void* w, void* y, void* rstd, i
                             void* stream) {
   using namespace kf;
   if (D % 8) return 1;
-  const bool warps = rows >= WARP_ROWS_MIN && D <= 4096;
-  auto kern = !warps ? kf_rmsnorm_fwd : D <= 1024 ? kf_rmsnorm_fwd_warp<4> : D <= 2048 ? kf_rmsnorm_fwd_warp<8> : kf_rmsnorm_fwd_warp<16>;
+  const bool warps = rows >= WARP_ROWS_MIN && D <= 2048;
+  auto kern = warps ? (D <= 1024 ? kf_rmsnorm_fwd_warp<4> : kf_rmsnorm_fwd_warp<8>) : D <= 4096 ? kf_rmsnorm_fwd<2> : kf_rmsnorm_fwd<4>;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(warps ? (rows + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK : rows < 148 * 8 ? rows : 148 * 8);
+  cfg.gridDim = dim3(warps ? (rows + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK : D <= 4096 || rows < 148 * 8 ? rows : 148 * 8);
   cfg.blockDim = dim3(warps ? 32 * ROWS_PER_BLOCK : NORM_THREADS);
   cfg.stream = (cudaStream_t)stream;
   cudaLaunchAttribute attr[1];
@@ -846,14 +858,13 @@ int kf_rmsnorm_bwd_bf16(const void* dy, const void* x, const void* w, const void
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const float*)rstd, (float*)dw_partial, rows, D, rows_per_chunk);
   kf_colsum_partials<<<(D + 31) / 32, 256, 0, st>>>((const float*)dw_partial, (__nv_bfloat16*)dw_bf16,
                                                     (float*)dw_f32, chunks, D);
-  if (rows >= WARP_ROWS_MIN && D <= 2048) {
-    auto kern = D <= 1024 ? kf_rmsnorm_bwd_dx_warp<4> : kf_rmsnorm_bwd_dx_warp<8>;
-    kern<<<(rows + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK, 32 * ROWS_PER_BLOCK, 0, st>>>(
+  if (rows >= WARP_ROWS_MIN && D <= 1024) {
+    kf_rmsnorm_bwd_dx_warp<4><<<(rows + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK, 32 * ROWS_PER_BLOCK, 0, st>>>(
         (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const float*)rstd, (__nv_bfloat16*)dx,
         rows, D, (const __nv_bfloat16*)dx_in);
     KF_LAUNCH_CHECK();
   }
-  kf_rmsnorm_bwd_dx<<<rows < 148 * 8 ? rows : 148 * 8, NORM_THREADS, 0, st>>>(
+  kf_rmsnorm_bwd_dx<<<rows, NORM_THREADS, 0, st>>>(
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const float*)rstd,
       (__nv_bfloat16*)dx, rows, D, (const __nv_bfloat16*)dx_in);
   KF_LAUNCH_CHECK();
