@@ -6,9 +6,11 @@
 // a multiple of 32 up to 256, chosen per launch: 1554 tokens are 7 tiles of 224 or 9 of 192.  Which of the two kernels runs,
 // and at which width, is decided by rounds x (512 + width), see tokens_width.  The sums over K have the same order, and so the
 // same bits, either way.
-// What bounds a narrow tile is not the products but the fetch of its 256 rows of W (a ring of eight stages instead of six, which
-// the width leaves room for, gives 1 %).  A block of a 7B model over 1554 tokens, us: o 56 -> 50, gate and up 280 -> 268, down
-// 163 -> 151, q | k | v 74 -> 73; over 300 tokens o 35 -> 26, down 95 -> 74.
+// What bounds a narrow tile is the shared-memory port, through which its MMAs read the 256 rows of W whatever the width: a k-block
+// takes 210 ns at 96 tokens, 245 at 128, 285 at 160, 330 at 192, 390 at 224 and 430 at 256, where the products are the longer part (a
+// ring of eight stages instead of six, which the width leaves room for, gives 1 %).  Against 256 x 256 tiles, both with lane 0 issuing
+// the products, a block of a 7B model over 1554 tokens, us: o 56 -> 50, gate and up 280 -> 268, down 163 -> 151, q | k | v
+// 74 -> 73; over 300 tokens o 35 -> 26, down 95 -> 74.  With an elected thread the block over 1554 tokens takes another tenth less.
 //
 // The epilogue, which turns the accumulators back into rows of tokens, is in tokens_epilogue.cuh.
 //
