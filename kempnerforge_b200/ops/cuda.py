@@ -82,6 +82,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "kf_embedding_fwd_bf16": [vp, vp, vp, ll, i, i, vp],
         "kf_embedding_bwd_bf16": [vp, vp, vp, ll, i, i, vp],
         "kf_ce_fwd_bwd_bf16": [vp, vp, vp, vp, vp, f, i, i, i, vp],
+        "kf_cache_rows_bf16": [vp, ll, vp, vp, i, i, i, ll, vp],
         "kf_ce_grad_bf16": [vp, vp, i, vp, vp, vp, vp, vp, f, i, i, i, vp],
         "kf_gemm_logits_width": [i, i, i, i],
         "kf_gemm_logits_bf16": [vp, vp, vp, vp, i, i, i, i, i, i, i, vp],
@@ -540,6 +541,15 @@ def rmsnorm_bwd(dy, x, w, rstd, residual_grad: torch.Tensor | None = None, out: 
         "kf_rmsnorm_bwd_bf16",
     )
     return dx, dw
+
+
+def cache_rows(kv: torch.Tensor, k: torch.Tensor, v: torch.Tensor, s: int) -> None:
+    """k[:, :s], v[:, :s] = the halves of kv (B * s, 2 * Hkv * hd), rows at any pitch, for contiguous bf16 caches (B, max_len, Hkv, hd)."""
+    b, width = k.shape[0], k.shape[2] * k.shape[3]
+    assert kv.shape == (b * s, 2 * width) and kv.stride(1) == 1 and k.shape == v.shape and s <= k.shape[1]
+    assert kv.dtype == k.dtype == v.dtype == torch.bfloat16 and k.is_contiguous() and v.is_contiguous() and kv.device == k.device == v.device
+    _check(lib().kf_cache_rows_bf16(kv.data_ptr(), kv.stride(0), k.data_ptr(), v.data_ptr(), b, s, width, k.stride(0), _stream()),
+           "kf_cache_rows_bf16")
 
 
 def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, n_rot: int, inverse: bool, out=None):

@@ -178,8 +178,12 @@ def run(block, x, cos, sin, cache):
     qkv = kc.qkv_rope(n1, [wq, wk, wv], cos, sin, s, hd)
     qkv4 = qkv.view(b, s, h + 2 * hkv, hd)
     q, k_new, v_new = qkv4[:, :, :h], qkv4[:, :, h : h + hkv], qkv4[:, :, h + hkv :]
-    if cache is not None:
-        cache.update(k_new, v_new)
+    if cache is not None:   # empty so far, and one that the plan has checked
+        if cache.k.device == cache.v.device == x.device and 2 * t * hkv * hd < 1 << 31:
+            kc.cache_rows(qkv[:, qc:], cache.k, cache.v, s)
+            cache.seq_len = s
+        else:
+            cache.update(k_new, v_new)
     attn, _ = kc.attn_fwd(q, k_new, v_new, True, None, scale)
     h1 = kc.gemm_rows(attn.view(t, qc), [wo], residual=x2)
     if not g2:

@@ -262,3 +262,15 @@ def test_swiglu_over_separate_weights_matches_the_stacked_one(native_lib, m, f, 
     assert native_lib.read_status() == 0 and torch.equal(h, h2) and torch.equal(gu, gu2)
     w = torch.cat([wg, wu])
     _check_dot(gu, x, w)
+
+
+@pytest.mark.parametrize("b,s,hkv,hd,max_len,pad", [(1, 1, 1, 64, 1, 0), (2, 777, 8, 128, 800, 4096), (3, 33, 3, 64, 33, 192), (1, 257, 40, 128, 300, 0)])
+def test_prompt_rows_into_both_caches(native_lib, b, s, hkv, hd, max_len, pad):
+    """Bit for bit the strided copies, and nothing beyond the prompt."""
+    width = hkv * hd
+    rows = torch.randn(b * s, pad + 2 * width, device="cuda").bfloat16()
+    k, v = (torch.full((b, max_len, hkv, hd), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    native_lib.cache_rows(rows[:, pad:], k, v, s)
+    kv = rows[:, pad:].reshape(b, s, 2, hkv, hd)
+    assert torch.equal(k[:, :s], kv[:, :, 0]) and torch.equal(v[:, :s], kv[:, :, 1])
+    assert (k[:, s:] == 7).all() and (v[:, s:] == 7).all()
