@@ -131,11 +131,12 @@ kf_rmsnorm_fwd(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
   }
 }
 
-// Many short rows: one warp per row, the whole row in registers (VPL 16-byte vectors per lane, all loads issued before the first
-// use), reduction by shuffles only; a block per row leaves threads of it without work.  us, warp / block per row, caches cold: 8192 x 768
-// 7.4 / 19.0, 4096 x 1024 5.7 / 10.9, 4096 x 2048 10.9 / 12.5, 1777 x 2048 6.9 / 7.0, but 8192 x 4096 31.9 / 28.7 (20.5 at the copy
-// rate) and 1554 x 4096 11.9 / 8.2: sixteen vectors per lane leave too few warps on an SM.  With few rows (decoding) a row spread over a
-// block finishes sooner.
+// Many rows: one warp per row, the whole row in registers (VPL 16-byte vectors per lane, all loads issued before the first
+// use), reduction by shuffles only; a block per row leaves threads of short rows without work.  us, warp / block per row, caches cold:
+// 8192 x 768 7.4 / 19.0, 4096 x 1024 5.7 / 10.9, 4096 x 2048 10.9 / 12.5, 1777 x 2048 6.9 / 7.0.  With few rows (decoding) a row
+// spread over a block finishes sooner.  So it does at 2056 to 4096 columns, 8192 x 4096 31.9 / 28.7 (20.5 at the copy rate) and 1554 x 4096
+// 11.9 / 8.2 (sixteen vectors per lane leave few warps on an SM), but a block adds the squares in another order, and what five
+// roundings to bf16 make of the last bits of rstd moves a block's output by 0.0035 of its norm: the order is kept.
 constexpr int ROWS_PER_BLOCK = 4;
 constexpr int WARP_ROWS_MIN = 1024;  // rows from which warps per row fill the machine (148 SMs x 8 rows in flight)
 
@@ -833,10 +834,11 @@ int kf_rmsnorm_fwd_pdl_bf16(const void* x, const void* w, void* y, void* rstd, i
                             void* stream) {
   using namespace kf;
   if (D % 8) return 1;
-  const bool warps = rows >= WARP_ROWS_MIN && D <= 2048;
-  auto kern = warps ? (D <= 1024 ? kf_rmsnorm_fwd_warp<4> : kf_rmsnorm_fwd_warp<8>) : D <= 4096 ? kf_rmsnorm_fwd<2> : kf_rmsnorm_fwd<4>;
+  const bool warps = rows >= WARP_ROWS_MIN && D <= 4096;
+  auto kern = warps ? (D <= 1024 ? kf_rmsnorm_fwd_warp<4> : D <= 2048 ? kf_rmsnorm_fwd_warp<8> : kf_rmsnorm_fwd_warp<16>)
+                    : D <= 4096 ? kf_rmsnorm_fwd<2> : kf_rmsnorm_fwd<4>;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(warps ? (rows + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK : D <= 4096 || rows < 148 * 8 ? rows : 148 * 8);
+  cfg.gridDim = dim3(warps ? (rows + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK : rows < 148 * 8 ? rows : 148 * 8);
   cfg.blockDim = dim3(warps ? 32 * ROWS_PER_BLOCK : NORM_THREADS);
   cfg.stream = (cudaStream_t)stream;
   cudaLaunchAttribute attr[1];

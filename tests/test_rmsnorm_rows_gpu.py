@@ -30,3 +30,21 @@ def test_against_double(native_lib, rows, d):
         err = 2.0**-17 * (first.abs() + (xd * r**3).abs() * (g * xd).abs().mean(-1, keepdim=True) + add.abs())
         total = first - second + add
         assert ((dx.double() - total).abs() <= total.abs() * 2.0**-8 + err).all()
+
+
+@pytest.mark.parametrize("rows,d", [(1024, 256), (1024, 1024), (1025, 2048), (1024, 4096), (1554, 4096)])
+def test_the_squares_of_many_rows_are_added_in_one_order(native_lib, rows, d):
+    """A warp per row, lane l the 16-byte words l, l + 32, ..., then the lanes in pairs 16, 8, 4, 2, 1 apart: a step through several
+    blocks turns other last bits of rstd into outputs that differ like independent roundings.  (Powers of two: the mean is exact.)"""
+    torch.manual_seed(rows + d)
+    x = torch.randn(rows, d, device=DEV).bfloat16()
+    _, rstd = native_lib.rmsnorm_fwd(x, torch.ones(d, device=DEV).bfloat16(), 1e-5)
+    words = x.float().view(rows, -1, 32, 8)
+    ss = torch.zeros(rows, 32, device=DEV)
+    for c in range(words.shape[1]):
+        for i in range(8):
+            ss = ss + words[:, c, :, i] ** 2   # the square of a bf16 value is exact in fp32
+    lane = torch.arange(32, device=DEV)
+    for o in (16, 8, 4, 2, 1):
+        ss = ss + ss[:, lane ^ o]
+    assert torch.equal(rstd, (ss[:, 0] / d + 1e-5).rsqrt())
