@@ -664,6 +664,10 @@ def scale_(x: torch.Tensor, factor: torch.Tensor) -> torch.Tensor:
 _DT = {torch.bfloat16: 0, torch.float32: 1}
 
 
+# A kernel writes through an address, which autograd and everything kept by a tensor's version (fp8 copies of weights) do not see
+_wrote = torch.autograd.graph.increment_version
+
+
 def adamw_flat(p, g, m, v, n_decay: int, lr: float, beta1: float, beta2: float, eps: float, wd: float,
                step: int, grad_scale: torch.Tensor | None = None, skip: torch.Tensor | None = None) -> None:
     """One fused AdamW update over flat 1-D buffers; elements [0, n_decay) are weight-decayed."""
@@ -678,6 +682,7 @@ def adamw_flat(p, g, m, v, n_decay: int, lr: float, beta1: float, beta2: float, 
         ),
         "kf_adamw_flat",
     )
+    _wrote(p)
 
 
 def sumsq(x: torch.Tensor, out: torch.Tensor, accumulate: bool = False) -> torch.Tensor:
@@ -962,6 +967,7 @@ def lion_step(p, g, m, lr: float, b1: float, b2: float, wd: float) -> bool:
     if getattr(lib(), "kf_lion", None) is None or not _same_flat(p, g, m):
         return False
     _check(lib().kf_lion(p.data_ptr(), g.data_ptr(), m.data_ptr(), p.numel(), _DT[p.dtype], lr, b1, b2, wd, _stream()), "kf_lion")
+    _wrote(p)
     return True
 
 
@@ -971,6 +977,7 @@ def sf_adamw_step(y, g, z, v, x, lr, b1, b2, eps, wd, bc2, ck, first: bool) -> b
         return False
     _check(lib().kf_sf_adamw(y.data_ptr(), g.data_ptr(), z.data_ptr(), v.data_ptr(), x.data_ptr(), y.numel(), _DT[y.dtype],
                              lr, b1, b2, eps, wd, bc2, ck, int(first), _stream()), "kf_sf_adamw")
+    _wrote(y)
     return True
 
 

@@ -20,6 +20,7 @@ from __future__ import annotations
 
 import torch
 from torch import nn
+from torch.multiprocessing.reductions import StorageWeakRef
 
 from kempnerforge_b200.metrics.logger import get_logger
 
@@ -95,21 +96,36 @@ def scaled_mm(a8, b8, sa, sb, a_e5m2=False, b_e5m2=False, out=None, accumulate=F
 def quantized_weight(weights, want_t: bool):
     """(scale, row-major fp8, transposed fp8 or None) of the weights stacked along the output dimension.
 
-    The quantised copies are kept on the first weight tensor and reused until a weight is modified in place (the
-    tensors' version counters change on every optimizer step), so the micro-batches, the recomputation and the
-    backward pass of one step quantise each weight once instead of once per use."""
+    The quantised copies are kept on the first weight tensor and reused until a weight is written, so the
+    micro-batches, the recomputation and the backward pass of one step quantise each weight once instead of once per use.
+    Every write has to move a version counter (:func:`_state`): tensor operations do, and so do this package's optimizers and
+    collectives, which write through raw pointers.  A program that writes a weight through ``.data`` or a pointer of its own,
+    or replays a captured optimizer step, calls ``torch.autograd.graph.increment_version(weight)`` after it.
+    Copies are reused on the stream that made them only, and neither taken into a captured graph nor out of it: a replay
+    reads the weights as they are then."""
     from kempnerforge_b200.ops import functional as F
 
-    versions = tuple(w._version for w in weights) + tuple(w.data_ptr() for w in weights)
+    stacked = lambda: F._stack_weight_rows(weights).detach()  # noqa: E731
+    if weights[0].is_cuda and torch.cuda.is_current_stream_capturing():
+        return quantize(stacked(), want_t=want_t)
+    state = tuple(map(_state, weights)), torch.cuda.current_stream(weights[0].device).cuda_stream if weights[0].is_cuda else None
     holder = weights[0]
     cached = getattr(holder, "_kf_fp8_cache", None)
-    if cached is None or cached[0] != versions:
-        sw, w8, _ = quantize(F._stack_weight_rows(weights).detach())
-        cached = [versions, sw, w8, None]
+    if cached is None or cached[0] != state or any(ref.expired() for ref in cached[4]):
+        sw, w8, _ = quantize(stacked())
+        # while a storage is referred to, no other one gets its identity
+        cached = [state, sw, w8, None, [StorageWeakRef(w.untyped_storage()) for w in weights]]
         holder._kf_fp8_cache = cached
     if want_t and cached[3] is None:
-        cached[3] = quantize(F._stack_weight_rows(weights).detach(), want_row=False, want_t=True, scale=cached[1])[2]
+        cached[3] = quantize(stacked(), want_row=False, want_t=True, scale=cached[1])[2]
     return cached[1], cached[2], cached[3]
+
+
+def _state(w: torch.Tensor) -> tuple:
+    """Changes whenever a weight's values may have: its version, the memory it lies in, and the version of the flat buffer that it is
+    a view of.  (Binding a parameter to the buffer leaves it a counter of its own, which a write of the buffer does not move.)"""
+    flat = getattr(w, "_kf_flat", None)
+    return w._version, w.data_ptr(), w.untyped_storage()._cdata, None if flat is None else flat.values_version
 
 
 class _Fp8LinearFn(torch.autograd.Function):
@@ -121,7 +137,7 @@ class _Fp8LinearFn(torch.autograd.Function):
         sx, x8, _ = quantize(x2)
         sw, w8, _ = quantized_weight(weights, want_t=False)
         y = scaled_mm(x8, w8, sx, sw)
-        ctx.save_for_backward(x2, sx, sw, *weights)
+        ctx.save_for_backward(x2, sx, *weights)
         ctx.x_shape = x.shape
         return y.view(*x.shape[:-1], w8.shape[0])
 
@@ -129,7 +145,7 @@ class _Fp8LinearFn(torch.autograd.Function):
     def backward(ctx, dy):
         from kempnerforge_b200.ops import functional as F
 
-        x2, sx, sw, *weights = ctx.saved_tensors
+        x2, sx, *weights = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
@@ -138,7 +154,7 @@ class _Fp8LinearFn(torch.autograd.Function):
         sg, g8, g8t = quantize(dy2, e5m2=True, want_row=need_dx, want_t=need_dw)
         dx = None
         if need_dx:
-            _, _, w8t = quantized_weight(weights, want_t=True)                      # (K, N)
+            sw, _, w8t = quantized_weight(weights, want_t=True)                     # (K, N)
             dx = scaled_mm(g8, w8t, sg, sw, a_e5m2=True).view(ctx.x_shape)
         wgrads = [None] * len(weights)
         if need_dw:
@@ -168,7 +184,7 @@ class _Fp8SwiGLUFn(torch.autograd.Function):
         sh, h8, h8t = quantize(h, scale=h_max, want_t=recording and ctx.needs_input_grad[3])
         sd, d8, _ = quantized_weight((wd,), want_t=False)
         y = scaled_mm(h8, d8, sh, sd)
-        ctx.save_for_backward(x2, sx, s_gu, gu, h8t, sh, sd, wg, wu, wd)
+        ctx.save_for_backward(x2, sx, gu, h8t, sh, wg, wu, wd)
         ctx.x_shape = x.shape
         return y.view(*x.shape[:-1], d8.shape[0])
 
@@ -177,7 +193,7 @@ class _Fp8SwiGLUFn(torch.autograd.Function):
         from kempnerforge_b200.ops import cuda as cu
         from kempnerforge_b200.ops import functional as F
 
-        x2, sx, s_gu, gu, h8t, sh, sd, wg, wu, wd = ctx.saved_tensors
+        x2, sx, gu, h8t, sh, wg, wu, wd = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
@@ -186,7 +202,7 @@ class _Fp8SwiGLUFn(torch.autograd.Function):
         sg, g8, g8t = quantize(dy2, e5m2=True, want_row=need_h, want_t=need_d)
         dx = g_wg = g_wu = g_wd = None
         if need_h:
-            _, _, d8t = quantized_weight((wd,), want_t=True)
+            sd, _, d8t = quantized_weight((wd,), want_t=True)
             dgu, dgu_max = cu.gemm_fp8_swiglu_bwd(g8, d8t, sg, sd, gu)
         if need_d:
             (g_wd,) = F._deposit_stacked_weight_grads(
@@ -195,7 +211,7 @@ class _Fp8SwiGLUFn(torch.autograd.Function):
             need_w = need_g or need_u
             s_dgu, q8, q8t = quantize(dgu, e5m2=True, want_row=need_x, want_t=need_w, scale=dgu_max)
             if need_x:
-                _, _, w8t = quantized_weight((wg, wu), want_t=True)
+                s_gu, _, w8t = quantized_weight((wg, wu), want_t=True)
                 dx = scaled_mm(q8, w8t, s_dgu, s_gu, a_e5m2=True).view(ctx.x_shape)
             if need_w:
                 _, _, x8t = quantize(x2, want_row=False, want_t=True, scale=sx)

@@ -92,6 +92,7 @@ class DataParallelEngine:
             if g.local:
                 continue
             dist.broadcast(g.param, src=root, group=self.pg)
+            g.values_written()   # which a broadcast does not do
 
     # ------------------------------------------------------------------ overlap of communication with compute
     def _install_overlap_hooks(self) -> None:

@@ -100,7 +100,8 @@ class FlatParamGroup:
         if self.sharded:
             self._init_sharded(alloc, allocator is not None)
             return
-        self.param = alloc(self.numel, self.dtype, self.device)
+        # .data: a version counter of its own, which writes of other buffers in the same arena do not move
+        self.param = alloc(self.numel, self.dtype, self.device).data
         self.grad = alloc(self.numel, self.dtype, self.device)
         # symmetric-memory descriptors of the two buffers (None with an ordinary allocator)
         self.param_symm = self.grad_symm = None
@@ -128,7 +129,7 @@ class FlatParamGroup:
         # padded length of every parameter = distance to the next offset
         ends = self.offsets[1:] + [self.numel]
         self.padded = [e - o for o, e in zip(self.offsets, ends)]
-        self.shard = alloc(self.shard_numel, self.dtype, self.device)          # this rank's piece of every parameter
+        self.shard = alloc(self.shard_numel, self.dtype, self.device).data     # this rank's piece of every parameter
         self.grad_shard = torch.zeros(self.shard_numel, dtype=self.dtype, device=self.device)
         self.grad_shard_live = False
         self.shard_symm = None
@@ -174,6 +175,16 @@ class FlatParamGroup:
             p.data = self.param[o : o + p.numel()].view(p.shape)
             if self.grad is not None:
                 p._kf_grad = self.grad[o : o + p.numel()].view(p.shape)
+
+    # ------------------------------------------------------------------ changes
+    @property
+    def values_version(self) -> int:
+        """Moves with every write of the parameters' buffer (of this rank's shard, which every rank updates in the same step)."""
+        return (self.shard if self.sharded else self.param)._version
+
+    def values_written(self) -> None:
+        """To be called by whatever wrote the buffer other than through tensor operations on it."""
+        torch.autograd.graph.increment_version(self.shard if self.sharded else self.param)
 
     # ------------------------------------------------------------------ shards
     @property

@@ -98,6 +98,7 @@ class ShardedDataParallelEngine(DataParallelEngine):
             if g.local or g.sharded:
                 continue
             dist.broadcast(g.param, src=root, group=self.pg)
+            g.values_written()   # which a broadcast does not do
 
     def _make_pre_hook(self, idxs):
         def hook(module, args):

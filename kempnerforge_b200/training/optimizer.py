@@ -86,6 +86,7 @@ class FusedAdamW(torch.optim.AdamW):
                     lo, hi = fg.shard_range
                     kcuda.symm_adamw_bcast(fg.param_symm, g, m, v, lo, hi - lo, fg.n_decay, lr, b1, b2, eps, wd,
                                            fg.step_count, self.grad_scale, self.skip_flag)
+                    fg.values_written()
                 else:  # one GPU: the same ordering, without publication
                     kcuda.adamw_flat(p, g, m, v, fg.n_decay_local, lr, b1, b2, eps, wd, fg.step_count,
                                      self.grad_scale, self.skip_flag)
@@ -105,6 +106,7 @@ class FusedAdamW(torch.optim.AdamW):
                 lo, hi = fg.shard_range
                 kcuda.symm_adamw_bcast(fg.param_symm, g, m, v, lo, hi - lo, fg.n_decay, lr, b1, b2, eps, wd,
                                        fg.step_count, self.grad_scale, self.skip_flag)
+                fg.values_written()
             elif p.is_cuda:
                 kcuda.adamw_flat(p, g, m, v, fg.n_decay_local, lr, b1, b2, eps, wd, fg.step_count,
                                  self.grad_scale, self.skip_flag)
@@ -400,6 +402,7 @@ class Muon(torch.optim.Optimizer):
                     # the owner's new values replace everybody's copy; the transfer overlaps the next matrices' math
                     src = dist.get_global_rank(dp, owner)
                     pending.append(dist.broadcast(pl if pl.is_contiguous() else pl.data, src=src, group=dp, async_op=True))
+                    torch.autograd.graph.increment_version(pl)   # which a broadcast does not do
         for work in pending:
             work.wait()
         if self._adam is not None:

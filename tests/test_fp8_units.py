@@ -114,3 +114,95 @@ def test_fp8_model_trains_on_cpu():
         loss.backward()
         opt.step()
     assert float(loss) < 0.7 * first
+
+
+def _bytes(weights):
+    sw, w8, w8t = fp8.quantized_weight(weights, want_t=True)
+    return sw, w8.view(torch.uint8), w8t.view(torch.uint8)
+
+
+def _fresh(weights):
+    sw, w8, w8t = fp8.quantize(torch.cat([w.detach() for w in weights]), want_t=True)
+    return sw, w8.view(torch.uint8), w8t.view(torch.uint8)
+
+
+def _flat_pair(world=1):
+    from kempnerforge_b200.parallel.flat import FlatParamGroup
+
+    net = nn.Sequential(_tagged_linear(32, 64), _tagged_linear(16, 64))
+    return net, [net[0].weight, net[1].weight], FlatParamGroup("unit", net.named_parameters(), world=world)
+
+
+def _adamw(net, fg):
+    from kempnerforge_b200.training.optimizer import FusedAdamW
+
+    opt = FusedAdamW(net.parameters(), lr=0.1, fused=False)
+    opt.attach_flat_groups([fg])
+    fg.grad.normal_()
+    opt.step()
+
+
+def _per_tensor(cls):
+    def step(net, fg):
+        import kempnerforge_b200.training.optimizer as o
+
+        for p in net.parameters():
+            p.grad = torch.randn_like(p)
+        getattr(o, cls)(net.parameters(), lr=0.1).step()
+
+    return step
+
+
+@pytest.mark.parametrize("write", [
+    lambda net, fg: fg.param.mul_(-3), lambda net, fg: fg.param[: fg.numel // 2].add_(1), _adamw, _per_tensor("Lion"), _per_tensor("ScheduleFreeAdamW"),
+    lambda net, fg: fg.values_written() or fg.param.data.mul_(-3),      # a kernel, a collective
+    lambda net, fg: torch.nn.Module.load_state_dict(net, {k: v * -3 for k, v in net.state_dict().items()}),
+], ids=["buffer", "part of it", "adamw", "lion", "schedule free", "announced", "checkpoint"])
+def test_copies_of_weights_in_a_flat_buffer_follow_every_write(write):
+    net, weights, fg = _flat_pair()
+    before = [t.clone() for t in _bytes(weights)]
+    assert all(torch.equal(a, b) for a, b in zip(_bytes(weights), before))
+    with torch.no_grad():
+        write(net, fg)
+    got, want = _bytes(weights), _fresh(weights)
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) and not torch.equal(got[1], before[1])
+
+
+def test_writes_of_other_units_leave_the_copies_alone():
+    arena = torch.zeros(1 << 14, dtype=torch.bfloat16)
+    used = [0]
+
+    def alloc(n, dt, dev):
+        used[0] += n
+        return arena[used[0] - n : used[0]]
+
+    from kempnerforge_b200.parallel.flat import FlatParamGroup
+
+    net = nn.Sequential(_tagged_linear(32, 64), _tagged_linear(16, 64))
+    a, b = (FlatParamGroup(str(i), net[i].named_parameters(), allocator=alloc) for i in range(2))
+    first = _bytes([net[0].weight])
+    b.param.mul_(2), a.grad.add_(1), b.grad.add_(1)
+    assert all(x.data_ptr() == y.data_ptr() for x, y in zip(first, _bytes([net[0].weight])))
+
+
+def test_copies_do_not_outlive_the_memory_that_the_weights_lay_in():
+    """A parameter that goes to another memory and back may find its old address, with other values and the same version."""
+    w = _tagged_linear().weight
+    _bytes([w])
+    refs = w._kf_fp8_cache[4]
+    w.data = w.data * -3
+    assert all(r.expired() for r in refs) and all(torch.equal(a, b) for a, b in zip(_bytes([w]), _fresh([w])))
+    w._kf_fp8_cache[1:] = None, None, None, refs    # the state of now, made of a memory that is gone
+    assert all(torch.equal(a, b) for a, b in zip(_bytes([w]), _fresh([w])))
+
+
+def test_the_input_gradient_takes_scale_and_copy_of_the_same_weights():
+    """Weights in a flat buffer that change between the passes (a delayed backward): the present ones count, as with bf16."""
+    net, weights, fg = _flat_pair()
+    x = torch.randn(16, 64, dtype=torch.bfloat16, requires_grad=True)
+    y = F.linear(x, weights[0])
+    fg.param.mul_(-3)
+    g = torch.randn_like(y)
+    y.backward(g)
+    want = g.float() @ weights[0].detach().float()
+    assert (x.grad.float() - want).norm() < 0.15 * want.norm()   # e5m2 gradients, e4m3 weights
