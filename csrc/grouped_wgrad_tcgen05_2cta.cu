@@ -12,8 +12,8 @@
 //   full 64-row blocks   as in gemm_tcgen05_2cta.cu: both CTAs' TMA bytes are counted on the leader's full[s]
 //   the tail block       (at most one per tile) each CTA's loads complete on its own tail[s]; warp 6 of each CTA waits
 //                        for it, zeroes the foreign rows of its own stage up to the next multiple of 16 (only those
-//                        k-steps are issued), fences them towards the async proxy and arrives on the leader's
-//                        ready[s]; the issuing thread waits for both arrivals before the MMAs.
+//                        k-steps are issued), fences them towards the async proxy and arrives (release) on the leader's
+//                        ready[s]; the issuing thread waits for both arrivals (cluster-scope acquire) before the MMAs.
 //                        The ring runs ahead of the MMAs, so the rows are usually clear before their turn; zeroing all
 //                        64 rows inside the issuing warp held up every tile by about as long as a k-block (64 experts of
 //                        2048 x 1408 over 10 662 rows: 484 -> 397 us for three gradients; 8 of 2048 x 7168: 464 -> 414).
@@ -218,7 +218,7 @@ kf_grouped_wgrad_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const _
           asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(chunk + r * 128), "r"(0u) : "memory");
         fence_async_smem();
         __syncwarp();
-        if (lane == 0) arrive_on_cta(ready_bar(s), 0);  // this CTA's half of the stage is in place
+        if (lane == 0) arrive_release_on_cta(ready_bar(s), 0);  // this CTA's half of the stage is in place
       }
       it += k_blocks;
     }

@@ -52,16 +52,24 @@ __device__ __forceinline__ void commit_pair(uint32_t bar) {
       "h"((uint16_t)0x3)
       : "memory");
 }
-// Arrival on a barrier of either CTA of the pair, for what the tensor cores alone depend on: an epilogue warp hands an accumulator back
-// (its values are in registers: tcgen05.wait::ld and the fence before), or a warp has changed its own CTA's operands in shared
-// memory (fence.proxy.async before; each SM's tensor core reads its own).  No other thread reads this thread's memory after it, and
-// a release at cluster scope waits for every store the warp has in flight first: 3000 clocks per tile of the grouped weight
-// gradient, in the epilogue and again for the cleared rows.
+// Arrival on a barrier of either CTA of the pair by an epilogue warp that hands an accumulator back: its values are in registers
+// (tcgen05.wait::ld and the fence before), and no thread reads memory of this one after it.  It releases at CTA scope; at cluster scope
+// it waited for every store the warp has in flight first, 3000 clocks per tile of the grouped weight gradient.
 __device__ __forceinline__ void arrive_on_cta(uint32_t bar, uint32_t cta) {
   asm volatile(
       "{\n\t.reg .b32 ra;\n\t"
       "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
       "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar),
+      "r"(cta)
+      : "memory");
+}
+// Arrival by a thread whose warp has written shared memory that the other CTA's matrix instructions are issued to read
+// (fence.proxy.async before): releases at cluster scope, for the issuing thread's wait that acquires there (mbar_wait_cluster).
+__device__ __forceinline__ void arrive_release_on_cta(uint32_t bar, uint32_t cta) {
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\t"
+      "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
+      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar),
       "r"(cta)
       : "memory");
 }
