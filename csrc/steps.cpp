@@ -86,10 +86,10 @@ const at::Tensor* tensor(PyObject* o) {
   return t.defined() && t.has_storage() && !t.unsafeGetTensorImpl()->is_python_dispatch() && !t.is_sparse() ? &t : nullptr;
 }
 
-long long address(const at::Tensor& t) {
-  const auto p = reinterpret_cast<long long>(t.const_data_ptr());
-  return p & 15 ? 0 : p;
-}
+long long aligned(const void* p) { return reinterpret_cast<uintptr_t>(p) & 15 ? 0 : reinterpret_cast<long long>(p); }
+long long address(const at::Tensor& t) { return aligned(t.const_data_ptr()); }
+// Of what the kernels write: memory that a lazy clone shares with its original is its own after this.
+long long target(const at::Tensor& t) { return aligned(t.mutable_data_ptr()); }
 
 // Address of the dense bf16 (rows, cols) weight of self.<sub>, 0 for anything else; rows < 0: any number, reported in *rows_out.
 long long matrix(const Attributes& m, PyObject* sub, long long rows, long long cols, long long* rows_out = nullptr) {
@@ -171,10 +171,11 @@ bool plan(PyObject* block, PyObject* cache, long long b, long long d, const at::
       !v->is_contiguous() || !k->is_cuda() || !v->is_cuda())
     return false;
   p.past = PyLong_AsLongLong(past);
-  p.kc = address(*k);
-  p.vc = address(*v);
+  if (p.past < 0 || p.past + 1 > k->size(1)) return false;
+  p.kc = target(*k);
+  p.vc = target(*v);
   p.step = k->stride(0);
-  return p.past >= 0 && p.past + 1 <= k->size(1) && p.kc && p.vc;
+  return p.kc && p.vc;
 }
 
 // decode(blocks, caches, x, cos, sin, foreign, stream, sms): blocks and caches are lists.  (y, launches), or None when some block is not
@@ -219,7 +220,7 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     // before it are complete.  n (D) | q (H hd) | hidden (F) | h1 (D) | attention (H hd) | outputs of even and odd blocks | rstd, lse
     const at::Tensor scratch = at::empty({b * cols + 2 * b + 2 * heads + 2 * b * d}, x->options());
     at::Tensor y = at::empty_like(*x);
-    const auto base = reinterpret_cast<long long>(scratch.data_ptr());
+    const auto base = reinterpret_cast<long long>(scratch.mutable_data_ptr());
     const long long hand[2] = {base + 2 * b * cols, base + 2 * b * (cols + d)}, rstd = base + 2 * b * (cols + 2 * d);
     std::vector<long long> ints(static_cast<size_t>(count) * INTS);
     std::vector<double> reals(static_cast<size_t>(count) * REALS);
@@ -227,7 +228,7 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     for (Py_ssize_t i = 0; i < count; ++i) {
       const Plan& p = plans[static_cast<size_t>(i)];
       const long long h1 = base + 2 * b * (d + p.h * p.hd + p.f);
-      const long long dst = i == count - 1 ? reinterpret_cast<long long>(y.data_ptr()) : hand[i & 1];
+      const long long dst = i == count - 1 ? reinterpret_cast<long long>(y.mutable_data_ptr()) : hand[i & 1];
       const long long row[INTS] = {src, p.weights[0], p.weights[1], p.weights[2], p.weights[3], p.weights[4], p.weights[5], p.weights[6],
                                    p.weights[7], p.weights[8], p.kc, p.vc, base, rstd, h1, dst, cosp, sinp, b, d, p.h, p.hkv, p.hd, p.f,
                                    p.past, p.step, sms, 7, p.hd == 64, h1 + 2 * b * d, rstd + 4 * b};

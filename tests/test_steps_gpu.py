@@ -132,3 +132,20 @@ def test_inputs_that_the_native_step_refuses(native_lib):
         with pytest.raises(TypeError):
             native_lib._steps.decode(1, 2)
     assert native_lib.read_status() == 0
+
+
+@pytest.mark.parametrize("batch", [1, 3])
+def test_a_cache_that_shares_its_memory_with_another_is_written_apart(native_lib, batch):
+    """A lazy clone (of a beam that forks) lies in its original's memory until either is written."""
+    block, cache, x, cos, sin = _block(batch=batch, heads=2)
+    kept = type(cache)(batch, 96, 2, 128, torch.bfloat16, torch.device(DEV))
+    kept.k, kept.v, kept.seq_len = cache.k, cache.v, cache.seq_len
+    k, v = cache.k.clone(), cache.v.clone()
+    cache.k, cache.v = torch._lazy_clone(kept.k), torch._lazy_clone(kept.v)
+    with torch.no_grad():
+        assert native_lib.blocks_decode([block], [cache], x, cos, sin, _none) is not None
+    assert torch.equal(kept.k, k) and torch.equal(kept.v, v)
+    rest = torch.arange(96, device=DEV) != 40
+    for new, old in ((cache.k, k), (cache.v, v)):
+        assert not torch.equal(new[:, 40], old[:, 40]) and torch.equal(new[:, rest], old[:, rest])
+    assert cache.seq_len == 41 and native_lib.read_status() == 0
