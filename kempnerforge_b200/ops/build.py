@@ -5,7 +5,8 @@ headers, so each translation unit compiles in seconds and the result is one
 shared object, ``kempnerforge_b200/lib/libkfb200.so``, loaded through ctypes.
 
 One host file reads Python modules and tensors (``csrc/steps.cpp``) and is built
-against the headers of Python and PyTorch into a CPython module beside it.
+against the headers of Python and PyTorch into a CPython module beside it.  It serves
+only the versions that it was built for, so its name holds them; the library serves any.
 """
 
 from __future__ import annotations
@@ -14,7 +15,6 @@ import hashlib
 import os
 import shutil
 import subprocess
-import sys
 import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
@@ -26,7 +26,7 @@ REPO_ROOT = PKG_ROOT.parent
 CSRC = REPO_ROOT / "csrc"
 LIB_DIR = PKG_ROOT / "lib"
 LIB_PATH = LIB_DIR / "libkfb200.so"
-STEPS_PATH = LIB_DIR / "kf_steps.so"
+STEPS_PATH = LIB_DIR / f"kf_steps.{sysconfig.get_config_var('SOABI')}.torch-{torch.__version__}.so"
 
 NVCC_FLAGS = [
     "-gencode",
@@ -59,7 +59,6 @@ def _fingerprint() -> str:
         h.update(f.name.encode())
         h.update(f.read_bytes())
     h.update(" ".join(NVCC_FLAGS).encode())
-    h.update(f"{sys.version} {torch.__version__}".encode())
     return h.hexdigest()
 
 

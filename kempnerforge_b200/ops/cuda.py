@@ -18,6 +18,7 @@ from typing import NamedTuple
 
 import torch
 
+from kempnerforge_b200.metrics.logger import get_logger
 from kempnerforge_b200.ops.build import LIB_PATH, STEPS_PATH
 
 _lib = None
@@ -477,14 +478,18 @@ def block_decode(y: torch.Tensor, attn_ptrs, mlp_ptrs, cache_ptrs, table_ptrs, d
     _check(fn(ip, rp, _stream()), "kf_block_decode_bf16", 5 + 2 * norms if mlp_ptrs else 3 + norms)
 
 
-_steps = None
+_steps = None   # the module once it is loaded, False when there is none for this Python and PyTorch
 
 
 def _load_steps():
-    """The CPython module of ``csrc/steps.cpp``, told the classes it looks for and the native entry."""
+    """The CPython module of ``csrc/steps.cpp``, told the classes it looks for and the native entry.  False when there is none for this
+    Python and PyTorch (its name holds both): the rules in Python (``fused_infer._plan``) then serve every call, with the same kernels."""
     global _steps
     if not STEPS_PATH.exists():
-        raise NativeKernelError(f"native module {STEPS_PATH} is missing; run `python -m kempnerforge_b200.ops.build`")
+        get_logger(__name__).warning("%s is missing: generation steps are checked in Python (run `python -m kempnerforge_b200.ops.build`)",
+                                     STEPS_PATH)
+        _steps = False
+        return _steps
     from kempnerforge_b200.models.attention import Attention, KVCache
     from kempnerforge_b200.models.mlp import SwiGLUMLP
     from kempnerforge_b200.models.norm import RMSNorm
@@ -503,7 +508,8 @@ def blocks_decode(blocks: list, caches: list, x: torch.Tensor, cos: torch.Tensor
     checks them as well (``csrc/steps.cpp``): the last block's output (B, 1, D), or None when one of them is not plainly
     covered.  Without ``foreign`` the call stands for the blocks themselves, so hooks on them count; a block that calls it
     gives its ``foreign(q (B, H hd), H, hd, position)`` -> (B, H hd) for the attention of heads of 64 over several sequences."""
-    r = (_steps or _load_steps()).decode(blocks, caches, x, cos, sin, foreign, _stream(), sm_count())
+    steps = _load_steps() if _steps is None else _steps
+    r = steps.decode(blocks, caches, x, cos, sin, foreign, _stream(), sm_count()) if steps else None
     if r is None:
         return None
     if type(r) is int:

@@ -149,3 +149,16 @@ def test_a_cache_that_shares_its_memory_with_another_is_written_apart(native_lib
     for new, old in ((cache.k, k), (cache.v, v)):
         assert not torch.equal(new[:, 40], old[:, 40]) and torch.equal(new[:, rest], old[:, rest])
     assert cache.seq_len == 41 and native_lib.read_status() == 0
+
+
+@pytest.mark.parametrize("batch,heads", [(1, 4), (3, 2), (3, 4)])
+def test_a_step_without_the_module_has_the_same_bits(native_lib, monkeypatch, batch, heads):
+    block, cache, x, cos, sin = _block(heads=heads, batch=batch)
+    k, v = cache.k.clone(), cache.v.clone()
+    with torch.no_grad():
+        got = block(x, cos, sin, kv_cache=cache), cache.k.clone(), cache.v.clone()
+        cache.k.copy_(k), cache.v.copy_(v)
+        cache.seq_len = 40
+        monkeypatch.setattr(native_lib, "_steps", False)
+        want = block(x, cos, sin, kv_cache=cache), cache.k, cache.v
+    assert cache.seq_len == 41 and all(torch.equal(a, b) for a, b in zip(got, want)) and native_lib.read_status() == 0
