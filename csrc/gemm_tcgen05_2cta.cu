@@ -190,6 +190,9 @@ __device__ __forceinline__ void row_stats(const Rows32& own, int valid, float& l
   largest = m;
 }
 
+// Whether the kernel's tiles are as wide as its launch says; the launch's tensor map of B has boxes of half that width.
+__host__ __device__ constexpr bool takes_width(int swiglu, bool b_mn, bool gather) { return (swiglu == 0 || swiglu == 6) && !b_mn && !gather; }
+
 template <bool A_MN, bool B_MN, typename OutT, int SWIGLU = 0, bool GATHER = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GATHER ? THREADS_GATHER : THREADS, 1)
 kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ WeightSegs ws,
@@ -214,7 +217,7 @@ kf_gemm_bf16_tcgen05_2cta(const __grid_constant__ CUtensorMap map_a, const __gri
   const int pair = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
   const int m_blocks = (M + TILE_M - 1) / TILE_M;
-  const int tile_n = SWIGLU == 0 && !B_MN && !GATHER ? tile_n_arg : TILE_N;
+  const int tile_n = takes_width(SWIGLU, B_MN, GATHER) ? tile_n_arg : TILE_N;
   const int half_n = tile_n >> 1;  // columns (rows of B) each CTA of the pair loads
   const int n_blocks = SWIGLU == 1 ? (N + HALF_N - 1) / HALF_N : (N + tile_n - 1) / tile_n;
   const int num_tiles = SWIGLU == 4 ? m_blocks * (m_blocks + 1) / 2 : m_blocks * n_blocks * (SWIGLU == 5 ? rope.splits : 1);
@@ -637,7 +640,7 @@ static int launch(const void* A, const void* B, void* C, const void* R, int M, i
   int rc = A_MN ? make_map_2d_bf16(&ma, A, K, M, lda, 64, BK) : make_map_2d_bf16(&ma, A, M, K, lda, BK, CTA_M);
   if (rc) return 100 + rc;
   int pairs = num_sms / 2;
-  const int tile_n = B_MN ? TILE_N : pair_tile_width(M, N, pairs, nullptr);
+  const int tile_n = takes_width(0, B_MN, false) ? pair_tile_width(M, N, pairs, nullptr) : TILE_N;
   rc = B_MN ? make_map_2d_bf16(&mb, B, K, N, ldb, 64, BK) : make_map_2d_bf16(&mb, B, N, K, ldb, BK, tile_n / 2);
   if (rc) return 200 + rc;
   auto kern = kf_gemm_bf16_tcgen05_2cta<A_MN, B_MN, OutT>;
@@ -975,6 +978,7 @@ static int launch_logits(const void* A, const void* B, void* C, void* stats, int
   int rc = make_map_2d_bf16(&ma, A, M, K, lda, BK, CTA_M);
   if (rc) return 100 + rc;
   int pairs = num_sms / 2;
+  static_assert(takes_width(6, false, false), "its boxes of B and its statistics are tile_n wide");
   const int tile_n = pair_tile_width(M, N, pairs, nullptr);
   rc = make_map_2d_bf16(&mb, B, N, K, ldb, BK, tile_n / 2);
   if (rc) return 200 + rc;

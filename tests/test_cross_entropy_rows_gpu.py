@@ -48,3 +48,10 @@ def test_products_of_other_kernels_leave_none(native_lib):
         h, w = torch.randn(rows, k, device=DEV).bfloat16(), torch.randn(v, k, device=DEV).bfloat16()
         logits, tiles = native_lib.gemm_logits(h, w)
         assert tiles is None and torch.equal(logits, native_lib.gemm(h, w))
+
+
+@pytest.mark.parametrize("rows,v,width", [(3840, 1032, 128), (512, 9480, 160), (1024, 6152, 192), (1152, 6152, 224), (2560, 4104, 192), (1001, 12000, 224)])
+def test_tiles_of_every_width(native_lib, monkeypatch, rows, v, width):
+    """The product takes narrower column tiles where 256 columns would leave the last round nearly empty."""
+    assert native_lib.lib().kf_gemm_logits_width(rows, v, 64, native_lib.sm_count()) == width
+    test_against_double(native_lib, monkeypatch, rows, v, 64)
