@@ -473,6 +473,8 @@ __global__ void kf_embedding_bwd(const long long* __restrict__ ids, const __nv_b
 // One block per row.  logits are overwritten with d(loss)/d(logits) where
 //   loss = inv_n * sum_valid (lse - logit[label]) + z_w * inv_n * sum_valid lse^2.
 // row_nll / row_lse2 receive the per-row terms (0 for ignored rows) for a deterministic host-side sum.
+// Columns of -inf (a masked part of the vocabulary) add zeros, also where a thread has met nothing else; a NaN among them stays one.
+__device__ __forceinline__ float exp_base(float largest) { return largest == -INFINITY ? 0.f : largest; }
 constexpr int CE_THREADS = 512;
 __global__ void __launch_bounds__(CE_THREADS)
 kf_ce_fwd_bwd(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ labels,
@@ -489,20 +491,21 @@ kf_ce_fwd_bwd(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ 
     float m2 = mx;
 #pragma unroll
     for (int i = 0; i < 8; ++i) m2 = fmaxf(m2, t.v[i]);
-    float s2 = sum * __expf(mx - m2);
+    const float base = exp_base(m2);
+    float s2 = sum * __expf(mx - base);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) s2 += __expf(t.v[i] - m2);
+    for (int i = 0; i < 8; ++i) s2 += __expf(t.v[i] - base);
     mx = m2;
     sum = s2;
   }
   for (int j = nvec * 8 + threadIdx.x; j < V; j += CE_THREADS) {  // ragged tail
     const float t = __bfloat162float(lr[j]);
     const float m2 = fmaxf(mx, t);
-    sum = sum * __expf(mx - m2) + __expf(t - m2);
+    sum = sum * __expf(mx - exp_base(m2)) + __expf(t - exp_base(m2));
     mx = m2;
   }
   const float gmax = block_max(mx, red);
-  const float gsum = block_sum(mx == -INFINITY ? 0.f : sum * __expf(mx - gmax), red);
+  const float gsum = block_sum(sum * __expf(mx - exp_base(gmax)), red);
   const float lse = gmax + __logf(gsum);
   const long long label = labels[row];
   const bool valid = label >= 0 && label < V;
@@ -545,7 +548,7 @@ kf_ce_join(const float2* __restrict__ stats, int tiles, const __nv_bfloat16* __r
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = blockIdx.x * 32 + lane;
   float m = -INFINITY, s = 0.f;
   auto join = [&](const float2 p) {
-    const float m2 = fmaxf(m, p.x), base = m2 == -INFINITY ? 0.f : m2;
+    const float m2 = fmaxf(m, p.x), base = exp_base(m2);
     s = s * __expf(m - base) + p.y * __expf(p.x - base);
     m = m2;
   };
@@ -650,20 +653,21 @@ kf_ce_vp_stats(const __nv_bfloat16* __restrict__ logits, const long long* __rest
     float m2 = mx;
 #pragma unroll
     for (int i = 0; i < 8; ++i) m2 = fmaxf(m2, t.v[i]);
-    float s2 = sum * __expf(mx - m2);
+    const float base = exp_base(m2);
+    float s2 = sum * __expf(mx - base);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) s2 += __expf(t.v[i] - m2);
+    for (int i = 0; i < 8; ++i) s2 += __expf(t.v[i] - base);
     mx = m2;
     sum = s2;
   }
   for (int j = nvec * 8 + threadIdx.x; j < V; j += CE_THREADS) {
     const float t = __bfloat162float(lr[j]);
     const float m2 = fmaxf(mx, t);
-    sum = sum * __expf(mx - m2) + __expf(t - m2);
+    sum = sum * __expf(mx - exp_base(m2)) + __expf(t - exp_base(m2));
     mx = m2;
   }
   const float gmax = block_max(mx, red);
-  const float gsum = block_sum(mx == -INFINITY ? 0.f : sum * __expf(mx - gmax), red);
+  const float gsum = block_sum(sum * __expf(mx - exp_base(gmax)), red);
   if (threadIdx.x == 0) {
     const long long local = labels[row] - vocab_start;
     row_max[row] = gmax;
