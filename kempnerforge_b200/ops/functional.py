@@ -428,15 +428,16 @@ def swiglu_stacked(gu: torch.Tensor) -> torch.Tensor:
 class _SwiGLUMLPFn(torch.autograd.Function):
     """A whole SwiGLU MLP: gate | up GEMM with the activation in its epilogue, down GEMM; backward with the SwiGLU gradient in
     the epilogue of the down projection's input gradient, one input-gradient and one weight-gradient GEMM for gate and up.
-    The same roundings as :class:`_LinearFn` and :class:`_SwiGLUFn` in a row."""
+    The same roundings as :class:`_LinearFn` and :class:`_SwiGLUFn` in a row.  ``recording``: whether a graph is (a weight asks for
+    its gradient under ``no_grad`` too); without one the pre-activations are not written."""
 
     @staticmethod
-    def forward(ctx, x, wg, wu, wd):
+    def forward(ctx, x, wg, wu, wd, recording):
         cu = _cuda()
         x2 = x.reshape(-1, x.shape[-1])
         if not x2.is_contiguous():
             x2 = x2.contiguous()
-        h, gu = cu.gemm_swiglu_pair(x2, wg, wu, want_gu=any(ctx.needs_input_grad))
+        h, gu = cu.gemm_swiglu_pair(x2, wg, wu, want_gu=recording and any(ctx.needs_input_grad))
         y = cu.gemm_rows(h, [wd])
         if gu is not None:
             ctx.save_for_backward(x2, wg, wu, wd, gu, h)
@@ -453,12 +454,12 @@ class _SwiGLUMLPFn(torch.autograd.Function):
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
-        dwd = _linear_weight_grads(cu, dy2, h, [wd], need[3:])
+        dwd = _linear_weight_grads(cu, dy2, h, [wd], need[3:4])
         if not any(need[:3]):
-            return (None, None, None, *dwd)
+            return (None, None, None, *dwd, None)
         dgu = cu.gemm_swiglu_bwd(dy2, wd, gu, out=_gradient_buffer(gu))
         dx = cu.dgrad_rows(dgu, [wg, wu]).view(ctx.x_shape) if need[0] else None
-        return (dx, *_linear_weight_grads(cu, dgu, x2, [wg, wu], need[1:3]), *dwd)
+        return (dx, *_linear_weight_grads(cu, dgu, x2, [wg, wu], need[1:3]), *dwd, None)
 
 
 def swiglu_mlp(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, wd: torch.Tensor) -> torch.Tensor | None:
@@ -478,7 +479,7 @@ def swiglu_mlp(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, wd: torch.Te
         return None
     if x.is_contiguous() and x.data_ptr() % 16:
         return None
-    return _SwiGLUMLPFn.apply(x, wg, wu, wd)
+    return _SwiGLUMLPFn.apply(x, wg, wu, wd, torch.is_grad_enabled())
 
 
 # --------------------------------------------------------------------------- embedding

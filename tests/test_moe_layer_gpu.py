@@ -3,6 +3,7 @@ expert, and the SwiGLU MLP as one node, each against the separate operations it 
 
 import pytest
 import torch
+import torch.utils.checkpoint
 
 pytestmark = pytest.mark.gpu
 
@@ -164,3 +165,26 @@ def test_forms_the_one_node_mlp_leaves_to_its_parts(native_lib):
     assert call(change=lambda w: [w[0], w[1][:128].contiguous(), w[2]]) is None                     # another width
     off = torch.zeros(256 * 64 + 1, device=DEV, dtype=torch.bfloat16)[1:].view(256, 64)
     assert call(change=lambda w: [off, *w[1:]]) is None                                # off 16 bytes
+
+
+def test_pre_activations_are_written_for_a_backward_only(native_lib, monkeypatch):
+    """Parameters ask for gradients under no_grad too: evaluation, generation, the first pass of a checkpointed layer."""
+    from kempnerforge_b200.models.mlp import SwiGLUMLP
+
+    with torch.device(DEV):
+        mlp = SwiGLUMLP(256, 384).to(torch.bfloat16)
+    x = _randn(300, 256, seed=1)
+    wanted, real = [], native_lib.gemm_swiglu_pair
+    monkeypatch.setattr(native_lib, "gemm_swiglu_pair", lambda *a, want_gu: wanted.append(want_gu) or real(*a, want_gu=want_gu))
+    y = mlp(x)
+    with torch.no_grad():
+        assert torch.equal(mlp(x), y)
+    with torch.inference_mode():
+        assert torch.equal(mlp(x), y)
+    xg = x.clone().requires_grad_(True)
+    again = torch.utils.checkpoint.checkpoint(mlp, xg, use_reentrant=True)
+    again.sum().backward()
+    for p in mlp.parameters():
+        p.requires_grad_(False)
+    assert torch.equal(mlp(x), y) and torch.equal(again, y)
+    assert wanted == [True, False, False, False, True, False] and native_lib.read_status() == 0
