@@ -839,17 +839,17 @@ def gemm_fp8(a8: torch.Tensor, b8: torch.Tensor, sa: torch.Tensor, sb: torch.Ten
     return out
 
 
-def gemm_fp8_swiglu(a8: torch.Tensor, b8: torch.Tensor, sa: torch.Tensor, sb: torch.Tensor):
-    """(gu, h, maxima of h): :func:`gemm_fp8` of e4m3 operands, b8 = [gate ; up] (2F rows), :func:`swiglu_fwd` of it and
+def gemm_fp8_swiglu(a8: torch.Tensor, b8: torch.Tensor, sa: torch.Tensor, sb: torch.Tensor, want_gu: bool = True):
+    """(gu or None, h, maxima of h): :func:`gemm_fp8` of e4m3 operands, b8 = [gate ; up] (2F rows), :func:`swiglu_fwd` of it and
     :func:`fp8_absmax` of that, from one kernel."""
     m, k = a8.shape
     f = b8.shape[0] // 2
     assert b8.shape == (2 * f, k) and a8.stride(1) == 1 and b8.stride(1) == 1
-    gu = torch.empty((m, 2 * f), dtype=torch.bfloat16, device=a8.device)
+    gu = torch.empty((m, 2 * f), dtype=torch.bfloat16, device=a8.device) if want_gu else None
     h = torch.empty((m, f), dtype=torch.bfloat16, device=a8.device)
     scratch = torch.empty(1 + 8 * sm_count(), dtype=torch.float32, device=a8.device)
     count = ctypes.c_int()
-    _check(lib().kf_gemm_fp8_swiglu(a8.data_ptr(), b8.data_ptr(), h.data_ptr(), gu.data_ptr(), m, f, k, a8.stride(0), b8.stride(0), f, 2 * f,
+    _check(lib().kf_gemm_fp8_swiglu(a8.data_ptr(), b8.data_ptr(), h.data_ptr(), _ptr(gu), m, f, k, a8.stride(0), b8.stride(0), f, 2 * f,
                                     sa.data_ptr(), sb.data_ptr(), scratch.data_ptr() + 4, ctypes.byref(count), sm_count(), _stream()),
            "kf_gemm_fp8_swiglu")
     return gu, h, PartialMax(scratch, count.value)

@@ -169,7 +169,8 @@ class _Fp8SwiGLUFn(torch.autograd.Function):
     """down(silu(x Wgᵀ) * (x Wuᵀ)) with fp8 products as one node: the arithmetic of two :class:`_Fp8LinearFn` around the SwiGLU
     kernel, except that the SwiGLU and its gradient, and the maxima that the casts of their results wait for, are taken in the
     epilogues of the products before them.  The hidden activation is cast once: where a gradient of ``wd`` will be wanted
-    (``recording``) its transposed fp8 copy is written together with the other one and kept in its stead, at half its bytes."""
+    (``recording``) its transposed fp8 copy is written together with the other one and kept in its stead, at half its bytes.  The
+    pre-activations are written only where they will be read, too."""
 
     @staticmethod
     def forward(ctx, x, wg, wu, wd, recording):
@@ -180,7 +181,7 @@ class _Fp8SwiGLUFn(torch.autograd.Function):
             x2 = x2.contiguous()
         sx, x8, _ = quantize(x2)
         s_gu, w8, _ = quantized_weight((wg, wu), want_t=False)
-        gu, h, h_max = cu.gemm_fp8_swiglu(x8, w8, sx, s_gu)
+        gu, h, h_max = cu.gemm_fp8_swiglu(x8, w8, sx, s_gu, want_gu=recording and any(ctx.needs_input_grad[:3]))
         sh, h8, h8t = quantize(h, scale=h_max, want_t=recording and ctx.needs_input_grad[3])
         sd, d8, _ = quantized_weight((wd,), want_t=False)
         y = scaled_mm(h8, d8, sh, sd)

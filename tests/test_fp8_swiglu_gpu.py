@@ -128,3 +128,25 @@ def test_hidden_activation_is_kept_only_as_its_transposed_copy(native_lib):
     finally:
         fp8.quantize = quantize
     assert wanted and not any(wanted)
+
+
+@pytest.mark.parametrize("t,dim,ffn", [(16, 32, 16), (272, 144, 1024), (2048, 256, 10752)])
+def test_pre_activations_are_written_for_a_backward_only(native_lib, monkeypatch, t, dim, ffn):
+    mlp = _mlp(dim, ffn)
+    x = torch.randn(t, dim, device=DEV).bfloat16()
+    wanted, real = [], native_lib.gemm_fp8_swiglu
+    monkeypatch.setattr(native_lib, "gemm_fp8_swiglu", lambda *a, want_gu: wanted.append((want_gu, real(*a, want_gu=want_gu))) or wanted[-1][1])
+    y = mlp(x)
+    with torch.no_grad():
+        assert torch.equal(mlp(x), y)
+    for p in (mlp.gate_proj.weight, mlp.up_proj.weight):   # the gradient of the down projection alone reads the hidden activation
+        p.requires_grad_(False)
+    assert torch.equal(mlp(x), y)
+    mlp.down_proj.weight.requires_grad_(False)
+    assert torch.equal(mlp(x), y)
+    assert torch.equal(mlp(x.clone().requires_grad_(True)), y)
+    assert [w for w, _ in wanted] == [True, False, False, False, True]
+    for w, (gu, h, maxima) in wanted:
+        assert (gu is not None) == w and torch.equal(h, wanted[0][1][1])
+        assert torch.equal(maxima.scratch[1 : 1 + maxima.count].max(), h.float().abs().max())
+    assert native_lib.read_status() == 0
