@@ -91,13 +91,15 @@ kf_router_topk(const T* __restrict__ logits, RouterBias bias, int tokens, int E,
           score[j] = __expf(raw[j] - mx) / se;
         }
         atomicAdd(&sh_prob[e], score[j]);
-        sel[j] = score[j];
+        sel[j] = isnan(score[j]) ? INFINITY : score[j];
       } else {
         score[j] = 0.f;
         sel[j] = -INFINITY;
       }
     }
-    // top-k: k rounds of warp arg-max (ties: the lower expert index wins, as torch.topk does for sorted input)
+    // top-k: k rounds of warp arg-max (ties: the lower expert index wins, as torch.topk does for sorted input).  A NaN, as in every score
+    // of a token whose activations are not finite, counts as the largest, as it does for torch.topk: k experts are always found (an
+    // index beyond them would be counted and sorted by), and the token's weights are NaN.
     float wsel[MAX_K];
     int isel[MAX_K];
     float wsum = 0.f;
@@ -117,9 +119,9 @@ kf_router_topk(const T* __restrict__ logits, RouterBias bias, int tokens, int E,
           const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
           if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
         }
-        wsel[r] = bv;
+        wsel[r] = bv == INFINITY ? __int_as_float(0x7fc00000) : bv;  // scores are 1 at most
         isel[r] = bi;
-        wsum += bv;
+        wsum += wsel[r];
 #pragma unroll
         for (int j = 0; j < MAX_E_PER_LANE; ++j)
           if (lane + 32 * j == bi) sel[j] = -INFINITY;

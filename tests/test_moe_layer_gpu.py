@@ -188,3 +188,48 @@ def test_pre_activations_are_written_for_a_backward_only(native_lib, monkeypatch
         p.requires_grad_(False)
     assert torch.equal(mlp(x), y) and torch.equal(again, y)
     assert wanted == [True, False, False, False, True, False] and native_lib.read_status() == 0
+
+
+@pytest.mark.parametrize("sigmoid", [False, True])
+@pytest.mark.parametrize("t,e,k", [(1, 1, 1), (9, 8, 2), (300, 64, 6), (40, 256, 8), (33, 8, 8)])
+def test_router_of_tokens_that_are_not_finite(native_lib, sigmoid, t, e, k):
+    """A NaN is the largest, as for torch.topk: k different experts are found for every token, and its weights say what happened."""
+    from kempnerforge_b200.ops import moe_ops
+
+    clean = _randn(t, e, seed=1, dtype=torch.float32)
+    logits = clean.clone()
+    bad = {0: slice(0, e), t // 2: slice(e // 2, e), t - 1: slice(e - 1, e)}
+    for row, cols in bad.items():
+        logits[row, cols] = float("nan")
+    if t > 8:
+        logits[1], logits[2] = -torch.inf, torch.inf   # no score at all; every one the largest
+        bad |= {1: slice(0, e), 2: slice(0, e)}
+    w, idx, counts, mean, z, balance = moe_ops.route_layer(logits, None, sigmoid, k, torch.float32)
+    scores = torch.sigmoid(logits) if sigmoid else torch.softmax(logits, -1)
+    order = torch.where(scores.isnan(), torch.inf, scores).sort(dim=-1, descending=True, stable=True).indices[:, :k]
+    rows = sorted(bad)
+    assert torch.equal(idx[rows], order[rows])
+    assert torch.equal(counts, torch.bincount(idx.reshape(-1), minlength=e).float()) and int(counts.sum()) == t * k
+    assert torch.equal(w.isnan().any(1), scores.gather(1, idx).isnan().any(1) | (scores.gather(1, idx).sum(1) == 0))
+    assert torch.equal(mean.isnan(), scores.isnan().any(0)) and not z.isfinite() and (sigmoid or balance.isnan())
+    fine = [i for i in range(t) if i not in bad]
+    if fine:
+        w2, idx2, *_ = moe_ops.route_layer(clean, None, sigmoid, k, torch.float32)
+        assert torch.equal(w[fine], w2[fine]) and torch.equal(idx[fine], idx2[fine])
+    assert native_lib.read_status() == 0
+
+
+@pytest.mark.parametrize("packed,router", [(True, "sigmoid_topk"), (False, "softmax_topk")])
+def test_a_token_that_is_not_finite_keeps_to_itself(native_lib, packed, router):
+    from kempnerforge_b200.models.moe import build_moe
+
+    torch.manual_seed(4)
+    with torch.device(DEV):
+        moe = build_moe(dim=128, hidden_dim=256, num_experts=8, top_k=2, router_type=router, packed_experts=packed).to(torch.bfloat16).eval()
+    x = _randn(1, 400, 128, seed=5)
+    with torch.no_grad():
+        want = moe(x)
+        x[0, 77] = float("nan")
+        got = moe(x)
+    others = torch.arange(400, device=DEV) != 77
+    assert got[0, 77].isnan().all() and torch.equal(got[0, others], want[0, others]) and native_lib.read_status() == 0
