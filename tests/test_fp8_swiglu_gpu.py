@@ -150,3 +150,36 @@ def test_pre_activations_are_written_for_a_backward_only(native_lib, monkeypatch
         assert (gu is not None) == w and torch.equal(h, wanted[0][1][1])
         assert torch.equal(maxima.scratch[1 : 1 + maxima.count].max(), h.float().abs().max())
     assert native_lib.read_status() == 0
+
+
+@pytest.mark.parametrize("scale", [30.0, 1e-18, 1e-19])   # ordinary, mostly infinite, all beyond fp32
+@pytest.mark.parametrize("t,k,f", [(48, 64, 272), (256, 64, 1040)])
+def test_values_that_are_not_finite_in_the_epilogues(native_lib, t, k, f, scale):
+    """NaN operands and products beyond bf16: what the separate passes make of them, and the maxima that they find (NaN aside)."""
+    cu = native_lib
+    torch.manual_seed(2)
+    q = lambda rows, e5m2=False: cu.fp8_cast(torch.randn(rows, k, device=DEV).bfloat16(), torch.full((1,), 30.0, device=DEV), e5m2)[0]
+    sa, sb = (torch.full((1,), s, device=DEV) for s in (scale, scale))
+
+    def same(a, b):
+        return torch.equal(a.isnan(), b.isnan()) and torch.equal(a[~a.isnan()], b[~b.isnan()])
+
+    def largest(x):
+        x = x.float().abs()
+        return x[~x.isnan()].max() if (~x.isnan()).any() else torch.zeros((), device=DEV)
+
+    x8, w8, g8, d8 = q(t), q(2 * f), q(t, True), q(f)
+    x8[t // 2, 3], w8[f + 5, 1], d8[7, 2] = 0x7F, 0x7F, 0x7F      # NaN of e4m3
+    g8[t - 1, 0], g8[1, k - 1], g8[2, 5] = 0x7C, 0xFC, 0x7E       # inf, -inf and NaN of e5m2
+    gu = cu.gemm_fp8(x8, w8, sa, sb)
+    h = cu.swiglu_fwd(gu)
+    for want_gu in (True, False):
+        got_gu, got, maxima = cu.gemm_fp8_swiglu(x8, w8, sa, sb, want_gu)
+        assert same(got, h) and (got_gu is None or same(got_gu, gu))
+        assert torch.equal(maxima.scratch[1 : 1 + maxima.count].max(), largest(h))
+    dh = cu.gemm_fp8(g8, d8, sa, sb, a_e5m2=True)
+    for saved in (gu, torch.randn_like(gu)):
+        want = cu.swiglu_bwd(dh, saved)
+        got, maxima = cu.gemm_fp8_swiglu_bwd(g8, d8, sa, sb, saved)
+        assert same(got, want) and torch.equal(maxima.scratch[1 : 1 + maxima.count].max(), largest(want))
+    assert native_lib.read_status() == 0
