@@ -98,7 +98,7 @@ def quantized_weight(weights, want_t: bool):
 
     The quantised copies are kept on the first weight tensor and reused until a weight is written, so the
     micro-batches, the recomputation and the backward pass of one step quantise each weight once instead of once per use.
-    Every write has to move a version counter (:func:`_state`): tensor operations do, and so do this package's optimizers and
+    Every write has to move a version counter: tensor operations do, and so do this package's optimizers and
     collectives, which write through raw pointers.  A program that writes a weight through ``.data`` or a pointer of its own,
     or replays a captured optimizer step, calls ``torch.autograd.graph.increment_version(weight)`` after it.
     Copies are reused on the stream that made them only, and neither taken into a captured graph nor out of it: a replay
@@ -106,26 +106,26 @@ def quantized_weight(weights, want_t: bool):
     from kempnerforge_b200.ops import functional as F
 
     stacked = lambda: F._stack_weight_rows(weights).detach()  # noqa: E731
-    if weights[0].is_cuda and torch.cuda.is_current_stream_capturing():
-        return quantize(stacked(), want_t=want_t)
-    state = tuple(map(_state, weights)), torch.cuda.current_stream(weights[0].device).cuda_stream if weights[0].is_cuda else None
+    state = [0]
+    if weights[0].is_cuda:
+        if torch._C._cuda_isCurrentStreamCapturing():
+            return quantize(stacked(), want_t=want_t)
+        state[0] = torch._C._cuda_getCurrentRawStream(weights[0].device.index)
+    for w in weights:
+        # its version, the memory it lies in, and the version of the flat buffer that it is a view of (binding a parameter
+        # to the buffer leaves it a counter of its own, which a write of the buffer does not move)
+        flat = getattr(w, "_kf_flat", None)
+        state += w._version, w.data_ptr(), w.untyped_storage()._cdata, None if flat is None else flat.values_version
     holder = weights[0]
     cached = getattr(holder, "_kf_fp8_cache", None)
-    if cached is None or cached[0] != state or any(ref.expired() for ref in cached[4]):
+    # while a storage is referred to, no other one gets its identity
+    if cached is None or cached[0] != state or any([torch.UntypedStorage._expired(ref.cdata) for ref in cached[4]]):
         sw, w8, _ = quantize(stacked())
-        # while a storage is referred to, no other one gets its identity
         cached = [state, sw, w8, None, [StorageWeakRef(w.untyped_storage()) for w in weights]]
         holder._kf_fp8_cache = cached
     if want_t and cached[3] is None:
         cached[3] = quantize(stacked(), want_row=False, want_t=True, scale=cached[1])[2]
     return cached[1], cached[2], cached[3]
-
-
-def _state(w: torch.Tensor) -> tuple:
-    """Changes whenever a weight's values may have: its version, the memory it lies in, and the version of the flat buffer that it is
-    a view of.  (Binding a parameter to the buffer leaves it a counter of its own, which a write of the buffer does not move.)"""
-    flat = getattr(w, "_kf_flat", None)
-    return w._version, w.data_ptr(), w.untyped_storage()._cdata, None if flat is None else flat.values_version
 
 
 class _Fp8LinearFn(torch.autograd.Function):
