@@ -52,7 +52,9 @@ constexpr int BLK_K = 128;  // keys per CTA
 constexpr int BLK_Q = 64;   // queries per iteration
 constexpr int THREADS = 448;
 constexpr int TMEM_COLS = 512;
-constexpr int ST_COL = 0;     // S^T buffers 0 / 1 (fp32, 64 cols each); P^T (bf16 pairs, 32 cols) aliases each start
+// S^T buffers 0 / 1 (fp32, 64 columns each).  In place of the 32 columns of either half of the queries its warps leave bf16 pairs:
+// columns 0 - 15 P^T and 16 - 31 dS^T of the first half, 32 - 47 P^T and 48 - 63 dS^T of the second.
+constexpr int ST_COL = 0;
 constexpr int DPT_COL = 128;  // dP^T (fp32, 64 cols)
 constexpr int DQT_COL = 192;  // dQ^T (fp32, 64 cols)
 constexpr int DV_COL = 256;   // dV accumulator (fp32, HD cols)
@@ -398,8 +400,7 @@ kf_attn_bwd_tcgen05(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       tmem_st_32x16(t_s + half * HQ, pk);
       tmem_st_32x16(t_s + half * HQ + HQ / 2, dsk);
       // dS^T into shared memory, 128B-swizzled rows (16-byte chunk c of row r lives at chunk c ^ (r % 8));
-      // the previous iteration's dK / dQ MMAs must have finished reading it
-      // (two buffers: the MMAs of iteration it-2 were the last readers of this one)
+      // the dQ MMAs, its only readers, must have finished with it (two buffers: those of iteration it-2 were this one's last)
       if (it > 1 && ok && !mbar_wait(ds_free(it & 1), ((it >> 1) - 1) & 1, status, KF_ERR_WAIT_TMEM_FULL)) ok = false;
       {
         uint8_t* row_ptr = ds_gen + (it & 1) * DS_BYTES + r_local * 128;

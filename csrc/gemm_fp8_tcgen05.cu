@@ -583,7 +583,8 @@ int kf_fp8_absmax_bf16(const void* x, long long n, void* partial, int* count, vo
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
-// scale[0] = fp8_max / absmax(x) for n bf16 values; amax_scratch holds AMAX_BLOCKS (1024) floats.
+// scale[0] = fp8_max / absmax(x) for n bf16 values; amax_scratch holds AMAX_BLOCKS (1024) floats.  For callers that want the scale
+// itself (tests, benchmarks): the fp8 layers leave it to the cast, which makes it of the partial maxima.
 int kf_fp8_scale_bf16(const void* x, long long n, int e5m2, void* amax_scratch, void* scale, void* stream) {
   using namespace kf::f8;
   int count = 0;

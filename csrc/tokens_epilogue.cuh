@@ -1,5 +1,5 @@
 // Epilogue of the CTA-pair kernels whose tiles have weight rows (features) as the M side and tokens as the N side
-// (gemm_tokens_tcgen05_2cta.cu, grouped_tokens_tcgen05_2cta.cu).
+// (gemm_tokens_tcgen05_2cta.cu, grouped_gemm_tcgen05_2cta.cu).
 //
 // The accumulator holds a feature per lane and a token per column.  The epilogue turns 32 x 32 blocks through shared memory
 // (fp32, XOR-swizzled 16-byte chunks: no bank conflicts), after which a lane holds 32 features of one token, as in the

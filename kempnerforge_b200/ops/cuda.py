@@ -795,7 +795,8 @@ def fp8_absmax(x2: torch.Tensor) -> PartialMax:
 
 
 def fp8_scale(x2: torch.Tensor, e5m2: bool = False) -> torch.Tensor:
-    """Device scalar fp8_max / absmax(x) (fp32, shape (1,))."""
+    """Device scalar fp8_max / absmax(x) (fp32, shape (1,)), for callers that want the scale itself; the fp8 layers leave it to
+    :func:`fp8_cast`."""
     scratch = torch.empty(1 + 1024, dtype=torch.float32, device=x2.device)   # the scale, then partial maxima
     if not x2.is_contiguous():
         x2 = x2.contiguous()
