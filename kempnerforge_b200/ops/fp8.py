@@ -93,6 +93,18 @@ def scaled_mm(a8, b8, sa, sb, a_e5m2=False, b_e5m2=False, out=None, accumulate=F
     return out
 
 
+class _Copies:
+    """The fp8 copies of (stacked) weights, kept on the first of them; a weight that is pickled or copied takes none along."""
+
+    __slots__ = ("state", "storages", "scale", "row", "transposed")
+
+    def __init__(self, state, storages, scale, row) -> None:
+        self.state, self.storages, self.scale, self.row, self.transposed = state, storages, scale, row, None
+
+    def __reduce__(self):
+        return type(None), ()
+
+
 def quantized_weight(weights, want_t: bool):
     """(scale, row-major fp8, transposed fp8 or None) of the weights stacked along the output dimension.
 
@@ -119,13 +131,12 @@ def quantized_weight(weights, want_t: bool):
     holder = weights[0]
     cached = getattr(holder, "_kf_fp8_cache", None)
     # while a storage is referred to, no other one gets its identity
-    if cached is None or cached[0] != state or any([torch.UntypedStorage._expired(ref.cdata) for ref in cached[4]]):
+    if type(cached) is not _Copies or cached.state != state or any([torch.UntypedStorage._expired(ref.cdata) for ref in cached.storages]):
         sw, w8, _ = quantize(stacked())
-        cached = [state, sw, w8, None, [StorageWeakRef(w.untyped_storage()) for w in weights]]
-        holder._kf_fp8_cache = cached
-    if want_t and cached[3] is None:
-        cached[3] = quantize(stacked(), want_row=False, want_t=True, scale=cached[1])[2]
-    return cached[1], cached[2], cached[3]
+        cached = holder._kf_fp8_cache = _Copies(state, [StorageWeakRef(w.untyped_storage()) for w in weights], sw, w8)
+    if want_t and cached.transposed is None:
+        cached.transposed = quantize(stacked(), want_row=False, want_t=True, scale=cached.scale)[2]
+    return cached.scale, cached.row, cached.transposed
 
 
 class _Fp8LinearFn(torch.autograd.Function):

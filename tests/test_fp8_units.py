@@ -189,10 +189,10 @@ def test_copies_do_not_outlive_the_memory_that_the_weights_lay_in():
     """A parameter that goes to another memory and back may find its old address, with other values and the same version."""
     w = _tagged_linear().weight
     _bytes([w])
-    refs = w._kf_fp8_cache[4]
+    refs = w._kf_fp8_cache.storages
     w.data = w.data * -3
     assert all(r.expired() for r in refs) and all(torch.equal(a, b) for a, b in zip(_bytes([w]), _fresh([w])))
-    w._kf_fp8_cache[1:] = None, None, None, refs    # the state of now, made of a memory that is gone
+    w._kf_fp8_cache = fp8._Copies(w._kf_fp8_cache.state, refs, None, None)   # the state of now, made of a memory that is gone
     assert all(torch.equal(a, b) for a, b in zip(_bytes([w]), _fresh([w])))
 
 
@@ -206,3 +206,25 @@ def test_the_input_gradient_takes_scale_and_copy_of_the_same_weights():
     y.backward(g)
     want = g.float() @ weights[0].detach().float()
     assert (x.grad.float() - want).norm() < 0.15 * want.norm()   # e5m2 gradients, e4m3 weights
+
+
+@pytest.mark.parametrize("copy_of", ["saved", "copied"])
+def test_saved_and_copied_models_carry_no_copies(copy_of):
+    import copy
+    import io
+
+    lin = _tagged_linear()
+    _bytes([lin.weight])
+    if copy_of == "saved":
+        file = io.BytesIO()
+        torch.save(lin, file)
+        file.seek(0)
+        other = torch.load(file, weights_only=False)
+        assert fp8.is_fp8_weight(other.weight)
+    else:
+        other = copy.deepcopy(lin)
+    assert getattr(other.weight, "_kf_fp8_cache", None) is None
+    other.weight.data.mul_(-3)
+    assert all(torch.equal(a, b) for a, b in zip(_bytes([other.weight]), _fresh([other.weight])))
+    old = other.weight._kf_fp8_cache = [(0, 0), None, None, None]    # what a file of an earlier form brings along
+    assert all(torch.equal(a, b) for a, b in zip(_bytes([other.weight]), _fresh([other.weight]))) and other.weight._kf_fp8_cache is not old
