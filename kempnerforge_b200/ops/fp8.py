@@ -122,15 +122,15 @@ def quantized_weight(weights, want_t: bool):
     if weights[0].is_cuda:
         if torch._C._cuda_isCurrentStreamCapturing():
             return quantize(stacked(), want_t=want_t)
-        state[0] = torch._C._cuda_getCurrentRawStream(weights[0].device.index)
+        state[0] = torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
     for w in weights:
-        # its version, the memory it lies in, and the version of the flat buffer that it is a view of (binding a parameter
-        # to the buffer leaves it a counter of its own, which a write of the buffer does not move)
+        # its version, its address, and the version of the flat buffer that it is a view of (binding a parameter to the buffer
+        # leaves it a counter of its own, which a write of the buffer does not move)
         flat = getattr(w, "_kf_flat", None)
-        state += w._version, w.data_ptr(), w.untyped_storage()._cdata, None if flat is None else flat.values_version
+        state += w._version, w.data_ptr(), None if flat is None else flat.values_version
     holder = weights[0]
     cached = getattr(holder, "_kf_fp8_cache", None)
-    # while a storage is referred to, no other one gets its identity
+    # where the storage that held an address is alive, no other one does
     if type(cached) is not _Copies or cached.state != state or any([torch.UntypedStorage._expired(ref.cdata) for ref in cached.storages]):
         sw, w8, _ = quantize(stacked())
         cached = holder._kf_fp8_cache = _Copies(state, [StorageWeakRef(w.untyped_storage()) for w in weights], sw, w8)
