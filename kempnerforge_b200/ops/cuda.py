@@ -670,8 +670,13 @@ def scale_(x: torch.Tensor, factor: torch.Tensor) -> torch.Tensor:
 _DT = {torch.bfloat16: 0, torch.float32: 1}
 
 
-# A kernel writes through an address, which autograd and everything kept by a tensor's version (fp8 copies of weights) do not see
-_wrote = torch.autograd.graph.increment_version
+# A kernel writes through an address, which what is kept by a tensor's version (fp8 copies of weights) does not see.  A flat buffer's version
+# is moved; a parameter's own is not, because graphs that hold the parameter would be refused by it: it carries a count.
+_wrote_buffer = torch.autograd.graph.increment_version
+
+
+def _wrote_parameter(p: torch.Tensor) -> None:
+    p._kf_writes = getattr(p, "_kf_writes", 0) + 1
 
 
 def adamw_flat(p, g, m, v, n_decay: int, lr: float, beta1: float, beta2: float, eps: float, wd: float,
@@ -688,7 +693,7 @@ def adamw_flat(p, g, m, v, n_decay: int, lr: float, beta1: float, beta2: float, 
         ),
         "kf_adamw_flat",
     )
-    _wrote(p)
+    _wrote_buffer(p)
 
 
 def sumsq(x: torch.Tensor, out: torch.Tensor, accumulate: bool = False) -> torch.Tensor:
@@ -974,7 +979,7 @@ def lion_step(p, g, m, lr: float, b1: float, b2: float, wd: float) -> bool:
     if getattr(lib(), "kf_lion", None) is None or not _same_flat(p, g, m):
         return False
     _check(lib().kf_lion(p.data_ptr(), g.data_ptr(), m.data_ptr(), p.numel(), _DT[p.dtype], lr, b1, b2, wd, _stream()), "kf_lion")
-    _wrote(p)
+    _wrote_parameter(p)
     return True
 
 
@@ -984,7 +989,7 @@ def sf_adamw_step(y, g, z, v, x, lr, b1, b2, eps, wd, bc2, ck, first: bool) -> b
         return False
     _check(lib().kf_sf_adamw(y.data_ptr(), g.data_ptr(), z.data_ptr(), v.data_ptr(), x.data_ptr(), y.numel(), _DT[y.dtype],
                              lr, b1, b2, eps, wd, bc2, ck, int(first), _stream()), "kf_sf_adamw")
-    _wrote(y)
+    _wrote_parameter(y)
     return True
 
 

@@ -110,8 +110,8 @@ def quantized_weight(weights, want_t: bool):
 
     The quantised copies are kept on the first weight tensor and reused until a weight is written, so the
     micro-batches, the recomputation and the backward pass of one step quantise each weight once instead of once per use.
-    Every write has to move a version counter: tensor operations do, and so do this package's optimizers and
-    collectives, which write through raw pointers.  A program that writes a weight through ``.data`` or a pointer of its own,
+    Tensor operations move a version counter; this package's optimizers and collectives, which write through raw pointers, move
+    one or count their writes.  A program that writes a weight through ``.data`` or a pointer of its own,
     or replays a captured optimizer step, calls ``torch.autograd.graph.increment_version(weight)`` after it.
     Copies are reused on the stream that made them only, and neither taken into a captured graph nor out of it: a replay
     reads the weights as they are then."""
@@ -124,10 +124,11 @@ def quantized_weight(weights, want_t: bool):
             return quantize(stacked(), want_t=want_t)
         state[0] = torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
     for w in weights:
-        # its version, its address, and the version of the flat buffer that it is a view of (binding a parameter to the buffer
-        # leaves it a counter of its own, which a write of the buffer does not move)
-        flat = getattr(w, "_kf_flat", None)
-        state += w._version, w.data_ptr(), None if flat is None else flat.values_version
+        # its version, its address, the writes of kernels, and the version of the flat buffer that it is a view of (binding a
+        # parameter to the buffer leaves it a counter of its own, which a write of the buffer does not move)
+        own = w.__dict__.get
+        flat = own("_kf_flat")
+        state += w._version, w.data_ptr(), own("_kf_writes"), None if flat is None else flat.values_version
     holder = weights[0]
     cached = getattr(holder, "_kf_fp8_cache", None)
     # where the storage that held an address is alive, no other one does

@@ -88,3 +88,21 @@ def test_copies_belong_to_the_stream_that_made_them(native_lib):
         there = fp8.quantized_weight(weights, want_t=True)
     torch.cuda.current_stream().wait_stream(side)
     assert there[1] is not here[1] and all(torch.equal(a, b) for a, b in zip(here, there))
+
+
+@pytest.mark.parametrize("how", ["lion", "schedule free"])
+def test_a_kept_graph_still_runs_after_a_native_update(native_lib, how):
+    """A second backward pass reads the weights as they are then, as before their writes were counted."""
+    from kempnerforge_b200.training import optimizer as o
+
+    torch.manual_seed(5)
+    lin = torch.nn.Linear(256, 128, bias=False, device=DEV, dtype=torch.bfloat16)
+    from kempnerforge_b200.ops import functional as F
+
+    x = torch.randn(64, 256, device=DEV).bfloat16().requires_grad_(True)
+    y = F.linear(x, lin.weight)
+    y.sum().backward(retain_graph=True)
+    {"lion": o.Lion, "schedule free": o.ScheduleFreeAdamW}[how](lin.parameters(), lr=0.5).step()
+    x.grad = None
+    y.sum().backward()
+    assert torch.allclose(x.grad.float(), lin.weight.detach().float().sum(0).expand(64, -1), rtol=2**-7, atol=2**-5)
